@@ -31,7 +31,7 @@
 extern "C" {
 #endif
 
-#define KB200_ABI_VERSION 3
+#define KB200_ABI_VERSION 4
 
 #define KB200_MAX_RANK 6      /* iteration dims after the host collapsed contiguous ones */
 #define KB200_MAX_OPERANDS 12 /* distinct tensors one fused kernel touches */
@@ -231,6 +231,19 @@ int kb200_plan_set_option(kb200_plan* plan, int option, int value);
  * Takes the place of the launch loop GPUExecutable._run
  * (kiln/gpu/runtime.py:164-179).  No synchronisation, no allocation. */
 int kb200_plan_launch(kb200_plan* plan, void* cuda_stream);
+
+/* 1 when every kernel that touches a graph input or output can be pointed at another buffer without
+ * binding again, so that kb200_plan_run may be used; 0 otherwise (the fused attention reads an input
+ * or writes an output itself) and for an unbound plan. */
+int kb200_plan_relocatable(const kb200_plan* plan);
+
+/* kb200_plan_launch on this call's own input and output buffers (null entry: the bound one), so that
+ * a call needs no copies into and out of fixed buffers.  The reference captures its launches over
+ * fixed addresses and copies both ways (kiln/gpu/runtime.py:181-217).  Buffers have the size and
+ * the 16-byte alignment of the bound ones, and an output overlaps no input.  Needs a relocatable
+ * plan.  No synchronisation, no allocation. */
+int kb200_plan_run(kb200_plan* plan, void* const* inputs, int n_inputs, void* const* outputs, int n_outputs,
+                   void* cuda_stream);
 
 /* Enqueues kernel `i` alone (profiling, autotuning). */
 int kb200_kernel_launch(kb200_plan* plan, int i, void* cuda_stream);

@@ -125,6 +125,16 @@ struct Plan {
   uint64_t arena_bytes = 0;
   std::vector<float*> consts, inputs, outputs;
   std::vector<uint64_t> const_bytes, input_bytes, output_bytes;
+  // Operands that lie in a graph input or output, and where those buffers are at the moment: a call may
+  // bring buffers of its own (kb200_plan_run)
+  struct IoRef {
+    int kernel, slot;
+    int buffer;          // inputs first, then outputs
+    int64_t offset;      // elements from the buffer's start
+  };
+  std::vector<IoRef> io_refs;
+  std::vector<float*> io_now;
+  bool relocatable = false;
 };
 
 // ---- tape analysis (host) ----
@@ -142,6 +152,7 @@ int choose_reduce(Plan& plan, PlanKernel& k);
 int launch_reduce(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 int choose_matmul(Plan& plan, PlanKernel& k);
 int bind_matmul(Plan& plan, PlanKernel& k);      // after pointers are resolved
+bool repoint_matmul(PlanKernel& k);              // operand pointers changed: follow in tensor maps and parameters
 bool matmul_wants_bf16_operands(const PlanKernel& k);
 void attention_set_shadow(PlanKernel& k, void* shadow_out);
 bool attention_operand_span(const PlanKernel& k, const float** lo, const float** hi);

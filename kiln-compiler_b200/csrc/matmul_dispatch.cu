@@ -8,6 +8,7 @@ bool tc_eligible(const PlanKernel& k);
 int tc_bind(Plan& plan, PlanKernel& k, int kernel_index);
 int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 void tc_destroy(PlanKernel& k);
+bool tc_repoint(PlanKernel& k);
 
 int choose_matmul(Plan& plan, PlanKernel& k) {
   (void)plan;
@@ -37,6 +38,8 @@ int launch_matmul(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   if (k.impl == IMPL_MM_TC) return tc_launch(plan, k, s);
   return launch_matmul_simt(plan, k, s);
 }
+
+bool repoint_matmul(PlanKernel& k) { return tc_repoint(k); }
 
 void destroy_matmul(PlanKernel& k) { tc_destroy(k); }
 

@@ -784,6 +784,18 @@ int pair_launch(const Plan& plan, const void* state, cudaStream_t s) {
   return KB200_OK;
 }
 
+bool pair_repoint(const PlanKernel& k, void* state, const void* a, const void* b) {
+  PairState* st = static_cast<PairState*>(state);
+  bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b)) &&
+            set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr);
+  for (int s = 0; s < st->params.n_steps && ok; ++s) {
+    const int slot = k.chain.steps[s].slot;
+    if (st->params.steps[s].kind == SIDE_COL) st->params.steps[s].ptr = k.ops[slot].ptr;
+    if (st->params.steps[s].kind == SIDE_RES) ok = set_map_address(&st->map_res, k.ops[slot].ptr);
+  }
+  return ok;
+}
+
 void pair_destroy(void* state) { delete static_cast<PairState*>(state); }
 
 }  // namespace kb200

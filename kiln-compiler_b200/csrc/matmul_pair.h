@@ -23,6 +23,8 @@ bool pair_eligible(const Plan& plan, const PlanKernel& k);
 // then uses the single-CTA kernel); a non-zero return is an error.
 int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, void** state);
 int pair_launch(const Plan& plan, const void* state, cudaStream_t s);
+// Follows moved operand pointers of `k`; `a` / `b` null: that operand's map stays.
+bool pair_repoint(const PlanKernel& k, void* state, const void* a, const void* b);
 void pair_destroy(void* state);
 
 }  // namespace kb200

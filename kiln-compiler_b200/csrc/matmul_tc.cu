@@ -1294,6 +1294,22 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   return KB200_OK;
 }
 
+// The operand pointers of `k` have moved (graph inputs and outputs of another call): the tensor maps
+// that hold their addresses follow.  Operands that are read from a bf16 copy keep its map; the pass
+// that fills the copy takes its source from `k`.
+bool tc_repoint(PlanKernel& k) {
+  TcState* st = static_cast<TcState*>(k.tc);
+  if (!st) return true;
+  const kb200_kernel_desc& d = k.desc;
+  for (int o = 0; o < k.n_ops; ++o) st->params.mm.ops[o].ptr = k.ops[o].ptr;
+  const void* a = st->bf16 ? nullptr : k.ops[d.a_slot].ptr;
+  const void* b = st->bf16 ? nullptr : k.ops[d.b_slot].ptr;
+  if (st->pair) return pair_repoint(k, st->pair, a, b);
+  bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b));
+  if (st->params.store_mode == 1) ok = ok && set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr);
+  return ok;
+}
+
 void tc_destroy(PlanKernel& k) {
   TcState* st = static_cast<TcState*>(k.tc);
   if (!st) return;

@@ -919,6 +919,8 @@ static int assign_shadows(Plan& plan) {
   return KB200_OK;
 }
 
+constexpr size_t kMaxIo = 16;      // inputs and outputs (each) a call may bring buffers for
+
 static int launch_one(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   if (numel_of(k.desc) == 0 || k.impl == IMPL_FUSED_AWAY) return KB200_OK;
   if (k.impl == IMPL_ATTN_FUSED) return attention_launch(plan, k, s);
@@ -928,6 +930,65 @@ static int launch_one(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     case KB200_K_REDUCE: return launch_reduce(plan, k, s);
     default: return launch_matmul(plan, k, s);
   }
+}
+
+// Every operand that lies inside a bound graph input or output, whatever pass pointed it there.
+static void collect_io_refs(Plan& plan) {
+  plan.io_refs.clear();
+  plan.io_now = plan.inputs;
+  plan.io_now.insert(plan.io_now.end(), plan.outputs.begin(), plan.outputs.end());
+  std::vector<uint64_t> bytes = plan.input_bytes;
+  bytes.insert(bytes.end(), plan.output_bytes.begin(), plan.output_bytes.end());
+  plan.relocatable = true;
+  for (size_t b = 0; b < plan.io_now.size(); ++b)
+    if (reinterpret_cast<uintptr_t>(plan.io_now[b]) & 15) plan.relocatable = false;     // implementations were chosen for this alignment
+  int covered = 0;           // kernels still covered by the fused attention met last: their operands are the fused kernel's
+  for (size_t i = 0; i < plan.kernels.size(); ++i) {
+    const PlanKernel& k = plan.kernels[i];
+    if (k.impl == IMPL_ATTN_FUSED) covered = attention_chain_length(k);
+    for (int o = 0; o < k.n_ops; ++o)
+      for (size_t b = 0; b < plan.io_now.size(); ++b) {
+        const float* lo = plan.io_now[b];
+        if (k.ops[o].ptr < lo || k.ops[o].ptr >= lo + bytes[b] / 4) continue;
+        if (covered > 0) plan.relocatable = false;
+        plan.io_refs.push_back({(int)i, o, (int)b, k.ops[o].ptr - lo});
+      }
+    if (covered > 0) --covered;
+  }
+}
+
+// Points the plan at these buffers.  What moved is a handful of pointers and tensor-map addresses on the
+// host; launches already enqueued took theirs by value.
+static int repoint(Plan& plan, float* const* want) {
+  bool moved = false;
+  for (size_t b = 0; b < plan.io_now.size(); ++b) moved = moved || want[b] != plan.io_now[b];
+  if (!moved) return KB200_OK;
+  for (size_t r = 0; r < plan.io_refs.size(); ++r) {
+    const Plan::IoRef& ref = plan.io_refs[r];
+    PlanKernel& k = plan.kernels[ref.kernel];
+    k.ops[ref.slot].ptr = want[ref.buffer] + ref.offset;
+    const bool last_of_kernel = r + 1 == plan.io_refs.size() || plan.io_refs[r + 1].kernel != ref.kernel;
+    if (last_of_kernel && k.impl == IMPL_MM_TC && !repoint_matmul(k))
+      return fail(KB200_ERR_CUDA, "kernel %d (%s): a tensor map could not be pointed at the call's buffers", ref.kernel, k.desc.name);
+  }
+  for (size_t b = 0; b < plan.io_now.size(); ++b) plan.io_now[b] = want[b];
+  return KB200_OK;
+}
+
+static int repoint_to_bound(Plan& plan) {
+  float* want[2 * kMaxIo];
+  if (plan.io_now.size() > 2 * kMaxIo) return KB200_OK;      // such a plan never left its bound buffers
+  for (size_t b = 0; b < plan.io_now.size(); ++b)
+    want[b] = b < plan.inputs.size() ? plan.inputs[b] : plan.outputs[b - plan.inputs.size()];
+  return repoint(plan, want);
+}
+
+static int launch_all(Plan& plan, cudaStream_t s) {
+  for (size_t i = 0; i < plan.kernels.size(); ++i) {
+    int rc = launch_one(plan, plan.kernels[i], s);
+    if (rc) return rc;
+  }
+  return KB200_OK;
 }
 
 }  // namespace kb200
@@ -1049,6 +1110,7 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   }
   cudaSetDevice(prev);
   if (rc) return rc;
+  collect_io_refs(plan);
   plan.bound = true;
   return KB200_OK;
 }
@@ -1073,11 +1135,33 @@ KB200_EXPORT int kb200_plan_launch(kb200_plan* p, void* stream) {
   if (p == nullptr) return fail(KB200_ERR_ARGUMENT, "kb200_plan_launch: plan is null");
   Plan& plan = *reinterpret_cast<Plan*>(p);
   if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_plan_launch: call kb200_plan_bind first");
-  for (size_t i = 0; i < plan.kernels.size(); ++i) {
-    int rc = launch_one(plan, plan.kernels[i], static_cast<cudaStream_t>(stream));
-    if (rc) return rc;
+  const int rc = repoint_to_bound(plan);
+  return rc ? rc : launch_all(plan, static_cast<cudaStream_t>(stream));
+}
+
+KB200_EXPORT int kb200_plan_relocatable(const kb200_plan* p) {
+  if (p == nullptr) return 0;
+  const Plan& plan = *reinterpret_cast<const Plan*>(p);
+  return plan.bound && plan.relocatable && plan.inputs.size() <= kMaxIo && plan.outputs.size() <= kMaxIo ? 1 : 0;
+}
+
+KB200_EXPORT int kb200_plan_run(kb200_plan* p, void* const* inputs, int n_inputs, void* const* outputs, int n_outputs,
+                                void* stream) {
+  if (p == nullptr) return fail(KB200_ERR_ARGUMENT, "kb200_plan_run: plan is null");
+  Plan& plan = *reinterpret_cast<Plan*>(p);
+  if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_plan_run: call kb200_plan_bind first");
+  if (!kb200_plan_relocatable(p)) return fail(KB200_ERR_UNSUPPORTED, "kb200_plan_run: this plan runs on its bound buffers only");
+  if (n_inputs != (int)plan.inputs.size() || n_outputs != (int)plan.outputs.size() || (n_inputs && !inputs) || (n_outputs && !outputs))
+    return fail(KB200_ERR_ARGUMENT, "kb200_plan_run: %d inputs and %d outputs, the plan has %d and %d", n_inputs, n_outputs,
+                (int)plan.inputs.size(), (int)plan.outputs.size());
+  float* want[2 * kMaxIo];
+  for (int b = 0; b < n_inputs + n_outputs; ++b) {
+    void* own = b < n_inputs ? inputs[b] : outputs[b - n_inputs];
+    if (reinterpret_cast<uintptr_t>(own) & 15) return fail(KB200_ERR_ARGUMENT, "kb200_plan_run: buffer %d is not 16-byte aligned", b);
+    want[b] = own ? static_cast<float*>(own) : (b < n_inputs ? plan.inputs[b] : plan.outputs[b - n_inputs]);
   }
-  return KB200_OK;
+  const int rc = repoint(plan, want);
+  return rc ? rc : launch_all(plan, static_cast<cudaStream_t>(stream));
 }
 
 KB200_EXPORT int kb200_kernel_launch(kb200_plan* p, int i, void* stream) {
@@ -1085,6 +1169,7 @@ KB200_EXPORT int kb200_kernel_launch(kb200_plan* p, int i, void* stream) {
   Plan& plan = *reinterpret_cast<Plan*>(p);
   if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_kernel_launch: call kb200_plan_bind first");
   if (i < 0 || i >= (int)plan.kernels.size()) return fail(KB200_ERR_ARGUMENT, "kb200_kernel_launch: no kernel %d", i);
+  if (const int rc = repoint_to_bound(plan)) return rc;
   return launch_one(plan, plan.kernels[i], static_cast<cudaStream_t>(stream));
 }
 

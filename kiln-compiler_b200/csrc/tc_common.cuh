@@ -356,6 +356,20 @@ inline bool encode_map_store(CUtensorMap* map, bool bf16, const void* base, int6
   return r == CUDA_SUCCESS;
 }
 
+// Another (16-byte aligned) address for an encoded map of the same shape and strides.
+inline bool set_map_address(CUtensorMap* map, const void* base) {
+  using Fn = CUresult (*)(CUtensorMap*, void*);
+  static const Fn fn = [] {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &sym, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<Fn>(sym)
+               : nullptr;
+  }();
+  return fn != nullptr && fn(map, const_cast<void*>(base)) == CUDA_SUCCESS;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 

@@ -8,18 +8,23 @@ missing, ``load()`` raises and nothing above it can run.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 from pathlib import Path
 
-ABI_VERSION = 3
+ABI_VERSION = 4
 MAX_RANK, MAX_OPERANDS, MAX_TAPE = 6, 12, 96
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC_DIR = PKG_DIR.parent / "csrc"
 INCLUDE_DIR = PKG_DIR.parent.parent / "include"
 LIB_PATH = PKG_DIR / "_lib" / "libkb200.so"
+CALL_SOURCE = CSRC_DIR / "host_call.cpp"
+CALL_PATH = PKG_DIR / "_lib" / "_kb200_call.so"
 
 K_ELEMENTWISE, K_ROW, K_REDUCE, K_MATMUL = 0, 1, 2, 3
 OPT_FUSE_ATTENTION = 1
@@ -69,6 +74,8 @@ EXPORTS = {
                                   C.POINTER(C.c_void_p), C.POINTER(C.c_uint64), C.c_int]),
     "kb200_plan_set_option": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "kb200_plan_launch": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "kb200_plan_relocatable": (C.c_int, [C.c_void_p]),
+    "kb200_plan_run": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p), C.c_int, C.POINTER(C.c_void_p), C.c_int, C.c_void_p]),
     "kb200_kernel_launch": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p]),
     "kb200_plan_launch_count": (C.c_int, [C.c_void_p]),
     "kb200_kernel_impl": (C.c_char_p, [C.c_void_p, C.c_int]),
@@ -82,6 +89,7 @@ EXPORTS = {
 }
 
 _lib = None
+_call = None
 
 
 def sources():
@@ -105,8 +113,37 @@ def needs_build():
     return any(d.stat().st_mtime > built for d in deps)
 
 
+def build_call(force=False):
+    """Compile csrc/host_call.cpp, the native side of GPUExecutable.__call__, against the installed torch."""
+    deps = [CALL_SOURCE, INCLUDE_DIR / "kb200.h"]
+    if not force and CALL_PATH.exists() and all(d.stat().st_mtime <= CALL_PATH.stat().st_mtime for d in deps):
+        return CALL_PATH
+    import torch
+    from torch.utils import cpp_extension
+
+    lib_dir = str(Path(torch.__file__).resolve().parent / "lib")
+    tmp = CALL_PATH.with_suffix(f".{os.getpid()}.tmp.so")
+    cmd = ["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{INCLUDE_DIR}", f"-I{sysconfig.get_paths()['include']}",
+           *[f"-isystem{p}" for p in cpp_extension.include_paths("cuda")], str(CALL_SOURCE), "-o", str(tmp),
+           f"-L{LIB_PATH.parent}", "-lkb200", f"-L{lib_dir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+           "-Wl,-rpath,$ORIGIN"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        tmp.unlink(missing_ok=True)
+        raise RuntimeError(f"kiln_b200: g++ failed\n{proc.stdout}\n{proc.stderr}")
+    tmp.replace(CALL_PATH)
+    return CALL_PATH
+
+
 def build(force=False, verbose=False):
-    """Compile csrc/*.cu into libkb200.so for sm_100a (cross-compiles without a GPU)."""
+    """Compile csrc/*.cu into libkb200.so for sm_100a (cross-compiles without a GPU), and the call extension."""
+    build_library(force, verbose)
+    build_call(force)
+    return LIB_PATH
+
+
+def build_library(force=False, verbose=False):
     if not force and not needs_build():
         return LIB_PATH
     if shutil.which("nvcc") is None:
@@ -139,6 +176,22 @@ def load():
         raise RuntimeError(f"kiln_b200: libkb200.so has ABI {lib.kb200_version()}, expected {ABI_VERSION}; rebuild")
     _lib = lib
     return lib
+
+
+def load_call():
+    """The call extension (csrc/host_call.cpp).  Raises if it is missing: there is no slower stand-in."""
+    global _call
+    if _call is None:
+        load()
+        import torch  # noqa: F401  (the extension's symbols come from torch's libraries)
+
+        if not CALL_PATH.exists():
+            raise RuntimeError(f"kiln_b200: {CALL_PATH} is missing; run kiln_b200.build()")
+        loader = importlib.machinery.ExtensionFileLoader("_kb200_call", str(CALL_PATH))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_kb200_call", loader))
+        loader.exec_module(module)
+        _call = module
+    return _call
 
 
 def check(status, lib=None):

@@ -142,6 +142,25 @@ def _ptr_array(tensors):
     return ptrs, sizes, n
 
 
+# A call of a plan of up to this many launches enqueues them on the caller's own tensors, with no copy in,
+# no graph and no clone out: a launch costs the host about 2 us, less than a kernel runs, and a graph
+# replay costs the GPU about that much per kernel besides ~5 us to begin.  Plans of more, smaller
+# kernels (nothing fused) are bound by the launches and replay a graph over fixed buffers.  A block of
+# the benchmark is 7 to 9 launches.
+DIRECT_LAUNCHES = 9
+
+
+def _usable(t, device):
+    """Can the kernels work on this tensor where it is?"""
+    return (t.device == device and t.dtype == torch.float32 and t.is_contiguous() and not t.is_neg() and t.numel() > 0
+            and t.data_ptr() % 16 == 0)
+
+
+def _overlap(a, b):
+    lo, hi = a.data_ptr(), b.data_ptr()
+    return lo < hi + 4 * b.numel() and hi < lo + 4 * a.numel()
+
+
 class GPUExecutable:
     """Runs one compiled graph on the GPU. Not reentrant: calls share one arena."""
 
@@ -223,6 +242,12 @@ class GPUExecutable:
         self.device_launches = self._lib.kb200_plan_launch_count(self._plan)
         self.graph = None
         self.use_cuda_graphs = bool(cuda_graphs)
+        self.relocatable = bool(self._lib.kb200_plan_relocatable(self._plan))
+        self._call_lib = _cabi.load_call()
+        self._caller = None
+        if self.relocatable and self.device_launches <= DIRECT_LAUNCHES:
+            self._caller = self._call_lib.caller(self._plan.value, self.device.index, self.input_shapes, self.output_shapes,
+                                                 self.static_inputs)
 
     # -- binding and launching ------------------------------------------------------------
 
@@ -285,7 +310,32 @@ class GPUExecutable:
         else:
             self._launch()
 
+    def run_on(self, inputs, outputs):
+        """Enqueue the kernels on these tensors where they can be used as they are (float32, contiguous,
+        16-byte aligned, on the device; an output overlapping no input) and through the static buffers
+        otherwise.  Capturable; the tensors' addresses are part of a captured graph."""
+        inputs = [t.detach() for t in inputs]
+        direct = [self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) for t, shape in zip(inputs, self.input_shapes)]
+        for static, t, d in zip(self.static_inputs, inputs, direct):
+            if not d:
+                static.copy_(t, non_blocking=True)
+        read = [t if d else static for static, t, d in zip(self.static_inputs, inputs, direct)]
+        written = [t if self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) and not any(_overlap(t, r) for r in read)
+                   else static for static, t, shape in zip(self.static_outputs, outputs, self.output_shapes)]
+        if self.relocatable:
+            ip, _, in_ = _ptr_array(read)
+            op, _, on = _ptr_array(written)
+            stream = torch.cuda.current_stream(self.device).cuda_stream
+            _cabi.check(self._lib.kb200_plan_run(self._plan, ip, in_, op, on, C.c_void_p(stream)), self._lib)
+        else:
+            self._launch()
+        for w, t in zip(written, outputs):
+            if w is not t:
+                t.copy_(w, non_blocking=True)
+
     def __call__(self, *inputs):
+        if self._caller is not None:
+            return self._call_lib.run(self._caller, *inputs)
         inputs = self._prepare(inputs)
         with torch.cuda.device(self.device):
             for static, t in zip(self.static_inputs, inputs):
@@ -327,6 +377,7 @@ class GPUExecutable:
         return list(by_kernel.items())
 
     def close(self):
+        self._caller = None
         if getattr(self, "_plan", None) is not None and self._plan:
             self._lib.kb200_plan_destroy(self._plan)
             self._plan = C.c_void_p()
@@ -379,9 +430,10 @@ class StreamedBatch:
         for i, (src, dst) in enumerate(zip(sources, sinks)):
             exe = self.executables[i % n]
             with torch.cuda.stream(self.streams[i % n]):
-                exe.static_inputs[0].copy_(src, non_blocking=True)
                 if kernels:
-                    exe.run_static()
+                    exe.run_on([src], [dst])        # device tensors without a copy, pinned host tensors through the static buffers
+                    continue
+                exe.static_inputs[0].copy_(src, non_blocking=True)
                 dst.copy_(exe.static_outputs[0], non_blocking=True)
         for st in self.streams:
             cur.wait_stream(st)

@@ -1,0 +1,48 @@
+"""A call reads its inputs and writes its results where they are: whatever form an input comes in, the
+same bits, in fresh tensors."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("case", ["linear_1x3072x768", "layernorm_2048x768", "mlp_2048", "gpt2_block_t128", "block_d64"])
+def test_every_form_of_input_gives_the_same_results(case, precision):
+    from gpu_helpers import build_executable
+    from helpers import case_data, load_plan
+
+    plan = load_plan(case)
+    (x,), consts, _ = case_data(case, plan)
+    exe = build_executable(case, precision, plan_json=plan, consts=consts)
+    x = torch.from_numpy(np.ascontiguousarray(x))
+    exe.static_inputs[0].copy_(x)
+    exe.run_static()
+    want = exe.static_outputs[0].clone()
+    dense = x.cuda()
+    unaligned = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape).copy_(x)
+    strided = torch.empty(x.shape[::-1], device="cuda").t().copy_(x)
+    held = []
+    for form in (dense, x, unaligned, strided, x.double(), dense.clone(), dense):
+        before = form.clone()
+        held.append(exe(form)[0])
+        assert torch.equal(form, before)
+    exe.run_static()                       # the fixed buffers again, after calls on others
+    held.append(exe.static_outputs[0])
+    sink = torch.empty_like(want)
+    exe.run_on([dense], [sink])
+    in_place = dense.clone()
+    if in_place.shape == want.shape:
+        exe.run_on([in_place], [in_place])
+        held.append(in_place)
+    torch.cuda.synchronize()
+    exe.status()
+    for got in held + [sink]:
+        assert torch.equal(got, want)
+    assert len({t.data_ptr() for t in held}) == len(held)
+    with pytest.raises(ValueError):
+        exe(dense[:, :-1])
+    with pytest.raises(TypeError):
+        exe(dense, dense)
