@@ -5,6 +5,7 @@
 //   ew_chain_vec4   the tape is a chain and every operand is contiguous (or constant) along the
 //                   innermost dim: 128-bit loads/stores, the running value stays in registers.
 //                   HBM-bound: reads each input once, writes the output once.
+//   ew_chain        the same with one element per access, for widths and alignments 128 bits cannot take.
 //   ew_transpose    a chain whose first input is contiguous along a different dim than the output
 //                   (head-split K^T copy, unfrozen weight transposes): 32x32 tiles through shared
 //                   memory so both the read and the write are coalesced.
@@ -52,11 +53,15 @@ __global__ void __launch_bounds__(256) ew_generic_kernel(const __grid_constant__
 constexpr int kVecRank = 4;
 
 struct EwChainParams {
-  uint32_t nvec;
-  uint32_t shape[kVecRank];      // last entry = inner / 4
+  uint32_t nvec;                 // accesses in all: elements / VEC
+  uint32_t shape[kVecRank];      // last entry = inner / VEC
+  // Quotients by shape[d] through a multiplication: x / d = x * ceil(2^(31 + s) / d) >> (31 + s) with
+  // 2^s >= d, exact for x < 2^31.
+  uint32_t magic[kVecRank];
+  int shift[kVecRank];
   float* ptr[KB200_MAX_OPERANDS];
   // element strides as 32-bit numbers (the host takes this kernel only when every offset fits),
-  // the innermost one already multiplied by 4: 4 (a float4 per index) or 0 (one scalar per row)
+  // the innermost one already multiplied by VEC: VEC (an access per index) or 0 (one scalar per row)
   int32_t stride[KB200_MAX_OPERANDS][kVecRank];
   Chain chain;
 };
@@ -69,28 +74,32 @@ __device__ __forceinline__ uint32_t ew_offset(const EwChainParams& p, int slot, 
   return off;
 }
 
-template <int RANK>
-__device__ __forceinline__ float4 ew_load4(const EwChainParams& p, int slot, const uint32_t* idx) {
+template <int RANK, int VEC>
+__device__ __forceinline__ void ew_load(const EwChainParams& p, int slot, const uint32_t* idx, float* v) {
   const float* ptr = p.ptr[slot] + ew_offset<RANK>(p, slot, idx);
-  if (p.stride[slot][RANK - 1] == 0) {
-    float s = __ldg(ptr);
-    return make_float4(s, s, s, s);
+  if (VEC == 1) {
+    *v = *ptr;
+  } else if (p.stride[slot][RANK - 1] == 0) {
+    v[0] = v[1] = v[2] = v[3] = __ldg(ptr);
+  } else {
+    const float4 x = *reinterpret_cast<const float4*>(ptr);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
   }
-  return *reinterpret_cast<const float4*>(ptr);
 }
 
-// U float4 per thread, a block's vectors contiguous per u (coalesced).  The rank is a template
-// parameter and all index arithmetic is 32-bit: at 8 bytes moved per element the kernel must stay
-// far below the instruction budget of the memory system (a generic 64-bit version of the same loop
-// spent 75 instructions per element and ran at a third of the copy bandwidth).
-template <int RANK, int U>
-__global__ void __launch_bounds__(256) ew_chain_vec4_kernel(const __grid_constant__ EwChainParams p) {
+// U accesses of VEC elements per thread, a block's accesses contiguous per u (coalesced).  The rank is a
+// template parameter and all index arithmetic is 32-bit, its divisions multiplications: at 8 bytes moved
+// per element the kernel must stay far below the instruction budget of the memory system (a generic
+// 64-bit version of the same loop spent 75 instructions per element and ran at a third of the copy
+// bandwidth).  Single elements take eight accesses per thread, for as many bytes in flight.
+template <int RANK, int U, int VEC>
+__global__ void __launch_bounds__(256) ew_chain_kernel(const __grid_constant__ EwChainParams p) {
   pdl_wait();                 // the producer of this kernel's inputs has completed
   pdl_launch_dependents();    // the next kernel may begin its start-up
   const uint32_t nvec = p.nvec;
   const uint32_t step = gridDim.x * blockDim.x * U;
   for (uint32_t base = blockIdx.x * blockDim.x * U + threadIdx.x; base < nvec; base += step) {
-    float v[4 * U];
+    float v[VEC * U];
     uint32_t idx[U][RANK];
     bool live[U];
 #pragma unroll
@@ -100,30 +109,33 @@ __global__ void __launch_bounds__(256) ew_chain_vec4_kernel(const __grid_constan
       uint32_t rest = live[u] ? i : 0;
 #pragma unroll
       for (int d = RANK - 1; d > 0; --d) {
-        const uint32_t q = rest / p.shape[d];
+        const uint32_t q = (uint32_t)(((uint64_t)rest * p.magic[d]) >> p.shift[d]);
         idx[u][d] = rest - q * p.shape[d];
         rest = q;
       }
       idx[u][0] = rest;
-      const float4 x = live[u] ? ew_load4<RANK>(p, p.chain.first_slot, idx[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[4 * u] = x.x; v[4 * u + 1] = x.y; v[4 * u + 2] = x.z; v[4 * u + 3] = x.w;
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[VEC * u + e] = 0.0f;
+      if (live[u]) ew_load<RANK, VEC>(p, p.chain.first_slot, idx[u], v + VEC * u);
     }
     for (int s = 0; s < p.chain.n; ++s) {
       const ChainStep st = p.chain.steps[s];
-      float side[4 * U];
+      float side[VEC * U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        float4 x = make_float4(st.imm, st.imm, st.imm, st.imm);
-        if (st.slot >= 0 && live[u]) x = ew_load4<RANK>(p, st.slot, idx[u]);
-        side[4 * u] = x.x; side[4 * u + 1] = x.y; side[4 * u + 2] = x.z; side[4 * u + 3] = x.w;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) side[VEC * u + e] = st.imm;
+        if (st.slot >= 0 && live[u]) ew_load<RANK, VEC>(p, st.slot, idx[u], side + VEC * u);
       }
-      chain_step<4 * U>(st.op, v, side);
+      chain_step<VEC * U>(st.op, v, side);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (live[u])
-        *reinterpret_cast<float4*>(p.ptr[p.chain.out_slot] + ew_offset<RANK>(p, p.chain.out_slot, idx[u])) =
-            make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+    for (int u = 0; u < U; ++u) {
+      if (!live[u]) continue;
+      float* out = p.ptr[p.chain.out_slot] + ew_offset<RANK>(p, p.chain.out_slot, idx[u]);
+      if (VEC == 1) *out = v[u];
+      else *reinterpret_cast<float4*>(out) = make_float4(v[VEC * u], v[VEC * u + 1], v[VEC * u + 2], v[VEC * u + VEC - 1]);
+    }
   }
 }
 
@@ -224,30 +236,28 @@ int choose_elementwise(Plan& plan, PlanKernel& k) {
   if (!chain_slots(k.chain, slots, &n_slots)) return KB200_OK;
   const int last = d.iter_rank - 1;
   const int64_t inner = d.iter_shape[last];
-  // vec4: every operand contiguous or constant along the innermost dim, everything 16-byte aligned
-  bool vec = inner % 4 == 0 && numel_of(d) / 4 < (int64_t(1) << 31);   // the kernel's indices are 32-bit
-  for (int i = 0; i < n_slots && vec; ++i) {
+  // a chain of accesses along the innermost dim: every operand contiguous or constant there, every
+  // element offset (and stride) within the kernel's 32-bit arithmetic; float4 accesses where width,
+  // strides and bases allow, else single elements
+  bool chain = numel_of(d) < (int64_t(1) << 31), vec = inner % 4 == 0;
+  for (int i = 0; i < n_slots && chain; ++i) {
     const DevOperand& o = k.ops[slots[i]];
     const bool is_out = slots[i] == k.chain.out_slot;
-    // every element offset (and stride) of the operand fits the kernel's 32-bit arithmetic
     int64_t span = 0;
-    for (int dd = 0; dd <= last && vec; ++dd) {
-      if (o.stride[dd] < 0) vec = false;
+    for (int dd = 0; dd <= last && chain; ++dd) {
+      if (o.stride[dd] < 0) chain = false;
       span += (d.iter_shape[dd] - 1) * o.stride[dd];
     }
-    if (span >= (int64_t(1) << 31)) vec = false;
-    if (!vec) break;
+    if (span >= (int64_t(1) << 31)) chain = false;
     if (o.stride[last] == 1) {
-      vec = (reinterpret_cast<uintptr_t>(o.ptr) & 15) == 0;
+      vec = vec && (reinterpret_cast<uintptr_t>(o.ptr) & 15) == 0;
       for (int dd = 0; dd < last && vec; ++dd) vec = o.stride[dd] % 4 == 0;
-    } else if (o.stride[last] == 0 && !is_out) {
-      // scalar along the row: fine
-    } else {
-      vec = false;
+    } else if (o.stride[last] != 0 || is_out) {
+      chain = false;         // (an operand that is constant along the row is fine)
     }
   }
-  if (vec) {
-    k.impl = IMPL_EW_CHAIN_VEC4;
+  if (chain) {
+    k.impl = vec ? IMPL_EW_CHAIN_VEC4 : IMPL_EW_CHAIN;
     return KB200_OK;
   }
   // transpose: output contiguous along the last dim, first input contiguous along another one
@@ -265,32 +275,45 @@ int choose_elementwise(Plan& plan, PlanKernel& k) {
   return KB200_OK;
 }
 
+template <int U, int VEC>
+static void launch_chain(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
+  const kb200_kernel_desc& d = k.desc;
+  EwChainParams p{};
+  const int rank = d.iter_rank;
+  for (int i = 0; i < rank; ++i) {
+    p.shape[i] = (uint32_t)d.iter_shape[i];
+    if (i == rank - 1) p.shape[i] /= VEC;
+    int log = 0;
+    while ((uint64_t(1) << log) < p.shape[i]) ++log;
+    p.shift[i] = 31 + log;
+    p.magic[i] = (uint32_t)(((uint64_t(1) << p.shift[i]) + p.shape[i] - 1) / p.shape[i]);
+  }
+  p.nvec = (uint32_t)(numel_of(d) / VEC);
+  for (int o = 0; o < d.n_operands; ++o) {
+    p.ptr[o] = k.ops[o].ptr;
+    for (int i = 0; i < rank; ++i) p.stride[o][i] = (int32_t)(k.ops[o].stride[i] * (i == rank - 1 ? VEC : 1));
+  }
+  p.chain = k.chain;
+  int64_t blocks = ((int64_t)p.nvec + 256 * U - 1) / (256 * U);
+  // beyond the cap every block takes the same number of grid-stride steps (no ragged last wave)
+  const int64_t cap = (int64_t)plan.sm_count * 64;
+  const int64_t steps = (blocks + cap - 1) / cap;
+  const unsigned grid = (unsigned)((blocks + steps - 1) / (steps > 0 ? steps : 1));
+  switch (rank) {
+    case 1: launch_kernel(plan.pdl, ew_chain_kernel<1, U, VEC>, dim3(grid), dim3(256), 0, s, p); break;
+    case 2: launch_kernel(plan.pdl, ew_chain_kernel<2, U, VEC>, dim3(grid), dim3(256), 0, s, p); break;
+    case 3: launch_kernel(plan.pdl, ew_chain_kernel<3, U, VEC>, dim3(grid), dim3(256), 0, s, p); break;
+    default: launch_kernel(plan.pdl, ew_chain_kernel<4, U, VEC>, dim3(grid), dim3(256), 0, s, p); break;
+  }
+}
+
 int launch_elementwise(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   const kb200_kernel_desc& d = k.desc;
   const int64_t numel = numel_of(d);
   if (k.impl == IMPL_EW_CHAIN_VEC4) {
-    EwChainParams p{};
-    const int rank = d.iter_rank;
-    for (int i = 0; i < rank; ++i) p.shape[i] = (uint32_t)d.iter_shape[i];
-    p.shape[rank - 1] /= 4;
-    p.nvec = (uint32_t)(numel / 4);
-    for (int o = 0; o < d.n_operands; ++o) {
-      p.ptr[o] = k.ops[o].ptr;
-      for (int i = 0; i < rank; ++i) p.stride[o][i] = (int32_t)(k.ops[o].stride[i] * (i == rank - 1 ? 4 : 1));
-    }
-    p.chain = k.chain;
-    constexpr int U = 2;
-    int64_t blocks = ((int64_t)p.nvec + 256 * U - 1) / (256 * U);
-    // beyond the cap every block takes the same number of grid-stride steps (no ragged last wave)
-    const int64_t cap = (int64_t)plan.sm_count * 64;
-    const int64_t steps = (blocks + cap - 1) / cap;
-    const unsigned grid = (unsigned)((blocks + steps - 1) / (steps > 0 ? steps : 1));
-    switch (rank) {
-      case 1: launch_kernel(plan.pdl, ew_chain_vec4_kernel<1, U>, dim3(grid), dim3(256), 0, s, p); break;
-      case 2: launch_kernel(plan.pdl, ew_chain_vec4_kernel<2, U>, dim3(grid), dim3(256), 0, s, p); break;
-      case 3: launch_kernel(plan.pdl, ew_chain_vec4_kernel<3, U>, dim3(grid), dim3(256), 0, s, p); break;
-      default: launch_kernel(plan.pdl, ew_chain_vec4_kernel<4, U>, dim3(grid), dim3(256), 0, s, p); break;
-    }
+    launch_chain<2, 4>(plan, k, s);
+  } else if (k.impl == IMPL_EW_CHAIN) {
+    launch_chain<8, 1>(plan, k, s);
   } else if (k.impl == IMPL_EW_TRANSPOSE) {
     EwTransposeParams p{};
     p.rank = d.iter_rank;

@@ -57,6 +57,7 @@ struct Chain {
 enum Impl : int {
   IMPL_EW_GENERIC = 0,
   IMPL_EW_CHAIN_VEC4,
+  IMPL_EW_CHAIN,
   IMPL_EW_TRANSPOSE,
   IMPL_ROW_GENERIC,
   IMPL_ROW_LAYERNORM,
@@ -86,6 +87,7 @@ struct PlanKernel {
   // ... whose input may be a short elementwise chain on the loaded row (x * scale + mask before a
   // softmax, a + b before a LayerNorm), and that value may itself be an output of the kernel
   Chain row_pre;          // steps applied to x_slot's row before the reductions (n == 0: none)
+  bool row_vec = false;   // 128-bit accesses (width, strides and bases of every tensor allow them)
   int pre_out_slot = -1;  // operand that receives the chain's value, or -1
   // matmul
   int64_t batch = 1, M = 0, N = 0, K = 0;

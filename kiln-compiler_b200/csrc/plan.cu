@@ -29,7 +29,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 const char* impl_name(int impl) {
   static const char* names[IMPL_COUNT] = {
-      "ew_generic", "ew_chain_vec4", "ew_transpose", "row_generic", "row_layernorm", "row_softmax",
+      "ew_generic", "ew_chain_vec4", "ew_chain", "ew_transpose", "row_generic", "row_layernorm", "row_softmax",
       "reduce_generic", "mm_simt_fp32", "mm_gemv", "mm_tcgen05", "attention_fused", "fused_away"};
   return impl >= 0 && impl < IMPL_COUNT ? names[impl] : "?";
 }
@@ -1195,7 +1195,7 @@ KB200_EXPORT int kb200_kernel_chain_length(const kb200_plan* p, int i) {
   if (i < 0 || i >= (int)plan.kernels.size() || !plan.bound) return -1;
   const PlanKernel& k = plan.kernels[i];
   switch (k.impl) {
-    case IMPL_MM_TC: case IMPL_MM_GEMV: case IMPL_MM_SIMT: case IMPL_EW_CHAIN_VEC4: case IMPL_EW_TRANSPOSE:
+    case IMPL_MM_TC: case IMPL_MM_GEMV: case IMPL_MM_SIMT: case IMPL_EW_CHAIN_VEC4: case IMPL_EW_CHAIN: case IMPL_EW_TRANSPOSE:
       return k.has_chain ? k.chain.n : 0;
     case IMPL_ROW_LAYERNORM: case IMPL_ROW_SOFTMAX: return k.row_pre.n;
     default: return 0;

@@ -6,9 +6,9 @@
 //                  the elementwise values recomputed from the inputs in every pass -- the scheme of
 //                  the reference's chunked rows (codegen.py:371-428), so memory use is constant for
 //                  any row length.
-//   row_layernorm  two-pass mean / variance LayerNorm with affine, one warp per row, the row held
-//   row_softmax    in registers (128-bit loads, shuffle reductions): one read and one write of
-//                  the tensor, HBM-bound.
+//   row_layernorm  two-pass mean / variance LayerNorm with affine, one to 32 warps per row, the row
+//   row_softmax    held in registers (128-bit loads where width and alignment allow, shuffle
+//                  reductions): one read and one write of the tensor, HBM-bound.
 #include <cuda_bf16.h>
 
 #include "device_math.cuh"
@@ -141,24 +141,68 @@ struct RowFastParams {
 
 enum { ROW_LAYERNORM = 0, ROW_SOFTMAX = 1 };
 
-// One warp per row; lane l owns float4 number l + 32 * i, i < VPL.
-template <int MODE, int VPL>
-__global__ void __launch_bounds__(256) row_warp_kernel(const __grid_constant__ RowFastParams p) {
-  const int lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  const int64_t row = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5);
-  const int nvec = p.inner >> 2;
+// VEC consecutive floats as one access.
+template <int VEC>
+__device__ __forceinline__ void row_load(float (&v)[VEC], const float* p) {
+  if (VEC == 1) {
+    v[0] = *p;
+  } else {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[VEC - 1] = t.w;
+  }
+}
+template <int VEC>
+__device__ __forceinline__ void row_store(float* p, const float (&v)[VEC]) {
+  if (VEC == 1) *p = v[0];
+  else *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[VEC - 1]);
+}
+template <int VEC>
+__device__ __forceinline__ float row_fold(const float (&v)[VEC]) { return VEC == 1 ? v[0] : (v[0] + v[1]) + (v[2] + v[VEC - 1]); }
+
+// N accesses of VEC floats per lane; the lanes of a row's warps take consecutive accesses, lane by
+// lane.  WIDE: the block's warps share one row (their partial reductions meet in shared memory), else
+// every warp has a row of its own.
+//
+// What bounds it is the memory system, so a row is read once and written once, all of its loads in flight
+// together.  A row that does not fit one warp's registers gets more warps instead of a second pass,
+// and a row that 128-bit accesses cannot take (an odd width puts every row on another alignment)
+// keeps the scheme with single floats: a warp still moves whole 128-byte lines.  LayerNorm 2048 x
+// 8192 and rows of odd width used to run on the tape interpreter above (1238 x 6944: 789 us,
+// now 16).  PRE: a chain in front of the reductions; its
+// switch over the scalar ops, unrolled over a lane's elements, costs a softmax of 512 columns 54
+// registers instead of 32.
+template <int MODE, int VEC, int N, bool WIDE, bool PRE>
+__global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_constant__ RowFastParams p) {
+  const int lane = WIDE ? threadIdx.x : (threadIdx.x & 31);
+  const int lanes = WIDE ? blockDim.x : 32;
+  const int64_t row = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int units = VEC == 1 ? p.inner : p.inner >> 2;
+  __shared__ float partial[WIDE ? 64 : 1];
+  // Each reduction of a WIDE row has its own half of `partial`: no barrier between the reads of one and the writes of the next.
+  auto across = [&](float v, bool is_max, int which) {
+    v = is_max ? warp_max(v) : warp_sum(v);
+    if (!WIDE) return v;
+    const int warps = lanes >> 5, l = threadIdx.x & 31;
+    if (l == 0) partial[32 * which + (threadIdx.x >> 5)] = v;
+    __syncthreads();
+    const float t = l < warps ? partial[32 * which + l] : (is_max ? -CUDART_INF_F : 0.0f);
+    return is_max ? warp_max(t) : warp_sum(t);
+  };
   // The affine parameters of a LayerNorm are constants of the plan, not outputs of the previous
   // kernel: they are fetched before this kernel waits for its producer, so their latency is off the
-  // path (fetched after the two reductions they added a dependent memory round trip to every row).
-  float4 g[MODE == ROW_LAYERNORM ? VPL : 1], b[MODE == ROW_LAYERNORM ? VPL : 1];
-  if (MODE == ROW_LAYERNORM) {
-    const float4* g4 = reinterpret_cast<const float4*>(p.gamma);
-    const float4* b4 = reinterpret_cast<const float4*>(p.beta);
+  // path (fetched after the two reductions they added a dependent memory round trip to every row).  The
+  // other rows of a WIDE block's SM cover that round trip, and its registers are worth more: there they
+  // are fetched where they are used.
+  constexpr bool kAhead = MODE == ROW_LAYERNORM && !WIDE;
+  float g[kAhead ? N : 1][VEC], b[kAhead ? N : 1][VEC];
+  if (kAhead) {
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int j = lane + 32 * i;
-      if (j < nvec) { g[i] = __ldg(g4 + j); b[i] = __ldg(b4 + j); }
+    for (int i = 0; i < N; ++i) {
+      const int j = lane + lanes * i;
+      if (j < units) {
+        row_load<VEC>(g[i], p.gamma + VEC * j);
+        row_load<VEC>(b[i], p.beta + VEC * j);
+      }
     }
   }
   pdl_wait();                 // the producer of this kernel's inputs has completed
@@ -166,117 +210,166 @@ __global__ void __launch_bounds__(256) row_warp_kernel(const __grid_constant__ R
   if (row >= p.n_rows) return;
   int64_t i0 = row, i1 = 0;
   if (p.rows_inner > 0) { i0 = row / p.rows_inner; i1 = row - i0 * p.rows_inner; }
-  const float4* x4 = reinterpret_cast<const float4*>(p.x + i0 * p.x_row_stride + i1 * p.x_stride1);
-  float4* o4 = reinterpret_cast<float4*>(p.out + i0 * p.out_row_stride + i1 * p.out_stride1);
-  const int64_t out16_off = i0 * p.out_row_stride + i1 * p.out_stride1;
-  float4 v[VPL];
-  bool live[VPL];
+  const float* x = p.x + i0 * p.x_row_stride + i1 * p.x_stride1;
+  const int64_t out_off = i0 * p.out_row_stride + i1 * p.out_stride1;
+  float* out = p.out + out_off;
+  float v[N][VEC];
+  bool live[N];
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const int j = lane + 32 * i;
-    live[i] = j < nvec;
-    if (live[i]) v[i] = x4[j];
+  for (int i = 0; i < N; ++i) {
+    const int j = lane + lanes * i;
+    live[i] = j < units;
+    if (live[i]) row_load<VEC>(v[i], x + VEC * j);
   }
-  for (int s = 0; s < p.n_pre; ++s) {
+  for (int s = 0; PRE && s < p.n_pre; ++s) {
     const RowFastParams::Pre st = p.pre[s];
     const float* side = st.kind == 2 ? st.ptr + i0 * st.stride0 + i1 * st.stride1 : nullptr;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
+    for (int i = 0; i < N; ++i) {
       if (!live[i]) continue;
-      float4 t = make_float4(st.imm, st.imm, st.imm, st.imm);
+      float t[VEC];
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) t[e] = st.imm;
       if (st.kind == 2) {
-        if (st.inner_stride == 1) t = *reinterpret_cast<const float4*>(side + 4 * (lane + 32 * i));
-        else { const float one = __ldg(side); t = make_float4(one, one, one, one); }
+        if (st.inner_stride == 1) {
+          row_load<VEC>(t, side + VEC * (lane + lanes * i));
+        } else {
+          const float one = __ldg(side);
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) t[e] = one;
+        }
       }
-      v[i].x = apply_chain(st.op, v[i].x, t.x);
-      v[i].y = apply_chain(st.op, v[i].y, t.y);
-      v[i].z = apply_chain(st.op, v[i].z, t.z);
-      v[i].w = apply_chain(st.op, v[i].w, t.w);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[i][e] = apply_chain(st.op, v[i][e], t[e]);
     }
   }
-  if (p.pre_out != nullptr) {
-    float4* z4 = reinterpret_cast<float4*>(p.pre_out + i0 * p.pre_out_stride0 + i1 * p.pre_out_stride1);
+  if (PRE && p.pre_out != nullptr) {
+    float* z = p.pre_out + i0 * p.pre_out_stride0 + i1 * p.pre_out_stride1;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i)
-      if (live[i]) z4[lane + 32 * i] = v[i];
+    for (int i = 0; i < N; ++i)
+      if (live[i]) row_store<VEC>(z + VEC * (lane + lanes * i), v[i]);
   }
   if (MODE == ROW_LAYERNORM) {
     float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i)
-      if (live[i]) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-    const float mean = warp_sum(s) * p.inv_n;
+    for (int i = 0; i < N; ++i)
+      if (live[i]) s += row_fold<VEC>(v[i]);
+    const float mean = across(s, false, 0) * p.inv_n;
     float q = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
+    for (int i = 0; i < N; ++i) {
       if (live[i]) {
-        v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
-        q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+        float sq[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          v[i][e] -= mean;
+          sq[e] = v[i][e] * v[i][e];
+        }
+        q += row_fold<VEC>(sq);
       }
     }
-    const float rstd = 1.0f / sqrtf(warp_sum(q) * p.inv_n + p.eps);
+    const float rstd = 1.0f / sqrtf(across(q, false, 1) * p.inv_n + p.eps);
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
+    for (int i = 0; i < N; ++i) {
       if (live[i]) {
-        const int j = lane + 32 * i;
-        float4 y;
-        y.x = v[i].x * rstd * g[i].x + b[i].x;
-        y.y = v[i].y * rstd * g[i].y + b[i].y;
-        y.z = v[i].z * rstd * g[i].z + b[i].z;
-        y.w = v[i].w * rstd * g[i].w + b[i].w;
-        if (p.store32) o4[j] = y;
+        const int j = lane + lanes * i;
+        float y[VEC];
+        const int at = kAhead ? i : 0;
+        if (!kAhead) {
+          row_load<VEC>(g[0], p.gamma + VEC * j);
+          row_load<VEC>(b[0], p.beta + VEC * j);
+        }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) y[e] = v[i][e] * rstd * g[at][e] + b[at][e];
+        if (p.store32) row_store<VEC>(out + VEC * j, y);
         if (p.out16 != nullptr) {
-          __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-          uint2 packed;
-          packed.x = *reinterpret_cast<uint32_t*>(&lo);
-          packed.y = *reinterpret_cast<uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(p.out16 + out16_off + 4 * j) = packed;
+          if (VEC == 1) {
+            p.out16[out_off + j] = __float2bfloat16_rn(y[0]);
+          } else {
+            __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[VEC > 1 ? 1 : 0]), hi = __floats2bfloat162_rn(y[VEC > 1 ? 2 : 0], y[VEC - 1]);
+            uint2 packed;
+            packed.x = *reinterpret_cast<uint32_t*>(&lo);
+            packed.y = *reinterpret_cast<uint32_t*>(&hi);
+            *reinterpret_cast<uint2*>(p.out16 + out_off + 4 * j) = packed;
+          }
         }
       }
     }
   } else {
     float m = -CUDART_INF_F;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i)
-      if (live[i]) m = fmaxf(m, fmaxf(fmaxf(v[i].x, v[i].y), fmaxf(v[i].z, v[i].w)));
-    m = warp_max(m);
+    for (int i = 0; i < N; ++i)
+      if (live[i])
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) m = fmaxf(m, v[i][e]);
+    m = across(m, true, 0);
     float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
+    for (int i = 0; i < N; ++i) {
       if (live[i]) {
-        // exp through ex2.approx (relative error 2^-22, what the reference's tl.exp lowers to as well)
-        v[i].x = __expf(v[i].x - m); v[i].y = __expf(v[i].y - m); v[i].z = __expf(v[i].z - m); v[i].w = __expf(v[i].w - m);
-        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        // one warp and 128-bit accesses: exp through ex2.approx (relative error 2^-22, what the reference's
+        // tl.exp lowers to as well); the forms that took over from the tape interpreter keep its expf
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) v[i][e] = VEC == 1 || WIDE ? expf(v[i][e] - m) : __expf(v[i][e] - m);
+        s += row_fold<VEC>(v[i]);
       }
     }
-    s = warp_sum(s);
+    s = across(s, false, 1);
     const float inv = 1.0f / s;     // one IEEE division per row; the elements are scaled by it (within an ulp of dividing)
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
+    for (int i = 0; i < N; ++i) {
       if (live[i]) {
-        float4 y;
-        y.x = v[i].x * inv; y.y = v[i].y * inv; y.z = v[i].z * inv; y.w = v[i].w * inv;
-        o4[lane + 32 * i] = y;
+        float y[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) y[e] = v[i][e] * inv;
+        row_store<VEC>(out + VEC * (lane + lanes * i), y);
       }
     }
   }
 }
 
-template <int MODE>
-static void launch_row_warp(const RowFastParams& p, int sm_count, bool pdl, cudaStream_t s) {
-  const int vpl = (p.inner / 4 + 31) / 32;
-  int warps = p.n_rows >= (int64_t)sm_count * 16 ? 8 : (p.n_rows >= (int64_t)sm_count * 4 ? 4 : 1);
-  const unsigned grid = (unsigned)((p.n_rows + warps - 1) / warps);
-  const unsigned block = warps * 32;
-#define KB200_ROW_CASE(V) launch_kernel(pdl, row_warp_kernel<MODE, V>, dim3(grid), dim3(block), 0, s, p)
-  if (vpl <= 1) KB200_ROW_CASE(1);
-  else if (vpl <= 2) KB200_ROW_CASE(2);
-  else if (vpl <= 4) KB200_ROW_CASE(4);
-  else if (vpl <= 6) KB200_ROW_CASE(6);
-  else if (vpl <= 8) KB200_ROW_CASE(8);
-  else if (vpl <= 12) KB200_ROW_CASE(12);
-  else KB200_ROW_CASE(16);
+// The widest row: 16 warps (more would halve the registers of a thread) of 8 float4 or 32 floats a lane.
+constexpr int64_t kRowLimit = 512 * 32;
+
+template <int MODE, bool PRE>
+static void launch_rows(const RowFastParams& p, bool vec, int sm_count, bool pdl, cudaStream_t s) {
+  const int units = vec ? p.inner / 4 : p.inner;
+  const int n = (units + 31) / 32;                  // accesses per lane if one warp takes the row
+#define KB200_ROW_CASE(VEC, N, WIDE) launch_kernel(pdl, row_kernel<MODE, VEC, N, WIDE, PRE>, dim3(grid), dim3(block), 0, s, p)
+  if (n <= (vec && MODE == ROW_LAYERNORM ? 6 : 8)) {
+    // a warp per row; few rows spread over more blocks.  (A LayerNorm of 8 float4 a lane, or either of 12,
+    // spills; four warps of a quarter each do not.)
+    const int warps = p.n_rows >= (int64_t)sm_count * 16 ? 8 : (p.n_rows >= (int64_t)sm_count * 4 ? 4 : 1);
+    const unsigned grid = (unsigned)((p.n_rows + warps - 1) / warps), block = warps * 32;
+    if (vec) {
+      if (n <= 1) KB200_ROW_CASE(4, 1, false);
+      else if (n <= 2) KB200_ROW_CASE(4, 2, false);
+      else if (n <= 4) KB200_ROW_CASE(4, 4, false);
+      else if (n <= 6) KB200_ROW_CASE(4, 6, false);
+      else if constexpr (MODE == ROW_SOFTMAX) KB200_ROW_CASE(4, 8, false);
+    } else {
+      if (n <= 2) KB200_ROW_CASE(1, 2, false);
+      else if (n <= 4) KB200_ROW_CASE(1, 4, false);
+      else KB200_ROW_CASE(1, 8, false);
+    }
+    return;
+  }
+  // a block per row, of as many warps (up to 16) as 4 float4 or 8 floats a lane leave
+  int per = vec ? 4 : 8;
+  while (per * 16 < n) per *= 2;
+  const unsigned grid = (unsigned)p.n_rows, block = (unsigned)((n + per - 1) / per) * 32;
+  if (vec && per == 4) KB200_ROW_CASE(4, 4, true);
+  else if (vec) KB200_ROW_CASE(4, 8, true);
+  else if (per == 8) KB200_ROW_CASE(1, 8, true);
+  else if (per == 16) KB200_ROW_CASE(1, 16, true);
+  else KB200_ROW_CASE(1, 32, true);
 #undef KB200_ROW_CASE
+}
+
+template <int MODE>
+static void launch_row_fast(const RowFastParams& p, bool vec, int sm_count, bool pdl, cudaStream_t s) {
+  if (p.n_pre > 0 || p.pre_out != nullptr) launch_rows<MODE, true>(p, vec, sm_count, pdl, s);
+  else launch_rows<MODE, false>(p, vec, sm_count, pdl, s);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -298,32 +391,27 @@ int choose_row(Plan& plan, PlanKernel& k) {
       return fail(KB200_ERR_UNSUPPORTED, "row kernel %s: more than %d reductions at one level of the chain", d.name, kMaxRowRed);
   }
   const int64_t inner = d.iter_shape[d.iter_rank - 1];
-  // register-resident rows: one or two row dims, rows of 4..2048 floats in 128-bit units
+  // register-resident rows: one or two row dims, every tensor contiguous (or one value per row) along the
+  // innermost; 128-bit accesses where all of width, strides and bases allow them
   const int last = d.iter_rank - 1;
-  const bool shape_ok = (d.iter_rank == 2 || d.iter_rank == 3) && inner % 4 == 0 && inner <= 2048 && inner >= 4;
-  if (!shape_ok) return KB200_OK;
+  if ((d.iter_rank != 2 && d.iter_rank != 3) || inner < 1 || inner > kRowLimit) return KB200_OK;
+  bool vec = inner % 4 == 0;
   auto row_tensor_ok = [&](int slot) {
     const DevOperand& o = k.ops[slot];
-    if (o.stride[last] != 1 || !aligned16(o.ptr)) return false;
-    for (int dd = 0; dd < last; ++dd)
-      if (o.stride[dd] % 4) return false;
-    return true;
+    vec = vec && aligned16(o.ptr);
+    for (int dd = 0; dd < last; ++dd) vec = vec && o.stride[dd] % 4 == 0;
+    return o.stride[last] == 1 || inner == 1;
   };
   auto vector_ok = [&](int slot) {
-    const DevOperand& o = k.ops[slot];
-    if (o.stride[last] != 1 || !aligned16(o.ptr)) return false;
     for (int dd = 0; dd < last; ++dd)
-      if (o.stride[dd] != 0) return false;
-    return true;
+      if (k.ops[slot].stride[dd] != 0) return false;
+    return row_tensor_ok(slot);
   };
   // operands of the chain in front of the reductions: a tensor like x, or one value per row
   auto pre_ok = [&]() {
     for (int st = 0; st < k.row_pre.n; ++st) {
       const int slot = k.row_pre.steps[st].slot;
-      if (slot < 0) continue;
-      const DevOperand& o = k.ops[slot];
-      if (o.stride[last] == 0) continue;
-      if (!row_tensor_ok(slot)) return false;
+      if (slot >= 0 && k.ops[slot].stride[last] != 0 && !row_tensor_ok(slot)) return false;
     }
     return k.pre_out_slot < 0 || row_tensor_ok(k.pre_out_slot);
   };
@@ -335,6 +423,7 @@ int choose_row(Plan& plan, PlanKernel& k) {
   } else if (match_softmax(d, &k)) {
     if (row_tensor_ok(k.x_slot) && row_tensor_ok(k.out_slot) && pre_ok()) k.impl = IMPL_ROW_SOFTMAX;
   }
+  k.row_vec = vec;
   return KB200_OK;
 }
 
@@ -381,9 +470,9 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
       p.eps = k.ln_eps;
       p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
       p.store32 = (k.mirror_only && p.out16 != nullptr) ? 0 : 1;
-      launch_row_warp<ROW_LAYERNORM>(p, plan.sm_count, plan.pdl, s);
+      launch_row_fast<ROW_LAYERNORM>(p, k.row_vec, plan.sm_count, plan.pdl, s);
     } else {
-      launch_row_warp<ROW_SOFTMAX>(p, plan.sm_count, plan.pdl, s);
+      launch_row_fast<ROW_SOFTMAX>(p, k.row_vec, plan.sm_count, plan.pdl, s);
     }
   } else {
     RowParams p{};

@@ -1,0 +1,51 @@
+"""Sizes at the edges of the kernels' tilings, for every module the performance cases describe: widths no
+vector access takes, rows longer than a warp's registers, sequences that end inside a tile.  Against
+the float64 evaluation of the plan, within the bounds of the other parity tests."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle.plan_oracle import run_plan, scale_relative_error
+
+pytestmark = pytest.mark.gpu
+
+BOUND = {"fp32": 1e-5, "tf32": 2e-3, "bf16": 2e-2}
+
+
+def check(case, impls=None, calls=1):
+    from perf import cases
+
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable
+
+    case = {"precision": "fp32", **case}
+    plan = cases._plan(case)
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(1))
+    exe = GPUExecutable(program_from_plan(plan, case["precision"]), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
+    std = case["k"] ** -0.5 if case["kind"] == "linear" else 1.0
+    for seed in range(calls):
+        x = (np.random.default_rng(2 + seed).standard_normal(plan.input_shapes[0]) * std).astype(np.float32)
+        (got,) = exe(torch.from_numpy(x).cuda())
+        torch.cuda.synchronize()
+        exe.status()
+        (want,) = run_plan(plan.to_json(), [x], consts, dtype=np.float64)
+        assert scale_relative_error(got.cpu().numpy(), want) <= BOUND[case["precision"]]
+    if impls:
+        assert set(exe.impls) == set(impls), exe.impls
+
+
+@pytest.mark.parametrize("rows", [1, 700])
+@pytest.mark.parametrize("d", [1, 3, 31, 33, 64, 127, 255, 257, 772, 1000, 1028, 2047, 2052, 4097, 8191, 8196, 16384])
+def test_rows_of_any_width(d, rows):
+    check({"kind": "layernorm", "rows": rows, "d": d}, ["row_layernorm"])
+    check({"kind": "softmax", "heads": 1, "rows": rows, "cols": d}, ["row_softmax"])
+
+
+def test_rows_beyond_the_registers():
+    check({"kind": "layernorm", "rows": 3, "d": 16388}, ["row_generic"])
+
+
+@pytest.mark.parametrize("rows,d", [(1, 5), (7, 33), (513, 1001), (65, 2050), (2047, 255)])
+def test_elementwise_chain_of_any_width(rows, d):
+    check({"kind": "bias_gelu", "rows": rows, "d": d}, ["ew_chain"])
