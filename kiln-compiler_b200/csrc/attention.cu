@@ -89,7 +89,7 @@ struct AttnF32Params {
   int64_t row_stride;        // floats between consecutive tokens of the Q / K / V views
   float* out;                // [B * T, H * 64] merged heads
   int64_t out_row_stride;
-  int T, H, B, q_tiles;      // q_tiles = T / 64
+  int T, H, B, q_tiles;      // q_tiles = ceil(T / 64)
   float scale_log2;
   // Query tiles from `split_from` on (the long causal prefixes) are worked on by two CTAs, one per half
   // of the key tiles; each leaves its unnormalised output and softmax state in `partial`, and the one
@@ -210,8 +210,9 @@ __device__ __forceinline__ float row_max32(const float (&v)[32], float m, int fi
 // half-warp only.  Online softmax in base 2 with Q pre-multiplied by scale * log2(e); causal tiles
 // above the diagonal are skipped; K / V tiles arrive through a two-deep cp.async ring.  The scores
 // never leave the SM.
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+// (`live` false: the 16 bytes are filled with zeros and nothing is read)
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
 }
 
 __global__ void __launch_bounds__(kFThreads, 2) attention_fp32_kernel(const __grid_constant__ AttnF32Params p) {
@@ -247,15 +248,19 @@ __global__ void __launch_bounds__(kFThreads, 2) attention_fp32_kernel(const __gr
     const int64_t first = (int64_t)j * kFTile;
 #pragma unroll
     for (int i = 0; i < kFRows; ++i) {
-      cp_async16(kd + (ld_r + 8 * i) * kFPitch + ld_c, kg + (first + ld_r + 8 * i) * rs + ld_c);
-      cp_async16(vd + (ld_r + 8 * i) * kHeadDim + ld_c, vg + (first + ld_r + 8 * i) * rs + ld_c);
+      // rows behind the sequence's last are zeros (masked keys; their values must be finite)
+      const bool live = first + ld_r + 8 * i < p.T;
+      const int64_t r = live ? first + ld_r + 8 * i : 0;
+      cp_async16(kd + (ld_r + 8 * i) * kFPitch + ld_c, kg + r * rs + ld_c, live);
+      cp_async16(vd + (ld_r + 8 * i) * kHeadDim + ld_c, vg + r * rs + ld_c, live);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(j_begin);
 #pragma unroll
   for (int i = 0; i < kFRows; ++i) {
-    float4 q4 = __ldg(reinterpret_cast<const float4*>(qg + (int64_t)(ld_r + 8 * i) * rs + ld_c));
+    float4 q4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (qt * kFTile + ld_r + 8 * i < p.T) q4 = __ldg(reinterpret_cast<const float4*>(qg + (int64_t)(ld_r + 8 * i) * rs + ld_c));
     q4.x *= p.scale_log2; q4.y *= p.scale_log2; q4.z *= p.scale_log2; q4.w *= p.scale_log2;
     *reinterpret_cast<float4*>(Qs + (ld_r + 8 * i) * kFPitch + ld_c) = q4;
   }
@@ -402,6 +407,7 @@ __global__ void __launch_bounds__(kFThreads, 2) attention_fp32_kernel(const __gr
   float* const og = p.out + (row0 + (int64_t)qt * kFTile) * p.out_row_stride + h * kHeadDim + 4 * tx;
 #pragma unroll
   for (int i = 0; i < kFRows; ++i) {
+    if (qt * kFTile + ty + 8 * i >= p.T) break;
     const float inv = 1.0f / l_run[i];
     *reinterpret_cast<float4*>(og + (int64_t)(ty + 8 * i) * p.out_row_stride) =
         make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
@@ -481,11 +487,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     const int w = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
     return w < n_items ? w : -1;
   };
-  struct Item { int h, q0, n_kv, row0, qt, j0, half, slot; bool split; };
+  struct Item { int h, seq, q0, n_kv, qt, j0, half, slot; bool split; };
   auto item_of = [&](int w) {
     Item it;
     it.h = w % p.H;
-    const int seq = (w / p.H) % p.B;
+    it.seq = (w / p.H) % p.B;
     const int v = w / (p.H * p.B);
     if (!SPLIT) {                                      // heaviest (longest causal prefix) first
       it.qt = p.q_tiles - 1 - v;
@@ -500,8 +506,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     const int n = it.qt + 1;                           // causal: key tiles 0..qt
     it.j0 = it.split && it.half ? n >> 1 : 0;          // this item's key tiles: j0 .. j0 + n_kv - 1
     it.n_kv = (it.split && !it.half ? n >> 1 : n) - it.j0;
-    it.slot = it.split ? (seq * p.H + it.h) * n_split + (it.qt - p.split_from) : 0;
-    it.row0 = seq * p.T;                               // this sequence's first row in Q, K, V and the output
+    it.slot = it.split ? (it.seq * p.H + it.h) * n_split + (it.qt - p.split_from) : 0;
     return it;
   };
 
@@ -567,38 +572,38 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         // the Q tile is free once every Q K^T of the previous item has been executed
         if (!mbar_wait(q_empty, (ii & 1) ^ 1, abort_ptr)) { give_up(0x13); break; }
         // EXACT, an operand buffer: the tile's two slabs, then the two slabs of its tails
-        [[maybe_unused]] auto load4 = [&](uint32_t dst, const CUtensorMap* heads, const CUtensorMap* tails, uint32_t bar, int first_row) {
+        [[maybe_unused]] auto load4 = [&](uint32_t dst, const CUtensorMap* heads, const CUtensorMap* tails, uint32_t bar, int t) {
           mbar_expect_tx(bar, kOpBytes);
-          tma_load_3d(dst, heads, bar, 0, first_row, it.h);
-          tma_load_3d(dst + kSlab, heads, bar, 32, first_row, it.h);
-          tma_load_3d(dst + kTileBytes, tails, bar, 0, first_row, it.h);
-          tma_load_3d(dst + kTileBytes + kSlab, tails, bar, 32, first_row, it.h);
+          tma_load_4d(dst, heads, bar, 0, t, it.h, it.seq);
+          tma_load_4d(dst + kSlab, heads, bar, 32, t, it.h, it.seq);
+          tma_load_4d(dst + kTileBytes, tails, bar, 0, t, it.h, it.seq);
+          tma_load_4d(dst + kTileBytes + kSlab, tails, bar, 32, t, it.h, it.seq);
         };
         if constexpr (EXACT) {
-          load4(q_smem, &map_q, &map_qt, q_full, it.row0 + it.q0);
+          load4(q_smem, &map_q, &map_qt, q_full, it.q0);
         } else {
           mbar_expect_tx(q_full, kTileBytes);
-          tma_load_3d(q_smem, &map_q, q_full, 0, it.row0 + it.q0, it.h);
-          if (!BF16) tma_load_3d(q_smem + kSlab, &map_q, q_full, 32, it.row0 + it.q0, it.h);
+          tma_load_4d(q_smem, &map_q, q_full, 0, it.q0, it.h, it.seq);
+          if (!BF16) tma_load_4d(q_smem + kSlab, &map_q, q_full, 32, it.q0, it.h, it.seq);
         }
         for (int j = 0; j < it.n_kv; ++j, ++t) {
           if constexpr (EXACT) {
             const uint32_t ph = t & 1;                   // one buffer: the phase alternates with every tile
             if (!mbar_wait(k_empty, ph ^ 1, abort_ptr)) { give_up(0x11); ok = false; break; }
-            load4(k_smem, &map_k, &map_kt, k_full, it.row0 + (it.j0 + j) * kRows);
+            load4(k_smem, &map_k, &map_kt, k_full, (it.j0 + j) * kRows);
             if (!mbar_wait(v_empty, ph ^ 1, abort_ptr)) { give_up(0x12); ok = false; break; }
-            load4(v_smem, &map_v, &map_vt, v_full, it.row0 + (it.j0 + j) * kRows);
+            load4(v_smem, &map_v, &map_vt, v_full, (it.j0 + j) * kRows);
           } else {
             const int s = t & 1;
             const uint32_t ph = (t >> 1) & 1;
             if (!mbar_wait(k_empty + 8 * s, ph ^ 1, abort_ptr)) { give_up(0x11); ok = false; break; }
             mbar_expect_tx(k_full + 8 * s, kTileBytes);
-            tma_load_3d(k_smem + s * kTileBytes, &map_k, k_full + 8 * s, 0, it.row0 + (it.j0 + j) * kRows, it.h);
-            if (!BF16) tma_load_3d(k_smem + s * kTileBytes + kSlab, &map_k, k_full + 8 * s, 32, it.row0 + (it.j0 + j) * kRows, it.h);
+            tma_load_4d(k_smem + s * kTileBytes, &map_k, k_full + 8 * s, 0, (it.j0 + j) * kRows, it.h, it.seq);
+            if (!BF16) tma_load_4d(k_smem + s * kTileBytes + kSlab, &map_k, k_full + 8 * s, 32, (it.j0 + j) * kRows, it.h, it.seq);
             if (!mbar_wait(v_empty + 8 * s, ph ^ 1, abort_ptr)) { give_up(0x12); ok = false; break; }
             mbar_expect_tx(v_full + 8 * s, kTileBytes);
-            tma_load_3d(v_smem + s * kTileBytes, &map_v, v_full + 8 * s, 0, it.row0 + (it.j0 + j) * kRows, it.h);
-            if (!BF16) tma_load_3d(v_smem + s * kTileBytes + kSlab, &map_v, v_full + 8 * s, 32, it.row0 + (it.j0 + j) * kRows, it.h);
+            tma_load_4d(v_smem + s * kTileBytes, &map_v, v_full + 8 * s, 0, (it.j0 + j) * kRows, it.h, it.seq);
+            if (!BF16) tma_load_4d(v_smem + s * kTileBytes + kSlab, &map_v, v_full + 8 * s, 32, (it.j0 + j) * kRows, it.h, it.seq);
           }
         }
       }
@@ -910,9 +915,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         for (int i = 0; i < 32; ++i) o[i] *= inv;
         if constexpr (EXACT) {
           // a lane holds 32 dims of ONE row: 128 contiguous bytes
-          float* const dst = p.out + (int64_t)(it.row0 + it.q0 + row) * p.out_row_stride + it.h * kHeadDim + group * 32;
+          float* const dst = p.out + ((int64_t)it.seq * p.T + it.q0 + row) * p.out_row_stride + it.h * kHeadDim + group * 32;
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+          for (int i = 0; i < 32; i += 4)
+            if (it.q0 + row < p.T) *reinterpret_cast<float4*>(dst + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
         } else {
           // A lane holds 32 dims of ONE row: the rows go through the warp's staging slot (128-byte rows, the
           // 16-byte unit XORed with the row against bank conflicts) and leave as bulk tensor stores.
@@ -921,10 +927,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           stage_rows(stage, stage + 4096, o, lane, p.out16 != nullptr, true);
           fence_async_smem();
           __syncwarp();
-          if (lane == 0) {
-            const int col = it.h * kHeadDim + group * 32, first_row = it.row0 + it.q0 + quad * 32;
-            tma_store_3d(&map_out, smem_u32(stage), col, first_row, 0);
-            if (p.out16 != nullptr) tma_store_3d(&map_out16, smem_u32(stage + 4096), col, first_row, 0);
+          if (lane == 0 && it.q0 + quad * 32 < p.T) {      // (the maps end at the sequence's last row)
+            const int col = it.h * kHeadDim + group * 32, first_row = it.q0 + quad * 32;
+            tma_store_3d(&map_out, smem_u32(stage), col, first_row, it.seq);
+            if (p.out16 != nullptr) tma_store_3d(&map_out16, smem_u32(stage + 4096), col, first_row, it.seq);
             tma_store_commit();
           }
         }
@@ -1044,7 +1050,8 @@ struct AttnChain {
 bool finish_fusion(Plan& plan, const AttnChain& c) {
   const int64_t T = c.T, H = c.H, B = c.B, hd = kHeadDim, rs = c.rs;
   if (!aligned16(c.q) || !aligned16(c.k) || !aligned16(c.v) || !aligned16(c.y->ptr)) return false;
-  if (B * H * (T / kRows) >= (int64_t(1) << 31)) return false;
+  const int64_t q_tiles = (T + kRows - 1) / kRows;
+  if (B * H * q_tiles >= (int64_t(1) << 31)) return false;
   // A later read that touches an intermediate is only acceptable if everything it reads was rewritten
   // after the chain (by the chain's own output Y, whose memory the planner may have taken from
   // them, or by a later kernel).
@@ -1084,7 +1091,8 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
       }
   }
 
-  // Q, K, V as [head, row, 64] views with rows b * T + t: a batch of sequences is more rows of the same map
+  // Q, K, V as [sequence, head, token, 64] views.  The token dim ends with the sequence, so the tile of
+  // its last tokens reads zeros behind them (as the stores' maps drop those rows): any length works.
   AttnState* st = new AttnState();
   st->exact = c.exact;
   // FP32 mode: the tensor-core kernel when its work items (128 queries each) fill at least a quarter
@@ -1093,13 +1101,13 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   // the plan option KB200_OPT_FP32_ATTENTION forces one of them.
   if (c.exact) {
     // (split operands turn an infinite element into a NaN tail: a plan that asked for IEEE behaviour keeps the FMA kernel)
-    st->exact_tc = !c.ieee && B * H * (T / kRows) * 4 >= plan.sm_count;
+    st->exact_tc = !c.ieee && B * H * q_tiles * 4 >= plan.sm_count;
     if (plan.fp32_attention == 1) st->exact_tc = false;
     if (plan.fp32_attention == 2) st->exact_tc = true;
   }
-  if ((!c.exact || st->exact_tc) && (!encode_map(&st->map_q, false, c.q, hd, B * T, H, rs, hd, 32, kRows, false) ||
-                                     !encode_map(&st->map_k, false, c.k, hd, B * T, H, rs, hd, 32, kRows, false) ||
-                                     !encode_map(&st->map_v, false, c.v, hd, B * T, H, rs, hd, 32, kRows, true))) {
+  if ((!c.exact || st->exact_tc) && (!encode_map_heads(&st->map_q, false, c.q, hd, T, H, B, rs, 32, kRows, false) ||
+                                     !encode_map_heads(&st->map_k, false, c.k, hd, T, H, B, rs, 32, kRows, false) ||
+                                     !encode_map_heads(&st->map_v, false, c.v, hd, T, H, B, rs, 32, kRows, true))) {
     delete st;
     return false;
   }
@@ -1113,9 +1121,9 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     st->span_lo = lo;
     st->span_n4 = span / 4;
     const bool ok = span % 4 == 0 && cudaMalloc(&st->tails, (size_t)span * sizeof(float)) == cudaSuccess &&
-                    encode_map(&st->map_qt, false, st->tails + (c.q - lo), hd, B * T, H, rs, hd, 32, kRows, false) &&
-                    encode_map(&st->map_kt, false, st->tails + (c.k - lo), hd, B * T, H, rs, hd, 32, kRows, false) &&
-                    encode_map(&st->map_vt, false, st->tails + (c.v - lo), hd, B * T, H, rs, hd, 32, kRows, true) &&
+                    encode_map_heads(&st->map_qt, false, st->tails + (c.q - lo), hd, T, H, B, rs, 32, kRows, false) &&
+                    encode_map_heads(&st->map_kt, false, st->tails + (c.k - lo), hd, T, H, B, rs, 32, kRows, false) &&
+                    encode_map_heads(&st->map_vt, false, st->tails + (c.v - lo), hd, T, H, B, rs, 32, kRows, true) &&
                     cudaFuncSetAttribute(attention_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kExactSmemBytes) == cudaSuccess &&
                     cudaFuncSetAttribute(attention_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1146,7 +1154,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   p.T = (int)T;
   p.H = (int)H;
   p.B = (int)B;
-  p.q_tiles = (int)(T / kRows);
+  p.q_tiles = (int)q_tiles;
   p.scale_log2 = c.scale * 1.4426950408889634f;
   p.out = c.y->ptr;
   p.out_row_stride = H * hd;
@@ -1170,8 +1178,8 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   p.idesc_pv = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | ((uint32_t)(kHeadDim >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
   p.kernel_index = (int)c.first;
   p.status = plan.d_status;
-  // the output rows leave by bulk tensor stores: [B * T, H * 64], boxes of 32 rows x 32 dims
-  if (!aligned16(p.out) || !encode_map_store(&st->map_out, false, p.out, H * hd, B * T, 1, p.out_row_stride, 0)) {
+  // the output rows leave by bulk tensor stores: [B][T, H * 64], boxes of 32 rows x 32 dims
+  if (!aligned16(p.out) || !encode_map_store(&st->map_out, false, p.out, H * hd, T, B, p.out_row_stride, T * H * hd)) {
     if (st->staged_out) cudaFree(st->staged_out);
     if (st->tails) cudaFree(st->tails);
     delete st;
@@ -1236,7 +1244,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     f.out = p.out;
     f.out_row_stride = p.out_row_stride;
     f.T = (int)T; f.H = (int)H; f.B = (int)B;
-    f.q_tiles = (int)(T / kFTile);
+    f.q_tiles = (int)((T + kFTile - 1) / kFTile);
     f.scale_log2 = p.scale_log2;
     // the upper half of the query tiles (the longest causal prefixes) is shared by two CTAs each
     f.split_from = f.q_tiles >= 2 ? f.q_tiles / 2 : f.q_tiles;
@@ -1282,7 +1290,7 @@ bool try_fuse_single(Plan& plan, size_t i) {
   // --- k3: scores = Q K^T * scale + mask ---
   if (k3.desc.kclass != KB200_K_MATMUL || !k3.has_chain) return false;
   const int64_t H = k3.batch, T = k3.M, hd = k3.K;
-  if (hd != kHeadDim || k3.N != T || T % kRows != 0 || T < kRows || H < 1 || H > 65535) return false;
+  if (hd != kHeadDim || k3.N != T || T < 2 || H < 1 || H > 65535) return false;
   const DevOperand& Q = k3.ops[k3.desc.a_slot];
   const DevOperand& Kt = k3.ops[k3.desc.b_slot];
   const int64_t rs = Q.stride[1];
@@ -1377,7 +1385,7 @@ bool try_fuse_batched(Plan& plan, size_t i) {
   // --- scores ---
   if (mm1.desc.kclass != KB200_K_MATMUL || !mm1.has_chain || mm1.chain.n != 0) return false;
   const int64_t BH = mm1.batch, T = mm1.M;
-  if (mm1.K != hd || mm1.N != T || T % kRows != 0 || T < kRows) return false;
+  if (mm1.K != hd || mm1.N != T || T < 2) return false;
   const DevOperand& Qc = mm1.ops[mm1.desc.a_slot];
   const DevOperand& Ktc = mm1.ops[mm1.desc.b_slot];
   const DevOperand& S = mm1.ops[mm1.chain.out_slot];
@@ -1543,12 +1551,12 @@ bool attention_use_mirror(PlanKernel& k, const float* arena_base, const void* mi
   const __nv_bfloat16* q = m + (st->q_ptr - arena_base);
   const __nv_bfloat16* kk = m + (st->k_ptr - arena_base);
   const __nv_bfloat16* v = m + (st->v_ptr - arena_base);
-  const int64_t T = (int64_t)st->params.B * st->params.T, H = st->params.H, rs = st->row_stride;   // rows of all sequences
+  const int64_t T = st->params.T, H = st->params.H, B = st->params.B, rs = st->row_stride;
   if (!aligned16(q) || !aligned16(kk) || !aligned16(v) || rs % 8) return false;
   CUtensorMap mq, mk, mv;
-  if (!encode_map(&mq, true, q, kHeadDim, T, H, rs, kHeadDim, 64, kRows, false) ||
-      !encode_map(&mk, true, kk, kHeadDim, T, H, rs, kHeadDim, 64, kRows, false) ||
-      !encode_map(&mv, true, v, kHeadDim, T, H, rs, kHeadDim, 64, kRows, false))
+  if (!encode_map_heads(&mq, true, q, kHeadDim, T, H, B, rs, 64, kRows, false) ||
+      !encode_map_heads(&mk, true, kk, kHeadDim, T, H, B, rs, 64, kRows, false) ||
+      !encode_map_heads(&mv, true, v, kHeadDim, T, H, B, rs, 64, kRows, false))
     return false;
   st->map_q = mq;
   st->map_k = mk;
@@ -1615,7 +1623,8 @@ void attention_set_shadow(PlanKernel& k, void* shadow_out) {
   // (its reader was told to expect it: assign_shadows asks attention_can_shadow first)
   __nv_bfloat16* out16 = static_cast<__nv_bfloat16*>(shadow_out);
   if (out16 != nullptr && encode_map_store(&st->map_out16, true, out16, (int64_t)st->params.H * kHeadDim,
-                                            (int64_t)st->params.B * st->params.T, 1, st->params.out16_row_stride, 0))
+                                            st->params.T, st->params.B, st->params.out16_row_stride,
+                                            st->params.T * st->params.out16_row_stride))
     st->params.out16 = out16;
 }
 

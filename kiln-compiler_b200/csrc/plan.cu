@@ -1006,11 +1006,14 @@ KB200_EXPORT int kb200_plan_create(const kb200_kernel_desc* descs, int n, int de
   int count = 0;
   KB200_CUDA(cudaGetDeviceCount(&count));
   if (device < 0 || device >= count) return fail(KB200_ERR_ARGUMENT, "kb200_plan_create: no CUDA device %d", device);
-  cudaDeviceProp prop;
-  KB200_CUDA(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10)
+  // (three attributes: cudaGetDeviceProperties takes 3 ms)
+  int major = 0, minor = 0, sm_count = 0;
+  KB200_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  KB200_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  KB200_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+  if (major != 10)
     return fail(KB200_ERR_UNSUPPORTED, "kb200_plan_create: device %d is sm_%d%d; this library is built for sm_100a only",
-                device, prop.major, prop.minor);
+                device, major, minor);
   for (int i = 0; i < n; ++i) {
     int rc = validate(descs[i], i);
     if (rc) return rc;
@@ -1018,7 +1021,7 @@ KB200_EXPORT int kb200_plan_create(const kb200_kernel_desc* descs, int n, int de
   Plan* plan = new (std::nothrow) Plan();
   if (!plan) return fail(KB200_ERR_ARGUMENT, "kb200_plan_create: out of host memory");
   plan->device = device;
-  plan->sm_count = prop.multiProcessorCount;
+  plan->sm_count = sm_count;
   plan->kernels.resize(n);
   for (int i = 0; i < n; ++i) {
     PlanKernel& k = plan->kernels[i];

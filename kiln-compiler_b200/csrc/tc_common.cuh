@@ -334,6 +334,24 @@ inline bool encode_map4(CUtensorMap* map, bool bf16, const void* base, int chunk
   return r == CUDA_SUCCESS;
 }
 
+// A 4-D map over [sequence, head, token, dim] views of a [sequence * token, row_stride] matrix whose rows
+// hold the heads side by side; box = (box_cols, box_rows, 1, 1).
+inline bool encode_map_heads(CUtensorMap* map, bool bf16, const void* base, int64_t dims_per_head, int64_t tokens, int64_t heads,
+                             int64_t sequences, int64_t row_stride_elems, int box_cols, int box_rows, bool atom32) {
+  EncodeFn fn = encode_fn();
+  if (!fn) return false;
+  const int esz = bf16 ? 2 : 4;
+  cuuint64_t dims[4] = {(cuuint64_t)dims_per_head, (cuuint64_t)tokens, (cuuint64_t)heads, (cuuint64_t)sequences};
+  cuuint64_t strides[3] = {(cuuint64_t)row_stride_elems * esz, (cuuint64_t)dims_per_head * esz, (cuuint64_t)row_stride_elems * tokens * esz};
+  cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1, 1};
+  cuuint32_t elem[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base),
+                  dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 // A 3-D map over [batch, rows, cols] (cols contiguous) for bulk stores of 32 x 32 blocks staged in
 // shared memory with rows of 128 bytes (float, 128-byte swizzle) or 64 bytes (bf16, 64-byte swizzle):
 // the swizzle lets both a lane-per-row and a lane-per-column writer fill the block without bank conflicts.

@@ -49,3 +49,19 @@ def test_rows_beyond_the_registers():
 @pytest.mark.parametrize("rows,d", [(1, 5), (7, 33), (513, 1001), (65, 2050), (2047, 255)])
 def test_elementwise_chain_of_any_width(rows, d):
     check({"kind": "bias_gelu", "rows": rows, "d": d}, ["ew_chain"])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("tokens", [2, 31, 63, 65, 127, 129, 255, 333, 1025])
+def test_sequences_of_any_length(tokens, precision):
+    check({"kind": "block", "tokens": tokens, "heads": 4, "precision": precision}, calls=2)
+    if tokens < 1000:
+        check({"kind": "batched_block", "batch": 3, "tokens": tokens, "heads": 2, "precision": precision}, calls=2)
+
+
+@pytest.mark.parametrize("choice", ["fma", "tensor"])
+@pytest.mark.parametrize("tokens", [33, 129, 1030])
+def test_both_fp32_attention_kernels_take_any_length(tokens, choice, monkeypatch):
+    monkeypatch.setenv("KILN_GPU_FP32_ATTENTION", choice)
+    check({"kind": "block", "tokens": tokens, "heads": 4})
+    check({"kind": "batched_block", "batch": 2, "tokens": tokens, "heads": 2})
