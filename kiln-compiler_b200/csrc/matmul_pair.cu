@@ -615,7 +615,7 @@ bool classify_steps(const PlanKernel& k, PairParams* p, const DevOperand** res_o
 
 }  // namespace
 
-bool pair_eligible(const Plan& plan, const PlanKernel& k) {
+bool pair_eligible(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
   if (d.precision == KB200_PREC_FP32 || !k.has_chain) return false;
   if (d.cfg[0] == 128) return false;                       // the tuner asked for single-CTA tiles
@@ -625,7 +625,7 @@ bool pair_eligible(const Plan& plan, const PlanKernel& k) {
   const int chunk_n = bf16 ? 64 : 32;
   const DevOperand& B = k.ops[d.b_slot];
   const bool b_nmajor = B.stride[2] == 1;
-  if (k.N < 128 || (b_nmajor && k.N % chunk_n)) return false;
+  if (k.N < 128 || k.N % 4 || (b_nmajor && b_cols % chunk_n)) return false;
   if (d.cfg[4] > 1) return false;                          // a forced split-K runs on the single-CTA kernel
   if (d.cfg[7] == 1 || d.cfg[7] == 2) return false;        // so do its epilogue variants
   if (((k.M + 255) / 256) * ((k.N + 127) / 128) * k.batch >= (int64_t(1) << 20)) return false;
@@ -741,7 +741,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
     if (ops.b_kmajor)
       ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, k.batch, ops.b_row, ops.b_batch, slab_k, p.half_bn, false);
     else
-      ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk_n, k.K, k.N / chunk_n, k.batch, ops.b_row, ops.b_batch, p.step_k,
+      ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk_n, k.K, ops.b_cols / chunk_n, k.batch, ops.b_row, ops.b_batch, p.step_k,
                        p.half_bn / chunk_n, !ops.bf16);
   }
   if (ok) ok = encode_map_store(&st->map_out, false, O.ptr, k.N, k.M, k.batch, O.stride[1], O.stride[0]);

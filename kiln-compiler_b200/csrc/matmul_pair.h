@@ -14,11 +14,12 @@ struct PairOperands {
   int64_t a_row, a_batch;    // strides in elements
   const void* b_base;        // [batch, K, N] N contiguous, or (b_kmajor) [batch, N, K] K contiguous
   int64_t b_row, b_batch;
+  int64_t b_cols;            // N-major B: columns its rows hold (N, or N padded to whole 128-byte chunks in a copy)
   bool b_kmajor;
 };
 
 // Shape, layout and epilogue tests that need no device pointers beyond those already resolved in `k`.
-bool pair_eligible(const Plan& plan, const PlanKernel& k);
+bool pair_eligible(const Plan& plan, const PlanKernel& k, int64_t b_cols);
 // Builds tensor maps and launch parameters.  *state stays null when the kernel declines (the caller
 // then uses the single-CTA kernel); a non-zero return is an error.
 int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, void** state);

@@ -795,6 +795,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         const int row = row_lo + r;
         const int64_t m = m0 + row, n = n0 + 4 * c4;
         if (m >= mm.M || n >= mm.N) continue;
+        const bool whole = n + 4 <= mm.N;          // the last columns of a width that is no multiple of four go one by one
         // the parked layout XORs the 16-byte slot within a 32-column group with the row
         const int slot = (c4 & ~7) | ((c4 & 7) ^ (row & 7));
         float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -810,12 +811,13 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           if (st.slot >= 0) {
             const DevOperand& o = mm.ops[st.slot];
             const float* src = o.ptr + batch * o.stride[0] + m * o.stride[1] + n * o.stride[2];
-            if (o.stride[2] == 1 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+            if (whole && o.stride[2] == 1 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
               const float4 t = __ldg(reinterpret_cast<const float4*>(src));
               side[0] = t.x; side[1] = t.y; side[2] = t.z; side[3] = t.w;
             } else {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) side[j] = __ldg(src + j * o.stride[2]);
+              for (int j = 0; j < 4; ++j)
+                if (n + j < mm.N) side[j] = __ldg(src + j * o.stride[2]);
             }
           }
 #pragma unroll
@@ -823,15 +825,16 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         }
         if (KB200_EXPERIMENT(1)) continue;
         float* dst = out_op.ptr + batch * out_op.stride[0] + m * out_op.stride[1] + n * out_op.stride[2];
-        if (out_op.stride[2] == 1 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        if (whole && out_op.stride[2] == 1 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
           *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) dst[j * out_op.stride[2]] = v[j];
+          for (int j = 0; j < 4; ++j)
+            if (n + j < mm.N) dst[j * out_op.stride[2]] = v[j];
         }
         if (p.out16 != nullptr) {
           __nv_bfloat16* dst16 = p.out16 + batch * out_op.stride[0] + m * out_op.stride[1] + n * out_op.stride[2];
-          if (out_op.stride[2] == 1 && (reinterpret_cast<uintptr_t>(dst16) & 7) == 0) {
+          if (whole && out_op.stride[2] == 1 && (reinterpret_cast<uintptr_t>(dst16) & 7) == 0) {
             __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
             uint2 packed;
             packed.x = *reinterpret_cast<uint32_t*>(&lo);
@@ -839,7 +842,8 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
             *reinterpret_cast<uint2*>(dst16) = packed;
           } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dst16[j * out_op.stride[2]] = __float2bfloat16_rn(v[j]);
+            for (int j = 0; j < 4; ++j)
+              if (n + j < mm.N) dst16[j * out_op.stride[2]] = __float2bfloat16_rn(v[j]);
           }
         }
       }
@@ -934,6 +938,46 @@ __global__ void __launch_bounds__(256) cvt_bf16_kernel(const float* __restrict__
   }
 }
 
+// Rows of any width and alignment -> rows of `pitch` elements (a multiple of 4), zeros behind the last
+// column, as bf16 or as they are: what a tensor map can describe.  Four elements per thread and step; a
+// warp's four loads of single floats cover the same 512 bytes.
+template <typename T>
+__global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict__ src, T* __restrict__ dst, uint32_t rows_all,
+                                                        uint32_t rows, uint32_t cols, uint32_t pitch, int64_t s_batch, int64_t s_row) {
+  pdl_wait();                 // the producer of this kernel's inputs has completed
+  pdl_launch_dependents();    // the next kernel may begin its start-up
+  const uint32_t per_row = pitch >> 2, total = rows_all * per_row;      // the host keeps this below 2^32
+  constexpr int U = 2;
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += step * U) {
+    float v[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + (uint32_t)u * step;
+      if (i >= total) continue;
+      const uint32_t row = i / per_row, c = (i - row * per_row) * 4;
+      const uint32_t bb = row / rows;
+      const float* at = src + (int64_t)bb * s_batch + (int64_t)(row - bb * rows) * s_row + c;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[u][e] = c + e < cols ? at[e] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + (uint32_t)u * step;
+      if (i >= total) continue;
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(dst + (size_t)i * 4) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+      } else {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(v[u][0], v[u][1]), hi = __floats2bfloat162_rn(v[u][2], v[u][3]);
+        uint2 packed;
+        packed.x = *reinterpret_cast<uint32_t*>(&lo);
+        packed.y = *reinterpret_cast<uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>(dst + (size_t)i * 4) = packed;
+      }
+    }
+  }
+}
+
 // Blocks of 256 threads with four vectors each, at most `cap` blocks.
 inline unsigned cvt_grid(int64_t vectors, int64_t cap) {
   const int64_t blocks = (vectors + 1023) / 1024;
@@ -947,12 +991,13 @@ struct TcState {
   size_t smem_bytes = 0;
   dim3 grid;
   bool bf16 = false;
-  // bf16 operand copies
-  __nv_bfloat16* a16 = nullptr;
-  __nv_bfloat16* b16 = nullptr;
-  bool b_const = false;       // B is a frozen constant: converted once at bind
-  bool a_shadow = false;      // A / B is read from the bf16 mirror its producer writes: no conversion launch
-  bool b_shadow = false;
+  // What the tensor maps describe instead of an operand itself: its bf16 values (BF16 mode, unless its
+  // producer writes them to the mirror), or its rows moved to a pitch of 16 bytes.
+  struct Copy {
+    void* data = nullptr;
+    int64_t rows = 0, cols = 0, pitch = 0;    // of one batch entry, in elements of the copy
+    bool once = false;                        // of a frozen constant: made at bind, not per launch
+  } a_copy, b_copy;
   void* pair = nullptr;       // state of the CTA-pair kernel (matmul_pair.cu) when it runs this matmul
 };
 
@@ -967,23 +1012,52 @@ bool tc_eligible(const PlanKernel& k) {
   if (!k.has_chain) return false;        // any other epilogue DAG runs on the SIMT kernel's tape path
   const DevOperand& A = k.ops[d.a_slot];
   const DevOperand& B = k.ops[d.b_slot];
-  if (k.M < 32 || k.N < 64 || k.K < 64) return false;
+  if (k.M < 2 || k.N < 64 || k.K < 64) return false;
   // tile indices are divided by multiplication, exact below 2^20 tiles (and every TMA coordinate fits an int)
   if (((k.M + 127) / 128) * ((k.N + 63) / 64) * k.batch >= (int64_t(1) << 20)) return false;
-  if (k.N % 4 || k.K % 4) return false;
-  if (d.precision == KB200_PREC_BF16 && (k.N % 8 || k.K % 8)) return false;
-  // the bf16 conversion pass indexes its vectors with 32 bits
-  if (d.precision == KB200_PREC_BF16 && (k.batch * k.M * k.K >= (int64_t(1) << 33) || k.batch * k.K * k.N >= (int64_t(1) << 33))) return false;
-  // A: K contiguous; B: N contiguous or K contiguous; 16-byte aligned bases and strides
+  // the passes that copy an operand index its vectors with 32 bits
+  if (k.batch * k.M * (k.K + 64) >= (int64_t(1) << 33) || k.batch * (k.K + 64) * (k.N + 64) >= (int64_t(1) << 33)) return false;
+  // A: K contiguous; B: N contiguous or K contiguous.  (Bases and strides that TMA cannot take are copied.)
   if (A.stride[2] != 1) return false;
   const bool b_nmajor = B.stride[2] == 1, b_kmajor = !b_nmajor && B.stride[1] == 1 && B.stride[2] != 0;
   if (!b_nmajor && !b_kmajor) return false;
-  if (A.stride[1] % 4 || A.stride[0] % 4 || B.stride[1] % 4 && b_nmajor || B.stride[2] % 4 && b_kmajor || B.stride[0] % 4) return false;
   if (A.stride[1] == 0 || (b_nmajor && B.stride[1] == 0)) return false;
   if (k.batch > 1 && (A.stride[0] == 0 || B.stride[0] == 0)) return false;
-  if (!aligned16(A.ptr) || !aligned16(B.ptr)) return false;
   return true;
 }
+
+namespace {
+
+void drop_copies(TcState* st) {
+  for (TcState::Copy* c : {&st->a_copy, &st->b_copy}) {
+    if (c->data) cudaFree(c->data);
+    *c = TcState::Copy();
+  }
+}
+
+// Can a tensor map of float32 elements describe rows of this stride at this address?
+bool rows_describable(const DevOperand& o, int64_t row_stride, int64_t batch) {
+  return aligned16(o.ptr) && row_stride % 4 == 0 && (batch == 1 || o.stride[0] % 4 == 0);
+}
+
+cudaError_t launch_copy(const TcState::Copy& c, bool bf16, const DevOperand& o, int64_t row_stride, int64_t batch, int64_t cap, bool pdl,
+                        cudaStream_t s) {
+  const int64_t units = batch * c.rows * (c.pitch / 4);
+  if (bf16 && c.pitch == c.cols && rows_describable(o, row_stride, batch))
+    return launch_kernel(pdl, cvt_bf16_kernel, dim3(cvt_grid(units, cap)), dim3(256), 0, s, (const float*)o.ptr,
+                         static_cast<__nv_bfloat16*>(c.data), batch, c.rows, c.cols, o.stride[0], row_stride);
+  const int64_t blocks = (units + 511) / 512;
+  const dim3 grid((unsigned)(blocks < cap ? blocks : cap));
+  if (bf16)
+    return launch_kernel(pdl, pack_rows_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, (const float*)o.ptr, static_cast<__nv_bfloat16*>(c.data),
+                         (uint32_t)(batch * c.rows), (uint32_t)c.rows, (uint32_t)c.cols, (uint32_t)c.pitch, o.stride[0], row_stride);
+  return launch_kernel(pdl, pack_rows_kernel<float>, grid, dim3(256), 0, s, (const float*)o.ptr, static_cast<float*>(c.data),
+                       (uint32_t)(batch * c.rows), (uint32_t)c.rows, (uint32_t)c.cols, (uint32_t)c.pitch, o.stride[0], row_stride);
+}
+
+}  // namespace
+
+void tc_destroy(PlanKernel& k);
 
 int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const kb200_kernel_desc& d = k.desc;
@@ -994,6 +1068,61 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   }
   st->bf16 = d.precision == KB200_PREC_BF16;
   const int chunk_n = st->bf16 ? 64 : 32, slab_k = st->bf16 ? 64 : 32;
+
+  // Operands as the tensor maps see them: A [M, K]; B [K, N] (N contiguous) or [N, K] (K contiguous)
+  const DevOperand& A = k.ops[d.a_slot];
+  const DevOperand& B = k.ops[d.b_slot];
+  const bool b_kmajor = B.stride[2] != 1;
+  const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = b_kmajor ? B.stride[2] : B.stride[1];
+  const void* a_base = A.ptr;
+  const void* b_base = B.ptr;
+  int64_t a_row = A.stride[1], a_batch = A.stride[0], b_row = b_src_row, b_batch = B.stride[0];
+  int64_t b_map_cols = b_cols;           // a copied N-major B is padded to whole 128-byte column chunks: one 4-D box per stage
+  drop_copies(st);
+  st->b_copy.once = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
+  const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
+  const bool copy_b = st->bf16 ? k.b_shadow == nullptr
+                               : !rows_describable(B, b_row, k.batch) || (st->b_copy.once && !b_kmajor && k.N % 4 == 0 && k.N % chunk_n != 0);
+  const int unit = st->bf16 ? 8 : 4, esz = st->bf16 ? 2 : 4;
+  auto make_copy = [&](TcState::Copy& c, int64_t rows, int64_t cols, int64_t to) {
+    c.rows = rows;
+    c.cols = cols;
+    c.pitch = (cols + to - 1) / to * to;
+    return cudaMalloc(&c.data, (size_t)k.batch * rows * c.pitch * esz);
+  };
+  k.launches = 1;
+  cudaError_t made = cudaSuccess;
+  if (copy_a) {
+    made = make_copy(st->a_copy, k.M, k.K, unit);
+    a_base = st->a_copy.data;
+    a_row = st->a_copy.pitch;
+    a_batch = k.M * a_row;
+    ++k.launches;
+  } else if (st->bf16) {
+    a_base = k.a_shadow;                 // the mirror has the operand's own strides
+  }
+  if (copy_b && made == cudaSuccess) {
+    made = make_copy(st->b_copy, b_rows, b_cols, b_kmajor ? unit : chunk_n);
+    b_base = st->b_copy.data;
+    b_row = st->b_copy.pitch;
+    b_batch = b_rows * b_row;
+    if (!b_kmajor) b_map_cols = b_row;
+    if (!st->b_copy.once) ++k.launches;
+  } else if (st->bf16) {
+    b_base = k.b_shadow;
+  }
+  if (made == cudaErrorMemoryAllocation && !st->bf16) {      // no room for an aligned copy: the CUDA-core kernel reads operands as they are
+    cudaGetLastError();
+    tc_destroy(k);
+    k.impl = IMPL_MM_SIMT;
+    k.launches = 1;
+    return KB200_OK;
+  }
+  KB200_CUDA(made);
+  if (copy_b && st->b_copy.once) {
+    KB200_CUDA(launch_copy(st->b_copy, st->bf16, B, b_src_row, k.batch, 4096, false, nullptr));
+    KB200_CUDA(cudaDeviceSynchronize());
+  }
   int bn = d.cfg[1];
   if (bn <= 0) {
     // the widest tile that still gives most SMs a tile of their own (measured: a second, partial
@@ -1061,8 +1190,8 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // pattern repeats every 4 rows; 16-bit elements use the ordinary 128-byte swizzle (8 rows).
   p.b_layout = st->bf16 ? 2 : 1;
   p.b_sbo_bytes = st->bf16 ? 1024 : 512;
-  p.b_kmajor = k.ops[d.b_slot].stride[2] == 1 ? 0 : 1;
-  p.b_mode = p.b_kmajor ? 0 : (k.N % chunk_n == 0 ? 1 : 2);
+  p.b_kmajor = b_kmajor ? 1 : 0;
+  p.b_mode = b_kmajor ? 0 : (b_map_cols % chunk_n == 0 ? 1 : 2);
   p.debug = d.cfg[6];
   p.issuers = issuers;
   p.split3 = split3 ? 1 : 0;
@@ -1157,58 +1286,19 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   st->grid = p.splits > 1 ? dim3((unsigned)p.num_units, 1, 1)     // one unit per CTA, clusters of `splits`
                           : dim3((unsigned)(p.num_units < plan.sm_count ? p.num_units : plan.sm_count), 1, 1);
 
-  const DevOperand& A = k.ops[d.a_slot];
-  const DevOperand& B = k.ops[d.b_slot];
-  const void* a_base = A.ptr;
-  const void* b_base = B.ptr;
-  // B as a [rows, cols] matrix with cols contiguous: [K, N] when N-major, [N, K] when K-major
-  const int64_t b_rows = p.b_kmajor ? k.N : k.K, b_cols = p.b_kmajor ? k.K : k.N;
-  int64_t a_row = A.stride[1], a_batch = A.stride[0], b_row = p.b_kmajor ? B.stride[2] : B.stride[1], b_batch = B.stride[0];
-  const int64_t b_src_row = b_row;
-  k.launches = 1;
-  if (st->bf16) {
-    if (st->a16) cudaFree(st->a16);
-    if (st->b16) cudaFree(st->b16);
-    st->a16 = st->b16 = nullptr;
-    st->a_shadow = k.a_shadow != nullptr;
-    st->b_shadow = k.b_shadow != nullptr;
-    if (!st->a_shadow) KB200_CUDA(cudaMalloc(&st->a16, (size_t)k.batch * k.M * k.K * 2));
-    if (!st->b_shadow) KB200_CUDA(cudaMalloc(&st->b16, (size_t)k.batch * k.K * k.N * 2));
-    st->b_const = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
-    if (st->b_const) {
-      const int64_t total = k.batch * b_rows * (b_cols / 4);
-      cvt_bf16_kernel<<<cvt_grid(total, 4096), 256>>>(
-          B.ptr, st->b16, k.batch, b_rows, b_cols, B.stride[0], b_src_row);
-      KB200_CUDA(cudaGetLastError());
-      KB200_CUDA(cudaDeviceSynchronize());
-    }
-    k.launches = 1 + (st->a_shadow ? 0 : 1) + ((st->b_const || st->b_shadow) ? 0 : 1);
-    if (st->a_shadow) {
-      a_base = k.a_shadow;              // the mirror has the operand's own strides
-    } else {
-      a_base = st->a16;
-      a_row = k.K; a_batch = k.M * k.K;
-    }
-    if (st->b_shadow) {
-      b_base = k.b_shadow;
-    } else {
-      b_base = st->b16;
-      b_row = b_cols; b_batch = k.K * k.N;
-    }
-  }
   // More than 128 rows: 256-row tiles on SM pairs (matmul_pair.cu) when that kernel covers the epilogue.
   if (st->pair) {
     pair_destroy(st->pair);
     st->pair = nullptr;
   }
-  if (pair_eligible(plan, k)) {
-    const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, p.b_kmajor != 0};
+  if (pair_eligible(plan, k, b_map_cols)) {
+    const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor};
     const int rc = pair_bind(plan, k, kernel_index, po, &st->pair);
     if (rc) return rc;
     if (st->pair) return KB200_OK;
   }
   if (!encode_map(&st->map_a, st->bf16, a_base, k.K, k.M, k.batch, a_row, a_batch, slab_k, kTileM, false) ||
-      !(p.b_mode == 1 ? encode_map4(&st->map_b, st->bf16, b_base, chunk_n, b_rows, b_cols / chunk_n, k.batch, b_row, b_batch, p.step_k,
+      !(p.b_mode == 1 ? encode_map4(&st->map_b, st->bf16, b_base, chunk_n, b_rows, b_map_cols / chunk_n, k.batch, b_row, b_batch, p.step_k,
                                     bn / chunk_n, !st->bf16)
                       : encode_map(&st->map_b, st->bf16, b_base, b_cols, b_rows, k.batch, b_row, b_batch, p.b_kmajor ? slab_k : chunk_n,
                                    p.b_kmajor ? bn : p.step_k, !st->bf16 && !p.b_kmajor)))
@@ -1227,7 +1317,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     p.store_mode = ok ? 1 : 0;
     // Without a matrix operand in the chain (only immediates and per-column vectors that 128-bit loads
     // can read) the epilogue needs no transpose: a lane keeps its accumulator row.
-    bool rowwise = ok && splits == 1 && d.cfg[7] != 2;
+    bool rowwise = ok && splits == 1 && d.cfg[7] != 2 && k.N % 4 == 0;
     for (int s_i = 0; s_i < k.chain.n && rowwise; ++s_i) {
       const int slot = k.chain.steps[s_i].slot;
       if (slot < 0) continue;
@@ -1248,23 +1338,11 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
 int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   const TcState* st = static_cast<const TcState*>(k.tc);
   const kb200_kernel_desc& d = k.desc;
-  if (st->bf16) {
-    const DevOperand& A = k.ops[d.a_slot];
-    const DevOperand& B = k.ops[d.b_slot];
-    const int64_t cap = (int64_t)plan.sm_count * 8;
-    int64_t total = k.batch * k.M * (k.K / 4);
-    if (!st->a_shadow)
-      KB200_CUDA(launch_kernel(plan.pdl, cvt_bf16_kernel, dim3(cvt_grid(total, cap)),
-                               dim3(256), 0, s, (const float*)A.ptr, st->a16, k.batch, k.M, k.K, A.stride[0], A.stride[1]));
-    if (!st->b_const && !st->b_shadow) {
-      const bool km = st->params.b_kmajor != 0;
-      const int64_t rows = km ? k.N : k.K, cols = km ? k.K : k.N;
-      total = k.batch * rows * (cols / 4);
-      KB200_CUDA(launch_kernel(plan.pdl, cvt_bf16_kernel, dim3(cvt_grid(total, cap)),
-                               dim3(256), 0, s, (const float*)B.ptr, st->b16, k.batch, rows, cols, B.stride[0],
-                               km ? B.stride[2] : B.stride[1]));
-    }
-  }
+  const int64_t cap = (int64_t)plan.sm_count * 8;
+  if (st->a_copy.data)
+    KB200_CUDA(launch_copy(st->a_copy, st->bf16, k.ops[d.a_slot], k.ops[d.a_slot].stride[1], k.batch, cap, plan.pdl, s));
+  if (st->b_copy.data && !st->b_copy.once)
+    KB200_CUDA(launch_copy(st->b_copy, st->bf16, k.ops[d.b_slot], k.ops[d.b_slot].stride[st->params.b_kmajor ? 2 : 1], k.batch, cap, plan.pdl, s));
   if (st->pair) return pair_launch(plan, st->pair, s);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = st->grid;
@@ -1302,8 +1380,8 @@ bool tc_repoint(PlanKernel& k) {
   if (!st) return true;
   const kb200_kernel_desc& d = k.desc;
   for (int o = 0; o < k.n_ops; ++o) st->params.mm.ops[o].ptr = k.ops[o].ptr;
-  const void* a = st->bf16 ? nullptr : k.ops[d.a_slot].ptr;
-  const void* b = st->bf16 ? nullptr : k.ops[d.b_slot].ptr;
+  const void* a = st->bf16 || st->a_copy.data ? nullptr : k.ops[d.a_slot].ptr;
+  const void* b = st->bf16 || st->b_copy.data ? nullptr : k.ops[d.b_slot].ptr;
   if (st->pair) return pair_repoint(k, st->pair, a, b);
   bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b));
   if (st->params.store_mode == 1) ok = ok && set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr);
@@ -1313,8 +1391,7 @@ bool tc_repoint(PlanKernel& k) {
 void tc_destroy(PlanKernel& k) {
   TcState* st = static_cast<TcState*>(k.tc);
   if (!st) return;
-  if (st->a16) cudaFree(st->a16);
-  if (st->b16) cudaFree(st->b16);
+  drop_copies(st);
   if (st->pair) pair_destroy(st->pair);
   delete st;
   k.tc = nullptr;

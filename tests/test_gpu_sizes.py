@@ -65,3 +65,11 @@ def test_both_fp32_attention_kernels_take_any_length(tokens, choice, monkeypatch
     monkeypatch.setenv("KILN_GPU_FP32_ATTENTION", choice)
     check({"kind": "block", "tokens": tokens, "heads": 4})
     check({"kind": "batched_block", "batch": 2, "tokens": tokens, "heads": 2})
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(2, 64, 64), (5, 65, 67), (16, 72, 200), (31, 100, 71), (128, 1001, 772), (129, 131, 770), (333, 1000, 771),
+                                   (257, 132, 65), (260, 1028, 68), (1000, 200, 1030)])
+def test_linear_of_any_size(m, n, k, precision):
+    """Operand rows off a 16-byte pitch, widths off a 128-byte column chunk, tiles with one row or column."""
+    check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
