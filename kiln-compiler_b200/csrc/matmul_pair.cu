@@ -60,12 +60,19 @@ constexpr int kPairATileBytes = 128 * 128;        // 128 rows x one 128-byte K s
 constexpr int kPairSmemCeiling = 200 * 1024;      // the trace arrays take static shared memory
 #define PAIR_STAMP(role, idx) do { if (blockIdx.x <= 1 && (idx) < 128) trace[role][idx] = clock64(); } while (0)
 #else
-constexpr int kPairSmemCeiling = 225 * 1024;      // opt-in ceiling, the same for every launch of the kernel
+constexpr int kPairSmemCeiling = 224 * 1024;      // opt-in ceiling, the same for every launch of the kernel
 #define PAIR_STAMP(role, idx) do { } while (0)
 #endif
 // barrier indices
 constexpr int kBarFull = 0, kBarEmpty = kPairMaxStages, kBarTFull = 2 * kPairMaxStages, kBarTEmpty = kBarTFull + 2,
               kBarRes = kBarTEmpty + 2, kBarCount = kBarRes + kPairEpiWarps;
+
+// The chains of a transformer's Linears have epilogues of their own; any other runs step by step.  A step of
+// the general form looks its descriptor up, branches on the operand's kind and jumps through a
+// switch over every scalar op: ~700 instructions of straight-line code per 32 x 32 block of the GELU
+// layer, which the warps fetched at ~25 cycles per 128-byte line (2000-2500 cycles per block, 14 000 per
+// tile against 6 100 of its main loop).  Written for one chain, in packed arithmetic, it is ~200.
+enum : int { EPI_CHAIN = 0, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RES };
 
 enum : int { SIDE_NONE = 0, SIDE_IMM = 1, SIDE_COL = 2, SIDE_RES = 3 };
 
@@ -80,6 +87,7 @@ struct PairStep {
 struct PairParams {
   // what the producer and the MMA thread need comes first (constant-bank lines touched at start-up)
   int bn, half_bn, stages, num_kb, slab_k, kps, step_k;
+  int b_static;          // B is a frozen constant: its first stages are requested before the previous kernel has finished
   int b_kmajor;          // B is [N, K] with K contiguous (boxes like A); else [K, N], one 4-D box per stage
   int chunk_n;           // columns per 128-byte row of an N-major B chunk: 32 (tf32) or 64 (bf16)
   uint32_t b_lbo_bytes, b_sbo_bytes, b_layout, b_step16, b_slab16;
@@ -156,7 +164,18 @@ __device__ __forceinline__ void store_wait_read(int allowed) {
   }
 }
 
-template <bool BF16, int KPS>
+// One stage of this CTA's half of the B tile.
+template <int KPS>
+__device__ __forceinline__ void load_b_pair(const PairParams& p, const CUtensorMap* map, uint32_t dst, uint32_t bar, int k_elem, int n_col,
+                                            int batch) {
+  if (p.b_kmajor) {
+    for (int j = 0; j < KPS; ++j) tma_load_3d_pair(dst + j * p.half_bn * 128, map, bar, k_elem + j * p.slab_k, n_col, batch);
+  } else {
+    tma_load_4d_pair(dst, map, bar, 0, k_elem, n_col / p.chunk_n, batch);
+  }
+}
+
+template <bool BF16, int KPS, int EPI>
 __global__ void __launch_bounds__(kPairThreads, 1)
 mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out16,
@@ -166,6 +185,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ PairStep chain_steps[kMaxChain];     // looked up by a run-time index for every block
+  __shared__ __align__(16) float columns[kPairEpiWarps][32];   // the bias of the block a warp is working on
 #ifdef KB200_TRACE
   __shared__ long long trace[5][128];
   __shared__ long long marks[8];
@@ -233,6 +253,20 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       *abort_ptr = 1;
     }
   }
+  // A frozen B is nobody's output: the first stages' weights are requested before the wait for the
+  // previous kernel, so that they are on their way, or here, when the activations are ready.
+  const uint32_t full_leader0 = map_to_cta(full0, 0);
+  int ahead = 0;                 // stages of the first tile whose B is requested already (producer thread)
+  if (p.b_static && threadIdx.x == 0 && pair < p.num_tiles) {
+    const int batch = pair_div(pair, p.magic_tpb);
+    const int rem = pair - batch * p.tiles_per_batch;
+    const int n_col = (rem - pair_div(rem, p.magic_tn) * p.tiles_n) * p.bn + (int)rank * p.half_bn;
+    ahead = p.stages < p.num_kb ? p.stages : p.num_kb;
+    for (int s = 0; s < ahead; ++s) {
+      if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
+      load_b_pair<KPS>(p, &tma_b, tiles + (uint32_t)(s * stage_bytes + a_stage_bytes), full_leader0 + 8 * s, s * p.step_k, n_col, batch);
+    }
+  }
   // Everything above may have overlapped the previous kernel's tail; from here on its output is read.
   pdl_wait();
   pdl_launch_dependents();
@@ -245,9 +279,8 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     if (lane == 0) {
       const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, slab_k = p.slab_k, step_k = p.step_k;
       constexpr int kps = KPS;
-      const int bn = p.bn, half_bn = p.half_bn, b_kmajor = p.b_kmajor, chunk_n = p.chunk_n;
+      const int bn = p.bn, half_bn = p.half_bn;
       const uint32_t tx_bytes = (uint32_t)stage_bytes;
-      const uint32_t full_leader0 = map_to_cta(full0, 0);
       int s = 0;
       uint32_t wait_parity = 1;
       bool ok = true;
@@ -268,16 +301,13 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           // the leader's barrier counts the bytes of both CTAs (the peer's may land first: the phase
           // cannot complete before this arrival)
           PAIR_STAMP(0, tp);
-          if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * tx_bytes);
+          const bool b_here = ahead > 0;           // expected and requested above
+          if (!b_here && rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * tx_bytes);
           const uint32_t bar = full_leader0 + 8 * s;
           const uint32_t dst = tiles + (uint32_t)(s * stage_bytes);
           for (int j = 0; j < kps; ++j) tma_load_3d_pair(dst + j * kPairATileBytes, &tma_a, bar, k_elem + j * slab_k, m_row, batch);
-          if (b_kmajor) {
-            for (int j = 0; j < kps; ++j)
-              tma_load_3d_pair(dst + a_stage_bytes + j * half_bn * 128, &tma_b, bar, k_elem + j * slab_k, n_col, batch);
-          } else {
-            tma_load_4d_pair(dst + a_stage_bytes, &tma_b, bar, 0, k_elem, n_col / chunk_n, batch);
-          }
+          if (b_here) --ahead;
+          else load_b_pair<KPS>(p, &tma_b, dst + a_stage_bytes, bar, k_elem, n_col, batch);
           PAIR_STAMP(1, tp);
 #ifdef KB200_TRACE
           ++tp;
@@ -491,7 +521,8 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           mbar_expect_tx(res_bar, 4096);
           tma_load_3d(slot0, &tma_res, res_bar, n, m_first, p.res_batched ? batch : 0);
         }
-        if (col_step >= 0 && scratch_off >= 0) reinterpret_cast<float*>(slot0_ptr + scratch_off)[lane] = mine;
+        if (EPI != EPI_CHAIN) columns[e][lane] = mine;
+        else if (col_step >= 0 && scratch_off >= 0) reinterpret_cast<float*>(slot0_ptr + scratch_off)[lane] = mine;
         float v[32];
 #ifdef KB200_TRACE
         if (p.debug & 4) {
@@ -504,7 +535,35 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 #ifdef KB200_TRACE
         if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
 #endif
-        run_chain(v, mine, n, batch);
+        if constexpr (EPI == EPI_CHAIN) {
+          run_chain(v, mine, n, batch);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {        // every lane reads the same 16 bytes: a broadcast
+            const float4 t = *reinterpret_cast<const float4*>(&columns[e][4 * q]);
+            const float2 a = fadd2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(t.x, t.y));
+            const float2 b = fadd2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(t.z, t.w));
+            v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = b.x; v[4 * q + 3] = b.y;
+          }
+          if constexpr (EPI == EPI_BIAS_GELU) {
+            if (BF16) gelu_tanh_approx_pairs(v);
+            else gelu_tanh_pairs(v);
+          }
+          if constexpr (EPI == EPI_BIAS_RES) {
+            if (!dry) {
+              bool landed = mbar_wait(res_bar, res_phase, abort_ptr);
+              if (!landed && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 5); *abort_ptr = 1; }
+              res_phase ^= 1u;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float4 t = *reinterpret_cast<const float4*>(slot0_ptr + lane * 128 + ((q ^ (lane & 7)) << 4));
+              const float2 a = fadd2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(t.x, t.y));
+              const float2 b = fadd2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(t.z, t.w));
+              v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = b.x; v[4 * q + 3] = b.y;
+            }
+          }
+        }
         __syncwarp();
 #ifdef KB200_TRACE
         if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
@@ -570,13 +629,34 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   }
 }
 
+using PairKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PairParams);
+
+template <bool BF16, int KPS>
+PairKernel pair_kernel(int epilogue) {
+  switch (epilogue) {
+    case EPI_BIAS: return mm_pair_kernel<BF16, KPS, EPI_BIAS>;
+    case EPI_BIAS_GELU: return mm_pair_kernel<BF16, KPS, EPI_BIAS_GELU>;
+    case EPI_BIAS_RES: return mm_pair_kernel<BF16, KPS, EPI_BIAS_RES>;
+    default: return mm_pair_kernel<BF16, KPS, EPI_CHAIN>;
+  }
+}
+
+int epilogue_of(const PairParams& p) {
+  const PairStep* s = p.steps;
+  const bool bias = p.n_steps >= 1 && s[0].op == CH_ADD && s[0].kind == SIDE_COL;
+  if (p.n_steps == 1 && bias) return EPI_BIAS;
+  if (p.n_steps == 2 && bias && (s[1].op == CH_GELU_TANH || s[1].op == CH_GELU_TANH_APPROX)) return EPI_BIAS_GELU;
+  if (p.n_steps == 2 && bias && s[1].op == CH_ADD && s[1].kind == SIDE_RES) return EPI_BIAS_RES;
+  return EPI_CHAIN;
+}
+
 struct PairState {
   CUtensorMap map_a, map_b, map_out, map_out16, map_res;
   PairParams params;
   size_t smem_bytes = 0;
   dim3 grid;
   bool bf16 = false;
-  void (*kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PairParams) = nullptr;
+  PairKernel kernel = nullptr;
 };
 
 // The chain step operands the epilogue can take: immediates, unary ops, per-column vectors readable
@@ -690,6 +770,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   p.step_k = kps * slab_k;
   p.num_kb = (int)((k.K + p.step_k - 1) / p.step_k);
   p.b_kmajor = ops.b_kmajor ? 1 : 0;
+  p.b_static = ops.b_static ? 1 : 0;
   p.chunk_n = chunk_n;
   p.b_lbo_bytes = (uint32_t)(p.step_k * 128);              // N-major: bytes between the column chunks of a stage
   p.b_sbo_bytes = ops.bf16 ? 1024 : 512;
@@ -750,8 +831,8 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   if (ok && out16) ok = encode_map_store(&st->map_out16, true, out16, k.N, k.M, k.batch, O.stride[1], O.stride[0]);
   if (ok && res) ok = encode_map_store(&st->map_res, false, res->ptr, k.N, k.M, p.res_batched ? k.batch : 1, res->stride[1], res->stride[0]);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = ops.bf16 ? (kps == 2 ? mm_pair_kernel<true, 2> : mm_pair_kernel<true, 1>)
-                        : (kps == 2 ? mm_pair_kernel<false, 2> : mm_pair_kernel<false, 1>);
+  st->kernel = ops.bf16 ? (kps == 2 ? pair_kernel<true, 2>(epilogue_of(p)) : pair_kernel<true, 1>(epilogue_of(p)))
+                        : (kps == 2 ? pair_kernel<false, 2>(epilogue_of(p)) : pair_kernel<false, 1>(epilogue_of(p)));
   cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemCeiling);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_pair_kernel)"); }
   *state = st;

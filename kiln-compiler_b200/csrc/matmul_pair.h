@@ -16,6 +16,7 @@ struct PairOperands {
   int64_t b_row, b_batch;
   int64_t b_cols;            // N-major B: columns its rows hold (N, or N padded to whole 128-byte chunks in a copy)
   bool b_kmajor;
+  bool b_static;             // a frozen constant, no kernel's output
 };
 
 // Shape, layout and epilogue tests that need no device pointers beyond those already resolved in `k`.

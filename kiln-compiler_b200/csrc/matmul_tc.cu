@@ -86,6 +86,7 @@ struct TcParams {
   int b_step_bytes;     // bytes between consecutive MMA K steps inside a B chunk
   int b_sbo_bytes;      // bytes between the row groups of one swizzle atom of B
   int b_layout;         // descriptor layout type of B (1 = 128-byte swizzle on 32-byte atoms, 2 = 128-byte swizzle)
+  int b_static;         // B is a frozen constant: loaded without waiting for the previous kernel
   int b_kmajor;         // B is read K-major ([N, K] with K contiguous) like A
   int b_mode;           // how B is fetched: 0 K-major (one box), 1 N-major, all chunks in one 4-D box, 2 N-major, a box per chunk
   int debug;            // trace builds only: 1 = no stores, 16 = no epilogue (results are then wrong), 32 = no warm-up pass
@@ -353,8 +354,9 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   // (the barrier itself takes thousands of cycles to complete; they pass under the main loop).
   if (p.splits > 1) cluster_arrive();
   // Everything above (barriers, TMEM, descriptor prefetch) may have overlapped the previous kernel's
-  // tail; from here on its output is read.
-  pdl_wait();
+  // tail; from here on its output is read.  A frozen B is nobody's output: its producer does not wait, so
+  // the first stages of a weight matrix are on their way, or here, when the activations are ready.
+  if (!(p.b_static && warp == kProducerBWarp)) pdl_wait();
   pdl_launch_dependents();
   volatile int* abort_ptr = &abort_flag;
 #ifdef KB200_TRACE
@@ -1191,6 +1193,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   p.b_layout = st->bf16 ? 2 : 1;
   p.b_sbo_bytes = st->bf16 ? 1024 : 512;
   p.b_kmajor = b_kmajor ? 1 : 0;
+  p.b_static = st->b_copy.once ? 1 : 0;
   p.b_mode = b_kmajor ? 0 : (b_map_cols % chunk_n == 0 ? 1 : 2);
   p.debug = d.cfg[6];
   p.issuers = issuers;
@@ -1292,7 +1295,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     st->pair = nullptr;
   }
   if (pair_eligible(plan, k, b_map_cols)) {
-    const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor};
+    const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor, st->b_copy.once};
     const int rc = pair_bind(plan, k, kernel_index, po, &st->pair);
     if (rc) return rc;
     if (st->pair) return KB200_OK;
