@@ -66,6 +66,8 @@ constexpr int kThreads = 64 + 32 * kEpiWarps + 64; // producer (A) warp, MMA war
 constexpr int kEpiStage16Offset = 4608;        // 512-byte aligned (64-byte swizzle); the float block is 1024-byte aligned
 constexpr int kEpiWarpBytes = 7168;
 constexpr int kEpiBytes = kEpiWarps * kEpiWarpBytes;
+constexpr int kExactEpiWarpBytes = 4096;       // exact-FP32 mode: no bf16 block, and a transpose within 32 x 32 floats, for a third stage
+constexpr int kExactEpiBytes = kEpiWarps * kExactEpiWarpBytes;
 constexpr int kEpiSlotBytes = 4096 + 2048;   // one float block + one bf16 block of the rotating staging slots
 #ifdef KB200_TRACE
 constexpr int kMaxDynamicSmem = 200 * 1024;   // the trace arrays take static shared memory
@@ -105,6 +107,7 @@ struct TcParams {
   int store_mode;       // 0: the epilogue warps store with ordinary global stores; 1: bulk tensor stores from shared memory
   int split3;           // exact-FP32 mode: every operand is split in shared memory into a TF32 head and a TF32 tail,
                         // and three MMAs per K step (head x head, head x tail, tail x head) give float32 products
+  int presplit;         // ... 1: the tails of a frozen B are loaded, from a copy made at bind; 2: those of A too, from one made per launch
   int issuers;          // 1, or 2: two threads issue the MMAs of alternate pipeline stages into accumulators of their own
   uint64_t magic_stages;   // ceil(2^40 / stages)
   int epi_rowwise;      // the epilogue keeps a lane per ROW (no transpose): the chain has no matrix operand
@@ -286,6 +289,7 @@ template <bool BF16, bool SPLIT3>
 __global__ void __launch_bounds__(kThreads, 1)
 mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
              const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out16,
+             const __grid_constant__ CUtensorMap tma_at, const __grid_constant__ CUtensorMap tma_bt,
              const __grid_constant__ TcParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kMaxStages + 6];   // + two cluster hand-shake barriers (split K) + per-stage "operands split" barriers
@@ -320,6 +324,10 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     // descriptor fetches overlap the set-up below instead of delaying the first copy
     prefetch_tensormap(&tma_a);
     prefetch_tensormap(&tma_b);
+    if (SPLIT3 && p.presplit) {
+      prefetch_tensormap(&tma_bt);
+      if (p.presplit == 2) prefetch_tensormap(&tma_at);
+    }
     if (p.store_mode == 1) {
       prefetch_tensormap(&tma_out);
       if (p.out16 != nullptr) prefetch_tensormap(&tma_out16);
@@ -376,7 +384,8 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
       const int bn = p.bn, chunk_n = p.chunk_n, b_mode = p.b_mode, n_chunks = p.n_chunks;
       const uint32_t chunk_bytes = (uint32_t)step_k * kSlabBytes;          // one column chunk of B: step_k rows of 128 bytes
       const uint32_t b_slab_bytes = (uint32_t)bn * kSlabBytes;             // K-major B: one slab of bn rows
-      const uint32_t tx_bytes = load_a ? (uint32_t)a_stage_bytes : (uint32_t)b_tile_bytes;
+      const int parts = SPLIT3 && p.presplit >= (load_a ? 2 : 1) ? 2 : 1;                      // the operand's tails follow it
+      const uint32_t tx_bytes = (uint32_t)parts * (load_a ? (uint32_t)a_stage_bytes : (uint32_t)b_tile_bytes);
       int s = 0;
       uint32_t wait_parity = 1;                // parity to wait for on the empty barriers of this pass over the ring
       bool ok = true;
@@ -396,19 +405,22 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           }
           if (load_a) KB200_STAMP(0, tp);
           mbar_expect_tx(full, tx_bytes);
-          const uint32_t a_dst = tiles + s * stage_bytes;
-          // a slab past the end of K (odd slab count with two slabs per stage) is a box outside the
-          // tensor: it arrives as zeros and adds nothing
-          if (load_a) {
-            for (int j = 0; j < kps; ++j) tma_load_3d(a_dst + j * kATileBytes, &tma_a, full, k_elem + j * slab_k, m0, batch);
-          } else if (b_mode == 0) {              // K-major B: one box per slab, like A
-            for (int j = 0; j < kps; ++j)
-              tma_load_3d(a_dst + a_stage_bytes + j * b_slab_bytes, &tma_b, full, k_elem + j * slab_k, n0, batch);
-          } else if (b_mode == 1) {              // N-major B, all column chunks of the tile and all slabs of the stage in one 4-D box
-            tma_load_4d(a_dst + a_stage_bytes, &tma_b, full, 0, k_elem, n0_chunk, batch);
-          } else {                               // N-major B, N not a multiple of the chunk: one box per chunk
-            for (int c = 0; c < n_chunks; ++c)
-              tma_load_3d(a_dst + a_stage_bytes + c * chunk_bytes, &tma_b, full, n0 + c * chunk_n, k_elem, batch);
+          for (int part = 0; part < parts; ++part) {
+            const uint32_t a_dst = tiles + s * stage_bytes + part * raw_bytes;
+            const CUtensorMap* map = SPLIT3 && part ? (load_a ? &tma_at : &tma_bt) : (load_a ? &tma_a : &tma_b);
+            // a slab past the end of K (odd slab count with two slabs per stage) is a box outside the
+            // tensor: it arrives as zeros and adds nothing
+            if (load_a) {
+              for (int j = 0; j < kps; ++j) tma_load_3d(a_dst + j * kATileBytes, map, full, k_elem + j * slab_k, m0, batch);
+            } else if (b_mode == 0) {              // K-major B: one box per slab, like A
+              for (int j = 0; j < kps; ++j)
+                tma_load_3d(a_dst + a_stage_bytes + j * b_slab_bytes, map, full, k_elem + j * slab_k, n0, batch);
+            } else if (b_mode == 1) {              // N-major B, all column chunks of the tile and all slabs of the stage in one 4-D box
+              tma_load_4d(a_dst + a_stage_bytes, map, full, 0, k_elem, n0_chunk, batch);
+            } else {                               // N-major B, N not a multiple of the chunk: one box per chunk
+              for (int c = 0; c < n_chunks; ++c)
+                tma_load_3d(a_dst + a_stage_bytes + c * chunk_bytes, map, full, n0 + c * chunk_n, k_elem, batch);
+            }
           }
           if (load_a) KB200_STAMP(1, tp);
 #ifdef KB200_TRACE
@@ -449,8 +461,10 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         int kb_begin, kb_end;
         slab_range(p, ks, kb_begin, kb_end);
         const int n_steps = kb_end - kb_begin;
-        const int acc = i & 1;
-        const uint32_t aph = (i >> 1) & 1;
+        // (loaded tails leave the order of a single buffer's tiles to these barriers: one pair, a phase per tile)
+        const bool one_buffer = SPLIT3 && p.presplit == 2 && !p.acc2;
+        const int acc = one_buffer ? 0 : i & 1;
+        const uint32_t aph = one_buffer ? i & 1 : (i >> 1) & 1;
         // the epilogue must have drained this accumulator (two tiles ago) before it is overwritten
         if (!mbar_wait(tempty0 + 8 * acc, aph ^ 1, abort_ptr)) {
           if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 4); *abort_ptr = 1; }
@@ -474,7 +488,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         int s = g_first - round * stages;
         for (int g = g_first; g < g0 + n_steps; g += nq) {
           // exact-FP32 mode: the stage is ready when the epilogue warps have split it, not when it lands
-          if (!mbar_wait((split3 ? split0 : full0) + 8 * s, (uint32_t)round & 1u, abort_ptr)) {
+          if (!mbar_wait((split3 && p.presplit != 2 ? split0 : full0) + 8 * s, (uint32_t)round & 1u, abort_ptr)) {
             if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 2); *abort_ptr = 1; }
             ok = false;
             break;
@@ -525,7 +539,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     const int e = warp - 2;
     const int quad = warp & 3;
     const int half = e >> 2;
-    float* tbuf = reinterpret_cast<float*>(epi_buf + e * kEpiWarpBytes);
+    float* tbuf = reinterpret_cast<float*>(epi_buf + e * (SPLIT3 ? kExactEpiWarpBytes : kEpiWarpBytes));
     __nv_bfloat16* stage16 = reinterpret_cast<__nv_bfloat16*>(epi_buf + e * kEpiWarpBytes + kEpiStage16Offset);
     const bool bulk = p.store_mode == 1 && p.splits == 1;
     const bool rowwise = bulk && p.epi_rowwise != 0;
@@ -538,13 +552,13 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     // leading bits, which is all the tensor core reads of the landed float) goes to the second half of
     // the stage; the MMA thread waits for all eight warps.  Steps are taken in the order of the ring.
     auto split_steps = [&](int count) {
-      const int n4 = raw_bytes / 16;
+      const int n4 = (p.presplit ? a_stage_bytes : raw_bytes) / 16;      // (with the tails of B loaded, A is what is left to do)
       for (int n = 0; n < count; ++n) {
         bool got = mbar_wait(full0 + 8 * sp_s, sp_parity, abort_ptr);
         if (!got && lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 7); *abort_ptr = 1; }
         if (__shfl_sync(0xffffffffu, got ? 1 : 0, 0) == 0 || *abort_ptr) return false;
         float4* head = reinterpret_cast<float4*>(smem_raw + (tiles - raw) + (size_t)sp_s * stage_bytes);
-        float4* tail = head + n4;
+        float4* tail = head + raw_bytes / 16;
         for (int idx = e * 32 + lane; idx < n4; idx += kEpiWarps * 32) {
           const float4 v = head[idx];
           float4 t;
@@ -574,8 +588,9 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     for (int unit = blockIdx.x; unit < p.num_units && ok; unit += gridDim.x, ++i) {
       int tile, ks, batch, tm_i, tn_i;
       unit_coords(p, unit, tile, ks, batch, tm_i, tn_i);
-      const int acc = i & 1;
-      const uint32_t aph = (i >> 1) & 1;
+      const bool one_buffer = SPLIT3 && p.presplit == 2 && !p.acc2;
+      const int acc = one_buffer ? 0 : i & 1;
+      const uint32_t aph = one_buffer ? i & 1 : (i >> 1) & 1;
       const int64_t m0 = (int64_t)tm_i * kTileM, n0 = (int64_t)tn_i * p.bn;
       const int64_t m_first = m0 + quad * 32;
       const bool direct = p.splits == 1;
@@ -594,8 +609,8 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
       // Before its first tile is ready a CTA has nothing for these warps to do, and their code (the
       // unrolled chain, some kilobytes) is not in the instruction cache yet: one dry pass of the loop
       // body over zeros, with nothing stored, takes those misses off the critical path.
-      const bool dry_pass = i == 0 && direct && bulk && !KB200_EXPERIMENT(32) && !SPLIT3;
-      if (SPLIT3) {
+      const bool dry_pass = i == 0 && direct && bulk && !KB200_EXPERIMENT(32) && !(SPLIT3 && p.presplit != 2);
+      if (SPLIT3 && p.presplit != 2) {
         ok = split_steps(unsplit);
         if (!ok) break;
         // With two accumulator buffers the next tile's first steps are split before this tile is
@@ -655,11 +670,12 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
 #endif
         if (!rowwise && direct) {
           // transpose through shared memory: lane = row  ->  lane = column
+          // (conflict-free by a pitch of 33, or within 32 x 32 by exchanging columns)
 #pragma unroll
-          for (int j = 0; j < 32; ++j) tbuf[lane * 33 + j] = v[j];
+          for (int j = 0; j < 32; ++j) tbuf[SPLIT3 ? lane * 32 + (j ^ lane) : lane * 33 + j] = v[j];
           __syncwarp();
 #pragma unroll
-          for (int r = 0; r < 32; ++r) v[r] = tbuf[r * 33 + lane];
+          for (int r = 0; r < 32; ++r) v[r] = tbuf[SPLIT3 ? r * 32 + (lane ^ r) : r * 33 + lane];
           __syncwarp();
         }
 #ifdef KB200_TRACE
@@ -980,6 +996,40 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict_
   }
 }
 
+// tail[r][c] = what the tensor core's 19 leading bits leave of src[r][c]: the second TF32 terms of an
+// exact-FP32 operand.  Rows 16-byte aligned; the floats that fill a last vector are multiplied with nothing.
+__global__ void __launch_bounds__(256) tail_rows_kernel(const float* __restrict__ src, float* __restrict__ tail, uint32_t rows, uint32_t cols,
+                                                        int64_t s_row, int64_t t_row) {
+  pdl_wait();                 // the producer of this kernel's inputs has completed
+  pdl_launch_dependents();    // the next kernel may begin its start-up
+  const uint32_t per_row = (cols + 3) >> 2, total = rows * per_row;
+  constexpr int U = 4;
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += step * U) {
+    float4 v[U];
+    uint32_t row[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + (uint32_t)u * step;
+      if (i >= total) continue;
+      row[u] = i / per_row;
+      c[u] = (i - row[u] * per_row) * 4;
+      const float* at = src + (int64_t)row[u] * s_row + c[u];
+      if (c[u] + 4 <= cols) {
+        v[u] = *reinterpret_cast<const float4*>(at);
+      } else {
+        v[u] = make_float4(at[0], c[u] + 1 < cols ? at[1] : 0.0f, c[u] + 2 < cols ? at[2] : 0.0f, 0.0f);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (base + (uint32_t)u * step >= total) continue;
+      *reinterpret_cast<float4*>(tail + (int64_t)row[u] * t_row + c[u]) =
+          make_float4(tf32_tail(v[u].x), tf32_tail(v[u].y), tf32_tail(v[u].z), tf32_tail(v[u].w));
+    }
+  }
+}
+
 // Blocks of 256 threads with four vectors each, at most `cap` blocks.
 inline unsigned cvt_grid(int64_t vectors, int64_t cap) {
   const int64_t blocks = (vectors + 1023) / 1024;
@@ -1000,6 +1050,11 @@ struct TcState {
     int64_t rows = 0, cols = 0, pitch = 0;    // of one batch entry, in elements of the copy
     bool once = false;                        // of a frozen constant: made at bind, not per launch
   } a_copy, b_copy;
+  // exact FP32 with a frozen B: the operands' tails (see tail_rows_kernel), [M, tail_pitch] and like B's map
+  float* a_tail = nullptr;
+  float* b_tail = nullptr;
+  int64_t tail_pitch = 0;
+  CUtensorMap map_at, map_bt;
   void* pair = nullptr;       // state of the CTA-pair kernel (matmul_pair.cu) when it runs this matmul
 };
 
@@ -1035,6 +1090,9 @@ void drop_copies(TcState* st) {
     if (c->data) cudaFree(c->data);
     *c = TcState::Copy();
   }
+  if (st->a_tail) cudaFree(st->a_tail);
+  if (st->b_tail) cudaFree(st->b_tail);
+  st->a_tail = st->b_tail = nullptr;
 }
 
 // Can a tensor map of float32 elements describe rows of this stride at this address?
@@ -1081,6 +1139,13 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   int64_t a_row = A.stride[1], a_batch = A.stride[0], b_row = b_src_row, b_batch = B.stride[0];
   int64_t b_map_cols = b_cols;           // a copied N-major B is padded to whole 128-byte column chunks: one 4-D box per stage
   drop_copies(st);
+  // Exact FP32: the tails of a frozen B are made here and loaded beside it.  Those of A come from a pass in
+  // front of every launch where CTAs walk several tiles (the epilogue warps, who otherwise make them in
+  // shared memory, would leave the tensor cores waiting while they drain a tile), with one row of tiles
+  // from those warps: they have nothing else to do then, and the pass would cost another launch.  An
+  // operand B of the plan's own is split by the warps too, 144 to 192 KB of traffic per step at 128
+  // bytes a clock.
+  const bool presplit = d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind == KB200_BASE_CONST && k.batch == 1;
   st->b_copy.once = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
   const bool copy_b = st->bf16 ? k.b_shadow == nullptr
@@ -1113,6 +1178,13 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   } else if (st->bf16) {
     b_base = k.b_shadow;
   }
+  const bool a_pass = presplit && k.M > kTileM;
+  if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
+  if (a_pass && made == cudaSuccess) {
+    st->tail_pitch = (k.K + 3) / 4 * 4;
+    made = cudaMalloc(&st->a_tail, (size_t)k.M * st->tail_pitch * sizeof(float));
+    ++k.launches;
+  }
   if (made == cudaErrorMemoryAllocation && !st->bf16) {      // no room for an aligned copy: the CUDA-core kernel reads operands as they are
     cudaGetLastError();
     tc_destroy(k);
@@ -1123,8 +1195,11 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   KB200_CUDA(made);
   if (copy_b && st->b_copy.once) {
     KB200_CUDA(launch_copy(st->b_copy, st->bf16, B, b_src_row, k.batch, 4096, false, nullptr));
-    KB200_CUDA(cudaDeviceSynchronize());
   }
+  if (presplit)
+    KB200_CUDA(launch_kernel(false, tail_rows_kernel, dim3(cvt_grid(b_rows * ((b_map_cols + 3) / 4), 4096)), dim3(256), 0, nullptr, static_cast<const float*>(b_base), st->b_tail,
+                             (uint32_t)b_rows, (uint32_t)b_map_cols, b_row, b_row));
+  if (presplit || (copy_b && st->b_copy.once)) KB200_CUDA(cudaDeviceSynchronize());
   int bn = d.cfg[1];
   if (bn <= 0) {
     // the widest tile that still gives most SMs a tile of their own (measured: a second, partial
@@ -1139,6 +1214,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     }
   }
   const bool split3 = d.precision == KB200_PREC_FP32;     // exact FP32: three TF32 MMAs on split operands
+  const int epi_bytes = split3 ? kExactEpiBytes : kEpiBytes;
   if (split3 && bn > 128) bn = 128;                        // a stage holds heads and tails of both operands
   if (split3 && d.cfg[1] <= 0 && bn == 64 && k.N >= 128) {
     // Exact-FP32 mode is bound by shared-memory traffic, of which a 128-column tile needs a third less
@@ -1165,7 +1241,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   int kps = d.cfg[2] == 1 || d.cfg[2] == 2 ? d.cfg[2] : (issuers == 2 ? 1 : (bn <= 128 && k.K >= 4 * slab_k ? 2 : 1));
   if (split3) kps = 1;
   const int stage_bytes = (split3 ? 2 : 1) * kps * (kATileBytes + bn * kSlabBytes);
-  while (stages > 2 && (size_t)stages * stage_bytes + kEpiBytes + 1024 > (size_t)kMaxDynamicSmem) --stages;
+  while (stages > 2 && (size_t)stages * stage_bytes + epi_bytes + 1024 > (size_t)kMaxDynamicSmem) --stages;
   // Two issuers take alternate pipeline steps.  A wait on an mbarrier tells apart only two consecutive
   // phases, so every stage must belong to ONE issuer, who then sees each of its phases in turn: with an
   // even stage count step g and stage g % stages have the same parity.  (With an odd count ownership
@@ -1198,6 +1274,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   p.debug = d.cfg[6];
   p.issuers = issuers;
   p.split3 = split3 ? 1 : 0;
+  p.presplit = a_pass ? 2 : presplit ? 1 : 0;
   p.tmem_cols = 32;
   while (p.tmem_cols < 2 * p.issuers * bn) p.tmem_cols *= 2;   // per issuer two accumulators: the epilogue drains one while the next tile fills the other
   p.nacc = 1;
@@ -1249,14 +1326,14 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   if (splits > 1) {
     const size_t tile_bytes = (size_t)kTileM * bn * sizeof(float);
     int fit = stages;
-    while (fit > 2 && (size_t)fit * stage_bytes + kEpiBytes + tile_bytes + 1024 > (size_t)kMaxDynamicSmem) --fit;
-    if ((size_t)fit * stage_bytes + kEpiBytes + tile_bytes + 1024 > (size_t)kMaxDynamicSmem || (size_t)fit * stage_bytes < tile_bytes) {
+    while (fit > 2 && (size_t)fit * stage_bytes + epi_bytes + tile_bytes + 1024 > (size_t)kMaxDynamicSmem) --fit;
+    if ((size_t)fit * stage_bytes + epi_bytes + tile_bytes + 1024 > (size_t)kMaxDynamicSmem || (size_t)fit * stage_bytes < tile_bytes) {
       splits = 1;
     } else {
       stages = fit;
       if (issuers == 2) stages &= ~1;
       p.stages = stages;
-      p.recv_offset = stages * stage_bytes + kEpiBytes;
+      p.recv_offset = stages * stage_bytes + epi_bytes;
     }
   }
   p.splits = splits;
@@ -1284,7 +1361,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     if (per_column && p.pre_col_step < 0) p.pre_col_step = st_i;
     else if (!per_column && p.pre_mat_step < 0) p.pre_mat_step = st_i;
   }
-  st->smem_bytes = (size_t)stages * stage_bytes + kEpiBytes + 1024 + (splits > 1 ? (size_t)kTileM * bn * sizeof(float) : 0);
+  st->smem_bytes = (size_t)stages * stage_bytes + epi_bytes + 1024 + (splits > 1 ? (size_t)kTileM * bn * sizeof(float) : 0);
   // persistent CTAs, one per SM: each walks the tile list with a stride of the grid size
   st->grid = p.splits > 1 ? dim3((unsigned)p.num_units, 1, 1)     // one unit per CTA, clusters of `splits`
                           : dim3((unsigned)(p.num_units < plan.sm_count ? p.num_units : plan.sm_count), 1, 1);
@@ -1306,6 +1383,11 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
                       : encode_map(&st->map_b, st->bf16, b_base, b_cols, b_rows, k.batch, b_row, b_batch, p.b_kmajor ? slab_k : chunk_n,
                                    p.b_kmajor ? bn : p.step_k, !st->bf16 && !p.b_kmajor)))
     return fail(KB200_ERR_UNSUPPORTED, "matmul %s: the operands cannot be described to TMA", d.name);
+  st->map_at = st->map_a;
+  st->map_bt = st->map_b;
+  if ((a_pass && !encode_map(&st->map_at, false, st->a_tail, k.K, k.M, 1, st->tail_pitch, 0, slab_k, kTileM, false)) ||
+      (presplit && !set_map_address(&st->map_bt, st->b_tail)))
+    return fail(KB200_ERR_UNSUPPORTED, "matmul %s: the operands' tails cannot be described to TMA", d.name);
   // Bulk tensor stores need a column-contiguous output with 16-byte aligned base and strides (and the
   // same of the bf16 mirror when there is one); anything else keeps the ordinary stores.
   {
@@ -1346,6 +1428,13 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     KB200_CUDA(launch_copy(st->a_copy, st->bf16, k.ops[d.a_slot], k.ops[d.a_slot].stride[1], k.batch, cap, plan.pdl, s));
   if (st->b_copy.data && !st->b_copy.once)
     KB200_CUDA(launch_copy(st->b_copy, st->bf16, k.ops[d.b_slot], k.ops[d.b_slot].stride[st->params.b_kmajor ? 2 : 1], k.batch, cap, plan.pdl, s));
+  if (st->a_tail) {
+    // from the aligned copy, where there is one
+    const float* src = st->a_copy.data ? static_cast<const float*>(st->a_copy.data) : k.ops[d.a_slot].ptr;
+    const int64_t row = st->a_copy.data ? st->a_copy.pitch : k.ops[d.a_slot].stride[1];
+    KB200_CUDA(launch_kernel(plan.pdl, tail_rows_kernel, dim3(cvt_grid(k.M * ((k.K + 3) / 4), cap)), dim3(256), 0, s, src, st->a_tail, (uint32_t)k.M,
+                             (uint32_t)k.K, row, st->tail_pitch));
+  }
   if (st->pair) return pair_launch(plan, st->pair, s);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = st->grid;
@@ -1368,9 +1457,9 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  if (st->bf16) KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<true, false>, st->map_a, st->map_b, st->map_out, st->map_out16, st->params));
-  else if (st->params.split3) KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<false, true>, st->map_a, st->map_b, st->map_out, st->map_out16, st->params));
-  else KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<false, false>, st->map_a, st->map_b, st->map_out, st->map_out16, st->params));
+  if (st->bf16) KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<true, false>, st->map_a, st->map_b, st->map_out, st->map_out16, st->map_at, st->map_bt, st->params));
+  else if (st->params.split3) KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<false, true>, st->map_a, st->map_b, st->map_out, st->map_out16, st->map_at, st->map_bt, st->params));
+  else KB200_CUDA(cudaLaunchKernelEx(&cfg, mm_tc_kernel<false, false>, st->map_a, st->map_b, st->map_out, st->map_out16, st->map_at, st->map_bt, st->params));
   KB200_CUDA(cudaGetLastError());
   return KB200_OK;
 }
@@ -1542,7 +1631,7 @@ int kb200_matmul_bf16_static(const float* a, const float* b, float* c, int64_t m
   dim3 grid((unsigned)(p.num_tiles < sms ? p.num_tiles : sms), 1, 1);
   p.store_mode = 0;   // ordinary stores: the two store maps are unused placeholders
   p.epi_rowwise = 0;
-  mm_tc_kernel<true, false><<<grid, kThreads, smem, s>>>(map_a, map_b, map_a, map_a, p);
+  mm_tc_kernel<true, false><<<grid, kThreads, smem, s>>>(map_a, map_b, map_a, map_a, map_a, map_b, p);
   KB200_CUDA(cudaGetLastError());
   return KB200_OK;
 }
