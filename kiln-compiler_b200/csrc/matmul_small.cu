@@ -1,0 +1,542 @@
+// Tensor-core matmul for problems of few tiles: one row of 128-row tiles (prompts of up to 128 tokens), or
+// so few in all that most SMs would idle.  Same role as matmul_tc.cu for the Linears of a transformer
+// (bias, bias + GELU, bias + residual; kiln/gpu/codegen.py:484-530, 563-598) in all three precisions.
+//
+// What bounds such a problem is latency: an SM takes ~64 bytes a clock from L2, so a lone CTA that walks
+// 768 of K (24 slabs of 24 KB) needs 5 us for its operands however fast the tensor cores are, and every
+// phase that runs once -- set-up, first copy, drain, exchange, epilogue -- costs its instruction fetches
+// from a cold cache on top of its latencies.  So:
+//   * K is split over the CTAs of a thread-block cluster until the SMs are used, and the whole K range of
+//     a CTA is in flight at once where shared memory holds it;
+//   * the partial tiles are exchanged straight from registers: the thread that reads a row of the
+//     accumulator writes it with st.async into the CTA that finishes that row's band, data and arrival
+//     count in one operation.  (matmul_tc.cu parks the tile in shared memory first and pushes bands
+//     with bulk copies; parking, the barrier behind it and the pushes took ~6000 cycles of a launch.)
+//   * the epilogue is written for its chain, over float4 items in row order: bias and residual are
+//     fetched before the accumulator is ready, stores cover whole lines;
+//   * weights are requested before the wait for the previous kernel.
+// The sum over the splits runs in rank order, so results do not depend on timing.
+//
+// Per CTA, 352 threads: warp 0 loads A, warp 10 loads B, warp 1 issues the MMAs, warps 2-9 (two per tensor-memory
+// lane quadrant) split A in the exact-FP32 mode, then drain, exchange and finish.  Waits are bounded as
+// in matmul_tc.cu.
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+#include "device_math.cuh"
+#include "kb200_internal.h"
+#include "matmul.h"
+#include "matmul_small.h"
+#include "tc_common.cuh"
+#include "tc_epilogue.cuh"
+
+namespace kb200 {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kSmallM = 128, kSmallN = 64;
+constexpr int kSmallThreads = 352;
+constexpr int kSmallEpiWarps = 8;
+constexpr int kSmallMaxStages = 8;
+constexpr int kSmallABytes = kSmallM * 128, kSmallBBytes = kSmallN * 128;      // one 128-byte K slab
+constexpr int kSmallExchange = kSmallM * kSmallN * 4;
+constexpr int kSmallSmem = 225 * 1024;
+
+enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2 };
+enum : int { FIN_NONE = 0, FIN_BIAS, FIN_BIAS_GELU, FIN_BIAS_RES };
+
+struct SmallParams {
+  int stages, num_slabs, slab_k, splits;
+  int b_kmajor, b_static;
+  int nacc;                        // exact FP32: accumulators the K steps rotate over, beside the one of the small products
+  uint32_t b_lbo, b_sbo, b_layout, b_step16;
+  uint32_t idesc;
+  int tmem_cols;
+  int tiles_n;
+  int kernel_index;
+  int* status;
+  int M, N;
+  const float* bias;
+  const float* res;
+  int64_t res_row;
+  float* out;                      // null: only the bf16 copy is stored
+  __nv_bfloat16* out16;            // or null
+  int64_t out_row;                 // of both
+};
+
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t bar, float4 v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
+               : "memory");
+}
+
+template <int MODE, int FIN>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
+  constexpr bool EXACT = MODE == SMALL_EXACT;
+  constexpr int kRaw = kSmallABytes + kSmallBBytes;             // a stage: A, B; exact FP32: then their tails
+  constexpr int kStage = EXACT ? 2 * kRaw : kRaw;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t ring = (raw + 1023u) & ~1023u;
+  const uint32_t recv = ring + (uint32_t)(p.stages * kStage);   // [split][128 / splits rows][64 floats], 16-byte units XORed with the row
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
+  const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8;
+  const int tile = blockIdx.x / p.splits;
+  const int rank = blockIdx.x - tile * p.splits;                // in the cluster: its CTAs are consecutive
+  const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
+  const int slab0 = rank * p.num_slabs / p.splits, n_slabs = (rank + 1) * p.num_slabs / p.splits - slab0;
+
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(full0 + 8 * s, 2);
+      mbar_init(empty0 + 8 * s, 1);
+      mbar_init(split0 + 8 * s, kSmallEpiWarps);
+    }
+    mbar_init(done, 1);
+    mbar_init(received, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(received, kSmallExchange);                   // (an arrival, too; a launch without a split does not use it)
+  }
+  if (threadIdx.x == 32) {
+    prefetch_tensormap(&tma_a);
+    prefetch_tensormap(&tma_b);
+    if (EXACT) prefetch_tensormap(&tma_bt);
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)p.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // The next kernel's set-up may overlap all of this one (it waits for it to complete) -- from here on: its
+  // CTAs must not take tensor memory that this one still has to allocate.
+  pdl_launch_dependents();
+  // Every CTA's barriers exist once all have arrived here; waited for in front of the exchange.  A launch
+  // without a split is no cluster launch and keeps off every cluster instruction (st.async in one is
+  // an illegal instruction).
+  const bool clustered = p.splits > 1;
+  if (clustered) cluster_arrive();
+  const uint32_t tmem = tmem_slot;
+  volatile int* abort_ptr = &abort_flag;
+  auto give_up = [&](int site) {
+    if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
+  };
+  // a frozen B is nobody's output: its producer does not wait for the previous kernel
+  if (!(warp == 10 && p.b_static)) pdl_wait();
+
+  if (warp == 0 || warp == 10) {
+    // ---------------- TMA producers, one per operand ----------------
+    if (lane == 0) {
+      const bool is_a = warp == 0;
+      int s = 0, k_elem = slab0 * p.slab_k;
+      uint32_t parity = 1;
+      for (int i = 0; i < n_slabs; ++i, k_elem += p.slab_k) {
+        if (!mbar_wait(empty0 + 8 * s, parity, abort_ptr)) { give_up(1); break; }
+        const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage);
+        if (is_a) {
+          mbar_expect_tx(bar, kSmallABytes);
+          tma_load_3d(dst, &tma_a, bar, k_elem, tm * kSmallM, 0);
+        } else {
+          mbar_expect_tx(bar, (EXACT ? 2 : 1) * kSmallBBytes);
+#pragma unroll
+          for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
+            const CUtensorMap* map = part ? &tma_bt : &tma_b;
+            const uint32_t at = dst + kSmallABytes + part * kRaw;
+            if (p.b_kmajor) tma_load_3d(at, map, bar, k_elem, tn * kSmallN, 0);
+            else tma_load_4d(at, map, bar, 0, k_elem, tn * (kSmallN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
+          }
+        }
+        if (++s == p.stages) { s = 0; parity ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      const uint64_t a_fixed = make_desc(0, 16, 1024);
+      const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
+      const uint32_t b_step = p.b_step16, idesc = p.idesc;
+      int s = 0, rot = 0;
+      uint32_t parity = 0;
+      bool ok = true;
+      for (int i = 0; i < n_slabs; ++i) {
+        if (!mbar_wait((EXACT ? split0 : full0) + 8 * s, parity, abort_ptr)) { give_up(2); ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a16 = (ring + (uint32_t)(s * kStage)) >> 4, b16 = a16 + (kSmallABytes >> 4);
+        // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
+        auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t a = a16 + 2 * k, b = b16 + k * b_step;
+          if (EXACT) {
+            // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
+            // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
+            // with the number of them (see matmul_tc.cu)
+            umma(tmem, desc(a_fixed, a + (kRaw >> 4)), desc(b_fixed, b), idesc, (i | k) != 0, false);
+            umma(tmem, desc(a_fixed, a), desc(b_fixed, b + (kRaw >> 4)), idesc, 1u, false);
+            umma(tmem + (uint32_t)((1 + rot) * kSmallN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
+          } else {
+            umma(tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
+          }
+        }
+        if (EXACT && ++rot == p.nacc) rot = 0;
+        if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
+        if (++s == p.stages) { s = 0; parity ^= 1; }
+      }
+      if (ok) umma_commit(done);
+    }
+  } else {
+    // ---------------- warps 2..9 ----------------
+    const int e = warp - 2, quad = warp & 3, half = e >> 2, t = threadIdx.x - 64;
+    const int band_rows = kSmallM / p.splits;
+    // this thread's items of the band: float4 number t, t + 256, ... in row order
+    const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * kSmallN;
+    const int n = n0 + 4 * (t & 15);
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (FIN != FIN_NONE && n < p.N) bias = __ldg(reinterpret_cast<const float4*>(p.bias + n));
+    float4 res[FIN == FIN_BIAS_RES ? 8 : 1];
+    if (FIN == FIN_BIAS_RES) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = (t >> 4) + 16 * j, m = m0 + band0 + r;
+        if (r < band_rows && m < p.M && n < p.N) res[j] = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
+      }
+    }
+    bool ok = true;
+    if (EXACT) {
+      // the tails of A: what its 19 leading bits leave
+      int s = 0;
+      uint32_t parity = 0;
+      for (int i = 0; i < n_slabs && ok; ++i) {
+        if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) { give_up(7); }
+        ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
+        if (!ok) break;
+        float4* head = reinterpret_cast<float4*>(smem_raw + (ring - raw) + s * kStage);
+#pragma unroll
+        for (int q = 0; q < kSmallABytes / 16 / 256; ++q) {
+          const float4 v = head[t + 256 * q];
+          head[kRaw / 16 + t + 256 * q] =
+              make_float4(v.x - __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u), v.y - __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u),
+                          v.z - __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u), v.w - __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u));
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(split0 + 8 * s);
+        if (++s == p.stages) { s = 0; parity ^= 1; }
+      }
+    }
+    if (ok && !mbar_wait(done, 0, abort_ptr)) give_up(3);
+    ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
+    __syncwarp();
+    if (clustered) cluster_wait();              // every CTA's `received` exists
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float v[32];
+      const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 32);
+      tmem_ld32(at, v);
+      if (EXACT) {
+        const int used = min(p.nacc, n_slabs);
+#pragma unroll 1
+        for (int a = 1; a <= used; ++a) {
+          float w[32];
+          tmem_ld32(at + (uint32_t)(a * kSmallN), w);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += w[j];
+        }
+      }
+      const int row = quad * 32 + lane;
+      if (clustered) {
+        // this row's half goes to the CTA that finishes its band
+        const int dest = row / band_rows, r = row - dest * band_rows;
+        const uint32_t to = map_to_cta(recv + (uint32_t)((rank * band_rows + r) * 256 + half * 128), (uint32_t)dest);
+        const uint32_t bar = map_to_cta(received, (uint32_t)dest);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          st_async(to + (uint32_t)((q ^ (r & 7)) << 4), bar, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+      } else {
+        uint8_t* const to = smem_raw + (recv - raw) + row * 256 + half * 128;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<float4*>(to + ((q ^ (row & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      }
+    }
+    __syncwarp();
+    if (!clustered) asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight warps
+    else if (!mbar_wait_cluster(received, 0, abort_ptr)) give_up(5);
+    __syncwarp();
+    ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
+    if (ok) {
+      const uint8_t* const parts = smem_raw + (recv - raw);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = (t >> 4) + 16 * j, m = m0 + band0 + r;
+        if (r >= band_rows) break;
+        const int u = t & 15;
+        const uint8_t* src = parts + r * 256 + (((u & 8) | ((u ^ r) & 7)) << 4);
+        float4 a = *reinterpret_cast<const float4*>(src);
+        for (int s = 1; s < p.splits; ++s) {
+          const float4 b = *reinterpret_cast<const float4*>(src + s * band_rows * 256);
+          a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        if (m >= p.M || n >= p.N) continue;
+        if (FIN != FIN_NONE) { a.x += bias.x; a.y += bias.y; a.z += bias.z; a.w += bias.w; }
+        if (FIN == FIN_BIAS_GELU) {
+          if (MODE == SMALL_BF16) {
+            a.x = f_gelu_tanh_approx(a.x); a.y = f_gelu_tanh_approx(a.y); a.z = f_gelu_tanh_approx(a.z); a.w = f_gelu_tanh_approx(a.w);
+          } else {
+            a.x = d_gelu_tanh(a.x); a.y = d_gelu_tanh(a.y); a.z = d_gelu_tanh(a.z); a.w = d_gelu_tanh(a.w);
+          }
+        }
+        if (FIN == FIN_BIAS_RES) { a.x += res[j].x; a.y += res[j].y; a.z += res[j].z; a.w += res[j].w; }
+        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = a;
+        if (p.out16 != nullptr) {
+          __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+          uint2 packed;
+          packed.x = *reinterpret_cast<uint32_t*>(&lo);
+          packed.y = *reinterpret_cast<uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
+        }
+      }
+    }
+  }
+  // The roles above ran in one lane: the warp has to be whole again for an .aligned barrier.
+  __syncwarp();
+  if (clustered && (warp < 2 || warp == 10)) cluster_wait();       // (the other warps have passed this phase above)
+  // ---------------- exit ----------------
+  if (abort_flag && threadIdx.x == 0) {
+    // copies may still be in flight towards this CTA's shared memory: give them a bounded time to land
+    const long long t0 = clock64();
+    while (clock64() - t0 < 400000) { }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  // A CTA that has received everything is written to no more.  One that gave up stays until the others of its cluster have left or given up too.
+  if (clustered && abort_flag) {
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)p.tmem_cols) : "memory");
+  }
+}
+
+using SmallKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, SmallParams);
+
+struct SmallState {
+  CUtensorMap map_a, map_b, map_bt;
+  SmallParams params;
+  SmallKernel kernel = nullptr;
+  unsigned grid = 0;
+  size_t smem = 0;
+  int bias_slot = -1, res_slot = -1;
+  bool a_moves = false, b_moves = false;      // the maps hold the operand's own address
+};
+
+template <int MODE>
+SmallKernel small_kernel(int fin) {
+  switch (fin) {
+    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS>;
+    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU>;
+    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES>;
+    default: return mm_small_kernel<MODE, FIN_NONE>;
+  }
+}
+
+// The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.
+int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot) {
+  const Chain& c = k.chain;
+  *bias_slot = *res_slot = -1;
+  if (c.n == 0) return FIN_NONE;
+  const ChainStep* s = c.steps;
+  if (s[0].op != CH_ADD || s[0].slot < 0) return -1;
+  const DevOperand& b = k.ops[s[0].slot];
+  if (b.stride[1] != 0 || b.stride[2] != 1 || !aligned16(b.ptr)) return -1;
+  *bias_slot = s[0].slot;
+  if (c.n == 1) return FIN_BIAS;
+  if (c.n != 2) return -1;
+  if (s[1].op == CH_GELU_TANH) return FIN_BIAS_GELU;
+  if (s[1].op != CH_ADD || s[1].slot < 0) return -1;
+  const DevOperand& r = k.ops[s[1].slot];
+  if (r.stride[2] != 1 || r.stride[1] < k.N || r.stride[1] % 4 || !aligned16(r.ptr)) return -1;
+  *res_slot = s[1].slot;
+  return FIN_BIAS_RES;
+}
+
+// Clusters of `splits` CTAs, one CTA per SM, that fit the GPU at once (147 SMs in use at most: the SMs of
+// a processing cluster need not be a multiple of the size).
+int resident_clusters(int splits, int sm_count) {
+  static int known[9] = {0};
+  if (splits == 1) return sm_count;
+  if (known[splits] == 0) {
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(splits * (sm_count / splits)), 1, 1);
+    cfg.blockDim = dim3(kSmallThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSmallSmem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = sm_count * 7 / 10 / splits;
+    }
+    known[splits] = n > 0 ? n : 1;
+  }
+  return known[splits];
+}
+
+struct SmallPlan { int splits; int64_t cycles; };
+
+// K split and estimated cycles.  A CTA's step costs the larger of its operands' way from L2 (~55 bytes a clock)
+// and the issue of its MMAs (~62 cycles each); the rest of a launch, set-up to last store, ~6500, plus
+// ~1500 for an exchange.
+SmallPlan plan_small(int64_t tiles, int64_t slabs, int mode, int sm_count) {
+  const int64_t step = mode == SMALL_EXACT ? 900 : 450;
+  SmallPlan best{1, 0};
+  for (int s : {1, 2, 4, 8}) {
+    if (s > slabs) break;
+    const int64_t resident = resident_clusters(s, sm_count);
+    const int64_t rounds = (tiles + resident - 1) / resident;
+    const int64_t cycles = rounds * (((slabs + s - 1) / s) * step + 6500 + (s > 1 ? 1500 : 0));
+    if (best.cycles == 0 || cycles < best.cycles) best = {s, cycles};
+  }
+  return best;
+}
+
+}  // namespace
+
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
+  const kb200_kernel_desc& d = k.desc;
+  const bool bf16 = d.precision == KB200_PREC_BF16;
+  int bias_slot, res_slot;
+  if (!k.has_chain || k.batch != 1 || finish_of(k, &bias_slot, &res_slot) < 0) return -1;
+  for (int i : {0, 1, 2, 3, 4, 6})
+    if (d.cfg[i] != 0) return -1;                     // a tile, stage or split was asked for (how to store is not a question here)
+  if (k.M >= (1 << 20) || k.N >= (1 << 24) || k.N % 4) return -1;
+  const DevOperand& B = k.ops[d.b_slot];
+  if (B.stride[2] == 1 && b_cols % (bf16 ? 64 : 32)) return -1;
+  if (d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind != KB200_BASE_CONST) return -1;
+  const DevOperand& O = k.ops[k.chain.out_slot];
+  if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
+  const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * ((k.N + kSmallN - 1) / kSmallN);
+  if (tiles > 4096) return -1;
+  const int slab_k = bf16 ? 64 : 32;
+  const int mode = bf16 ? SMALL_BF16 : d.precision == KB200_PREC_FP32 ? SMALL_EXACT : SMALL_TF32;
+  return plan_small(tiles, (k.K + slab_k - 1) / slab_k, mode, plan.sm_count).cycles;
+}
+
+int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, void** state) {
+  *state = nullptr;
+  SmallState* st = new SmallState();
+  SmallParams& p = st->params;
+  const kb200_kernel_desc& d = k.desc;
+  const int mode = ops.bf16 ? SMALL_BF16 : b_tail ? SMALL_EXACT : SMALL_TF32;
+  const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
+  const int slab_k = ops.bf16 ? 64 : 32, chunk = ops.bf16 ? 64 : 32;
+  p.slab_k = slab_k;
+  p.num_slabs = (int)((k.K + slab_k - 1) / slab_k);
+  p.tiles_n = (int)((k.N + kSmallN - 1) / kSmallN);
+  const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
+  p.splits = plan_small(tiles, p.num_slabs, mode, plan.sm_count).splits;
+  const int stage_bytes = (mode == SMALL_EXACT ? 2 : 1) * (kSmallABytes + kSmallBBytes);
+  const int most = (p.num_slabs + p.splits - 1) / p.splits;
+  p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
+  while ((size_t)p.stages * stage_bytes + kSmallExchange + 1024 > (size_t)kSmallSmem) --p.stages;
+  st->smem = (size_t)p.stages * stage_bytes + kSmallExchange + 1024;
+  st->grid = (unsigned)(tiles * p.splits);
+  p.b_kmajor = ops.b_kmajor ? 1 : 0;
+  p.b_static = ops.b_static ? 1 : 0;
+  p.b_lbo = (uint32_t)(slab_k * 128);
+  p.b_sbo = ops.bf16 ? 1024 : 512;
+  p.b_layout = ops.bf16 ? 2 : 1;
+  p.b_step16 = ops.b_kmajor ? 2u : (uint32_t)((ops.bf16 ? 16 : 8) * 128) >> 4;
+  const uint32_t fmt = ops.bf16 ? 1u : 2u;
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(kSmallN >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
+  p.nacc = 1;
+  p.tmem_cols = kSmallN;
+  if (mode == SMALL_EXACT) {
+    // one accumulator per 512 of K for the large products, beside that of the small ones
+    const int64_t want = ((int64_t)most * slab_k + 511) / 512;
+    p.nacc = want > 7 ? 7 : (int)want;
+    while (p.tmem_cols < (1 + p.nacc) * kSmallN) p.tmem_cols *= 2;
+  }
+  p.kernel_index = kernel_index;
+  p.status = plan.d_status;
+  p.M = (int)k.M;
+  p.N = (int)k.N;
+  p.bias = st->bias_slot >= 0 ? k.ops[st->bias_slot].ptr : nullptr;
+  p.res = st->res_slot >= 0 ? k.ops[st->res_slot].ptr : nullptr;
+  p.res_row = st->res_slot >= 0 ? k.ops[st->res_slot].stride[1] : 0;
+  const DevOperand& O = k.ops[k.chain.out_slot];
+  p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
+  p.out = k.mirror_only && p.out16 ? nullptr : O.ptr;
+  p.out_row = O.stride[1];
+  st->a_moves = ops.a_base == k.ops[d.a_slot].ptr;
+  st->b_moves = ops.b_base == k.ops[d.b_slot].ptr;
+  bool ok = encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, 1, ops.a_row, 0, slab_k, kSmallM, false);
+  if (ok && ops.b_kmajor) ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, 1, ops.b_row, 0, slab_k, kSmallN, false);
+  else if (ok) ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk, k.K, ops.b_cols / chunk, 1, ops.b_row, 0, slab_k, kSmallN / chunk, !ops.bf16);
+  st->map_bt = st->map_b;
+  if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
+  if (!ok) { delete st; return KB200_OK; }
+  st->kernel = mode == SMALL_BF16 ? small_kernel<SMALL_BF16>(fin) : mode == SMALL_EXACT ? small_kernel<SMALL_EXACT>(fin) : small_kernel<SMALL_TF32>(fin);
+  const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
+  if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
+  *state = st;
+  return KB200_OK;
+}
+
+int small_launch(const Plan& plan, const void* state, cudaStream_t s) {
+  const SmallState* st = static_cast<const SmallState*>(state);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(st->grid, 1, 1);
+  cfg.blockDim = dim3(kSmallThreads, 1, 1);
+  cfg.dynamicSmemBytes = st->smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (st->params.splits > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)st->params.splits;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (plan.pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  KB200_CUDA(cudaLaunchKernelEx(&cfg, st->kernel, st->map_a, st->map_b, st->map_bt, st->params));
+  return KB200_OK;
+}
+
+bool small_repoint(const PlanKernel& k, void* state) {
+  SmallState* st = static_cast<SmallState*>(state);
+  if (st->bias_slot >= 0) st->params.bias = k.ops[st->bias_slot].ptr;
+  if (st->res_slot >= 0) st->params.res = k.ops[st->res_slot].ptr;
+  if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
+  return (!st->a_moves || set_map_address(&st->map_a, k.ops[k.desc.a_slot].ptr)) &&
+         (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));
+}
+
+void small_destroy(void* state) { delete static_cast<SmallState*>(state); }
+
+}  // namespace kb200

@@ -36,6 +36,7 @@
 #include "kb200_internal.h"
 #include "matmul.h"
 #include "matmul_pair.h"
+#include "matmul_small.h"
 #include "tc_common.cuh"
 #include "tc_epilogue.cuh"
 
@@ -1055,6 +1056,7 @@ struct TcState {
   float* b_tail = nullptr;
   int64_t tail_pitch = 0;
   CUtensorMap map_at, map_bt;
+  void* small = nullptr;      // state of the kernel for few tiles (matmul_small.cu) when it runs this matmul
   void* pair = nullptr;       // state of the CTA-pair kernel (matmul_pair.cu) when it runs this matmul
 };
 
@@ -1145,6 +1147,8 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // from those warps: they have nothing else to do then, and the pass would cost another launch.  An
   // operand B of the plan's own is split by the warps too, 144 to 192 KB of traffic per step at 128
   // bytes a clock.
+  if (st->small) small_destroy(st->small);
+  st->small = nullptr;
   const bool presplit = d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind == KB200_BASE_CONST && k.batch == 1;
   st->b_copy.once = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
@@ -1178,6 +1182,9 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   } else if (st->bf16) {
     b_base = k.b_shadow;
   }
+  // Few tiles: the kernel written for latency.
+  const int64_t b_pad = st->b_copy.once && copy_b && !b_kmajor ? (k.N + chunk_n - 1) / chunk_n * chunk_n : k.N;
+  const bool small = k.M <= kTileM && small_cycles(plan, k, b_pad) > 0;
   const bool a_pass = presplit && k.M > kTileM;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
@@ -1366,13 +1373,18 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   st->grid = p.splits > 1 ? dim3((unsigned)p.num_units, 1, 1)     // one unit per CTA, clusters of `splits`
                           : dim3((unsigned)(p.num_units < plan.sm_count ? p.num_units : plan.sm_count), 1, 1);
 
+  const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor, st->b_copy.once};
+  if (small) {
+    const int rc = small_bind(plan, k, kernel_index, po, st->b_tail, &st->small);
+    if (rc) return rc;
+    if (st->small) return KB200_OK;
+  }
   // More than 128 rows: 256-row tiles on SM pairs (matmul_pair.cu) when that kernel covers the epilogue.
   if (st->pair) {
     pair_destroy(st->pair);
     st->pair = nullptr;
   }
   if (pair_eligible(plan, k, b_map_cols)) {
-    const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor, st->b_copy.once};
     const int rc = pair_bind(plan, k, kernel_index, po, &st->pair);
     if (rc) return rc;
     if (st->pair) return KB200_OK;
@@ -1435,6 +1447,7 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     KB200_CUDA(launch_kernel(plan.pdl, tail_rows_kernel, dim3(cvt_grid(k.M * ((k.K + 3) / 4), cap)), dim3(256), 0, s, src, st->a_tail, (uint32_t)k.M,
                              (uint32_t)k.K, row, st->tail_pitch));
   }
+  if (st->small) return small_launch(plan, st->small, s);
   if (st->pair) return pair_launch(plan, st->pair, s);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = st->grid;
@@ -1474,6 +1487,7 @@ bool tc_repoint(PlanKernel& k) {
   for (int o = 0; o < k.n_ops; ++o) st->params.mm.ops[o].ptr = k.ops[o].ptr;
   const void* a = st->bf16 || st->a_copy.data ? nullptr : k.ops[d.a_slot].ptr;
   const void* b = st->bf16 || st->b_copy.data ? nullptr : k.ops[d.b_slot].ptr;
+  if (st->small) return small_repoint(k, st->small);
   if (st->pair) return pair_repoint(k, st->pair, a, b);
   bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b));
   if (st->params.store_mode == 1) ok = ok && set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr);
@@ -1485,6 +1499,7 @@ void tc_destroy(PlanKernel& k) {
   if (!st) return;
   drop_copies(st);
   if (st->pair) pair_destroy(st->pair);
+  if (st->small) small_destroy(st->small);
   delete st;
   k.tc = nullptr;
 }

@@ -73,3 +73,17 @@ def test_both_fp32_attention_kernels_take_any_length(tokens, choice, monkeypatch
 def test_linear_of_any_size(m, n, k, precision):
     """Operand rows off a 16-byte pitch, widths off a 128-byte column chunk, tiles with one row or column."""
     check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(2, 64, 64), (128, 64, 4096), (127, 68, 1000), (128, 3072, 768), (100, 768, 3072), (17, 2304, 96), (128, 4096, 128),
+                                   (65, 1028, 3000)])
+def test_few_tiles(m, n, k, precision):
+    """One row of tiles: K split over 1 to 8 CTAs, K ranges longer and shorter than the ring, ragged last slabs."""
+    check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("tokens,d", [(3, 132), (64, 512), (128, 1024), (129, 260)])
+def test_mlp_of_few_tokens(tokens, d, precision):
+    check({"kind": "mlp", "tokens": tokens, "d": d, "precision": precision}, ["mm_tcgen05"], calls=2)
