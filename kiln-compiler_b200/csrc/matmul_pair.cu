@@ -256,16 +256,19 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // A frozen B is nobody's output: the first stages' weights are requested before the wait for the
   // previous kernel, so that they are on their way, or here, when the activations are ready.
   const uint32_t full_leader0 = map_to_cta(full0, 0);
-  int ahead = 0;                 // stages of the first tile whose B is requested already (producer thread)
-  if (p.b_static && threadIdx.x == 0 && pair < p.num_tiles) {
+  int ahead = 0;                 // stages of the first tile whose B is requested already (producer warp)
+  if (p.b_static && warp == 0 && pair < p.num_tiles) {
     const int batch = pair_div(pair, p.magic_tpb);
     const int rem = pair - batch * p.tiles_per_batch;
     const int n_col = (rem - pair_div(rem, p.magic_tn) * p.tiles_n) * p.bn + (int)rank * p.half_bn;
     ahead = p.stages < p.num_kb ? p.stages : p.num_kb;
-    for (int s = 0; s < ahead; ++s) {
-      if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
-      load_b_pair<KPS>(p, &tma_b, tiles + (uint32_t)(s * stage_bytes + a_stage_bytes), full_leader0 + 8 * s, s * p.step_k, n_col, batch);
+    if (elect_one()) {
+      for (int s = 0; s < ahead; ++s) {
+        if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
+        load_b_pair<KPS>(p, &tma_b, tiles + (uint32_t)(s * stage_bytes + a_stage_bytes), full_leader0 + 8 * s, s * p.step_k, n_col, batch);
+      }
     }
+    __syncwarp();
   }
   // Everything above may have overlapped the previous kernel's tail; from here on its output is read.
   pdl_wait();
@@ -276,52 +279,53 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, slab_k = p.slab_k, step_k = p.step_k;
-      constexpr int kps = KPS;
-      const int bn = p.bn, half_bn = p.half_bn;
-      const uint32_t tx_bytes = (uint32_t)stage_bytes;
-      int s = 0;
-      uint32_t wait_parity = 1;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int batch = pair_div(tile, p.magic_tpb);
-        const int rem = tile - batch * p.tiles_per_batch;
-        const int tm_i = pair_div(rem, p.magic_tn);
-        const int tn_i = rem - tm_i * p.tiles_n;
-        const int m_row = tm_i * 256 + (int)rank * 128;
-        const int n_col = tn_i * bn + (int)rank * half_bn;
-        int k_elem = 0;
-        for (int kb = 0; kb < num_kb; ++kb, k_elem += step_k) {
-          if (!mbar_wait_cluster(empty0 + 8 * s, wait_parity, abort_ptr)) {
-            if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 1); *abort_ptr = 1; }
-            ok = false;
-            break;
-          }
-          // the leader's barrier counts the bytes of both CTAs (the peer's may land first: the phase
-          // cannot complete before this arrival)
-          PAIR_STAMP(0, tp);
-          const bool b_here = ahead > 0;           // expected and requested above
-          if (!b_here && rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * tx_bytes);
-          const uint32_t bar = full_leader0 + 8 * s;
-          const uint32_t dst = tiles + (uint32_t)(s * stage_bytes);
-          for (int j = 0; j < kps; ++j) tma_load_3d_pair(dst + j * kPairATileBytes, &tma_a, bar, k_elem + j * slab_k, m_row, batch);
-          if (b_here) --ahead;
-          else load_b_pair<KPS>(p, &tma_b, dst + a_stage_bytes, bar, k_elem, n_col, batch);
-          PAIR_STAMP(1, tp);
-#ifdef KB200_TRACE
-          ++tp;
-#endif
-          if (++s == stages) { s = 0; wait_parity ^= 1; }
+    // (like the MMA issuer's, a role that the whole warp walks, one lane issuing: see elect_one)
+    const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, slab_k = p.slab_k, step_k = p.step_k;
+    const int bn = p.bn, half_bn = p.half_bn;
+    int s = 0;
+    uint32_t wait_parity = 1;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      const int batch = pair_div(tile, p.magic_tpb);
+      const int rem = tile - batch * p.tiles_per_batch;
+      const int tm_i = pair_div(rem, p.magic_tn);
+      const int tn_i = rem - tm_i * p.tiles_n;
+      const int m_row = tm_i * 256 + (int)rank * 128;
+      const int n_col = tn_i * bn + (int)rank * half_bn;
+      int k_elem = 0;
+      for (int kb = 0; kb < num_kb; ++kb, k_elem += step_k) {
+        const bool got = mbar_wait_cluster(empty0 + 8 * s, wait_parity, abort_ptr);
+        if (!__all_sync(0xffffffffu, got ? 1 : 0)) {
+          if (lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 1); *abort_ptr = 1; }
+          ok = false;
+          break;
         }
+        // the leader's barrier counts the bytes of both CTAs (the peer's may land first: the phase
+        // cannot complete before this arrival)
+        PAIR_STAMP(0, tp);
+        const bool b_here = ahead > 0;           // expected and requested above
+        const uint32_t bar = full_leader0 + 8 * s;
+        const uint32_t dst = tiles + (uint32_t)(s * stage_bytes);
+        if (elect_one()) {
+          if (!b_here && rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
+#pragma unroll
+          for (int j = 0; j < KPS; ++j) tma_load_3d_pair(dst + j * kPairATileBytes, &tma_a, bar, k_elem + j * slab_k, m_row, batch);
+          if (!b_here) load_b_pair<KPS>(p, &tma_b, dst + a_stage_bytes, bar, k_elem, n_col, batch);
+        }
+        __syncwarp();
+        if (b_here) --ahead;
+        PAIR_STAMP(1, tp);
+#ifdef KB200_TRACE
+        ++tp;
+#endif
+        if (++s == stages) { s = 0; wait_parity ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA) ----------------
-    // A lone thread pays full latency for every instruction: ~60 cycles per tcgen05.mma, ~100 per
-    // commit, whatever the tile size.  So a step is one barrier probe, 4 * KPS MMAs whose descriptor
-    // words advance by additions, and ONE commit for both CTAs.
-    if (lane == 0 && rank == 0) {
+    // A step is one barrier probe, 4 * KPS MMAs whose descriptor words advance by additions, and ONE commit
+    // for both CTAs (a commit costs about as much as two MMAs).
+    if (rank == 0) {
       const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, bn = p.bn;
       const uint32_t idesc = p.idesc;
       const uint64_t a_fixed = make_desc(0, 16, 1024);
@@ -340,46 +344,36 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         const int acc = i & 1;
         const uint32_t aph = (i >> 1) & 1;
         // both CTAs' epilogue warps have drained this accumulator (two tiles ago)
-        if (!mbar_wait_cluster(tempty0 + 8 * acc, aph ^ 1, abort_ptr)) {
-          if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 4); *abort_ptr = 1; }
+        const bool drained = mbar_wait_cluster(tempty0 + 8 * acc, aph ^ 1, abort_ptr);
+        if (!__all_sync(0xffffffffu, drained ? 1 : 0)) {
+          if (lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 4); *abort_ptr = 1; }
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_d = tmem_base + (uint32_t)(acc * bn);
-        uint32_t accumulate = 0;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) {
-            if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 2); *abort_ptr = 1; }
+          const bool landed = mbar_wait(full0 + 8 * s, parity, abort_ptr);
+          if (!__all_sync(0xffffffffu, landed ? 1 : 0)) {
+            if (lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 2); *abort_ptr = 1; }
             ok = false;
             break;
           }
           PAIR_STAMP(2, tq);
-#ifdef KB200_TRACE
-          long long fine[6];
-          fine[0] = clock64();
-#endif
+          if (elect_one()) {
 #pragma unroll
-          for (int j = 0; j < KPS; ++j) {
+            for (int j = 0; j < KPS; ++j) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t adesc = ((uint64_t)a_hi << 32) | (a_lo_fixed | ((a16 + (uint32_t)(j * (kPairATileBytes >> 4) + 2 * k)) & 0x3FFFu));
-              const uint64_t bdesc = ((uint64_t)b_hi << 32) | (b_lo_fixed | ((b16 + (uint32_t)j * b_slab16 + (uint32_t)k * b_step16) & 0x3FFFu));
-#ifdef KB200_TRACE
-              if (!(p.debug & 32))
-#endif
-              umma_pair<BF16>(tmem_d, adesc, bdesc, idesc, accumulate);
-              accumulate = 1;
-#ifdef KB200_TRACE
-              if (j == 0) fine[1 + k] = clock64();
-#endif
+              for (int k = 0; k < 4; ++k) {
+                const uint64_t adesc = ((uint64_t)a_hi << 32) | (a_lo_fixed | ((a16 + (uint32_t)(j * (kPairATileBytes >> 4) + 2 * k)) & 0x3FFFu));
+                const uint64_t bdesc = ((uint64_t)b_hi << 32) | (b_lo_fixed | ((b16 + (uint32_t)j * b_slab16 + (uint32_t)k * b_step16) & 0x3FFFu));
+                umma_pair<BF16>(tmem_d, adesc, bdesc, idesc, (kb | j | k) != 0 ? 1u : 0u);
+              }
             }
+            // the stage is free in both CTAs once these MMAs have read it
+            umma_pair_commit(empty0 + 8 * s);
+            if (kb + 1 == num_kb) umma_pair_commit(tfull0 + 8 * acc);
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          umma_pair_commit(empty0 + 8 * s);
-#ifdef KB200_TRACE
-          fine[5] = clock64();
-          (void)fine;
-#endif
+          __syncwarp();
           PAIR_STAMP(3, tq);
 #ifdef KB200_TRACE
           ++tq;
@@ -388,7 +382,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           b16 += stage16;
           if (++s == stages) { s = 0; parity ^= 1; a16 = a_first; b16 = b_first; }
         }
-        if (ok) umma_pair_commit(tfull0 + 8 * acc);
       }
     }
   } else if (warp >= kPairFirstEpiWarp && warp < kPairFirstEpiWarp + kPairEpiWarps) {
@@ -695,7 +688,7 @@ bool classify_steps(const PlanKernel& k, PairParams* p, const DevOperand** res_o
 
 }  // namespace
 
-bool pair_eligible(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
+bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
   if (d.precision == KB200_PREC_FP32 || !k.has_chain) return false;
   if (d.cfg[0] == 128) return false;                       // the tuner asked for single-CTA tiles
@@ -703,9 +696,7 @@ bool pair_eligible(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
   if (plan.sm_count < 2) return false;
   const bool bf16 = d.precision == KB200_PREC_BF16;
   const int chunk_n = bf16 ? 64 : 32;
-  const DevOperand& B = k.ops[d.b_slot];
-  const bool b_nmajor = B.stride[2] == 1;
-  if (k.N < 128 || k.N % 4 || (b_nmajor && b_cols % chunk_n)) return false;
+  if (k.N < 128 || k.N % 4 || (!b_kmajor && b_cols % chunk_n)) return false;
   if (d.cfg[4] > 1) return false;                          // a forced split-K runs on the single-CTA kernel
   if (d.cfg[7] == 1 || d.cfg[7] == 2) return false;        // so do its epilogue variants
   if (((k.M + 255) / 256) * ((k.N + 127) / 128) * k.batch >= (int64_t(1) << 20)) return false;

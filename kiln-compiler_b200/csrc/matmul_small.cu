@@ -8,10 +8,9 @@
 // from a cold cache on top of its latencies.  So:
 //   * K is split over the CTAs of a thread-block cluster until the SMs are used, and the whole K range of
 //     a CTA is in flight at once where shared memory holds it;
-//   * the partial tiles are exchanged straight from registers: the thread that reads a row of the
-//     accumulator writes it with st.async into the CTA that finishes that row's band, data and arrival
-//     count in one operation.  (matmul_tc.cu parks the tile in shared memory first and pushes bands
-//     with bulk copies; parking, the barrier behind it and the pushes took ~6000 cycles of a launch.)
+//   * every warp sends the rows it has read from the accumulator to the CTA that finishes their band as
+//     soon as it has staged them, data and arrival count in one bulk copy.  (matmul_tc.cu parks the whole
+//     tile, passes a barrier and pushes bands: ~6000 cycles of a launch.)
 //   * the epilogue is written for its chain, over float4 items in row order: bias and residual are
 //     fetched before the accumulator is ready, stores cover whole lines;
 //   * weights are requested before the wait for the previous kernel.
@@ -66,12 +65,6 @@ struct SmallParams {
   int64_t out_row;                 // of both
 };
 
-__device__ __forceinline__ void st_async(uint32_t addr, uint32_t bar, float4 v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-               ::"r"(addr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(bar)
-               : "memory");
-}
-
 template <int MODE, int FIN>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -85,7 +78,11 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   __shared__ int abort_flag;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
-  const uint32_t recv = ring + (uint32_t)(p.stages * kStage);   // [split][128 / splits rows][64 floats], 16-byte units XORed with the row
+  // This CTA's partial tile, a 4 KB block per warp: in the ring, idle by then, where it is large enough
+  const bool in_ring = p.stages * kStage >= kSmallExchange;
+  const uint32_t recv = in_ring ? ring : ring + (uint32_t)(p.stages * kStage);
+  // A cluster: the others' parts of this CTA's band
+  const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kSmallExchange);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
   const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8;
@@ -104,7 +101,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     mbar_init(done, 1);
     mbar_init(received, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(received, kSmallExchange);                   // (an arrival, too; a launch without a split does not use it)
+    mbar_expect_tx(received, (uint32_t)(kSmallExchange / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
   if (threadIdx.x == 32) {
     prefetch_tensormap(&tma_a);
@@ -123,8 +120,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   // CTAs must not take tensor memory that this one still has to allocate.
   pdl_launch_dependents();
   // Every CTA's barriers exist once all have arrived here; waited for in front of the exchange.  A launch
-  // without a split is no cluster launch and keeps off every cluster instruction (st.async in one is
-  // an illegal instruction).
+  // without a split is no cluster launch and keeps off the cluster instructions (a store to a mapped
+  // address in one is an illegal instruction).
   const bool clustered = p.splits > 1;
   if (clustered) cluster_arrive();
   const uint32_t tmem = tmem_slot;
@@ -135,15 +132,20 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   // a frozen B is nobody's output: its producer does not wait for the previous kernel
   if (!(warp == 10 && p.b_static)) pdl_wait();
 
+  // A whole warp walks each of the three roles below; its waits end for all lanes or none.
+  auto all_waited = [&](bool got, int site) {
+    if (!got && lane == 0) give_up(site);
+    return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
+  };
   if (warp == 0 || warp == 10) {
     // ---------------- TMA producers, one per operand ----------------
-    if (lane == 0) {
-      const bool is_a = warp == 0;
-      int s = 0, k_elem = slab0 * p.slab_k;
-      uint32_t parity = 1;
-      for (int i = 0; i < n_slabs; ++i, k_elem += p.slab_k) {
-        if (!mbar_wait(empty0 + 8 * s, parity, abort_ptr)) { give_up(1); break; }
-        const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage);
+    const bool is_a = warp == 0;
+    int s = 0, k_elem = slab0 * p.slab_k;
+    uint32_t parity = 1;
+    for (int i = 0; i < n_slabs; ++i, k_elem += p.slab_k) {
+      if (i >= p.stages && !all_waited(mbar_wait(empty0 + 8 * s, parity, abort_ptr), 1)) break;
+      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage);
+      if (elect_one()) {
         if (is_a) {
           mbar_expect_tx(bar, kSmallABytes);
           tma_load_3d(dst, &tma_a, bar, k_elem, tm * kSmallM, 0);
@@ -157,24 +159,26 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             else tma_load_4d(at, map, bar, 0, k_elem, tn * (kSmallN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
           }
         }
-        if (++s == p.stages) { s = 0; parity ^= 1; }
       }
+      __syncwarp();
+      if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint64_t a_fixed = make_desc(0, 16, 1024);
-      const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
-      const uint32_t b_step = p.b_step16, idesc = p.idesc;
-      int s = 0, rot = 0;
-      uint32_t parity = 0;
-      bool ok = true;
-      for (int i = 0; i < n_slabs; ++i) {
-        if (!mbar_wait((EXACT ? split0 : full0) + 8 * s, parity, abort_ptr)) { give_up(2); ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a16 = (ring + (uint32_t)(s * kStage)) >> 4, b16 = a16 + (kSmallABytes >> 4);
-        // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
-        auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
+    const uint64_t a_fixed = make_desc(0, 16, 1024);
+    const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
+    const uint32_t b_step = p.b_step16, idesc = p.idesc;
+    int s = 0, rot = 0;
+    uint32_t parity = 0;
+    bool ok = true;
+    for (int i = 0; i < n_slabs && ok; ++i) {
+      ok = all_waited(mbar_wait((EXACT ? split0 : full0) + 8 * s, parity, abort_ptr), 2);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t a16 = (ring + (uint32_t)(s * kStage)) >> 4, b16 = a16 + (kSmallABytes >> 4);
+      // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
+      auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t a = a16 + 2 * k, b = b16 + k * b_step;
@@ -189,11 +193,12 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             umma(tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
           }
         }
-        if (EXACT && ++rot == p.nacc) rot = 0;
         if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
-        if (++s == p.stages) { s = 0; parity ^= 1; }
+        if (i + 1 == n_slabs) umma_commit(done);
       }
-      if (ok) umma_commit(done);
+      __syncwarp();
+      if (EXACT && ++rot == p.nacc) rot = 0;
+      if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else {
     // ---------------- warps 2..9 ----------------
@@ -254,53 +259,79 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           for (int j = 0; j < 32; ++j) v[j] += w[j];
         }
       }
-      const int row = quad * 32 + lane;
+      // This warp's 32 x 32 block goes to the CTA that finishes its rows (two CTAs, 16 rows each, with eight
+      // splits): staged in 128-byte rows, the 16-byte unit XORed with the row, then one bulk copy per
+      // destination that carries its arrival.  The blocks of this CTA's own band stay where they are
+      // staged: its own part of the exchange area.  (st.async straight from the registers, 16 bytes per
+      // lane and packet, took 3700 cycles to land where these take ~1500.)
+      const uint32_t block = (uint32_t)(e * 4096);
+      uint8_t* const mine = smem_raw + (recv - raw) + block + lane * 128;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(mine + ((q ^ (lane & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       if (clustered) {
-        // this row's half goes to the CTA that finishes its band
-        const int dest = row / band_rows, r = row - dest * band_rows;
-        const uint32_t to = map_to_cta(recv + (uint32_t)((rank * band_rows + r) * 256 + half * 128), (uint32_t)dest);
-        const uint32_t bar = map_to_cta(received, (uint32_t)dest);
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          st_async(to + (uint32_t)((q ^ (r & 7)) << 4), bar, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
-      } else {
-        uint8_t* const to = smem_raw + (recv - raw) + row * 256 + half * 128;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<float4*>(to + ((q ^ (row & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        fence_async_smem();
+        __syncwarp();
+        const int pieces = band_rows < 32 ? 2 : 1, rows = band_rows < 32 ? 16 : 32;
+        if (lane < pieces) {
+          const int row = quad * 32 + lane * rows, dest = row / band_rows;
+          if (dest != rank) {
+            // in the destination's area: [source][half][row of the band]
+            const uint32_t to = parts0 + (uint32_t)((rank * 2 + half) * band_rows + (row - dest * band_rows)) * 128u;
+            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(map_to_cta(to, (uint32_t)dest)), "r"(recv + block + (uint32_t)(lane * rows * 128)), "r"((uint32_t)(rows * 128)),
+                           "r"(map_to_cta(received, (uint32_t)dest))
+                         : "memory");
+          }
+        }
       }
     }
     __syncwarp();
-    if (!clustered) asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight warps
-    else if (!mbar_wait_cluster(received, 0, abort_ptr)) give_up(5);
-    __syncwarp();
+    if (clustered) {
+      if (!mbar_wait_cluster(received, 0, abort_ptr)) give_up(5);
+      __syncwarp();
+      cluster_arrive_relaxed();
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight warps have staged this CTA's own part
     ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
     if (ok) {
-      const uint8_t* const parts = smem_raw + (recv - raw);
+      // Item j of this thread: row (t / 16) + 16 j of the band, float4 number t % 16.  All loads before the sums,
+      // all sums before the stores: the latencies of an item's few steps are what a lone item pays.
+      const int u = t & 15, h = u >> 3;
+      float4 a[8];
+      const uint8_t* const area = smem_raw + (parts0 - raw);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = (t >> 4) + 16 * j;
+        a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (16 * j < band_rows) {
+          for (int s = 0; s < p.splits; ++s) {
+            // the own part lies in the staging blocks: block of (row / 32, half)
+            const int row = band0 + r;
+            const uint8_t* src = s == rank ? smem_raw + (recv - raw) + (h * 4 + (((row >> 5) + 2) & 3)) * 4096 + (row & 31) * 128
+                                           : area + ((s * 2 + h) * band_rows + r) * 128;
+            const float4 b = *reinterpret_cast<const float4*>(src + (((u ^ r) & 7) << 4));
+            a[j].x += b.x; a[j].y += b.y; a[j].z += b.z; a[j].w += b.w;
+          }
+        }
+      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int r = (t >> 4) + 16 * j, m = m0 + band0 + r;
-        if (r >= band_rows) break;
-        const int u = t & 15;
-        const uint8_t* src = parts + r * 256 + (((u & 8) | ((u ^ r) & 7)) << 4);
-        float4 a = *reinterpret_cast<const float4*>(src);
-        for (int s = 1; s < p.splits; ++s) {
-          const float4 b = *reinterpret_cast<const float4*>(src + s * band_rows * 256);
-          a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-        }
-        if (m >= p.M || n >= p.N) continue;
-        if (FIN != FIN_NONE) { a.x += bias.x; a.y += bias.y; a.z += bias.z; a.w += bias.w; }
+        if (16 * j >= band_rows || m >= p.M || n >= p.N) continue;
+        float4 y = a[j];
+        if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
         if (FIN == FIN_BIAS_GELU) {
           if (MODE == SMALL_BF16) {
-            a.x = f_gelu_tanh_approx(a.x); a.y = f_gelu_tanh_approx(a.y); a.z = f_gelu_tanh_approx(a.z); a.w = f_gelu_tanh_approx(a.w);
+            y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
           } else {
-            a.x = d_gelu_tanh(a.x); a.y = d_gelu_tanh(a.y); a.z = d_gelu_tanh(a.z); a.w = d_gelu_tanh(a.w);
+            y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
           }
         }
-        if (FIN == FIN_BIAS_RES) { a.x += res[j].x; a.y += res[j].y; a.z += res[j].z; a.w += res[j].w; }
-        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = a;
+        if (FIN == FIN_BIAS_RES) { y.x += res[j].x; y.y += res[j].y; y.z += res[j].z; y.w += res[j].w; }
+        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
         if (p.out16 != nullptr) {
-          __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+          __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
           uint2 packed;
           packed.x = *reinterpret_cast<uint32_t*>(&lo);
           packed.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -309,9 +340,12 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       }
     }
   }
-  // The roles above ran in one lane: the warp has to be whole again for an .aligned barrier.
+  // (the warp has to be whole for an .aligned barrier)
   __syncwarp();
-  if (clustered && (warp < 2 || warp == 10)) cluster_wait();       // (the other warps have passed this phase above)
+  if (clustered && (warp < 2 || warp == 10)) {
+    cluster_wait();       // (the other warps have passed this phase above)
+    cluster_arrive_relaxed();
+  }
   // ---------------- exit ----------------
   if (abort_flag && threadIdx.x == 0) {
     // copies may still be in flight towards this CTA's shared memory: give them a bounded time to land
@@ -320,11 +354,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  // A CTA that has received everything is written to no more.  One that gave up stays until the others of its cluster have left or given up too.
-  if (clustered && abort_flag) {
-    cluster_arrive();
-    cluster_wait();
-  }
+  // Every CTA of the cluster has received everything: so every copy out of THIS shared memory has landed
+  if (clustered) cluster_wait();
   if (warp == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)p.tmem_cols) : "memory");
@@ -421,7 +452,7 @@ SmallPlan plan_small(int64_t tiles, int64_t slabs, int mode, int sm_count) {
 
 }  // namespace
 
-int64_t small_cycles(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
   const bool bf16 = d.precision == KB200_PREC_BF16;
   int bias_slot, res_slot;
@@ -429,8 +460,7 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, int64_t b_cols) {
   for (int i : {0, 1, 2, 3, 4, 6})
     if (d.cfg[i] != 0) return -1;                     // a tile, stage or split was asked for (how to store is not a question here)
   if (k.M >= (1 << 20) || k.N >= (1 << 24) || k.N % 4) return -1;
-  const DevOperand& B = k.ops[d.b_slot];
-  if (B.stride[2] == 1 && b_cols % (bf16 ? 64 : 32)) return -1;
+  if (!b_kmajor && b_cols % (bf16 ? 64 : 32)) return -1;
   if (d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind != KB200_BASE_CONST) return -1;
   const DevOperand& O = k.ops[k.chain.out_slot];
   if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
@@ -457,8 +487,10 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   const int stage_bytes = (mode == SMALL_EXACT ? 2 : 1) * (kSmallABytes + kSmallBBytes);
   const int most = (p.num_slabs + p.splits - 1) / p.splits;
   p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
-  while ((size_t)p.stages * stage_bytes + kSmallExchange + 1024 > (size_t)kSmallSmem) --p.stages;
-  st->smem = (size_t)p.stages * stage_bytes + kSmallExchange + 1024;
+  auto exchange_of = [&](int stages) { return (p.splits > 1 ? kSmallExchange : 0) + (stages * stage_bytes >= kSmallExchange ? 0 : kSmallExchange); };
+  while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
+  const int exchange = exchange_of(p.stages);
+  st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
   st->grid = (unsigned)(tiles * p.splits);
   p.b_kmajor = ops.b_kmajor ? 1 : 0;
   p.b_static = ops.b_static ? 1 : 0;

@@ -7,7 +7,7 @@
 namespace kb200 {
 
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
-int64_t small_cycles(const Plan& plan, const PlanKernel& k, int64_t b_cols);
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols);
 // Tensor maps and launch parameters.  `b_tail`: exact FP32, the tails of B in the layout of ops.b_base.
 // *state stays null when the operands cannot be described; a non-zero return is an error.
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, void** state);

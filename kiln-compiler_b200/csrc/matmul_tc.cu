@@ -997,6 +997,18 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict_
   }
 }
 
+// A frozen [K, N] weight as [N, K] rows of `pitch` elements, zeros behind the last: once, at bind.
+template <typename T>
+__global__ void __launch_bounds__(256) transpose_rows_kernel(const float* __restrict__ src, T* __restrict__ dst, int K, int N, int64_t s_row,
+                                                             int64_t pitch) {
+  __shared__ float tile[32][33];
+  const int k0 = blockIdx.x * 32, n0 = blockIdx.y * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int j = y; j < 32; j += 8) tile[j][x] = k0 + j < K && n0 + x < N ? src[(int64_t)(k0 + j) * s_row + n0 + x] : 0.0f;
+  __syncthreads();
+  for (int j = y; j < 32; j += 8)
+    if (n0 + j < N && k0 + x < pitch) dst[(int64_t)(n0 + j) * pitch + k0 + x] = T(tile[x][j]);
+}
+
 // tail[r][c] = what the tensor core's 19 leading bits leave of src[r][c]: the second TF32 terms of an
 // exact-FP32 operand.  Rows 16-byte aligned; the floats that fill a last vector are multiplied with nothing.
 __global__ void __launch_bounds__(256) tail_rows_kernel(const float* __restrict__ src, float* __restrict__ tail, uint32_t rows, uint32_t cols,
@@ -1050,6 +1062,7 @@ struct TcState {
     void* data = nullptr;
     int64_t rows = 0, cols = 0, pitch = 0;    // of one batch entry, in elements of the copy
     bool once = false;                        // of a frozen constant: made at bind, not per launch
+    bool turned = false;                      // ... of an N-contiguous B, as rows along K
   } a_copy, b_copy;
   // exact FP32 with a frozen B: the operands' tails (see tail_rows_kernel), [M, tail_pitch] and like B's map
   float* a_tail = nullptr;
@@ -1104,6 +1117,14 @@ bool rows_describable(const DevOperand& o, int64_t row_stride, int64_t batch) {
 
 cudaError_t launch_copy(const TcState::Copy& c, bool bf16, const DevOperand& o, int64_t row_stride, int64_t batch, int64_t cap, bool pdl,
                         cudaStream_t s) {
+  if (c.turned) {
+    const dim3 grid((unsigned)((c.pitch + 31) / 32), (unsigned)((c.rows + 31) / 32));
+    if (bf16)
+      return launch_kernel(pdl, transpose_rows_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, (const float*)o.ptr, static_cast<__nv_bfloat16*>(c.data),
+                           (int)c.cols, (int)c.rows, row_stride, c.pitch);
+    return launch_kernel(pdl, transpose_rows_kernel<float>, grid, dim3(256), 0, s, (const float*)o.ptr, static_cast<float*>(c.data), (int)c.cols,
+                         (int)c.rows, row_stride, c.pitch);
+  }
   const int64_t units = batch * c.rows * (c.pitch / 4);
   if (bf16 && c.pitch == c.cols && rows_describable(o, row_stride, batch))
     return launch_kernel(pdl, cvt_bf16_kernel, dim3(cvt_grid(units, cap)), dim3(256), 0, s, (const float*)o.ptr,
@@ -1134,8 +1155,12 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // Operands as the tensor maps see them: A [M, K]; B [K, N] (N contiguous) or [N, K] (K contiguous)
   const DevOperand& A = k.ops[d.a_slot];
   const DevOperand& B = k.ops[d.b_slot];
-  const bool b_kmajor = B.stride[2] != 1;
-  const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = b_kmajor ? B.stride[2] : B.stride[1];
+  // A frozen B is laid out along K once: both operands then use the ordinary 128-byte swizzle, and a tile may
+  // have any width (an N-major one comes in whole 128-byte column chunks).
+  const bool frozen = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
+  const bool turn = frozen && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
+  const bool b_kmajor = turn || B.stride[2] != 1;
+  const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = B.stride[2] != 1 ? B.stride[2] : B.stride[1];
   const void* a_base = A.ptr;
   const void* b_base = B.ptr;
   int64_t a_row = A.stride[1], a_batch = A.stride[0], b_row = b_src_row, b_batch = B.stride[0];
@@ -1149,11 +1174,12 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // bytes a clock.
   if (st->small) small_destroy(st->small);
   st->small = nullptr;
-  const bool presplit = d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind == KB200_BASE_CONST && k.batch == 1;
-  st->b_copy.once = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
+  const bool presplit = d.precision == KB200_PREC_FP32 && frozen && k.batch == 1;
+  st->b_copy.once = frozen;
+  st->b_copy.turned = turn;
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
   const bool copy_b = st->bf16 ? k.b_shadow == nullptr
-                               : !rows_describable(B, b_row, k.batch) || (st->b_copy.once && !b_kmajor && k.N % 4 == 0 && k.N % chunk_n != 0);
+                               : turn || !rows_describable(B, b_row, k.batch);
   const int unit = st->bf16 ? 8 : 4, esz = st->bf16 ? 2 : 4;
   auto make_copy = [&](TcState::Copy& c, int64_t rows, int64_t cols, int64_t to) {
     c.rows = rows;
@@ -1183,8 +1209,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     b_base = k.b_shadow;
   }
   // Few tiles: the kernel written for latency.
-  const int64_t b_pad = st->b_copy.once && copy_b && !b_kmajor ? (k.N + chunk_n - 1) / chunk_n * chunk_n : k.N;
-  const bool small = k.M <= kTileM && small_cycles(plan, k, b_pad) > 0;
+  const bool small = k.M <= kTileM && small_cycles(plan, k, b_kmajor, b_map_cols) > 0;
   const bool a_pass = presplit && k.M > kTileM;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
@@ -1384,7 +1409,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     pair_destroy(st->pair);
     st->pair = nullptr;
   }
-  if (pair_eligible(plan, k, b_map_cols)) {
+  if (pair_eligible(plan, k, b_kmajor, b_map_cols)) {
     const int rc = pair_bind(plan, k, kernel_index, po, &st->pair);
     if (rc) return rc;
     if (st->pair) return KB200_OK;

@@ -113,6 +113,16 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t addr, uint32_t lbo_bytes,
   return d;
 }
 
+// One lane of a converged warp.  A role that a whole warp walks, with only its tcgen05 and copy instructions in
+// the elected lane, keeps addresses and descriptors in uniform registers; walked by one lane alone it
+// moves every descriptor word over for every instruction (765 cycles per four MMAs and their wait
+// instead of ~350, measured in matmul_small.cu).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on));
+  return on != 0;
+}
+
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
                                      bool bf16) {
   if (bf16) {
@@ -229,6 +239,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // ---- thread-block clusters ----
 // The two halves of the hardware cluster barrier, usable apart: arrive early, wait when the result is needed.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// (orders nothing: for a barrier that only says "this far")
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta); orders this thread's
 // earlier writes -- and, through a preceding CTA barrier, its CTA's -- before the arrival, cluster-wide.
