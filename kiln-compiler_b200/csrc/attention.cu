@@ -445,9 +445,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
 #ifdef KB200_TRACE
   __shared__ long long trace[4][16];
-  __shared__ long long mma_trace[64];
   __shared__ long long marks[4];
-  int tm = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     unsigned long long g;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
@@ -455,16 +453,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     marks[1] = clock64();
   }
 #define ATTN_STAMP(role, idx) do { if (blockIdx.x == 0 && threadIdx.x == 64 && (idx) < 16) trace[role][idx] = clock64(); } while (0)
-#define ATTN_MMA_STAMP(idx) do { if (blockIdx.x == 0 && (idx) < 64) mma_trace[idx] = clock64(); } while (0)
 #else
 #define ATTN_STAMP(role, idx) do { } while (0)
-#define ATTN_MMA_STAMP(idx) do { } while (0)
 #endif
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t q_smem = (raw + 1023u) & ~1023u;
   const uint32_t k_smem = q_smem + (EXACT ? kOpBytes : kTileBytes);   // ring of 2 tiles | EXACT: one buffer (tile, then its tails)
   const uint32_t v_smem = k_smem + 2 * kTileBytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // bars (EXACT uses only the first of each K / V pair): 0 q_full | 1,2 k_full | 3,4 k_empty | 5,6 v_full | 7,8 v_empty | 9,10 s_full |
   //       11..14 p_full[group][s buffer] | 15..18 o_full[group][o buffer] | 19 q_empty
   const uint32_t q_full = smem_u32(&bars[0]), k_full = smem_u32(&bars[1]), k_empty = smem_u32(&bars[3]);
@@ -560,164 +556,138 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
   };
 
+  // A whole warp walks each of the two roles below, one lane issuing (see elect_one); its waits end for all
+  // lanes or none.
+  auto all_waited = [&](bool got, int site) {
+    if (!got && lane == 0) give_up(site);
+    return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
+  };
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int t = 0;                                     // key tiles loaded so far, over all items
-      bool ok = true;
-      for (int ii = 0; ok; ++ii) {
-        const int w = nth_item(ii);
-        if (w < 0) break;
-        const Item it = item_of(w);
-        // the Q tile is free once every Q K^T of the previous item has been executed
-        if (!mbar_wait(q_empty, (ii & 1) ^ 1, abort_ptr)) { give_up(0x13); break; }
-        // EXACT, an operand buffer: the tile's two slabs, then the two slabs of its tails
-        [[maybe_unused]] auto load4 = [&](uint32_t dst, const CUtensorMap* heads, const CUtensorMap* tails, uint32_t bar, int t) {
-          mbar_expect_tx(bar, kOpBytes);
-          tma_load_4d(dst, heads, bar, 0, t, it.h, it.seq);
-          tma_load_4d(dst + kSlab, heads, bar, 32, t, it.h, it.seq);
-          tma_load_4d(dst + kTileBytes, tails, bar, 0, t, it.h, it.seq);
-          tma_load_4d(dst + kTileBytes + kSlab, tails, bar, 32, t, it.h, it.seq);
-        };
+    int t = 0;                                     // key tiles loaded so far, over all items
+    bool ok = true;
+    // one operand tile: its 128-byte-wide slabs, and (EXACT) those of its tails behind it
+    auto load = [&](uint32_t dst, const CUtensorMap* map, [[maybe_unused]] const CUtensorMap* tails, uint32_t bar, int token, int h, int seq) {
+      if (elect_one()) {
+        mbar_expect_tx(bar, EXACT ? kOpBytes : kTileBytes);
+        tma_load_4d(dst, map, bar, 0, token, h, seq);
+        if (!BF16) tma_load_4d(dst + kSlab, map, bar, 32, token, h, seq);
         if constexpr (EXACT) {
-          load4(q_smem, &map_q, &map_qt, q_full, it.q0);
-        } else {
-          mbar_expect_tx(q_full, kTileBytes);
-          tma_load_4d(q_smem, &map_q, q_full, 0, it.q0, it.h, it.seq);
-          if (!BF16) tma_load_4d(q_smem + kSlab, &map_q, q_full, 32, it.q0, it.h, it.seq);
+          tma_load_4d(dst + kTileBytes, tails, bar, 0, token, h, seq);
+          tma_load_4d(dst + kTileBytes + kSlab, tails, bar, 32, token, h, seq);
         }
-        for (int j = 0; j < it.n_kv; ++j, ++t) {
-          if constexpr (EXACT) {
-            const uint32_t ph = t & 1;                   // one buffer: the phase alternates with every tile
-            if (!mbar_wait(k_empty, ph ^ 1, abort_ptr)) { give_up(0x11); ok = false; break; }
-            load4(k_smem, &map_k, &map_kt, k_full, (it.j0 + j) * kRows);
-            if (!mbar_wait(v_empty, ph ^ 1, abort_ptr)) { give_up(0x12); ok = false; break; }
-            load4(v_smem, &map_v, &map_vt, v_full, (it.j0 + j) * kRows);
-          } else {
-            const int s = t & 1;
-            const uint32_t ph = (t >> 1) & 1;
-            if (!mbar_wait(k_empty + 8 * s, ph ^ 1, abort_ptr)) { give_up(0x11); ok = false; break; }
-            mbar_expect_tx(k_full + 8 * s, kTileBytes);
-            tma_load_4d(k_smem + s * kTileBytes, &map_k, k_full + 8 * s, 0, (it.j0 + j) * kRows, it.h, it.seq);
-            if (!BF16) tma_load_4d(k_smem + s * kTileBytes + kSlab, &map_k, k_full + 8 * s, 32, (it.j0 + j) * kRows, it.h, it.seq);
-            if (!mbar_wait(v_empty + 8 * s, ph ^ 1, abort_ptr)) { give_up(0x12); ok = false; break; }
-            mbar_expect_tx(v_full + 8 * s, kTileBytes);
-            tma_load_4d(v_smem + s * kTileBytes, &map_v, v_full + 8 * s, 0, (it.j0 + j) * kRows, it.h, it.seq);
-            if (!BF16) tma_load_4d(v_smem + s * kTileBytes + kSlab, &map_v, v_full + 8 * s, 32, (it.j0 + j) * kRows, it.h, it.seq);
-          }
-        }
+      }
+      __syncwarp();
+    };
+    for (int ii = 0; ok; ++ii) {
+      const int w = nth_item(ii);
+      if (w < 0) break;
+      const Item it = item_of(w);
+      // the Q tile is free once every Q K^T of the previous item has been executed
+      if (!all_waited(mbar_wait(q_empty, (ii & 1) ^ 1, abort_ptr), 0x13)) break;
+      load(q_smem, &map_q, &map_qt, q_full, it.q0, it.h, it.seq);
+      for (int j = 0; j < it.n_kv; ++j, ++t) {
+        // a ring of two tiles; EXACT: one buffer, whose phase alternates with every tile
+        const int s = EXACT ? 0 : t & 1;
+        const uint32_t ph = EXACT ? t & 1 : (t >> 1) & 1;
+        const int token = (it.j0 + j) * kRows;
+        if (!all_waited(mbar_wait(k_empty + 8 * s, ph ^ 1, abort_ptr), 0x11)) { ok = false; break; }
+        load(k_smem + s * kTileBytes, &map_k, &map_kt, k_full + 8 * s, token, it.h, it.seq);
+        if (!all_waited(mbar_wait(v_empty + 8 * s, ph ^ 1, abort_ptr), 0x12)) { ok = false; break; }
+        load(v_smem + s * kTileBytes, &map_v, &map_vt, v_full + 8 * s, token, it.h, it.seq);
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      bool ok = true;
-      // Tiles are numbered over all items (t): ring slot, S buffer and O_part buffer are t & 1, phases (t >> 1) & 1
-      // (EXACT: the single K and V buffers change phase with every tile).
-      auto issue_qk = [&](int t) {
-        const int s = t & 1;
-        if (!mbar_wait(EXACT ? k_full : k_full + 8 * s, EXACT ? (t & 1) : ((t >> 1) & 1), abort_ptr)) { give_up(0x22); ok = false; return; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t kb = EXACT ? k_smem : k_smem + s * kTileBytes;
-        // 32 bytes of the head dimension per instruction: 8 float32 (TF32) or 16 bf16
-        if constexpr (EXACT) {
-          // heads x heads, heads x tails, tails x heads
+    bool ok = true;
+    // Tiles are numbered over all items (t): ring slot, S buffer and O_part buffer are t & 1, phases (t >> 1) & 1
+    // (EXACT: the single K and V buffers change phase with every tile).
+    auto issue_qk = [&](int t, bool last_of_item) {
+      const int s = t & 1;
+      ok = all_waited(mbar_wait(EXACT ? k_full : k_full + 8 * s, EXACT ? (t & 1) : ((t >> 1) & 1), abort_ptr), 0x22);
+      if (!ok) return;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t kb = EXACT ? k_smem : k_smem + s * kTileBytes;
+      const uint32_t on = elect_one() ? 1u : 0u;
+      // 32 bytes of the head dimension per instruction: 8 float32 (TF32) or 16 bf16.
+      // EXACT: heads x heads, heads x tails, tails x heads
 #pragma unroll
-          for (int pass = 0; pass < 3; ++pass) {
-            const uint32_t qa = q_smem + (pass == 2 ? kTileBytes : 0), ka = kb + (pass == 1 ? kTileBytes : 0);
+      for (int pass = 0; pass < (EXACT ? 3 : 1); ++pass) {
+        const uint32_t qa = q_smem + (pass == 2 ? kTileBytes : 0), ka = kb + (pass == 1 ? kTileBytes : 0);
 #pragma unroll
-            for (int kd = 0; kd < kTileSlabs * 4; ++kd) {
-              const uint32_t off = (uint32_t)(kd >> 2) * kSlab + (uint32_t)(kd & 3) * 32;
-              umma(tmem_base + (uint32_t)s * 128, make_desc(qa + off, 16, 1024), make_desc(ka + off, 16, 1024), p.idesc_qk,
-                   (pass | kd) != 0 ? 1u : 0u, false);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int kd = 0; kd < kTileSlabs * 4; ++kd) {
-            const uint32_t off = (uint32_t)(kd >> 2) * kSlab + (uint32_t)(kd & 3) * 32;
-            umma(tmem_base + (uint32_t)s * 128, make_desc(q_smem + off, 16, 1024), make_desc(kb + off, 16, 1024), p.idesc_qk,
-                 kd != 0 ? 1u : 0u, BF16);
-          }
+        for (int kd = 0; kd < kTileSlabs * 4; ++kd) {
+          const uint32_t off = (uint32_t)(kd >> 2) * kSlab + (uint32_t)(kd & 3) * 32;
+          umma_if(on, tmem_base + (uint32_t)s * 128, make_desc(qa + off, 16, 1024), make_desc(ka + off, 16, 1024), p.idesc_qk,
+                  (pass | kd) != 0 ? 1u : 0u, BF16);
         }
+      }
+      if (on) {
         umma_commit(sfull0 + 8 * s);
         umma_commit(EXACT ? k_empty : k_empty + 8 * s);
-      };
-      // P V of tile t: the 128 keys of both threads of a row pair into the O_part buffer (t & 1), as two
-      // runs of MMAs (a group's P occupies the first columns of its 64-column share of S).  In-order
-      // execution of the tensor pipe keeps S[s] intact until these reads of P are done (the next Q K^T
-      // into S[s] is issued later), and the buffer (t & 1) was folded by the softmax threads before
-      // they published P of tile t.
-      auto issue_pv = [&](int t) {
-        const int s = t & 1;
-        const uint32_t ph = (t >> 1) & 1;
-        if (!mbar_wait(EXACT ? v_full : v_full + 8 * s, EXACT ? (uint32_t)(t & 1) : ph, abort_ptr)) { give_up(0x23); ok = false; return; }
-        const uint32_t vb = EXACT ? v_smem : v_smem + s * kTileBytes;
-        const uint32_t o_addr = tmem_o0 + (uint32_t)s * 64;
-        for (int g = 0; g < 2; ++g) {
-          if (!mbar_wait(pfull0 + 8 * (g * 2 + s), ph, abort_ptr)) { give_up(0x24); ok = false; return; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if constexpr (EXACT) {
-            // P x V, P x tails of V, tails of P x V
+        if (last_of_item) umma_commit(q_empty);       // its last scores are issued: the Q tile is handed back
+      }
+      __syncwarp();
+    };
+    // P V of tile t: the 128 keys of both threads of a row pair into the O_part buffer (t & 1), as two
+    // runs of MMAs (a group's P occupies the first columns of its 64-column share of S).  In-order
+    // execution of the tensor pipe keeps S[s] intact until these reads of P are done (the next Q K^T
+    // into S[s] is issued later), and the buffer (t & 1) was folded by the softmax threads before
+    // they published P of tile t.
+    auto issue_pv = [&](int t) {
+      const int s = t & 1;
+      const uint32_t ph = (t >> 1) & 1;
+      ok = all_waited(mbar_wait(EXACT ? v_full : v_full + 8 * s, EXACT ? (uint32_t)(t & 1) : ph, abort_ptr), 0x23);
+      if (!ok) return;
+      const uint32_t vb = EXACT ? v_smem : v_smem + s * kTileBytes;
+      const uint32_t o_addr = tmem_o0 + (uint32_t)s * 64;
+      const uint32_t on = elect_one() ? 1u : 0u;
 #pragma unroll
-            for (int pass = 0; pass < 3; ++pass) {
-              const uint32_t pa = pass == 2 ? tmem_pt : tmem_base + (uint32_t)s * 128;
-              const uint32_t va = vb + (pass == 1 ? kTileBytes : 0);
+      for (int g = 0; g < 2; ++g) {
+        ok = all_waited(mbar_wait(pfull0 + 8 * (g * 2 + s), ph, abort_ptr), 0x24);
+        if (!ok) return;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if constexpr (BF16) {
+          // P: two bf16 per TMEM column, 16 keys = 8 columns per instruction; V: [keys x 64 dims] bf16,
+          // one 128-byte swizzled row per key, 16 rows per instruction
 #pragma unroll
-              for (int kk = 0; kk < 8; ++kk)
-                umma_ts(o_addr, pa + (uint32_t)(g * 64 + kk * 8), make_desc(va + (uint32_t)(g * 8 + kk) * 1024, kSlab, 512, 1),
-                        p.idesc_pv, (g | kk | pass) != 0 ? 1u : 0u, false);
-            }
-          } else if (BF16) {
-            // P: two bf16 per TMEM column, 16 keys = 8 columns per instruction; V: [keys x 64 dims] bf16,
-            // one 128-byte swizzled row per key, 16 rows per instruction
+          for (int kk = 0; kk < 4; ++kk)
+            umma_ts_if(on, o_addr, tmem_base + (uint32_t)s * 128 + (uint32_t)(g * 64 + kk * 8),
+                       make_desc(vb + (uint32_t)(g * 4 + kk) * 2048, kSlab, 1024, 2), p.idesc_pv, (g | kk) != 0 ? 1u : 0u, true);
+        } else {
+          // EXACT: P x V, P x tails of V, tails of P x V
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              umma_ts(o_addr, tmem_base + (uint32_t)s * 128 + (uint32_t)(g * 64 + kk * 8),
-                      make_desc(vb + (uint32_t)(g * 4 + kk) * 2048, kSlab, 1024, 2), p.idesc_pv, (g | kk) != 0 ? 1u : 0u, true);
-          } else {
+          for (int pass = 0; pass < (EXACT ? 3 : 1); ++pass) {
+            const uint32_t pa = pass == 2 ? tmem_pt : tmem_base + (uint32_t)s * 128;
+            const uint32_t va = vb + (pass == 1 ? kTileBytes : 0);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              umma_ts(o_addr, tmem_base + (uint32_t)s * 128 + (uint32_t)(g * 64 + kk * 8),
-                      make_desc(vb + (uint32_t)(g * 8 + kk) * 1024, kSlab, 512, 1), p.idesc_pv, (g | kk) != 0 ? 1u : 0u, false);
+              umma_ts_if(on, o_addr, pa + (uint32_t)(g * 64 + kk * 8), make_desc(va + (uint32_t)(g * 8 + kk) * 1024, kSlab, 512, 1),
+                         p.idesc_pv, (g | kk | pass) != 0 ? 1u : 0u, false);
           }
         }
+      }
+      if (on) {
         umma_commit(ofull0 + 8 * s);
         umma_commit(EXACT ? v_empty : v_empty + 8 * s);
-      };
-      // An item's first scores: its Q must have landed; once its last scores are issued, the Q tile is handed back.
-      auto first_qk = [&](int ii, int t, int n_kv) {
-        if (!mbar_wait(q_full, ii & 1, abort_ptr)) { give_up(0x21); ok = false; return; }
-        issue_qk(t);
-        if (ok && n_kv == 1) umma_commit(q_empty);
-      };
-      int t = 0;
-      for (int ii = 0; ok; ++ii) {
-        const int w = nth_item(ii);
-        if (w < 0) break;
-        const int n_kv = item_of(w).n_kv;
-        // (The next item's first scores are NOT issued ahead of this item's last P V: the softmax warps
-        // wait for that P V to finish the item, and have the merge and the stores to do before they
-        // need the next scores.)
-        first_qk(ii, t, n_kv);
-        for (int j = 0; j < n_kv && ok; ++j) {
-#ifdef KB200_TRACE
-          ATTN_MMA_STAMP(tm); ++tm;
-#endif
-          if (j + 1 < n_kv) {
-            issue_qk(t + j + 1);                     // the next scores are computed while the softmax warps work on tile j
-            if (ok && j + 2 == n_kv) umma_commit(q_empty);
-          }
-#ifdef KB200_TRACE
-          ATTN_MMA_STAMP(tm); ++tm;
-#endif
-          if (ok) issue_pv(t + j);
-#ifdef KB200_TRACE
-          ATTN_MMA_STAMP(tm); ++tm;
-#endif
-        }
-        t += n_kv;
       }
+      __syncwarp();
+    };
+    int t = 0;
+    for (int ii = 0; ok; ++ii) {
+      const int w = nth_item(ii);
+      if (w < 0) break;
+      const int n_kv = item_of(w).n_kv;
+      // (The next item's first scores are NOT issued ahead of this item's last P V: the softmax warps
+      // wait for that P V to finish the item, and have the merge and the stores to do before they
+      // need the next scores.)
+      ok = all_waited(mbar_wait(q_full, ii & 1, abort_ptr), 0x21);
+      if (!ok) break;
+      issue_qk(t, n_kv == 1);
+      for (int j = 0; j < n_kv && ok; ++j) {
+        if (j + 1 < n_kv) issue_qk(t + j + 1, j + 2 == n_kv);      // the next scores are computed while the softmax warps work on tile j
+        if (ok) issue_pv(t + j);
+      }
+      t += n_kv;
     }
   } else {
     // ---------------- softmax / output (warps 2..9) ----------------
@@ -951,9 +921,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
            (long long)g - marks[0], clock64() - marks[1], item_of(blockIdx.x).n_kv);
     printf("softmax thread per item (tiles done, states exchanged, rows stored):");
     for (int j = 0; j < 15; ++j) printf(" %lld", trace[2][j] - marks[1]);
-    printf("\n");
-    printf("MMA thread (per tile: loop top, after Q K^T of the next tile, after P V):");
-    for (int j = 0; j < 48; ++j) printf(" %lld", mma_trace[j] - marks[1]);
     printf("\n");
     for (int j = 0; j < item_of(blockIdx.x).n_kv && j < 16; ++j)
       printf("kv %2d  s_ready %7lld p_stored %7lld folded %7lld\n", j, trace[0][j] - marks[1], trace[1][j] - marks[1],

@@ -126,18 +126,18 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap
       : "memory");
 }
 template <bool BF16>
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_pair(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   if (BF16) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
   } else {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
   }
 }
@@ -199,7 +199,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   const int b_stage_bytes = KPS * p.half_bn * 128;
   const int stage_bytes = a_stage_bytes + b_stage_bytes;
   const uint32_t epi_base = tiles + (uint32_t)(p.stages * stage_bytes);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
@@ -359,16 +359,18 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             break;
           }
           PAIR_STAMP(2, tq);
-          if (elect_one()) {
+          // (the lane that issues is a predicate, not a branch: see umma_if)
+          const uint32_t on = elect_one() ? 1u : 0u;
 #pragma unroll
-            for (int j = 0; j < KPS; ++j) {
+          for (int j = 0; j < KPS; ++j) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const uint64_t adesc = ((uint64_t)a_hi << 32) | (a_lo_fixed | ((a16 + (uint32_t)(j * (kPairATileBytes >> 4) + 2 * k)) & 0x3FFFu));
-                const uint64_t bdesc = ((uint64_t)b_hi << 32) | (b_lo_fixed | ((b16 + (uint32_t)j * b_slab16 + (uint32_t)k * b_step16) & 0x3FFFu));
-                umma_pair<BF16>(tmem_d, adesc, bdesc, idesc, (kb | j | k) != 0 ? 1u : 0u);
-              }
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t adesc = ((uint64_t)a_hi << 32) | (a_lo_fixed | ((a16 + (uint32_t)(j * (kPairATileBytes >> 4) + 2 * k)) & 0x3FFFu));
+              const uint64_t bdesc = ((uint64_t)b_hi << 32) | (b_lo_fixed | ((b16 + (uint32_t)j * b_slab16 + (uint32_t)k * b_step16) & 0x3FFFu));
+              umma_pair<BF16>(on, tmem_d, adesc, bdesc, idesc, (kb | j | k) != 0 ? 1u : 0u);
             }
+          }
+          if (on) {
             // the stage is free in both CTAs once these MMAs have read it
             umma_pair_commit(empty0 + 8 * s);
             if (kb + 1 == num_kb) umma_pair_commit(tfull0 + 8 * acc);

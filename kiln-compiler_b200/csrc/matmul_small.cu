@@ -83,7 +83,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const uint32_t recv = in_ring ? ring : ring + (uint32_t)(p.stages * kStage);
   // A cluster: the others' parts of this CTA's band
   const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kSmallExchange);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
   const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8;
   const int tile = blockIdx.x / p.splits;
@@ -178,7 +178,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       const uint32_t a16 = (ring + (uint32_t)(s * kStage)) >> 4, b16 = a16 + (kSmallABytes >> 4);
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
       auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
-      if (elect_one()) {
+      {
+        const uint32_t on = elect_one() ? 1u : 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t a = a16 + 2 * k, b = b16 + k * b_step;
@@ -186,15 +187,17 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
             // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
             // with the number of them (see matmul_tc.cu)
-            umma(tmem, desc(a_fixed, a + (kRaw >> 4)), desc(b_fixed, b), idesc, (i | k) != 0, false);
-            umma(tmem, desc(a_fixed, a), desc(b_fixed, b + (kRaw >> 4)), idesc, 1u, false);
-            umma(tmem + (uint32_t)((1 + rot) * kSmallN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
+            umma_if(on, tmem, desc(a_fixed, a + (kRaw >> 4)), desc(b_fixed, b), idesc, (i | k) != 0, false);
+            umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b + (kRaw >> 4)), idesc, 1u, false);
+            umma_if(on, tmem + (uint32_t)((1 + rot) * kSmallN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
           } else {
-            umma(tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
+            umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
           }
         }
-        if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
-        if (i + 1 == n_slabs) umma_commit(done);
+        if (on) {
+          if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
+          if (i + 1 == n_slabs) umma_commit(done);
+        }
       }
       __syncwarp();
       if (EXACT && ++rot == p.nacc) rot = 0;

@@ -316,7 +316,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   const int raw_bytes = a_stage_bytes + b_tile_bytes;       // what TMA delivers per stage
   const int stage_bytes = SPLIT3 ? 2 * raw_bytes : raw_bytes;   // exact-FP32 mode: the tails of both operands follow
   uint8_t* epi_buf = smem_raw + (tiles - raw) + (size_t)p.stages * stage_bytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kMaxStages]);
   const uint32_t tfull0 = smem_u32(&bars[2 * kMaxStages]), tempty0 = smem_u32(&bars[2 * kMaxStages + 2]);
   const uint32_t split0 = smem_u32(&bars[2 * kMaxStages + 6]);
@@ -372,39 +372,42 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   if (blockIdx.x <= 1 && threadIdx.x == 0) marks[2] = clock64();
 #endif
 
+  // A whole warp walks each of the producer and issuer roles, one lane issuing (see elect_one); its waits end
+  // for all lanes or none.
+  auto all_waited = [&](bool got, int site) {
+    if (!got && lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
+    return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
+  };
   if (warp == 0 || warp == kProducerBWarp) {
     // ---------------- TMA producers ----------------
-    // Two threads in two warps, one per operand: issuing a bulk tensor copy costs a lone thread a few
-    // hundred cycles, and with narrow tiles that issue time, not the tensor pipe, bounded the K loop.
+    // Two warps, one per operand: issuing a bulk tensor copy costs a few hundred cycles, and with
+    // narrow tiles that issue time, not the tensor pipe, bounded the K loop.
     // Both wait on the stage's empty barrier and each arrives on its full barrier with its own bytes.
-    if (lane == 0) {
-      const bool load_a = warp == 0;
-      // everything the loop needs in registers: a lone thread pays full latency for every
-      // dependent instruction, so the per-slab instruction count is what bounds the issue rate
-      const int stages = p.stages, num_units = p.num_units, slab_k = p.slab_k, step_k = p.step_k, kps = p.kps;
-      const int bn = p.bn, chunk_n = p.chunk_n, b_mode = p.b_mode, n_chunks = p.n_chunks;
-      const uint32_t chunk_bytes = (uint32_t)step_k * kSlabBytes;          // one column chunk of B: step_k rows of 128 bytes
-      const uint32_t b_slab_bytes = (uint32_t)bn * kSlabBytes;             // K-major B: one slab of bn rows
-      const int parts = SPLIT3 && p.presplit >= (load_a ? 2 : 1) ? 2 : 1;                      // the operand's tails follow it
-      const uint32_t tx_bytes = (uint32_t)parts * (load_a ? (uint32_t)a_stage_bytes : (uint32_t)b_tile_bytes);
-      int s = 0;
-      uint32_t wait_parity = 1;                // parity to wait for on the empty barriers of this pass over the ring
-      bool ok = true;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
-        int tile, ks, batch, tm_i, tn_i, kb_begin, kb_end;
-        unit_coords(p, unit, tile, ks, batch, tm_i, tn_i);
-        slab_range(p, ks, kb_begin, kb_end);
-        const int m0 = tm_i * kTileM, n0 = tn_i * bn;
-        const int n0_chunk = tn_i * n_chunks;
-        int k_elem = kb_begin * step_k;
-        for (int kb = kb_begin; kb < kb_end; ++kb, k_elem += step_k) {
-          const uint32_t full = full0 + 8 * s;
-          if (!mbar_wait(empty0 + 8 * s, wait_parity, abort_ptr)) {
-            if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 1); *abort_ptr = 1; }
-            ok = false;
-            break;
-          }
-          if (load_a) KB200_STAMP(0, tp);
+    const bool load_a = warp == 0;
+    // everything the loop needs in registers: a lone thread pays full latency for every
+    // dependent instruction, so the per-slab instruction count is what bounds the issue rate
+    const int stages = p.stages, num_units = p.num_units, slab_k = p.slab_k, step_k = p.step_k, kps = p.kps;
+    const int bn = p.bn, chunk_n = p.chunk_n, b_mode = p.b_mode, n_chunks = p.n_chunks;
+    const uint32_t chunk_bytes = (uint32_t)step_k * kSlabBytes;          // one column chunk of B: step_k rows of 128 bytes
+    const uint32_t b_slab_bytes = (uint32_t)bn * kSlabBytes;             // K-major B: one slab of bn rows
+    const int parts = SPLIT3 && p.presplit >= (load_a ? 2 : 1) ? 2 : 1;                      // the operand's tails follow it
+    const uint32_t tx_bytes = (uint32_t)parts * (load_a ? (uint32_t)a_stage_bytes : (uint32_t)b_tile_bytes);
+    int s = 0;
+    uint32_t wait_parity = 1;                // parity to wait for on the empty barriers of this pass over the ring
+    bool ok = true;
+    for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+      int tile, ks, batch, tm_i, tn_i, kb_begin, kb_end;
+      unit_coords(p, unit, tile, ks, batch, tm_i, tn_i);
+      slab_range(p, ks, kb_begin, kb_end);
+      const int m0 = tm_i * kTileM, n0 = tn_i * bn;
+      const int n0_chunk = tn_i * n_chunks;
+      int k_elem = kb_begin * step_k;
+      for (int kb = kb_begin; kb < kb_end; ++kb, k_elem += step_k) {
+        const uint32_t full = full0 + 8 * s;
+        ok = all_waited(mbar_wait(empty0 + 8 * s, wait_parity, abort_ptr), 1);
+        if (!ok) break;
+        if (load_a) KB200_STAMP(0, tp);
+        if (elect_one()) {
           mbar_expect_tx(full, tx_bytes);
           for (int part = 0; part < parts; ++part) {
             const uint32_t a_dst = tiles + s * stage_bytes + part * raw_bytes;
@@ -423,12 +426,13 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
                 tma_load_3d(a_dst + a_stage_bytes + c * chunk_bytes, map, full, n0 + c * chunk_n, k_elem, batch);
             }
           }
-          if (load_a) KB200_STAMP(1, tp);
-#ifdef KB200_TRACE
-          ++tp;
-#endif
-          if (++s == stages) { s = 0; wait_parity ^= 1; }
         }
+        __syncwarp();
+        if (load_a) KB200_STAMP(1, tp);
+#ifdef KB200_TRACE
+        ++tp;
+#endif
+        if (++s == stages) { s = 0; wait_parity ^= 1; }
       }
     }
   } else if (warp == 1 || warp == kIssuerBWarp) {
@@ -437,7 +441,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     // its issuing thread exceed its tensor time) two threads in two warps issue alternate pipeline
     // stages, each into an accumulator of its own; the epilogue adds the two.
     const int q = warp == 1 ? 0 : 1;
-    if (lane == 0 && q < p.issuers) {
+    if (q < p.issuers) {
       const int nq = p.issuers;
       const int stages = p.stages, splits = p.splits, num_units = p.num_units, bn = p.bn;
       const uint64_t magic_stages = p.magic_stages;
@@ -467,10 +471,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         const int acc = one_buffer ? 0 : i & 1;
         const uint32_t aph = one_buffer ? i & 1 : (i >> 1) & 1;
         // the epilogue must have drained this accumulator (two tiles ago) before it is overwritten
-        if (!mbar_wait(tempty0 + 8 * acc, aph ^ 1, abort_ptr)) {
-          if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 4); *abort_ptr = 1; }
-          break;
-        }
+        if (!all_waited(mbar_wait(tempty0 + 8 * acc, aph ^ 1, abort_ptr), 4)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // Exact-FP32 mode: the tensor core truncates every accumulation, an error that grows with the
         // number of MMAs summed into one accumulator (whatever the size of the addend).  The two small
@@ -489,11 +490,8 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         int s = g_first - round * stages;
         for (int g = g_first; g < g0 + n_steps; g += nq) {
           // exact-FP32 mode: the stage is ready when the epilogue warps have split it, not when it lands
-          if (!mbar_wait((split3 && p.presplit != 2 ? split0 : full0) + 8 * s, (uint32_t)round & 1u, abort_ptr)) {
-            if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 2); *abort_ptr = 1; }
-            ok = false;
-            break;
-          }
+          ok = all_waited(mbar_wait((split3 && p.presplit != 2 ? split0 : full0) + 8 * s, (uint32_t)round & 1u, abort_ptr), 2);
+          if (!ok) break;
           if (split3) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           if (q == 0) KB200_STAMP(2, tm);
           const uint32_t tmem_d = tmem_t + (uint32_t)((rot + (split3 ? 1 : 0)) * bn);
@@ -501,6 +499,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           uint32_t accumulate_small = n_done > 0 ? 1u : 0u;
           if (++rot == nacc) rot = 0;
           ++n_done;
+          const uint32_t on = elect_one() ? 1u : 0u;
           for (int j = 0; j < kps; ++j) {
             const uint32_t a16 = tiles16 + (uint32_t)s * stage16 + (uint32_t)j * a_tile16;
             const uint32_t b16 = tiles16 + (uint32_t)s * stage16 + a_stage16 + (uint32_t)j * b_slab16;
@@ -510,18 +509,19 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
               // its upper bits, which must not spill into the neighbouring descriptor fields
               if (split3) {
                 // a*b = (ah + al)(bh + bl) ~ al*bh + ah*bl + ah*bh: the small terms first, al*bl (2^-22 a*b) dropped
-                umma(tmem_t, a_fixed | (uint64_t)((a16 + raw16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + k * b_step16) & 0x3FFFu),
+                umma_if(on, tmem_t, a_fixed | (uint64_t)((a16 + raw16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + k * b_step16) & 0x3FFFu),
                      idesc, accumulate_small, false);
-                umma(tmem_t, a_fixed | (uint64_t)((a16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + raw16 + k * b_step16) & 0x3FFFu),
+                umma_if(on, tmem_t, a_fixed | (uint64_t)((a16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + raw16 + k * b_step16) & 0x3FFFu),
                      idesc, 1u, false);
                 accumulate_small = 1;
               }
-              umma(tmem_d, a_fixed | (uint64_t)((a16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + k * b_step16) & 0x3FFFu), idesc,
+              umma_if(on, tmem_d, a_fixed | (uint64_t)((a16 + 2 * k) & 0x3FFFu), b_fixed | (uint64_t)((b16 + k * b_step16) & 0x3FFFu), idesc,
                    accumulate, BF16);
               accumulate = 1;
             }
           }
-          umma_commit(empty0 + 8 * s);   // frees the stage once these MMAs have read it
+          if (on) umma_commit(empty0 + 8 * s);   // frees the stage once these MMAs have read it
+          __syncwarp();
           if (q == 0) KB200_STAMP(3, tm);
 #ifdef KB200_TRACE
           ++tm;
@@ -530,7 +530,8 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           if (s >= stages) { s -= stages; ++round; }
         }
         g0 += n_steps;
-        if (ok) umma_commit(tfull0 + 8 * acc);   // arrives when every MMA this thread issued for the tile has completed
+        if (ok && elect_one()) umma_commit(tfull0 + 8 * acc);   // arrives when every MMA this thread issued for the tile has completed
+        __syncwarp();
       }
     }
   } else if (warp < 2 + kEpiWarps) {
