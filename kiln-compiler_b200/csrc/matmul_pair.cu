@@ -53,7 +53,7 @@ constexpr int kPairThreads = 512;
 constexpr int kPairEpiWarps = 12;
 constexpr int kPairFirstEpiWarp = 2;
 constexpr int kPairWarpsPerQuad = kPairEpiWarps / 4;
-constexpr int kPairBlocksPerWarp = (8 + kPairWarpsPerQuad - 1) / kPairWarpsPerQuad;   // 32-column blocks of a 256-column tile
+constexpr int kPairBlocksPerWarp = (8 + kPairWarpsPerQuad - 1) / kPairWarpsPerQuad;   // 32-column blocks of a 256-column tile (narrower ones have fewer)
 constexpr int kPairMaxStages = 8;
 constexpr int kPairATileBytes = 128 * 128;        // 128 rows x one 128-byte K slab
 #ifdef KB200_TRACE
@@ -690,6 +690,49 @@ bool classify_steps(const PlanKernel& k, PairParams* p, const DevOperand** res_o
 
 }  // namespace
 
+namespace {
+
+// SM pairs this plan counts on: with several plans in flight (plan option CONCURRENCY) each takes its share.
+int pair_share(const Plan& plan) {
+  const int pairs = plan.sm_count / 2, share = plan.concurrency > 1 ? pairs / plan.concurrency : pairs;
+  return share > 0 ? share : 1;
+}
+
+struct PairPlan { int bn; int64_t cycles; };
+
+// Tile width and estimated cycles of the slowest SM pair.  A slab costs the tensor cores 2 cycles per column
+// (measured 2.2), the issuing thread ~275 whatever the width, and the GPU ~5000 bytes a clock from L2 to
+// all SMs together: 256-column tiles on 72 pairs take 944 cycles per slab, on 48 pairs 629, where the
+// tensor cores need 512.  So the width that moves the fewest bytes in the fewest rounds; a narrower tile
+// that only evens out the last round loses (8192 x 768 x 3072: 192 columns 42.3 us, 256 40.6).  A tile
+// drains at ~20 bytes per clock and SM, under the next tile's main loop or, the last one, after it; the
+// rest of a launch is ~6300.  An N-major B comes in whole 128-byte column chunks per CTA: 128 or 256.
+PairPlan plan_pair(const PlanKernel& k, bool b_kmajor, int64_t share) {
+  const int slab_k = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;
+  const int64_t slabs = (k.K + slab_k - 1) / slab_k;
+  const int64_t bytes = k.mirror_only && k.shadow_out ? 2 : 4;
+  PairPlan best{128, 0};
+  for (int bn : {256, 224, 192, 160, 128}) {
+    if ((!b_kmajor && bn != 256 && bn != 128) || (bn > 128 && bn / 2 >= k.N)) continue;
+    const int64_t tiles = ((k.M + 255) / 256) * ((k.N + bn - 1) / bn) * k.batch;
+    const int64_t rounds = (tiles + share - 1) / share;
+    const int64_t active = (tiles + rounds - 1) / rounds;
+    const int64_t supply = (kPairATileBytes + bn * 64) * 2 * active / 5000;
+    int64_t per_slab = bn * 22 / 10;
+    if (per_slab < 275) per_slab = 275;
+    if (per_slab < supply) per_slab = supply;
+    const int64_t drain = (int64_t)bn * 128 * bytes / 20;
+    const int64_t main_loop = slabs * per_slab > drain ? slabs * per_slab : drain;
+    const int64_t cycles = rounds * main_loop + 6300 + drain;
+    if (best.cycles == 0 || cycles < best.cycles) best = {bn, cycles};
+  }
+  return best;
+}
+
+}  // namespace
+
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(k, b_kmajor, plan.sm_count / 2).cycles; }
+
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
   if (d.precision == KB200_PREC_FP32 || !k.has_chain) return false;
@@ -725,29 +768,13 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
       if (p.steps[s].op == CH_TANH) p.steps[s].op = CH_TANH_APPROX;
       else if (p.steps[s].op == CH_GELU_TANH) p.steps[s].op = CH_GELU_TANH_APPROX;
     }
-  const int pairs = plan.sm_count / 2;
   const int slab_k = ops.bf16 ? 64 : 32, chunk_n = ops.bf16 ? 64 : 32;
-  // Tile width and K slabs per pipeline step, by a cost model in cycles of the slowest SM pair.  A step
-  // costs the issuing thread ~60 cycles per MMA plus ~250 for the probe and the commit, whatever the
-  // width, and the tensor cores 2 cycles per column and slab: 256 columns are bound by the tensor
-  // cores (512 per slab), 128 columns by the issue (~490, or ~365 with two slabs per step).  The
-  // last tile's epilogue (~1200 cycles per 32-column block and warp) is not hidden.  When several
-  // plans share the GPU (plan option CONCURRENCY) each can count on its share of the pairs only.
+  // Tile width by the cost model above; K slabs per pipeline step below.
   int bn = d.cfg[1] == 128 || d.cfg[1] == 256 ? d.cfg[1] : 0;
   int kps = d.cfg[2] == 1 || d.cfg[2] == 2 ? d.cfg[2] : 0;
-  const int share = plan.concurrency > 1 ? (pairs / plan.concurrency > 0 ? pairs / plan.concurrency : 1) : pairs;
+  const int share = pair_share(plan);
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  if (bn == 0) {
-    int64_t best = 0;
-    for (int cand : {256, 128}) {
-      if (cand > 128 && cand / 2 >= k.N) continue;
-      const int64_t n_tiles = ((k.M + 255) / 256) * ((k.N + cand - 1) / cand) * k.batch;
-      const int64_t rounds = (n_tiles + share - 1) / share;
-      const int64_t per_slab = cand == 256 ? 512 : (kps == 1 ? 490 : 365);
-      const int64_t cost = rounds * slabs * per_slab + (cand / 64) * 1200;
-      if (bn == 0 || cost < best) { bn = cand; best = cost; }
-    }
-  }
+  if (bn == 0) bn = plan_pair(k, ops.b_kmajor, share).bn;
   while (bn > 128 && bn / 2 >= k.N) bn /= 2;
   // Staging per epilogue warp: one slot for a 32 x 32 block, float32 (also where a matrix operand of
   // the chain lands; left out when only the mirror is stored) and its bf16 copy.

@@ -35,12 +35,11 @@ namespace {
 
 using namespace tc;
 
-constexpr int kSmallM = 128, kSmallN = 64;
+constexpr int kSmallM = 128;
 constexpr int kSmallThreads = 352;
 constexpr int kSmallEpiWarps = 8;
 constexpr int kSmallMaxStages = 8;
-constexpr int kSmallABytes = kSmallM * 128, kSmallBBytes = kSmallN * 128;      // one 128-byte K slab
-constexpr int kSmallExchange = kSmallM * kSmallN * 4;
+constexpr int kSmallABytes = kSmallM * 128;      // one 128-byte K slab
 constexpr int kSmallSmem = 225 * 1024;
 
 enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2 };
@@ -65,12 +64,16 @@ struct SmallParams {
   int64_t out_row;                 // of both
 };
 
-template <int MODE, int FIN>
+// BN: columns of a tile, 64 or 128.
+template <int MODE, int FIN, int BN>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                 const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
   constexpr bool EXACT = MODE == SMALL_EXACT;
+  constexpr int kSmallBBytes = BN * 128;
   constexpr int kRaw = kSmallABytes + kSmallBBytes;             // a stage: A, B; exact FP32: then their tails
+  constexpr int kTileBytes = kSmallM * BN * 4;
+  constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
   constexpr int kStage = EXACT ? 2 * kRaw : kRaw;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 2];
@@ -78,11 +81,11 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   __shared__ int abort_flag;
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
-  // This CTA's partial tile, a 4 KB block per warp: in the ring, idle by then, where it is large enough
-  const bool in_ring = p.stages * kStage >= kSmallExchange;
+  // This CTA's partial tile in 32 x 32 blocks of 4 KB: in the ring, idle by then, where it is large enough
+  const bool in_ring = p.stages * kStage >= kTileBytes;
   const uint32_t recv = in_ring ? ring : ring + (uint32_t)(p.stages * kStage);
   // A cluster: the others' parts of this CTA's band
-  const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kSmallExchange);
+  const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kTileBytes);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
   const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8;
@@ -101,7 +104,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     mbar_init(done, 1);
     mbar_init(received, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(received, (uint32_t)(kSmallExchange / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
+    mbar_expect_tx(received, (uint32_t)(kTileBytes / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
   if (threadIdx.x == 32) {
     prefetch_tensormap(&tma_a);
@@ -155,8 +158,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
             const CUtensorMap* map = part ? &tma_bt : &tma_b;
             const uint32_t at = dst + kSmallABytes + part * kRaw;
-            if (p.b_kmajor) tma_load_3d(at, map, bar, k_elem, tn * kSmallN, 0);
-            else tma_load_4d(at, map, bar, 0, k_elem, tn * (kSmallN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
+            if (p.b_kmajor) tma_load_3d(at, map, bar, k_elem, tn * BN, 0);
+            else tma_load_4d(at, map, bar, 0, k_elem, tn * (BN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
           }
         }
       }
@@ -189,7 +192,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             // with the number of them (see matmul_tc.cu)
             umma_if(on, tmem, desc(a_fixed, a + (kRaw >> 4)), desc(b_fixed, b), idesc, (i | k) != 0, false);
             umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b + (kRaw >> 4)), idesc, 1u, false);
-            umma_if(on, tmem + (uint32_t)((1 + rot) * kSmallN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
+            umma_if(on, tmem + (uint32_t)((1 + rot) * BN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
           } else {
             umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
           }
@@ -207,19 +210,24 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // ---------------- warps 2..9 ----------------
     const int e = warp - 2, quad = warp & 3, half = e >> 2, t = threadIdx.x - 64;
     const int band_rows = kSmallM / p.splits;
-    // this thread's items of the band: float4 number t, t + 256, ... in row order
-    const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * kSmallN;
-    const int n = n0 + 4 * (t & 15);
+    // this thread's items of the band: float4 number t, t + 256, ... in row order, eight at a time
+    constexpr int kUnits = BN / 4, kRowsAtOnce = 256 / kUnits;
+    const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * BN;
+    const int u = t & (kUnits - 1), r0 = t / kUnits;
+    const int n = n0 + 4 * u;
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (FIN != FIN_NONE && n < p.N) bias = __ldg(reinterpret_cast<const float4*>(p.bias + n));
     float4 res[FIN == FIN_BIAS_RES ? 8 : 1];
-    if (FIN == FIN_BIAS_RES) {
+    auto load_res = [&](int first) {
+      if constexpr (FIN == FIN_BIAS_RES) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int r = (t >> 4) + 16 * j, m = m0 + band0 + r;
-        if (r < band_rows && m < p.M && n < p.N) res[j] = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
+        for (int j = 0; j < 8; ++j) {
+          const int r = first + r0 + kRowsAtOnce * j, m = m0 + band0 + r;
+          if (r < band_rows && m < p.M && n < p.N) res[j] = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
+        }
       }
-    }
+    };
+    load_res(0);
     bool ok = true;
     if (EXACT) {
       // the tails of A: what its 19 leading bits leave
@@ -249,42 +257,47 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (clustered) cluster_wait();              // every CTA's `received` exists
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float v[32];
-      const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 32);
-      tmem_ld32(at, v);
-      if (EXACT) {
-        const int used = min(p.nacc, n_slabs);
 #pragma unroll 1
-        for (int a = 1; a <= used; ++a) {
-          float w[32];
-          tmem_ld32(at + (uint32_t)(a * kSmallN), w);
+      for (int i = 0; i < kBlocks / 2; ++i) {
+        const int cb = half * (kBlocks / 2) + i;
+        float v[32];
+        const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb * 32);
+        tmem_ld32(at, v);
+        if (EXACT) {
+          const int used = min(p.nacc, n_slabs);
+#pragma unroll 1
+          for (int a = 1; a <= used; ++a) {
+            float w[32];
+            tmem_ld32(at + (uint32_t)(a * BN), w);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += w[j];
+            for (int j = 0; j < 32; ++j) v[j] += w[j];
+          }
         }
-      }
-      // This warp's 32 x 32 block goes to the CTA that finishes its rows (two CTAs, 16 rows each, with eight
-      // splits): staged in 128-byte rows, the 16-byte unit XORed with the row, then one bulk copy per
-      // destination that carries its arrival.  The blocks of this CTA's own band stay where they are
-      // staged: its own part of the exchange area.  (st.async straight from the registers, 16 bytes per
-      // lane and packet, took 3700 cycles to land where these take ~1500.)
-      const uint32_t block = (uint32_t)(e * 4096);
-      uint8_t* const mine = smem_raw + (recv - raw) + block + lane * 128;
+        // This 32 x 32 block goes to the CTA that finishes its rows (two CTAs, 16 rows each, with eight
+        // splits): staged in 128-byte rows, the 16-byte unit XORed with the row, then one bulk copy per
+        // destination that carries its arrival.  The rows of this CTA's own band stay where they are
+        // staged.  (st.async straight from the registers, 16 bytes per lane and packet, took 3700 cycles
+        // to land where these take ~1500.)
+        const uint32_t block = (uint32_t)((cb * 4 + quad) * 4096);
+        uint8_t* const mine = smem_raw + (recv - raw) + block + lane * 128;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<float4*>(mine + ((q ^ (lane & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-      if (clustered) {
-        fence_async_smem();
-        __syncwarp();
-        const int pieces = band_rows < 32 ? 2 : 1, rows = band_rows < 32 ? 16 : 32;
-        if (lane < pieces) {
-          const int row = quad * 32 + lane * rows, dest = row / band_rows;
-          if (dest != rank) {
-            // in the destination's area: [source][half][row of the band]
-            const uint32_t to = parts0 + (uint32_t)((rank * 2 + half) * band_rows + (row - dest * band_rows)) * 128u;
-            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(map_to_cta(to, (uint32_t)dest)), "r"(recv + block + (uint32_t)(lane * rows * 128)), "r"((uint32_t)(rows * 128)),
-                           "r"(map_to_cta(received, (uint32_t)dest))
-                         : "memory");
+        for (int q = 0; q < 8; ++q)
+          *reinterpret_cast<float4*>(mine + ((q ^ (lane & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        if (clustered) {
+          fence_async_smem();
+          __syncwarp();
+          const int pieces = band_rows < 32 ? 2 : 1, rows = band_rows < 32 ? 16 : 32;
+          if (lane < pieces) {
+            const int row = quad * 32 + lane * rows, dest = row / band_rows;
+            if (dest != rank) {
+              // in the destination's area: [source, the destination left out][32-column block][row of the band]
+              const int source = rank < dest ? rank : rank - 1;
+              const uint32_t to = parts0 + (uint32_t)((source * kBlocks + cb) * band_rows + (row - dest * band_rows)) * 128u;
+              asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                           ::"r"(map_to_cta(to, (uint32_t)dest)), "r"(recv + block + (uint32_t)(lane * rows * 128)), "r"((uint32_t)(rows * 128)),
+                             "r"(map_to_cta(received, (uint32_t)dest))
+                           : "memory");
+            }
           }
         }
       }
@@ -298,47 +311,52 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight warps have staged this CTA's own part
     ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
     if (ok) {
-      // Item j of this thread: row (t / 16) + 16 j of the band, float4 number t % 16.  All loads before the sums,
-      // all sums before the stores: the latencies of an item's few steps are what a lone item pays.
-      const int u = t & 15, h = u >> 3;
-      float4 a[8];
+      // Item j of this thread: row r0 + kRowsAtOnce * j, float4 number u.  All loads before the sums, all sums before
+      // the stores: the latencies of an item's few steps are what a lone item pays.
       const uint8_t* const area = smem_raw + (parts0 - raw);
+      const uint8_t* const own = smem_raw + (recv - raw);
+      const int cb = u >> 3;
+#pragma unroll 1
+      for (int first = 0; first < band_rows; first += 8 * kRowsAtOnce) {
+        float4 a[8];
+        if (first > 0) load_res(first);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int r = (t >> 4) + 16 * j;
-        a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (16 * j < band_rows) {
-          for (int s = 0; s < p.splits; ++s) {
-            // the own part lies in the staging blocks: block of (row / 32, half)
-            const int row = band0 + r;
-            const uint8_t* src = s == rank ? smem_raw + (recv - raw) + (h * 4 + (((row >> 5) + 2) & 3)) * 4096 + (row & 31) * 128
-                                           : area + ((s * 2 + h) * band_rows + r) * 128;
-            const float4 b = *reinterpret_cast<const float4*>(src + (((u ^ r) & 7) << 4));
-            a[j].x += b.x; a[j].y += b.y; a[j].z += b.z; a[j].w += b.w;
+        for (int j = 0; j < 8; ++j) {
+          const int r = first + r0 + kRowsAtOnce * j, row = band0 + r;
+          const int swizzled = ((u ^ r) & 7) << 4;
+          a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (first + kRowsAtOnce * j < band_rows) {      // (bands are multiples of 16 rows: the same answer for every thread)
+            for (int s = 0; s < p.splits; ++s) {          // in rank order
+              const uint8_t* src = s == rank ? own + (cb * 4 + (row >> 5)) * 4096 + (row & 31) * 128
+                                             : area + (((s < rank ? s : s - 1) * kBlocks + cb) * band_rows + r) * 128;
+              const float4 b = *reinterpret_cast<const float4*>(src + swizzled);
+              a[j].x += b.x; a[j].y += b.y; a[j].z += b.z; a[j].w += b.w;
+            }
           }
         }
-      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int r = (t >> 4) + 16 * j, m = m0 + band0 + r;
-        if (16 * j >= band_rows || m >= p.M || n >= p.N) continue;
-        float4 y = a[j];
-        if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
-        if (FIN == FIN_BIAS_GELU) {
-          if (MODE == SMALL_BF16) {
-            y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
-          } else {
-            y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
+        for (int j = 0; j < 8; ++j) {
+          const int r = first + r0 + kRowsAtOnce * j, m = m0 + band0 + r;
+          if (first + kRowsAtOnce * j >= band_rows) break;
+          if (m >= p.M || n >= p.N) continue;
+          float4 y = a[j];
+          if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
+          if (FIN == FIN_BIAS_GELU) {
+            if (MODE == SMALL_BF16) {
+              y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
+            } else {
+              y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
+            }
           }
-        }
-        if (FIN == FIN_BIAS_RES) { y.x += res[j].x; y.y += res[j].y; y.z += res[j].z; y.w += res[j].w; }
-        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
-        if (p.out16 != nullptr) {
-          __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-          uint2 packed;
-          packed.x = *reinterpret_cast<uint32_t*>(&lo);
-          packed.y = *reinterpret_cast<uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
+          if (FIN == FIN_BIAS_RES) { y.x += res[j].x; y.y += res[j].y; y.z += res[j].z; y.w += res[j].w; }
+          if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
+          if (p.out16 != nullptr) {
+            __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+            uint2 packed;
+            packed.x = *reinterpret_cast<uint32_t*>(&lo);
+            packed.y = *reinterpret_cast<uint32_t*>(&hi);
+            *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
+          }
         }
       }
     }
@@ -377,14 +395,20 @@ struct SmallState {
   bool a_moves = false, b_moves = false;      // the maps hold the operand's own address
 };
 
-template <int MODE>
-SmallKernel small_kernel(int fin) {
+template <int MODE, int BN>
+SmallKernel small_kernel_of(int fin) {
   switch (fin) {
-    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS>;
-    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU>;
-    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES>;
-    default: return mm_small_kernel<MODE, FIN_NONE>;
+    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN>;
+    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN>;
+    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN>;
+    default: return mm_small_kernel<MODE, FIN_NONE, BN>;
   }
+}
+
+SmallKernel small_kernel(int mode, int fin, int bn) {
+  if (mode == SMALL_BF16) return bn == 128 ? small_kernel_of<SMALL_BF16, 128>(fin) : small_kernel_of<SMALL_BF16, 64>(fin);
+  if (mode == SMALL_EXACT) return bn == 128 ? small_kernel_of<SMALL_EXACT, 128>(fin) : small_kernel_of<SMALL_EXACT, 64>(fin);
+  return bn == 128 ? small_kernel_of<SMALL_TF32, 128>(fin) : small_kernel_of<SMALL_TF32, 64>(fin);
 }
 
 // The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.
@@ -424,7 +448,7 @@ int resident_clusters(int splits, int sm_count) {
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS>;
+    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS, 64>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
@@ -435,20 +459,26 @@ int resident_clusters(int splits, int sm_count) {
   return known[splits];
 }
 
-struct SmallPlan { int splits; int64_t cycles; };
+struct SmallPlan { int bn, splits; int64_t cycles; };
 
-// K split and estimated cycles.  A CTA's step costs the larger of its operands' way from L2 (~55 bytes a clock)
-// and the issue of its MMAs (~62 cycles each); the rest of a launch, set-up to last store, ~6500, plus
-// ~1500 for an exchange.
-SmallPlan plan_small(int64_t tiles, int64_t slabs, int mode, int sm_count) {
-  const int64_t step = mode == SMALL_EXACT ? 900 : 450;
-  SmallPlan best{1, 0};
-  for (int s : {1, 2, 4, 8}) {
-    if (s > slabs) break;
-    const int64_t resident = resident_clusters(s, sm_count);
-    const int64_t rounds = (tiles + resident - 1) / resident;
-    const int64_t cycles = rounds * (((slabs + s - 1) / s) * step + 6500 + (s > 1 ? 1500 : 0));
-    if (best.cycles == 0 || cycles < best.cycles) best = {s, cycles};
+// Tile width, K split and estimated cycles, from fits to measured launches (128 to 1024 rows, 768 and 3072 of K, each
+// width and split).  A step, one 128-byte slab of K, is bound by shared memory: the operands land there
+// at 128 bytes a clock, every MMA reads its A and B again, and in exact FP32 (twelve MMAs) the tails of A
+// are made there.  Everything that runs once, launch to exit, is the rest: wide tiles have more to
+// drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
+SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count) {
+  SmallPlan best{64, 1, 0};
+  for (int bn : {64, 128}) {
+    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 1045 : 1480) : (bn == 64 ? 465 : 500);
+    const int64_t once = bn == 64 ? (mode == SMALL_EXACT ? 9700 : 8200) : 10700;
+    const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
+    for (int s : {1, 2, 4, 8}) {
+      if (s > slabs) break;
+      const int64_t resident = resident_clusters(s, sm_count);
+      const int64_t rounds = (tiles + resident - 1) / resident;
+      const int64_t cycles = rounds * (((slabs + s - 1) / s) * step + once + (s == 8 ? 1700 : s == 4 ? 500 : 0));
+      if (best.cycles == 0 || cycles < best.cycles) best = {bn, s, cycles};
+    }
   }
   return best;
 }
@@ -467,11 +497,10 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
   if (d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind != KB200_BASE_CONST) return -1;
   const DevOperand& O = k.ops[k.chain.out_slot];
   if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
-  const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * ((k.N + kSmallN - 1) / kSmallN);
-  if (tiles > 4096) return -1;
+  if (((k.M + kSmallM - 1) / kSmallM) * ((k.N + 63) / 64) > 4096) return -1;
   const int slab_k = bf16 ? 64 : 32;
   const int mode = bf16 ? SMALL_BF16 : d.precision == KB200_PREC_FP32 ? SMALL_EXACT : SMALL_TF32;
-  return plan_small(tiles, (k.K + slab_k - 1) / slab_k, mode, plan.sm_count).cycles;
+  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, mode, plan.sm_count).cycles;
 }
 
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, void** state) {
@@ -484,13 +513,17 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   const int slab_k = ops.bf16 ? 64 : 32, chunk = ops.bf16 ? 64 : 32;
   p.slab_k = slab_k;
   p.num_slabs = (int)((k.K + slab_k - 1) / slab_k);
-  p.tiles_n = (int)((k.N + kSmallN - 1) / kSmallN);
+  const SmallPlan how = plan_small(k.M, k.N, p.num_slabs, mode, plan.sm_count);
+  const int bn = how.bn;
+  p.splits = how.splits;
+  p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
-  p.splits = plan_small(tiles, p.num_slabs, mode, plan.sm_count).splits;
-  const int stage_bytes = (mode == SMALL_EXACT ? 2 : 1) * (kSmallABytes + kSmallBBytes);
+  const int stage_bytes = (mode == SMALL_EXACT ? 2 : 1) * (kSmallABytes + bn * 128);
   const int most = (p.num_slabs + p.splits - 1) / p.splits;
   p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
-  auto exchange_of = [&](int stages) { return (p.splits > 1 ? kSmallExchange : 0) + (stages * stage_bytes >= kSmallExchange ? 0 : kSmallExchange); };
+  const int tile_bytes = kSmallM * bn * 4;
+  // the others' parts of a band, and the own partial tile where the ring cannot hold it
+  auto exchange_of = [&](int stages) { return tile_bytes / p.splits * (p.splits - 1) + (stages * stage_bytes >= tile_bytes ? 0 : tile_bytes); };
   while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
   const int exchange = exchange_of(p.stages);
   st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
@@ -502,14 +535,15 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.b_layout = ops.bf16 ? 2 : 1;
   p.b_step16 = ops.b_kmajor ? 2u : (uint32_t)((ops.bf16 ? 16 : 8) * 128) >> 4;
   const uint32_t fmt = ops.bf16 ? 1u : 2u;
-  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(kSmallN >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
+  p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
   p.nacc = 1;
-  p.tmem_cols = kSmallN;
+  p.tmem_cols = bn;
   if (mode == SMALL_EXACT) {
     // one accumulator per 512 of K for the large products, beside that of the small ones
     const int64_t want = ((int64_t)most * slab_k + 511) / 512;
-    p.nacc = want > 7 ? 7 : (int)want;
-    while (p.tmem_cols < (1 + p.nacc) * kSmallN) p.tmem_cols *= 2;
+    const int room = 512 / bn - 1;
+    p.nacc = want > room ? room : (int)want;
+    while (p.tmem_cols < (1 + p.nacc) * bn) p.tmem_cols *= 2;
   }
   p.kernel_index = kernel_index;
   p.status = plan.d_status;
@@ -525,12 +559,12 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   st->a_moves = ops.a_base == k.ops[d.a_slot].ptr;
   st->b_moves = ops.b_base == k.ops[d.b_slot].ptr;
   bool ok = encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, 1, ops.a_row, 0, slab_k, kSmallM, false);
-  if (ok && ops.b_kmajor) ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, 1, ops.b_row, 0, slab_k, kSmallN, false);
-  else if (ok) ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk, k.K, ops.b_cols / chunk, 1, ops.b_row, 0, slab_k, kSmallN / chunk, !ops.bf16);
+  if (ok && ops.b_kmajor) ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, 1, ops.b_row, 0, slab_k, bn, false);
+  else if (ok) ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk, k.K, ops.b_cols / chunk, 1, ops.b_row, 0, slab_k, bn / chunk, !ops.bf16);
   st->map_bt = st->map_b;
   if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = mode == SMALL_BF16 ? small_kernel<SMALL_BF16>(fin) : mode == SMALL_EXACT ? small_kernel<SMALL_EXACT>(fin) : small_kernel<SMALL_TF32>(fin);
+  st->kernel = small_kernel(mode, fin, bn);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
   *state = st;

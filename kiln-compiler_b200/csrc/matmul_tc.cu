@@ -1210,8 +1210,17 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     b_base = k.b_shadow;
   }
   // Few tiles: the kernel written for latency.
-  const bool small = k.M <= kTileM && small_cycles(plan, k, b_kmajor, b_map_cols) > 0;
-  const bool a_pass = presplit && k.M > kTileM;
+  // Where the other kernels cover the shape too, by the estimates of both.  The exact-FP32 form of this
+  // file's kernel: 128-column tiles at 1150 cycles per slab (shared memory), ~16500 once, the pass over A included.
+  const int64_t few = small_cycles(plan, k, b_kmajor, b_map_cols);
+  int64_t many = 0;
+  if (few > 0 && k.M > kTileM) {
+    const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
+    if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
+    else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k, b_kmajor);
+  }
+  const bool small = few > 0 && (many == 0 || few < many);
+  const bool a_pass = presplit && k.M > kTileM && !small;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
     st->tail_pitch = (k.K + 3) / 4 * 4;
