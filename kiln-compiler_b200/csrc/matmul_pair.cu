@@ -700,38 +700,35 @@ int pair_share(const Plan& plan) {
 
 struct PairPlan { int bn; int64_t cycles; };
 
-// Tile width and estimated cycles of the slowest SM pair.  A slab costs the tensor cores 2 cycles per column
-// (measured 2.2), the issuing thread ~275 whatever the width, and the GPU ~5000 bytes a clock from L2 to
-// all SMs together: 256-column tiles on 72 pairs take 944 cycles per slab, on 48 pairs 629, where the
-// tensor cores need 512.  So the width that moves the fewest bytes in the fewest rounds; a narrower tile
-// that only evens out the last round loses (8192 x 768 x 3072: 192 columns 42.3 us, 256 40.6).  A tile
-// drains at ~20 bytes per clock and SM, under the next tile's main loop or, the last one, after it; the
-// rest of a launch is ~6300.  An N-major B comes in whole 128-byte column chunks per CTA: 128 or 256.
-PairPlan plan_pair(const PlanKernel& k, bool b_kmajor, int64_t share) {
+// Tile width and estimated cycles of the slowest SM pair.  Width: a slab of a 256-column tile takes its 512
+// tensor cycles (541 measured; reading and filling shared memory takes as many), one of a 128-column
+// tile is bound by the issue (~490, ~365 with two slabs per step), and the last tile's epilogue
+// (~1200 cycles per 32-column block and warp) is not hidden.  Widths between the two were built and lost:
+// 192 columns even out the last round of 8192 x 768 (K = 3072 BF16: 42.3 against 40.6 us) and of
+// 8192 x 3072, but stage more bytes per FLOP (8192 x 2304: 28.0 against 22.8 us).
+// The estimate is a fit to launches of 256 to 2048 rows: 330 or 541 cycles per slab, ~20 bytes a clock to
+// drain the last tile, ~6300 for the rest.
+PairPlan plan_pair(const PlanKernel& k, bool two_slabs, int64_t share) {
   const int slab_k = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  const int64_t bytes = k.mirror_only && k.shadow_out ? 2 : 4;
-  PairPlan best{128, 0};
-  for (int bn : {256, 224, 192, 160, 128}) {
-    if ((!b_kmajor && bn != 256 && bn != 128) || (bn > 128 && bn / 2 >= k.N)) continue;
+  PairPlan best{0, 0};
+  int64_t least = 0;
+  for (int bn : {256, 128}) {
+    if (bn > 128 && bn / 2 >= k.N) continue;
     const int64_t tiles = ((k.M + 255) / 256) * ((k.N + bn - 1) / bn) * k.batch;
     const int64_t rounds = (tiles + share - 1) / share;
-    const int64_t active = (tiles + rounds - 1) / rounds;
-    const int64_t supply = (kPairATileBytes + bn * 64) * 2 * active / 5000;
-    int64_t per_slab = bn * 22 / 10;
-    if (per_slab < 275) per_slab = 275;
-    if (per_slab < supply) per_slab = supply;
-    const int64_t drain = (int64_t)bn * 128 * bytes / 20;
-    const int64_t main_loop = slabs * per_slab > drain ? slabs * per_slab : drain;
-    const int64_t cycles = rounds * main_loop + 6300 + drain;
-    if (best.cycles == 0 || cycles < best.cycles) best = {bn, cycles};
+    const int64_t cost = rounds * slabs * (bn == 256 ? 512 : two_slabs ? 365 : 490) + (bn / 64) * 1200;
+    if (best.bn == 0 || cost < least) {
+      best = {bn, rounds * slabs * (bn == 256 ? 541 : 330) + 6300 + (int64_t)bn * 128 * 4 / 20};
+      least = cost;
+    }
   }
   return best;
 }
 
 }  // namespace
 
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(k, b_kmajor, plan.sm_count / 2).cycles; }
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k) { return plan_pair(k, true, plan.sm_count / 2).cycles; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
@@ -774,7 +771,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   int kps = d.cfg[2] == 1 || d.cfg[2] == 2 ? d.cfg[2] : 0;
   const int share = pair_share(plan);
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  if (bn == 0) bn = plan_pair(k, ops.b_kmajor, share).bn;
+  if (bn == 0) bn = plan_pair(k, kps != 1, share).bn;
   while (bn > 128 && bn / 2 >= k.N) bn /= 2;
   // Staging per epilogue warp: one slot for a 32 x 32 block, float32 (also where a matrix operand of
   // the chain lands; left out when only the mirror is stored) and its bf16 copy.

@@ -71,12 +71,11 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
   constexpr bool EXACT = MODE == SMALL_EXACT;
   constexpr int kSmallBBytes = BN * 128;
-  constexpr int kRaw = kSmallABytes + kSmallBBytes;             // a stage: A, B; exact FP32: then their tails
   constexpr int kTileBytes = kSmallM * BN * 4;
   constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
-  constexpr int kStage = EXACT ? 2 * kRaw : kRaw;
+  constexpr int kStage = kSmallABytes + (EXACT ? 2 : 1) * kSmallBBytes;         // A, B; exact FP32: then the tails of B
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 2];
+  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 4];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const uint32_t raw = smem_u32(smem_raw);
@@ -88,7 +87,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kTileBytes);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
-  const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8;
+  const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8, tfree0 = done + 16;
   const int tile = blockIdx.x / p.splits;
   const int rank = blockIdx.x - tile * p.splits;                // in the cluster: its CTAs are consecutive
   const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
@@ -103,6 +102,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     }
     mbar_init(done, 1);
     mbar_init(received, 1);
+    mbar_init(tfree0, 1);
+    mbar_init(tfree0 + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(received, (uint32_t)(kTileBytes / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
@@ -128,12 +129,13 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const bool clustered = p.splits > 1;
   if (clustered) cluster_arrive();
   const uint32_t tmem = tmem_slot;
+  [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((1 + p.nacc) * BN);      // exact FP32: two slabs of A and its tails
   volatile int* abort_ptr = &abort_flag;
   auto give_up = [&](int site) {
     if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
   };
   // a frozen B is nobody's output: its producer does not wait for the previous kernel
-  if (!(warp == 10 && p.b_static)) pdl_wait();
+  if (warp < 2 || (warp == 10 && !p.b_static)) pdl_wait();
 
   // A whole warp walks each of the three roles below; its waits end for all lanes or none.
   auto all_waited = [&](bool got, int site) {
@@ -157,7 +159,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #pragma unroll
           for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
             const CUtensorMap* map = part ? &tma_bt : &tma_b;
-            const uint32_t at = dst + kSmallABytes + part * kRaw;
+            const uint32_t at = dst + kSmallABytes + part * kSmallBBytes;
             if (p.b_kmajor) tma_load_3d(at, map, bar, k_elem, tn * BN, 0);
             else tma_load_4d(at, map, bar, 0, k_elem, tn * (BN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
           }
@@ -187,18 +189,20 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         for (int k = 0; k < 4; ++k) {
           const uint32_t a = a16 + 2 * k, b = b16 + k * b_step;
           if (EXACT) {
-            // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
-            // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
-            // with the number of them (see matmul_tc.cu)
-            umma_if(on, tmem, desc(a_fixed, a + (kRaw >> 4)), desc(b_fixed, b), idesc, (i | k) != 0, false);
-            umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b + (kRaw >> 4)), idesc, 1u, false);
-            umma_if(on, tmem + (uint32_t)((1 + rot) * BN), desc(a_fixed, a), desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
+            // a b ~ tail(a) b + a tail(b) + a b, A from tensor memory.  The small products have an accumulator of their
+            // own and the large ones rotate over nacc: the tensor core truncates every accumulation, an
+            // error that grows with the number of them (see matmul_tc.cu)
+            const uint32_t ta = tmem_a + (uint32_t)((i & 1) * 64 + 8 * k);
+            umma_ts_if(on, tmem, ta + 32, desc(b_fixed, b), idesc, (i | k) != 0, false);
+            umma_ts_if(on, tmem, ta, desc(b_fixed, b + (kSmallBBytes >> 4)), idesc, 1u, false);
+            umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
           } else {
             umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
           }
         }
         if (on) {
           if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
+          if (EXACT && i + 2 < n_slabs) umma_commit(tfree0 + 8 * (i & 1));
           if (i + 1 == n_slabs) umma_commit(done);
         }
       }
@@ -210,11 +214,15 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // ---------------- warps 2..9 ----------------
     const int e = warp - 2, quad = warp & 3, half = e >> 2, t = threadIdx.x - 64;
     const int band_rows = kSmallM / p.splits;
+    // The parameters are read through the constant cache, cold at every launch: touch what the end of the
+    // kernel needs now, under the wait.
+    asm volatile("" ::"l"(p.bias), "l"(p.res), "l"(p.res_row), "l"(p.out), "l"(p.out16), "l"(p.out_row), "r"(p.M), "r"(p.N), "r"(p.nacc) : "memory");
     // this thread's items of the band: float4 number t, t + 256, ... in row order, eight at a time
     constexpr int kUnits = BN / 4, kRowsAtOnce = 256 / kUnits;
     const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * BN;
     const int u = t & (kUnits - 1), r0 = t / kUnits;
     const int n = n0 + 4 * u;
+    pdl_wait();
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (FIN != FIN_NONE && n < p.N) bias = __ldg(reinterpret_cast<const float4*>(p.bias + n));
     float4 res[FIN == FIN_BIAS_RES ? 8 : 1];
@@ -230,22 +238,33 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     load_res(0);
     bool ok = true;
     if (EXACT) {
-      // the tails of A: what its 19 leading bits leave
+      // A goes to tensor memory, values and tails (what its 19 leading bits leave), 64 columns a slab and two
+      // slabs: read from there it leaves shared memory, which bounds this mode, to B -- with A and its
+      // tails in shared memory a slab of a 64-column tile moved 136 KB at 128 bytes a clock (960 cycles
+      // measured), now 72.  A lane has a row; each of the two warps of a lane quadrant 16 of the 32 values.
       int s = 0;
       uint32_t parity = 0;
+      const int row = quad * 32 + lane;
       for (int i = 0; i < n_slabs && ok; ++i) {
-        if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) { give_up(7); }
+        if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
+        if (i >= 2 && !mbar_wait(tfree0 + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
-        float4* head = reinterpret_cast<float4*>(smem_raw + (ring - raw) + s * kStage);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + row * 128;
+        float v[16], w[16];
 #pragma unroll
-        for (int q = 0; q < kSmallABytes / 16 / 256; ++q) {
-          const float4 v = head[t + 256 * q];
-          head[kRaw / 16 + t + 256 * q] =
-              make_float4(v.x - __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u), v.y - __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u),
-                          v.z - __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u), v.w - __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u));
+        for (int q = 0; q < 4; ++q) {
+          const float4 x = *reinterpret_cast<const float4*>(src + (((half * 4 + q) ^ (row & 7)) << 4));
+          v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
         }
-        fence_async_smem();
+#pragma unroll
+        for (int q = 0; q < 16; ++q) w[q] = v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
+        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)((i & 1) * 64 + half * 16);
+        tmem_st16(at, v);
+        tmem_st16(at + 32, w);
+        tmem_st_wait();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(split0 + 8 * s);
         if (++s == p.stages) { s = 0; parity ^= 1; }
@@ -459,21 +478,26 @@ int resident_clusters(int splits, int sm_count) {
   return known[splits];
 }
 
+// Exact FP32: accumulators for the large products, beside that of the small ones and 128 columns of A.
+constexpr int exact_accumulators(int bn) { return (512 - 128) / bn - 1; }
+
 struct SmallPlan { int bn, splits; int64_t cycles; };
 
 // Tile width, K split and estimated cycles, from fits to measured launches (128 to 1024 rows, 768 and 3072 of K, each
 // width and split).  A step, one 128-byte slab of K, is bound by shared memory: the operands land there
-// at 128 bytes a clock, every MMA reads its A and B again, and in exact FP32 (twelve MMAs) the tails of A
-// are made there.  Everything that runs once, launch to exit, is the rest: wide tiles have more to
+// at 128 bytes a clock and every MMA reads its operands again (exact FP32: twelve of them, A from tensor
+// memory).  Everything that runs once, launch to exit, is the rest: wide tiles have more to
 // drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
 SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count) {
   SmallPlan best{64, 1, 0};
   for (int bn : {64, 128}) {
-    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 1045 : 1480) : (bn == 64 ? 465 : 500);
-    const int64_t once = bn == 64 ? (mode == SMALL_EXACT ? 9700 : 8200) : 10700;
+    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : (bn == 64 ? 465 : 500);
+    const int64_t once = bn == 64 ? 8300 : 10800;
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
     for (int s : {1, 2, 4, 8}) {
       if (s > slabs) break;
+      // (exact FP32: at most 1024 of K in one accumulator)
+      if (mode == SMALL_EXACT && (slabs + s - 1) / s > 32 * exact_accumulators(bn)) continue;
       const int64_t resident = resident_clusters(s, sm_count);
       const int64_t rounds = (tiles + resident - 1) / resident;
       const int64_t cycles = rounds * (((slabs + s - 1) / s) * step + once + (s == 8 ? 1700 : s == 4 ? 500 : 0));
@@ -518,7 +542,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
-  const int stage_bytes = (mode == SMALL_EXACT ? 2 : 1) * (kSmallABytes + bn * 128);
+  const int stage_bytes = kSmallABytes + (mode == SMALL_EXACT ? 2 : 1) * bn * 128;
   const int most = (p.num_slabs + p.splits - 1) / p.splits;
   p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
   const int tile_bytes = kSmallM * bn * 4;
@@ -541,9 +565,8 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   if (mode == SMALL_EXACT) {
     // one accumulator per 512 of K for the large products, beside that of the small ones
     const int64_t want = ((int64_t)most * slab_k + 511) / 512;
-    const int room = 512 / bn - 1;
-    p.nacc = want > room ? room : (int)want;
-    while (p.tmem_cols < (1 + p.nacc) * bn) p.tmem_cols *= 2;
+    p.nacc = want > exact_accumulators(bn) ? exact_accumulators(bn) : (int)want;
+    while (p.tmem_cols < (1 + p.nacc) * bn + 128) p.tmem_cols *= 2;
   }
   p.kernel_index = kernel_index;
   p.status = plan.d_status;

@@ -1217,7 +1217,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   if (few > 0 && k.M > kTileM) {
     const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
     if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
-    else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k, b_kmajor);
+    else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
   }
   const bool small = few > 0 && (many == 0 || few < many);
   const bool a_pass = presplit && k.M > kTileM && !small;
