@@ -40,6 +40,7 @@ constexpr int kSmallThreads = 352;
 constexpr int kSmallEpiWarps = 8;
 constexpr int kSmallMaxStages = 8;
 constexpr int kSmallABytes = kSmallM * 128;      // one 128-byte K slab
+constexpr int kSmallACols = 128;                 // tensor-memory columns for slabs of A
 constexpr int kSmallSmem = 225 * 1024;
 
 enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2 };
@@ -72,10 +73,11 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr bool EXACT = MODE == SMALL_EXACT;
   constexpr int kSmallBBytes = BN * 128;
   constexpr int kTileBytes = kSmallM * BN * 4;
+  constexpr int kACols = EXACT ? 64 : 32, kABuffers = kSmallACols / kACols;      // columns of a slab of A (and its tails), slabs
   constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
   constexpr int kStage = kSmallABytes + (EXACT ? 2 : 1) * kSmallBBytes;         // A, B; exact FP32: then the tails of B
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 4];
+  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 6];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const uint32_t raw = smem_u32(smem_raw);
@@ -102,8 +104,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     }
     mbar_init(done, 1);
     mbar_init(received, 1);
-    mbar_init(tfree0, 1);
-    mbar_init(tfree0 + 8, 1);
+    for (int i = 0; i < kABuffers; ++i) mbar_init(tfree0 + 8 * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(received, (uint32_t)(kTileBytes / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
@@ -129,7 +130,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const bool clustered = p.splits > 1;
   if (clustered) cluster_arrive();
   const uint32_t tmem = tmem_slot;
-  [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((1 + p.nacc) * BN);      // exact FP32: two slabs of A and its tails
+  [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((1 + p.nacc) * BN);      // the slabs of A
   volatile int* abort_ptr = &abort_flag;
   auto give_up = [&](int site) {
     if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
@@ -170,44 +171,43 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    const uint64_t a_fixed = make_desc(0, 16, 1024);
     const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
     const uint32_t b_step = p.b_step16, idesc = p.idesc;
-    int s = 0, rot = 0;
+    int s = 0, rot = 0, buf = 0;
     uint32_t parity = 0;
     bool ok = true;
     for (int i = 0; i < n_slabs && ok; ++i) {
-      ok = all_waited(mbar_wait((EXACT ? split0 : full0) + 8 * s, parity, abort_ptr), 2);
+      ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // the slab of A is in tensor memory (and so that of B has landed)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a16 = (ring + (uint32_t)(s * kStage)) >> 4, b16 = a16 + (kSmallABytes >> 4);
+      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSmallABytes)) >> 4;
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
       auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
       {
         const uint32_t on = elect_one() ? 1u : 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t a = a16 + 2 * k, b = b16 + k * b_step;
+          const uint32_t b = b16 + k * b_step, ta = tmem_a + (uint32_t)(buf * kACols + 8 * k);
           if (EXACT) {
-            // a b ~ tail(a) b + a tail(b) + a b, A from tensor memory.  The small products have an accumulator of their
-            // own and the large ones rotate over nacc: the tensor core truncates every accumulation, an
-            // error that grows with the number of them (see matmul_tc.cu)
-            const uint32_t ta = tmem_a + (uint32_t)((i & 1) * 64 + 8 * k);
+            // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
+            // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
+            // with the number of them (see matmul_tc.cu)
             umma_ts_if(on, tmem, ta + 32, desc(b_fixed, b), idesc, (i | k) != 0, false);
             umma_ts_if(on, tmem, ta, desc(b_fixed, b + (kSmallBBytes >> 4)), idesc, 1u, false);
             umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
           } else {
-            umma_if(on, tmem, desc(a_fixed, a), desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
+            umma_ts_if(on, tmem, ta, desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
           }
         }
         if (on) {
           if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
-          if (EXACT && i + 2 < n_slabs) umma_commit(tfree0 + 8 * (i & 1));
+          if (i + kABuffers < n_slabs) umma_commit(tfree0 + 8 * buf);
           if (i + 1 == n_slabs) umma_commit(done);
         }
       }
       __syncwarp();
       if (EXACT && ++rot == p.nacc) rot = 0;
+      if (++buf == kABuffers) buf = 0;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else {
@@ -225,49 +225,50 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     pdl_wait();
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
     if (FIN != FIN_NONE && n < p.N) bias = __ldg(reinterpret_cast<const float4*>(p.bias + n));
-    float4 res[FIN == FIN_BIAS_RES ? 8 : 1];
-    auto load_res = [&](int first) {
-      if constexpr (FIN == FIN_BIAS_RES) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = first + r0 + kRowsAtOnce * j, m = m0 + band0 + r;
-          if (r < band_rows && m < p.M && n < p.N) res[j] = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
-        }
-      }
+    auto load_res = [&](int r) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      const int m = m0 + band0 + r;
+      if (FIN == FIN_BIAS_RES && r < band_rows && m < p.M && n < p.N) x = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
+      return x;
     };
-    load_res(0);
+    float4 res = load_res(r0);
     bool ok = true;
-    if (EXACT) {
-      // A goes to tensor memory, values and tails (what its 19 leading bits leave), 64 columns a slab and two
-      // slabs: read from there it leaves shared memory, which bounds this mode, to B -- with A and its
-      // tails in shared memory a slab of a 64-column tile moved 136 KB at 128 bytes a clock (960 cycles
-      // measured), now 72.  A lane has a row; each of the two warps of a lane quadrant 16 of the 32 values.
-      int s = 0;
-      uint32_t parity = 0;
+    {
+      // A goes to tensor memory, 32 columns a slab (exact FP32: values and tails, what their 19 leading bits leave).
+      // The tensor core reads an operand from shared memory at ~64 bytes a clock: with A there an MMA of 128
+      // rows and 64 columns took 133 cycles, from tensor memory ~65, and in exact FP32, where A and its
+      // tails were made in shared memory, a slab moved 136 KB through it (960 cycles a slab, now 690).
+      // A lane has a row; each of the two warps of a lane quadrant 64 of its 128 bytes.
+      int s = 0, buf = 0;
+      uint32_t parity = 0, free_parity = 0;
       const int row = quad * 32 + lane;
       for (int i = 0; i < n_slabs && ok; ++i) {
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
-        if (i >= 2 && !mbar_wait(tfree0 + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_ptr)) give_up(6);
+        if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, free_parity, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + row * 128;
-        float v[16], w[16];
+        float v[16];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 x = *reinterpret_cast<const float4*>(src + (((half * 4 + q) ^ (row & 7)) << 4));
           v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
         }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) w[q] = v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
-        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)((i & 1) * 64 + half * 16);
+        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kACols + half * 16);
         tmem_st16(at, v);
-        tmem_st16(at + 32, w);
+        if (EXACT) {
+          float w[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q) w[q] = v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
+          tmem_st16(at + 32, w);
+        }
         tmem_st_wait();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(split0 + 8 * s);
         if (++s == p.stages) { s = 0; parity ^= 1; }
+        if (++buf == kABuffers) { buf = 0; if (i >= kABuffers) free_parity ^= 1; }
       }
     }
     if (ok && !mbar_wait(done, 0, abort_ptr)) give_up(3);
@@ -330,52 +331,43 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight warps have staged this CTA's own part
     ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
     if (ok) {
-      // Item j of this thread: row r0 + kRowsAtOnce * j, float4 number u.  All loads before the sums, all sums before
-      // the stores: the latencies of an item's few steps are what a lone item pays.
+      // Item by item: row r0 + kRowsAtOnce * j, float4 number u.  A rolled loop: the code runs once, cold, and
+      // eight unrolled items were 2000 to 3000 cycles of instruction fetches whatever their number.
       const uint8_t* const area = smem_raw + (parts0 - raw);
       const uint8_t* const own = smem_raw + (recv - raw);
       const int cb = u >> 3;
 #pragma unroll 1
-      for (int first = 0; first < band_rows; first += 8 * kRowsAtOnce) {
-        float4 a[8];
-        if (first > 0) load_res(first);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = first + r0 + kRowsAtOnce * j, row = band0 + r;
-          const int swizzled = ((u ^ r) & 7) << 4;
-          a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (first + kRowsAtOnce * j < band_rows) {      // (bands are multiples of 16 rows: the same answer for every thread)
-            for (int s = 0; s < p.splits; ++s) {          // in rank order
-              const uint8_t* src = s == rank ? own + (cb * 4 + (row >> 5)) * 4096 + (row & 31) * 128
-                                             : area + (((s < rank ? s : s - 1) * kBlocks + cb) * band_rows + r) * 128;
-              const float4 b = *reinterpret_cast<const float4*>(src + swizzled);
-              a[j].x += b.x; a[j].y += b.y; a[j].z += b.z; a[j].w += b.w;
-            }
+      for (int r = r0; r < band_rows; r += kRowsAtOnce) {
+        const float4 res_next = load_res(r + kRowsAtOnce);
+        const int row = band0 + r, m = m0 + row;
+        const int swizzled = ((u ^ r) & 7) << 4;
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint8_t* part = area + (cb * band_rows + r) * 128 + swizzled;
+#pragma unroll 1
+        for (int s = 0; s < p.splits; ++s) {          // in rank order
+          const bool mine = s == rank;
+          const float4 b = *reinterpret_cast<const float4*>(mine ? own + (cb * 4 + (row >> 5)) * 4096 + (row & 31) * 128 + swizzled : part);
+          if (!mine) part += kBlocks * band_rows * 128;
+          y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w;
+        }
+        if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
+        if (FIN == FIN_BIAS_GELU) {
+          if (MODE == SMALL_BF16) {
+            y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
+          } else {
+            y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
           }
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = first + r0 + kRowsAtOnce * j, m = m0 + band0 + r;
-          if (first + kRowsAtOnce * j >= band_rows) break;
-          if (m >= p.M || n >= p.N) continue;
-          float4 y = a[j];
-          if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
-          if (FIN == FIN_BIAS_GELU) {
-            if (MODE == SMALL_BF16) {
-              y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
-            } else {
-              y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
-            }
-          }
-          if (FIN == FIN_BIAS_RES) { y.x += res[j].x; y.y += res[j].y; y.z += res[j].z; y.w += res[j].w; }
-          if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
-          if (p.out16 != nullptr) {
-            __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-            uint2 packed;
-            packed.x = *reinterpret_cast<uint32_t*>(&lo);
-            packed.y = *reinterpret_cast<uint32_t*>(&hi);
-            *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
-          }
+        if (FIN == FIN_BIAS_RES) { y.x += res.x; y.y += res.y; y.z += res.z; y.w += res.w; }
+        res = res_next;
+        if (m >= p.M || n >= p.N) continue;
+        if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
+        if (p.out16 != nullptr) {
+          __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+          uint2 packed;
+          packed.x = *reinterpret_cast<uint32_t*>(&lo);
+          packed.y = *reinterpret_cast<uint32_t*>(&hi);
+          *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
         }
       }
     }
@@ -478,8 +470,8 @@ int resident_clusters(int splits, int sm_count) {
   return known[splits];
 }
 
-// Exact FP32: accumulators for the large products, beside that of the small ones and 128 columns of A.
-constexpr int exact_accumulators(int bn) { return (512 - 128) / bn - 1; }
+// Exact FP32: accumulators for the large products, beside that of the small ones and the slabs of A.
+constexpr int exact_accumulators(int bn) { return (512 - kSmallACols) / bn - 1; }
 
 struct SmallPlan { int bn, splits; int64_t cycles; };
 
@@ -561,13 +553,14 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   const uint32_t fmt = ops.bf16 ? 1u : 2u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
   p.nacc = 1;
-  p.tmem_cols = bn;
+  p.tmem_cols = 32;
   if (mode == SMALL_EXACT) {
     // one accumulator per 512 of K for the large products, beside that of the small ones
     const int64_t want = ((int64_t)most * slab_k + 511) / 512;
     p.nacc = want > exact_accumulators(bn) ? exact_accumulators(bn) : (int)want;
-    while (p.tmem_cols < (1 + p.nacc) * bn + 128) p.tmem_cols *= 2;
+
   }
+  while (p.tmem_cols < (mode == SMALL_EXACT ? 1 + p.nacc : 1) * bn + kSmallACols) p.tmem_cols *= 2;
   p.kernel_index = kernel_index;
   p.status = plan.d_status;
   p.M = (int)k.M;
