@@ -100,7 +100,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full0 + 8 * s, 2);
       mbar_init(empty0 + 8 * s, 1);
-      mbar_init(split0 + 8 * s, kSmallEpiWarps);
+      mbar_init(split0 + 8 * s, kSmallEpiWarps / 2);
     }
     mbar_init(done, 1);
     mbar_init(received, 1);
@@ -238,37 +238,40 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       // The tensor core reads an operand from shared memory at ~64 bytes a clock: with A there an MMA of 128
       // rows and 64 columns took 133 cycles, from tensor memory ~65, and in exact FP32, where A and its
       // tails were made in shared memory, a slab moved 136 KB through it (960 cycles a slab, now 690).
-      // A lane has a row; each of the two warps of a lane quadrant 64 of its 128 bytes.
-      int s = 0, buf = 0;
-      uint32_t parity = 0, free_parity = 0;
+      // A lane has a row.  A slab is a chain of waits, loads, stores to tensor memory and an arrival, ~500 cycles
+      // whatever its size: two groups of four warps, one per lane quadrant, take alternate slabs.  (Every
+      // stage and buffer belongs to one group, which then sees each phase of its barriers: an even number
+      // of stages where the ring is used again.)
+      int s = half;
+      uint32_t parity = 0;
       const int row = quad * 32 + lane;
-      for (int i = 0; i < n_slabs && ok; ++i) {
+      for (int i = half; i < n_slabs && ok; i += 2) {
+        const int buf = i % kABuffers;
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
-        if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, free_parity, abort_ptr)) give_up(6);
+        if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, ((i / kABuffers) & 1) ^ 1, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + row * 128;
-        float v[16];
+        float v[32];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 x = *reinterpret_cast<const float4*>(src + (((half * 4 + q) ^ (row & 7)) << 4));
+        for (int q = 0; q < 8; ++q) {
+          const float4 x = *reinterpret_cast<const float4*>(src + ((q ^ (row & 7)) << 4));
           v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
         }
-        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kACols + half * 16);
-        tmem_st16(at, v);
+        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kACols);
+        tmem_st32(at, v);
         if (EXACT) {
-          float w[16];
 #pragma unroll
-          for (int q = 0; q < 16; ++q) w[q] = v[q] - __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
-          tmem_st16(at + 32, w);
+          for (int q = 0; q < 32; ++q) v[q] -= __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
+          tmem_st32(at + 32, v);
         }
         tmem_st_wait();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(split0 + 8 * s);
-        if (++s == p.stages) { s = 0; parity ^= 1; }
-        if (++buf == kABuffers) { buf = 0; if (i >= kABuffers) free_parity ^= 1; }
+        s += 2;
+        if (s >= p.stages) { s -= p.stages; parity ^= 1; }
       }
     }
     if (ok && !mbar_wait(done, 0, abort_ptr)) give_up(3);
@@ -541,6 +544,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   // the others' parts of a band, and the own partial tile where the ring cannot hold it
   auto exchange_of = [&](int stages) { return tile_bytes / p.splits * (p.splits - 1) + (stages * stage_bytes >= tile_bytes ? 0 : tile_bytes); };
   while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
+  if (p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
   const int exchange = exchange_of(p.stages);
   st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
   st->grid = (unsigned)(tiles * p.splits);
