@@ -47,7 +47,7 @@ enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2 };
 enum : int { FIN_NONE = 0, FIN_BIAS, FIN_BIAS_GELU, FIN_BIAS_RES };
 
 struct SmallParams {
-  int stages, num_slabs, slab_k, splits;
+  int stages, num_steps, slab_k, splits;
   int b_kmajor, b_static;
   int nacc;                        // exact FP32: accumulators the K steps rotate over, beside the one of the small products
   uint32_t b_lbo, b_sbo, b_layout, b_step16;
@@ -65,6 +65,10 @@ struct SmallParams {
   int64_t out_row;                 // of both
 };
 
+// 128-byte slabs of K per pipeline step.  A step costs the issuing warp ~400 cycles of wait, branches and commits
+// beside ~25 per MMA; exact FP32 has twelve MMAs to a slab and no room for more.
+__host__ __device__ constexpr int slabs_per_step(int mode) { return mode == SMALL_EXACT ? 1 : 2; }
+
 // BN: columns of a tile, 64 or 128.
 template <int MODE, int FIN, int BN>
 __global__ void __launch_bounds__(kSmallThreads, 1)
@@ -73,9 +77,10 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr bool EXACT = MODE == SMALL_EXACT;
   constexpr int kSmallBBytes = BN * 128;
   constexpr int kTileBytes = kSmallM * BN * 4;
-  constexpr int kACols = EXACT ? 64 : 32, kABuffers = kSmallACols / kACols;      // columns of a slab of A (and its tails), slabs
+  constexpr int kABuffers = 2;                                  // steps of A in tensor memory, 64 columns each
   constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
-  constexpr int kStage = kSmallABytes + (EXACT ? 2 : 1) * kSmallBBytes;         // A, B; exact FP32: then the tails of B
+  constexpr int kSlabs = slabs_per_step(MODE);
+  constexpr int kStage = kSlabs * kSmallABytes + 2 * kSmallBBytes;     // the slabs of A, then those of B; exact FP32: A, B, the tails of B
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 6];
   __shared__ uint32_t tmem_slot;
@@ -93,14 +98,14 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const int tile = blockIdx.x / p.splits;
   const int rank = blockIdx.x - tile * p.splits;                // in the cluster: its CTAs are consecutive
   const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
-  const int slab0 = rank * p.num_slabs / p.splits, n_slabs = (rank + 1) * p.num_slabs / p.splits - slab0;
+  const int step0 = rank * p.num_steps / p.splits, n_steps = (rank + 1) * p.num_steps / p.splits - step0;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(full0 + 8 * s, 2);
       mbar_init(empty0 + 8 * s, 1);
-      mbar_init(split0 + 8 * s, kSmallEpiWarps / 2);
+      mbar_init(split0 + 8 * s, EXACT ? kSmallEpiWarps / 2 : kSmallEpiWarps);
     }
     mbar_init(done, 1);
     mbar_init(received, 1);
@@ -146,27 +151,28 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   if (warp == 0 || warp == 10) {
     // ---------------- TMA producers, one per operand ----------------
     const bool is_a = warp == 0;
-    int s = 0, k_elem = slab0 * p.slab_k;
+    int s = 0, k_elem = step0 * kSlabs * p.slab_k;
     uint32_t parity = 1;
-    for (int i = 0; i < n_slabs; ++i, k_elem += p.slab_k) {
+    for (int i = 0; i < n_steps; ++i) {
       if (i >= p.stages && !all_waited(mbar_wait(empty0 + 8 * s, parity, abort_ptr), 1)) break;
-      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage);
+      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kSlabs * kSmallABytes;
       if (elect_one()) {
-        if (is_a) {
-          mbar_expect_tx(bar, kSmallABytes);
-          tma_load_3d(dst, &tma_a, bar, k_elem, tm * kSmallM, 0);
-        } else {
-          mbar_expect_tx(bar, (EXACT ? 2 : 1) * kSmallBBytes);
+        mbar_expect_tx(bar, is_a ? kSlabs * kSmallABytes : 2 * kSmallBBytes);
+        // (a slab past the end of K, in the last step of an odd number, is a box outside the tensor: zeros)
 #pragma unroll
-          for (int part = 0; part < (EXACT ? 2 : 1); ++part) {
-            const CUtensorMap* map = part ? &tma_bt : &tma_b;
-            const uint32_t at = dst + kSmallABytes + part * kSmallBBytes;
-            if (p.b_kmajor) tma_load_3d(at, map, bar, k_elem, tn * BN, 0);
-            else tma_load_4d(at, map, bar, 0, k_elem, tn * (BN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
+        for (int j = 0; j < 2; ++j) {
+          const int k = EXACT ? k_elem : k_elem + j * p.slab_k;
+          if (is_a) {
+            if (j < kSlabs) tma_load_3d(dst + j * kSmallABytes, &tma_a, bar, k, tm * kSmallM, 0);
+          } else {
+            const CUtensorMap* map = EXACT && j ? &tma_bt : &tma_b;
+            if (p.b_kmajor) tma_load_3d(b_dst + j * kSmallBBytes, map, bar, k, tn * BN, 0);
+            else tma_load_4d(b_dst + j * kSmallBBytes, map, bar, 0, k, tn * (BN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
           }
         }
       }
       __syncwarp();
+      k_elem += kSlabs * p.slab_k;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else if (warp == 1) {
@@ -176,38 +182,36 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     int s = 0, rot = 0, buf = 0;
     uint32_t parity = 0;
     bool ok = true;
-    for (int i = 0; i < n_slabs && ok; ++i) {
-      ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // the slab of A is in tensor memory (and so that of B has landed)
+    for (int i = 0; i < n_steps && ok; ++i) {
+      ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // this step's A is in tensor memory (and so its B has landed)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSmallABytes)) >> 4;
+      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSlabs * kSmallABytes)) >> 4;
+      const uint32_t on = elect_one() ? 1u : 0u;
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
-      auto desc = [](uint64_t fixed, uint32_t at) { return fixed | (uint64_t)(at & 0x3FFFu); };
-      {
-        const uint32_t on = elect_one() ? 1u : 0u;
+      auto desc = [&](uint32_t at) { return b_fixed | (uint64_t)(at & 0x3FFFu); };
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t b = b16 + k * b_step, ta = tmem_a + (uint32_t)(buf * kACols + 8 * k);
-          if (EXACT) {
-            // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
-            // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
-            // with the number of them (see matmul_tc.cu)
-            umma_ts_if(on, tmem, ta + 32, desc(b_fixed, b), idesc, (i | k) != 0, false);
-            umma_ts_if(on, tmem, ta, desc(b_fixed, b + (kSmallBBytes >> 4)), idesc, 1u, false);
-            umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b_fixed, b), idesc, i >= p.nacc || k != 0, false);
-          } else {
-            umma_ts_if(on, tmem, ta, desc(b_fixed, b), idesc, (i | k) != 0, MODE == SMALL_BF16);
-          }
+      for (int k = 0; k < 4 * kSlabs; ++k) {
+        const uint32_t b = b16 + (k >> 2) * (kSmallBBytes >> 4) + (k & 3) * b_step, ta = tmem_a + (uint32_t)(buf * 64 + 8 * k);
+        if (EXACT) {
+          // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
+          // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
+          // with the number of them (see matmul_tc.cu)
+          umma_ts_if(on, tmem, ta + 32, desc(b), idesc, (i | k) != 0, false);
+          umma_ts_if(on, tmem, ta, desc(b + (kSmallBBytes >> 4)), idesc, 1u, false);
+          umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b), idesc, i >= p.nacc || k != 0, false);
+        } else {
+          umma_ts_if(on, tmem, ta, desc(b), idesc, (i | k) != 0, MODE == SMALL_BF16);
         }
-        if (on) {
-          if (i + p.stages < n_slabs) umma_commit(empty0 + 8 * s);
-          if (i + kABuffers < n_slabs) umma_commit(tfree0 + 8 * buf);
-          if (i + 1 == n_slabs) umma_commit(done);
-        }
+      }
+      if (on) {
+        if (i + p.stages < n_steps) umma_commit(empty0 + 8 * s);
+        if (i + kABuffers < n_steps) umma_commit(tfree0 + 8 * buf);
+        if (i + 1 == n_steps) umma_commit(done);
       }
       __syncwarp();
       if (EXACT && ++rot == p.nacc) rot = 0;
-      if (++buf == kABuffers) buf = 0;
+      buf ^= 1;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else {
@@ -239,27 +243,28 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       // rows and 64 columns took 133 cycles, from tensor memory ~65, and in exact FP32, where A and its
       // tails were made in shared memory, a slab moved 136 KB through it (960 cycles a slab, now 690).
       // A lane has a row.  A slab is a chain of waits, loads, stores to tensor memory and an arrival, ~500 cycles
-      // whatever its size: two groups of four warps, one per lane quadrant, take alternate slabs.  (Every
-      // stage and buffer belongs to one group, which then sees each phase of its barriers: an even number
-      // of stages where the ring is used again.)
-      int s = half;
+      // whatever its size: of two groups of four warps, one per lane quadrant, each takes one slab of a step,
+      // or, one slab to a step, alternate steps.  (Every stage and buffer then belongs to one group, which
+      // sees each phase of its barriers: an even number of stages where the ring is used again.)
+      constexpr int kEvery = EXACT ? 2 : 1;
+      int s = EXACT ? half : 0;
       uint32_t parity = 0;
       const int row = quad * 32 + lane;
-      for (int i = half; i < n_slabs && ok; i += 2) {
+      for (int i = s; i < n_steps && ok; i += kEvery) {
         const int buf = i % kABuffers;
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
         if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, ((i / kABuffers) & 1) ^ 1, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + row * 128;
+        const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + (EXACT ? 0 : half * kSmallABytes) + row * 128;
         float v[32];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const float4 x = *reinterpret_cast<const float4*>(src + ((q ^ (row & 7)) << 4));
           v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
         }
-        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * kACols);
+        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 64 + (EXACT ? 0 : half * 32));
         tmem_st32(at, v);
         if (EXACT) {
 #pragma unroll
@@ -270,7 +275,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(split0 + 8 * s);
-        s += 2;
+        s += kEvery;
         if (s >= p.stages) { s -= p.stages; parity ^= 1; }
       }
     }
@@ -287,7 +292,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb * 32);
         tmem_ld32(at, v);
         if (EXACT) {
-          const int used = min(p.nacc, n_slabs);
+          const int used = min(p.nacc, n_steps);
 #pragma unroll 1
           for (int a = 1; a <= used; ++a) {
             float w[32];
@@ -486,16 +491,17 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count) {
   SmallPlan best{64, 1, 0};
   for (int bn : {64, 128}) {
-    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : (bn == 64 ? 465 : 500);
-    const int64_t once = bn == 64 ? 8300 : 10800;
+    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : (bn == 64 ? 302 : 406);
+    const int64_t once = (bn == 64 ? 7500 : 10050) + (mode == SMALL_EXACT ? 600 : 0);
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
     for (int s : {1, 2, 4, 8}) {
-      if (s > slabs) break;
+      const int64_t steps = (slabs + slabs_per_step(mode) - 1) / slabs_per_step(mode);
+      if (s > steps) break;
       // (exact FP32: at most 1024 of K in one accumulator)
       if (mode == SMALL_EXACT && (slabs + s - 1) / s > 32 * exact_accumulators(bn)) continue;
       const int64_t resident = resident_clusters(s, sm_count);
       const int64_t rounds = (tiles + resident - 1) / resident;
-      const int64_t cycles = rounds * (((slabs + s - 1) / s) * step + once + (s == 8 ? 1700 : s == 4 ? 500 : 0));
+      const int64_t cycles = rounds * ((steps + s - 1) / s * slabs_per_step(mode) * step + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
       if (best.cycles == 0 || cycles < best.cycles) best = {bn, s, cycles};
     }
   }
@@ -531,20 +537,21 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
   const int slab_k = ops.bf16 ? 64 : 32, chunk = ops.bf16 ? 64 : 32;
   p.slab_k = slab_k;
-  p.num_slabs = (int)((k.K + slab_k - 1) / slab_k);
-  const SmallPlan how = plan_small(k.M, k.N, p.num_slabs, mode, plan.sm_count);
+  const int slabs = (int)((k.K + slab_k - 1) / slab_k), per_step = slabs_per_step(mode);
+  p.num_steps = (slabs + per_step - 1) / per_step;
+  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, plan.sm_count);
   const int bn = how.bn;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
-  const int stage_bytes = kSmallABytes + (mode == SMALL_EXACT ? 2 : 1) * bn * 128;
-  const int most = (p.num_slabs + p.splits - 1) / p.splits;
+  const int stage_bytes = per_step * kSmallABytes + 2 * bn * 128;
+  const int most = (p.num_steps + p.splits - 1) / p.splits;
   p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
   const int tile_bytes = kSmallM * bn * 4;
   // the others' parts of a band, and the own partial tile where the ring cannot hold it
   auto exchange_of = [&](int stages) { return tile_bytes / p.splits * (p.splits - 1) + (stages * stage_bytes >= tile_bytes ? 0 : tile_bytes); };
   while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
-  if (p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
+  if (mode == SMALL_EXACT && p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
   const int exchange = exchange_of(p.stages);
   st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
   st->grid = (unsigned)(tiles * p.splits);
