@@ -5,7 +5,8 @@
 //   ew_chain_vec4   the tape is a chain and every operand is contiguous (or constant) along the
 //                   innermost dim: 128-bit loads/stores, the running value stays in registers.
 //                   HBM-bound: reads each input once, writes the output once.
-//   ew_chain        the same with one element per access, for widths and alignments 128 bits cannot take.
+//   ew_chain        the same for widths and alignments that 128 bits cannot take: float4 along the flat
+//                   tensor where the output and the first input are dense, else one element per access.
 //   ew_transpose    a chain whose first input is contiguous along a different dim than the output
 //                   (head-split K^T copy, unfrozen weight transposes): 32x32 tiles through shared
 //                   memory so both the read and the write are coalesced.
@@ -135,6 +136,84 @@ __global__ void __launch_bounds__(256) ew_chain_kernel(const __grid_constant__ E
       float* out = p.ptr[p.chain.out_slot] + ew_offset<RANK>(p, p.chain.out_slot, idx[u]);
       if (VEC == 1) *out = v[u];
       else *reinterpret_cast<float4*>(out) = make_float4(v[VEC * u], v[VEC * u + 1], v[VEC * u + 2], v[VEC * u + VEC - 1]);
+    }
+  }
+}
+
+// Two dims, any width: the output and the first input are dense, so the tensor is walked as float4 whose elements
+// may belong to two rows.  Other dense operands come the same way, the rest (a value per column or per
+// row) element by element, from cache.  bias + GELU 8192 x 4093: 79.6 us as single elements, 51 % of
+// the copy bandwidth.
+struct EwFlatParams {
+  uint32_t numel, inner, magic;
+  int shift;
+  float* ptr[KB200_MAX_OPERANDS];
+  int32_t stride_row[KB200_MAX_OPERANDS], stride_col[KB200_MAX_OPERANDS];
+  uint32_t dense;                // bit per operand
+  Chain chain;
+};
+
+template <int U>
+__global__ void __launch_bounds__(256) ew_flat_kernel(const __grid_constant__ EwFlatParams p) {
+  pdl_wait();                 // the producer of this kernel's inputs has completed
+  pdl_launch_dependents();    // the next kernel may begin its start-up
+  const uint32_t nvec = (p.numel + 3) >> 2, step = gridDim.x * blockDim.x * U;
+  for (uint32_t base = blockIdx.x * blockDim.x * U + threadIdx.x; base < nvec; base += step) {
+    float v[4 * U];
+    uint32_t row[U] = {}, col[U] = {};
+    auto load = [&](int slot, int u, float* x) {
+      const uint32_t f = (base + (uint32_t)u * blockDim.x) * 4;
+      if ((p.dense >> slot) & 1) {
+        if (f + 4 <= p.numel) {
+          const float4 t = *reinterpret_cast<const float4*>(p.ptr[slot] + f);
+          x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = f + e < p.numel ? p.ptr[slot][f + e] : 0.0f;
+        }
+      } else {
+        uint32_t r = row[u], c = col[u];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x[e] = f + e < p.numel ? __ldg(p.ptr[slot] + r * (uint32_t)p.stride_row[slot] + c * (uint32_t)p.stride_col[slot]) : 0.0f;
+          if (++c == p.inner) { c = 0; ++r; }
+        }
+      }
+    };
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + (uint32_t)u * blockDim.x;
+      if (i < nvec) {
+        row[u] = (uint32_t)(((uint64_t)(i * 4) * p.magic) >> p.shift);
+        col[u] = i * 4 - row[u] * p.inner;
+        load(p.chain.first_slot, u, v + 4 * u);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[4 * u + e] = 0.0f;
+      }
+    }
+    for (int s = 0; s < p.chain.n; ++s) {
+      const ChainStep st = p.chain.steps[s];
+      float side[4 * U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) side[4 * u + e] = st.imm;
+        if (st.slot >= 0 && base + (uint32_t)u * blockDim.x < nvec) load(st.slot, u, side + 4 * u);
+      }
+      chain_step<4 * U>(st.op, v, side);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t f = (base + (uint32_t)u * blockDim.x) * 4;
+      float* out = p.ptr[p.chain.out_slot] + f;
+      if (f + 4 <= p.numel) {
+        *reinterpret_cast<float4*>(out) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (f + e < p.numel) out[e] = v[4 * u + e];
+      }
     }
   }
 }
@@ -307,13 +386,48 @@ static void launch_chain(const Plan& plan, const PlanKernel& k, cudaStream_t s) 
   }
 }
 
+// Does ew_flat_kernel take this chain (already known to fit 32-bit offsets)?
+static bool flat_ok(const PlanKernel& k) {
+  const kb200_kernel_desc& d = k.desc;
+  if (d.iter_rank != 2 || numel_of(d) > (int64_t(1) << 30)) return false;
+  for (int slot : {k.chain.first_slot, k.chain.out_slot}) {
+    const DevOperand& o = k.ops[slot];
+    if (o.stride[1] != 1 || o.stride[0] != d.iter_shape[1] || (reinterpret_cast<uintptr_t>(o.ptr) & 15)) return false;
+  }
+  return true;
+}
+
+static void launch_flat(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
+  const kb200_kernel_desc& d = k.desc;
+  EwFlatParams p{};
+  p.numel = (uint32_t)numel_of(d);
+  p.inner = (uint32_t)d.iter_shape[1];
+  int log = 0;
+  while ((uint64_t(1) << log) < p.inner) ++log;
+  p.shift = 31 + log;
+  p.magic = (uint32_t)(((uint64_t(1) << p.shift) + p.inner - 1) / p.inner);
+  for (int o = 0; o < d.n_operands; ++o) {
+    const DevOperand& op = k.ops[o];
+    p.ptr[o] = op.ptr;
+    p.stride_row[o] = (int32_t)op.stride[0];
+    p.stride_col[o] = (int32_t)op.stride[1];
+    if (op.stride[1] == 1 && op.stride[0] == d.iter_shape[1] && (reinterpret_cast<uintptr_t>(op.ptr) & 15) == 0) p.dense |= 1u << o;
+  }
+  p.chain = k.chain;
+  constexpr int U = 2;
+  const int64_t blocks = ((int64_t)p.numel + 1024 * U - 1) / (1024 * U), cap = (int64_t)plan.sm_count * 64;
+  const int64_t steps = (blocks + cap - 1) / cap;
+  launch_kernel(plan.pdl, ew_flat_kernel<U>, dim3((unsigned)((blocks + steps - 1) / (steps > 0 ? steps : 1))), dim3(256), 0, s, p);
+}
+
 int launch_elementwise(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   const kb200_kernel_desc& d = k.desc;
   const int64_t numel = numel_of(d);
   if (k.impl == IMPL_EW_CHAIN_VEC4) {
     launch_chain<2, 4>(plan, k, s);
   } else if (k.impl == IMPL_EW_CHAIN) {
-    launch_chain<8, 1>(plan, k, s);
+    if (flat_ok(k)) launch_flat(plan, k, s);
+    else launch_chain<8, 1>(plan, k, s);
   } else if (k.impl == IMPL_EW_TRANSPOSE) {
     EwTransposeParams p{};
     p.rank = d.iter_rank;

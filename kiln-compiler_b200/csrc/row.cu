@@ -135,6 +135,7 @@ struct RowFastParams {
     int64_t stride0, stride1;
     int inner_stride;      // 1, or 0 for one value per row
   } pre[kMaxRowPre];
+  const float* x_end;      // behind x's last element
   float* pre_out;          // receives the chain's value (same shape as x), or null
   int64_t pre_out_stride0, pre_out_stride1;
 };
@@ -171,12 +172,20 @@ __device__ __forceinline__ float row_fold(const float (&v)[VEC]) { return VEC ==
 // now 16).  PRE: a chain in front of the reductions; its
 // switch over the scalar ops, unrolled over a lane's elements, costs a softmax of 512 columns 54
 // registers instead of 32.
-template <int MODE, int VEC, int N, bool WIDE, bool PRE>
+//
+// SHIFT: rows that start off a 16-byte boundary by a number of floats that varies with the row (odd widths).
+// The accesses are the aligned float4 that cover a row; of the first and last one only the row's own
+// elements count, the neighbours' are read with them and left alone.  x and out have the same shift;
+// the last float4 of the tensor is read element by element where it would reach past its end.
+// Softmax only (16384 x 333: 18.0 us with single floats, 10.2; 16384 x 4093: 124, 114): the affine parameters of
+// a LayerNorm would still come as single floats, four lanes apart, and 16384 x 771 took 30.9 us against 28.2.
+template <int MODE, int VEC, int N, bool WIDE, bool PRE, bool SHIFT, bool AHEAD>
 __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_constant__ RowFastParams p) {
   const int lane = WIDE ? threadIdx.x : (threadIdx.x & 31);
   const int lanes = WIDE ? blockDim.x : 32;
   const int64_t row = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int units = VEC == 1 ? p.inner : p.inner >> 2;
+  static_assert(!SHIFT || (VEC == 4 && !PRE && MODE == ROW_SOFTMAX), "shifted rows come as float4, without operands beside them");
+  const int units = SHIFT ? (p.inner + 6) >> 2 : VEC == 1 ? p.inner : p.inner >> 2;
   __shared__ float partial[WIDE ? 64 : 1];
   // Each reduction of a WIDE row has its own half of `partial`: no barrier between the reads of one and the writes of the next.
   auto across = [&](float v, bool is_max, int which) {
@@ -190,10 +199,11 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
   };
   // The affine parameters of a LayerNorm are constants of the plan, not outputs of the previous
   // kernel: they are fetched before this kernel waits for its producer, so their latency is off the
-  // path (fetched after the two reductions they added a dependent memory round trip to every row).  The
-  // other rows of a WIDE block's SM cover that round trip, and its registers are worth more: there they
-  // are fetched where they are used.
-  constexpr bool kAhead = MODE == ROW_LAYERNORM && !WIDE;
+  // path (fetched after the two reductions they added a dependent memory round trip to every row).  Where other
+  // rows on the SM cover that round trip their registers are worth more: in WIDE blocks, and with rows of
+  // four or more float4 a lane in several waves, they are fetched where they are used (16384 x 768:
+  // 19.6 -> 17.9 us).
+  constexpr bool kAhead = MODE == ROW_LAYERNORM && AHEAD;
   float g[kAhead ? N : 1][VEC], b[kAhead ? N : 1][VEC];
   if (kAhead) {
 #pragma unroll
@@ -211,15 +221,31 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
   int64_t i0 = row, i1 = 0;
   if (p.rows_inner > 0) { i0 = row / p.rows_inner; i1 = row - i0 * p.rows_inner; }
   const float* x = p.x + i0 * p.x_row_stride + i1 * p.x_stride1;
-  const int64_t out_off = i0 * p.out_row_stride + i1 * p.out_stride1;
+  int64_t out_off = i0 * p.out_row_stride + i1 * p.out_stride1;
+  // element e of access j is column 4 j + e - shift
+  const int shift = SHIFT ? (int)((reinterpret_cast<uintptr_t>(x) >> 2) & 3) : 0;
+  x -= shift;
+  out_off -= shift;
+  auto column_ok = [&](int j, int e) { return !SHIFT || (unsigned)(4 * j + e - shift) < (unsigned)p.inner; };
   float* out = p.out + out_off;
   float v[N][VEC];
   bool live[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const int j = lane + lanes * i;
-    live[i] = j < units;
-    if (live[i]) row_load<VEC>(v[i], x + VEC * j);
+    live[i] = SHIFT ? 4 * j - shift < p.inner : j < units;
+    if (!live[i]) continue;
+    if (!SHIFT || x + VEC * j + VEC <= p.x_end) {
+      row_load<VEC>(v[i], x + VEC * j);
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[i][e] = column_ok(j, e) ? x[VEC * j + e] : 0.0f;
+    }
+    if (SHIFT) {                 // what a neighbour's element must be for this row's reduction
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        if (!column_ok(j, e)) v[i][e] = -CUDART_INF_F;
+    }
   }
   for (int s = 0; PRE && s < p.n_pre; ++s) {
     const RowFastParams::Pre st = p.pre[s];
@@ -310,7 +336,7 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
         // one warp and 128-bit accesses: exp through ex2.approx (relative error 2^-22, what the reference's
         // tl.exp lowers to as well); the forms that took over from the tape interpreter keep its expf
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) v[i][e] = VEC == 1 || WIDE ? expf(v[i][e] - m) : __expf(v[i][e] - m);
+        for (int e = 0; e < VEC; ++e) v[i][e] = VEC == 1 || WIDE || SHIFT ? expf(v[i][e] - m) : __expf(v[i][e] - m);
         s += row_fold<VEC>(v[i]);
       }
     }
@@ -322,54 +348,87 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
         float y[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) y[e] = v[i][e] * inv;
-        row_store<VEC>(out + VEC * (lane + lanes * i), y);
+        const int j = lane + lanes * i;
+        if (column_ok(j, 0) && column_ok(j, VEC - 1)) {
+          row_store<VEC>(out + VEC * j, y);
+        } else {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e)
+            if (column_ok(j, e)) out[VEC * j + e] = y[e];
+        }
       }
     }
   }
 }
 
 // The widest row: 16 warps (more would halve the registers of a thread) of 8 float4 or 32 floats a lane.
-constexpr int64_t kRowLimit = 512 * 32;
+constexpr int64_t kRowLimit = 512 * 32, kShiftedLimit = kRowLimit - 8;
+
+enum { ROW_FLOATS = 0, ROW_VECTORS = 1, ROW_SHIFTED = 2 };      // how rows are accessed
 
 template <int MODE, bool PRE>
-static void launch_rows(const RowFastParams& p, bool vec, int sm_count, bool pdl, cudaStream_t s) {
-  const int units = vec ? p.inner / 4 : p.inner;
+static void launch_rows(const RowFastParams& p, int access, int sm_count, bool pdl, cudaStream_t s) {
+  const bool vec = access != ROW_FLOATS;
+  const int units = access == ROW_SHIFTED ? (p.inner + 6) / 4 : vec ? p.inner / 4 : p.inner;
   const int n = (units + 31) / 32;                  // accesses per lane if one warp takes the row
-#define KB200_ROW_CASE(VEC, N, WIDE) launch_kernel(pdl, row_kernel<MODE, VEC, N, WIDE, PRE>, dim3(grid), dim3(block), 0, s, p)
+  unsigned grid, block;
+#define KB200_ROW_CASE(VEC, N, WIDE, AHEAD) launch_kernel(pdl, row_kernel<MODE, VEC, N, WIDE, PRE, false, AHEAD>, dim3(grid), dim3(block), 0, s, p)
+#define KB200_SHIFT_CASE(N, WIDE) launch_kernel(pdl, row_kernel<MODE, 4, N, WIDE, false, true, false>, dim3(grid), dim3(block), 0, s, p)
   if (n <= (vec && MODE == ROW_LAYERNORM ? 6 : 8)) {
     // a warp per row; few rows spread over more blocks.  (A LayerNorm of 8 float4 a lane, or either of 12,
     // spills; four warps of a quarter each do not.)
     const int warps = p.n_rows >= (int64_t)sm_count * 16 ? 8 : (p.n_rows >= (int64_t)sm_count * 4 ? 4 : 1);
-    const unsigned grid = (unsigned)((p.n_rows + warps - 1) / warps), block = warps * 32;
+    grid = (unsigned)((p.n_rows + warps - 1) / warps);
+    block = warps * 32;
+    if constexpr (!PRE && MODE == ROW_SOFTMAX) {
+      if (access == ROW_SHIFTED) {
+        if (n <= 2) KB200_SHIFT_CASE(2, false);
+        else if (n <= 4) KB200_SHIFT_CASE(4, false);
+        else KB200_SHIFT_CASE(8, false);
+        return;
+      }
+    }
+    const bool few = MODE == ROW_SOFTMAX || p.n_rows < (int64_t)sm_count * 64;
     if (vec) {
-      if (n <= 1) KB200_ROW_CASE(4, 1, false);
-      else if (n <= 2) KB200_ROW_CASE(4, 2, false);
-      else if (n <= 4) KB200_ROW_CASE(4, 4, false);
-      else if (n <= 6) KB200_ROW_CASE(4, 6, false);
-      else if constexpr (MODE == ROW_SOFTMAX) KB200_ROW_CASE(4, 8, false);
+      if (n <= 1) KB200_ROW_CASE(4, 1, false, true);
+      else if (n <= 2) KB200_ROW_CASE(4, 2, false, true);
+      else if (n <= 4 && few) KB200_ROW_CASE(4, 4, false, true);
+      else if (n <= 4) KB200_ROW_CASE(4, 4, false, false);
+      else if (n <= 6 && few) KB200_ROW_CASE(4, 6, false, true);
+      else if (n <= 6) KB200_ROW_CASE(4, 6, false, false);
+      else if constexpr (MODE == ROW_SOFTMAX) KB200_ROW_CASE(4, 8, false, true);
     } else {
-      if (n <= 2) KB200_ROW_CASE(1, 2, false);
-      else if (n <= 4) KB200_ROW_CASE(1, 4, false);
-      else KB200_ROW_CASE(1, 8, false);
+      if (n <= 2) KB200_ROW_CASE(1, 2, false, true);
+      else if (n <= 4) KB200_ROW_CASE(1, 4, false, true);
+      else KB200_ROW_CASE(1, 8, false, true);
     }
     return;
   }
   // a block per row, of as many warps (up to 16) as 4 float4 or 8 floats a lane leave
   int per = vec ? 4 : 8;
   while (per * 16 < n) per *= 2;
-  const unsigned grid = (unsigned)p.n_rows, block = (unsigned)((n + per - 1) / per) * 32;
-  if (vec && per == 4) KB200_ROW_CASE(4, 4, true);
-  else if (vec) KB200_ROW_CASE(4, 8, true);
-  else if (per == 8) KB200_ROW_CASE(1, 8, true);
-  else if (per == 16) KB200_ROW_CASE(1, 16, true);
-  else KB200_ROW_CASE(1, 32, true);
+  grid = (unsigned)p.n_rows;
+  block = (unsigned)((n + per - 1) / per) * 32;
+  if constexpr (!PRE && MODE == ROW_SOFTMAX) {
+    if (access == ROW_SHIFTED) {
+      if (per == 4) KB200_SHIFT_CASE(4, true);
+      else KB200_SHIFT_CASE(8, true);
+      return;
+    }
+  }
+  if (vec && per == 4) KB200_ROW_CASE(4, 4, true, false);
+  else if (vec) KB200_ROW_CASE(4, 8, true, false);
+  else if (per == 8) KB200_ROW_CASE(1, 8, true, false);
+  else if (per == 16) KB200_ROW_CASE(1, 16, true, false);
+  else KB200_ROW_CASE(1, 32, true, false);
 #undef KB200_ROW_CASE
+#undef KB200_SHIFT_CASE
 }
 
 template <int MODE>
-static void launch_row_fast(const RowFastParams& p, bool vec, int sm_count, bool pdl, cudaStream_t s) {
-  if (p.n_pre > 0 || p.pre_out != nullptr) launch_rows<MODE, true>(p, vec, sm_count, pdl, s);
-  else launch_rows<MODE, false>(p, vec, sm_count, pdl, s);
+static void launch_row_fast(const RowFastParams& p, int access, int sm_count, bool pdl, cudaStream_t s) {
+  if (p.n_pre > 0 || p.pre_out != nullptr) launch_rows<MODE, true>(p, access, sm_count, pdl, s);
+  else launch_rows<MODE, false>(p, access, sm_count, pdl, s);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -446,6 +505,7 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     p.x_stride1 = two ? k.ops[k.x_slot].stride[1] : 0;
     p.out_stride1 = two ? k.ops[k.out_slot].stride[1] : 0;
     p.n_pre = k.row_pre.n;
+    p.x_end = p.x + (n_rows > 0 ? k.ops[k.x_slot].stride[0] * (d.iter_shape[0] - 1) + p.x_stride1 * (two ? d.iter_shape[1] - 1 : 0) + inner : 0);
     for (int st = 0; st < k.row_pre.n; ++st) {
       const ChainStep& cs = k.row_pre.steps[st];
       RowFastParams::Pre& pr = p.pre[st];
@@ -460,6 +520,15 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
         pr.inner_stride = (int)o.stride[d.iter_rank - 1];
       }
     }
+    // Softmax rows that do not start on 16 bytes: shifted float4, when x and the output are shifted alike in every
+    // row and no chain in front brings operands of its own.
+    int access = k.row_vec ? ROW_VECTORS : ROW_FLOATS;
+    {
+      const DevOperand &x = k.ops[k.x_slot], &o = k.ops[k.out_slot];
+      bool alike = aligned16(x.ptr) && aligned16(o.ptr);
+      for (int dd = 0; dd < d.iter_rank - 1; ++dd) alike = alike && (x.stride[dd] - o.stride[dd]) % 4 == 0;
+      if (k.impl == IMPL_ROW_SOFTMAX && !k.row_vec && alike && k.row_pre.n == 0 && k.pre_out_slot < 0 && inner >= 32 && inner <= kShiftedLimit) access = ROW_SHIFTED;
+    }
     p.pre_out = k.pre_out_slot >= 0 ? k.ops[k.pre_out_slot].ptr : nullptr;
     p.pre_out_stride0 = k.pre_out_slot >= 0 ? k.ops[k.pre_out_slot].stride[0] : 0;
     p.pre_out_stride1 = k.pre_out_slot >= 0 && two ? k.ops[k.pre_out_slot].stride[1] : 0;
@@ -470,9 +539,9 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
       p.eps = k.ln_eps;
       p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
       p.store32 = (k.mirror_only && p.out16 != nullptr) ? 0 : 1;
-      launch_row_fast<ROW_LAYERNORM>(p, k.row_vec, plan.sm_count, plan.pdl, s);
+      launch_row_fast<ROW_LAYERNORM>(p, access, plan.sm_count, plan.pdl, s);
     } else {
-      launch_row_fast<ROW_SOFTMAX>(p, k.row_vec, plan.sm_count, plan.pdl, s);
+      launch_row_fast<ROW_SOFTMAX>(p, access, plan.sm_count, plan.pdl, s);
     }
   } else {
     RowParams p{};

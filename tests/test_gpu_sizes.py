@@ -36,7 +36,7 @@ def check(case, impls=None, calls=1):
 
 
 @pytest.mark.parametrize("rows", [1, 700])
-@pytest.mark.parametrize("d", [1, 3, 31, 33, 64, 127, 255, 257, 772, 1000, 1028, 2047, 2052, 4097, 8191, 8196, 16384])
+@pytest.mark.parametrize("d", [1, 3, 31, 32, 33, 34, 35, 64, 127, 250, 255, 257, 772, 1021, 1000, 1028, 2047, 2052, 4097, 8191, 8196, 16384])
 def test_rows_of_any_width(d, rows):
     check({"kind": "layernorm", "rows": rows, "d": d}, ["row_layernorm"])
     check({"kind": "softmax", "heads": 1, "rows": rows, "cols": d}, ["row_softmax"])
@@ -46,7 +46,7 @@ def test_rows_beyond_the_registers():
     check({"kind": "layernorm", "rows": 3, "d": 16388}, ["row_generic"])
 
 
-@pytest.mark.parametrize("rows,d", [(1, 5), (7, 33), (513, 1001), (65, 2050), (2047, 255)])
+@pytest.mark.parametrize("rows,d", [(1, 5), (3, 1), (7, 33), (513, 1001), (65, 2050), (2047, 255), (5, 3), (1000, 2047)])
 def test_elementwise_chain_of_any_width(rows, d):
     check({"kind": "bias_gelu", "rows": rows, "d": d}, ["ew_chain"])
 
