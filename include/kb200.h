@@ -15,7 +15,9 @@
  * synchronised, only while a plan is set up: kb200_plan_create allocates the
  * plan's status word, and kb200_plan_bind allocates the library-owned scratch
  * (in BF16 mode a bf16 mirror of the arena and packed bf16 copies of constant
- * matmul operands; a staging buffer for a fused attention whose output aliases
+ * matmul operands; in the other modes copies of them laid out along K and, for
+ * exact FP32, their tails, where memory is plenty; aligned copies of operands
+ * that a tensor map cannot describe; a staging buffer for a fused attention whose output aliases
  * its inputs; in FP32 mode the fused attention's scratch: the operands' tails or
  * the split tiles' partial results), converts the constants (cudaDeviceSynchronize) and reads the
  * attention mask back once (a blocking copy).  kb200_plan_launch and

@@ -17,7 +17,8 @@
 // The sum over the splits runs in rank order, so results do not depend on timing.
 //
 // Per CTA, 352 threads: warp 0 loads A, warp 10 loads B, warp 1 issues the MMAs, warps 2-9 (two per tensor-memory
-// lane quadrant) split A in the exact-FP32 mode, then drain, exchange and finish.  Waits are bounded as
+// lane quadrant) move A to tensor memory, then drain, exchange and finish.  An A that a tensor map cannot describe, or
+// that is float32 where the MMAs want bf16, is read by warps 2-9 themselves (GATHER).  Waits are bounded as
 // in matmul_tc.cu.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -43,7 +44,9 @@ constexpr int kSmallABytes = kSmallM * 128;      // one 128-byte K slab
 constexpr int kSmallACols = 128;                 // tensor-memory columns for slabs of A
 constexpr int kSmallSmem = 225 * 1024;
 
-enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2 };
+// SMALL_BF16_A32: bf16 products of an A that is still float32, rounded on its way to tensor memory.  (A Linear of the caller's
+// own input; a launch that made a bf16 copy of it cost ~2.3 us in front of this one.)
+enum : int { SMALL_TF32 = 0, SMALL_BF16 = 1, SMALL_EXACT = 2, SMALL_BF16_A32 = 3 };
 enum : int { FIN_NONE = 0, FIN_BIAS, FIN_BIAS_GELU, FIN_BIAS_RES };
 
 struct SmallParams {
@@ -60,17 +63,58 @@ struct SmallParams {
   const float* bias;
   const float* res;
   int64_t res_row;
+  const float* a;                  // GATHER: A as it is in memory, rows of K elements a_row apart
+  int64_t a_row;
+  int K;
+  int a_rows;                      // rows of a box of A: the tile's, or M where that is less
   float* out;                      // null: only the bf16 copy is stored
   __nv_bfloat16* out16;            // or null
   int64_t out_row;                 // of both
 };
 
 // 128-byte slabs of K per pipeline step.  A step costs the issuing warp ~400 cycles of wait, branches and commits
-// beside ~25 per MMA; exact FP32 has twelve MMAs to a slab and no room for more.
-__host__ __device__ constexpr int slabs_per_step(int mode) { return mode == SMALL_EXACT ? 1 : 2; }
+// beside ~25 per MMA; exact FP32 has twelve MMAs to a slab and, like the float32 A, no room for more.
+__host__ __device__ constexpr int slabs_per_step(int mode) { return mode == SMALL_EXACT || mode == SMALL_BF16_A32 ? 1 : 2; }
+// A stage: the slabs of A (one of float32 for bf16 products is two boxes of 32 columns), then those of B (exact FP32: and its tails)
+__host__ __device__ constexpr int a_slab_bytes(int mode) { return mode == SMALL_BF16_A32 ? 2 * kSmallABytes : kSmallABytes; }
+__host__ __device__ constexpr int b_boxes(int mode) { return mode == SMALL_BF16_A32 ? 1 : 2; }
+__host__ __device__ constexpr int stage_bytes_of(int mode, int bn) { return slabs_per_step(mode) * a_slab_bytes(mode) + b_boxes(mode) * bn * 128; }
 
-// BN: columns of a tile, 64 or 128.
-template <int MODE, int FIN, int BN>
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// This warp's 32 rows of a slab of A, for GATHER: float32 in global memory, rows from any element on.  Lane l has column l
+// of every row (BF16: columns 2l and 2l + 1), so that a warp reads whole lines.  Rows past the last are the last one
+// again (they make accumulator rows that nobody reads), columns past K are zeros.
+template <bool BF16>
+__device__ __forceinline__ void gather_rows(float (&raw)[BF16 ? 64 : 32], const SmallParams& p, int row0, int col0, int lane) {
+  const int last = p.M - 1;
+  constexpr int kCols = BF16 ? 2 : 1;
+  const int col = col0 + kCols * lane;
+#pragma unroll
+  for (int r = 0; r < 32; ++r) {
+    const float* const at = p.a + min(row0 + r, last) * p.a_row + col;
+#pragma unroll
+    for (int c = 0; c < kCols; ++c) raw[kCols * r + c] = col + c < p.K ? at[c] : 0.f;
+  }
+}
+
+// The same rows into a slab of A as the copy engine would have left them: 128-byte rows, 16-byte units XORed with the row.
+template <bool BF16>
+__device__ __forceinline__ void park_rows(uint8_t* slab, const float (&raw)[BF16 ? 64 : 32], int row0, int lane) {
+#pragma unroll
+  for (int r = 0; r < 32; ++r) {
+    const int row = row0 + r;
+    uint32_t* const at = reinterpret_cast<uint32_t*>(slab + row * 128 + (((lane >> 2) ^ (row & 7)) << 4)) + (lane & 3);
+    *at = BF16 ? pack_bf16(raw[(2 * r) % (BF16 ? 64 : 32)], raw[(2 * r + 1) % (BF16 ? 64 : 32)]) : __float_as_uint(raw[r]);
+  }
+}
+
+// BN: columns of a tile, 64 or 128.  GATHER: warps 2-9 read A from global memory.  Of a Linear of 333 x 1000 x 771 the
+// pass that copied A to aligned rows, and the one that made bf16 of a float32 A, was a launch of ~2.3 us in front of this one.
+template <int MODE, int FIN, int BN, bool GATHER>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                 const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
@@ -80,13 +124,15 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr int kABuffers = 2;                                  // steps of A in tensor memory, 64 columns each
   constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
   constexpr int kSlabs = slabs_per_step(MODE);
-  constexpr int kStage = kSlabs * kSmallABytes + 2 * kSmallBBytes;     // the slabs of A, then those of B; exact FP32: A, B, the tails of B
+  constexpr bool A32 = MODE == SMALL_BF16_A32, BF16 = MODE == SMALL_BF16 || A32;
+  constexpr bool ALTERNATE = kSlabs == 1;                       // the two groups of warps that move A take alternate steps
+  constexpr int kSlabA = a_slab_bytes(MODE), kBBoxes = b_boxes(MODE), kStage = stage_bytes_of(MODE, BN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 6];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t ring = (raw + 1023u) & ~1023u;
+  const uint32_t raw_at = smem_u32(smem_raw);
+  const uint32_t ring = (raw_at + 1023u) & ~1023u;
   // This CTA's partial tile in 32 x 32 blocks of 4 KB: in the ring, idle by then, where it is large enough
   const bool in_ring = p.stages * kStage >= kTileBytes;
   const uint32_t recv = in_ring ? ring : ring + (uint32_t)(p.stages * kStage);
@@ -103,9 +149,9 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full0 + 8 * s, 2);
+      mbar_init(full0 + 8 * s, GATHER ? 1 : 2);
       mbar_init(empty0 + 8 * s, 1);
-      mbar_init(split0 + 8 * s, EXACT ? kSmallEpiWarps / 2 : kSmallEpiWarps);
+      mbar_init(split0 + 8 * s, ALTERNATE ? kSmallEpiWarps / 2 : kSmallEpiWarps);
     }
     mbar_init(done, 1);
     mbar_init(received, 1);
@@ -148,26 +194,26 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (!got && lane == 0) give_up(site);
     return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
   };
-  if (warp == 0 || warp == 10) {
+  if ((warp == 0 && !GATHER) || warp == 10) {
     // ---------------- TMA producers, one per operand ----------------
-    const bool is_a = warp == 0;
+    const bool is_a = !GATHER && warp == 0;
     int s = 0, k_elem = step0 * kSlabs * p.slab_k;
     uint32_t parity = 1;
     for (int i = 0; i < n_steps; ++i) {
       if (i >= p.stages && !all_waited(mbar_wait(empty0 + 8 * s, parity, abort_ptr), 1)) break;
-      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kSlabs * kSmallABytes;
+      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kSlabs * kSlabA;
       if (elect_one()) {
-        mbar_expect_tx(bar, is_a ? kSlabs * kSmallABytes : 2 * kSmallBBytes);
+        mbar_expect_tx(bar, is_a ? kSlabs * (kSlabA / kSmallM) * p.a_rows : kBBoxes * kSmallBBytes);
         // (a slab past the end of K, in the last step of an odd number, is a box outside the tensor: zeros)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const int k = EXACT ? k_elem : k_elem + j * p.slab_k;
+          const int k = EXACT ? k_elem : A32 ? k_elem + j * 32 : k_elem + j * p.slab_k;
           if (is_a) {
-            if (j < kSlabs) tma_load_3d(dst + j * kSmallABytes, &tma_a, bar, k, tm * kSmallM, 0);
-          } else {
+            if (j < kSlabs || A32) tma_load_3d(dst + j * kSmallABytes, &tma_a, bar, k, tm * kSmallM, 0);
+          } else if (j < kBBoxes) {
             const CUtensorMap* map = EXACT && j ? &tma_bt : &tma_b;
             if (p.b_kmajor) tma_load_3d(b_dst + j * kSmallBBytes, map, bar, k, tn * BN, 0);
-            else tma_load_4d(b_dst + j * kSmallBBytes, map, bar, 0, k, tn * (BN / (MODE == SMALL_BF16 ? 64 : 32)), 0);
+            else tma_load_4d(b_dst + j * kSmallBBytes, map, bar, 0, k, tn * (BN / (BF16 ? 64 : 32)), 0);
           }
         }
       }
@@ -175,6 +221,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       k_elem += kSlabs * p.slab_k;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
+  } else if (warp == 0) {
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
@@ -186,7 +233,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // this step's A is in tensor memory (and so its B has landed)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSlabs * kSmallABytes)) >> 4;
+      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSlabs * kSlabA)) >> 4;
       const uint32_t on = elect_one() ? 1u : 0u;
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
       auto desc = [&](uint32_t at) { return b_fixed | (uint64_t)(at & 0x3FFFu); };
@@ -201,7 +248,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           umma_ts_if(on, tmem, ta, desc(b + (kSmallBBytes >> 4)), idesc, 1u, false);
           umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b), idesc, i >= p.nacc || k != 0, false);
         } else {
-          umma_ts_if(on, tmem, ta, desc(b), idesc, (i | k) != 0, MODE == SMALL_BF16);
+          umma_ts_if(on, tmem, ta, desc(b), idesc, (i | k) != 0, BF16);
         }
       }
       if (on) {
@@ -246,25 +293,44 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       // whatever its size: of two groups of four warps, one per lane quadrant, each takes one slab of a step,
       // or, one slab to a step, alternate steps.  (Every stage and buffer then belongs to one group, which
       // sees each phase of its barriers: an even number of stages where the ring is used again.)
-      constexpr int kEvery = EXACT ? 2 : 1;
-      int s = EXACT ? half : 0;
+      constexpr int kEvery = ALTERNATE ? 2 : 1;
+      int s = ALTERNATE ? half : 0;
       uint32_t parity = 0;
       const int row = quad * 32 + lane;
+      // GATHER: a step ahead in registers, then through this warp's rows of the slab in shared memory
+      constexpr int kRaw = BF16 ? 64 : 32;
+      [[maybe_unused]] float raw[GATHER ? kRaw : 1];
+      [[maybe_unused]] auto fetch = [&](int i) {
+        if constexpr (GATHER)
+          gather_rows<BF16>(raw, p, m0 + quad * 32, ((step0 + i) * kSlabs + (ALTERNATE ? 0 : half)) * p.slab_k, lane);
+      };
+      if (GATHER && s < n_steps) fetch(s);
       for (int i = s; i < n_steps && ok; i += kEvery) {
         const int buf = i % kABuffers;
+        if constexpr (GATHER) {
+          // (what the MMAs read of this stage went to tensor memory: only this warp has used its rows)
+          __syncwarp();
+          park_rows<BF16>(smem_raw + (ring - raw_at) + s * kStage + (ALTERNATE ? 0 : half * kSlabA), raw, quad * 32, lane);
+          __syncwarp();
+          if (i + kEvery < n_steps) fetch(i + kEvery);
+        }
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
         if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, ((i / kABuffers) & 1) ^ 1, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint8_t* const src = smem_raw + (ring - raw) + s * kStage + (EXACT ? 0 : half * kSmallABytes) + row * 128;
+        const uint8_t* const src = smem_raw + (ring - raw_at) + s * kStage + (ALTERNATE ? 0 : half * kSlabA) + row * 128;
         float v[32];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 x = *reinterpret_cast<const float4*>(src + ((q ^ (row & 7)) << 4));
-          v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+        for (int q = 0; q < (A32 ? 16 : 8); ++q) {
+          const float4 x = *reinterpret_cast<const float4*>(src + (q >> 3) * kSmallABytes + (((q & 7) ^ (row & 7)) << 4));
+          if (A32) {
+            v[2 * q] = __uint_as_float(pack_bf16(x.x, x.y)); v[2 * q + 1] = __uint_as_float(pack_bf16(x.z, x.w));
+          } else {
+            v[(4 * q) & 31] = x.x; v[(4 * q + 1) & 31] = x.y; v[(4 * q + 2) & 31] = x.z; v[(4 * q + 3) & 31] = x.w;
+          }
         }
-        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 64 + (EXACT ? 0 : half * 32));
+        const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 64 + (ALTERNATE ? 0 : half * 32));
         tmem_st32(at, v);
         if (EXACT) {
 #pragma unroll
@@ -307,7 +373,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         // staged.  (st.async straight from the registers, 16 bytes per lane and packet, took 3700 cycles
         // to land where these take ~1500.)
         const uint32_t block = (uint32_t)((cb * 4 + quad) * 4096);
-        uint8_t* const mine = smem_raw + (recv - raw) + block + lane * 128;
+        uint8_t* const mine = smem_raw + (recv - raw_at) + block + lane * 128;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<float4*>(mine + ((q ^ (lane & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
@@ -341,8 +407,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (ok) {
       // Item by item: row r0 + kRowsAtOnce * j, float4 number u.  A rolled loop: the code runs once, cold, and
       // eight unrolled items were 2000 to 3000 cycles of instruction fetches whatever their number.
-      const uint8_t* const area = smem_raw + (parts0 - raw);
-      const uint8_t* const own = smem_raw + (recv - raw);
+      const uint8_t* const area = smem_raw + (parts0 - raw_at);
+      const uint8_t* const own = smem_raw + (recv - raw_at);
       const int cb = u >> 3;
 #pragma unroll 1
       for (int r = r0; r < band_rows; r += kRowsAtOnce) {
@@ -360,7 +426,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         }
         if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
         if (FIN == FIN_BIAS_GELU) {
-          if (MODE == SMALL_BF16) {
+          if (BF16) {
             y.x = f_gelu_tanh_approx(y.x); y.y = f_gelu_tanh_approx(y.y); y.z = f_gelu_tanh_approx(y.z); y.w = f_gelu_tanh_approx(y.w);
           } else {
             y.x = d_gelu_tanh(y.x); y.y = d_gelu_tanh(y.y); y.z = d_gelu_tanh(y.z); y.w = d_gelu_tanh(y.w);
@@ -411,23 +477,40 @@ struct SmallState {
   unsigned grid = 0;
   size_t smem = 0;
   int bias_slot = -1, res_slot = -1;
+  bool gather = false;                        // warps 2-9 read A
   bool a_moves = false, b_moves = false;      // the maps hold the operand's own address
 };
 
-template <int MODE, int BN>
+template <int MODE, int BN, bool GATHER>
 SmallKernel small_kernel_of(int fin) {
   switch (fin) {
-    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN>;
-    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN>;
-    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN>;
-    default: return mm_small_kernel<MODE, FIN_NONE, BN>;
+    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN, GATHER>;
+    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN, GATHER>;
+    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN, GATHER>;
+    default: return mm_small_kernel<MODE, FIN_NONE, BN, GATHER>;
   }
 }
 
-SmallKernel small_kernel(int mode, int fin, int bn) {
-  if (mode == SMALL_BF16) return bn == 128 ? small_kernel_of<SMALL_BF16, 128>(fin) : small_kernel_of<SMALL_BF16, 64>(fin);
-  if (mode == SMALL_EXACT) return bn == 128 ? small_kernel_of<SMALL_EXACT, 128>(fin) : small_kernel_of<SMALL_EXACT, 64>(fin);
-  return bn == 128 ? small_kernel_of<SMALL_TF32, 128>(fin) : small_kernel_of<SMALL_TF32, 64>(fin);
+template <int MODE>
+SmallKernel small_kernel_of(int fin, int bn, bool gather) {
+  if constexpr (MODE != SMALL_BF16_A32) {
+    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true>(fin) : small_kernel_of<MODE, 64, true>(fin);
+  }
+  return bn == 128 ? small_kernel_of<MODE, 128, false>(fin) : small_kernel_of<MODE, 64, false>(fin);
+}
+
+SmallKernel small_kernel(int mode, int fin, int bn, bool gather) {
+  switch (mode) {
+    case SMALL_BF16: return small_kernel_of<SMALL_BF16>(fin, bn, gather);
+    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32>(fin, bn, gather);
+    case SMALL_EXACT: return small_kernel_of<SMALL_EXACT>(fin, bn, gather);
+    default: return small_kernel_of<SMALL_TF32>(fin, bn, gather);
+  }
+}
+
+int small_mode(int precision, SmallA form) {
+  if (precision == KB200_PREC_FP32) return SMALL_EXACT;
+  return precision != KB200_PREC_BF16 ? SMALL_TF32 : form == SMALL_A_FLOAT32 ? SMALL_BF16_A32 : SMALL_BF16;
 }
 
 // The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.
@@ -467,7 +550,7 @@ int resident_clusters(int splits, int sm_count) {
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS, 64>;
+    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS, 64, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
@@ -488,10 +571,13 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 // at 128 bytes a clock and every MMA reads its operands again (exact FP32: twelve of them, A from tensor
 // memory).  Everything that runs once, launch to exit, is the rest: wide tiles have more to
 // drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
-SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count) {
+// GATHER: a warp loads, parks and reads back a slab of A one step ahead of its use, bound by the load/store unit (rows off the
+// lines: two of them to a load): what it adds to a step against the copied A (65 to 3000 of K).
+SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, bool gather, int sm_count) {
   SmallPlan best{64, 1, 0};
+  const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
   for (int bn : {64, 128}) {
-    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : (bn == 64 ? 302 : 406);
+    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : mode == SMALL_BF16_A32 ? (bn == 64 ? 500 : 550) : (bn == 64 ? 302 : 406);
     const int64_t once = (bn == 64 ? 7500 : 10050) + (mode == SMALL_EXACT ? 600 : 0);
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
     for (int s : {1, 2, 4, 8}) {
@@ -501,7 +587,7 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count
       if (mode == SMALL_EXACT && (slabs + s - 1) / s > 32 * exact_accumulators(bn)) continue;
       const int64_t resident = resident_clusters(s, sm_count);
       const int64_t rounds = (tiles + resident - 1) / resident;
-      const int64_t cycles = rounds * ((steps + s - 1) / s * slabs_per_step(mode) * step + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
+      const int64_t cycles = rounds * ((steps + s - 1) / s * (slabs_per_step(mode) * step + fetch) + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
       if (best.cycles == 0 || cycles < best.cycles) best = {bn, s, cycles};
     }
   }
@@ -510,7 +596,7 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, int sm_count
 
 }  // namespace
 
-int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form) {
   const kb200_kernel_desc& d = k.desc;
   const bool bf16 = d.precision == KB200_PREC_BF16;
   int bias_slot, res_slot;
@@ -524,34 +610,34 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
   if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
   if (((k.M + kSmallM - 1) / kSmallM) * ((k.N + 63) / 64) > 4096) return -1;
   const int slab_k = bf16 ? 64 : 32;
-  const int mode = bf16 ? SMALL_BF16 : d.precision == KB200_PREC_FP32 ? SMALL_EXACT : SMALL_TF32;
-  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, mode, plan.sm_count).cycles;
+  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, small_mode(d.precision, form), form == SMALL_A_GATHERED, plan.sm_count).cycles;
 }
 
-int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, void** state) {
+int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, void** state) {
   *state = nullptr;
   SmallState* st = new SmallState();
   SmallParams& p = st->params;
   const kb200_kernel_desc& d = k.desc;
-  const int mode = ops.bf16 ? SMALL_BF16 : b_tail ? SMALL_EXACT : SMALL_TF32;
+  const int mode = small_mode(d.precision, form);
+  const bool gather = form == SMALL_A_GATHERED;
   const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
   const int slab_k = ops.bf16 ? 64 : 32, chunk = ops.bf16 ? 64 : 32;
   p.slab_k = slab_k;
   const int slabs = (int)((k.K + slab_k - 1) / slab_k), per_step = slabs_per_step(mode);
   p.num_steps = (slabs + per_step - 1) / per_step;
-  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, plan.sm_count);
+  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, gather, plan.sm_count);
   const int bn = how.bn;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
-  const int stage_bytes = per_step * kSmallABytes + 2 * bn * 128;
+  const int stage_bytes = stage_bytes_of(mode, bn);
   const int most = (p.num_steps + p.splits - 1) / p.splits;
   p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
   const int tile_bytes = kSmallM * bn * 4;
   // the others' parts of a band, and the own partial tile where the ring cannot hold it
   auto exchange_of = [&](int stages) { return tile_bytes / p.splits * (p.splits - 1) + (stages * stage_bytes >= tile_bytes ? 0 : tile_bytes); };
   while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
-  if (mode == SMALL_EXACT && p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
+  if (per_step == 1 && p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
   const int exchange = exchange_of(p.stages);
   st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
   st->grid = (unsigned)(tiles * p.splits);
@@ -583,15 +669,24 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
   p.out = k.mirror_only && p.out16 ? nullptr : O.ptr;
   p.out_row = O.stride[1];
-  st->a_moves = ops.a_base == k.ops[d.a_slot].ptr;
+  st->gather = gather;
+  const DevOperand& A = k.ops[d.a_slot];
+  p.a = gather ? A.ptr : nullptr;
+  p.a_row = A.stride[1];
+  p.K = (int)k.K;
+  // (Rows of shared memory that no box fills make accumulator rows that nobody reads.)
+  p.a_rows = (int)(k.M < kSmallM ? k.M : kSmallM);
+  st->a_moves = form == SMALL_A_FLOAT32 || (!gather && ops.a_base == A.ptr);
   st->b_moves = ops.b_base == k.ops[d.b_slot].ptr;
-  bool ok = encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, 1, ops.a_row, 0, slab_k, kSmallM, false);
+  bool ok = gather || (form == SMALL_A_FLOAT32 ? encode_map(&st->map_a, false, A.ptr, k.K, k.M, 1, A.stride[1], 0, 32, p.a_rows, false)
+                                               : encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, 1, ops.a_row, 0, slab_k, p.a_rows, false));
   if (ok && ops.b_kmajor) ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, 1, ops.b_row, 0, slab_k, bn, false);
   else if (ok) ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk, k.K, ops.b_cols / chunk, 1, ops.b_row, 0, slab_k, bn / chunk, !ops.bf16);
+  if (gather) st->map_a = st->map_b;          // not used
   st->map_bt = st->map_b;
   if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = small_kernel(mode, fin, bn);
+  st->kernel = small_kernel(mode, fin, bn, gather);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
   *state = st;
@@ -628,6 +723,7 @@ bool small_repoint(const PlanKernel& k, void* state) {
   SmallState* st = static_cast<SmallState*>(state);
   if (st->bias_slot >= 0) st->params.bias = k.ops[st->bias_slot].ptr;
   if (st->res_slot >= 0) st->params.res = k.ops[st->res_slot].ptr;
+  if (st->gather) st->params.a = k.ops[k.desc.a_slot].ptr;
   if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
   return (!st->a_moves || set_map_address(&st->map_a, k.ops[k.desc.a_slot].ptr)) &&
          (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));

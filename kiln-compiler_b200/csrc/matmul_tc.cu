@@ -1158,15 +1158,21 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const DevOperand& B = k.ops[d.b_slot];
   // A frozen B is laid out along K once: both operands then use the ordinary 128-byte swizzle, and a tile may
   // have any width (an N-major one comes in whole 128-byte column chunks).
+  // In FP32 and TF32 that copy, and the tails of the exact mode, are additions to the weights: where they would
+  // take more than a quarter of what is free, the operand is read as it is.
   const bool frozen = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
-  const bool turn = frozen && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
+  drop_copies(st);
+  size_t free_bytes = 0, total_bytes = 0;
+  KB200_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+  const size_t copied = (size_t)k.N * k.K * sizeof(float) * (d.precision == KB200_PREC_FP32 ? 2 : 1);
+  const bool room = st->bf16 || copied <= free_bytes / 4;
+  const bool turn = frozen && room && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
   const bool b_kmajor = turn || B.stride[2] != 1;
   const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = B.stride[2] != 1 ? B.stride[2] : B.stride[1];
   const void* a_base = A.ptr;
   const void* b_base = B.ptr;
   int64_t a_row = A.stride[1], a_batch = A.stride[0], b_row = b_src_row, b_batch = B.stride[0];
   int64_t b_map_cols = b_cols;           // a copied N-major B is padded to whole 128-byte column chunks: one 4-D box per stage
-  drop_copies(st);
   // Exact FP32: the tails of a frozen B are made here and loaded beside it.  Those of A come from a pass in
   // front of every launch where CTAs walk several tiles (the epilogue warps, who otherwise make them in
   // shared memory, would leave the tensor cores waiting while they drain a tile), with one row of tiles
@@ -1175,7 +1181,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // bytes a clock.
   if (st->small) small_destroy(st->small);
   st->small = nullptr;
-  const bool presplit = d.precision == KB200_PREC_FP32 && frozen && k.batch == 1;
+  const bool presplit = d.precision == KB200_PREC_FP32 && frozen && room && k.batch == 1;
   st->b_copy.once = frozen;
   st->b_copy.turned = turn;
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
@@ -1190,7 +1196,29 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   };
   k.launches = 1;
   cudaError_t made = cudaSuccess;
-  if (copy_a) {
+  // Few tiles: the kernel written for latency, where the other kernels cover the shape too by the estimates of both.
+  // The exact-FP32 form of this file's kernel: 128-column tiles at 1150 cycles per slab (shared memory), ~16500
+  // once, the pass over A included.  A copy of A is a launch of its own, ~4000 cycles; the small kernel can do without.
+  if (copy_b && !b_kmajor) b_map_cols = (b_cols + chunk_n - 1) / chunk_n * chunk_n;
+  SmallA form = SMALL_A_MAPPED;
+  int64_t few = small_cycles(plan, k, b_kmajor, b_map_cols, form);
+  if (few > 0 && copy_a) {
+    const SmallA as_it_is = rows_describable(A, a_row, k.batch) ? SMALL_A_FLOAT32 : SMALL_A_GATHERED;
+    const int64_t direct = small_cycles(plan, k, b_kmajor, b_map_cols, as_it_is);
+    few += 4000;
+    if (direct < few) { form = as_it_is; few = direct; }
+  }
+  int64_t many = 0;
+  if (few > 0 && k.M > kTileM) {
+    const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
+    if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
+    else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
+    if (many > 0 && copy_a) many += 4000;
+  }
+  const bool small = few > 0 && (many == 0 || few < many);
+  if (small && form != SMALL_A_MAPPED) {
+    a_base = nullptr;
+  } else if (copy_a) {
     made = make_copy(st->a_copy, k.M, k.K, unit);
     a_base = st->a_copy.data;
     a_row = st->a_copy.pitch;
@@ -1204,22 +1232,10 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     b_base = st->b_copy.data;
     b_row = st->b_copy.pitch;
     b_batch = b_rows * b_row;
-    if (!b_kmajor) b_map_cols = b_row;
     if (!st->b_copy.once) ++k.launches;
   } else if (st->bf16) {
     b_base = k.b_shadow;
   }
-  // Few tiles: the kernel written for latency.
-  // Where the other kernels cover the shape too, by the estimates of both.  The exact-FP32 form of this
-  // file's kernel: 128-column tiles at 1150 cycles per slab (shared memory), ~16500 once, the pass over A included.
-  const int64_t few = small_cycles(plan, k, b_kmajor, b_map_cols);
-  int64_t many = 0;
-  if (few > 0 && k.M > kTileM) {
-    const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
-    if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
-    else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
-  }
-  const bool small = few > 0 && (many == 0 || few < many);
   const bool a_pass = presplit && k.M > kTileM && !small;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
@@ -1410,9 +1426,10 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
 
   const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor, st->b_copy.once};
   if (small) {
-    const int rc = small_bind(plan, k, kernel_index, po, st->b_tail, &st->small);
+    const int rc = small_bind(plan, k, kernel_index, po, st->b_tail, form, &st->small);
     if (rc) return rc;
     if (st->small) return KB200_OK;
+    if (form != SMALL_A_MAPPED) return fail(KB200_ERR_UNSUPPORTED, "matmul %s: the operands cannot be described to TMA", d.name);
   }
   // More than 128 rows: 256-row tiles on SM pairs (matmul_pair.cu) when that kernel covers the epilogue.
   if (st->pair) {

@@ -180,6 +180,8 @@ class GPUExecutable:
         # what the library allocates itself when buffers are bound, in BF16 mode: a bf16 mirror of the
         # arena, packed bf16 copies of the constant matmul operands, and (worst case) bf16 copies of
         # unmirrored activations no larger than the inputs and the arena together
+        # (the copies of weights that FP32 and TF32 matmuls prefer to read are made only where they leave
+        # most of the free memory, so nothing is set aside for them)
         library_bytes = 0
         if program.precision == "bf16":
             library_bytes = arena_bytes // 2 + 256 + const_bytes // 2 + (io_bytes + arena_bytes) // 2

@@ -84,6 +84,13 @@ def test_few_tiles(m, n, k, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(5, 64, 67), (2, 68, 65), (128, 4096, 129), (33, 768, 3071), (300, 128, 1023), (130, 64, 2050), (1000, 64, 4099)])
+def test_few_tiles_with_rows_on_no_pitch(m, n, k, precision):
+    """A read by the kernel's own warps: rows from any element on, a partial last slab, a ring that is used again."""
+    check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
 @pytest.mark.parametrize("tokens,d", [(3, 132), (64, 512), (128, 1024), (129, 260)])
 def test_mlp_of_few_tokens(tokens, d, precision):
     check({"kind": "mlp", "tokens": tokens, "d": d, "precision": precision}, ["mm_tcgen05"], calls=2)
