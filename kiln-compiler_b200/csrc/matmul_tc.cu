@@ -1187,11 +1187,13 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
   const bool copy_b = st->bf16 ? k.b_shadow == nullptr
                                : turn || !rows_describable(B, b_row, k.batch);
-  const int unit = st->bf16 ? 8 : 4, esz = st->bf16 ? 2 : 4;
-  auto make_copy = [&](TcState::Copy& c, int64_t rows, int64_t cols, int64_t to) {
+  const int esz = st->bf16 ? 2 : 4;
+  // Rows of copies start on 128-byte lines: the 128-byte rows of a box are then one line each and not parts of two
+  // (2048 x 3072 x 771, copy included: TF32 34.0 -> 25.9 us, BF16 23.4 -> 19.5; 333 x 1000 x 771 TF32 9.9 -> 8.8)
+  auto make_copy = [&](TcState::Copy& c, int64_t rows, int64_t cols) {
     c.rows = rows;
     c.cols = cols;
-    c.pitch = (cols + to - 1) / to * to;
+    c.pitch = (cols + chunk_n - 1) / chunk_n * chunk_n;
     return cudaMalloc(&c.data, (size_t)k.batch * rows * c.pitch * esz);
   };
   k.launches = 1;
@@ -1219,7 +1221,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   if (small && form != SMALL_A_MAPPED) {
     a_base = nullptr;
   } else if (copy_a) {
-    made = make_copy(st->a_copy, k.M, k.K, unit);
+    made = make_copy(st->a_copy, k.M, k.K);
     a_base = st->a_copy.data;
     a_row = st->a_copy.pitch;
     a_batch = k.M * a_row;
@@ -1228,7 +1230,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     a_base = k.a_shadow;                 // the mirror has the operand's own strides
   }
   if (copy_b && made == cudaSuccess) {
-    made = make_copy(st->b_copy, b_rows, b_cols, b_kmajor ? unit : chunk_n);
+    made = make_copy(st->b_copy, b_rows, b_cols);
     b_base = st->b_copy.data;
     b_row = st->b_copy.pitch;
     b_batch = b_rows * b_row;
@@ -1239,7 +1241,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const bool a_pass = presplit && k.M > kTileM && !small;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
-    st->tail_pitch = (k.K + 3) / 4 * 4;
+    st->tail_pitch = (k.K + chunk_n - 1) / chunk_n * chunk_n;
     made = cudaMalloc(&st->a_tail, (size_t)k.M * st->tail_pitch * sizeof(float));
     ++k.launches;
   }
