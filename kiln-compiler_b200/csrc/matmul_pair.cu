@@ -34,7 +34,6 @@
 #include <cuda_bf16.h>
 
 #include <cstdio>
-#include <cstdlib>
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
@@ -107,7 +106,6 @@ struct PairParams {
   int n_steps;
   PairStep steps[kMaxChain];
 #ifdef KB200_TRACE
-  int debug;             // experiments of the trace build: 1 no bulk stores, 2 no staging, 4 no tensor-memory loads
 #endif
 };
 
@@ -519,12 +517,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         if (EPI != EPI_CHAIN) columns[e][lane] = mine;
         else if (col_step >= 0 && scratch_off >= 0) reinterpret_cast<float*>(slot0_ptr + scratch_off)[lane] = mine;
         float v[32];
-#ifdef KB200_TRACE
-        if (p.debug & 4) {
-#pragma unroll
-          for (int q = 0; q < 32; ++q) v[q] = 1.0f;
-        } else
-#endif
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * p.bn + c), v);
         __syncwarp();
 #ifdef KB200_TRACE
@@ -566,11 +558,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         stage_rows(slot0_ptr, slot0_ptr + (with32 || has_res ? 4096 : 0), v, lane, with16, with32);
         fence_async_smem();
         __syncwarp();
-#ifdef KB200_TRACE
-        if (lane == 0 && !dry && !(p.debug & 1)) {
-#else
         if (lane == 0 && !dry) {
-#endif
           if (with32) tma_store_3d(&tma_out, slot0, n, m_first, batch);
           if (with16) tma_store_3d(&tma_out16, slot0 + (with32 || has_res ? 4096u : 0u), n, m_first, batch);
           tma_store_commit();
@@ -598,7 +586,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
 #ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0 && !(p.debug & 64)) {
+  if (blockIdx.x <= 1 && threadIdx.x == 0) {
     const long long t0 = marks[0];
     printf("PAIR block %d: alloc+sync done %lld cluster barrier done %lld after pdl %lld exit %lld | tiles %d bn %d stages %d num_kb %d grid %d\n",
            (int)blockIdx.x, marks[1] - t0, marks[2] - t0, marks[3] - t0, clock64() - t0, p.num_tiles, p.bn, p.stages, p.num_kb, (int)gridDim.x);
@@ -809,9 +797,6 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   p.magic_tpb = ((uint64_t(1) << 40) + p.tiles_per_batch - 1) / p.tiles_per_batch;
   p.kernel_index = kernel_index;
   p.status = plan.d_status;
-#ifdef KB200_TRACE
-  p.debug = getenv("KB200_PAIR_DEBUG") ? atoi(getenv("KB200_PAIR_DEBUG")) : 0;
-#endif
   p.M = k.M;
   p.N = k.N;
   p.out16 = out16;

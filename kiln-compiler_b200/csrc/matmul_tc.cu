@@ -46,14 +46,6 @@ namespace {
 
 using namespace tc;
 
-// Experiments that change results exist in trace builds only; a shipped library ignores the bits.
-#ifdef KB200_TRACE
-#define KB200_EXPERIMENT(bit) (p.debug & (bit))
-#else
-#define KB200_EXPERIMENT(bit) false
-#endif
-
-
 constexpr int kTileM = 128;
 constexpr int kSlabBytes = 128;           // bytes of K (A) or N (B) per swizzled row
 constexpr int kATileBytes = kTileM * kSlabBytes;
@@ -92,7 +84,6 @@ struct TcParams {
   int b_static;         // B is a frozen constant: loaded without waiting for the previous kernel
   int b_kmajor;         // B is read K-major ([N, K] with K contiguous) like A
   int b_mode;           // how B is fetched: 0 K-major (one box), 1 N-major, all chunks in one 4-D box, 2 N-major, a box per chunk
-  int debug;            // trace builds only: 1 = no stores, 16 = no epilogue (results are then wrong), 32 = no warm-up pass
   int tmem_cols;        // power of two >= bn, >= 32
   int nacc;             // exact-FP32 mode: accumulators a tile's K steps rotate over (1 otherwise)
   int acc2;             // exact-FP32 mode: the accumulators of a tile fit twice (256 columns each): two buffers
@@ -222,7 +213,6 @@ __device__ __forceinline__ void epilogue_compute32(const TcParams& p, float (&x)
 
 __device__ __forceinline__ void epilogue_store32(const TcParams& p, const float (&x)[32], int64_t b, int64_t m_first, int64_t n,
                                                  int row_limit = 32) {
-  if (KB200_EXPERIMENT(1)) return;
   const MatmulParams& mm = p.mm;
   const DevOperand& o = mm.ops[mm.chain.out_slot];
   float* out = o.ptr + b * o.stride[0] + m_first * o.stride[1] + n * o.stride[2];
@@ -611,7 +601,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
       // Before its first tile is ready a CTA has nothing for these warps to do, and their code (the
       // unrolled chain, some kilobytes) is not in the instruction cache yet: one dry pass of the loop
       // body over zeros, with nothing stored, takes those misses off the critical path.
-      const bool dry_pass = i == 0 && direct && bulk && !KB200_EXPERIMENT(32) && !(SPLIT3 && p.presplit != 2);
+      const bool dry_pass = i == 0 && direct && bulk && !(SPLIT3 && p.presplit != 2);
       if (SPLIT3 && p.presplit != 2) {
         ok = split_steps(unsplit);
         if (!ok) break;
@@ -638,7 +628,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
 #endif
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        if (!dry && (n0 + c >= p.mm.N || KB200_EXPERIMENT(16))) break;   // uniform across the warp
+        if (!dry && n0 + c >= p.mm.N) break;   // uniform across the warp
         float v[32];
         if (dry) {
 #pragma unroll
@@ -716,7 +706,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
             else stage_columns(sf, sh, v, lane, p.out16 != nullptr);
             fence_async_smem();
             __syncwarp();
-            if (lane == 0 && m_first < p.mm.M && !KB200_EXPERIMENT(1) && !dry) {
+            if (lane == 0 && m_first < p.mm.M && !dry) {
               tma_store_3d(&tma_out, smem_u32(sf), (int)(n0 + c), (int)m_first, batch);
               if (p.out16 != nullptr) tma_store_3d(&tma_out16, smem_u32(sh), (int)(n0 + c), (int)m_first, batch);
               tma_store_commit();
@@ -843,7 +833,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] = chain_apply_scalar(st.op, v[j], side[j]);
         }
-        if (KB200_EXPERIMENT(1)) continue;
         float* dst = out_op.ptr + batch * out_op.stride[0] + m * out_op.stride[1] + n * out_op.stride[2];
         if (whole && out_op.stride[2] == 1 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
           *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
@@ -1331,7 +1320,6 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   p.b_kmajor = b_kmajor ? 1 : 0;
   p.b_static = st->b_copy.once ? 1 : 0;
   p.b_mode = b_kmajor ? 0 : (b_map_cols % chunk_n == 0 ? 1 : 2);
-  p.debug = d.cfg[6];
   p.issuers = issuers;
   p.split3 = split3 ? 1 : 0;
   p.presplit = a_pass ? 2 : presplit ? 1 : 0;
