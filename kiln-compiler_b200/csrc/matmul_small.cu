@@ -112,7 +112,7 @@ __device__ __forceinline__ void park_rows(uint8_t* slab, const float (&raw)[BF16
   }
 }
 
-// BN: columns of a tile, 64 or 128.  GATHER: warps 2-9 read A from global memory.  Of a Linear of 333 x 1000 x 771 the
+// BN: columns of a tile, 64, 96 or 128.  GATHER: warps 2-9 read A from global memory.  Of a Linear of 333 x 1000 x 771 the
 // pass that copied A to aligned rows, and the one that made bf16 of a float32 A, was a launch of ~2.3 us in front of this one.
 template <int MODE, int FIN, int BN, bool GATHER>
 __global__ void __launch_bounds__(kSmallThreads, 1)
@@ -122,7 +122,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr int kSmallBBytes = BN * 128;
   constexpr int kTileBytes = kSmallM * BN * 4;
   constexpr int kABuffers = 2;                                  // steps of A in tensor memory, 64 columns each
-  constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile; a warp has kBlocks / 2 of them
+  constexpr int kBlocks = BN / 32;                              // 32-column blocks of the tile, the first (or only) half of them to the first group of four warps
   constexpr int kSlabs = slabs_per_step(MODE);
   constexpr bool A32 = MODE == SMALL_BF16_A32, BF16 = MODE == SMALL_BF16 || A32;
   constexpr bool ALTERNATE = kSlabs == 1;                       // the two groups of warps that move A take alternate steps
@@ -271,7 +271,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // this thread's items of the band: float4 number t, t + 256, ... in row order, eight at a time
     constexpr int kUnits = BN / 4, kRowsAtOnce = 256 / kUnits;
     const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * BN;
-    const int u = t & (kUnits - 1), r0 = t / kUnits;
+    const int u = t % kUnits, r0 = t < kUnits * kRowsAtOnce ? t / kUnits : kSmallM;      // (96 columns: 16 threads have none)
     const int n = n0 + 4 * u;
     pdl_wait();
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -352,8 +352,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int i = 0; i < kBlocks / 2; ++i) {
-        const int cb = half * (kBlocks / 2) + i;
+      for (int cb = half * ((kBlocks + 1) / 2); cb < (half ? kBlocks : (kBlocks + 1) / 2); ++cb) {
         float v[32];
         const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb * 32);
         tmem_ld32(at, v);
@@ -494,9 +493,9 @@ SmallKernel small_kernel_of(int fin) {
 template <int MODE>
 SmallKernel small_kernel_of(int fin, int bn, bool gather) {
   if constexpr (MODE != SMALL_BF16_A32) {
-    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true>(fin) : small_kernel_of<MODE, 64, true>(fin);
+    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true>(fin) : bn == 96 ? small_kernel_of<MODE, 96, true>(fin) : small_kernel_of<MODE, 64, true>(fin);
   }
-  return bn == 128 ? small_kernel_of<MODE, 128, false>(fin) : small_kernel_of<MODE, 64, false>(fin);
+  return bn == 128 ? small_kernel_of<MODE, 128, false>(fin) : bn == 96 ? small_kernel_of<MODE, 96, false>(fin) : small_kernel_of<MODE, 64, false>(fin);
 }
 
 SmallKernel small_kernel(int mode, int fin, int bn, bool gather) {
@@ -569,15 +568,18 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 // Tile width, K split and estimated cycles, from fits to measured launches (128 to 1024 rows, 768 and 3072 of K, each
 // width and split).  A step, one 128-byte slab of K, is bound by shared memory: the operands land there
 // at 128 bytes a clock and every MMA reads its operands again (exact FP32: twelve of them, A from tensor
-// memory).  Everything that runs once, launch to exit, is the rest: wide tiles have more to
-// drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
+// memory).  Everything that runs once, launch to exit, is the rest: tiles of 96 columns and
+// more have two blocks to a warp to drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
+// 96 columns fit some row counts better than either neighbour (exact FP32: 1024 x 3072 x 768 36.4 -> 32.6 us,
+// 1024 x 768 x 3072 31.2 -> 27.8, 364 x 768 x 3072 22.3 -> 16.4).
 // GATHER: a warp loads, parks and reads back a slab of A one step ahead of its use, bound by the load/store unit (rows off the
 // lines: two of them to a load): what it adds to a step against the copied A (65 to 3000 of K).
-SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, bool gather, int sm_count) {
+SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, bool gather, bool chunked, int sm_count) {
   SmallPlan best{64, 1, 0};
   const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
-  for (int bn : {64, 128}) {
-    const int64_t step = mode == SMALL_EXACT ? (bn == 64 ? 690 : 945) : mode == SMALL_BF16_A32 ? (bn == 64 ? 500 : 550) : (bn == 64 ? 302 : 406);
+  for (int bn : {64, 96, 128}) {
+    if (bn == 96 && chunked) continue;                  // an N-major B comes in chunks of 64 bf16 columns
+    const int64_t step = mode == SMALL_EXACT ? 435 + 4 * bn : mode == SMALL_BF16_A32 ? 450 + bn * 25 / 32 : 198 + bn * 13 / 8;
     const int64_t once = (bn == 64 ? 7500 : 10050) + (mode == SMALL_EXACT ? 600 : 0);
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
     for (int s : {1, 2, 4, 8}) {
@@ -610,7 +612,7 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
   if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
   if (((k.M + kSmallM - 1) / kSmallM) * ((k.N + 63) / 64) > 4096) return -1;
   const int slab_k = bf16 ? 64 : 32;
-  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, small_mode(d.precision, form), form == SMALL_A_GATHERED, plan.sm_count).cycles;
+  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, plan.sm_count).cycles;
 }
 
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, void** state) {
@@ -625,7 +627,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.slab_k = slab_k;
   const int slabs = (int)((k.K + slab_k - 1) / slab_k), per_step = slabs_per_step(mode);
   p.num_steps = (slabs + per_step - 1) / per_step;
-  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, gather, plan.sm_count);
+  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, gather, ops.bf16 && !ops.b_kmajor, plan.sm_count);
   const int bn = how.bn;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);

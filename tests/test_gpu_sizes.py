@@ -77,7 +77,7 @@ def test_linear_of_any_size(m, n, k, precision):
 
 @pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
 @pytest.mark.parametrize("m,n,k", [(2, 64, 64), (128, 64, 4096), (127, 68, 1000), (128, 3072, 768), (100, 768, 3072), (17, 2304, 96), (128, 4096, 128),
-                                   (65, 1028, 3000)])
+                                   (65, 1028, 3000), (512, 768, 3072), (1024, 772, 3072), (364, 2308, 768), (1020, 3072, 768)])
 def test_few_tiles(m, n, k, precision):
     """One row of tiles: K split over 1 to 8 CTAs, K ranges longer and shorter than the ring, ragged last slabs."""
     check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
