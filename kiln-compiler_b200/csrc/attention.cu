@@ -1062,13 +1062,18 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   // its last tokens reads zeros behind them (as the stores' maps drop those rows): any length works.
   AttnState* st = new AttnState();
   st->exact = c.exact;
-  // FP32 mode: the tensor-core kernel when its work items (128 queries each) fill at least a quarter
-  // of the SMs, the CUDA-core kernel (64 queries per CTA, long prefixes split) for the short sequences
-  // below that (one 128-token sequence: 8.6 against 10.4 us; 512 tokens: 22.4 against 20.9);
-  // the plan option KB200_OPT_FP32_ATTENTION forces one of them.
+  // FP32 mode: the CUDA-core kernel (64 queries per CTA, long prefixes split) or the tensor-core kernel (128 queries
+  // and a pass over Q, K and V for their tails), whichever is estimated faster.  Both are a line through launches of 16 to
+  // 333 tokens and 4 to 96 heads, in ns: a fixed part, key tiles times rounds of the SMs, and that pass's bytes.
+  // (It was a quarter of the SMs' worth of work items: 48 heads of 64 tokens took 9.8 us on the tensor
+  // cores and 6.6 without, 4 heads of 200 tokens 13.0 and 11.3 on them.)  The plan option
+  // KB200_OPT_FP32_ATTENTION forces one of them.
   if (c.exact) {
     // (split operands turn an infinite element into a NaN tail: a plan that asked for IEEE behaviour keeps the FMA kernel)
-    st->exact_tc = !c.ieee && B * H * q_tiles * 4 >= plan.sm_count;
+    const int64_t sms = plan.sm_count, tiles64 = T <= 64 ? 1 : 2 * q_tiles;       // (three take as long as four)
+    const int64_t fma_ns = 4200 + 2250 * tiles64 * ((B * H * tiles64 + sms - 1) / sms);
+    const int64_t tc_ns = 6800 + 2400 * q_tiles * ((B * H * q_tiles + sms - 1) / sms) + B * T * 3 * H * hd * 8 / 6500;
+    st->exact_tc = !c.ieee && tc_ns <= fma_ns;
     if (plan.fp32_attention == 1) st->exact_tc = false;
     if (plan.fp32_attention == 2) st->exact_tc = true;
   }
