@@ -18,8 +18,8 @@ int choose_matmul(Plan& plan, PlanKernel& k) {
   k.launches = 1;
   const DevOperand& B = k.ops[d.b_slot];
   const int forced = d.cfg[5];   // 0 auto, 1 simt, 2 tc, 3 gemv
-  if ((forced == 0 || forced == 3) && k.M == 1 && B.stride[2] == 1 && B.stride[1] % 2 == 0 && B.stride[0] % 2 == 0 &&
-      (reinterpret_cast<uintptr_t>(B.ptr) & 7) == 0) {
+  if ((forced == 0 || forced == 3) && k.M == 1 && B.stride[2] == 1) {
+    // (single floats, a warp along a row of B: rows may begin anywhere; 1 x 2355 x 152 took 13.2 us in the SIMT tiles, 7.7 here)
     k.impl = IMPL_MM_GEMV;
     return KB200_OK;
   }

@@ -83,6 +83,11 @@ def test_few_tiles(m, n, k, precision):
     check({"kind": "linear", "m": m, "n": n, "k": k, "precision": precision}, ["mm_tcgen05"], calls=2)
 
 
+@pytest.mark.parametrize("n,k", [(2, 3), (33, 7), (2355, 152), (1001, 3071)])
+def test_one_row_of_any_size(n, k):
+    check({"kind": "linear", "m": 1, "n": n, "k": k}, ["mm_gemv"], calls=2)
+
+
 @pytest.mark.parametrize("precision", ["fp32", "tf32", "bf16"])
 @pytest.mark.parametrize("m,n,k", [(5, 64, 67), (2, 68, 65), (128, 4096, 129), (33, 768, 3071), (300, 128, 1023), (130, 64, 2050), (1000, 64, 4099)])
 def test_few_tiles_with_rows_on_no_pitch(m, n, k, precision):
