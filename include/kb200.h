@@ -216,7 +216,10 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores.
  * KB200_OPT_ATTENTION_SPLIT (default 1): in a launch that leaves SMs idle (one long sequence,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
- * merge their halves through a workspace.  0 keeps every query tile on one CTA. */
+ * merge their halves through a workspace.  0 keeps every query tile on one CTA.
+ * KB200_OPT_WEIGHT_COPIES (default 1, FP32 and TF32 precision): frozen weights are also kept laid out along K
+ * and, for FP32, with their tails, where memory is plenty (up to twice the weight's own bytes in FP32, once in
+ * TF32).  0 = every weight is read where it is, as it is when memory is short. */
 typedef enum kb200_option {
   KB200_OPT_FUSE_ATTENTION = 1,
   KB200_OPT_DEPENDENT_LAUNCH = 2,
@@ -225,7 +228,8 @@ typedef enum kb200_option {
   KB200_OPT_ABSORB_ELEMENTWISE = 5,
   KB200_OPT_MIRROR_ONLY = 6,
   KB200_OPT_FP32_ATTENTION = 7,
-  KB200_OPT_ATTENTION_SPLIT = 8
+  KB200_OPT_ATTENTION_SPLIT = 8,
+  KB200_OPT_WEIGHT_COPIES = 9
 } kb200_option;
 int kb200_plan_set_option(kb200_plan* plan, int option, int value);
 

@@ -617,6 +617,8 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
 
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, void** state) {
   *state = nullptr;
+  if (k.desc.precision == KB200_PREC_FP32 && b_tail == nullptr)
+    return fail(KB200_ERR_ARGUMENT, "matmul %s: the tails of B are missing", k.desc.name);
   SmallState* st = new SmallState();
   SmallParams& p = st->params;
   const kb200_kernel_desc& d = k.desc;

@@ -1154,7 +1154,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   size_t free_bytes = 0, total_bytes = 0;
   KB200_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
   const size_t copied = (size_t)k.N * k.K * sizeof(float) * (d.precision == KB200_PREC_FP32 ? 2 : 1);
-  const bool room = st->bf16 || copied <= free_bytes / 4;
+  const bool room = st->bf16 || (plan.weight_copies && copied <= free_bytes / 4);
   const bool turn = frozen && room && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
   const bool b_kmajor = turn || B.stride[2] != 1;
   const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = B.stride[2] != 1 ? B.stride[2] : B.stride[1];
@@ -1206,7 +1206,9 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
     if (many > 0 && copy_a) many += 4000;
   }
-  const bool small = few > 0 && (many == 0 || few < many);
+  // (its exact-FP32 form multiplies with the tails of B: without room for them the kernel above makes them as it goes)
+  const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
+  const bool small = few > 0 && tails_ready && (many == 0 || few < many);
   if (small && form != SMALL_A_MAPPED) {
     a_base = nullptr;
   } else if (copy_a) {

@@ -1134,6 +1134,7 @@ KB200_EXPORT int kb200_plan_set_option(kb200_plan* p, int option, int value) {
     case KB200_OPT_MIRROR_ONLY: plan.mirror_only = value != 0; return KB200_OK;
     case KB200_OPT_FP32_ATTENTION: plan.fp32_attention = value < 0 || value > 2 ? 0 : value; return KB200_OK;
     case KB200_OPT_ATTENTION_SPLIT: plan.attention_split = value != 0; return KB200_OK;
+    case KB200_OPT_WEIGHT_COPIES: plan.weight_copies = value != 0; return KB200_OK;
     default: return fail(KB200_ERR_ARGUMENT, "kb200_plan_set_option: unknown option %d", option);
   }
 }

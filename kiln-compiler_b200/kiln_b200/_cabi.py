@@ -35,6 +35,7 @@ OPT_ABSORB_ELEMENTWISE = 5
 OPT_MIRROR_ONLY = 6
 OPT_FP32_ATTENTION = 7
 OPT_ATTENTION_SPLIT = 8
+OPT_WEIGHT_COPIES = 9
 BASE_KINDS = {"arena": 0, "const": 1, "input": 2, "output": 3}
 PRECISIONS = {"fp32": 0, "tf32": 1, "bf16": 2}
 OPCODES = {

@@ -233,6 +233,10 @@ class GPUExecutable:
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_FP32_ATTENTION, fp32_attention), self._lib)
         split = os.environ.get("KILN_GPU_ATTENTION_SPLIT", "1") not in ("0", "false", "False", "")
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_ATTENTION_SPLIT, int(split)), self._lib)
+        # FP32 and TF32: weights also laid out along K (KILN_GPU_WEIGHT_COPIES=0: read where they are, for a GPU
+        # whose memory is needed for something else).
+        copies = os.environ.get("KILN_GPU_WEIGHT_COPIES", "1") not in ("0", "false", "False", "")
+        _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_WEIGHT_COPIES, int(copies)), self._lib)
         self._bind()
         # launch_names: one per device launch of the plan (k3_matmul, k2_ew0 ...); kernel_names: the Kiln
         # kernels they come from, which is what CompiledModule.profile keys on (kiln/api.py:204-211)
