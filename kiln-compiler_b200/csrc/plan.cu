@@ -1,5 +1,6 @@
 // The C ABI of libkb200.so: descriptor validation, buffer binding with bounds checks, launch
 // dispatch.  Declared and documented in include/kb200.h.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -967,6 +968,8 @@ static int repoint(Plan& plan, float* const* want) {
   bool moved = false;
   for (size_t b = 0; b < plan.io_now.size(); ++b) moved = moved || want[b] != plan.io_now[b];
   if (!moved) return KB200_OK;
+  // Nowhere until all of it has moved: after a failure half of the operands have, and the next call points every one again.
+  std::fill(plan.io_now.begin(), plan.io_now.end(), nullptr);
   for (size_t r = 0; r < plan.io_refs.size(); ++r) {
     const Plan::IoRef& ref = plan.io_refs[r];
     PlanKernel& k = plan.kernels[ref.kernel];

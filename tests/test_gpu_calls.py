@@ -46,3 +46,29 @@ def test_every_form_of_input_gives_the_same_results(case, precision):
         exe(dense[:, :-1])
     with pytest.raises(TypeError):
         exe(dense, dense)
+
+
+@pytest.mark.parametrize("case", ["linear_128x768x768", "linear_2048x3072x768"])
+def test_calls_from_a_thread_that_has_used_no_gpu(case):
+    """The first call of a thread may be one on buffers of its own; whatever becomes of it, the next call finds the plan whole."""
+    import threading
+
+    from gpu_helpers import build_executable
+
+    exe = build_executable(case, "tf32")
+    x = torch.randn(exe.input_shapes[0], device="cuda")
+    exe.static_inputs[0].copy_(x)
+    exe.run_static()
+    want = exe.static_outputs[0].clone()
+    torch.cuda.synchronize()
+    got = []
+    thread = threading.Thread(target=lambda: got.extend(exe(x)))
+    thread.start()
+    thread.join()
+    exe.static_outputs[0].zero_()
+    exe.run_static()
+    torch.cuda.synchronize()
+    exe.status()
+    assert torch.equal(exe.static_outputs[0], want)
+    for y in got:
+        assert torch.equal(y, want)
