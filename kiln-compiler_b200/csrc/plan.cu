@@ -964,10 +964,7 @@ static void collect_io_refs(Plan& plan) {
 
 // Points the plan at these buffers.  What moved is a handful of pointers and tensor-map addresses on the
 // host; launches already enqueued took theirs by value.
-static int repoint(Plan& plan, float* const* want) {
-  bool moved = false;
-  for (size_t b = 0; b < plan.io_now.size(); ++b) moved = moved || want[b] != plan.io_now[b];
-  if (!moved) return KB200_OK;
+static int point_at(Plan& plan, float* const* want) {
   // Nowhere until all of it has moved: after a failure half of the operands have, and the next call points every one again.
   std::fill(plan.io_now.begin(), plan.io_now.end(), nullptr);
   for (size_t r = 0; r < plan.io_refs.size(); ++r) {
@@ -980,6 +977,19 @@ static int repoint(Plan& plan, float* const* want) {
   }
   for (size_t b = 0; b < plan.io_now.size(); ++b) plan.io_now[b] = want[b];
   return KB200_OK;
+}
+
+static int repoint(Plan& plan, float* const* want) {
+  bool moved = false;
+  for (size_t b = 0; b < plan.io_now.size(); ++b) moved = moved || want[b] != plan.io_now[b];
+  if (!moved || point_at(plan, want) == KB200_OK) return KB200_OK;
+  // Tensor maps are the driver's, which needs a current context; a thread that has called nothing of the runtime has none.
+  int prev = 0;
+  KB200_CUDA(cudaGetDevice(&prev));
+  KB200_CUDA(cudaSetDevice(plan.device));
+  const int rc = point_at(plan, want);
+  if (prev != plan.device) KB200_CUDA(cudaSetDevice(prev));
+  return rc;
 }
 
 static int repoint_to_bound(Plan& plan) {
