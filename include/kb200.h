@@ -8,7 +8,9 @@
  * plain-old-data structs below; nothing in this interface is a torch type.
  *
  * Threading: a plan is not re-entrant (one arena), exactly like the
- * reference's GPUExecutable (kiln/gpu/runtime.py:135-136).  All functions
+ * reference's GPUExecutable (kiln/gpu/runtime.py:135-136).  Launches from several
+ * threads are enqueued whole, one after the other, each on its own buffers; on
+ * one stream a call then sees nothing of another's.  All functions
  * return 0 on success and a negative kb200_status otherwise; the text of the
  * last failure on the calling thread is returned by kb200_last_error().
  * Nothing here aborts or throws.  Device memory is allocated, and the device

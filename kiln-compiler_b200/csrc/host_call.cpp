@@ -18,6 +18,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -32,6 +33,13 @@ struct Caller {
   c10::Device device{c10::kCUDA, 0};
   std::vector<std::vector<int64_t>> in_shapes, out_shapes;
   std::vector<at::Tensor> fixed_inputs;      // where an input goes that the kernels cannot read as it is
+  std::mutex copies;                         // held from such a copy to the launches that read it
+};
+
+// The interpreter is left to other threads; taken again on the way out, by an exception too.
+struct WithoutInterpreter {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~WithoutInterpreter() { PyEval_RestoreThread(state); }
 };
 
 constexpr const char* kCapsule = "kb200.caller";
@@ -118,18 +126,14 @@ PyObject* run(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   }
   const c10::cuda::CUDAGuard guard(c->device);
   void* in[kMaxBuffers];
+  bool copied = false;
   for (size_t i = 0; i < n_in; ++i) {
     const at::Tensor& t = THPVariable_Unpack(args[1 + i]);
     // read where it is: float32, dense, on this device, 16-byte aligned (128-bit loads, tensor maps)
     const bool direct = t.layout() == c10::kStrided && t.scalar_type() == c10::kFloat && t.device() == c->device && t.is_contiguous() && !t.is_neg() &&
                         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
-    if (direct) {
-      in[i] = t.data_ptr();
-    } else {
-      const c10::NoGradGuard no_grad;
-      c->fixed_inputs[i].copy_(t.detach(), /*non_blocking=*/true);
-      in[i] = nullptr;
-    }
+    in[i] = direct ? t.data_ptr() : nullptr;
+    copied = copied || !direct;
   }
   void* out[kMaxBuffers];
   std::vector<at::Tensor> results;
@@ -140,9 +144,17 @@ PyObject* run(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   }
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(c->device.index()).stream();
   int status;
-  Py_BEGIN_ALLOW_THREADS
-  status = kb200_plan_run(c->plan, in, (int)n_in, out, (int)n_out, stream);
-  Py_END_ALLOW_THREADS
+  {
+    const WithoutInterpreter others_run;
+    std::unique_lock<std::mutex> one_copy(c->copies, std::defer_lock);
+    if (copied) {
+      one_copy.lock();
+      const c10::NoGradGuard no_grad;
+      for (size_t i = 0; i < n_in; ++i)
+        if (in[i] == nullptr) c->fixed_inputs[i].copy_(THPVariable_Unpack(args[1 + i]).detach(), /*non_blocking=*/true);
+    }
+    status = kb200_plan_run(c->plan, in, (int)n_in, out, (int)n_out, stream);
+  }
   if (status != KB200_OK) return raise(status);
   PyObject* list = PyList_New((Py_ssize_t)n_out);
   for (size_t i = 0; list && i < n_out; ++i) PyList_SET_ITEM(list, (Py_ssize_t)i, THPVariable_Wrap(std::move(results[i])));

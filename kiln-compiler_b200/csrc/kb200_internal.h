@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "kb200.h"
@@ -107,6 +108,9 @@ struct PlanKernel {
 };
 
 struct Plan {
+  // Held while the plan's pointers and tensor maps are moved and launched from: calls from several threads come one after the
+  // other, each with its own buffers.
+  std::mutex calls;
   int device = 0;
   int sm_count = 148;
   bool bound = false;

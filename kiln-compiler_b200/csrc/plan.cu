@@ -1076,6 +1076,7 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   if (n_consts < 0 || n_inputs < 0 || n_outputs < 0 || (n_consts && (!consts || !const_bytes)) ||
       (n_inputs && (!inputs || !input_bytes)) || (n_outputs && (!outputs || !output_bytes)))
     return fail(KB200_ERR_ARGUMENT, "kb200_plan_bind: bad buffer arrays");
+  const std::lock_guard<std::mutex> one_call(plan.calls);
   plan.bound = false;
   plan.arena = static_cast<float*>(arena);
   plan.arena_bytes = arena_bytes;
@@ -1155,6 +1156,7 @@ KB200_EXPORT int kb200_plan_set_option(kb200_plan* p, int option, int value) {
 KB200_EXPORT int kb200_plan_launch(kb200_plan* p, void* stream) {
   if (p == nullptr) return fail(KB200_ERR_ARGUMENT, "kb200_plan_launch: plan is null");
   Plan& plan = *reinterpret_cast<Plan*>(p);
+  const std::lock_guard<std::mutex> one_call(plan.calls);
   if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_plan_launch: call kb200_plan_bind first");
   const int rc = repoint_to_bound(plan);
   return rc ? rc : launch_all(plan, static_cast<cudaStream_t>(stream));
@@ -1170,6 +1172,7 @@ KB200_EXPORT int kb200_plan_run(kb200_plan* p, void* const* inputs, int n_inputs
                                 void* stream) {
   if (p == nullptr) return fail(KB200_ERR_ARGUMENT, "kb200_plan_run: plan is null");
   Plan& plan = *reinterpret_cast<Plan*>(p);
+  const std::lock_guard<std::mutex> one_call(plan.calls);
   if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_plan_run: call kb200_plan_bind first");
   if (!kb200_plan_relocatable(p)) return fail(KB200_ERR_UNSUPPORTED, "kb200_plan_run: this plan runs on its bound buffers only");
   if (n_inputs != (int)plan.inputs.size() || n_outputs != (int)plan.outputs.size() || (n_inputs && !inputs) || (n_outputs && !outputs))
@@ -1188,6 +1191,7 @@ KB200_EXPORT int kb200_plan_run(kb200_plan* p, void* const* inputs, int n_inputs
 KB200_EXPORT int kb200_kernel_launch(kb200_plan* p, int i, void* stream) {
   if (p == nullptr) return fail(KB200_ERR_ARGUMENT, "kb200_kernel_launch: plan is null");
   Plan& plan = *reinterpret_cast<Plan*>(p);
+  const std::lock_guard<std::mutex> one_call(plan.calls);
   if (!plan.bound) return fail(KB200_ERR_UNBOUND, "kb200_kernel_launch: call kb200_plan_bind first");
   if (i < 0 || i >= (int)plan.kernels.size()) return fail(KB200_ERR_ARGUMENT, "kb200_kernel_launch: no kernel %d", i);
   if (const int rc = repoint_to_bound(plan)) return rc;

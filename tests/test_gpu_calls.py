@@ -71,3 +71,30 @@ def test_calls_from_a_thread_that_has_used_no_gpu(case):
     exe.status()
     assert torch.equal(exe.static_outputs[0], want)
     assert len(got) == 1 and torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("case,precision", [("layernorm_2048x768", "fp32"), ("linear_128x768x768", "tf32"), ("linear_2048x3072x768", "bf16"),
+                                            ("mlp_2048", "bf16")])
+def test_calls_from_several_threads_keep_to_their_own_tensors(case, precision):
+    """On one stream the calls of a module run one after the other, whichever thread they come from."""
+    import threading
+
+    from gpu_helpers import build_executable
+
+    exe = build_executable(case, precision)
+    inputs = [torch.randn(exe.input_shapes[0], device="cuda") for _ in range(6)]
+    inputs[3:] = [x.t().contiguous().t() for x in inputs[3:]]      # (read through the fixed buffer)
+    want = [exe(x)[0] for x in inputs]
+    torch.cuda.synchronize()
+    right = []
+
+    def calls(x, y):
+        right.append(sum(torch.equal(exe(x)[0], y) for _ in range(50)))
+
+    threads = [threading.Thread(target=calls, args=pair) for pair in zip(inputs, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    exe.status()
+    assert right == [50] * 6
