@@ -129,11 +129,13 @@ PyObject* run(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   bool copied = false;
   for (size_t i = 0; i < n_in; ++i) {
     const at::Tensor& t = THPVariable_Unpack(args[1 + i]);
-    // read where it is: float32, dense, on this device, 16-byte aligned (128-bit loads, tensor maps)
+    // read where it is: float32, dense, on this device, 16-byte aligned (128-bit loads, tensor maps); a tensor without memory
+    // (zeros that autograd made, a wrapper) has its values copied
     const bool direct = t.layout() == c10::kStrided && t.scalar_type() == c10::kFloat && t.device() == c->device && t.is_contiguous() && !t.is_neg() &&
-                        (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
-    in[i] = direct ? t.data_ptr() : nullptr;
-    copied = copied || !direct;
+                        !t._is_zerotensor();
+    const void* at = direct ? t.const_data_ptr() : nullptr;
+    in[i] = (reinterpret_cast<uintptr_t>(at) & 15) == 0 ? const_cast<void*>(at) : nullptr;
+    copied = copied || in[i] == nullptr;
   }
   void* out[kMaxBuffers];
   std::vector<at::Tensor> results;

@@ -152,8 +152,8 @@ DIRECT_LAUNCHES = 9
 
 def _usable(t, device):
     """Can the kernels work on this tensor where it is?"""
-    return (t.device == device and t.dtype == torch.float32 and t.is_contiguous() and not t.is_neg() and t.numel() > 0
-            and t.data_ptr() % 16 == 0)
+    return (t.device == device and t.dtype == torch.float32 and t.is_contiguous() and not t.is_neg() and not t._is_zerotensor()
+            and t.numel() > 0 and t.data_ptr() != 0 and t.data_ptr() % 16 == 0)
 
 
 def _overlap(a, b):

@@ -98,3 +98,19 @@ def test_calls_from_several_threads_keep_to_their_own_tensors(case, precision):
         t.join()
     exe.status()
     assert right == [50] * 6
+
+
+def test_a_tensor_without_memory_is_read_as_its_values():
+    """Zeros that have no memory to point at are copied; what an earlier call left in the fixed buffer is not used."""
+    from gpu_helpers import build_executable
+
+    exe = build_executable("layernorm_2048x768", "fp32")
+    x = torch.randn(exe.input_shapes[0], device="cuda")
+    want = exe(torch.zeros_like(x))[0]
+    none = torch._efficientzerotensor(exe.input_shapes[0], device="cuda")
+    exe(x.cpu())
+    assert torch.equal(exe(none)[0], want)
+    exe(x.cpu())
+    sink = torch.empty_like(want)
+    exe.run_on([none], [sink])
+    assert torch.equal(sink, want)
