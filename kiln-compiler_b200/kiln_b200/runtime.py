@@ -319,15 +319,18 @@ class GPUExecutable:
     def run_on(self, inputs, outputs):
         """Enqueue the kernels on these tensors where they can be used as they are (float32, contiguous,
         16-byte aligned, on the device; an output overlapping no input) and through the static buffers
-        otherwise.  Capturable; the tensors' addresses are part of a captured graph."""
+        otherwise.  Capturable; the tensors' addresses are part of a captured graph.  A module with more inputs or
+        outputs than are given reads and writes its static buffers for the rest."""
         inputs = [t.detach() for t in inputs]
         direct = [self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) for t, shape in zip(inputs, self.input_shapes)]
         for static, t, d in zip(self.static_inputs, inputs, direct):
             if not d:
                 static.copy_(t, non_blocking=True)
         read = [t if d else static for static, t, d in zip(self.static_inputs, inputs, direct)]
+        read += self.static_inputs[len(read):]
         written = [t if self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) and not any(_overlap(t, r) for r in read)
                    else static for static, t, shape in zip(self.static_outputs, outputs, self.output_shapes)]
+        written += self.static_outputs[len(written):]
         if self.relocatable:
             ip, _, in_ = _ptr_array(read)
             op, _, on = _ptr_array(written)

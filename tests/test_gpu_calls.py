@@ -114,3 +114,30 @@ def test_a_tensor_without_memory_is_read_as_its_values():
     sink = torch.empty_like(want)
     exe.run_on([none], [sink])
     assert torch.equal(sink, want)
+
+
+def test_requests_bring_the_first_input_of_a_module_with_more():
+    """A step's sources are first inputs and its sinks first outputs; the others are the module's fixed buffers."""
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable, StreamedBatch
+    from kiln_b200.spec import KernelSpec, NodeSpec, OperandSpec, PlanSpec
+
+    shape = (40, 64)
+
+    def module():
+        at = lambda base, i: OperandSpec((base, i), 0, shape, (64, 1))     # noqa: E731
+        kernels = [KernelSpec(f"k{i}", "elementwise", [NodeSpec(op, [("operand", 0), ("operand", 1)], shape, {})], [at("input", 0), at("input", 1)],
+                              [(0, at("output", i))]) for i, op in enumerate(["add", "sub"])]
+        plan = PlanSpec("sum_and_difference", [shape, shape], [shape, shape], 0, {}, kernels)
+        return GPUExecutable(program_from_plan(plan, "fp32"), 0, {}, plan.input_shapes, plan.output_shapes, cuda_graphs=False)
+
+    modules = [module() for _ in range(2)]
+    sources = [torch.randn(shape, device="cuda") for _ in range(4)]
+    sinks = [torch.empty(shape, device="cuda") for _ in range(4)]
+    for i, m in enumerate(modules):
+        m.static_inputs[1].fill_(1.0 + i)
+    StreamedBatch(modules).capture(sources, sinks).run()
+    torch.cuda.synchronize()
+    for i, (x, y) in enumerate(zip(sources, sinks)):
+        assert torch.equal(y, x + (1.0 + i % 2))
+    assert torch.equal(modules[1].static_outputs[1], sources[3] - 2.0)
