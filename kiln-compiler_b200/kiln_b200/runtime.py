@@ -328,8 +328,9 @@ class GPUExecutable:
                 static.copy_(t, non_blocking=True)
         read = [t if d else static for static, t, d in zip(self.static_inputs, inputs, direct)]
         read += self.static_inputs[len(read):]
-        written = [t if self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) and not any(_overlap(t, r) for r in read)
-                   else static for static, t, shape in zip(self.static_outputs, outputs, self.output_shapes)]
+        # (a leaf that requires a gradient is left to copy_, which refuses it)
+        written = [t if self.relocatable and tuple(t.shape) == shape and _usable(t, self.device) and not t.requires_grad
+                   and not any(_overlap(t, r) for r in read) else static for static, t, shape in zip(self.static_outputs, outputs, self.output_shapes)]
         written += self.static_outputs[len(written):]
         if self.relocatable:
             ip, _, in_ = _ptr_array(read)
@@ -341,6 +342,8 @@ class GPUExecutable:
         for w, t in zip(written, outputs):
             if w is not t:
                 t.copy_(w, non_blocking=True)
+            else:
+                torch.autograd.graph.increment_version(t)      # the kernels wrote into it
 
     def __call__(self, *inputs):
         if self._caller is not None:

@@ -141,3 +141,18 @@ def test_requests_bring_the_first_input_of_a_module_with_more():
     for i, (x, y) in enumerate(zip(sources, sinks)):
         assert torch.equal(y, x + (1.0 + i % 2))
     assert torch.equal(modules[1].static_outputs[1], sources[3] - 2.0)
+
+
+def test_a_result_that_autograd_watches_is_refused():
+    """Writing into a leaf that requires a gradient is an error, and so is a backward pass over a tensor written since."""
+    from gpu_helpers import build_executable
+
+    exe = build_executable("layernorm_2048x768", "fp32", cuda_graphs=False)
+    x = torch.randn(exe.input_shapes[0], device="cuda")
+    with pytest.raises(RuntimeError, match="requires grad"):
+        exe.run_on([x], [torch.empty_like(x).requires_grad_()])
+    saved = torch.empty_like(x)
+    loss = (saved * torch.ones_like(x).requires_grad_()).sum()
+    exe.run_on([x], [saved])
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
