@@ -114,6 +114,7 @@ struct RowFastParams {
   float* out;
   const float* gamma;
   const float* beta;
+  int affine_static;       // both are frozen constants: no kernel writes them
   int64_t n_rows;
   int64_t x_row_stride, out_row_stride;
   int inner;
@@ -197,8 +198,8 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
     const float t = l < warps ? partial[32 * which + l] : (is_max ? -CUDART_INF_F : 0.0f);
     return is_max ? warp_max(t) : warp_sum(t);
   };
-  // The affine parameters of a LayerNorm are constants of the plan, not outputs of the previous
-  // kernel: they are fetched before this kernel waits for its producer, so their latency is off the
+  // The affine parameters of a LayerNorm are mostly constants of the plan, not outputs of the previous
+  // kernel: then they are fetched before this kernel waits for its producer, so their latency is off the
   // path (fetched after the two reductions they added a dependent memory round trip to every row).  Where other
   // rows on the SM cover that round trip their registers are worth more: in WIDE blocks, and with rows of
   // four or more float4 a lane in several waves, they are fetched where they are used (16384 x 768:
@@ -206,6 +207,7 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
   constexpr bool kAhead = MODE == ROW_LAYERNORM && AHEAD;
   float g[kAhead ? N : 1][VEC], b[kAhead ? N : 1][VEC];
   if (kAhead) {
+    if (!p.affine_static) pdl_wait();
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int j = lane + lanes * i;
@@ -534,6 +536,7 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     p.pre_out_stride1 = k.pre_out_slot >= 0 && two ? k.ops[k.pre_out_slot].stride[1] : 0;
     if (k.impl == IMPL_ROW_LAYERNORM) {
       p.gamma = k.ops[k.g_slot].ptr;
+      p.affine_static = d.operands[k.g_slot].base_kind == KB200_BASE_CONST && d.operands[k.b_slot].base_kind == KB200_BASE_CONST;
       p.beta = k.ops[k.b_slot].ptr;
       p.inv_n = k.ln_inv_n;
       p.eps = k.ln_eps;
