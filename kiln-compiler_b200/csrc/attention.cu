@@ -1036,7 +1036,8 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
         for (const Range& w : rewritten) fresh = fresh || covers(w, r);
         if (!fresh) return false;
       }
-      for (int slot : writes) rewritten.push_back(operand_range(plan.kernels[j], slot));
+      for (int slot : writes)
+        if (writes_whole_span(plan.kernels[j], slot)) rewritten.push_back(operand_range(plan.kernels[j], slot));
     }
   }
   // the fused kernel writes Y while other CTAs still read Q, K, V: if the planner reused their

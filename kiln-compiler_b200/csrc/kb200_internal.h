@@ -150,6 +150,8 @@ bool match_layernorm(const kb200_kernel_desc& d, PlanKernel* k);
 bool match_softmax(const kb200_kernel_desc& d, PlanKernel* k);
 constexpr int kMaxRowPre = 4;   // chain steps in front of a register-resident row kernel
 
+bool writes_whole_span(const PlanKernel& k, int slot);      // (plan.cu)
+
 // ---- per-class entry points ----
 int choose_elementwise(Plan& plan, PlanKernel& k);
 int launch_elementwise(const Plan& plan, const PlanKernel& k, cudaStream_t s);

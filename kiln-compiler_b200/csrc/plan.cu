@@ -446,6 +446,21 @@ void reads_and_writes(const PlanKernel& k, std::vector<int>* reads, std::vector<
 }
 bool spans_overlap(const Span& a, const Span& b) { return a.lo < b.hi && b.lo < a.hi; }
 }  // namespace
+// Does the kernel write every element of the operand's span?  (One with gaps leaves what was in them.)
+bool writes_whole_span(const PlanKernel& k, int slot) {
+  int64_t elems = 1;
+  for (int i = 0; i < k.desc.iter_rank; ++i)
+    if (k.ops[slot].stride[i] != 0) elems *= k.desc.iter_shape[i];      // (stride 0: reduced, or one value for all)
+  const Span s = span_of(k, slot);
+  return s.hi - s.lo == elems;
+}
+namespace {
+// Does it leave nothing of `old`?
+bool overwrites(const PlanKernel& k, int slot, const Span& old) {
+  const Span w = span_of(k, slot);
+  return w.lo <= old.lo && w.hi >= old.hi && writes_whole_span(k, slot);
+}
+}  // namespace
 
 // The buffer-assignment pass of the reference makes every matmul's B operand N-contiguous, with a
 // copy kernel where the value is not (kiln/passes/buffers.py:208-217): unfrozen weights, `x @ y.T`
@@ -539,7 +554,7 @@ static void fold_operand_copies(Plan& plan) {
         if (!(i == j && slot == bs) && spans_overlap(span_of(k, slot), b_span)) ok = false;
       for (int slot : writes) {
         const Span w = span_of(k, slot);
-        if (w.lo <= b_span.lo && w.hi >= b_span.hi) rewritten = true;
+        if (overwrites(k, slot, b_span)) rewritten = true;
         else if (spans_overlap(w, b_span) && i != j) ok = false;
       }
     }
@@ -667,7 +682,7 @@ static void absorb_elementwise(Plan& plan) {
       for (int slot : reads) ok = ok && !spans_overlap(span_of(k, slot), mo_span);
       for (int slot : writes) {
         const Span w = span_of(k, slot);
-        if (w.lo <= mo_span.lo && w.hi >= mo_span.hi) rewritten = true;
+        if (overwrites(k, slot, mo_span)) rewritten = true;
         else if (spans_overlap(w, mo_span)) ok = false;
       }
     }
@@ -762,7 +777,7 @@ static void absorb_elementwise(Plan& plan) {
       for (int slot : writes) {
         const Span x = span_of(k, slot);
         if (spans_overlap(x, mo_span)) ok = false;
-        if (x.lo <= eo_span.lo && x.hi >= eo_span.hi) dead = true;
+        if (overwrites(k, slot, eo_span)) dead = true;
         else if (spans_overlap(x, eo_span)) ok = false;
       }
     }
@@ -790,14 +805,17 @@ static int assign_shadows(Plan& plan) {
       if (pj.impl == IMPL_FUSED_AWAY) continue;
       const DevOperand* out = nullptr;
       int64_t out_elems = 0;
+      bool whole = true;
       if (pj.impl == IMPL_ATTN_FUSED) {
         out = attention_output(plan, j, &out_elems);
       } else if (pj.impl == IMPL_ROW_LAYERNORM && pj.desc.iter_rank == 2) {
         out = &pj.ops[pj.out_slot];
         out_elems = (pj.desc.iter_shape[0] - 1) * out->stride[0] + pj.desc.iter_shape[1];
+        whole = writes_whole_span(pj, pj.out_slot);
       } else if (pj.impl == IMPL_MM_TC && pj.has_chain) {
         out = &pj.ops[pj.chain.out_slot];
         out_elems = (pj.batch - 1) * out->stride[0] + (pj.M - 1) * out->stride[1] + (pj.N - 1) * out->stride[2] + 1;
+        whole = writes_whole_span(pj, pj.chain.out_slot);
       } else {
         // some other kernel: does it write into the operand at all?
         bool writes = false;
@@ -811,7 +829,7 @@ static int assign_shadows(Plan& plan) {
       }
       const Span w{out->ptr, out->ptr + out_elems};
       if (!(w.lo < x.hi && x.lo < w.hi)) continue;                 // does not touch the operand
-      if (w.lo <= x.lo && w.hi >= x.hi && w.lo >= arena_lo && w.hi <= arena_hi) return &pj;
+      if (whole && w.lo <= x.lo && w.hi >= x.hi && w.lo >= arena_lo && w.hi <= arena_hi) return &pj;
       return nullptr;
     }
     return nullptr;
@@ -917,7 +935,10 @@ static int assign_shadows(Plan& plan) {
         if (mirrored && w.lo <= x.lo && w.hi >= x.hi) ++readers;
         else only = false;
       }
-      for (int slot : writes) overwritten_by(span_of(r, slot));
+      for (int slot : writes) {
+        if (writes_whole_span(r, slot)) overwritten_by(span_of(r, slot));
+        else if (spans_overlap(span_of(r, slot), w)) only = false;
+      }
     }
     k.mirror_only = only && readers > 0;
   }
