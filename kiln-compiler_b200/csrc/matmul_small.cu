@@ -43,6 +43,7 @@ constexpr int kSmallMaxStages = 8;
 constexpr int kSmallABytes = kSmallM * 128;      // one 128-byte K slab
 constexpr int kSmallACols = 128;                 // tensor-memory columns for slabs of A
 constexpr int kSmallSmem = 225 * 1024;
+constexpr int kSmallMaxSlots = 5;                // exact FP32: accumulators of 64 columns beside that of the small products and the slabs of A
 
 // SMALL_BF16_A32: bf16 products of an A that is still float32, rounded on its way to tensor memory.  (A Linear of the caller's
 // own input; a launch that made a bf16 copy of it cost ~2.3 us in front of this one.)
@@ -52,7 +53,9 @@ enum : int { FIN_NONE = 0, FIN_BIAS, FIN_BIAS_GELU, FIN_BIAS_RES };
 struct SmallParams {
   int stages, num_steps, slab_k, splits;
   int b_kmajor, b_static;
-  int nacc;                        // exact FP32: accumulators the K steps rotate over, beside the one of the small products
+  // Exact FP32: accumulators of the large products (that of the small ones is behind them); log2 of the MMAs of a step that go
+  // into one, and, where that is all of them (2), the steps.
+  int acc_slots, acc_shift, acc_steps;
   uint32_t b_lbo, b_sbo, b_layout, b_step16;
   uint32_t idesc;
   int tmem_cols;
@@ -63,13 +66,16 @@ struct SmallParams {
   const float* bias;
   const float* res;
   int64_t res_row;
-  const float* a;                  // GATHER: A as it is in memory, rows of K elements a_row apart
+  const float* a;                  // GATHER and exact FP32: A as it is in memory, rows of K elements a_row apart
   int64_t a_row;
+  const float* b;                  // exact FP32: B as it is in memory, and its strides along K and N
+  int64_t b_k, b_n;
   int K;
   int a_rows;                      // rows of a box of A: the tile's, or M where that is less
   float* out;                      // null: only the bf16 copy is stored
   __nv_bfloat16* out16;            // or null
   int64_t out_row;                 // of both
+  int vectors;                     // exact FP32: 0 where N or a row's start is off float4: bias, residual and output element by element
 };
 
 // 128-byte slabs of K per pipeline step.  A step costs the issuing warp ~400 cycles of wait, branches and commits
@@ -112,9 +118,32 @@ __device__ __forceinline__ void park_rows(uint8_t* slab, const float (&raw)[BF16
   }
 }
 
+// Exact FP32: an infinite operand makes a NaN of its tail's products (inf x 0, inf - inf) where float32 has an infinity.  Results
+// that are NaN, of rows m, m + rows_apart, ... below m_end and columns n to n + 3, done over as the CUDA cores do them.
+template <int FIN>
+__device__ __noinline__ void redo_in_float32(const SmallParams& p, int m, int m_end, int rows_apart, int n) {
+  for (; m < m_end; m += rows_apart) {
+    for (int c = n; c < n + 4 && c < p.N; ++c) {
+      float* const out = p.out + (int64_t)m * p.out_row + c;
+      if (*out == *out) continue;
+      const float* const a = p.a + m * p.a_row;
+      const float* const b = p.b + c * p.b_n;
+      float y = 0.0f;
+#pragma unroll 8
+      for (int k = 0; k < p.K; ++k) y = fmaf(a[k], b[k * p.b_k], y);
+      if (FIN != FIN_NONE) y += p.bias[c];
+      if (FIN == FIN_BIAS_GELU) y = d_gelu_tanh(y);
+      if (FIN == FIN_BIAS_RES) y += p.res[(int64_t)m * p.res_row + c];
+      *out = y;
+    }
+  }
+}
+
 // BN: columns of a tile, 64, 96 or 128.  GATHER: warps 2-9 read A from global memory.  Of a Linear of 333 x 1000 x 771 the
 // pass that copied A to aligned rows, and the one that made bf16 of a float32 A, was a launch of ~2.3 us in front of this one.
-template <int MODE, int FIN, int BN, bool GATHER>
+// DRAINS: exact FP32, more steps than the accumulators take.  (The adding up in the loop, and its registers, cost 3 % where it does
+// nothing: 1024 x 768 x 3072 29.0 us, 27.9 without.)
+template <int MODE, int FIN, int BN, bool GATHER, bool DRAINS>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                 const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
@@ -128,7 +157,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr bool ALTERNATE = kSlabs == 1;                       // the two groups of warps that move A take alternate steps
   constexpr int kSlabA = a_slab_bytes(MODE), kBBoxes = b_boxes(MODE), kStage = stage_bytes_of(MODE, BN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 6];
+  __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 4 + kSmallMaxSlots];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const uint32_t raw_at = smem_u32(smem_raw);
@@ -140,7 +169,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const uint32_t parts0 = ring + (uint32_t)(p.stages * kStage) + (in_ring ? 0u : (uint32_t)kTileBytes);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kSmallMaxStages]), split0 = smem_u32(&bars[2 * kSmallMaxStages]);
-  const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8, tfree0 = done + 16;
+  const uint32_t done = smem_u32(&bars[3 * kSmallMaxStages]), received = done + 8, tfree0 = done + 16, drained0 = done + 32;
   const int tile = blockIdx.x / p.splits;
   const int rank = blockIdx.x - tile * p.splits;                // in the cluster: its CTAs are consecutive
   const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
@@ -156,6 +185,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     mbar_init(done, 1);
     mbar_init(received, 1);
     for (int i = 0; i < kABuffers; ++i) mbar_init(tfree0 + 8 * i, 1);
+    for (int i = 0; DRAINS && i < p.acc_slots; ++i) mbar_init(drained0 + 8 * i, kSmallEpiWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(received, (uint32_t)(kTileBytes / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
@@ -181,7 +211,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const bool clustered = p.splits > 1;
   if (clustered) cluster_arrive();
   const uint32_t tmem = tmem_slot;
-  [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((1 + p.nacc) * BN);      // the slabs of A
+  [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((EXACT ? p.acc_slots + 1 : 1) * BN);      // the slabs of A
   volatile int* abort_ptr = &abort_flag;
   auto give_up = [&](int site) {
     if (!*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
@@ -226,10 +256,16 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // ---------------- MMA issuer ----------------
     const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
     const uint32_t b_step = p.b_step16, idesc = p.idesc;
-    int s = 0, rot = 0, buf = 0;
+    int s = 0, buf = 0;
+    [[maybe_unused]] int slot = 0, in_slot = 0;
+    [[maybe_unused]] uint32_t acc_at = tmem;       // the slot's columns
+    [[maybe_unused]] bool again = false;           // the slots are being used again ...
+    [[maybe_unused]] uint32_t refill = 1;          // ... and are free with this phase of `drained`
     uint32_t parity = 0;
     bool ok = true;
     for (int i = 0; i < n_steps && ok; ++i) {
+      if (DRAINS && again && in_slot == 0) ok = all_waited(mbar_wait(drained0 + 8 * slot, refill, abort_ptr), 8);
+      if (!ok) break;
       ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // this step's A is in tensor memory (and so its B has landed)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -237,17 +273,30 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       const uint32_t on = elect_one() ? 1u : 0u;
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
       auto desc = [&](uint32_t at) { return b_fixed | (uint64_t)(at & 0x3FFFu); };
+      if constexpr (EXACT) {
+        // a b ~ tail(a) b + a tail(b) + a b.  The tensor core truncates every accumulation, an error of ~2^-24 of what the
+        // accumulator holds each time (positive operands, 3072 of K over eight CTAs, one accumulator: 2.7e-6).  So
+        // no accumulator takes more than the host allows (see accumulate_as), and the warps below add them up in
+        // float32.  The small products, whose error is 2^-11 of that, have one of their own.
+        const uint32_t apart = tmem + (uint32_t)(p.acc_slots * BN);
+        const uint32_t more = in_slot != 0 ? 1u : 0u;
 #pragma unroll
-      for (int k = 0; k < 4 * kSlabs; ++k) {
-        const uint32_t b = b16 + (k >> 2) * (kSmallBBytes >> 4) + (k & 3) * b_step, ta = tmem_a + (uint32_t)(buf * 64 + 8 * k);
-        if (EXACT) {
-          // a b ~ tail(a) b + a tail(b) + a b.  The small products have an accumulator of their own and the large
-          // ones rotate over nacc: the tensor core truncates every accumulation, an error that grows
-          // with the number of them (see matmul_tc.cu)
-          umma_ts_if(on, tmem, ta + 32, desc(b), idesc, (i | k) != 0, false);
-          umma_ts_if(on, tmem, ta, desc(b + (kSmallBBytes >> 4)), idesc, 1u, false);
-          umma_ts_if(on, tmem + (uint32_t)((1 + rot) * BN), ta, desc(b), idesc, i >= p.nacc || k != 0, false);
-        } else {
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t b = b16 + k * b_step, ta = tmem_a + (uint32_t)(buf * 64 + 8 * k);
+          umma_ts_if(on, apart, ta + 32, desc(b), idesc, (i | k) != 0, false);
+          umma_ts_if(on, apart, ta, desc(b + (kSmallBBytes >> 4)), idesc, 1u, false);
+          umma_ts_if(on, acc_at, ta, desc(b), idesc, k == 0 ? more : p.acc_shift == 2 || (p.acc_shift == 1 && (k & 1)) ? 1u : 0u, false);
+          if (p.acc_shift == 0 || (p.acc_shift == 1 && (k & 1))) acc_at += BN;
+        }
+        if (p.acc_shift == 2 && ++in_slot == p.acc_steps) {
+          in_slot = 0;
+          acc_at += BN;
+          if (DRAINS && ++slot == p.acc_slots) { slot = 0; acc_at = tmem; again = true; refill ^= 1; }
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4 * kSlabs; ++k) {
+          const uint32_t b = b16 + (k >> 2) * (kSmallBBytes >> 4) + (k & 3) * b_step, ta = tmem_a + (uint32_t)(buf * 64 + 8 * k);
           umma_ts_if(on, tmem, ta, desc(b), idesc, (i | k) != 0, BF16);
         }
       }
@@ -257,7 +306,6 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         if (i + 1 == n_steps) umma_commit(done);
       }
       __syncwarp();
-      if (EXACT && ++rot == p.nacc) rot = 0;
       buf ^= 1;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
@@ -267,7 +315,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     const int band_rows = kSmallM / p.splits;
     // The parameters are read through the constant cache, cold at every launch: touch what the end of the
     // kernel needs now, under the wait.
-    asm volatile("" ::"l"(p.bias), "l"(p.res), "l"(p.res_row), "l"(p.out), "l"(p.out16), "l"(p.out_row), "r"(p.M), "r"(p.N), "r"(p.nacc) : "memory");
+    asm volatile("" ::"l"(p.bias), "l"(p.res), "l"(p.res_row), "l"(p.out), "l"(p.out16), "l"(p.out_row), "r"(p.M), "r"(p.N), "r"(p.acc_slots), "r"(p.acc_steps) : "memory");
     // this thread's items of the band: float4 number t, t + 256, ... in row order, eight at a time
     constexpr int kUnits = BN / 4, kRowsAtOnce = 256 / kUnits;
     const int band0 = rank * band_rows, m0 = tm * kSmallM, n0 = tn * BN;
@@ -275,15 +323,49 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     const int n = n0 + 4 * u;
     pdl_wait();
     float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (FIN != FIN_NONE && n < p.N) bias = __ldg(reinterpret_cast<const float4*>(p.bias + n));
+    auto load4 = [&](const float* from) {
+      if (!EXACT || p.vectors) return *reinterpret_cast<const float4*>(from);
+      return make_float4(from[0], n + 1 < p.N ? from[1] : 0.f, n + 2 < p.N ? from[2] : 0.f, n + 3 < p.N ? from[3] : 0.f);
+    };
+    if (FIN != FIN_NONE && n < p.N) bias = load4(p.bias + n);
     auto load_res = [&](int r) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
       const int m = m0 + band0 + r;
-      if (FIN == FIN_BIAS_RES && r < band_rows && m < p.M && n < p.N) x = *reinterpret_cast<const float4*>(p.res + (int64_t)m * p.res_row + n);
+      if (FIN == FIN_BIAS_RES && r < band_rows && m < p.M && n < p.N) x = load4(p.res + (int64_t)m * p.res_row + n);
       return x;
     };
     float4 res = load_res(r0);
     bool ok = true;
+    // Exact FP32: this warp's rows of its half of the tile's columns, added up from the accumulators
+    constexpr int kHalfBlocks = (kBlocks + 1) / 2;
+    [[maybe_unused]] float sum[EXACT ? kHalfBlocks : 1][32];
+    [[maybe_unused]] int drained = 0, drain_slot = 0;             // accumulators added so far, and the next one's slot
+    [[maybe_unused]] auto add_slot = [&](int slot) {
+#pragma unroll
+      for (int c = 0; c < (EXACT ? kHalfBlocks : 0); ++c) {
+        if (half * kHalfBlocks + c >= kBlocks) continue;
+        float w[32];
+        tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(slot * BN + (half * kHalfBlocks + c) * 32), w);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[c][j] += w[j];
+      }
+    };
+    [[maybe_unused]] auto drain = [&](bool free_it) {
+      add_slot(drain_slot);
+      if (free_it) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(drained0 + 8 * drain_slot);
+      }
+      ++drained;
+      if (++drain_slot == p.acc_slots) drain_slot = 0;
+    };
+    if constexpr (EXACT) {
+#pragma unroll
+      for (int c = 0; c < kHalfBlocks; ++c)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[c][j] = 0.0f;
+    }
     {
       // A goes to tensor memory, 32 columns a slab (exact FP32: values and tails, what their 19 leading bits leave).
       // The tensor core reads an operand from shared memory at ~64 bytes a clock: with A there an MMA of 128
@@ -315,6 +397,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           if (i + kEvery < n_steps) fetch(i + kEvery);
         }
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
+        // (loading and splitting A in front of this wait takes no less time: the issuing warp, in whose scheduler two of these
+        // warps are, is held up by them then)
         if (i >= kABuffers && !mbar_wait(tfree0 + 8 * buf, ((i / kABuffers) & 1) ^ 1, abort_ptr)) give_up(6);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
@@ -332,15 +416,19 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         }
         const uint32_t at = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 64 + (ALTERNATE ? 0 : half * 32));
         tmem_st32(at, v);
-        if (EXACT) {
+        if constexpr (EXACT) {
 #pragma unroll
-          for (int q = 0; q < 32; ++q) v[q] -= __uint_as_float(__float_as_uint(v[q]) & 0xFFFFE000u);
+          for (int q = 0; q < 32; ++q) v[q] = cut_tail(v[q]);
           tmem_st32(at + 32, v);
         }
         tmem_st_wait();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(split0 + 8 * s);
+        // Accumulators that the ring of slots needs again: those whose steps end at i - 2, whose MMAs the wait for this
+        // step's buffer of A has seen complete.
+        if (DRAINS && n_steps > p.acc_slots * p.acc_steps)
+          while ((drained + 1) * p.acc_steps + 1 <= i) drain(true);
         s += kEvery;
         if (s >= p.stages) { s -= p.stages; parity ^= 1; }
       }
@@ -351,20 +439,21 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (clustered) cluster_wait();              // every CTA's `received` exists
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if constexpr (EXACT) {
 #pragma unroll 1
-      for (int cb = half * ((kBlocks + 1) / 2); cb < (half ? kBlocks : (kBlocks + 1) / 2); ++cb) {
+        for (const int all = (n_steps << (2 - p.acc_shift)) + p.acc_steps - 1; (drained + 1) * p.acc_steps <= all;) drain(false);
+        add_slot(p.acc_slots);
+      }
+#pragma unroll(EXACT ? kHalfBlocks : 1)
+      for (int c = 0; c < kHalfBlocks; ++c) {
+        const int cb = half * kHalfBlocks + c;
+        if (cb >= kBlocks) break;
         float v[32];
-        const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb * 32);
-        tmem_ld32(at, v);
-        if (EXACT) {
-          const int used = min(p.nacc, n_steps);
-#pragma unroll 1
-          for (int a = 1; a <= used; ++a) {
-            float w[32];
-            tmem_ld32(at + (uint32_t)(a * BN), w);
+        if constexpr (EXACT) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += w[j];
-          }
+          for (int j = 0; j < 32; ++j) v[j] = sum[c][j];
+        } else {
+          tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb * 32), v);
         }
         // This 32 x 32 block goes to the CTA that finishes its rows (two CTAs, 16 rows each, with eight
         // splits): staged in 128-byte rows, the 16-byte unit XORed with the row, then one bulk copy per
@@ -409,6 +498,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       const uint8_t* const area = smem_raw + (parts0 - raw_at);
       const uint8_t* const own = smem_raw + (recv - raw_at);
       const int cb = u >> 3;
+      [[maybe_unused]] bool any_nan = false;
 #pragma unroll 1
       for (int r = r0; r < band_rows; r += kRowsAtOnce) {
         const float4 res_next = load_res(r + kRowsAtOnce);
@@ -423,6 +513,10 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           if (!mine) part += kBlocks * band_rows * 128;
           y.x += b.x; y.y += b.y; y.z += b.z; y.w += b.w;
         }
+        if (EXACT) {
+          const float all = (y.x + y.y) + (y.z + y.w);
+          any_nan = any_nan || all != all;
+        }
         if (FIN != FIN_NONE) { y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w; }
         if (FIN == FIN_BIAS_GELU) {
           if (BF16) {
@@ -434,6 +528,14 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         if (FIN == FIN_BIAS_RES) { y.x += res.x; y.y += res.y; y.z += res.z; y.w += res.w; }
         res = res_next;
         if (m >= p.M || n >= p.N) continue;
+        if (EXACT && !p.vectors) {
+          float* const to = p.out + (int64_t)m * p.out_row + n;
+          to[0] = y.x;
+          if (n + 1 < p.N) to[1] = y.y;
+          if (n + 2 < p.N) to[2] = y.z;
+          if (n + 3 < p.N) to[3] = y.w;
+          continue;
+        }
         if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
         if (p.out16 != nullptr) {
           __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
@@ -443,6 +545,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
         }
       }
+      if (EXACT && any_nan) redo_in_float32<FIN>(p, m0 + band0 + r0, min(p.M, m0 + band0 + band_rows), kRowsAtOnce, n);
     }
   }
   // (the warp has to be whole for an .aligned barrier)
@@ -476,34 +579,35 @@ struct SmallState {
   unsigned grid = 0;
   size_t smem = 0;
   int bias_slot = -1, res_slot = -1;
-  bool gather = false;                        // warps 2-9 read A
   bool a_moves = false, b_moves = false;      // the maps hold the operand's own address
 };
 
-template <int MODE, int BN, bool GATHER>
+template <int MODE, int BN, bool GATHER, bool DRAINS>
 SmallKernel small_kernel_of(int fin) {
   switch (fin) {
-    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN, GATHER>;
-    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN, GATHER>;
-    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN, GATHER>;
-    default: return mm_small_kernel<MODE, FIN_NONE, BN, GATHER>;
+    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN, GATHER, DRAINS>;
+    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN, GATHER, DRAINS>;
+    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN, GATHER, DRAINS>;
+    default: return mm_small_kernel<MODE, FIN_NONE, BN, GATHER, DRAINS>;
   }
 }
 
-template <int MODE>
+template <int MODE, bool DRAINS>
 SmallKernel small_kernel_of(int fin, int bn, bool gather) {
-  if constexpr (MODE != SMALL_BF16_A32) {
-    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true>(fin) : bn == 96 ? small_kernel_of<MODE, 96, true>(fin) : small_kernel_of<MODE, 64, true>(fin);
+  if constexpr (MODE == SMALL_EXACT) {
+    if (gather) return small_kernel_of<MODE, 64, true, DRAINS>(fin);
+  } else if constexpr (MODE != SMALL_BF16_A32) {
+    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true, DRAINS>(fin) : bn == 96 ? small_kernel_of<MODE, 96, true, DRAINS>(fin) : small_kernel_of<MODE, 64, true, DRAINS>(fin);
   }
-  return bn == 128 ? small_kernel_of<MODE, 128, false>(fin) : bn == 96 ? small_kernel_of<MODE, 96, false>(fin) : small_kernel_of<MODE, 64, false>(fin);
+  return bn == 128 ? small_kernel_of<MODE, 128, false, DRAINS>(fin) : bn == 96 ? small_kernel_of<MODE, 96, false, DRAINS>(fin) : small_kernel_of<MODE, 64, false, DRAINS>(fin);
 }
 
-SmallKernel small_kernel(int mode, int fin, int bn, bool gather) {
+SmallKernel small_kernel(int mode, int fin, int bn, bool gather, bool drains) {
   switch (mode) {
-    case SMALL_BF16: return small_kernel_of<SMALL_BF16>(fin, bn, gather);
-    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32>(fin, bn, gather);
-    case SMALL_EXACT: return small_kernel_of<SMALL_EXACT>(fin, bn, gather);
-    default: return small_kernel_of<SMALL_TF32>(fin, bn, gather);
+    case SMALL_BF16: return small_kernel_of<SMALL_BF16, false>(fin, bn, gather);
+    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32, false>(fin, bn, gather);
+    case SMALL_EXACT: return drains ? small_kernel_of<SMALL_EXACT, true>(fin, bn, gather) : small_kernel_of<SMALL_EXACT, false>(fin, bn, gather);
+    default: return small_kernel_of<SMALL_TF32, false>(fin, bn, gather);
   }
 }
 
@@ -512,22 +616,27 @@ int small_mode(int precision, SmallA form) {
   return precision != KB200_PREC_BF16 ? SMALL_TF32 : form == SMALL_A_FLOAT32 ? SMALL_BF16_A32 : SMALL_BF16;
 }
 
-// The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.
-int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot) {
+// The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.  `vectors`: whether all that it
+// reads and writes there is in float4.
+int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot, bool* vectors) {
   const Chain& c = k.chain;
+  const DevOperand& o = k.ops[c.out_slot];
+  *vectors = k.N % 4 == 0 && o.stride[1] % 4 == 0 && aligned16(o.ptr);
   *bias_slot = *res_slot = -1;
   if (c.n == 0) return FIN_NONE;
   const ChainStep* s = c.steps;
   if (s[0].op != CH_ADD || s[0].slot < 0) return -1;
   const DevOperand& b = k.ops[s[0].slot];
-  if (b.stride[1] != 0 || b.stride[2] != 1 || !aligned16(b.ptr)) return -1;
+  if (b.stride[1] != 0 || b.stride[2] != 1) return -1;
+  *vectors = *vectors && aligned16(b.ptr);
   *bias_slot = s[0].slot;
   if (c.n == 1) return FIN_BIAS;
   if (c.n != 2) return -1;
   if (s[1].op == CH_GELU_TANH) return FIN_BIAS_GELU;
   if (s[1].op != CH_ADD || s[1].slot < 0) return -1;
   const DevOperand& r = k.ops[s[1].slot];
-  if (r.stride[2] != 1 || r.stride[1] < k.N || r.stride[1] % 4 || !aligned16(r.ptr)) return -1;
+  if (r.stride[2] != 1 || r.stride[1] < k.N) return -1;
+  *vectors = *vectors && r.stride[1] % 4 == 0 && aligned16(r.ptr);
   *res_slot = s[1].slot;
   return FIN_BIAS_RES;
 }
@@ -549,7 +658,7 @@ int resident_clusters(int splits, int sm_count) {
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS, 64, false>;
+    const SmallKernel kernel = mm_small_kernel<SMALL_TF32, FIN_BIAS, 64, false, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
@@ -560,8 +669,44 @@ int resident_clusters(int splits, int sm_count) {
   return known[splits];
 }
 
-// Exact FP32: accumulators for the large products, beside that of the small ones and the slabs of A.
-constexpr int exact_accumulators(int bn) { return (512 - kSmallACols) / bn - 1; }
+// Exact FP32: accumulators beside that of the small products and the slabs of A.
+constexpr int exact_slots(int bn) { return (512 - kSmallACols) / bn - 1; }
+static_assert(exact_slots(64) == kSmallMaxSlots, "barriers of the slots");
+
+// How exact FP32 accumulates `most` steps of a CTA: at most `limit` MMAs along K into one accumulator.  Where the
+// accumulators do not last for all steps, the warps that move A add them up as they go (`drains`).
+struct Accumulate { int slots, shift, steps; bool drains; };
+
+Accumulate accumulate_as(int most, int bn, int limit) {
+  const int all = exact_slots(bn);
+  Accumulate a{all, 2, 1, false};
+  // few steps: an accumulator for every one, two or four MMAs
+  a.shift = limit >= 4 ? 2 : limit >= 2 ? 1 : 0;
+  while (a.shift > 0 && (most << (3 - a.shift)) <= all) --a.shift;
+  if (most << (2 - a.shift) <= all) {
+    a.slots = most << (2 - a.shift);
+    return a;
+  }
+  a.shift = 2;
+  const int steps = limit / 4 > 1 ? limit / 4 : 1;
+  a.steps = (most + all - 1) / all;
+  a.drains = a.steps > steps;
+  if (a.drains) a.steps = steps;
+  else a.slots = (most + a.steps - 1) / a.steps;
+  return a;
+}
+
+// MMAs along K that may go into one accumulator: each adds 3.3e-8 to an error of ~5e-8 (positive operands).  Float32 sums
+// over K on the CUDA cores, which take the operands that this kernel and no other may have (`close`), err by 1.5e-8 sqrt(K)
+// (64: 1.3e-7; 768: 4.2e-7; 3072: 8.5e-7), matmul_tc.cu with K split over a cluster, up to 16 of its
+// tiles, by 5.0e-7 to 6.2e-7 and else by 1.1e-6 and more.
+int accumulate_limit(int64_t m, int64_t n, int64_t k, bool close) {
+  const bool many = m > kSmallM && ((m + 127) / 128) * ((n + 127) / 128) > 16;
+  if (many && !close) return 64;
+  for (int limit : {12, 8, 4, 2})
+    if ((limit + 1.5) * (limit + 1.5) <= 0.2 * (double)k) return limit;
+  return 1;
+}
 
 struct SmallPlan { int bn, splits; int64_t cycles; };
 
@@ -574,19 +719,23 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 // 1024 x 768 x 3072 31.2 -> 27.8, 364 x 768 x 3072 22.3 -> 16.4).
 // GATHER: a warp loads, parks and reads back a slab of A one step ahead of its use, bound by the load/store unit (rows off the
 // lines: two of them to a load): what it adds to a step against the copied A (65 to 3000 of K).
-SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, bool gather, bool chunked, int sm_count) {
+SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, bool chunked, bool close, int sm_count) {
+  const int64_t slab_k = mode == SMALL_BF16 || mode == SMALL_BF16_A32 ? 64 : 32, slabs = (k + slab_k - 1) / slab_k;
   SmallPlan best{64, 1, 0};
   const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
   for (int bn : {64, 96, 128}) {
     if (bn == 96 && chunked) continue;                  // an N-major B comes in chunks of 64 bf16 columns
+    if (bn > 64 && gather && mode == SMALL_EXACT) continue;      // rows of A and 64 sums do not fit the registers together
     const int64_t step = mode == SMALL_EXACT ? 435 + 4 * bn : mode == SMALL_BF16_A32 ? 450 + bn * 25 / 32 : 198 + bn * 13 / 8;
     const int64_t once = (bn == 64 ? 7500 : 10050) + (mode == SMALL_EXACT ? 600 : 0);
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
     for (int s : {1, 2, 4, 8}) {
       const int64_t steps = (slabs + slabs_per_step(mode) - 1) / slabs_per_step(mode);
       if (s > steps) break;
-      // (exact FP32: at most 1024 of K in one accumulator)
-      if (mode == SMALL_EXACT && (slabs + s - 1) / s > 32 * exact_accumulators(bn)) continue;
+      if (mode == SMALL_EXACT) {
+        const Accumulate a = accumulate_as((int)((steps + s - 1) / s), bn, accumulate_limit(m, n, k, close));
+        if (a.drains && (a.slots - 1) * a.steps < 2) continue;        // a slot would be needed before its steps are drained
+      }
       const int64_t resident = resident_clusters(s, sm_count);
       const int64_t rounds = (tiles + resident - 1) / resident;
       const int64_t cycles = rounds * ((steps + s - 1) / s * (slabs_per_step(mode) * step + fetch) + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
@@ -598,24 +747,25 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t slabs, int mode, bool gather,
 
 }  // namespace
 
-int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form) {
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form, bool close) {
   const kb200_kernel_desc& d = k.desc;
   const bool bf16 = d.precision == KB200_PREC_BF16;
   int bias_slot, res_slot;
-  if (!k.has_chain || k.batch != 1 || finish_of(k, &bias_slot, &res_slot) < 0) return -1;
+  bool vectors;
+  if (!k.has_chain || k.batch != 1 || finish_of(k, &bias_slot, &res_slot, &vectors) < 0) return -1;
+  if (!vectors && d.precision != KB200_PREC_FP32) return -1;
   for (int i : {0, 1, 2, 3, 4, 6})
     if (d.cfg[i] != 0) return -1;                     // a tile, stage or split was asked for (how to store is not a question here)
-  if (k.M >= (1 << 20) || k.N >= (1 << 24) || k.N % 4) return -1;
+  if (k.M >= (1 << 20) || k.N >= (1 << 24)) return -1;
   if (!b_kmajor && b_cols % (bf16 ? 64 : 32)) return -1;
   if (d.precision == KB200_PREC_FP32 && d.operands[d.b_slot].base_kind != KB200_BASE_CONST) return -1;
   const DevOperand& O = k.ops[k.chain.out_slot];
-  if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
+  if (O.stride[2] != 1 || O.stride[1] < k.N) return -1;
   if (((k.M + kSmallM - 1) / kSmallM) * ((k.N + 63) / 64) > 4096) return -1;
-  const int slab_k = bf16 ? 64 : 32;
-  return plan_small(k.M, k.N, (k.K + slab_k - 1) / slab_k, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, plan.sm_count).cycles;
+  return plan_small(k.M, k.N, k.K, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, close, plan.sm_count).cycles;
 }
 
-int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, void** state) {
+int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, bool close, void** state) {
   *state = nullptr;
   if (k.desc.precision == KB200_PREC_FP32 && b_tail == nullptr)
     return fail(KB200_ERR_ARGUMENT, "matmul %s: the tails of B are missing", k.desc.name);
@@ -624,12 +774,14 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   const kb200_kernel_desc& d = k.desc;
   const int mode = small_mode(d.precision, form);
   const bool gather = form == SMALL_A_GATHERED;
-  const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
+  bool vectors;
+  const int fin = finish_of(k, &st->bias_slot, &st->res_slot, &vectors);
+  p.vectors = vectors ? 1 : 0;
   const int slab_k = ops.bf16 ? 64 : 32, chunk = ops.bf16 ? 64 : 32;
   p.slab_k = slab_k;
   const int slabs = (int)((k.K + slab_k - 1) / slab_k), per_step = slabs_per_step(mode);
   p.num_steps = (slabs + per_step - 1) / per_step;
-  const SmallPlan how = plan_small(k.M, k.N, slabs, mode, gather, ops.bf16 && !ops.b_kmajor, plan.sm_count);
+  const SmallPlan how = plan_small(k.M, k.N, k.K, mode, gather, ops.bf16 && !ops.b_kmajor, close, plan.sm_count);
   const int bn = how.bn;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
@@ -653,15 +805,17 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.b_step16 = ops.b_kmajor ? 2u : (uint32_t)((ops.bf16 ? 16 : 8) * 128) >> 4;
   const uint32_t fmt = ops.bf16 ? 1u : 2u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
-  p.nacc = 1;
+  bool drains = false;
+  p.acc_slots = 1;
   p.tmem_cols = 32;
   if (mode == SMALL_EXACT) {
-    // one accumulator per 512 of K for the large products, beside that of the small ones
-    const int64_t want = ((int64_t)most * slab_k + 511) / 512;
-    p.nacc = want > exact_accumulators(bn) ? exact_accumulators(bn) : (int)want;
-
+    const Accumulate how_exact = accumulate_as(most, bn, accumulate_limit(k.M, k.N, k.K, close));
+    p.acc_slots = how_exact.slots;
+    p.acc_shift = how_exact.shift;
+    p.acc_steps = how_exact.steps;
+    drains = how_exact.drains;
   }
-  while (p.tmem_cols < (mode == SMALL_EXACT ? 1 + p.nacc : 1) * bn + kSmallACols) p.tmem_cols *= 2;
+  while (p.tmem_cols < (mode == SMALL_EXACT ? p.acc_slots + 1 : 1) * bn + kSmallACols) p.tmem_cols *= 2;
   p.kernel_index = kernel_index;
   p.status = plan.d_status;
   p.M = (int)k.M;
@@ -673,9 +827,12 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
   p.out = k.mirror_only && p.out16 ? nullptr : O.ptr;
   p.out_row = O.stride[1];
-  st->gather = gather;
   const DevOperand& A = k.ops[d.a_slot];
-  p.a = gather ? A.ptr : nullptr;
+  p.a = gather || mode == SMALL_EXACT ? A.ptr : nullptr;
+  const DevOperand& B = k.ops[d.b_slot];
+  p.b = B.ptr;
+  p.b_k = B.stride[1];
+  p.b_n = B.stride[2];
   p.a_row = A.stride[1];
   p.K = (int)k.K;
   // (Rows of shared memory that no box fills make accumulator rows that nobody reads.)
@@ -690,7 +847,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   st->map_bt = st->map_b;
   if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = small_kernel(mode, fin, bn, gather);
+  st->kernel = small_kernel(mode, fin, bn, gather, drains);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
   *state = st;
@@ -727,7 +884,7 @@ bool small_repoint(const PlanKernel& k, void* state) {
   SmallState* st = static_cast<SmallState*>(state);
   if (st->bias_slot >= 0) st->params.bias = k.ops[st->bias_slot].ptr;
   if (st->res_slot >= 0) st->params.res = k.ops[st->res_slot].ptr;
-  if (st->gather) st->params.a = k.ops[k.desc.a_slot].ptr;
+  if (st->params.a) st->params.a = k.ops[k.desc.a_slot].ptr;
   if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
   return (!st->a_moves || set_map_address(&st->map_a, k.ops[k.desc.a_slot].ptr)) &&
          (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));

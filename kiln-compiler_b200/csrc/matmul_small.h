@@ -11,10 +11,12 @@ namespace kb200 {
 enum SmallA : int { SMALL_A_MAPPED, SMALL_A_FLOAT32, SMALL_A_GATHERED };
 
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
-int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form);
+// `close`: exact FP32 as near to float64 as float32 sums on the CUDA cores.
+int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form, bool close);
 // Tensor maps and launch parameters.  `b_tail`: exact FP32, the tails of B in the layout of ops.b_base.
 // *state stays null when the operands cannot be described; a non-zero return is an error.
-int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, void** state);
+int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, bool close,
+               void** state);
 int small_launch(const Plan& plan, const void* state, cudaStream_t s);
 bool small_repoint(const PlanKernel& k, void* state);     // the operand pointers of `k` have moved
 void small_destroy(void* state);

@@ -1001,8 +1001,12 @@ __global__ void __launch_bounds__(256) transpose_rows_kernel(const float* __rest
 
 // tail[r][c] = what the tensor core's 19 leading bits leave of src[r][c]: the second TF32 terms of an
 // exact-FP32 operand.  Rows 16-byte aligned; the floats that fill a last vector are multiplied with nothing.
-__global__ void __launch_bounds__(256) tail_rows_kernel(const float* __restrict__ src, float* __restrict__ tail, uint32_t rows, uint32_t cols,
-                                                        int64_t s_row, int64_t t_row) {
+// Of a frozen weight, `heads` is the copy that the tensor core reads (src itself) and takes the rounded heads (see split_head);
+// null where the weight is read where it is, and cut off.
+template <bool WEIGHT>
+__global__ void __launch_bounds__(256) tail_rows_kernel(const float* src, float* __restrict__ tail, uint32_t rows, uint32_t cols,
+                                                        int64_t s_row, int64_t t_row, float* heads) {
+  auto tail_of = [heads](float x) { return !WEIGHT ? tf32_tail(x) : heads != nullptr ? split_tail(x) : cut_tail(x); };
   pdl_wait();                 // the producer of this kernel's inputs has completed
   pdl_launch_dependents();    // the next kernel may begin its start-up
   const uint32_t per_row = (cols + 3) >> 2, total = rows * per_row;
@@ -1028,7 +1032,10 @@ __global__ void __launch_bounds__(256) tail_rows_kernel(const float* __restrict_
     for (int u = 0; u < U; ++u) {
       if (base + (uint32_t)u * step >= total) continue;
       *reinterpret_cast<float4*>(tail + (int64_t)row[u] * t_row + c[u]) =
-          make_float4(tf32_tail(v[u].x), tf32_tail(v[u].y), tf32_tail(v[u].z), tf32_tail(v[u].w));
+          make_float4(tail_of(v[u].x), tail_of(v[u].y), tail_of(v[u].z), tail_of(v[u].w));
+      if (WEIGHT && heads != nullptr)
+        *reinterpret_cast<float4*>(heads + (int64_t)row[u] * s_row + c[u]) =
+            make_float4(split_head(v[u].x), split_head(v[u].y), split_head(v[u].z), split_head(v[u].w));
     }
   }
 }
@@ -1187,15 +1194,20 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   };
   k.launches = 1;
   cudaError_t made = cudaSuccess;
+  // FP32 operands of fewer than 32 rows, or that a tensor map cannot describe: the small kernel, which adds up in float32 as
+  // often as the CUDA cores' error asks for, or those.  (This file's kernel sums up to 1000 of K in the tensor
+  // core: 1000 x 1001 x 3071 of positive operands 7.1e-6 from exact, CUDA cores 8.5e-7, the small kernel 6.1e-7.)
+  const bool plain = k.M >= 32 && k.N % 4 == 0 && k.K % 4 == 0 && rows_describable(A, A.stride[1], k.batch) && rows_describable(B, b_src_row, k.batch);
+  const bool close_only = d.precision == KB200_PREC_FP32 && !plain;
   // Few tiles: the kernel written for latency, where the other kernels cover the shape too by the estimates of both.
   // The exact-FP32 form of this file's kernel: 128-column tiles at 1150 cycles per slab (shared memory), ~16500
   // once, the pass over A included.  A copy of A is a launch of its own, ~4000 cycles; the small kernel can do without.
   if (copy_b && !b_kmajor) b_map_cols = (b_cols + chunk_n - 1) / chunk_n * chunk_n;
   SmallA form = SMALL_A_MAPPED;
-  int64_t few = small_cycles(plan, k, b_kmajor, b_map_cols, form);
+  int64_t few = small_cycles(plan, k, b_kmajor, b_map_cols, form, close_only);
   if (few > 0 && copy_a) {
     const SmallA as_it_is = rows_describable(A, a_row, k.batch) ? SMALL_A_FLOAT32 : SMALL_A_GATHERED;
-    const int64_t direct = small_cycles(plan, k, b_kmajor, b_map_cols, as_it_is);
+    const int64_t direct = small_cycles(plan, k, b_kmajor, b_map_cols, as_it_is, close_only);
     few += 4000;
     if (direct < few) { form = as_it_is; few = direct; }
   }
@@ -1206,9 +1218,15 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
     if (many > 0 && copy_a) many += 4000;
   }
-  // (its exact-FP32 form multiplies with the tails of B: without room for them the kernel above makes them as it goes)
+  // (its exact-FP32 form multiplies with the tails of B: without room for them this file's kernel makes them as it goes)
   const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
-  const bool small = few > 0 && tails_ready && (many == 0 || few < many);
+  const bool small = few > 0 && tails_ready && (many == 0 || few < many || close_only);
+  if (close_only && !small) {
+    tc_destroy(k);
+    k.impl = IMPL_MM_SIMT;
+    k.launches = 1;
+    return KB200_OK;
+  }
   if (small && form != SMALL_A_MAPPED) {
     a_base = nullptr;
   } else if (copy_a) {
@@ -1248,8 +1266,8 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     KB200_CUDA(launch_copy(st->b_copy, st->bf16, B, b_src_row, k.batch, 4096, false, nullptr));
   }
   if (presplit)
-    KB200_CUDA(launch_kernel(false, tail_rows_kernel, dim3(cvt_grid(b_rows * ((b_map_cols + 3) / 4), 4096)), dim3(256), 0, nullptr, static_cast<const float*>(b_base), st->b_tail,
-                             (uint32_t)b_rows, (uint32_t)b_map_cols, b_row, b_row));
+    KB200_CUDA(launch_kernel(false, tail_rows_kernel<true>, dim3(cvt_grid(b_rows * ((b_map_cols + 3) / 4), 4096)), dim3(256), 0, nullptr, static_cast<const float*>(b_base), st->b_tail,
+                             (uint32_t)b_rows, (uint32_t)b_map_cols, b_row, b_row, static_cast<float*>(st->b_copy.data)));
   if (presplit || (copy_b && st->b_copy.once)) KB200_CUDA(cudaDeviceSynchronize());
   int bn = d.cfg[1];
   if (bn <= 0) {
@@ -1418,7 +1436,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
 
   const PairOperands po{st->bf16, a_base, a_row, a_batch, b_base, b_row, b_batch, b_map_cols, b_kmajor, st->b_copy.once};
   if (small) {
-    const int rc = small_bind(plan, k, kernel_index, po, st->b_tail, form, &st->small);
+    const int rc = small_bind(plan, k, kernel_index, po, st->b_tail, form, close_only, &st->small);
     if (rc) return rc;
     if (st->small) return KB200_OK;
     if (form != SMALL_A_MAPPED) return fail(KB200_ERR_UNSUPPORTED, "matmul %s: the operands cannot be described to TMA", d.name);
@@ -1488,8 +1506,8 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     // from the aligned copy, where there is one
     const float* src = st->a_copy.data ? static_cast<const float*>(st->a_copy.data) : k.ops[d.a_slot].ptr;
     const int64_t row = st->a_copy.data ? st->a_copy.pitch : k.ops[d.a_slot].stride[1];
-    KB200_CUDA(launch_kernel(plan.pdl, tail_rows_kernel, dim3(cvt_grid(k.M * ((k.K + 3) / 4), cap)), dim3(256), 0, s, src, st->a_tail, (uint32_t)k.M,
-                             (uint32_t)k.K, row, st->tail_pitch));
+    KB200_CUDA(launch_kernel(plan.pdl, tail_rows_kernel<false>, dim3(cvt_grid(k.M * ((k.K + 3) / 4), cap)), dim3(256), 0, s, src, st->a_tail, (uint32_t)k.M,
+                             (uint32_t)k.K, row, st->tail_pitch, (float*)nullptr));
   }
   if (st->small) return small_launch(plan, st->small, s);
   if (st->pair) return pair_launch(plan, st->pair, s);

@@ -224,6 +224,18 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// Exact FP32: x as two TF32 values, a head and a tail.  The tensor core cuts both off after 11 bits, which loses up to two of
+// the 13 that a head cut off leaves, always towards zero (768 x 768 of 128 rows: 4.0e-7 from exact).  So the tail is
+// rounded, and the head too where it is made once, at bind: its tail then has a sign of its own, and what is
+// dropped, tail x tail, no bias (1.4e-7).  Heads that would round to an infinity are cut off.
+__device__ __forceinline__ float rounded_tail(float t) { return __uint_as_float(__float_as_uint(t) + 0x1000u); }
+__device__ __forceinline__ float cut_tail(float x) { return rounded_tail(x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u)); }
+__device__ __forceinline__ float split_head(float x) {
+  const uint32_t u = __float_as_uint(x);
+  return __uint_as_float(((u & 0x7FFFFFFFu) < 0x7F7FF000u ? u + 0x1000u : u) & 0xFFFFE000u);
+}
+__device__ __forceinline__ float split_tail(float x) { return rounded_tail(x - split_head(x)); }
+
 // ---- thread-block clusters ----
 // The two halves of the hardware cluster barrier, usable apart: arrive early, wait when the result is needed.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
