@@ -213,9 +213,9 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * the float32 values: that arena region then holds stale data, which no planned kernel reads.  0 stores
  * both, for a caller that inspects intermediate buffers.
  * KB200_OPT_FP32_ATTENTION (default 0, FP32 precision): which kernel runs the fused attention.
- * 0 = by size (the tensor-core kernel, three TF32 products per float32 product, when its work items
- * fill a quarter of the SMs and no matmul of the chain asked for IEEE behaviour on non-finite
- * operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores.
+ * 0 = by size (the tensor-core kernel, three TF32 products per float32 product, for sequences of whole
+ * tiles of 128 tokens whose work items fill a quarter of the SMs, where it is estimated faster and no
+ * matmul of the chain asked for IEEE behaviour on non-finite operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores.
  * KB200_OPT_ATTENTION_SPLIT (default 1): in a launch that leaves SMs idle (one long sequence,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.

@@ -1063,18 +1063,19 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   // its last tokens reads zeros behind them (as the stores' maps drop those rows): any length works.
   AttnState* st = new AttnState();
   st->exact = c.exact;
-  // FP32 mode: the CUDA-core kernel (64 queries per CTA, long prefixes split) or the tensor-core kernel (128 queries
-  // and a pass over Q, K and V for their tails), whichever is estimated faster.  Both are a line through launches of 16 to
-  // 333 tokens and 4 to 96 heads, in ns: a fixed part, key tiles times rounds of the SMs, and that pass's bytes.
-  // (It was a quarter of the SMs' worth of work items: 48 heads of 64 tokens took 9.8 us on the tensor
-  // cores and 6.6 without, 4 heads of 200 tokens 13.0 and 11.3 on them.)  The plan option
-  // KB200_OPT_FP32_ATTENTION forces one of them.
+  // FP32 mode: the CUDA-core kernel (64 queries per CTA, long prefixes split), or the tensor-core kernel (128 queries and a pass
+  // over Q, K and V for their tails) for sequences of whole tiles that fill a quarter of the SMs, where that is estimated
+  // faster.  Both estimates are a line through launches of 16 to 333 tokens and 4 to 96 heads, in ns: a fixed part, key
+  // tiles times rounds of the SMs, and that pass's bytes (48 heads of 64 tokens: 9.8 us on the tensor cores, 6.6
+  // without).  Its sums are truncated in the tensor core: 1.9e-6 from float64 for 16 heads of 333 tokens, the CUDA cores'
+  // 2.0e-7 (16 against 24 us), so lengths and sizes that had been computed in float32 before there was a fused kernel for
+  // them keep that.  The plan option KB200_OPT_FP32_ATTENTION forces one of them.
   if (c.exact) {
     // (split operands turn an infinite element into a NaN tail: a plan that asked for IEEE behaviour keeps the FMA kernel)
     const int64_t sms = plan.sm_count, tiles64 = T <= 64 ? 1 : 2 * q_tiles;       // (three take as long as four)
     const int64_t fma_ns = 4200 + 2250 * tiles64 * ((B * H * tiles64 + sms - 1) / sms);
     const int64_t tc_ns = 6800 + 2400 * q_tiles * ((B * H * q_tiles + sms - 1) / sms) + B * T * 3 * H * hd * 8 / 6500;
-    st->exact_tc = !c.ieee && tc_ns <= fma_ns;
+    st->exact_tc = !c.ieee && T % kRows == 0 && B * H * q_tiles * 4 >= sms && tc_ns <= fma_ns;
     if (plan.fp32_attention == 1) st->exact_tc = false;
     if (plan.fp32_attention == 2) st->exact_tc = true;
   }

@@ -89,3 +89,46 @@ def test_infinities_through_every_epilogue(tokens, d):
     assert bool(torch.isinf(hidden[0]).all())
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
     assert float((got[1:].double() - want[1:]).norm() / want[1:].norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("batch,tokens,heads", [(4, 333, 4), (2, 1023, 4), (3, 129, 2), (1, 200, 12), (2, 256, 4)])
+def test_attention_of_any_length_is_as_exact_as_float32_sums(batch, tokens, heads):
+    """A score is a sum of 64 products scaled by 1/8, its partial sums at most about 1: 64 roundings of 2^-24 / sqrt(3) of half of that in the
+    mean square are 2e-7, which is the relative error of an unnormalised weight; the sum over the values
+    averages it.  (Truncated sums on the tensor cores: 1.3e-6 to 2.2e-6.)"""
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable
+    from perf import cases
+
+    d, hd = 64 * heads, 64
+    if batch == 1:                                   # the chain of one sequence: scale and mask in the first matmul
+        p = cases._Plan("attention", (tokens, 3 * d), (tokens, heads, hd))
+        kt, s, w, o = p.buffer(heads, hd, tokens), p.buffer(heads, tokens, tokens), p.buffer(heads, tokens, tokens), p.buffer(heads, tokens, hd)
+        p.copy(p.x.as_((heads, hd, tokens), (hd, 1, 3 * d), d), kt)
+        p.bmm(p.x.as_((heads, tokens, hd), (hd, 3 * d, 1)), kt, s, 0.125, p.const("mask", tokens, tokens))
+        p.softmax(s, w)
+        p.bmm(w, p.x.as_((heads, tokens, hd), (hd, 3 * d, 1), 2 * d), o)
+        p.copy(o.as_((tokens, heads, hd), (hd, tokens * hd, 1)), p.y)
+    else:
+        p = cases._Plan("attention", (batch * tokens, 3 * d), (batch, tokens, heads, hd))
+        rows = (tokens * 3 * d, hd, 3 * d, 1)
+        q, kt, v = p.buffer(batch, heads, tokens, hd), p.buffer(batch, heads, hd, tokens), p.buffer(batch, heads, tokens, hd)
+        s, w, o = p.buffer(batch * heads, tokens, tokens), p.buffer(batch, heads, tokens, tokens), p.buffer(batch * heads, tokens, hd)
+        p.copy(p.x.as_((batch, heads, tokens, hd), rows), q)
+        p.copy(p.x.as_((batch, heads, hd, tokens), (tokens * 3 * d, hd, 1, 3 * d), d), kt)
+        p.bmm(q.as_((batch * heads, tokens, hd)), kt.as_((batch * heads, hd, tokens)), s)
+        p.softmax(s.as_((batch, heads, tokens, tokens)), w, 0.125, p.const("mask", tokens, tokens))
+        p.copy(p.x.as_((batch, heads, tokens, hd), rows, 2 * d), v)
+        p.bmm(w.as_((batch * heads, tokens, tokens)), v.as_((batch * heads, tokens, hd)), o)
+        p.copy(o.as_((batch, tokens, heads, hd), (heads * tokens * hd, hd, tokens * hd, 1)), p.y)
+    plan = p.spec()
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    exe = GPUExecutable(program_from_plan(plan, "fp32"), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
+    assert "attention_fused" in exe.impls
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    x = torch.randn(plan.input_shapes[0], generator=gen, device="cuda")
+    got = exe(x)[0].double().view(batch, tokens, heads, hd)
+    q, k, v = x.double().view(batch, tokens, 3, heads, hd).permute(2, 0, 3, 1, 4)
+    mask = torch.from_numpy(consts["mask"]).cuda().double()
+    want = (torch.softmax(q @ k.transpose(-1, -2) * 0.125 + mask, -1) @ v).permute(0, 2, 1, 3)
+    assert float((got - want).norm() / want.norm()) <= 4e-7
