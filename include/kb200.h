@@ -17,9 +17,9 @@
  * synchronised, only while a plan is set up: kb200_plan_create allocates the
  * plan's status word, and kb200_plan_bind allocates the library-owned scratch
  * (in BF16 mode a bf16 mirror of the arena and packed bf16 copies of constant
- * matmul operands; in the other modes copies of them laid out along K and, for
- * exact FP32, their tails, where memory is plenty; aligned copies of operands
- * that a tensor map cannot describe; a staging buffer for a fused attention whose output aliases
+ * matmul operands; in the other modes copies of them laid out along K, for exact
+ * FP32 the operands' tails, and aligned copies of operands that a tensor map cannot
+ * describe, a quarter of the free memory for all of them; a staging buffer for a fused attention whose output aliases
  * its inputs; in FP32 mode the fused attention's scratch: the operands' tails or
  * the split tiles' partial results), converts the constants (cudaDeviceSynchronize) and reads the
  * attention mask back once (a blocking copy).  kb200_plan_launch and
@@ -220,8 +220,8 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.
  * KB200_OPT_WEIGHT_COPIES (default 1, FP32 and TF32 precision): frozen weights are also kept laid out along K
- * and, for FP32, with their tails, where memory is plenty (up to twice the weight's own bytes in FP32, once in
- * TF32).  0 = every weight is read where it is, as it is when memory is short. */
+ * and, for FP32, with their tails (twice the weight's own bytes in FP32, once in TF32), as far as a quarter of the
+ * free memory goes.  0 = every weight is read where it is, as it is beyond that. */
 typedef enum kb200_option {
   KB200_OPT_FUSE_ATTENTION = 1,
   KB200_OPT_DEPENDENT_LAUNCH = 2,

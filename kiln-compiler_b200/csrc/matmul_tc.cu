@@ -1154,15 +1154,16 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const DevOperand& B = k.ops[d.b_slot];
   // A frozen B is laid out along K once: both operands then use the ordinary 128-byte swizzle, and a tile may
   // have any width (an N-major one comes in whole 128-byte column chunks).
-  // In FP32 and TF32 that copy, and the tails of the exact mode, are additions to the weights: where they would
-  // take more than a quarter of what is free, the operand is read as it is.
+  // In FP32 and TF32 that copy, and the tails of the exact mode, are additions to the weights: they come out of the
+  // plan's budget for all of its copies, and where that is used up the operand is read as it is.
   const bool frozen = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
   drop_copies(st);
-  size_t free_bytes = 0, total_bytes = 0;
-  KB200_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-  const size_t copied = (size_t)k.N * k.K * sizeof(float) * (d.precision == KB200_PREC_FP32 ? 2 : 1);
-  const bool room = st->bf16 || (plan.weight_copies && copied <= free_bytes / 4);
-  const bool turn = frozen && room && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
+  const bool may_turn = frozen && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
+  const bool may_presplit = d.precision == KB200_PREC_FP32 && frozen && k.batch == 1;
+  const uint64_t additions = st->bf16 ? 0 : (uint64_t)k.N * ((k.K + 31) / 32 * 32) * sizeof(float) * ((may_turn ? 1 : 0) + (may_presplit ? 1 : 0));
+  const bool room = st->bf16 || (plan.weight_copies && additions <= plan.copy_budget);
+  if (room) plan.copy_budget -= additions;
+  const bool turn = may_turn && room;
   const bool b_kmajor = turn || B.stride[2] != 1;
   const int64_t b_rows = b_kmajor ? k.N : k.K, b_cols = b_kmajor ? k.K : k.N, b_src_row = B.stride[2] != 1 ? B.stride[2] : B.stride[1];
   const void* a_base = A.ptr;
@@ -1177,7 +1178,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // bytes a clock.
   if (st->small) small_destroy(st->small);
   st->small = nullptr;
-  const bool presplit = d.precision == KB200_PREC_FP32 && frozen && room && k.batch == 1;
+  const bool presplit = may_presplit && room;
   st->b_copy.once = frozen;
   st->b_copy.turned = turn;
   const bool copy_a = st->bf16 ? k.a_shadow == nullptr : !rows_describable(A, a_row, k.batch);
@@ -1190,7 +1191,12 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     c.rows = rows;
     c.cols = cols;
     c.pitch = (cols + chunk_n - 1) / chunk_n * chunk_n;
-    return cudaMalloc(&c.data, (size_t)k.batch * rows * c.pitch * esz);
+    const uint64_t bytes = (uint64_t)k.batch * rows * c.pitch * esz;
+    if (!st->bf16 && !c.turned) {                     // (a weight's copy along K is paid for above)
+      if (bytes > plan.copy_budget) return cudaErrorMemoryAllocation;
+      plan.copy_budget -= bytes;
+    }
+    return cudaMalloc(&c.data, bytes);
   };
   k.launches = 1;
   cudaError_t made = cudaSuccess;
@@ -1222,6 +1228,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
   const bool small = few > 0 && tails_ready && (many == 0 || few < many || close_only);
   if (close_only && !small) {
+    if (room) plan.copy_budget += additions;
     tc_destroy(k);
     k.impl = IMPL_MM_SIMT;
     k.launches = 1;
@@ -1247,14 +1254,16 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   } else if (st->bf16) {
     b_base = k.b_shadow;
   }
-  const bool a_pass = presplit && k.M > kTileM && !small;
+  const uint64_t a_tail_bytes = (uint64_t)k.M * ((k.K + chunk_n - 1) / chunk_n * chunk_n) * sizeof(float);
+  const bool a_pass = presplit && k.M > kTileM && !small && a_tail_bytes <= plan.copy_budget;
+  if (a_pass) plan.copy_budget -= a_tail_bytes;
   if (presplit && made == cudaSuccess) made = cudaMalloc(&st->b_tail, (size_t)b_rows * b_row * sizeof(float));
   if (a_pass && made == cudaSuccess) {
     st->tail_pitch = (k.K + chunk_n - 1) / chunk_n * chunk_n;
     made = cudaMalloc(&st->a_tail, (size_t)k.M * st->tail_pitch * sizeof(float));
     ++k.launches;
   }
-  if (made == cudaErrorMemoryAllocation && !st->bf16) {      // no room for an aligned copy: the CUDA-core kernel reads operands as they are
+  if (made == cudaErrorMemoryAllocation && !st->bf16) {      // no room for an aligned copy: the CUDA-core kernel reads operands as they are ("mm_simt_fp32" says so)
     cudaGetLastError();
     tc_destroy(k);
     k.impl = IMPL_MM_SIMT;

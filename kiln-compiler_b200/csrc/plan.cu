@@ -1145,7 +1145,19 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   if (rc == KB200_OK) rc = assign_shadows(plan);
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i)
     if (plan.kernels[i].impl == IMPL_ATTN_FUSED) attention_elide_copy(plan, i);
-  // phase 4: tensor maps, packed weights, split-K workspaces
+  // phase 4: tensor maps, packed weights, split-K workspaces.  What FP32 and TF32 matmuls add to make operands quicker to read
+  // (a weight along K, its tails, aligned rows, the tails of A) takes a quarter of what is free in all, beside
+  // a call's outputs; each on its own was allowed that much, and a plan of many Linears left nothing for its caller.
+  if (rc == KB200_OK) {
+    for (PlanKernel& k : plan.kernels)
+      if (k.desc.kclass == KB200_K_MATMUL) destroy_matmul(k);
+    size_t free_bytes = 0, total_bytes = 0;
+    const cudaError_t e = cudaMemGetInfo(&free_bytes, &total_bytes);
+    if (e != cudaSuccess) rc = cuda_fail(e, "cudaMemGetInfo");
+    uint64_t outputs = 0;
+    for (uint64_t bytes : plan.output_bytes) outputs += bytes;
+    plan.copy_budget = free_bytes > outputs ? (free_bytes - outputs) / 4 : 0;
+  }
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
     PlanKernel& k = plan.kernels[i];
     if (k.desc.kclass == KB200_K_MATMUL && k.impl != IMPL_FUSED_AWAY) rc = bind_matmul(plan, k);

@@ -179,12 +179,18 @@ class GPUExecutable:
         out_bytes = sum(4 * int(np.prod(s)) for s in self.output_shapes)
         # what the library allocates itself when buffers are bound, in BF16 mode: a bf16 mirror of the
         # arena, packed bf16 copies of the constant matmul operands, and (worst case) bf16 copies of
-        # unmirrored activations no larger than the inputs and the arena together
-        # (the copies of weights that FP32 and TF32 matmuls prefer to read are made only where they leave
-        # most of the free memory, so nothing is set aside for them)
+        # unmirrored activations no larger than the inputs and the arena together, with rows padded to
+        # 128-byte lines
+        # (what FP32 and TF32 matmuls copy to read it quicker takes at most a quarter of the memory that is free
+        # beside a call's outputs when buffers are bound, and is not made beyond that: nothing is set aside for it)
         library_bytes = 0
+        descs = lowering.lower(program.plan, program.launches, program.precision, used)
         if program.precision == "bf16":
             library_bytes = arena_bytes // 2 + 256 + const_bytes // 2 + (io_bytes + arena_bytes) // 2
+            for d in descs[:len(program.launches)]:
+                if d.kclass == _cabi.K_MATMUL:
+                    batch, m, n = d.iter_shape[:3]
+                    library_bytes += 2 * batch * ((m + n) * (-d.k_extent % 64) + d.k_extent * (-n % 64))
         elif program.precision == "fp32":
             # the fused attention's scratch: the tails of Q, K and V (a copy of part of the arena) or the
             # split tiles' partial results (smaller than the merged heads)
@@ -204,7 +210,6 @@ class GPUExecutable:
                               if int(np.prod(s)) else torch.zeros(s, device=self.device) for s in self.input_shapes]
         self.static_outputs = [torch.empty(s, device=self.device) for s in self.output_shapes]
 
-        descs = lowering.lower(program.plan, program.launches, program.precision, self.const_names)
         self._descs = descs
         _cabi.check(self._lib.kb200_plan_create(descs, len(program.launches), self.device.index,
                                                 C.byref(self._plan)), self._lib)
