@@ -119,6 +119,7 @@ struct Plan {
   bool fuse_attention = true;    // replace the five-kernel attention chain by the fused kernel when it matches
   int fp32_attention = 0;        // FP32 precision: 0 = pick the fused attention kernel by size, 1 = CUDA cores, 2 = tensor cores
   bool attention_split = true;   // share long query tiles between two CTAs when a launch would leave SMs idle
+  mutable int resident_clusters[9] = {};   // by cluster size, as the few-tiles matmul asked for them (0: not yet)
   uint64_t copy_budget = 0;      // bytes that FP32 and TF32 matmuls may still take for copies, while the plan is bound
   bool weight_copies = true;     // FP32 and TF32: frozen weights are also kept along K, and with their tails, where memory is plenty
   bool fold_copies = true;       // a matmul reads a K-contiguous B at its source; the plan's transposing copy is not launched

@@ -643,10 +643,11 @@ int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot, bool* vectors)
 
 // Clusters of `splits` CTAs, one CTA per SM, that fit the GPU at once (147 SMs in use at most: the SMs of
 // a processing cluster need not be a multiple of the size).
-int resident_clusters(int splits, int sm_count) {
-  static int known[9] = {0};
+int resident_clusters(const Plan& plan, int splits) {
+  const int sm_count = plan.sm_count;
   if (splits == 1) return sm_count;
-  if (known[splits] == 0) {
+  int& known = plan.resident_clusters[splits];
+  if (known == 0) {
     int n = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(splits * (sm_count / splits)), 1, 1);
@@ -664,9 +665,9 @@ int resident_clusters(int splits, int sm_count) {
       cudaGetLastError();
       n = sm_count * 7 / 10 / splits;
     }
-    known[splits] = n > 0 ? n : 1;
+    known = n > 0 ? n : 1;
   }
-  return known[splits];
+  return known;
 }
 
 // Exact FP32: accumulators beside that of the small products and the slabs of A.
@@ -719,7 +720,7 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 // 1024 x 768 x 3072 31.2 -> 27.8, 364 x 768 x 3072 22.3 -> 16.4).
 // GATHER: a warp loads, parks and reads back a slab of A one step ahead of its use, bound by the load/store unit (rows off the
 // lines: two of them to a load): what it adds to a step against the copied A (65 to 3000 of K).
-SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, bool chunked, bool close, int sm_count) {
+SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, bool chunked, bool close, const Plan& plan) {
   const int64_t slab_k = mode == SMALL_BF16 || mode == SMALL_BF16_A32 ? 64 : 32, slabs = (k + slab_k - 1) / slab_k;
   SmallPlan best{64, 1, 0};
   const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
@@ -736,7 +737,7 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, boo
         const Accumulate a = accumulate_as((int)((steps + s - 1) / s), bn, accumulate_limit(m, n, k, close));
         if (a.drains && (a.slots - 1) * a.steps < 2) continue;        // a slot would be needed before its steps are drained
       }
-      const int64_t resident = resident_clusters(s, sm_count);
+      const int64_t resident = resident_clusters(plan, s);
       const int64_t rounds = (tiles + resident - 1) / resident;
       const int64_t cycles = rounds * ((steps + s - 1) / s * (slabs_per_step(mode) * step + fetch) + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
       if (best.cycles == 0 || cycles < best.cycles) best = {bn, s, cycles};
@@ -762,7 +763,7 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
   const DevOperand& O = k.ops[k.chain.out_slot];
   if (O.stride[2] != 1 || O.stride[1] < k.N) return -1;
   if (((k.M + kSmallM - 1) / kSmallM) * ((k.N + 63) / 64) > 4096) return -1;
-  return plan_small(k.M, k.N, k.K, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, close, plan.sm_count).cycles;
+  return plan_small(k.M, k.N, k.K, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, close, plan).cycles;
 }
 
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, bool close, void** state) {
@@ -781,7 +782,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.slab_k = slab_k;
   const int slabs = (int)((k.K + slab_k - 1) / slab_k), per_step = slabs_per_step(mode);
   p.num_steps = (slabs + per_step - 1) / per_step;
-  const SmallPlan how = plan_small(k.M, k.N, k.K, mode, gather, ops.bf16 && !ops.b_kmajor, close, plan.sm_count);
+  const SmallPlan how = plan_small(k.M, k.N, k.K, mode, gather, ops.bf16 && !ops.b_kmajor, close, plan);
   const int bn = how.bn;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
