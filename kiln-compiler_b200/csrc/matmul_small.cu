@@ -43,6 +43,7 @@ constexpr int kSmallMaxStages = 8;
 constexpr int kSmallABytes = kSmallM * 128;      // one 128-byte K slab
 constexpr int kSmallACols = 128;                 // tensor-memory columns for slabs of A
 constexpr int kSmallSmem = 225 * 1024;
+constexpr size_t kSmallAloneSmem = 164 * 1024;   // beside this, 228 KB an SM have less left than the 65 KB of the smallest clustered launch
 constexpr int kSmallMaxSlots = 5;                // exact FP32: accumulators of 64 columns beside that of the small products and the slabs of A
 
 // SMALL_BF16_A32: bf16 products of an A that is still float32, rounded on its way to tensor memory.  (A Linear of the caller's
@@ -817,6 +818,10 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
     drains = how_exact.drains;
   }
   while (p.tmem_cols < (mode == SMALL_EXACT ? p.acc_slots + 1 : 1) * bn + kSmallACols) p.tmem_cols *= 2;
+  // Two clusters of plans on different streams must not share SMs where their tensor memory does not fit both: a CTA of each
+  // could wait for columns that the other's neighbour holds, until the bounded waits end both.  Of 256 columns two fit (and
+  // registers allow no third); with more, shared memory that leaves no room for the smallest such CTA keeps it away.
+  if (p.splits > 1 && p.tmem_cols > 256 && st->smem < kSmallAloneSmem) st->smem = kSmallAloneSmem;
   p.kernel_index = kernel_index;
   p.status = plan.d_status;
   p.M = (int)k.M;
