@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define KB200_ABI_VERSION 4
+#define KB200_ABI_VERSION 5
 
 #define KB200_MAX_RANK 6      /* iteration dims after the host collapsed contiguous ones */
 #define KB200_MAX_OPERANDS 12 /* distinct tensors one fused kernel touches */
@@ -221,7 +221,12 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.
  * KB200_OPT_WEIGHT_COPIES (default 1, FP32 and TF32 precision): frozen weights are also kept laid out along K
  * and, for FP32, with their tails (twice the weight's own bytes in FP32, once in TF32), as far as a quarter of the
- * free memory goes.  0 = every weight is read where it is, as it is beyond that. */
+ * free memory goes.  0 = every weight is read where it is, as it is beyond that.
+ * KB200_OPT_FEW_TILES (default 0): asks the matmul kernel for few tiles for one of its forms instead of the one it
+ * estimates to be quickest, where it covers a matmul: tile columns (64, 96 or 128) + 1000 * K splits (1, 2, 4 or 8)
+ * + 10000 * (1 + how A comes, if not through a tensor map of its own: 0 a copy, 1 as float32 for BF16, 2 read by the
+ * kernel's warps); a part that is 0 is left to the estimate, a form that the matmul cannot take to the other
+ * kernels. */
 typedef enum kb200_option {
   KB200_OPT_FUSE_ATTENTION = 1,
   KB200_OPT_DEPENDENT_LAUNCH = 2,
@@ -231,7 +236,8 @@ typedef enum kb200_option {
   KB200_OPT_MIRROR_ONLY = 6,
   KB200_OPT_FP32_ATTENTION = 7,
   KB200_OPT_ATTENTION_SPLIT = 8,
-  KB200_OPT_WEIGHT_COPIES = 9
+  KB200_OPT_WEIGHT_COPIES = 9,
+  KB200_OPT_FEW_TILES = 10
 } kb200_option;
 int kb200_plan_set_option(kb200_plan* plan, int option, int value);
 
@@ -261,8 +267,12 @@ int kb200_kernel_launch(kb200_plan* plan, int i, void* cuda_stream);
 int kb200_plan_launch_count(const kb200_plan* plan);
 
 /* Name of the implementation chosen for kernel `i` ("ew_chain_vec4",
- * "row_layernorm_warp", "mm_tcgen05_tf32", ...).  Never NULL for a valid i. */
+ * "row_layernorm", "mm_tcgen05", ...).  Never NULL for a valid i. */
 const char* kb200_kernel_impl(const kb200_plan* plan, int i);
+
+/* What runs a bound kernel `i`, in more words: for a tensor-core matmul the kernel ("mm_small", "mm_pair", "mm_tc"),
+ * its tile, its split and the operands it copies.  Valid until the thread's next call of this function. */
+const char* kb200_kernel_detail(const kb200_plan* plan, int i);
 
 /* Number of fused scalar steps kernel `i` applies per element as bound: the epilogue chain of a
  * matmul (including the steps of an elementwise or row kernel it took over, see

@@ -119,6 +119,7 @@ struct Plan {
   bool fuse_attention = true;    // replace the five-kernel attention chain by the fused kernel when it matches
   int fp32_attention = 0;        // FP32 precision: 0 = pick the fused attention kernel by size, 1 = CUDA cores, 2 = tensor cores
   bool attention_split = true;   // share long query tiles between two CTAs when a launch would leave SMs idle
+  int few_tiles = 0;             // KB200_OPT_FEW_TILES: the form of the matmul kernel for few tiles that is to be used, 0 = by estimate
   mutable int resident_clusters[9] = {};   // by cluster size, as the few-tiles matmul asked for them (0: not yet)
   uint64_t copy_budget = 0;      // bytes that FP32 and TF32 matmuls may still take for copies, while the plan is bound
   bool weight_copies = true;     // FP32 and TF32: frozen weights are also kept along K, and with their tails, where memory is plenty
@@ -163,6 +164,7 @@ int choose_reduce(Plan& plan, PlanKernel& k);
 int launch_reduce(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 int choose_matmul(Plan& plan, PlanKernel& k);
 int bind_matmul(Plan& plan, PlanKernel& k);      // after pointers are resolved
+std::string matmul_detail(const PlanKernel& k);   // which kernel, tile and split a bound matmul uses
 bool repoint_matmul(PlanKernel& k);              // operand pointers changed: follow in tensor maps and parameters
 bool matmul_wants_bf16_operands(const PlanKernel& k);
 void attention_set_shadow(PlanKernel& k, void* shadow_out);

@@ -9,6 +9,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index);
 int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 void tc_destroy(PlanKernel& k);
 bool tc_repoint(PlanKernel& k);
+std::string tc_detail(const PlanKernel& k);
 
 int choose_matmul(Plan& plan, PlanKernel& k) {
   (void)plan;
@@ -40,6 +41,8 @@ int launch_matmul(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
 }
 
 bool repoint_matmul(PlanKernel& k) { return tc_repoint(k); }
+
+std::string matmul_detail(const PlanKernel& k) { return tc_detail(k); }
 
 void destroy_matmul(PlanKernel& k) { tc_destroy(k); }
 

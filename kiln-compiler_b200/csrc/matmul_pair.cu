@@ -879,6 +879,11 @@ bool pair_repoint(const PlanKernel& k, void* state, const void* a, const void* b
   return ok;
 }
 
+std::string pair_detail(const void* state) {
+  const PairState* st = static_cast<const PairState*>(state);
+  return "mm_pair " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.kps) + " slabs";
+}
+
 void pair_destroy(void* state) { delete static_cast<PairState*>(state); }
 
 }  // namespace kb200

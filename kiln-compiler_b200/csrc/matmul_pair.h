@@ -28,6 +28,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
 int pair_launch(const Plan& plan, const void* state, cudaStream_t s);
 // Follows moved operand pointers of `k`; `a` / `b` null: that operand's map stays.
 bool pair_repoint(const PlanKernel& k, void* state, const void* a, const void* b);
+std::string pair_detail(const void* state);
 void pair_destroy(void* state);
 
 }  // namespace kb200

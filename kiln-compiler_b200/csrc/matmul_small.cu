@@ -580,6 +580,9 @@ struct SmallState {
   unsigned grid = 0;
   size_t smem = 0;
   int bias_slot = -1, res_slot = -1;
+  int bn = 0;                                 // (these three for small_detail)
+  SmallA form = SMALL_A_MAPPED;
+  bool drains = false;
   bool a_moves = false, b_moves = false;      // the maps hold the operand's own address
 };
 
@@ -725,7 +728,9 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, boo
   const int64_t slab_k = mode == SMALL_BF16 || mode == SMALL_BF16_A32 ? 64 : 32, slabs = (k + slab_k - 1) / slab_k;
   SmallPlan best{64, 1, 0};
   const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
+  const int asked_bn = plan.few_tiles % 1000, asked_splits = plan.few_tiles / 1000 % 10;
   for (int bn : {64, 96, 128}) {
+    if (asked_bn != 0 && bn != asked_bn) continue;
     if (bn == 96 && chunked) continue;                  // an N-major B comes in chunks of 64 bf16 columns
     if (bn > 64 && gather && mode == SMALL_EXACT) continue;      // rows of A and 64 sums do not fit the registers together
     const int64_t step = mode == SMALL_EXACT ? 435 + 4 * bn : mode == SMALL_BF16_A32 ? 450 + bn * 25 / 32 : 198 + bn * 13 / 8;
@@ -734,6 +739,7 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, boo
     for (int s : {1, 2, 4, 8}) {
       const int64_t steps = (slabs + slabs_per_step(mode) - 1) / slabs_per_step(mode);
       if (s > steps) break;
+      if (asked_splits != 0 && s != asked_splits) continue;
       if (mode == SMALL_EXACT) {
         const Accumulate a = accumulate_as((int)((steps + s - 1) / s), bn, accumulate_limit(m, n, k, close));
         if (a.drains && (a.slots - 1) * a.steps < 2) continue;        // a slot would be needed before its steps are drained
@@ -785,6 +791,8 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.num_steps = (slabs + per_step - 1) / per_step;
   const SmallPlan how = plan_small(k.M, k.N, k.K, mode, gather, ops.bf16 && !ops.b_kmajor, close, plan);
   const int bn = how.bn;
+  st->bn = bn;
+  st->form = form;
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
@@ -807,7 +815,6 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.b_step16 = ops.b_kmajor ? 2u : (uint32_t)((ops.bf16 ? 16 : 8) * 128) >> 4;
   const uint32_t fmt = ops.bf16 ? 1u : 2u;
   p.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((ops.b_kmajor ? 0u : 1u) << 16) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kSmallM >> 4) << 24);
-  bool drains = false;
   p.acc_slots = 1;
   p.tmem_cols = 32;
   if (mode == SMALL_EXACT) {
@@ -815,7 +822,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
     p.acc_slots = how_exact.slots;
     p.acc_shift = how_exact.shift;
     p.acc_steps = how_exact.steps;
-    drains = how_exact.drains;
+    st->drains = how_exact.drains;
   }
   while (p.tmem_cols < (mode == SMALL_EXACT ? p.acc_slots + 1 : 1) * bn + kSmallACols) p.tmem_cols *= 2;
   // Two clusters of plans on different streams must not share SMs where their tensor memory does not fit both: a CTA of each
@@ -853,7 +860,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   st->map_bt = st->map_b;
   if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = small_kernel(mode, fin, bn, gather, drains);
+  st->kernel = small_kernel(mode, fin, bn, gather, st->drains);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
   *state = st;
@@ -894,6 +901,13 @@ bool small_repoint(const PlanKernel& k, void* state) {
   if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
   return (!st->a_moves || set_map_address(&st->map_a, k.ops[k.desc.a_slot].ptr)) &&
          (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));
+}
+
+std::string small_detail(const void* state) {
+  const SmallState* st = static_cast<const SmallState*>(state);
+  const char* const a = st->form == SMALL_A_GATHERED ? ", A gathered" : st->form == SMALL_A_FLOAT32 ? ", A float32" : "";
+  return "mm_small " + std::to_string(st->bn) + " columns, " + std::to_string(st->params.splits) + " splits, " + std::to_string(st->params.stages) +
+         " stages" + a + (st->drains ? ", drains" : "");
 }
 
 void small_destroy(void* state) { delete static_cast<SmallState*>(state); }

@@ -19,6 +19,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
                void** state);
 int small_launch(const Plan& plan, const void* state, cudaStream_t s);
 bool small_repoint(const PlanKernel& k, void* state);     // the operand pointers of `k` have moved
+std::string small_detail(const void* state);
 void small_destroy(void* state);
 
 }  // namespace kb200

@@ -1217,8 +1217,14 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     few += 4000;
     if (direct < few) { form = as_it_is; few = direct; }
   }
+  if (few > 0 && plan.few_tiles >= 10000 && copy_a) {          // (a form is asked for)
+    const int asked = plan.few_tiles / 10000 - 1;
+    const bool takes = asked == SMALL_A_MAPPED || asked == SMALL_A_GATHERED || (asked == SMALL_A_FLOAT32 && st->bf16 && rows_describable(A, a_row, k.batch));
+    form = takes ? static_cast<SmallA>(asked) : SMALL_A_MAPPED;
+    few = takes ? small_cycles(plan, k, b_kmajor, b_map_cols, form, close_only) : -1;
+  }
   int64_t many = 0;
-  if (few > 0 && k.M > kTileM) {
+  if (few > 0 && k.M > kTileM && plan.few_tiles == 0) {
     const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
     if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
     else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k);
@@ -1563,6 +1569,15 @@ bool tc_repoint(PlanKernel& k) {
   bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b));
   if (st->params.store_mode == 1) ok = ok && set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr);
   return ok;
+}
+
+std::string tc_detail(const PlanKernel& k) {
+  const TcState* st = static_cast<const TcState*>(k.tc);
+  if (!st) return "";
+  const std::string copies = std::string(st->a_copy.data ? ", A copied" : "") + (st->b_copy.data ? ", B copied" : "");
+  if (st->small) return small_detail(st->small) + copies;
+  if (st->pair) return pair_detail(st->pair) + copies;
+  return "mm_tc " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.splits) + " splits" + copies;
 }
 
 void tc_destroy(PlanKernel& k) {

@@ -1182,6 +1182,7 @@ KB200_EXPORT int kb200_plan_set_option(kb200_plan* p, int option, int value) {
     case KB200_OPT_FP32_ATTENTION: plan.fp32_attention = value < 0 || value > 2 ? 0 : value; return KB200_OK;
     case KB200_OPT_ATTENTION_SPLIT: plan.attention_split = value != 0; return KB200_OK;
     case KB200_OPT_WEIGHT_COPIES: plan.weight_copies = value != 0; return KB200_OK;
+    case KB200_OPT_FEW_TILES: plan.few_tiles = value < 0 ? 0 : value; return KB200_OK;
     default: return fail(KB200_ERR_ARGUMENT, "kb200_plan_set_option: unknown option %d", option);
   }
 }
@@ -1245,6 +1246,16 @@ KB200_EXPORT const char* kb200_kernel_impl(const kb200_plan* p, int i) {
   if (i < 0 || i >= (int)plan.kernels.size()) return "?";
   if (!plan.bound) return "unbound";
   return impl_name(plan.kernels[i].impl);
+}
+
+KB200_EXPORT const char* kb200_kernel_detail(const kb200_plan* p, int i) {
+  static thread_local std::string text;
+  if (p == nullptr) return "";
+  const Plan& plan = *reinterpret_cast<const Plan*>(p);
+  if (i < 0 || i >= (int)plan.kernels.size() || !plan.bound) return "";
+  const PlanKernel& k = plan.kernels[i];
+  text = k.impl == IMPL_MM_TC ? matmul_detail(k) : impl_name(k.impl);
+  return text.c_str();
 }
 
 KB200_EXPORT int kb200_kernel_chain_length(const kb200_plan* p, int i) {

@@ -16,7 +16,7 @@ import subprocess
 import sysconfig
 from pathlib import Path
 
-ABI_VERSION = 4
+ABI_VERSION = 5
 MAX_RANK, MAX_OPERANDS, MAX_TAPE = 6, 12, 96
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -36,6 +36,7 @@ OPT_MIRROR_ONLY = 6
 OPT_FP32_ATTENTION = 7
 OPT_ATTENTION_SPLIT = 8
 OPT_WEIGHT_COPIES = 9
+OPT_FEW_TILES = 10
 BASE_KINDS = {"arena": 0, "const": 1, "input": 2, "output": 3}
 PRECISIONS = {"fp32": 0, "tf32": 1, "bf16": 2}
 OPCODES = {
@@ -79,6 +80,7 @@ EXPORTS = {
     "kb200_plan_run": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p), C.c_int, C.POINTER(C.c_void_p), C.c_int, C.c_void_p]),
     "kb200_kernel_launch": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p]),
     "kb200_plan_launch_count": (C.c_int, [C.c_void_p]),
+    "kb200_kernel_detail": (C.c_char_p, [C.c_void_p, C.c_int]),
     "kb200_kernel_impl": (C.c_char_p, [C.c_void_p, C.c_int]),
     "kb200_kernel_chain_length": (C.c_int, [C.c_void_p, C.c_int]),
     "kb200_plan_status": (C.c_int, [C.c_void_p]),
