@@ -156,3 +156,29 @@ def test_a_result_that_autograd_watches_is_refused():
     exe.run_on([x], [saved])
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         loss.backward()
+
+
+@pytest.mark.parametrize("beyond", [0, 1])
+def test_both_sides_of_the_limit_of_direct_calls(beyond):
+    """A plan of as many launches as are enqueued directly, and one of one more, which replays a graph: the same results."""
+    from kiln_b200 import runtime
+    from kiln_b200.codegen import program_from_plan
+    from perf import cases
+
+    rows, d, n = 37, 260, runtime.DIRECT_LAUNCHES + beyond
+    p = cases._Plan("norms", (rows, d), (rows, d))
+    x = p.x
+    for i in range(n):
+        y = p.y if i + 1 == n else p.buffer(rows, d)
+        p.layernorm(x, f"{i}.", y)
+        x = y
+    plan = p.spec()
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    exe = runtime.GPUExecutable(program_from_plan(plan, "fp32"), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
+    assert exe.device_launches == n and (exe._caller is None) == bool(beyond)
+    inputs = [torch.randn(rows, d, device="cuda") for _ in range(3)]
+    outputs = [exe(x)[0] for x in inputs]
+    for x, got in zip(inputs, outputs):
+        exe.static_inputs[0].copy_(x)
+        exe._launch()
+        assert torch.equal(exe.static_outputs[0], got)
