@@ -443,19 +443,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __shared__ int abort_flag;
   __shared__ int arrived[4];                  // split items: was this lane quadrant's half the second to arrive?
 
-#ifdef KB200_TRACE
-  __shared__ long long trace[4][16];
-  __shared__ long long marks[4];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    unsigned long long g;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
-    marks[0] = (long long)g;
-    marks[1] = clock64();
-  }
-#define ATTN_STAMP(role, idx) do { if (blockIdx.x == 0 && threadIdx.x == 64 && (idx) < 16) trace[role][idx] = clock64(); } while (0)
-#else
-#define ATTN_STAMP(role, idx) do { } while (0)
-#endif
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t q_smem = (raw + 1023u) & ~1023u;
   const uint32_t k_smem = q_smem + (EXACT ? kOpBytes : kTileBytes);   // ring of 2 tiles | EXACT: one buffer (tile, then its tails)
@@ -752,7 +739,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const int s = t & 1;
         const uint32_t ph = (t >> 1) & 1;
         if (!mbar_wait(sfull0 + 8 * s, ph, abort_ptr)) give_up(0x31);
-        ATTN_STAMP(0, j);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t s_addr = tmem_base + lane_addr + (uint32_t)(s * 128 + c0);
         const bool diagonal = it.j0 + j == it.qt;
@@ -785,7 +771,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           // Fold the PREVIOUS tile's O_part first: that it is complete also says that its P V has read the
           // tails of P, whose single buffer is written next.
           if (j > 0) fold(t - 1, alpha_prev);
-          ATTN_STAMP(3, j);
           const uint32_t pt_addr = tmem_pt + lane_addr + (uint32_t)c0;
           float ta[32];
           tmem_st32(s_addr, va);
@@ -816,11 +801,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         tmem_st_wait();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         mbar_arrive(pfull0 + 8 * (group * 2 + s));
-        ATTN_STAMP(1, j);
         // fold the PREVIOUS tile's O_part while the tensor pipe works on this one
         if constexpr (!EXACT) {
           if (j > 0) fold(t - 1, alpha_prev);
-          ATTN_STAMP(3, j);
         }
         alpha_prev = alpha;
         l_run = l_run * alpha + sum;
@@ -828,11 +811,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       }
       if (ok) fold(t0 + n_kv - 1, alpha_prev);
       t0 += n_kv;
-      ATTN_STAMP(2, 3 * ii);
       // ---- the row sum is the two threads' partial sums; thread g normalises and stores dims g*32 .. g*32+31 ----
       xsum[((ii & 1) * 2 + group) * kRows + row] = l_run;
       if (pair_sync_aborted()) ok = false;
-      ATTN_STAMP(2, 3 * ii + 1);
       // ---- a split item: leave this half's rows and state in the workspace; whoever arrives second merges.
       // Nobody waits for the other half.  The arrival is counted per lane quadrant (its 64 threads have a
       // barrier of their own, the one that also carries the abort flag), so no CTA-wide barrier is needed.
@@ -905,7 +886,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           }
         }
       }
-      ATTN_STAMP(2, 3 * ii + 2);
     }
     if (!EXACT && lane == 0) tma_store_wait_read();    // shared memory must outlive the stores that read it
   }
@@ -913,20 +893,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-#ifdef KB200_TRACE
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    unsigned long long g;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
-    printf("ATTN block0 globaltimer start %lld end %lld (ns) dur %lld | exit cycles %lld n_kv %d\n", marks[0], (long long)g,
-           (long long)g - marks[0], clock64() - marks[1], item_of(blockIdx.x).n_kv);
-    printf("softmax thread per item (tiles done, states exchanged, rows stored):");
-    for (int j = 0; j < 15; ++j) printf(" %lld", trace[2][j] - marks[1]);
-    printf("\n");
-    for (int j = 0; j < item_of(blockIdx.x).n_kv && j < 16; ++j)
-      printf("kv %2d  s_ready %7lld p_stored %7lld folded %7lld\n", j, trace[0][j] - marks[1], trace[1][j] - marks[1],
-             trace[3][j] - marks[1]);
-  }
-#endif
   if (abort_flag && threadIdx.x == 0) {
     for (int s = 0; s < (EXACT ? 1 : 2); ++s)
       for (uint32_t i = 0; i < 4096u; ++i)

@@ -33,7 +33,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
-#include <cstdio>
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
@@ -55,13 +54,7 @@ constexpr int kPairWarpsPerQuad = kPairEpiWarps / 4;
 constexpr int kPairBlocksPerWarp = (8 + kPairWarpsPerQuad - 1) / kPairWarpsPerQuad;   // 32-column blocks of a 256-column tile (narrower ones have fewer)
 constexpr int kPairMaxStages = 8;
 constexpr int kPairATileBytes = 128 * 128;        // 128 rows x one 128-byte K slab
-#ifdef KB200_TRACE
-constexpr int kPairSmemCeiling = 200 * 1024;      // the trace arrays take static shared memory
-#define PAIR_STAMP(role, idx) do { if (blockIdx.x <= 1 && (idx) < 128) trace[role][idx] = clock64(); } while (0)
-#else
 constexpr int kPairSmemCeiling = 224 * 1024;      // opt-in ceiling, the same for every launch of the kernel
-#define PAIR_STAMP(role, idx) do { } while (0)
-#endif
 // barrier indices
 constexpr int kBarFull = 0, kBarEmpty = kPairMaxStages, kBarTFull = 2 * kPairMaxStages, kBarTEmpty = kBarTFull + 2,
               kBarRes = kBarTEmpty + 2, kBarCount = kBarRes + kPairEpiWarps;
@@ -105,8 +98,6 @@ struct PairParams {
   int res_batched;       // that operand has one matrix per batch entry (else the same for all)
   int n_steps;
   PairStep steps[kMaxChain];
-#ifdef KB200_TRACE
-#endif
 };
 
 __device__ __forceinline__ int pair_div(int x, uint64_t magic) { return (int)(((uint64_t)(uint32_t)x * magic) >> 40); }
@@ -184,12 +175,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   __shared__ int abort_flag;
   __shared__ PairStep chain_steps[kMaxChain];     // looked up by a run-time index for every block
   __shared__ __align__(16) float columns[kPairEpiWarps][32];   // the bias of the block a warp is working on
-#ifdef KB200_TRACE
-  __shared__ long long trace[5][128];
-  __shared__ long long marks[8];
-  int tp = 0, tq = 0, te = 0;
-  if (blockIdx.x <= 1 && threadIdx.x == 0) marks[0] = clock64();
-#endif
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles = (raw + 1023u) & ~1023u;     // the 128-byte swizzle pattern repeats every 1024 bytes
@@ -235,13 +220,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_base_slot;
-#ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0) marks[1] = clock64();
-#endif
   cluster_wait();
-#ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0) marks[2] = clock64();
-#endif
   volatile int* abort_ptr = &abort_flag;
   // The MMA instruction names one TMEM address for both CTAs: the two allocations must agree.
   if (threadIdx.x == 0 && rank == 1) {
@@ -271,9 +250,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // Everything above may have overlapped the previous kernel's tail; from here on its output is read.
   pdl_wait();
   pdl_launch_dependents();
-#ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0) marks[3] = clock64();
-#endif
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -300,7 +276,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         }
         // the leader's barrier counts the bytes of both CTAs (the peer's may land first: the phase
         // cannot complete before this arrival)
-        PAIR_STAMP(0, tp);
         const bool b_here = ahead > 0;           // expected and requested above
         const uint32_t bar = full_leader0 + 8 * s;
         const uint32_t dst = tiles + (uint32_t)(s * stage_bytes);
@@ -312,10 +287,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         }
         __syncwarp();
         if (b_here) --ahead;
-        PAIR_STAMP(1, tp);
-#ifdef KB200_TRACE
-        ++tp;
-#endif
         if (++s == stages) { s = 0; wait_parity ^= 1; }
       }
     }
@@ -356,7 +327,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             ok = false;
             break;
           }
-          PAIR_STAMP(2, tq);
           // (the lane that issues is a predicate, not a branch: see umma_if)
           const uint32_t on = elect_one() ? 1u : 0u;
 #pragma unroll
@@ -374,10 +344,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             if (kb + 1 == num_kb) umma_pair_commit(tfull0 + 8 * acc);
           }
           __syncwarp();
-          PAIR_STAMP(3, tq);
-#ifdef KB200_TRACE
-          ++tq;
-#endif
           a16 += stage16;
           b16 += stage16;
           if (++s == stages) { s = 0; parity ^= 1; a16 = a_first; b16 = b_first; }
@@ -385,9 +351,9 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       }
     }
   } else if (warp >= kPairFirstEpiWarp && warp < kPairFirstEpiWarp + kPairEpiWarps) {
-    // ---------------- epilogue (warps 2..17) ----------------
-    // Four warps per TMEM lane quadrant (a warp may only touch lanes 32 * (warp % 4) ..+31); warp g of a
-    // quadrant takes the 32-column blocks g, g + 4 of the tile.  Sixteen warps, because the epilogue is
+    // ---------------- epilogue (warps 2..13) ----------------
+    // Three warps per TMEM lane quadrant (a warp may only touch lanes 32 * (warp % 4) ..+31); warp g of a
+    // quadrant takes the 32-column blocks g, g + 3, g + 6 of the tile.  Twelve warps and not eight, because the epilogue is
     // bound by instruction issue and by the latencies inside a pass (tensor-memory load, the wait for
     // the slot's last store, the proxy fence): with two warps per scheduler the schedulers issued in
     // 46 % of the cycles, a probe of independent multiply-adds in 90 %.
@@ -493,9 +459,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         if (!ok) break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#ifdef KB200_TRACE
-      if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
-#endif
 #pragma unroll 1
       for (int j = 0; j < kPairBlocksPerWarp; ++j) {
         const int c = 32 * (group + kPairWarpsPerQuad * j);
@@ -519,9 +482,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         float v[32];
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * p.bn + c), v);
         __syncwarp();
-#ifdef KB200_TRACE
-        if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
-#endif
         if constexpr (EPI == EPI_CHAIN) {
           run_chain(v, mine, n, batch);
         } else {
@@ -552,9 +512,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           }
         }
         __syncwarp();
-#ifdef KB200_TRACE
-        if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
-#endif
         stage_rows(slot0_ptr, slot0_ptr + (with32 || has_res ? 4096 : 0), v, lane, with16, with32);
         fence_async_smem();
         __syncwarp();
@@ -563,9 +520,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           if (with16) tma_store_3d(&tma_out16, slot0 + (with32 || has_res ? 4096u : 0u), n, m_first, batch);
           tma_store_commit();
         }
-#ifdef KB200_TRACE
-        if (warp == 4 && lane == 0) { PAIR_STAMP(4, te); ++te; }
-#endif
         if (dry) break;
       }
       if (dry) {
@@ -585,19 +539,6 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-#ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0) {
-    const long long t0 = marks[0];
-    printf("PAIR block %d: alloc+sync done %lld cluster barrier done %lld after pdl %lld exit %lld | tiles %d bn %d stages %d num_kb %d grid %d\n",
-           (int)blockIdx.x, marks[1] - t0, marks[2] - t0, marks[3] - t0, clock64() - t0, p.num_tiles, p.bn, p.stages, p.num_kb, (int)gridDim.x);
-    for (int i2 = 0; i2 < 64; ++i2)
-      printf("  b%d step %3d  prod_wait_done %7lld issued %7lld | mma_full %7lld committed %7lld\n", (int)blockIdx.x, i2, trace[0][i2] - t0,
-             trace[1][i2] - t0, trace[2][i2] - t0, trace[3][i2] - t0);
-    printf("  b%d epilogue warp 4 (tile ready; per block: loaded, slot free, computed, stored):", (int)blockIdx.x);
-    for (int i2 = 0; i2 < 80; ++i2) printf(" %lld", trace[4][i2] - t0);
-    printf("\n");
-  }
-#endif
   if (abort_flag && threadIdx.x == 0) {
     // copies may still be in flight towards this CTA's shared memory: give them a bounded time to land
     const long long t0 = clock64();

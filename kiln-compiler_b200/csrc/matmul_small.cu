@@ -253,6 +253,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
   } else if (warp == 0) {
+    // (GATHER: A is read by warps 2-9)
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);

@@ -29,7 +29,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
-#include <cstdio>
 #include <mutex>
 
 #include "device_math.cuh"
@@ -62,11 +61,7 @@ constexpr int kEpiBytes = kEpiWarps * kEpiWarpBytes;
 constexpr int kExactEpiWarpBytes = 4096;       // exact-FP32 mode: no bf16 block, and a transpose within 32 x 32 floats, for a third stage
 constexpr int kExactEpiBytes = kEpiWarps * kExactEpiWarpBytes;
 constexpr int kEpiSlotBytes = 4096 + 2048;   // one float block + one bf16 block of the rotating staging slots
-#ifdef KB200_TRACE
-constexpr int kMaxDynamicSmem = 200 * 1024;   // the trace arrays take static shared memory
-#else
 constexpr int kMaxDynamicSmem = 225 * 1024;   // opt-in ceiling, the same for every launch of the kernel
-#endif
 
 struct TcParams {
   // scalars the producer and MMA threads need first come first: the parameter block is read through
@@ -232,11 +227,6 @@ __device__ __forceinline__ void epilogue_store32(const TcParams& p, const float 
   }
 }
 
-#ifdef KB200_TRACE
-#define KB200_STAMP(role, idx) do { if (blockIdx.x == 0 && (idx) < 160) trace[role][idx] = clock64(); } while (0)
-#else
-#define KB200_STAMP(role, idx) do { } while (0)
-#endif
 
 // The chain on a block held a lane per ROW (v[j] = column n + j of this lane's row): every operand is
 // an immediate or one value per column, read as eight 128-bit loads from an address all lanes share.
@@ -286,17 +276,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   __shared__ __align__(8) uint64_t bars[3 * kMaxStages + 6];   // + two cluster hand-shake barriers (split K) + per-stage "operands split" barriers
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-#ifdef KB200_TRACE
-  __shared__ long long trace[6][160];
-  __shared__ long long marks[8];
-  int tp = 0, tm = 0, te = 0;
-  if (blockIdx.x <= 1 && threadIdx.x == 0) {
-    unsigned long long g;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
-    marks[0] = (long long)g;
-    marks[1] = clock64();
-  }
-#endif
 
   // 1024-byte aligned tile area (the 128-byte swizzle pattern repeats every 1024 bytes)
   const uint32_t raw = smem_u32(smem_raw);
@@ -358,9 +337,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   if (!(p.b_static && warp == kProducerBWarp)) pdl_wait();
   pdl_launch_dependents();
   volatile int* abort_ptr = &abort_flag;
-#ifdef KB200_TRACE
-  if (blockIdx.x <= 1 && threadIdx.x == 0) marks[2] = clock64();
-#endif
 
   // A whole warp walks each of the producer and issuer roles, one lane issuing (see elect_one); its waits end
   // for all lanes or none.
@@ -396,7 +372,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         const uint32_t full = full0 + 8 * s;
         ok = all_waited(mbar_wait(empty0 + 8 * s, wait_parity, abort_ptr), 1);
         if (!ok) break;
-        if (load_a) KB200_STAMP(0, tp);
         if (elect_one()) {
           mbar_expect_tx(full, tx_bytes);
           for (int part = 0; part < parts; ++part) {
@@ -418,10 +393,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           }
         }
         __syncwarp();
-        if (load_a) KB200_STAMP(1, tp);
-#ifdef KB200_TRACE
-        ++tp;
-#endif
         if (++s == stages) { s = 0; wait_parity ^= 1; }
       }
     }
@@ -483,7 +454,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           ok = all_waited(mbar_wait((split3 && p.presplit != 2 ? split0 : full0) + 8 * s, (uint32_t)round & 1u, abort_ptr), 2);
           if (!ok) break;
           if (split3) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (q == 0) KB200_STAMP(2, tm);
           const uint32_t tmem_d = tmem_t + (uint32_t)((rot + (split3 ? 1 : 0)) * bn);
           uint32_t accumulate = n_done >= nacc ? 1u : 0u;
           uint32_t accumulate_small = n_done > 0 ? 1u : 0u;
@@ -512,10 +482,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           }
           if (on) umma_commit(empty0 + 8 * s);   // frees the stage once these MMAs have read it
           __syncwarp();
-          if (q == 0) KB200_STAMP(3, tm);
-#ifdef KB200_TRACE
-          ++tm;
-#endif
           s += nq;
           if (s >= stages) { s -= stages; ++round; }
         }
@@ -623,9 +589,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           if (!got && lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 3); *abort_ptr = 1; }
           ok = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0 && !*abort_ptr;
           if (!ok) break;
-#ifdef KB200_TRACE
-          if (warp == 2 && lane == 0) { KB200_STAMP(4, te); ++te; }
-#endif
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         if (!dry && n0 + c >= p.mm.N) break;   // uniform across the warp
@@ -657,9 +620,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           if (lane == 0) tma_store_wait_read();
           __syncwarp();
         }
-#ifdef KB200_TRACE
-        if (warp == 2 && lane == 0 && !dry) { KB200_STAMP(4, te); ++te; }
-#endif
         if (!rowwise && direct) {
           // transpose through shared memory: lane = row  ->  lane = column
           // (conflict-free by a pitch of 33, or within 32 x 32 by exchanging columns)
@@ -670,9 +630,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           for (int r = 0; r < 32; ++r) v[r] = tbuf[SPLIT3 ? r * 32 + (lane ^ r) : r * 33 + lane];
           __syncwarp();
         }
-#ifdef KB200_TRACE
-        if (warp == 2 && lane == 0 && !dry) { KB200_STAMP(4, te); ++te; }
-#endif
         if (direct) {
           // The next block's operands are fetched where their latency hides and no fence waits on them:
           // the per-column value before this block's arithmetic, the matrix operand (whose registers
@@ -683,9 +640,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           if (rowwise) epilogue_compute_rows(p, v, batch, n0 + (dry ? half * 32 : c));
           else epilogue_compute32(p, v, pre_col, pre_mat, batch, m_first, n0 + (dry ? half * 32 : c) + lane);
           pre_col = next_col;
-#ifdef KB200_TRACE
-          if (warp == 2 && lane == 0 && !dry) { KB200_STAMP(4, te); ++te; }
-#endif
           if (more && !bulk) prefetch_mat(p, pre_mat, batch, m_first, n0 + c + 64 + lane);
           if (bulk) {
             // dense row-major 32 x 32 blocks in shared memory, then one bulk tensor store each: the
@@ -715,9 +669,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           } else {
             epilogue_store32(p, v, batch, m_first, n0 + c + lane);
           }
-#ifdef KB200_TRACE
-          if (warp == 2 && lane == 0 && !dry) { KB200_STAMP(4, te); ++te; }
-#endif
         } else {
           // split K: park this lane's row of the partial tile, eight 128-bit stores whose 16-byte slot
           // within the 32-column group is XORed with the row (no bank conflicts; the reduction undoes it)
@@ -731,9 +682,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tempty0 + 8 * acc) : "memory");
-#ifdef KB200_TRACE
-      if (warp == 2 && lane == 0) { KB200_STAMP(4, te); ++te; }
-#endif
     }
     if (bulk && lane == 0) tma_store_wait_read();   // shared memory must outlive the stores that read it
   }
@@ -760,9 +708,6 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
     if (threadIdx.x == 0) mbar_expect_tx(received, (uint32_t)(p.splits - 1) * band_bytes);
     cluster_wait();          // completes the arrive made before the main loop: every CTA's barriers are initialised
     __syncthreads();         // every warp of this CTA has parked its part (and fenced it to the async proxy)
-#ifdef KB200_TRACE
-    if (blockIdx.x <= 1 && threadIdx.x == 0) marks[3] = clock64();
-#endif
     if (lane == 0 && warp < p.splits && warp != (int)rank && !abort_flag) {
       // my partial of band `warp` -> slot `rank` of CTA `warp`'s receive area.  One copy per WARP: issued
       // by the lanes of one warp the seven copies went out one after the other, ~680 cycles each
@@ -773,17 +718,11 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
                    ::"r"(dst), "r"(tiles + (uint32_t)warp * band_bytes), "r"(band_bytes), "r"(bar)
                    : "memory");
     }
-#ifdef KB200_TRACE
-    if (blockIdx.x <= 1 && warp == kIssuerBWarp && lane == 0) marks[7] = clock64();
-#endif
     if (!mbar_wait(received, 0, abort_ptr) && threadIdx.x == 0 && !*abort_ptr) {
       atomicCAS(p.status, 0, (p.kernel_index << 8) | 5);
       *abort_ptr = 1;
     }
     cluster_arrive();        // what this CTA was to receive has landed (or it gave up): see the wait below
-#ifdef KB200_TRACE
-    if (blockIdx.x <= 1 && threadIdx.x == 0) marks[4] = clock64();
-#endif
     if (warp >= 2 && warp < 2 + kEpiWarps && !abort_flag) {
       // The band is small (128 / splits rows): all eight warps walk it as float4 items in row-major
       // order, so every load of a side operand and every store covers whole 128-byte lines, and an
@@ -857,42 +796,13 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         }
       }
     }
-#ifdef KB200_TRACE
-    if (blockIdx.x <= 1 && threadIdx.x == 64) marks[5] = clock64();
-#endif
     // every CTA of the cluster has received everything: so every push out of THIS shared memory has landed
     cluster_wait();
-#ifdef KB200_TRACE
-    if (blockIdx.x <= 1 && threadIdx.x == 0) marks[6] = clock64();
-#endif
   }
 
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-#ifdef KB200_TRACE
-  if (blockIdx.x == 1 && threadIdx.x == 0 && p.splits > 1)
-    printf("block1 split phase: entry globaltimer %lld setup_done %lld before cluster sync %lld arrived %lld after %lld reduce done %lld after 2nd sync %lld\n",
-           marks[0], marks[2] - marks[1], marks[3] - marks[1], marks[7] - marks[1], marks[4] - marks[1], marks[5] - marks[1], marks[6] - marks[1]);
-#endif
-#ifdef KB200_TRACE
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    unsigned long long g;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
-    printf("KERNEL block0 globaltimer start %lld end %lld (ns) dur %lld | cycles: entry 0 setup_done %lld first_prod %lld exit %lld | units/CTA~%d splits %d num_kb %d bn %d stages %d\n",
-           marks[0], (long long)g, (long long)g - marks[0], marks[2] - marks[1], trace[0][0] - marks[1], clock64() - marks[1],
-           (p.num_units + (int)gridDim.x - 1) / (int)gridDim.x, p.splits, p.num_kb, p.bn, p.stages);
-    if (p.splits > 1) printf("split phase: before cluster sync %lld after %lld warp2 reduce done %lld after 2nd sync %lld (cycles since entry)\n",
-           marks[3] - marks[1], marks[4] - marks[1], marks[5] - marks[1], marks[6] - marks[1]);
-    const long long t0 = trace[0][0];
-    for (int i = 0; i < 160 && i < p.num_kb * 3; ++i)
-      printf("slab %3d  prod_wait_done %7lld issued %7lld | mma_full %7lld committed %7lld\n", i, trace[0][i] - t0,
-             trace[1][i] - t0, trace[2][i] - t0, trace[3][i] - t0);
-    printf("epilogue stamps (tile ready, then per chunk: loaded, transposed, computed, stored; then accumulator released):");
-    for (int i = 0; i < 20; ++i) printf(" %lld", trace[4][i] - t0);
-    printf("\n");
-  }
-#endif
   if (abort_flag && threadIdx.x == 0) {
     // give copies that may still be in flight a bounded time to land before shared memory is released
     for (int s = 0; s < p.stages; ++s)
@@ -1311,7 +1221,6 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   bn = (bn / 64) * 64;                                    // the two epilogue warps of a quadrant take 32 columns each
   if (bn < 64) bn = 64;
   while (bn > 64 && bn / 2 >= k.N) bn /= 2;               // do not make the tile wider than the problem
-  (void)chunk_n;
   int stages = d.cfg[3] > 0 ? d.cfg[3] : kMaxStages;   // as deep as shared memory allows: the ring hides ~2000 cycles of TMA latency
   if (stages > kMaxStages) stages = kMaxStages;
   // Two K slabs per stage for narrow tiles: a stage costs the producers and the MMA thread a fixed

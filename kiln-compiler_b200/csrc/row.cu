@@ -6,7 +6,7 @@
 //                  the elementwise values recomputed from the inputs in every pass -- the scheme of
 //                  the reference's chunked rows (codegen.py:371-428), so memory use is constant for
 //                  any row length.
-//   row_layernorm  two-pass mean / variance LayerNorm with affine, one to 32 warps per row, the row
+//   row_layernorm  two-pass mean / variance LayerNorm with affine, one to 16 warps per row, the row
 //   row_softmax    held in registers (128-bit loads where width and alignment allow, shuffle
 //                  reductions): one read and one write of the tensor, HBM-bound.
 #include <cuda_bf16.h>
@@ -378,7 +378,8 @@ static void launch_rows(const RowFastParams& p, int access, int sm_count, bool p
 #define KB200_SHIFT_CASE(N, WIDE) launch_kernel(pdl, row_kernel<MODE, 4, N, WIDE, false, true, false>, dim3(grid), dim3(block), 0, s, p)
   if (n <= (vec && MODE == ROW_LAYERNORM ? 6 : 8)) {
     // a warp per row; few rows spread over more blocks.  (A LayerNorm of 8 float4 a lane, or either of 12,
-    // spills; four warps of a quarter each do not.)
+    // spills; four warps of a quarter each do not.  With a chain in front, a LayerNorm of four float4 and softmaxes of four or
+    // six, or of eight floats, spill 4 to 20 bytes.)
     const int warps = p.n_rows >= (int64_t)sm_count * 16 ? 8 : (p.n_rows >= (int64_t)sm_count * 4 ? 4 : 1);
     grid = (unsigned)((p.n_rows + warps - 1) / warps);
     block = warps * 32;
