@@ -387,21 +387,6 @@ def kernel_flops(kernel):
     return flops, byts
 
 
-# DRAM bytes (read + write) per launch, copied from `ncu --set full` captures of the same shapes as the
-# bench (no scaling): the eight-sequence graph's kernels from
-# profiles/gpt2_block_b8_t1024_bf16_launches_and_top_kernels.md ("bf16:b8:" keys; outputs that the next
-# kernel reads stay in the 126 MB L2 and are not written back inside the launch).
-NCU_DRAM_BYTES = {
-    "bf16:b8:k0_row": 25245440,
-    "bf16:b8:k1_matmul": 17290496,
-    "bf16:b8:k2_ew0": 41667840,
-    "bf16:b8:k9_matmul": 39930112,
-    "bf16:b8:k10_row": 25245952,
-    "bf16:b8:k11_matmul": 21331968,
-    "bf16:b8:k13_matmul": 85108992,
-}
-
-
 def roofline_of(built, precision, iters=10):
     """Per-launch CUDA-event times of every kernel of the module (each launch alone on the GPU, `iters`
     launches per CUDA graph); roofline of the one with the largest share."""
@@ -430,7 +415,7 @@ def roofline_of(built, precision, iters=10):
         if exe.impls[j] == "mm_tcgen05" and t > 0:
             matmuls[n] = round(f / (t * 1e-3) / 1e12 / peak, 3)
     return {"bound": bound, "achieved": achieved, "peak": peak, "unit": unit, "frac": achieved / peak,
-            "traffic": NCU_DRAM_BYTES.get(f"{precision}:b{GROUP}:{name}"),
+            "traffic": None,      # (the captured DRAM bytes were of kernels that have changed)
             "traffic_unit": "bytes per launch (ncu dram read + write)", "kernel": f"{name} ({exe.impls[i]})", "ms_per_launch": ms,
             "share": ms / total, "peak_source": peak_note, "matmul_frac_of_peak": matmuls,
             "per_kernel_ms": {n: round(t, 5) for n, t in times if t > 0.0}}

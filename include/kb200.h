@@ -72,8 +72,8 @@ typedef enum kb200_kclass {
  * FP32 corresponds to input_precision="ieee", TF32 to "tf32"
  * (codegen.py:515-516); BF16 is a backend-internal mode with no IR dtype.
  * FP32 on the tensor cores is three TF32 products of split operands: within 1e-5 of exact for
- * finite operands, but NOT IEEE for non-finite ones (an infinite operand element yields NaN, see
- * cfg[6] bit 1024 below for the CUDA-core kernel that is). */
+ * finite operands, but in the kernels for many tiles NOT IEEE for non-finite ones (an infinite operand
+ * element yields NaN, see cfg[6] bit 1024 below for the CUDA-core kernel that is). */
 typedef enum kb200_precision {
   KB200_PREC_FP32 = 0,
   KB200_PREC_TF32 = 1,
