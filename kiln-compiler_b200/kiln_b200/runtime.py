@@ -144,11 +144,12 @@ def _ptr_array(tensors):
 
 # A call of a plan of up to this many launches enqueues them on the caller's own tensors, with no copy in,
 # no graph and no clone out: each launch costs the host about 2 us, where a graph costs ~5 us to begin and the two
-# copies their own launches.  Kernels shorter than a launch decide the limit.  Calls in a row of n
+# copies their own launches.  Kernels shorter than a launch decide the limit, which
+# is kept well below where a graph is quicker for them.  Calls in a row of n
 # LayerNorms of 64 x 256, graph against direct: 8: 21.6 / 19.0 us, 12: 27.8 / 26.7, 16: 31.7 / 36.4, 24: 44.2 / 52.8; of
 # 2048 x 768, 12: 45.1 / 38.6, 24: 78.1 / 76.9, 48: 146.5 / 154.8; of n transformer blocks of 128 tokens in TF32, 14
 # launches: 78.5 / 71.7, 28: 158.0 / 152.2.
-DIRECT_LAUNCHES = 12
+DIRECT_LAUNCHES = 10
 
 
 def _usable(t, device):
