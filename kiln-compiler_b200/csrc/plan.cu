@@ -1148,9 +1148,14 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   // phase 4: tensor maps, packed weights, split-K workspaces.  What FP32 and TF32 matmuls add to make operands quicker to read
   // (a weight along K, its tails, aligned rows, the tails of A) takes a quarter of what is free in all, beside
   // a call's outputs; each on its own was allowed that much, and a plan of many Linears left nothing for its caller.
-  if (rc == KB200_OK) {
-    for (PlanKernel& k : plan.kernels)
-      if (k.desc.kclass == KB200_K_MATMUL) destroy_matmul(k);
+  bool copies = false;
+  for (PlanKernel& k : plan.kernels)
+    if (k.desc.kclass == KB200_K_MATMUL) {
+      destroy_matmul(k);
+      copies = copies || (k.impl == IMPL_MM_TC && k.desc.precision != KB200_PREC_BF16);
+    }
+  plan.copy_budget = 0;
+  if (rc == KB200_OK && copies) {          // (asking costs 0.1 ms and more)
     size_t free_bytes = 0, total_bytes = 0;
     const cudaError_t e = cudaMemGetInfo(&free_bytes, &total_bytes);
     if (e != cudaSuccess) rc = cuda_fail(e, "cudaMemGetInfo");

@@ -44,15 +44,18 @@ def test_all_copies_of_a_plan_share_a_quarter_of_the_free_memory(precision):
     _cabi.check(exe._lib.kb200_plan_set_option(exe._plan, _cabi.OPT_WEIGHT_COPIES, 0))
     exe._bind()
     hold = torch.empty(torch.cuda.mem_get_info()[0] - (512 << 20), dtype=torch.uint8, device="cuda")
-    _cabi.check(exe._lib.kb200_plan_set_option(exe._plan, _cabi.OPT_WEIGHT_COPIES, 1))
-    free = torch.cuda.mem_get_info()[0]
+    try:
+        _cabi.check(exe._lib.kb200_plan_set_option(exe._plan, _cabi.OPT_WEIGHT_COPIES, 1))
+        free = torch.cuda.mem_get_info()[0]
+        exe._bind()
+        taken = free - torch.cuda.mem_get_info()[0]
+        (got,) = exe(x)
+        torch.cuda.synchronize()
+        exe.status()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
     assert free < 600 << 20
-    exe._bind()
-    taken = free - torch.cuda.mem_get_info()[0]
-    (got,) = exe(x)
-    torch.cuda.synchronize()
-    exe.status()
-    del hold
     assert 0 < taken <= free // 4 + (16 << 20)             # (allocations are rounded up to 2 MB)
     error = float((got - want).norm() / want.norm())
     assert error <= {"fp32": 1e-5, "tf32": 2e-3}[precision]      # the bounds of the precisions, as in the other tests
