@@ -149,7 +149,7 @@ def _ptr_array(tensors):
 # LayerNorms of 64 x 256, graph against direct: 8: 21.6 / 19.0 us, 12: 27.8 / 26.7, 16: 31.7 / 36.4, 24: 44.2 / 52.8; of
 # 2048 x 768, 12: 45.1 / 38.6, 24: 78.1 / 76.9, 48: 146.5 / 154.8; of n transformer blocks of 128 tokens in TF32, 14
 # launches: 78.5 / 71.7, 28: 158.0 / 152.2.
-DIRECT_LAUNCHES = 10
+DIRECT_LAUNCHES = 9
 
 
 def _usable(t, device):
