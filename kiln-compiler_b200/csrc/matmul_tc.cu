@@ -1112,7 +1112,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   cudaError_t made = cudaSuccess;
   // FP32 operands of fewer than 32 rows, or that a tensor map cannot describe: the small kernel, which adds up in float32 as
   // often as the CUDA cores' error asks for, or those.  (This file's kernel sums up to 1000 of K in the tensor
-  // core: 1000 x 1001 x 3071 of positive operands 7.1e-6 from exact, CUDA cores 8.5e-7, the small kernel 6.1e-7.)
+  // core: 1000 x 1001 x 3071 of positive operands 7.1e-6 from exact, CUDA cores 8.5e-7, the small kernel 4.5e-7.)
   const bool plain = k.M >= 32 && k.N % 4 == 0 && k.K % 4 == 0 && rows_describable(A, A.stride[1], k.batch) && rows_describable(B, b_src_row, k.batch);
   const bool close_only = d.precision == KB200_PREC_FP32 && !plain;
   // Few tiles: the kernel written for latency, where the other kernels cover the shape too by the estimates of both.
