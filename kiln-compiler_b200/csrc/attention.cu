@@ -8,10 +8,10 @@
 // chain and the mask is the causal one, a fused kernel replaces the five launches: it reads Q, K and
 // V as strided views of the QKV projection's output and writes the merged-heads buffer, the only
 // value of the chain that is live afterwards.  The plan itself (kernel list, arena offsets) is
-// untouched; the score buffers are simply never written.  Two kernels: `attention_kernel` on the tensor
-// cores -- for the TF32 and BF16 matmul modes (described next) and, with its EXACT parameter, for FP32
-// mode (the same structure with three TF32 MMAs per product) -- and `attention_fp32_kernel` for short
-// sequences in FP32 mode (CUDA cores).
+// untouched; the score buffers are simply never written.  Three kernels: `attention_kernel` on the tensor
+// cores -- for TF32 operands (described next) and, with its EXACT parameter, for FP32
+// mode (the same structure with three TF32 MMAs per product) --, `attention_fp32_kernel` for short
+// sequences in FP32 mode (CUDA cores), and the one for bf16 operands in attention_bf16.cu.
 //
 // Persistent CTAs (one per SM) walk the (sequence, head, 128-query tile) work items, heaviest first, in
 // steps of the grid size: barrier set-up, the TMEM allocation and the latency of an item's first
@@ -36,6 +36,7 @@
 #include <utility>
 #include <vector>
 
+#include "attention.h"
 #include "device_math.cuh"
 #include "kb200_internal.h"
 #include "tc_common.cuh"
@@ -47,34 +48,16 @@ namespace {
 
 using namespace tc;
 
-constexpr int kRows = 128;                   // queries per CTA and keys per tile
-constexpr int kHeadDim = 64;
+constexpr int kRows = kAttnRows;
+constexpr int kHeadDim = kAttnHeadDim;
 constexpr int kSlab = kRows * 128;           // one [128 rows x 128 bytes] swizzled slab
 constexpr int kAttnThreads = 64 + 256;
 constexpr int kExchangeBytes = 2 * (2 * 2 * kRows * 4);   // the pairs' maxima (two tile parities) and row sums (two item parities)
 constexpr int kStageBytes = 4096 + 2048;      // a warp's output rows: 32 x 32 float32 and their bf16 copy
-// Q + 2 x K + 2 x V tiles (two 16 KB slabs each in float32, one in bf16), the two merge buffers, alignment slack
-constexpr int attn_smem(bool bf16) { return 5 * (bf16 ? 1 : 2) * kSlab + kExchangeBytes + 8 * kStageBytes + 1024; }
+// Q + 2 x K + 2 x V tiles (two 16 KB slabs each), the two merge buffers, alignment slack
+constexpr int kSmemBytes = 5 * 2 * kSlab + kExchangeBytes + 8 * kStageBytes + 1024;
 // FP32 mode on the tensor cores: Q, K, V once each with their tails (4 slabs per operand), the exchange area, slack
 constexpr int kExactSmemBytes = 3 * 4 * kSlab + kExchangeBytes + 1024;
-
-struct AttnParams {
-  int T, H, q_tiles;
-  int B;                     // sequences in the graph (1 for the two-dimensional block); rows of Q, K, V and of the output are b * T + t
-  float scale_log2;          // softmax scale times log2(e): exponentials are taken in base 2
-  float* out;                // [T, H * 64] merged heads
-  int64_t out_row_stride;
-  __nv_bfloat16* out16;      // optional bf16 copy of the merged heads, row stride H * 64, or null
-  int64_t out16_row_stride;
-  uint32_t idesc_qk, idesc_pv;
-  int kernel_index;
-  int* status;
-  int split_from;            // query tiles from this one on are shared by two CTAs (q_tiles: none)
-  float* partial;            // [split tile][2 halves][128 x 64 unnormalised output | 128 maxima | 128 sums]
-  int* arrivals;             // [split tile][4 lane quadrants], zero between launches
-  const unsigned short* order;   // with split tiles: (query tile << 1 | half) of the q_tiles + split tiles entries, heaviest first
-};
-constexpr int kPartialFloats = kRows * kHeadDim + 2 * kRows;
 
 constexpr int kFTile = 64;                 // queries per CTA and keys per tile
 constexpr int kFPitch = 68;                // floats per shared-memory row of Q, K and P (16-byte aligned, rows 4 banks apart)
@@ -112,6 +95,7 @@ struct AttnState {
   int64_t row_stride = 0;
   AttnParams params;
   dim3 grid;
+  bool alone = false;              // kernel for bf16 operands: one CTA to an SM
   // When the planner put the merged-heads buffer over the (by then dead) QKV buffer, the fused
   // kernel cannot write it while other CTAs still read Q, K and V: it writes here, a copy follows.
   const DevOperand* y = nullptr;   // the head-merge kernel's output operand (the chain's only live result)
@@ -152,14 +136,6 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const float4* __restrict
   pdl_wait();                 // the producer of this kernel's inputs has completed
   pdl_launch_dependents();    // the next kernel may begin its start-up
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) dst[i] = src[i];
-}
-
-// 2^x for x <= 0 through the bare special-function instruction (exp2f adds a range fix-up for
-// denormal results, which a probability does not need; the softmax is bound by this pipe).
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // Scores of one 32-column block -> probabilities, in place; returns their sum.  `first_col` is the
@@ -424,17 +400,16 @@ __global__ void __launch_bounds__(kFThreads, 2) attention_fp32_kernel(const __gr
 // run under the softmax, which is the long pole), the tails of P have one buffer (a thread folds the
 // previous tile's O_part -- whose completion says its P V has read them -- before it writes the
 // next), and the output rows leave by ordinary stores (no staging slots).
-template <bool BF16, bool SPLIT, bool EXACT>
+template <bool SPLIT, bool EXACT>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
                  const __grid_constant__ CUtensorMap map_out16, const __grid_constant__ CUtensorMap map_qt,
                  const __grid_constant__ CUtensorMap map_kt, const __grid_constant__ CUtensorMap map_vt,
                  const __grid_constant__ AttnParams p) {
-  static_assert(!(BF16 && EXACT), "the FP32 mode has float32 operands");
-  // a [128 rows x 64 dims] operand tile is two 128-byte-wide slabs in float32, one in bf16;
+  // a [128 rows x 64 dims] operand tile is two 128-byte-wide slabs;
   // EXACT: an operand buffer holds the tile and, behind it, its tails
-  constexpr int kTileSlabs = BF16 ? 1 : 2;
+  constexpr int kTileSlabs = 2;
   constexpr int kTileBytes = kTileSlabs * kSlab;
   constexpr int kOpBytes = 2 * kTileBytes;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -455,43 +430,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const uint32_t sfull0 = smem_u32(&bars[9]), pfull0 = smem_u32(&bars[11]), ofull0 = smem_u32(&bars[15]);
   const uint32_t q_empty = smem_u32(&bars[19]);
 
-  // work item w -> (head, sequence, query tile): heaviest (longest causal prefix) tiles first, of every sequence
-  // Query tiles from p.split_from on (the longest causal prefixes; none when split_from = q_tiles) are
-  // TWO items, one per half of their key tiles: each leaves its unnormalised rows and softmax state in
-  // a workspace, and the one that arrives second (a counter per tile and lane quadrant) merges them.
   // (SPLIT is a template parameter so that the kernel without split tiles keeps its code: with the
   // choice made at run time the eight-sequence attention took 44.4 instead of 43.4 us.)
-  const int n_split = SPLIT ? p.q_tiles - p.split_from : 0;
-  const int n_items = p.B * p.H * (p.q_tiles + n_split);
-  // This CTA's r-th item (-1: none).  Rounds alternate direction over the CTAs, so that the CTA with the
-  // heaviest item of one round takes the lightest of the next (24 key tiles at most per CTA instead of
-  // 27 for 8 x 12 x 8 items on 148 CTAs).
-  auto nth_item = [&](int r) {
-    const int w = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
-    return w < n_items ? w : -1;
-  };
-  struct Item { int h, seq, q0, n_kv, qt, j0, half, slot; bool split; };
-  auto item_of = [&](int w) {
-    Item it;
-    it.h = w % p.H;
-    it.seq = (w / p.H) % p.B;
-    const int v = w / (p.H * p.B);
-    if (!SPLIT) {                                      // heaviest (longest causal prefix) first
-      it.qt = p.q_tiles - 1 - v;
-      it.half = 0;
-    } else {                                           // whole tiles and halves in descending order of their key tiles (host table)
-      const unsigned e = __ldg(p.order + v);
-      it.qt = (int)(e >> 1);
-      it.half = (int)(e & 1);
-    }
-    it.split = SPLIT && it.qt >= p.split_from;
-    it.q0 = it.qt * kRows;
-    const int n = it.qt + 1;                           // causal: key tiles 0..qt
-    it.j0 = it.split && it.half ? n >> 1 : 0;          // this item's key tiles: j0 .. j0 + n_kv - 1
-    it.n_kv = (it.split && !it.half ? n >> 1 : n) - it.j0;
-    it.slot = it.split ? (it.seq * p.H + it.h) * n_split + (it.qt - p.split_from) : 0;
-    return it;
-  };
+  const int n_items = p.B * p.H * (p.q_tiles + (SPLIT ? p.q_tiles - p.split_from : 0));
 
   if (threadIdx.x == 32) {
     prefetch_tensormap(&map_q);
@@ -558,7 +499,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (elect_one()) {
         mbar_expect_tx(bar, EXACT ? kOpBytes : kTileBytes);
         tma_load_4d(dst, map, bar, 0, token, h, seq);
-        if (!BF16) tma_load_4d(dst + kSlab, map, bar, 32, token, h, seq);
+        tma_load_4d(dst + kSlab, map, bar, 32, token, h, seq);
         if constexpr (EXACT) {
           tma_load_4d(dst + kTileBytes, tails, bar, 0, token, h, seq);
           tma_load_4d(dst + kTileBytes + kSlab, tails, bar, 32, token, h, seq);
@@ -567,9 +508,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       __syncwarp();
     };
     for (int ii = 0; ok; ++ii) {
-      const int w = nth_item(ii);
+      const int w = attn_nth_item(ii, n_items);
       if (w < 0) break;
-      const Item it = item_of(w);
+      const AttnItem it = attn_item<SPLIT>(p, w);
       // the Q tile is free once every Q K^T of the previous item has been executed
       if (!all_waited(mbar_wait(q_empty, (ii & 1) ^ 1, abort_ptr), 0x13)) break;
       load(q_smem, &map_q, &map_qt, q_full, it.q0, it.h, it.seq);
@@ -596,7 +537,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t kb = EXACT ? k_smem : k_smem + s * kTileBytes;
       const uint32_t on = elect_one() ? 1u : 0u;
-      // 32 bytes of the head dimension per instruction: 8 float32 (TF32) or 16 bf16.
+      // 32 bytes of the head dimension per instruction: 8 float32.
       // EXACT: heads x heads, heads x tails, tails x heads
 #pragma unroll
       for (int pass = 0; pass < (EXACT ? 3 : 1); ++pass) {
@@ -605,7 +546,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         for (int kd = 0; kd < kTileSlabs * 4; ++kd) {
           const uint32_t off = (uint32_t)(kd >> 2) * kSlab + (uint32_t)(kd & 3) * 32;
           umma_if(on, tmem_base + (uint32_t)s * 128, make_desc(qa + off, 16, 1024), make_desc(ka + off, 16, 1024), p.idesc_qk,
-                  (pass | kd) != 0 ? 1u : 0u, BF16);
+                  (pass | kd) != 0 ? 1u : 0u, false);
         }
       }
       if (on) {
@@ -633,24 +574,15 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         ok = all_waited(mbar_wait(pfull0 + 8 * (g * 2 + s), ph, abort_ptr), 0x24);
         if (!ok) return;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if constexpr (BF16) {
-          // P: two bf16 per TMEM column, 16 keys = 8 columns per instruction; V: [keys x 64 dims] bf16,
-          // one 128-byte swizzled row per key, 16 rows per instruction
+        // EXACT: P x V, P x tails of V, tails of P x V
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ts_if(on, o_addr, tmem_base + (uint32_t)s * 128 + (uint32_t)(g * 64 + kk * 8),
-                       make_desc(vb + (uint32_t)(g * 4 + kk) * 2048, kSlab, 1024, 2), p.idesc_pv, (g | kk) != 0 ? 1u : 0u, true);
-        } else {
-          // EXACT: P x V, P x tails of V, tails of P x V
+        for (int pass = 0; pass < (EXACT ? 3 : 1); ++pass) {
+          const uint32_t pa = pass == 2 ? tmem_pt : tmem_base + (uint32_t)s * 128;
+          const uint32_t va = vb + (pass == 1 ? kTileBytes : 0);
 #pragma unroll
-          for (int pass = 0; pass < (EXACT ? 3 : 1); ++pass) {
-            const uint32_t pa = pass == 2 ? tmem_pt : tmem_base + (uint32_t)s * 128;
-            const uint32_t va = vb + (pass == 1 ? kTileBytes : 0);
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              umma_ts_if(on, o_addr, pa + (uint32_t)(g * 64 + kk * 8), make_desc(va + (uint32_t)(g * 8 + kk) * 1024, kSlab, 512, 1),
-                         p.idesc_pv, (g | kk | pass) != 0 ? 1u : 0u, false);
-          }
+          for (int kk = 0; kk < 8; ++kk)
+            umma_ts_if(on, o_addr, pa + (uint32_t)(g * 64 + kk * 8), make_desc(va + (uint32_t)(g * 8 + kk) * 1024, kSlab, 512, 1),
+                       p.idesc_pv, (g | kk | pass) != 0 ? 1u : 0u, false);
         }
       }
       if (on) {
@@ -661,9 +593,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     };
     int t = 0;
     for (int ii = 0; ok; ++ii) {
-      const int w = nth_item(ii);
+      const int w = attn_nth_item(ii, n_items);
       if (w < 0) break;
-      const int n_kv = item_of(w).n_kv;
+      const int n_kv = attn_item<SPLIT>(p, w).n_kv;
       // (The next item's first scores are NOT issued ahead of this item's last P V: the softmax warps
       // wait for that P V to finish the item, and have the merge and the stores to do before they
       // need the next scores.)
@@ -709,9 +641,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     bool ok = true;
     int t0 = 0;                                      // tiles of the items before this one
     for (int ii = 0; ok; ++ii) {
-      const int w = nth_item(ii);
+      const int w = attn_nth_item(ii, n_items);
       if (w < 0) break;
-      const Item it = item_of(w);
+      const AttnItem it = attn_item<SPLIT>(p, w);
       const int n_kv = it.n_kv;
       float o[32];
 #pragma unroll
@@ -782,18 +714,6 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
           for (int i = 0; i < 32; ++i) tb[i] = vb[i] - __uint_as_float(__float_as_uint(vb[i]) & 0xFFFFE000u);
           tmem_st32(pt_addr + 32, tb);
-        } else if (BF16) {
-          // P rounded to bf16, two keys per 32-bit column: the thread's 64 keys take the first 32 columns of
-          // its own 64-column share of the S buffer
-          float packed[32];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 lo = __floats2bfloat162_rn(va[2 * i], va[2 * i + 1]);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(vb[2 * i], vb[2 * i + 1]);
-            packed[i] = __uint_as_float(*reinterpret_cast<uint32_t*>(&lo));
-            packed[16 + i] = __uint_as_float(*reinterpret_cast<uint32_t*>(&hi));
-          }
-          tmem_st32(s_addr, packed);
         } else {
           tmem_st32(s_addr, va);
           tmem_st32(s_addr + 32, vb);
@@ -820,8 +740,8 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       bool writes = ok;
       float l_tot = ok ? l_run + xsum[((ii & 1) * 2 + (group ^ 1)) * kRows + row] : 1.0f;
       if (SPLIT && ok && it.split) {
-        float* const mine = p.partial + ((size_t)it.slot * 2 + it.half) * kPartialFloats;
-        const float* const other = p.partial + ((size_t)it.slot * 2 + (it.half ^ 1)) * kPartialFloats;
+        float* const mine = p.partial + ((size_t)it.slot * 2 + it.half) * kAttnPartialFloats;
+        const float* const other = p.partial + ((size_t)it.slot * 2 + (it.half ^ 1)) * kAttnPartialFloats;
         float4* const mine4 = reinterpret_cast<float4*>(mine + row * kHeadDim + group * 32);
 #pragma unroll
         for (int i = 0; i < 8; ++i) __stcg(mine4 + i, make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]));
@@ -1064,9 +984,9 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
                     encode_map_heads(&st->map_qt, false, st->tails + (c.q - lo), hd, T, H, B, rs, 32, kRows, false) &&
                     encode_map_heads(&st->map_kt, false, st->tails + (c.k - lo), hd, T, H, B, rs, 32, kRows, false) &&
                     encode_map_heads(&st->map_vt, false, st->tails + (c.v - lo), hd, T, H, B, rs, 32, kRows, true) &&
-                    cudaFuncSetAttribute(attention_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    cudaFuncSetAttribute(attention_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kExactSmemBytes) == cudaSuccess &&
-                    cudaFuncSetAttribute(attention_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                    cudaFuncSetAttribute(attention_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kExactSmemBytes) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
@@ -1075,11 +995,10 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
       return false;
     }
   }
-  if (cudaFuncSetAttribute(attention_kernel<false, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(false)) != cudaSuccess ||
-      cudaFuncSetAttribute(attention_kernel<false, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(false)) != cudaSuccess ||
+  if (cudaFuncSetAttribute(attention_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
+      cudaFuncSetAttribute(attention_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
       cudaFuncSetAttribute(attention_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemBytes) != cudaSuccess ||
-      cudaFuncSetAttribute(attention_kernel<true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(true)) != cudaSuccess ||
-      cudaFuncSetAttribute(attention_kernel<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(true)) != cudaSuccess) {
+      !attention_bf16_prepare()) {
     cudaGetLastError();
     delete st;
     return false;
@@ -1098,6 +1017,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   p.scale_log2 = c.scale * 1.4426950408889634f;
   p.out = c.y->ptr;
   p.out_row_stride = H * hd;
+  p.out32 = true;
   p.out16 = nullptr;
   p.out16_row_stride = H * hd;
   st->y = c.y;
@@ -1128,37 +1048,30 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   st->map_out16 = st->map_out;
   // When the items do not fill the persistent CTAs, the launch takes as long as its longest item: the
   // upper half of the query tiles is then shared by two CTAs each (one sequence of 1024 tokens: 96
-  // items of 1..8 key tiles become 144 of at most 4).  A split item costs about three BF16 key tiles
+  // items of 1..8 key tiles become 144 of at most 4).  A split item costs about three key tiles
   // (partial rows out, fence, counter, the other half's rows in), so it pays only for long items in an
-  // underfilled launch -- measured, one sequence: BF16 1024 tokens 14.4 -> 13.4 us but 512 tokens 9.6
-  // -> 10.8 and 2048 tokens (192 items, two rounds) 24.4 -> 29.4; FP32 mode, whose tiles take three
-  // times the MMAs, 1024 tokens 37.0 -> 28.1 and 2048 tokens 67.8 -> 65.4.
+  // underfilled launch -- measured, one sequence, FP32 mode, whose tiles take three
+  // times the MMAs: 1024 tokens 37.0 -> 28.1 us and 2048 tokens 67.8 -> 65.4.  The kernel for bf16 operands goes by an
+  // estimate of both.
   p.split_from = p.q_tiles;
   p.partial = nullptr;
   p.arrivals = nullptr;
   p.order = nullptr;
-  if (!(c.exact && !st->exact_tc) && p.q_tiles >= 8 && B * H * p.q_tiles <= (c.exact ? 2 : 1) * (int64_t)plan.sm_count &&
-      plan.concurrency == 1 &&                       // other plans in flight fill the SMs this one leaves idle
-      plan.attention_split) {
+  const bool may_split = plan.concurrency == 1 &&          // (other plans in flight fill the SMs this one leaves idle)
+                         plan.attention_split;
+  if (c.bf16 && !aliased) {      // (the kernel for bf16 operands, unless nobody writes them)
+    const AttnSchedule schedule = attention_bf16_schedule(B * H, p.q_tiles, plan.sm_count, may_split);
+    p.split_from = schedule.split_from;
+    st->alone = schedule.alone;
+  } else if (!(c.exact && !st->exact_tc) && p.q_tiles >= 8 && B * H * p.q_tiles <= (c.exact ? 2 : 1) * (int64_t)plan.sm_count && may_split) {
     p.split_from = p.q_tiles / 2;
+  }
+  if (p.split_from < p.q_tiles) {
     const int64_t split_tiles = B * H * (p.q_tiles - p.split_from);
-    const size_t partial_bytes = (size_t)split_tiles * 2 * kPartialFloats * sizeof(float);
+    const size_t partial_bytes = (size_t)split_tiles * 2 * kAttnPartialFloats * sizeof(float);
     const size_t counter_bytes = (size_t)split_tiles * 4 * sizeof(int);
-    // whole tiles and halves by descending number of key tiles, so that the alternating rounds of the
-    // persistent CTAs pair a long item with a short one
-    std::vector<std::pair<int, unsigned short>> entries;
-    for (int qt = 0; qt < p.q_tiles; ++qt) {
-      const int n = qt + 1;
-      if (qt >= p.split_from) {
-        entries.push_back({n >> 1, (unsigned short)(qt << 1)});
-        entries.push_back({n - (n >> 1), (unsigned short)(qt << 1 | 1)});
-      } else {
-        entries.push_back({n, (unsigned short)(qt << 1)});
-      }
-    }
-    std::stable_sort(entries.begin(), entries.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-    std::vector<unsigned short> order;
-    for (const auto& e : entries) order.push_back(e.second);
+    const std::vector<int> entries = attention_item_order(p.q_tiles, p.split_from);
+    const std::vector<unsigned short> order(entries.begin(), entries.end());
     const size_t order_bytes = (order.size() * sizeof(unsigned short) + 15) & ~size_t(15);
     if (cudaMalloc(&st->split_scratch, partial_bytes + counter_bytes + order_bytes) != cudaSuccess ||
         cudaMemset(static_cast<uint8_t*>(st->split_scratch) + partial_bytes, 0, counter_bytes) != cudaSuccess ||
@@ -1433,27 +1346,22 @@ int attention_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
                              reinterpret_cast<const float4*>(st->span_lo), reinterpret_cast<float4*>(st->tails), st->span_n4));
     // (the store maps are not used by this instantiation)
     if (split)
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, true, true>, st->grid, dim3(kAttnThreads), kExactSmemBytes, s, st->map_q,
+      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<true, true>, st->grid, dim3(kAttnThreads), kExactSmemBytes, s, st->map_q,
                                st->map_k, st->map_v, st->map_out, st->map_out16, st->map_qt, st->map_kt, st->map_vt, st->params));
     else
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, false, true>, st->grid, dim3(kAttnThreads), kExactSmemBytes, s, st->map_q,
+      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, true>, st->grid, dim3(kAttnThreads), kExactSmemBytes, s, st->map_q,
                                st->map_k, st->map_v, st->map_out, st->map_out16, st->map_qt, st->map_kt, st->map_vt, st->params));
   } else if (st->exact) {
     KB200_CUDA(launch_kernel(plan.pdl, attention_fp32_kernel, st->grid, dim3(kFThreads), kFSmemBytes, s, st->f32));
   } else if (st->bf16) {
+    KB200_CUDA(attention_bf16_launch(plan.pdl, st->grid, st->alone, s, st->map_q, st->map_k, st->map_v, st->map_out, st->map_out16, st->params));
+  } else {
     // (the maps of the tails are not used by these instantiations: any valid map will do)
     if (split)
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<true, true, false>, st->grid, dim3(kAttnThreads), attn_smem(true), s, st->map_q,
+      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<true, false>, st->grid, dim3(kAttnThreads), kSmemBytes, s, st->map_q,
                                st->map_k, st->map_v, st->map_out, st->map_out16, st->map_q, st->map_k, st->map_v, st->params));
     else
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<true, false, false>, st->grid, dim3(kAttnThreads), attn_smem(true), s, st->map_q,
-                               st->map_k, st->map_v, st->map_out, st->map_out16, st->map_q, st->map_k, st->map_v, st->params));
-  } else {
-    if (split)
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, true, false>, st->grid, dim3(kAttnThreads), attn_smem(false), s, st->map_q,
-                               st->map_k, st->map_v, st->map_out, st->map_out16, st->map_q, st->map_k, st->map_v, st->params));
-    else
-      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, false, false>, st->grid, dim3(kAttnThreads), attn_smem(false), s, st->map_q,
+      KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<false, false>, st->grid, dim3(kAttnThreads), kSmemBytes, s, st->map_q,
                                st->map_k, st->map_v, st->map_out, st->map_out16, st->map_q, st->map_k, st->map_v, st->params));
   }
   if (st->staged_out && st->final_out) {
@@ -1481,7 +1389,14 @@ bool attention_operand_span(const PlanKernel& k, const float** lo, const float**
 
 // BF16 mode: the producer of Q, K and V also writes them as bf16 into the mirror at `mirror_base +
 // (ptr - arena_base)`; read them from there (half the bytes, twice the tensor rate, P rounded to bf16).
-bool attention_use_mirror(PlanKernel& k, const float* arena_base, const void* mirror_base) {
+// The bf16 copy of the merged heads leaves through a store map of its own; without one it is not written.  The kernel for bf16
+// operands stores whole heads (rows of 128 bytes), the other one halves of them.
+static bool encode_out16(AttnState* st, void* out16) {
+  return encode_map_store(&st->map_out16, true, out16, (int64_t)st->params.H * kHeadDim, st->params.T, st->params.B, st->params.out16_row_stride,
+                          st->params.T * st->params.out16_row_stride, st->bf16);
+}
+
+bool attention_use_mirror(const Plan& plan, PlanKernel& k, const float* arena_base, const void* mirror_base) {
   AttnState* st = static_cast<AttnState*>(k.attn);
   if (!st) return false;
   // When the planner put the output over the QKV buffer, the output's mirror lies over the operands'
@@ -1502,6 +1417,10 @@ bool attention_use_mirror(PlanKernel& k, const float* arena_base, const void* mi
   st->map_k = mk;
   st->map_v = mv;
   st->bf16 = true;
+  if (st->params.out16 != nullptr && !encode_out16(st, st->params.out16)) st->params.out16 = nullptr;
+  const int64_t items = B * H * (st->params.q_tiles + (st->params.q_tiles - st->params.split_from));
+  const int64_t ctas = (st->alone ? 1 : 2) * (int64_t)plan.sm_count;
+  st->grid = dim3((unsigned)(items < ctas ? items : ctas), 1, 1);
   // D = F32, A/B = BF16: Q K^T both K-major, N = 128; P V with B N-major, N = 64; M = 128
   st->params.idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRows >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
   st->params.idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(kHeadDim >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
@@ -1554,18 +1473,19 @@ void attention_elide_copy(Plan& plan, size_t first) {
   holder.launches = 1 + (st->exact_tc ? 1 : 0);
 }
 
+bool attention_may_drop_float32(const PlanKernel& k) {
+  const AttnState* st = static_cast<const AttnState*>(k.attn);
+  return st && st->bf16 && st->params.out16 != nullptr;
+}
+void attention_drop_float32(PlanKernel& k) { static_cast<AttnState*>(k.attn)->params.out32 = false; }
+
 bool attention_reads_mirror(const PlanKernel& k) { return k.attn && static_cast<const AttnState*>(k.attn)->bf16; }
 
 void attention_set_shadow(PlanKernel& k, void* shadow_out) {
   AttnState* st = static_cast<AttnState*>(k.attn);
   if (!st || st->exact) return;
-  // the bf16 copy of the merged heads needs a store map of its own; without one it is not written
-  // (its reader was told to expect it: assign_shadows asks attention_can_shadow first)
-  __nv_bfloat16* out16 = static_cast<__nv_bfloat16*>(shadow_out);
-  if (out16 != nullptr && encode_map_store(&st->map_out16, true, out16, (int64_t)st->params.H * kHeadDim,
-                                            st->params.T, st->params.B, st->params.out16_row_stride,
-                                            st->params.T * st->params.out16_row_stride))
-    st->params.out16 = out16;
+  // (its reader was told to expect it)
+  if (shadow_out != nullptr && encode_out16(st, shadow_out)) st->params.out16 = static_cast<__nv_bfloat16*>(shadow_out);
 }
 
 const DevOperand* attention_output(const Plan& plan, size_t first, int64_t* elems) {

@@ -170,7 +170,7 @@ bool matmul_wants_bf16_operands(const PlanKernel& k);
 void attention_set_shadow(PlanKernel& k, void* shadow_out);
 bool attention_operand_span(const PlanKernel& k, const float** lo, const float** hi);
 void attention_elide_copy(Plan& plan, size_t first);
-bool attention_use_mirror(PlanKernel& k, const float* arena_base, const void* mirror_base);
+bool attention_use_mirror(const Plan& plan, PlanKernel& k, const float* arena_base, const void* mirror_base);
 const DevOperand* attention_output(const Plan& plan, size_t first, int64_t* elems);
 int launch_matmul(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 void destroy_matmul(PlanKernel& k);
@@ -178,6 +178,8 @@ int attention_try_fuse(Plan& plan, size_t first);    // plan kernels replaced fr
 int attention_chain_length(const PlanKernel& k);
 bool attention_wants_bf16(const PlanKernel& k);
 bool attention_reads_mirror(const PlanKernel& k);
+bool attention_may_drop_float32(const PlanKernel& k);    // writes a bf16 copy, and its float32 rows only where they were planned
+void attention_drop_float32(PlanKernel& k);
 bool tc_eligible(const PlanKernel& k);
 int attention_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 void attention_destroy(PlanKernel& k);

@@ -890,15 +890,24 @@ static int assign_shadows(Plan& plan) {
     if (k.a_shadow) k.a_shadow = mirror_of(k.ops[k.desc.a_slot].ptr);
     if (k.b_shadow) k.b_shadow = mirror_of(k.ops[k.desc.b_slot].ptr);
   }
-  for (size_t ki : attention_readers) attention_use_mirror(plan.kernels[ki], plan.arena, plan.arena16);
+  for (size_t ki : attention_readers) attention_use_mirror(plan, plan.kernels[ki], plan.arena, plan.arena16);
   if (!plan.mirror_only) return KB200_OK;
-  // A LayerNorm or matmul that writes the mirror drops its float32 store when, until that memory is
+  // A LayerNorm, matmul or fused attention that writes the mirror drops its float32 store when, until that memory is
   // rewritten (or the plan ends: arena contents are dead then), every reader takes the mirror.
   for (size_t ki = 0; ki < plan.kernels.size(); ++ki) {
     PlanKernel& k = plan.kernels[ki];
-    if (!k.shadow_out || (k.impl != IMPL_ROW_LAYERNORM && k.impl != IMPL_MM_TC)) continue;
-    const int out_slot = k.impl == IMPL_ROW_LAYERNORM ? k.out_slot : k.chain.out_slot;
-    Span w = span_of(k, out_slot);             // what of the output is still there
+    if (!k.shadow_out) continue;
+    Span w{nullptr, nullptr};                  // what of the output is still there
+    if (k.impl == IMPL_ATTN_FUSED) {
+      if (!attention_may_drop_float32(k)) continue;
+      int64_t elems = 0;
+      const DevOperand* y = attention_output(plan, ki, &elems);
+      w = Span{y->ptr, y->ptr + elems};
+    } else if (k.impl == IMPL_ROW_LAYERNORM || k.impl == IMPL_MM_TC) {
+      w = span_of(k, k.impl == IMPL_ROW_LAYERNORM ? k.out_slot : k.chain.out_slot);
+    } else {
+      continue;
+    }
     bool only = true, rewritten = false;
     int readers = 0;
     // The planner places buffers by size, so a later one may begin or end inside this one: what it leaves is still this
@@ -941,6 +950,7 @@ static int assign_shadows(Plan& plan) {
       }
     }
     k.mirror_only = only && readers > 0;
+    if (k.mirror_only && k.impl == IMPL_ATTN_FUSED) attention_drop_float32(k);
   }
   return KB200_OK;
 }
