@@ -629,35 +629,36 @@ int pair_share(const Plan& plan) {
 
 struct PairPlan { int bn; int64_t cycles; };
 
-// Tile width and estimated cycles of the slowest SM pair.  Width: a slab of a 256-column tile takes its 512
-// tensor cycles (541 measured; reading and filling shared memory takes as many), one of a 128-column
-// tile is bound by the issue (~490, ~365 with two slabs per step), and the last tile's epilogue
-// (~1200 cycles per 32-column block and warp) is not hidden.  Widths between the two were built and lost:
-// 192 columns even out the last round of 8192 x 768 (K = 3072 BF16: 42.3 against 40.6 us) and of
-// 8192 x 3072, but stage more bytes per FLOP (8192 x 2304: 28.0 against 22.8 us).
-// The estimate is a fit to launches of 256 to 2048 rows: 330 or 541 cycles per slab, ~20 bytes a clock to
-// drain the last tile, ~6300 for the rest.
-PairPlan plan_pair(const PlanKernel& k, bool two_slabs, int64_t share) {
-  const int slab_k = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;
+// Tile width and estimated cycles of the slowest SM pair: rounds of tiles, the cycles of a slab, ~20 bytes a clock to drain the
+// last tile, ~6300 for the rest.  A slab of 256 columns takes its 512 tensor cycles and a little; below that the 24 to 28 KB of
+// its operands' way from L2 take longer than the multiplying, more so with most SMs at it (an SM gets 60 to 75 bytes a
+// clock; two slabs per step at 128 columns, 490 with one).  Fitted to 2048 x 3072 x 768 and 2048 x 768 x 3072 in TF32.
+// The widths between 128 and 256 are for the last round: 2048 x 3072 x 768 TF32 20.2 us at 128 columns (three rounds, 64 of 74 pairs),
+// 22.2 at 256 (96 tiles), 18.3 at 192 (128 tiles, two rounds); 8192 x 768 x 3072 BF16 66.2 at 256, 59.5 at 192 (with its pass
+// over A); 8192 x 2304 x 768 36.1 at 256, 39.7 at 192.
+struct PairWidth { int bn, busy_cycles, light_cycles; };      // cycles of a slab with most of the pairs at work | with at most three quarters
+constexpr PairWidth kPairWidths[] = {{256, 553, 553}, {224, 490, 482}, {192, 433, 408}, {160, 395, 362}, {128, 365, 325}};
+
+PairPlan plan_pair(const PlanKernel& k, bool two_slabs, int64_t share, bool b_kmajor) {
+  const bool bf16 = k.desc.precision == KB200_PREC_BF16;
+  const int slab_k = bf16 ? 64 : 32, chunk_n = bf16 ? 64 : 32;
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
   PairPlan best{0, 0};
-  int64_t least = 0;
-  for (int bn : {256, 128}) {
-    if (bn > 128 && bn / 2 >= k.N) continue;
-    const int64_t tiles = ((k.M + 255) / 256) * ((k.N + bn - 1) / bn) * k.batch;
+  for (const PairWidth& w : kPairWidths) {
+    if (w.bn > 128 && w.bn / 2 >= k.N) continue;
+    if (!b_kmajor && w.bn / 2 % chunk_n) continue;         // an N-major B comes in whole chunks of columns
+    const int64_t tiles = ((k.M + 255) / 256) * ((k.N + w.bn - 1) / w.bn) * k.batch;
     const int64_t rounds = (tiles + share - 1) / share;
-    const int64_t cost = rounds * slabs * (bn == 256 ? 512 : two_slabs ? 365 : 490) + (bn / 64) * 1200;
-    if (best.bn == 0 || cost < least) {
-      best = {bn, rounds * slabs * (bn == 256 ? 541 : 330) + 6300 + (int64_t)bn * 128 * 4 / 20};
-      least = cost;
-    }
+    const int slab_cycles = w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
+    const int64_t cycles = rounds * slabs * slab_cycles + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, cycles};
   }
   return best;
 }
 
 }  // namespace
 
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k) { return plan_pair(k, true, plan.sm_count / 2).cycles; }
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(k, true, plan.sm_count / 2, b_kmajor).cycles; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
@@ -700,8 +701,8 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   int kps = d.cfg[2] == 1 || d.cfg[2] == 2 ? d.cfg[2] : 0;
   const int share = pair_share(plan);
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  if (bn == 0) bn = plan_pair(k, kps != 1, share).bn;
-  while (bn > 128 && bn / 2 >= k.N) bn /= 2;
+  if (bn == 0) bn = plan_pair(k, kps != 1, share, ops.b_kmajor).bn;
+  while (bn == 256 && bn / 2 >= k.N) bn /= 2;
   // Staging per epilogue warp: one slot for a 32 x 32 block, float32 (also where a matrix operand of
   // the chain lands; left out when only the mirror is stored) and its bf16 copy.
   const bool store32 = !(k.mirror_only && out16 != nullptr);

@@ -21,7 +21,7 @@ struct PairOperands {
 
 // Shape, layout and epilogue tests that need no device pointers beyond those already resolved in `k`.
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols);
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k);      // estimated cycles of a launch that has the GPU to itself
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor);      // estimated cycles of a launch that has the GPU to itself
 // Builds tensor maps and launch parameters.  *state stays null when the kernel declines (the caller
 // then uses the single-CTA kernel); a non-zero return is an error.
 int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, void** state);

@@ -1,0 +1,58 @@
+"""The matmul kernel on SM pairs at each of its tile widths: ragged last tiles of rows and columns, K off a slab,
+weights along K and operands along N."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# float32 sums of operands rounded to 2^-9 (bf16) or cut to 2^-10 (TF32), relative to the 2-norm: about 0.8 of that per product
+BOUND = {"tf32": 1e-3, "bf16": 3e-3}
+
+
+def run(p, precision):
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable
+    from perf import cases
+
+    plan = p.spec()
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    exe = GPUExecutable(program_from_plan(plan, precision), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
+    x = torch.randn(plan.input_shapes[0], generator=torch.Generator(device="cuda").manual_seed(0), device="cuda")
+    outs = [exe(x)[0] for _ in range(3)]
+    exe.status()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    return exe, x.double(), {name: torch.from_numpy(c).cuda().double() for name, c in consts.items()}, outs[0].double()
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k,width", [(4096, 640, 640, 160), (4000, 612, 200, 160), (1024, 3072, 768, 192), (1000, 3028, 772, 192), (2432, 1568, 1536, 224),
+                                         (2305, 1444, 1028, 224), (8192, 2304, 512, 256), (8190, 2304, 516, 256)])
+def test_linear_at_every_width(m, n, k, width, precision):
+    from perf import cases
+
+    p = cases._Plan("linear", (m, k), (m, n))
+    p.linear(p.x, "", n, p.y)
+    exe, x, c, got = run(p, precision)
+    assert f"mm_pair {width} columns" in exe.details[0], exe.details
+    want = x @ c["weight.transpose"] + c["bias"]
+    assert float((got - want).norm() / want.norm()) <= BOUND[precision]
+    assert float((got - want).abs().max() / want.std()) <= 10 * BOUND[precision]
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("m,n", [(1024, 3072), (1000, 3008)])
+def test_an_operand_along_n(m, n, precision):
+    """B is an activation [K, N]: whole chunks of its columns only (192 columns in TF32, not in BF16)."""
+    from perf import cases
+
+    k = 512
+    p = cases._Plan("product", (k, 128), (1, m, n))
+    b = p.buffer(k, n)
+    p.linear(p.x, "0.", n, b)
+    p.bmm(p.const("a", 1, m, k), b.as_((1, k, n)), p.y)
+    exe, x, c, got = run(p, precision)
+    assert "mm_pair" in exe.details[1] and ("192 columns" in exe.details[1]) == (precision == "tf32"), exe.details
+    want = c["a"] @ (x @ c["0.weight.transpose"] + c["0.bias"])
+    assert float((got - want).norm() / want.norm()) <= 2 * BOUND[precision]
