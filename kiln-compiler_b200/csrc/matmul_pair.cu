@@ -27,6 +27,10 @@
 //               runs under the main loop of tile i + 1; both CTAs' warps release the buffer on the
 //               leader's `tempty` barrier.  (Warps 14 and 15 are idle: 512 threads are what leaves
 //               the compiler 128 registers per thread.)
+//
+// Few tiles and a long K (SPLIT): the cluster is two pairs, each with half of K for the same tile.  Their accumulators meet
+// through shared memory: every epilogue warp sends the 32 x 32 blocks of the other pair's half of the columns as bulk copies
+// into that CTA's ring, idle by then, and finishes its own.
 // Every mbarrier wait is bounded: on expiry the thread records (kernel, site) in the plan's status
 // word, raises its CTA's abort flag, all roles fall through to the exit, which passes the cluster
 // barrier (every path reaches it), frees TMEM and returns.  The other CTA's waits run out by themselves.
@@ -57,7 +61,7 @@ constexpr int kPairATileBytes = 128 * 128;        // 128 rows x one 128-byte K s
 constexpr int kPairSmemCeiling = 224 * 1024;      // opt-in ceiling, the same for every launch of the kernel
 // barrier indices
 constexpr int kBarFull = 0, kBarEmpty = kPairMaxStages, kBarTFull = 2 * kPairMaxStages, kBarTEmpty = kBarTFull + 2,
-              kBarRes = kBarTEmpty + 2, kBarCount = kBarRes + kPairEpiWarps;
+              kBarRes = kBarTEmpty + 2, kBarRecv = kBarRes + kPairEpiWarps, kBarPeer = kBarRecv + kPairEpiWarps, kBarCount = kBarPeer + 1;
 
 // The chains of a transformer's Linears have epilogues of their own; any other runs step by step.  A step of
 // the general form looks its descriptor up, branches on the operand's kind and jumps through a
@@ -79,6 +83,7 @@ struct PairStep {
 struct PairParams {
   // what the producer and the MMA thread need comes first (constant-bank lines touched at start-up)
   int bn, half_bn, stages, num_kb, slab_k, kps, step_k;
+  int first_kb;          // SPLIT: steps of the first pair
   int b_static;          // B is a frozen constant: its first stages are requested before the previous kernel has finished
   int b_kmajor;          // B is [N, K] with K contiguous (boxes like A); else [K, N], one 4-D box per stage
   int chunk_n;           // columns per 128-byte row of an N-major B chunk: 32 (tf32) or 64 (bf16)
@@ -133,15 +138,21 @@ __device__ __forceinline__ void umma_pair(uint32_t on, uint32_t tmem_d, uint64_t
 // Arrives, when every MMA issued so far by this thread has completed, on the mbarrier at this offset
 // in BOTH CTAs of the pair (a commit, not a copy: the arrival is what is sent to the two CTAs).  One
 // instruction: a commit costs the issuing thread about as much as two MMAs.
-__device__ __forceinline__ void umma_pair_commit(uint32_t bar) {
+__device__ __forceinline__ void umma_pair_commit(uint32_t bar, uint16_t pair_ctas) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"((uint16_t)3)
+               ::"r"(bar), "h"(pair_ctas)
                : "memory");
 }
 __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
+}
+// Bulk copy from this CTA's shared memory into another's of the cluster, where it completes on a barrier.
+__device__ __forceinline__ void push_block(uint32_t remote_dst, uint32_t src, uint32_t bytes, uint32_t remote_bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(remote_dst), "r"(src), "r"(bytes), "r"(remote_bar)
+               : "memory");
 }
 // At most `allowed` of this thread's most recent bulk-store groups may still be reading shared memory.
 __device__ __forceinline__ void store_wait_read(int allowed) {
@@ -164,7 +175,7 @@ __device__ __forceinline__ void load_b_pair(const PairParams& p, const CUtensorM
   }
 }
 
-template <bool BF16, int KPS, int EPI>
+template <bool BF16, int KPS, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(kPairThreads, 1)
 mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                const __grid_constant__ CUtensorMap tma_out, const __grid_constant__ CUtensorMap tma_out16,
@@ -185,7 +196,13 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   const int warp = warp_index(), lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  // with SPLIT the CTAs 0, 1 and 2, 3 of a cluster are a pair each, `pair` counts clusters, and a cluster has one tile
+  const uint32_t leader = SPLIT ? rank & 2u : 0u, cta = rank;
+  rank &= 1u;
+  const int pair = blockIdx.x >> (SPLIT ? 2 : 1), num_pairs = gridDim.x >> (SPLIT ? 2 : 1);
+  const int first_kb = SPLIT && leader != 0 ? p.first_kb : 0;                                          // this pair's steps of K
+  const int my_kb = !SPLIT ? p.num_kb : leader != 0 ? p.num_kb - p.first_kb : p.first_kb;
+  const uint16_t pair_ctas = (uint16_t)(3u << leader);
   const uint32_t full0 = smem_u32(&bars[kBarFull]), empty0 = smem_u32(&bars[kBarEmpty]);
   const uint32_t tfull0 = smem_u32(&bars[kBarTFull]), tempty0 = smem_u32(&bars[kBarTEmpty]);
 
@@ -224,7 +241,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   volatile int* abort_ptr = &abort_flag;
   // The MMA instruction names one TMEM address for both CTAs: the two allocations must agree.
   if (threadIdx.x == 0 && rank == 1) {
-    const uint32_t leader_base = ld_cluster_u32(map_to_cta(smem_u32(&tmem_base_slot), 0));
+    const uint32_t leader_base = ld_cluster_u32(map_to_cta(smem_u32(&tmem_base_slot), leader));
     if (leader_base != tmem_base) {
       atomicCAS(p.status, 0, (p.kernel_index << 8) | 9);
       *abort_ptr = 1;
@@ -232,17 +249,17 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   }
   // A frozen B is nobody's output: the first stages' weights are requested before the wait for the
   // previous kernel, so that they are on their way, or here, when the activations are ready.
-  const uint32_t full_leader0 = map_to_cta(full0, 0);
+  const uint32_t full_leader0 = map_to_cta(full0, leader);
   int ahead = 0;                 // stages of the first tile whose B is requested already (producer warp)
   if (p.b_static && warp == 0 && pair < p.num_tiles) {
     const int batch = pair_div(pair, p.magic_tpb);
     const int rem = pair - batch * p.tiles_per_batch;
     const int n_col = (rem - pair_div(rem, p.magic_tn) * p.tiles_n) * p.bn + (int)rank * p.half_bn;
-    ahead = p.stages < p.num_kb ? p.stages : p.num_kb;
+    ahead = p.stages < my_kb ? p.stages : my_kb;
     if (elect_one()) {
       for (int s = 0; s < ahead; ++s) {
         if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
-        load_b_pair<KPS>(p, &tma_b, tiles + (uint32_t)(s * stage_bytes + a_stage_bytes), full_leader0 + 8 * s, s * p.step_k, n_col, batch);
+        load_b_pair<KPS>(p, &tma_b, tiles + (uint32_t)(s * stage_bytes + a_stage_bytes), full_leader0 + 8 * s, (first_kb + s) * p.step_k, n_col, batch);
       }
     }
     __syncwarp();
@@ -254,7 +271,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     // (like the MMA issuer's, a role that the whole warp walks, one lane issuing: see elect_one)
-    const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, slab_k = p.slab_k, step_k = p.step_k;
+    const int stages = p.stages, num_tiles = p.num_tiles, num_kb = my_kb, slab_k = p.slab_k, step_k = p.step_k;
     const int bn = p.bn, half_bn = p.half_bn;
     int s = 0;
     uint32_t wait_parity = 1;
@@ -266,7 +283,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       const int tn_i = rem - tm_i * p.tiles_n;
       const int m_row = tm_i * 256 + (int)rank * 128;
       const int n_col = tn_i * bn + (int)rank * half_bn;
-      int k_elem = 0;
+      int k_elem = first_kb * step_k;
       for (int kb = 0; kb < num_kb; ++kb, k_elem += step_k) {
         const bool got = mbar_wait_cluster(empty0 + 8 * s, wait_parity, abort_ptr);
         if (!__all_sync(0xffffffffu, got ? 1 : 0)) {
@@ -295,7 +312,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     // A step is one barrier probe, 4 * KPS MMAs whose descriptor words advance by additions, and ONE commit
     // for both CTAs (a commit costs about as much as two MMAs).
     if (rank == 0) {
-      const int stages = p.stages, num_tiles = p.num_tiles, num_kb = p.num_kb, bn = p.bn;
+      const int stages = p.stages, num_tiles = p.num_tiles, num_kb = my_kb, bn = p.bn;
       const uint32_t idesc = p.idesc;
       const uint64_t a_fixed = make_desc(0, 16, 1024);
       const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo_bytes, p.b_sbo_bytes, p.b_layout);
@@ -340,8 +357,8 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
           }
           if (on) {
             // the stage is free in both CTAs once these MMAs have read it
-            umma_pair_commit(empty0 + 8 * s);
-            if (kb + 1 == num_kb) umma_pair_commit(tfull0 + 8 * acc);
+            umma_pair_commit(empty0 + 8 * s, pair_ctas);
+            if (kb + 1 == num_kb) umma_pair_commit(tfull0 + 8 * acc, pair_ctas);
           }
           __syncwarp();
           a16 += stage16;
@@ -362,7 +379,9 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     const uint32_t slot0 = epi_base + (uint32_t)(e * slot_bytes);
     uint8_t* const slot0_ptr = smem_raw + (slot0 - raw);
     const uint32_t res_bar = smem_u32(&bars[kBarRes + e]);
-    const uint32_t tempty_leader0 = map_to_cta(tempty0, 0);
+    const uint32_t tempty_leader0 = map_to_cta(tempty0, leader);
+    // the columns of a tile that this pair finishes
+    const int c_first = SPLIT && leader != 0 ? p.half_bn : 0, c_end = SPLIT ? c_first + p.half_bn : p.bn;
     const bool has_res = p.res_step >= 0, with16 = p.out16 != nullptr, with32 = p.store32 != 0;
     // where the block's per-column operand passes through shared memory (-1: broadcast by shuffles)
     const int scratch_off = !has_res ? 0 : (with16 ? 4096 : -1);
@@ -438,17 +457,17 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         const float* src = chain_steps[col_step].ptr + (int64_t)batch * chain_steps[col_step].batch_stride + n0 + lane;
 #pragma unroll
         for (int j = 0; j < kPairBlocksPerWarp; ++j) {
-          const int c = 32 * (group + kPairWarpsPerQuad * j);
-          col_pre[j] = (c < p.bn && n0 + c + lane < p.N) ? __ldg(src + c) : 0.0f;
+          const int c = c_first + 32 * (group + kPairWarpsPerQuad * j);
+          col_pre[j] = (c < c_end && n0 + c + lane < p.N) ? __ldg(src + c) : 0.0f;
         }
       }
       // the first block's matrix operand is requested before the accumulator is ready
       bool res_ready = false;
-      if (has_res && !dry && rows_ok && 32 * group < p.bn && n0 + 32 * group < p.N) {
+      if (has_res && !dry && rows_ok && c_first + 32 * group < c_end && n0 + c_first + 32 * group < p.N) {
         if (lane == 0) {
           store_wait_read(0);
           mbar_expect_tx(res_bar, 4096);
-          tma_load_3d(slot0, &tma_res, res_bar, n0 + 32 * group, m_first, p.res_batched ? batch : 0);
+          tma_load_3d(slot0, &tma_res, res_bar, n0 + c_first + 32 * group, m_first, p.res_batched ? batch : 0);
         }
         res_ready = true;
       }
@@ -459,11 +478,45 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         if (!ok) break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // SPLIT: the sums of the other pair's columns leave for its CTA with the same rows, those of this one's columns come from
+      // there.  The rings are idle: one half of this CTA's is what it sends, the other half what it gets.
+      [[maybe_unused]] const uint32_t recv_bar = smem_u32(&bars[kBarRecv + e]);
+      [[maybe_unused]] const uint32_t recv_area = (uint32_t)(p.half_bn / 32 * 4 * 4096);
+      if constexpr (SPLIT) {
+        if (!dry) {
+          const uint32_t other = cta ^ 2u;
+          if (e == 0 && lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars[kBarPeer]), other));      // this CTA's ring may be written
+          uint32_t coming = 0;
+          for (int c = 32 * group; c < p.half_bn; c += 32 * kPairWarpsPerQuad)
+            if (rows_ok && n0 + c_first + c < p.N) coming += 4096;
+          if (lane == 0 && coming != 0) mbar_expect_tx(recv_bar, coming);
+          const int c_other = p.half_bn - c_first;
+          bool free = false;
+#pragma unroll 1
+          for (int c = 32 * group; c < p.half_bn; c += 32 * kPairWarpsPerQuad) {
+            if (!rows_ok || n0 + c_other + c >= p.N) break;
+            const uint32_t at = (uint32_t)((c / 32 * 4 + quad) * 4096);
+            float v[32];
+            tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c_other + c), v);
+            uint8_t* const mine = smem_raw + (tiles - raw) + at;
+            stage_rows(mine, mine, v, lane, false);
+            fence_async_smem();
+            __syncwarp();
+            if (!free) {
+              const bool got = mbar_wait_cluster(smem_u32(&bars[kBarPeer]), 0, abort_ptr);
+              if (!got && lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 7); *abort_ptr = 1; }
+              free = __all_sync(0xffffffffu, got ? 1 : 0) != 0;
+              if (!free) break;
+            }
+            if (lane == 0) push_block(map_to_cta(tiles + recv_area + at, other), tiles + at, 4096, map_to_cta(recv_bar, other));
+          }
+        }
+      }
 #pragma unroll 1
       for (int j = 0; j < kPairBlocksPerWarp; ++j) {
-        const int c = 32 * (group + kPairWarpsPerQuad * j);
+        const int c = c_first + 32 * (group + kPairWarpsPerQuad * j);
         const int n = n0 + c;
-        if (c >= p.bn || !rows_ok || n >= p.N) break;          // uniform across the warp
+        if (c >= c_end || !rows_ok || n >= p.N) break;          // uniform across the warp
         float mine = col_pre[0];
 #pragma unroll
         for (int q = 1; q < kPairBlocksPerWarp; ++q)
@@ -482,6 +535,21 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         float v[32];
         tmem_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * p.bn + c), v);
         __syncwarp();
+        if constexpr (SPLIT) {
+          if (!dry) {
+            const bool got = mbar_wait_cluster(recv_bar, 0, abort_ptr);
+            if (!got && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 6); *abort_ptr = 1; }
+            __syncwarp();
+            const uint8_t* const theirs = smem_raw + (tiles - raw) + recv_area + ((c - c_first) / 32 * 4 + quad) * 4096;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const float4 t = *reinterpret_cast<const float4*>(theirs + lane * 128 + ((q ^ (lane & 7)) << 4));
+              const float2 a = fadd2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(t.x, t.y));
+              const float2 b = fadd2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(t.z, t.w));
+              v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = b.x; v[4 * q + 3] = b.y;
+            }
+          }
+        }
         if constexpr (EPI == EPI_CHAIN) {
           run_chain(v, mine, n, batch);
         } else {
@@ -555,13 +623,13 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 
 using PairKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, PairParams);
 
-template <bool BF16, int KPS>
+template <bool BF16, int KPS, bool SPLIT>
 PairKernel pair_kernel(int epilogue) {
   switch (epilogue) {
-    case EPI_BIAS: return mm_pair_kernel<BF16, KPS, EPI_BIAS>;
-    case EPI_BIAS_GELU: return mm_pair_kernel<BF16, KPS, EPI_BIAS_GELU>;
-    case EPI_BIAS_RES: return mm_pair_kernel<BF16, KPS, EPI_BIAS_RES>;
-    default: return mm_pair_kernel<BF16, KPS, EPI_CHAIN>;
+    case EPI_BIAS: return mm_pair_kernel<BF16, KPS, EPI_BIAS, SPLIT>;
+    case EPI_BIAS_GELU: return mm_pair_kernel<BF16, KPS, EPI_BIAS_GELU, SPLIT>;
+    case EPI_BIAS_RES: return mm_pair_kernel<BF16, KPS, EPI_BIAS_RES, SPLIT>;
+    default: return mm_pair_kernel<BF16, KPS, EPI_CHAIN, SPLIT>;
   }
 }
 
@@ -580,6 +648,7 @@ struct PairState {
   size_t smem_bytes = 0;
   dim3 grid;
   bool bf16 = false;
+  bool split = false;      // clusters of two pairs, half of K each
   PairKernel kernel = nullptr;
 };
 
@@ -627,7 +696,33 @@ int pair_share(const Plan& plan) {
   return share > 0 ? share : 1;
 }
 
-struct PairPlan { int bn; int64_t cycles; };
+struct PairPlan { int bn; bool split; int64_t cycles; };
+
+// Clusters of two pairs that fit the GPU at once.
+int resident_quads(const Plan& plan) {
+  int& known = plan.resident_quads;
+  if (known == 0) {
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(plan.sm_count / 4 * 4), 1, 1);
+    cfg.blockDim = dim3(kPairThreads, 1, 1);
+    cfg.dynamicSmemBytes = kPairSmemCeiling;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 4;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const PairKernel kernel = mm_pair_kernel<true, 1, EPI_BIAS, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemCeiling) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known = n > 0 ? n : -1;
+  }
+  return known;
+}
 
 // Tile width and estimated cycles of the slowest SM pair: rounds of tiles, the cycles of a slab, ~20 bytes a clock to drain the
 // last tile, ~6300 for the rest.  A slab of 256 columns takes its 512 tensor cycles and a little; below that the 24 to 28 KB of
@@ -639,11 +734,11 @@ struct PairPlan { int bn; int64_t cycles; };
 struct PairWidth { int bn, busy_cycles, light_cycles; };      // cycles of a slab with most of the pairs at work | with at most three quarters
 constexpr PairWidth kPairWidths[] = {{256, 553, 553}, {224, 490, 482}, {192, 433, 408}, {160, 395, 362}, {128, 365, 325}};
 
-PairPlan plan_pair(const PlanKernel& k, bool two_slabs, int64_t share, bool b_kmajor) {
+PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, int64_t share, bool b_kmajor) {
   const bool bf16 = k.desc.precision == KB200_PREC_BF16;
   const int slab_k = bf16 ? 64 : 32, chunk_n = bf16 ? 64 : 32;
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  PairPlan best{0, 0};
+  PairPlan best{0, false, 0};
   for (const PairWidth& w : kPairWidths) {
     if (w.bn > 128 && w.bn / 2 >= k.N) continue;
     if (!b_kmajor && w.bn / 2 % chunk_n) continue;         // an N-major B comes in whole chunks of columns
@@ -651,14 +746,18 @@ PairPlan plan_pair(const PlanKernel& k, bool two_slabs, int64_t share, bool b_km
     const int64_t rounds = (tiles + share - 1) / share;
     const int slab_cycles = w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
     const int64_t cycles = rounds * slabs * slab_cycles + 6300 + (int64_t)w.bn * 128 * 4 / 20;
-    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, cycles};
+    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
+    // K in halves on twice the pairs: the exchange of half a tile costs ~2500, and half as much is left to drain
+    if (w.bn % 64 || w.bn == 128 || plan.concurrency > 1 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
+    const int64_t halved = (slabs + 1) / 2 * (8 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles) + 6300 + 2500 + (int64_t)w.bn * 64 * 4 / 20;
+    if (halved < best.cycles) best = {w.bn, true, halved};
   }
   return best;
 }
 
 }  // namespace
 
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(k, true, plan.sm_count / 2, b_kmajor).cycles; }
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, plan.sm_count / 2, b_kmajor).cycles; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
@@ -701,7 +800,11 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   int kps = d.cfg[2] == 1 || d.cfg[2] == 2 ? d.cfg[2] : 0;
   const int share = pair_share(plan);
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
-  if (bn == 0) bn = plan_pair(k, kps != 1, share, ops.b_kmajor).bn;
+  if (bn == 0) {
+    const PairPlan how = plan_pair(plan, k, kps != 1, share, ops.b_kmajor);
+    bn = how.bn;
+    st->split = how.split && d.cfg[3] == 0 && kps != 2;
+  }
   while (bn == 256 && bn / 2 >= k.N) bn /= 2;
   // Staging per epilogue warp: one slot for a 32 x 32 block, float32 (also where a matrix operand of
   // the chain lands; left out when only the mirror is stored) and its bf16 copy.
@@ -716,6 +819,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   p.kps = kps;
   p.step_k = kps * slab_k;
   p.num_kb = (int)((k.K + p.step_k - 1) / p.step_k);
+  p.first_kb = (p.num_kb + 1) / 2;
   p.b_kmajor = ops.b_kmajor ? 1 : 0;
   p.b_static = ops.b_static ? 1 : 0;
   p.chunk_n = chunk_n;
@@ -751,6 +855,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   if (stages > kPairMaxStages) stages = kPairMaxStages;
   while (stages > 2 && (size_t)stages * stage_bytes + epi_bytes + 1024 > (size_t)kPairSmemCeiling) --stages;
   if ((size_t)stages * stage_bytes + epi_bytes + 1024 > (size_t)kPairSmemCeiling) { delete st; return KB200_OK; }
+  if (stages * stage_bytes < 2 * p.half_bn * 128 * 4) st->split = false;       // (what is sent and what is received lie in the ring)
   p.stages = stages;
   st->smem_bytes = (size_t)stages * stage_bytes + epi_bytes + 1024;
   // Persistent pairs: as many as there are tiles, up to this plan's share of the GPU.  With several
@@ -759,7 +864,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   // share of the pairs every pair walks several tiles and drains one while it multiplies the next.
   const int rounds = (p.num_tiles + share - 1) / share;
   const int n_pairs = (p.num_tiles + rounds - 1) / rounds;
-  st->grid = dim3((unsigned)(2 * n_pairs), 1, 1);
+  st->grid = dim3((unsigned)(st->split ? 4 * p.num_tiles : 2 * n_pairs), 1, 1);
 
   bool ok = encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, k.batch, ops.a_row, ops.a_batch, slab_k, 128, false);
   if (ok) {
@@ -775,8 +880,10 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   if (ok && out16) ok = encode_map_store(&st->map_out16, true, out16, k.N, k.M, k.batch, O.stride[1], O.stride[0]);
   if (ok && res) ok = encode_map_store(&st->map_res, false, res->ptr, k.N, k.M, p.res_batched ? k.batch : 1, res->stride[1], res->stride[0]);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = ops.bf16 ? (kps == 2 ? pair_kernel<true, 2>(epilogue_of(p)) : pair_kernel<true, 1>(epilogue_of(p)))
-                        : (kps == 2 ? pair_kernel<false, 2>(epilogue_of(p)) : pair_kernel<false, 1>(epilogue_of(p)));
+  const int epilogue = epilogue_of(p);
+  if (st->split) st->kernel = ops.bf16 ? pair_kernel<true, 1, true>(epilogue) : pair_kernel<false, 1, true>(epilogue);
+  else if (kps == 2) st->kernel = ops.bf16 ? pair_kernel<true, 2, false>(epilogue) : pair_kernel<false, 2, false>(epilogue);
+  else st->kernel = ops.bf16 ? pair_kernel<true, 1, false>(epilogue) : pair_kernel<false, 1, false>(epilogue);
   cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemCeiling);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_pair_kernel)"); }
   *state = st;
@@ -793,7 +900,7 @@ int pair_launch(const Plan& plan, const void* state, cudaStream_t s) {
   cudaLaunchAttribute attr[2];
   int n_attr = 0;
   attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-  attr[n_attr].val.clusterDim.x = 2;
+  attr[n_attr].val.clusterDim.x = st->split ? 4 : 2;
   attr[n_attr].val.clusterDim.y = 1;
   attr[n_attr].val.clusterDim.z = 1;
   ++n_attr;
@@ -823,7 +930,7 @@ bool pair_repoint(const PlanKernel& k, void* state, const void* a, const void* b
 
 std::string pair_detail(const void* state) {
   const PairState* st = static_cast<const PairState*>(state);
-  return "mm_pair " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.kps) + " slabs";
+  return "mm_pair " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.kps) + " slabs" + (st->split ? ", 2 splits" : "");
 }
 
 void pair_destroy(void* state) { delete static_cast<PairState*>(state); }

@@ -56,3 +56,25 @@ def test_an_operand_along_n(m, n, precision):
     assert "mm_pair" in exe.details[1] and ("192 columns" in exe.details[1]) == (precision == "tf32"), exe.details
     want = c["a"] @ (x @ c["0.weight.transpose"] + c["0.bias"])
     assert float((got - want).norm() / want.norm()) <= 2 * BOUND[precision]
+
+
+@pytest.mark.parametrize("epilogue", ["bias", "gelu", "residual", "relu"])
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(2048, 768, 3072), (1998, 768, 3080), (1793, 708, 4100), (600, 2048, 2048)])
+def test_k_in_halves(m, n, k, precision, epilogue):
+    """Two pairs per tile, half of K each: ragged rows and columns (blocks of 32 columns that one of the pairs has not), steps of K that do not
+    come out even, every kind of epilogue."""
+    from perf import cases
+
+    p = cases._Plan("linear", (m, k), (m, n))
+    if epilogue == "relu":
+        p.kernel("matmul", [("matmul", [("operand", 0), ("operand", 1)], (m, n)), ("add", [("node", 0), ("operand", 2)], (m, n)), ("relu", [("node", 1)], (m, n))],
+                 [p.x, p.const("weight.transpose", k, n), p.const("bias", n)], [(2, p.y)])
+    else:
+        p.linear(p.x, "", n, p.y, gelu=epilogue == "gelu", residual=p.const("other", m, n) if epilogue == "residual" else None)
+    exe, x, c, got = run(p, precision)
+    assert "2 splits" in exe.details[0] and "mm_pair" in exe.details[0], exe.details
+    want = x @ c["weight.transpose"] + c["bias"]
+    want = {"bias": want, "relu": want.relu(), "gelu": torch.nn.functional.gelu(want, approximate="tanh")}.get(epilogue, want + c.get("other", 0))
+    assert float((got - want).norm() / want.norm()) <= BOUND[precision]
+    assert float((got - want).abs().max() / want.std()) <= 10 * BOUND[precision]
