@@ -87,60 +87,125 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) mm_simt_kernel(const __
 }
 
 // Decode shape, M == 1: the weight matrix is read exactly once, so the kernel is bound by how many
-// bytes it keeps in flight.  Each CTA owns 32 output columns (one per lane: a warp reads 128
-// contiguous bytes of a row of B); its 32 warps split K, each with up to sixteen rows in flight (6 MB
-// over the 96 CTAs of a 3072-wide layer), and combine through shared memory in warp order, which
-// keeps the result deterministic.  (64 columns and 8 warps with four rows in flight gave 48 CTAs and
-// 0.9 TB/s; staging the vector in shared memory to have 32 rows in flight measured slower.)
+// bytes it keeps in flight and by the latencies around that.  Each CTA owns 32 output columns; its 32 warps split K and
+// combine through shared memory in warp order, which keeps the result deterministic.  A warp reads four rows of 128 bytes per
+// instruction (VEC = 4; one where rows are off a 16-byte pitch), up to 24 rows at once: all of K = 768, 9.4 MB over the 96 CTAs of a
+// 3072-wide layer.  Those of a frozen weight are requested before the wait for the previous kernel, whose
+// tail they then arrive under.  The parameters are this kernel's own 0.4 KB: those of the general epilogue are 2.9 KB, which every
+// launch pays for on the host and again in a cold constant cache.
 constexpr int kGemvWarps = 32;
 constexpr int kGemvCols = 32;
-__global__ void __launch_bounds__(kGemvWarps * 32) mm_gemv_kernel(const __grid_constant__ MatmulParams p) {
-  pdl_wait();                 // the producer of this kernel's inputs has completed
-  pdl_launch_dependents();    // the next kernel may begin its start-up
-  __shared__ float part[kGemvWarps][kGemvCols];
+constexpr int kGemvRows = 24;        // rows of B a warp has in flight
+
+struct GemvOperand {
+  float* ptr;
+  int64_t batch_stride, stride;      // elements per batch entry | per column (per k for A, per row for B)
+};
+struct GemvParams {
+  int64_t N, K;
+  GemvOperand a, b, out, side[kMaxChain];
+  int frozen;                        // B is a constant: nobody before this kernel writes it
+  int n_steps;
+  int op[kMaxChain];
+  float imm[kMaxChain];              // used where side[].ptr is null
+};
+
+// One column's sum -> the fused chain -> memory.
+__device__ __forceinline__ void gemv_store(const GemvParams& p, float v, int64_t b, int64_t n) {
+#pragma unroll 1
+  for (int s = 0; s < p.n_steps; ++s) {
+    const float* const side = p.side[s].ptr;
+    v = apply_chain(p.op[s], v, side != nullptr ? side[b * p.side[s].batch_stride + n * p.side[s].stride] : p.imm[s]);
+  }
+  p.out.ptr[b * p.out.batch_stride + n * p.out.stride] = v;
+}
+// (an epilogue that is no chain)
+__device__ __forceinline__ void gemv_store(const MatmulParams& p, float v, int64_t b, int64_t n) { epilogue_store(p, v, b, 0, n); }
+
+__device__ __forceinline__ GemvOperand gemv_a(const GemvParams& p) { return p.a; }
+__device__ __forceinline__ GemvOperand gemv_b(const GemvParams& p) { return p.b; }
+__device__ __forceinline__ bool gemv_frozen(const GemvParams& p) { return p.frozen != 0; }
+__device__ __forceinline__ GemvOperand gemv_a(const MatmulParams& p) { return {p.ops[p.a_slot].ptr, p.ops[p.a_slot].stride[0], p.ops[p.a_slot].stride[2]}; }
+__device__ __forceinline__ GemvOperand gemv_b(const MatmulParams& p) { return {p.ops[p.b_slot].ptr, p.ops[p.b_slot].stride[0], p.ops[p.b_slot].stride[1]}; }
+__device__ __forceinline__ bool gemv_frozen(const MatmulParams&) { return false; }
+
+template <typename Params, int VEC>
+__global__ void __launch_bounds__(kGemvWarps * 32) mm_gemv_kernel(const __grid_constant__ Params p) {
+  __shared__ __align__(16) float part[kGemvWarps][kGemvCols];
+  constexpr int kLanes = kGemvCols / VEC;         // lanes a row takes
+  constexpr int kStep = 32 / kLanes;              // rows per instruction
+  constexpr int kLoads = kGemvRows / kStep;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t b = blockIdx.z;
-  const float* A = p.ops[p.a_slot].ptr + b * p.ops[p.a_slot].stride[0];
-  const float* B = p.ops[p.b_slot].ptr + b * p.ops[p.b_slot].stride[0];
-  const int64_t a_sk = p.ops[p.a_slot].stride[2];
-  const int64_t b_sk = p.ops[p.b_slot].stride[1];
-  const int64_t n = (int64_t)blockIdx.x * kGemvCols + lane;
-  const int64_t k_per = (p.K + kGemvWarps - 1) / kGemvWarps;
-  const int64_t k_lo = warp * k_per, k_hi = (k_lo + k_per < p.K) ? k_lo + k_per : p.K;
-  float acc = 0.0f;
-  if (n < p.N) {
-    int64_t k = k_lo;
-    for (; k + 16 <= k_hi; k += 16) {
-      float w[16], a[16];
+  const GemvOperand oa = gemv_a(p), ob = gemv_b(p);
+  const int64_t n = (int64_t)blockIdx.x * kGemvCols + lane % kLanes * VEC;
+  const int K = (int)p.K, k_per = (K + kGemvWarps - 1) / kGemvWarps;
+  const int k_end = min((warp + 1) * k_per, K);
+  const int k_first = warp * k_per + lane / kLanes;
+  const float* const A = oa.ptr + b * oa.batch_stride;
+  const float* const B = ob.ptr + b * ob.batch_stride + n;
+  const bool live = n < p.N;                      // (VEC = 4: N is a multiple of four)
+  float w[kLoads][VEC], acc[VEC];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        w[u] = __ldg(B + (k + u) * b_sk + n);
-        a[u] = __ldg(A + (k + u) * a_sk);
+  for (int e = 0; e < VEC; ++e) acc[e] = 0.0f;
+  auto fetch = [&](int k0) {
+    const float* row = B + k0 * ob.stride;
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      if (live && k0 + u * kStep < k_end) {
+        if constexpr (VEC == 4) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(row));
+          w[u][0] = t.x; w[u][1] = t.y; w[u][2] = t.z; w[u][3] = t.w;
+        } else {
+          w[u][0] = __ldg(row);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) w[u][e] = 0.0f;
       }
-#pragma unroll
-      for (int u = 0; u < 16; ++u) acc = fmaf(a[u], w[u], acc);
+      row += kStep * ob.stride;
     }
-    for (; k + 8 <= k_hi; k += 8) {
-      float w[8], a[8];
+  };
+  const bool early = gemv_frozen(p);
+  if (early) fetch(k_first);
+  pdl_wait();                 // the producer of this kernel's inputs has completed
+  pdl_launch_dependents();    // the next kernel may begin its start-up
+  if (!early) fetch(k_first);
+  for (int k0 = k_first;;) {
+    float a[kLoads];
+    const float* x = A + k0 * oa.stride;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        w[u] = __ldg(B + (k + u) * b_sk + n);
-        a[u] = __ldg(A + (k + u) * a_sk);
+    for (int u = 0; u < kLoads; ++u) {
+      a[u] = k0 + u * kStep < k_end ? __ldg(x) : 0.0f;
+      x += kStep * oa.stride;
+    }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u)
+      if (k0 + u * kStep < k_end) {               // (an infinite or NaN element of neither operand may meet a row that is not there)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(a[u], w[u][e], acc[e]);
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc = fmaf(a[u], w[u], acc);
-    }
-    for (; k < k_hi; ++k) acc = fmaf(__ldg(A + k * a_sk), __ldg(B + k * b_sk + n), acc);
+    k0 += kGemvRows;
+    if (k0 - lane / kLanes >= k_end) break;       // (the same for all lanes)
+    fetch(k0);
   }
-  part[warp][lane] = acc;
+  // the rows that a warp has read side by side
+#pragma unroll
+  for (int d = kLanes; d < 32; d *= 2)
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], d);
+  if (lane < kLanes) {
+    if constexpr (VEC == 4) *reinterpret_cast<float4*>(&part[warp][lane * 4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    else part[warp][lane] = acc[0];
+  }
   __syncthreads();
   if (threadIdx.x < kGemvCols) {
     const int64_t gn = (int64_t)blockIdx.x * kGemvCols + threadIdx.x;
     if (gn < p.N) {
-      float t = 0.0f;
+      float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-      for (int w = 0; w < kGemvWarps; ++w) t += part[w][threadIdx.x];
-      epilogue_store(p, t, b, 0, gn);
+      for (int i = 0; i < kGemvWarps; ++i) t[i & 3] += part[i][threadIdx.x];
+      gemv_store(p, (t[0] + t[1]) + (t[2] + t[3]), b, gn);
     }
   }
 }
@@ -160,13 +225,40 @@ void fill_matmul_params(const PlanKernel& k, MatmulParams* p) {
   p->tape = k.tape;
 }
 
+static void launch_gemv(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
+  const int a_slot = k.desc.a_slot, b_slot = k.desc.b_slot;
+  const dim3 grid((unsigned)((k.N + kGemvCols - 1) / kGemvCols), 1, (unsigned)k.batch), block(kGemvWarps * 32);
+  const DevOperand& B = k.ops[b_slot];
+  const bool vec = k.N % 4 == 0 && B.stride[1] % 4 == 0 && B.stride[0] % 4 == 0 && reinterpret_cast<uintptr_t>(B.ptr) % 16 == 0;
+  if (!k.has_chain) {
+    MatmulParams p{};
+    fill_matmul_params(k, &p);
+    launch_kernel(plan.pdl, vec ? mm_gemv_kernel<MatmulParams, 4> : mm_gemv_kernel<MatmulParams, 1>, grid, block, 0, s, p);
+    return;
+  }
+  GemvParams g{};
+  auto operand = [&](int slot, int d) { return GemvOperand{k.ops[slot].ptr, k.ops[slot].stride[0], k.ops[slot].stride[d]}; };
+  g.N = k.N;
+  g.K = k.K;
+  g.a = operand(a_slot, 2);
+  g.b = operand(b_slot, 1);
+  g.out = operand(k.chain.out_slot, 2);
+  g.frozen = k.desc.operands[b_slot].base_kind == KB200_BASE_CONST ? 1 : 0;
+  g.n_steps = k.chain.n;
+  for (int i = 0; i < k.chain.n; ++i) {
+    g.op[i] = k.chain.steps[i].op;
+    g.imm[i] = k.chain.steps[i].imm;
+    if (k.chain.steps[i].slot >= 0) g.side[i] = operand(k.chain.steps[i].slot, 2);
+  }
+  launch_kernel(plan.pdl, vec ? mm_gemv_kernel<GemvParams, 4> : mm_gemv_kernel<GemvParams, 1>, grid, block, 0, s, g);
+}
+
 int launch_matmul_simt(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
-  MatmulParams p{};
-  fill_matmul_params(k, &p);
   if (k.impl == IMPL_MM_GEMV) {
-    dim3 grid((unsigned)((p.N + kGemvCols - 1) / kGemvCols), 1, (unsigned)p.batch);
-    launch_kernel(plan.pdl, mm_gemv_kernel, grid, dim3(kGemvWarps * 32), 0, s, p);
+    launch_gemv(plan, k, s);
   } else {
+    MatmulParams p{};
+    fill_matmul_params(k, &p);
     const int64_t big_tiles = ((p.M + 127) / 128) * ((p.N + 127) / 128) * p.batch;
     if (big_tiles >= plan.sm_count) {
       dim3 grid((unsigned)(((p.M + 127) / 128) * ((p.N + 127) / 128)), 1, (unsigned)p.batch);
