@@ -60,6 +60,7 @@ struct EwChainParams {
   // 2^s >= d, exact for x < 2^31.
   uint32_t magic[kVecRank];
   int shift[kVecRank];
+  int stream_out;                // a large result that only the caller reads: see streams_out
   float* ptr[KB200_MAX_OPERANDS];
   // element strides as 32-bit numbers (the host takes this kernel only when every offset fits),
   // the innermost one already multiplied by VEC: VEC (an access per index) or 0 (one scalar per row)
@@ -135,7 +136,11 @@ __global__ void __launch_bounds__(256) ew_chain_kernel(const __grid_constant__ E
       if (!live[u]) continue;
       float* out = p.ptr[p.chain.out_slot] + ew_offset<RANK>(p, p.chain.out_slot, idx[u]);
       if (VEC == 1) *out = v[u];
-      else *reinterpret_cast<float4*>(out) = make_float4(v[VEC * u], v[VEC * u + 1], v[VEC * u + 2], v[VEC * u + VEC - 1]);
+      else {
+        const float4 t = make_float4(v[VEC * u], v[VEC * u + 1], v[VEC * u + 2], v[VEC * u + VEC - 1]);
+        if (p.stream_out) __stcs(reinterpret_cast<float4*>(out), t);
+        else *reinterpret_cast<float4*>(out) = t;
+      }
     }
   }
 }
@@ -373,6 +378,7 @@ static void launch_chain(const Plan& plan, const PlanKernel& k, cudaStream_t s) 
     for (int i = 0; i < rank; ++i) p.stride[o][i] = (int32_t)(k.ops[o].stride[i] * (i == rank - 1 ? VEC : 1));
   }
   p.chain = k.chain;
+  p.stream_out = streams_out(k, k.chain.out_slot, numel_of(d)) ? 1 : 0;
   int64_t blocks = ((int64_t)p.nvec + 256 * U - 1) / (256 * U);
   // beyond the cap every block takes the same number of grid-stride steps (no ragged last wave)
   const int64_t cap = (int64_t)plan.sm_count * 64;

@@ -212,6 +212,13 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
+// Is this output a result that only the caller reads, and large (an eighth of L2 or more)?  It is then written so that it
+// leaves L2 first: the next call's inputs and weights are read again, it is not.  (bias + GELU 2048 x 3072, 25 MB in and out,
+// calls on several tensors in turn: 11.5 -> 10.6 us.)
+inline bool streams_out(const PlanKernel& k, int slot, int64_t elems) {
+  return slot >= 0 && slot < k.desc.n_operands && k.desc.operands[slot].base_kind == KB200_BASE_OUTPUT && elems >= (int64_t(4) << 20);
+}
+
 inline int64_t numel_of(const kb200_kernel_desc& d) {
   int64_t n = 1;
   for (int i = 0; i < d.iter_rank; ++i) n *= d.iter_shape[i];

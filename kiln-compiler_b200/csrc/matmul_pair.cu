@@ -97,6 +97,7 @@ struct PairParams {
   // epilogue
   int64_t M, N;
   __nv_bfloat16* out16;  // bf16 mirror of the output (same strides), or null
+  int stream_out;        // the float32 output leaves L2 first: see streams_out
   int store32;           // 0: only the mirror is stored (every reader of this output takes the mirror)
   int slots, slot_bytes;
   int res_step;          // chain step whose operand arrives by bulk tensor load, or -1
@@ -389,6 +390,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
     int col_step = -1;
     for (int s = 0; s < n_steps && col_step < 0; ++s)
       if (chain_steps[s].kind == SIDE_COL) col_step = s;
+    const uint64_t out_policy = l2_policy(p.stream_out != 0);
     float col_pre[kPairBlocksPerWarp];
 #pragma unroll
     for (int j = 0; j < kPairBlocksPerWarp; ++j) col_pre[j] = 0.0f;
@@ -584,7 +586,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         fence_async_smem();
         __syncwarp();
         if (lane == 0 && !dry) {
-          if (with32) tma_store_3d(&tma_out, slot0, n, m_first, batch);
+          if (with32) tma_store_3d(&tma_out, slot0, n, m_first, batch, out_policy);
           if (with16) tma_store_3d(&tma_out16, slot0 + (with32 || has_res ? 4096u : 0u), n, m_first, batch);
           tma_store_commit();
         }
@@ -847,6 +849,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   p.N = k.N;
   p.out16 = out16;
   p.store32 = store32 ? 1 : 0;
+  p.stream_out = streams_out(k, k.chain.out_slot, k.batch * k.M * k.N) ? 1 : 0;
   p.slot_bytes = slot_bytes_wanted;
   p.slots = 1;
   const int stage_bytes = kps * (kPairATileBytes + p.half_bn * 128);
