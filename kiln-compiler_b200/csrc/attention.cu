@@ -114,10 +114,12 @@ struct AttnState {
   float* tails = nullptr;          // tails (x minus its 19 leading bits) of the span of the QKV buffer the views cover
   const float* span_lo = nullptr;
   int64_t span_n4 = 0;
+  bool tails_ready = false;        // ... written by the projection in front
+  bool own_pass = false;           // ... always by a pass of this launch's own: the kernel was asked for, not chosen
 };
 
 // tails[i] = src[i] minus its 19 leading bits (what a TF32 operand keeps): the second terms of the
-// split products of the FP32-mode tensor-core attention.
+// split products of the FP32-mode tensor-core attention, where the projection in front does not write them itself.
 __global__ void __launch_bounds__(256) tails_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int64_t n4) {
   pdl_wait();                 // the producer of Q, K and V has completed
   pdl_launch_dependents();
@@ -957,7 +959,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     const int64_t tc_ns = 6800 + 2400 * q_tiles * ((B * H * q_tiles + sms - 1) / sms) + B * T * 3 * H * hd * 8 / 6500;
     st->exact_tc = !c.ieee && T % kRows == 0 && B * H * q_tiles * 4 >= sms && tc_ns <= fma_ns;
     if (plan.fp32_attention == 1) st->exact_tc = false;
-    if (plan.fp32_attention == 2) st->exact_tc = true;
+    if (plan.fp32_attention == 2) st->exact_tc = st->own_pass = true;
   }
   if ((!c.exact || st->exact_tc) && (!encode_map_heads(&st->map_q, false, c.q, hd, T, H, B, rs, 32, kRows, false) ||
                                      !encode_map_heads(&st->map_k, false, c.k, hd, T, H, B, rs, 32, kRows, false) ||
@@ -1336,8 +1338,9 @@ int attention_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   const bool split = st->params.split_from < st->params.q_tiles;     // some query tiles are shared by two CTAs
   if (st->exact_tc) {
     const int64_t blocks = (st->span_n4 + 255) / 256;
-    KB200_CUDA(launch_kernel(plan.pdl, tails_kernel, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), dim3(256), 0, s,
-                             reinterpret_cast<const float4*>(st->span_lo), reinterpret_cast<float4*>(st->tails), st->span_n4));
+    if (!st->tails_ready)
+      KB200_CUDA(launch_kernel(plan.pdl, tails_kernel, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), dim3(256), 0, s,
+                               reinterpret_cast<const float4*>(st->span_lo), reinterpret_cast<float4*>(st->tails), st->span_n4));
     // (the store maps are not used by this instantiation)
     if (split)
       KB200_CUDA(launch_kernel(plan.pdl, attention_kernel<true, true>, st->grid, dim3(kAttnThreads), kExactSmemBytes, s, st->map_q,
@@ -1464,7 +1467,7 @@ void attention_elide_copy(Plan& plan, size_t first) {
   }
   for (auto& [k, slot] : redirect) k->ops[slot].ptr = st->staged_out;
   st->final_out = nullptr;
-  holder.launches = 1 + (st->exact_tc ? 1 : 0);
+  holder.launches = 1 + (st->exact_tc && !st->tails_ready ? 1 : 0);
 }
 
 bool attention_may_drop_float32(const PlanKernel& k) {
@@ -1472,6 +1475,16 @@ bool attention_may_drop_float32(const PlanKernel& k) {
   return st && st->bf16 && st->params.out16 != nullptr;
 }
 void attention_drop_float32(PlanKernel& k) { static_cast<AttnState*>(k.attn)->params.out32 = false; }
+
+float* attention_tails(const PlanKernel& k) {
+  const AttnState* st = static_cast<const AttnState*>(k.attn);
+  return st && !st->own_pass ? st->tails : nullptr;
+}
+void attention_tails_come_ready(PlanKernel& k) {
+  AttnState* st = static_cast<AttnState*>(k.attn);
+  if (!st->tails_ready) --k.launches;
+  st->tails_ready = true;
+}
 
 bool attention_reads_mirror(const PlanKernel& k) { return k.attn && static_cast<const AttnState*>(k.attn)->bf16; }
 

@@ -99,6 +99,7 @@ struct PlanKernel {
   void* shadow_out = nullptr;     // producer side: mirror address of this kernel's (single) output, or null
   const void* a_shadow = nullptr; // consumer side: mirror address of operand A / B, or null (convert per launch)
   const void* b_shadow = nullptr;
+  float* tail_out = nullptr;      // FP32: where the tails of the output (what a TF32 operand drops) go as well, same offsets, or null
   bool mirror_only = false;       // producer side: every reader of the output takes the mirror, the float32 store is dropped
   // An elementwise kernel that only continues the matmul in front of it (the activation or the residual
   // add behind a Linear on a [batch, tokens, d] input, which the reference's fusion pass cannot put into
@@ -179,6 +180,9 @@ int attention_try_fuse(Plan& plan, size_t first);    // plan kernels replaced fr
 int attention_chain_length(const PlanKernel& k);
 bool attention_wants_bf16(const PlanKernel& k);
 bool attention_reads_mirror(const PlanKernel& k);
+float* attention_tails(const PlanKernel& k);            // FP32 on the tensor cores: the tails of Q, K and V, or null
+void attention_tails_come_ready(PlanKernel& k);         // ... which the projection writes
+bool matmul_writes_tails(const PlanKernel& k);
 bool attention_may_drop_float32(const PlanKernel& k);    // writes a bf16 copy, and its float32 rows only where they were planned
 void attention_drop_float32(PlanKernel& k);
 bool tc_eligible(const PlanKernel& k);

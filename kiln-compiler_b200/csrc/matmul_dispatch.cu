@@ -10,6 +10,7 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s);
 void tc_destroy(PlanKernel& k);
 bool tc_repoint(PlanKernel& k);
 std::string tc_detail(const PlanKernel& k);
+bool tc_writes_tails(const PlanKernel& k);
 
 int choose_matmul(Plan& plan, PlanKernel& k) {
   (void)plan;
@@ -43,6 +44,8 @@ int launch_matmul(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
 bool repoint_matmul(PlanKernel& k) { return tc_repoint(k); }
 
 std::string matmul_detail(const PlanKernel& k) { return tc_detail(k); }
+
+bool matmul_writes_tails(const PlanKernel& k) { return k.impl == IMPL_MM_TC && tc_writes_tails(k); }
 
 void destroy_matmul(PlanKernel& k) { tc_destroy(k); }
 

@@ -75,6 +75,7 @@ struct SmallParams {
   int a_rows;                      // rows of a box of A: the tile's, or M where that is less
   float* out;                      // null: only the bf16 copy is stored
   __nv_bfloat16* out16;            // or null
+  float* out_tail;                 // exact FP32: the output minus its 19 leading bits, for a consumer that splits it, or null
   int64_t out_row;                 // of both
   int vectors;                     // exact FP32: 0 where N or a row's start is off float4: bias, residual and output element by element
 };
@@ -119,6 +120,9 @@ __device__ __forceinline__ void park_rows(uint8_t* slab, const float (&raw)[BF16
   }
 }
 
+// What a TF32 operand does not hold of x.
+__device__ __forceinline__ float dropped_bits(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
+
 // Exact FP32: an infinite operand makes a NaN of its tail's products (inf x 0, inf - inf) where float32 has an infinity.  Results
 // that are NaN, of rows m, m + rows_apart, ... below m_end and columns n to n + 3, done over as the CUDA cores do them.
 template <int FIN>
@@ -136,6 +140,7 @@ __device__ __noinline__ void redo_in_float32(const SmallParams& p, int m, int m_
       if (FIN == FIN_BIAS_GELU) y = d_gelu_tanh(y);
       if (FIN == FIN_BIAS_RES) y += p.res[(int64_t)m * p.res_row + c];
       *out = y;
+      if (p.out_tail != nullptr) p.out_tail[(int64_t)m * p.out_row + c] = dropped_bits(y);
     }
   }
 }
@@ -539,6 +544,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           continue;
         }
         if (p.out != nullptr) *reinterpret_cast<float4*>(p.out + (int64_t)m * p.out_row + n) = y;
+        if (EXACT && p.out_tail != nullptr)
+          *reinterpret_cast<float4*>(p.out_tail + (int64_t)m * p.out_row + n) = make_float4(dropped_bits(y.x), dropped_bits(y.y), dropped_bits(y.z), dropped_bits(y.w));
         if (p.out16 != nullptr) {
           __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
           uint2 packed;
@@ -841,6 +848,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
   p.out = k.mirror_only && p.out16 ? nullptr : O.ptr;
   p.out_row = O.stride[1];
+  p.out_tail = mode == SMALL_EXACT && vectors ? k.tail_out : nullptr;
   const DevOperand& A = k.ops[d.a_slot];
   p.a = gather || mode == SMALL_EXACT ? A.ptr : nullptr;
   const DevOperand& B = k.ops[d.b_slot];
@@ -910,6 +918,8 @@ std::string small_detail(const void* state) {
   return "mm_small " + std::to_string(st->bn) + " columns, " + std::to_string(st->params.splits) + " splits, " + std::to_string(st->params.stages) +
          " stages" + a + (st->drains ? ", drains" : "");
 }
+
+bool small_writes_tails(const void* state) { return static_cast<const SmallState*>(state)->params.out_tail != nullptr; }
 
 void small_destroy(void* state) { delete static_cast<SmallState*>(state); }
 

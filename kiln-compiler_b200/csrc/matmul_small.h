@@ -20,6 +20,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
 int small_launch(const Plan& plan, const void* state, cudaStream_t s);
 bool small_repoint(const PlanKernel& k, void* state);     // the operand pointers of `k` have moved
 std::string small_detail(const void* state);
+bool small_writes_tails(const void* state);
 void small_destroy(void* state);
 
 }  // namespace kb200

@@ -1489,6 +1489,11 @@ std::string tc_detail(const PlanKernel& k) {
   return "mm_tc " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.splits) + " splits" + copies;
 }
 
+bool tc_writes_tails(const PlanKernel& k) {
+  const TcState* st = static_cast<const TcState*>(k.tc);
+  return st && st->small && small_writes_tails(st->small);
+}
+
 void tc_destroy(PlanKernel& k) {
   TcState* st = static_cast<TcState*>(k.tc);
   if (!st) return;

@@ -790,6 +790,46 @@ static void absorb_elementwise(Plan& plan) {
   }
 }
 
+// The latest kernel before `ki` that writes into the span x: returned when it is one that can also
+// emit bf16 (LayerNorm, tensor-core matmul, fused attention) and its output covers x inside the arena.
+static PlanKernel* mirroring_producer(Plan& plan, size_t ki, const Span& x) {
+  const float* arena_lo = plan.arena;
+  const float* arena_hi = plan.arena + plan.arena_bytes / 4;
+  for (size_t j = ki; j-- > 0;) {
+    PlanKernel& pj = plan.kernels[j];
+    if (pj.impl == IMPL_FUSED_AWAY) continue;
+    const DevOperand* out = nullptr;
+    int64_t out_elems = 0;
+    bool whole = true;
+    if (pj.impl == IMPL_ATTN_FUSED) {
+      out = attention_output(plan, j, &out_elems);
+    } else if (pj.impl == IMPL_ROW_LAYERNORM && pj.desc.iter_rank == 2) {
+      out = &pj.ops[pj.out_slot];
+      out_elems = (pj.desc.iter_shape[0] - 1) * out->stride[0] + pj.desc.iter_shape[1];
+      whole = writes_whole_span(pj, pj.out_slot);
+    } else if (pj.impl == IMPL_MM_TC && pj.has_chain) {
+      out = &pj.ops[pj.chain.out_slot];
+      out_elems = (pj.batch - 1) * out->stride[0] + (pj.M - 1) * out->stride[1] + (pj.N - 1) * out->stride[2] + 1;
+      whole = writes_whole_span(pj, pj.chain.out_slot);
+    } else {
+      // some other kernel: does it write into the operand at all?
+      bool writes = false;
+      for (int t = 0; t < pj.desc.n_tape; ++t)
+        if (pj.desc.tape[t].opcode == KB200_OP_STORE) {
+          const Span w = span_of(pj, pj.desc.tape[t].b);
+          writes = writes || (w.lo < x.hi && x.lo < w.hi);
+        }
+      if (writes) return nullptr;      // written by a kernel that cannot emit bf16: keep the conversion pass
+      continue;
+    }
+    const Span w{out->ptr, out->ptr + out_elems};
+    if (!(w.lo < x.hi && x.lo < w.hi)) continue;                 // does not touch the operand
+    if (whole && w.lo <= x.lo && w.hi >= x.hi && w.lo >= arena_lo && w.hi <= arena_hi) return &pj;
+    return nullptr;
+  }
+  return nullptr;
+}
+
 // For every BF16 tensor-core matmul operand that lives in the arena: if the last kernel that wrote
 // that memory covers it completely and can also emit bf16, let it write the bf16 mirror and let the
 // matmul read the mirror.  Anything else keeps the per-launch conversion pass.
@@ -797,43 +837,6 @@ static int assign_shadows(Plan& plan) {
   const float* arena_lo = plan.arena;
   const float* arena_hi = plan.arena + plan.arena_bytes / 4;
   bool any = false;
-  // The latest kernel before `ki` that writes into the span x: returned when it is one that can also
-  // emit bf16 (LayerNorm, tensor-core matmul, fused attention) and its output covers x inside the arena.
-  auto mirroring_producer = [&](size_t ki, const Span& x) -> PlanKernel* {
-    for (size_t j = ki; j-- > 0;) {
-      PlanKernel& pj = plan.kernels[j];
-      if (pj.impl == IMPL_FUSED_AWAY) continue;
-      const DevOperand* out = nullptr;
-      int64_t out_elems = 0;
-      bool whole = true;
-      if (pj.impl == IMPL_ATTN_FUSED) {
-        out = attention_output(plan, j, &out_elems);
-      } else if (pj.impl == IMPL_ROW_LAYERNORM && pj.desc.iter_rank == 2) {
-        out = &pj.ops[pj.out_slot];
-        out_elems = (pj.desc.iter_shape[0] - 1) * out->stride[0] + pj.desc.iter_shape[1];
-        whole = writes_whole_span(pj, pj.out_slot);
-      } else if (pj.impl == IMPL_MM_TC && pj.has_chain) {
-        out = &pj.ops[pj.chain.out_slot];
-        out_elems = (pj.batch - 1) * out->stride[0] + (pj.M - 1) * out->stride[1] + (pj.N - 1) * out->stride[2] + 1;
-        whole = writes_whole_span(pj, pj.chain.out_slot);
-      } else {
-        // some other kernel: does it write into the operand at all?
-        bool writes = false;
-        for (int t = 0; t < pj.desc.n_tape; ++t)
-          if (pj.desc.tape[t].opcode == KB200_OP_STORE) {
-            const Span w = span_of(pj, pj.desc.tape[t].b);
-            writes = writes || (w.lo < x.hi && x.lo < w.hi);
-          }
-        if (writes) return nullptr;      // written by a kernel that cannot emit bf16: keep the conversion pass
-        continue;
-      }
-      const Span w{out->ptr, out->ptr + out_elems};
-      if (!(w.lo < x.hi && x.lo < w.hi)) continue;                 // does not touch the operand
-      if (whole && w.lo <= x.lo && w.hi >= x.hi && w.lo >= arena_lo && w.hi <= arena_hi) return &pj;
-      return nullptr;
-    }
-    return nullptr;
-  };
   std::vector<size_t> attention_readers;
   for (size_t ki = 0; ki < plan.kernels.size(); ++ki) {
     PlanKernel& k = plan.kernels[ki];
@@ -842,7 +845,7 @@ static int assign_shadows(Plan& plan) {
       // projection can write them so
       Span x{nullptr, nullptr};
       if (attention_operand_span(k, &x.lo, &x.hi) && x.lo >= arena_lo && x.hi <= arena_hi && (x.lo - arena_lo) % 8 == 0) {
-        if (PlanKernel* pj = mirroring_producer(ki, x)) {
+        if (PlanKernel* pj = mirroring_producer(plan, ki, x)) {
           pj->shadow_out = reinterpret_cast<void*>(1);
           attention_readers.push_back(ki);
           any = true;
@@ -859,7 +862,7 @@ static int assign_shadows(Plan& plan) {
       // the mirror is read through TMA: 16-byte aligned base and strides in 2-byte elements
       const DevOperand& xo = k.ops[slot];
       if ((x.lo - arena_lo) % 8 || xo.stride[0] % 8 || xo.stride[1] % 8 || xo.stride[2] % 8 && xo.stride[2] != 1) continue;
-      if (PlanKernel* pj = mirroring_producer(ki, x)) {
+      if (PlanKernel* pj = mirroring_producer(plan, ki, x)) {
         pj->shadow_out = reinterpret_cast<void*>(1);                // marked; the address is filled in below
         (role == 0 ? k.a_shadow : k.b_shadow) = reinterpret_cast<const void*>(1);
         any = true;
@@ -1130,6 +1133,7 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     k.shadow_out = nullptr;
     k.a_shadow = k.b_shadow = nullptr;
     k.mirror_only = false;
+    k.tail_out = nullptr;
     k.absorbed_by = -1;
     k.n_ops = k.desc.n_operands;
     rc = resolve(plan, k, (int)i);
@@ -1155,6 +1159,16 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   if (rc == KB200_OK) rc = assign_shadows(plan);
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i)
     if (plan.kernels[i].impl == IMPL_ATTN_FUSED) attention_elide_copy(plan, i);
+  // FP32 attention on the tensor cores: the projection that wrote exactly Q, K and V can write their tails as well
+  for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
+    Span x{nullptr, nullptr};
+    float* tails = plan.kernels[i].impl == IMPL_ATTN_FUSED ? attention_tails(plan.kernels[i]) : nullptr;
+    if (tails == nullptr || !attention_operand_span(plan.kernels[i], &x.lo, &x.hi)) continue;
+    PlanKernel* const from = mirroring_producer(plan, i, x);
+    if (from == nullptr || from->impl != IMPL_MM_TC) continue;
+    const Span w = span_of(*from, from->chain.out_slot);
+    if (w.lo == x.lo && w.hi == x.hi) from->tail_out = tails;
+  }
   // phase 4: tensor maps, packed weights, split-K workspaces.  What FP32 and TF32 matmuls add to make operands quicker to read
   // (a weight along K, its tails, aligned rows, the tails of A) takes a quarter of what is free in all, beside
   // a call's outputs; each on its own was allowed that much, and a plan of many Linears left nothing for its caller.
@@ -1177,6 +1191,10 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     PlanKernel& k = plan.kernels[i];
     if (k.desc.kclass == KB200_K_MATMUL && k.impl != IMPL_FUSED_AWAY) rc = bind_matmul(plan, k);
   }
+  for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i)
+    for (const PlanKernel& k : plan.kernels)
+      if (plan.kernels[i].impl == IMPL_ATTN_FUSED && k.tail_out != nullptr && k.tail_out == attention_tails(plan.kernels[i]) && matmul_writes_tails(k))
+        attention_tails_come_ready(plan.kernels[i]);
   cudaSetDevice(prev);
   if (rc) return rc;
   collect_io_refs(plan);
