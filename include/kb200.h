@@ -226,7 +226,10 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * estimates to be quickest, where it covers a matmul: tile columns (64, 96 or 128) + 1000 * K splits (1, 2, 4 or 8)
  * + 10000 * (1 + how A comes, if not through a tensor map of its own: 0 a copy, 1 as float32 for BF16, 2 read by the
  * kernel's warps); a part that is 0 is left to the estimate, a form that the matmul cannot take to the other
- * kernels. */
+ * kernels.
+ * KB200_OPT_OTHERS_IN_FLIGHT (default 0): 1 = other plans run on this GPU at the same time, each with the whole of it
+ * (KB200_OPT_CONCURRENCY 1): the last round of a matmul's tiles is then filled by them, and the tile width goes by the work
+ * of all tiles instead of by rounds.  Results are the same bits. */
 typedef enum kb200_option {
   KB200_OPT_FUSE_ATTENTION = 1,
   KB200_OPT_DEPENDENT_LAUNCH = 2,
@@ -237,7 +240,8 @@ typedef enum kb200_option {
   KB200_OPT_FP32_ATTENTION = 7,
   KB200_OPT_ATTENTION_SPLIT = 8,
   KB200_OPT_WEIGHT_COPIES = 9,
-  KB200_OPT_FEW_TILES = 10
+  KB200_OPT_FEW_TILES = 10,
+  KB200_OPT_OTHERS_IN_FLIGHT = 11
 } kb200_option;
 int kb200_plan_set_option(kb200_plan* plan, int option, int value);
 

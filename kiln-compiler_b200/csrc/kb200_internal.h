@@ -129,6 +129,7 @@ struct Plan {
   bool pdl = true;               // programmatic dependent launch: a kernel's start-up overlaps its predecessor's tail
   bool absorb_elementwise = true; // a tensor-core matmul also runs the elementwise kernel that only continues it
   bool mirror_only = true;       // BF16 mode: an output that only mirror readers consume is not stored as float32
+  bool others_in_flight = false; // KB200_OPT_OTHERS_IN_FLIGHT
   int concurrency = 1;           // plans the caller keeps in flight on this GPU at once (tile heuristics assume their share of the SMs)
   void* arena16 = nullptr;       // bf16 mirror of the arena (library-owned, only when some matmul reads it)
   uint64_t arena16_bytes = 0;

@@ -747,7 +747,10 @@ PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, int64_
     const int64_t tiles = ((k.M + 255) / 256) * ((k.N + w.bn - 1) / w.bn) * k.batch;
     const int64_t rounds = (tiles + share - 1) / share;
     const int slab_cycles = w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
-    const int64_t cycles = rounds * slabs * slab_cycles + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    // (Other plans fill a launch's last round and run under its drains, and the tile that moves least for its work also takes the least
+    // power: the step of 64 contexts, eight modules in flight, 1377 us by rounds, mostly 192 columns, 1352 with 256.)
+    const bool by_work = plan.others_in_flight && plan.concurrency == 1 && tiles >= share;
+    const int64_t cycles = by_work ? tiles * slabs * slab_cycles / share + 6300 : rounds * slabs * slab_cycles + 6300 + (int64_t)w.bn * 128 * 4 / 20;
     if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
     // K in halves on twice the pairs: the exchange of half a tile costs ~2500, and half as much is left to drain
     if (w.bn % 64 || w.bn == 128 || plan.concurrency > 1 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;

@@ -1209,6 +1209,7 @@ KB200_EXPORT int kb200_plan_set_option(kb200_plan* p, int option, int value) {
     case KB200_OPT_FUSE_ATTENTION: plan.fuse_attention = value != 0; return KB200_OK;
     case KB200_OPT_DEPENDENT_LAUNCH: plan.pdl = value != 0; return KB200_OK;
     case KB200_OPT_FOLD_OPERAND_COPIES: plan.fold_copies = value != 0; return KB200_OK;
+    case KB200_OPT_OTHERS_IN_FLIGHT: plan.others_in_flight = value != 0; return KB200_OK;
     case KB200_OPT_CONCURRENCY: plan.concurrency = value < 1 ? 1 : value; return KB200_OK;
     case KB200_OPT_ABSORB_ELEMENTWISE: plan.absorb_elementwise = value != 0; return KB200_OK;
     case KB200_OPT_MIRROR_ONLY: plan.mirror_only = value != 0; return KB200_OK;

@@ -37,6 +37,7 @@ OPT_FP32_ATTENTION = 7
 OPT_ATTENTION_SPLIT = 8
 OPT_WEIGHT_COPIES = 9
 OPT_FEW_TILES = 10
+OPT_OTHERS_IN_FLIGHT = 11
 BASE_KINDS = {"arena": 0, "const": 1, "input": 2, "output": 3}
 PRECISIONS = {"fp32": 0, "tf32": 1, "bf16": 2}
 OPCODES = {

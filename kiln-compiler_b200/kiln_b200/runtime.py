@@ -436,6 +436,8 @@ class StreamedBatch:
                 raise ValueError("StreamedBatch captures the launches itself: build the executables with cuda_graphs=False")
         self.executables = list(executables)
         for e in self.executables:
+            # (a hint only, before the plan is bound again: the last round of a matmul's tiles is filled by the other modules)
+            _cabi.check(e._lib.kb200_plan_set_option(e._plan, _cabi.OPT_OTHERS_IN_FLIGHT, int(len(self.executables) > 1)), e._lib)
             e.set_concurrency(len(self.executables) if concurrency is None else concurrency)
         self.device = executables[0].device
         self.streams = [torch.cuda.Stream(device=self.device) for _ in executables]
