@@ -16,7 +16,7 @@
 //     probabilities mends that for 2.5 us more.)  Nothing crosses between threads: no barrier among the softmax warps.
 //   * 112 KB of shared memory: two tiles each of Q, K and V, a 4 KB staging slot per softmax warp.
 // 32-key blocks above the diagonal are not computed (3/8 of a diagonal tile's exponentials); an item's rows are finished behind
-// the first exponentials of the next.  Eight sequences of 1024 tokens and 12 heads: 39.4 us with one query tile per SM, 27.8 now
+// the first exponentials of the next.  Eight sequences of 1024 tokens and 12 heads: 39.4 us with one query tile per SM, 27.5 now
 // (the exponentials alone: 11.3); 2048 tokens of one sequence 22.6 -> 20.9, six sequences of 333 tokens 9.3 -> 8.5.
 //
 // 192 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 softmax, one per tensor-memory lane quadrant.  CTAs are
@@ -156,9 +156,10 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   pdl_launch_dependents();
   const uint32_t tmem = tmem_base_slot;
   volatile int* abort_ptr = &abort_flag;
-  // A wait that ends for all lanes of the warp or none; where it runs out the CTA gives up.
+  // A wait that ends for all lanes of the warp or none; where it runs out the CTA gives up.  (The form that suspends: beside another
+  // CTA's exponentials, polling warps take its issue slots, 27.9 us for eight sequences of 1024 tokens, 27.5 so.)
   auto wait = [&](uint32_t bar, uint32_t parity, int site) {
-    const bool got = mbar_wait(bar, parity, abort_ptr);
+    const bool got = mbar_wait_cluster(bar, parity, abort_ptr);
     if (!got && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | site); *abort_ptr = 1; }
     return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
   };
