@@ -245,15 +245,12 @@ class GPUExecutable:
         copies = os.environ.get("KILN_GPU_WEIGHT_COPIES", "1") not in ("0", "false", "False", "")
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_WEIGHT_COPIES, int(copies)), self._lib)
         self._bind()
+        self.shares = (1, False)
         # launch_names: one per device launch of the plan (k3_matmul, k2_ew0 ...); kernel_names: the Kiln
         # kernels they come from, which is what CompiledModule.profile keys on (kiln/api.py:204-211)
         self.launch_names = [l.name for l in program.launches]
         self.kernel_names = list(dict.fromkeys(l.kernel for l in program.launches))
-        self.impls = [self._lib.kb200_kernel_impl(self._plan, i).decode() for i in range(len(program.launches))]
-        self.details = [self._lib.kb200_kernel_detail(self._plan, i).decode() for i in range(len(program.launches))]
-        # fused scalar steps per element of every launch as bound (a matmul that took over the kernel behind it shows more)
-        self.chain_lengths = [self._lib.kb200_kernel_chain_length(self._plan, i) for i in range(len(program.launches))]
-        self.device_launches = self._lib.kb200_plan_launch_count(self._plan)
+        self._read_plan()
         self.graph = None
         self.use_cuda_graphs = bool(cuda_graphs)
         self.relocatable = bool(self._lib.kb200_plan_relocatable(self._plan))
@@ -274,12 +271,27 @@ class GPUExecutable:
             _cabi.check(self._lib.kb200_plan_bind(self._plan, self.arena.data_ptr(), self.arena.numel(),
                                                   cp, cs, cn, ip, is_, in_, op, os_, on), self._lib)
 
-    def set_concurrency(self, plans_in_flight):
+    def set_concurrency(self, plans_in_flight, others=False):
         """Tell the library how many plans share the GPU at once (a hint for its tile heuristics:
-        each matmul then counts on its share of the SMs and prefers fewer, wider tiles); re-binds."""
+        each matmul then counts on its share of the SMs and prefers fewer, wider tiles), or, with
+        ``others``, that other plans run beside this one and each has the whole GPU; re-binds.
+        ``set_concurrency(1)`` is a plan that runs alone, as it is when it is built."""
+        self.shares = None
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_CONCURRENCY, int(plans_in_flight)), self._lib)
+        _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_OTHERS_IN_FLIGHT, int(bool(others))), self._lib)
         self._bind()
+        self.shares = (int(plans_in_flight), bool(others))
+        self._read_plan()
         self.graph = None
+
+    def _read_plan(self):
+        """What the plan, as it is bound now, runs."""
+        launches = range(len(self.program.launches))
+        self.impls = [self._lib.kb200_kernel_impl(self._plan, i).decode() for i in launches]
+        self.details = [self._lib.kb200_kernel_detail(self._plan, i).decode() for i in launches]
+        # fused scalar steps per element of every launch as bound (a matmul that took over the kernel behind it shows more)
+        self.chain_lengths = [self._lib.kb200_kernel_chain_length(self._plan, i) for i in launches]
+        self.device_launches = self._lib.kb200_plan_launch_count(self._plan)
 
     def _launch(self):
         stream = torch.cuda.current_stream(self.device).cuda_stream
@@ -435,14 +447,20 @@ class StreamedBatch:
             if e.use_cuda_graphs:
                 raise ValueError("StreamedBatch captures the launches itself: build the executables with cuda_graphs=False")
         self.executables = list(executables)
-        for e in self.executables:
-            # (a hint only, before the plan is bound again: the last round of a matmul's tiles is filled by the other modules)
-            _cabi.check(e._lib.kb200_plan_set_option(e._plan, _cabi.OPT_OTHERS_IN_FLIGHT, int(len(self.executables) > 1)), e._lib)
-            e.set_concurrency(len(self.executables) if concurrency is None else concurrency)
+        self.concurrency = len(self.executables) if concurrency is None else concurrency
+        self._tell(len(self.executables))
         self.device = executables[0].device
         self.streams = [torch.cuda.Stream(device=self.device) for _ in executables]
         self.graph = None
         self.requests = 0
+
+    def _tell(self, requests):
+        """Tell the plans about each other (a step of one request has no other module beside it); those that
+        know are not bound again, so that graphs captured over them stay good."""
+        shares = (self.concurrency, min(requests, len(self.executables)) > 1)
+        for e in self.executables:
+            if e.shares != shares:
+                e.set_concurrency(*shares)
 
     def _enqueue(self, sources, sinks, kernels=True):
         cur = torch.cuda.current_stream(self.device)
@@ -469,6 +487,7 @@ class StreamedBatch:
         for t in list(sources) + list(sinks):
             if not t.is_cuda and not t.is_pinned():
                 raise ValueError("host tensors of a StreamedBatch must be pinned")
+        self._tell(len(sources))
         with torch.cuda.device(self.device):
             side = torch.cuda.Stream(device=self.device)
             side.wait_stream(torch.cuda.current_stream(self.device))
