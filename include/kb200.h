@@ -201,7 +201,8 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * KB200_OPT_CONCURRENCY (default 1): how many plans the caller keeps in flight on this GPU at the
  * same time (a server overlapping requests on several streams).  Only a hint for the tile
  * heuristics, which the reference leaves to its autotuner (kiln/gpu/codegen.py:563-598): with n > 1 a
- * matmul counts on 1/n of the SMs and prefers fewer, wider tiles.  Results do not depend on it.
+ * matmul counts on 1/n of the SMs and prefers fewer, wider tiles.  A matmul's results do not depend on it; with n > 1 the fused
+ * attention shares no query tiles between CTAs (KB200_OPT_ATTENTION_SPLIT), which adds up in another order.
  * KB200_OPT_ABSORB_ELEMENTWISE (default 1): an elementwise kernel that directly follows a tensor-core
  * matmul and only continues it -- its one arena input is exactly the matmul's output, which nothing
  * else reads -- runs as the tail of the matmul's epilogue, and the matmul writes that kernel's output.
@@ -229,7 +230,7 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * kernels.
  * KB200_OPT_OTHERS_IN_FLIGHT (default 0): 1 = other plans run on this GPU at the same time, each with the whole of it
  * (KB200_OPT_CONCURRENCY 1): the last round of a matmul's tiles is then filled by them, and the tile width goes by the work
- * of all tiles instead of by rounds.  Results are the same bits. */
+ * of all tiles instead of by rounds.  Results do not depend on it. */
 typedef enum kb200_option {
   KB200_OPT_FUSE_ATTENTION = 1,
   KB200_OPT_DEPENDENT_LAUNCH = 2,

@@ -736,33 +736,59 @@ int resident_quads(const Plan& plan) {
 struct PairWidth { int bn, busy_cycles, light_cycles; };      // cycles of a slab with most of the pairs at work | with at most three quarters
 constexpr PairWidth kPairWidths[] = {{256, 553, 553}, {224, 490, 482}, {192, 433, 408}, {160, 395, 362}, {128, 365, 325}};
 
-PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, int64_t share, bool b_kmajor) {
-  const bool bf16 = k.desc.precision == KB200_PREC_BF16;
-  const int slab_k = bf16 ? 64 : 32, chunk_n = bf16 ? 64 : 32;
-  const int64_t slabs = (k.K + slab_k - 1) / slab_k;
+int64_t slabs_of(const PlanKernel& k) {
+  const int slab_k = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;
+  return (k.K + slab_k - 1) / slab_k;
+}
+int64_t tiles_of(const PlanKernel& k, const PairWidth& w) { return ((k.M + 255) / 256) * ((k.N + w.bn - 1) / w.bn) * k.batch; }
+bool width_fits(const PlanKernel& k, const PairWidth& w, bool b_kmajor) {
+  const int chunk_n = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;      // an N-major B comes in whole chunks of columns
+  return !(w.bn > 128 && w.bn / 2 >= k.N) && (b_kmajor || w.bn / 2 % chunk_n == 0);
+}
+int64_t slab_cycles(const PairWidth& w, int64_t tiles, int64_t share, bool two_slabs) {
+  return w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
+}
+
+// A launch that has the GPU to itself.  What decides the order of a matmul's sums -- whether K goes in halves, and by these cycles
+// whether another kernel runs it -- is said here, by its shape and the GPU alone: results must not depend on plans in flight.
+PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, bool b_kmajor) {
+  const int64_t share = plan.sm_count / 2, slabs = slabs_of(k);
   PairPlan best{0, false, 0};
   for (const PairWidth& w : kPairWidths) {
-    if (w.bn > 128 && w.bn / 2 >= k.N) continue;
-    if (!b_kmajor && w.bn / 2 % chunk_n) continue;         // an N-major B comes in whole chunks of columns
-    const int64_t tiles = ((k.M + 255) / 256) * ((k.N + w.bn - 1) / w.bn) * k.batch;
-    const int64_t rounds = (tiles + share - 1) / share;
-    const int slab_cycles = w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
-    // (Other plans fill a launch's last round and run under its drains, and the tile that moves least for its work also takes the least
-    // power: the step of 64 contexts, eight modules in flight, 1377 us by rounds, mostly 192 columns, 1352 with 256.)
-    const bool by_work = plan.others_in_flight && plan.concurrency == 1 && tiles >= share;
-    const int64_t cycles = by_work ? tiles * slabs * slab_cycles / share + 6300 : rounds * slabs * slab_cycles + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    if (!width_fits(k, w, b_kmajor)) continue;
+    const int64_t tiles = tiles_of(k, w);
+    const int64_t cycles = (tiles + share - 1) / share * slabs * slab_cycles(w, tiles, share, two_slabs) + 6300 + (int64_t)w.bn * 128 * 4 / 20;
     if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
     // K in halves on twice the pairs: the exchange of half a tile costs ~2500, and half as much is left to drain
-    if (w.bn % 64 || w.bn == 128 || plan.concurrency > 1 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
+    if (w.bn % 64 || w.bn == 128 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
     const int64_t halved = (slabs + 1) / 2 * (8 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles) + 6300 + 2500 + (int64_t)w.bn * 64 * 4 / 20;
     if (halved < best.cycles) best = {w.bn, true, halved};
   }
   return best;
 }
 
+// Tile width of a launch that shares the GPU, K in one go: any of them gives the same bits.  A plan with its share of the SM pairs goes
+// by rounds of those.  Where other plans run beside it on all of them, they fill its last round, so the work of its tiles counts, and the
+// tile that moves least for its work also takes the least power (the step of 64 contexts, eight modules in flight: 1377 us by
+// rounds, mostly 192 columns, 1352 with 256).  The last drain is charged only where tiles do not cover the pairs, each has one
+// and nothing to run under it: 2048 x 2304 x 768 TF32, four modules, 13.5 us at 192 columns (48 pairs, two tiles each), 14.4 at 256 (72 pairs); K = 256 7.8 and 9.8.
+int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool b_kmajor) {
+  const int64_t share = pair_share(plan), slabs = slabs_of(k);
+  int best = 0;
+  int64_t least = 0;
+  for (const PairWidth& w : kPairWidths) {
+    if (!width_fits(k, w, b_kmajor)) continue;
+    const int64_t tiles = tiles_of(k, w), slab = slab_cycles(w, tiles, share, two_slabs);
+    const bool by_work = plan.others_in_flight && plan.concurrency == 1 && tiles >= share;
+    const int64_t cycles = by_work ? tiles * slabs * slab / share + 6300 : (tiles + share - 1) / share * slabs * slab + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    if (best == 0 || cycles < least) best = w.bn, least = cycles;
+  }
+  return best;
+}
+
 }  // namespace
 
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, plan.sm_count / 2, b_kmajor).cycles; }
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, b_kmajor).cycles; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
@@ -806,9 +832,9 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   const int share = pair_share(plan);
   const int64_t slabs = (k.K + slab_k - 1) / slab_k;
   if (bn == 0) {
-    const PairPlan how = plan_pair(plan, k, kps != 1, share, ops.b_kmajor);
-    bn = how.bn;
+    const PairPlan how = plan_pair(plan, k, kps != 1, ops.b_kmajor);
     st->split = how.split && d.cfg[3] == 0 && kps != 2;
+    bn = st->split || (plan.concurrency == 1 && !plan.others_in_flight) ? how.bn : width_in_flight(plan, k, kps != 1, ops.b_kmajor);
   }
   while (bn == 256 && bn / 2 >= k.N) bn /= 2;
   // Staging per epilogue warp: one slot for a 32 x 32 block, float32 (also where a matrix operand of

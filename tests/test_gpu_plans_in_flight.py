@@ -50,3 +50,43 @@ def test_a_module_is_alone_again_after_a_step():
     modules[0].set_concurrency(1)
     assert modules[0].details == alone
     assert torch.equal(modules[0](xs[0])[0], want[0])
+
+
+def order_of_sums(detail):
+    """The kernel and its K splits, of a detail string."""
+    words = detail.replace(",", "").split()
+    return words[0], words[words.index("splits") - 1] if "splits" in words else "1"
+
+
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(2048, 768, 3072), (600, 2048, 2048), (1793, 708, 4100),          # K in halves
+                                   (9472, 160, 1024), (556, 3136, 128),                            # between two kernels
+                                   (1024, 3072, 768), (700, 4096, 4096), (1000, 1000, 772)])
+def test_the_order_of_sums_is_the_shape_s(m, n, k, precision):
+    exe, x = build(linear(m, n, k), precision)
+    want, alone = exe(x)[0], exe.details[0]
+    for plans, others in ((1, True), (2, False), (4, False), (8, False), (8, True)):
+        exe.set_concurrency(plans, others)
+        assert order_of_sums(exe.details[0]) == order_of_sums(alone), (plans, others, exe.details, alone)
+        assert torch.equal(exe(x)[0], want), (plans, others)
+
+
+@pytest.mark.parametrize("concurrency", [None, 1])
+def test_a_step_gives_the_bits_of_a_call(concurrency):
+    """An MLP of 2048 tokens, whose second matmul takes K in halves."""
+    from kiln_b200.runtime import StreamedBatch
+    from perf import cases
+
+    def mlp():
+        p = cases._Plan("mlp", (2048, 768), (2048, 768))
+        f = p.buffer(2048, 3072)
+        p.linear(p.x, "0.", 3072, f, gelu=True)
+        p.linear(f, "2.", 768, p.y)
+        return p
+
+    made = [build(mlp(), "tf32", seed) for seed in range(3)]
+    assert "2 splits" in made[0][0].details[1]
+    want = [e(x)[0] for e, x in made]
+    outs = [torch.empty_like(w) for w in want]
+    StreamedBatch([e for e, _ in made], concurrency=concurrency).capture([x for _, x in made], outs).run()
+    assert all(torch.equal(a, b) for a, b in zip(outs, want))
