@@ -109,7 +109,7 @@ struct AttnState {
   bool exact_tc = false;           // ... on the tensor cores (enough work items to fill the GPU), else the CUDA-core kernel
   AttnF32Params f32;
   void* f32_scratch = nullptr;     // CUDA-core kernel: the split tiles' partial results and arrival counters
-  void* split_scratch = nullptr;   // tensor-core kernels: the same for their split tiles
+  void* split_scratch = nullptr;   // tensor-core kernels: the same for their split tiles, and what CTAs keep between runs of key tiles
   CUtensorMap map_qt, map_kt, map_vt;   // tensor-core FP32 kernel: Q, K, V views of the tails buffer
   float* tails = nullptr;          // tails (x minus its 19 leading bits) of the span of the QKV buffer the views cover
   const float* span_lo = nullptr;
@@ -1062,14 +1062,17 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   } else if (!(c.exact && !st->exact_tc) && p.q_tiles >= 8 && B * H * p.q_tiles <= (c.exact ? 2 : 1) * (int64_t)plan.sm_count && may_split) {
     p.split_from = p.q_tiles / 2;
   }
-  if (p.split_from < p.q_tiles) {
+  p.kept = nullptr;
+  const std::vector<int> entries = attention_item_order(p.q_tiles, p.split_from);
+  const bool runs = c.bf16 && !aliased && attention_item_tiles(entries[0], p.split_from) > kAttnRun;
+  if (p.split_from < p.q_tiles || runs) {
     const int64_t split_tiles = B * H * (p.q_tiles - p.split_from);
     const size_t partial_bytes = (size_t)split_tiles * 2 * kAttnPartialFloats * sizeof(float);
     const size_t counter_bytes = (size_t)split_tiles * 4 * sizeof(int);
-    const std::vector<int> entries = attention_item_order(p.q_tiles, p.split_from);
     const std::vector<unsigned short> order(entries.begin(), entries.end());
     const size_t order_bytes = (order.size() * sizeof(unsigned short) + 15) & ~size_t(15);
-    if (cudaMalloc(&st->split_scratch, partial_bytes + counter_bytes + order_bytes) != cudaSuccess ||
+    const size_t kept_bytes = runs ? attention_bf16_ctas(st->alone, plan.sm_count) * kAttnPartialFloats * sizeof(float) : 0;
+    if (cudaMalloc(&st->split_scratch, partial_bytes + counter_bytes + order_bytes + kept_bytes) != cudaSuccess ||
         cudaMemset(static_cast<uint8_t*>(st->split_scratch) + partial_bytes, 0, counter_bytes) != cudaSuccess ||
         cudaMemcpy(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes, order.data(),
                    order.size() * sizeof(unsigned short), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -1083,6 +1086,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     p.partial = static_cast<float*>(st->split_scratch);
     p.arrivals = reinterpret_cast<int*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes);
     p.order = reinterpret_cast<const unsigned short*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes);
+    if (runs) p.kept = reinterpret_cast<float*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes + order_bytes);
   }
   const int64_t items = B * H * (p.q_tiles + (p.q_tiles - p.split_from));
   st->grid = dim3((unsigned)(items < plan.sm_count ? items : plan.sm_count), 1, 1);     // persistent: at most one CTA per SM
@@ -1416,7 +1420,7 @@ bool attention_use_mirror(const Plan& plan, PlanKernel& k, const float* arena_ba
   st->bf16 = true;
   if (st->params.out16 != nullptr && !encode_out16(st, st->params.out16)) st->params.out16 = nullptr;
   const int64_t items = B * H * (st->params.q_tiles + (st->params.q_tiles - st->params.split_from));
-  const int64_t ctas = (st->alone ? 1 : 2) * (int64_t)plan.sm_count;
+  const int64_t ctas = attention_bf16_ctas(st->alone, plan.sm_count);
   st->grid = dim3((unsigned)(items < ctas ? items : ctas), 1, 1);
   // D = F32, A/B = BF16: Q K^T both K-major, N = 128; P V with B N-major, N = 64; M = 128
   st->params.idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRows >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);

@@ -29,9 +29,11 @@ struct AttnParams {
   int split_from;            // query tiles from this one on are shared by two CTAs (q_tiles: none)
   float* partial;            // [split tile][2 halves][128 x 64 unnormalised output | 128 maxima | 128 sums]
   int* arrivals;             // [split tile][4 lane quadrants], zero between launches
+  float* kept;               // bf16 kernel, items of more than kAttnRun key tiles: [CTA][a partial like those above], or null
   const unsigned short* order;   // with split tiles: (query tile << 1 | half) of the q_tiles + split tiles entries, heaviest first
 };
 constexpr int kAttnPartialFloats = kAttnRows * kAttnHeadDim + 2 * kAttnRows;
+constexpr int kAttnRun = 16;                 // bf16 kernel: key tiles whose output adds up in tensor memory (see attention_bf16.cu)
 
 #ifdef __CUDACC__
 // A work item: one query tile of one head of one sequence, or (split tiles) one half of its key tiles.
@@ -85,6 +87,7 @@ __device__ __forceinline__ float ex2(float x) {
 // persistent CTAs pair a long item with a short one; query tiles from split_from on are two halves.
 std::vector<int> attention_item_order(int q_tiles, int split_from);
 int attention_item_tiles(int entry, int split_from);      // key tiles of an entry of that list
+inline int64_t attention_bf16_ctas(bool alone, int sms) { return (alone ? 1 : 2) * (int64_t)sms; }
 
 // How the kernel for bf16 operands spreads `heads` (sequences times heads) of q_tiles query tiles over the SMs.
 struct AttnSchedule {

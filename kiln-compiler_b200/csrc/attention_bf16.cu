@@ -14,6 +14,11 @@
 //     where it has grown by 2^8 would save 0.6 of 27.8 us, but the largest probability of a row would no longer be 1, which bf16
 //     holds exactly: error 2.4e-4 -> 3.3e-4 for rows that a few keys dominate.  The sum over the rounded
 //     probabilities mends that for 2.5 us more.)  Nothing crosses between threads: no barrier among the softmax warps.
+//   * The tensor core cuts off what does not fit a sum, once per 16 keys, so a sum that only ever grew there would be short by
+//     more the longer the sequence (values around 1, 16384 keys: 3.8e-5 short, error 6.1e-5; with rounded float32 additions 0.3e-5
+//     and 5.4e-5).  An item of more than kAttnRun key tiles (LONG) is therefore finished as often, and each thread adds its row to
+//     the one it keeps in a workspace of its CTA's in float32: 0.5e-5 and 5.4e-5, for 84.0 instead of 78.6 us at two
+//     sequences of 4096 tokens and 12 heads.
 //   * 112 KB of shared memory: two tiles each of Q, K and V, a 4 KB staging slot per softmax warp.
 // 32-key blocks above the diagonal are not computed (3/8 of a diagonal tile's exponentials); an item's rows are finished behind
 // the first exponentials of the next.  Eight sequences of 1024 tokens and 12 heads: 39.4 us with one query tile per SM, 27.5 now
@@ -112,7 +117,7 @@ __device__ __forceinline__ void probabilities(const float (&v)[128], uint32_t (&
   }
 }
 
-template <bool SPLIT>
+template <bool SPLIT, bool LONG>
 __global__ void __launch_bounds__(kThreads, 2)
 attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
@@ -244,7 +249,7 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       for (int j = 0; j < n_kv && ok; ++j, ++t) {
         if (j + 1 < n_kv) ok = issue_qk(t + 1, ii, false, j + 2 == n_kv);
         else if (w >= 0) ok = issue_qk(t + 1, ii + 1, true, n_next == 1);
-        ok = ok && issue_pv(t, j == 0);
+        ok = ok && issue_pv(t, LONG ? j % kAttnRun == 0 : j == 0);
       }
       n_kv = n_next;
     }
@@ -265,6 +270,7 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     int w = attn_nth_item(0, n_items);
     AttnItem it = attn_item<SPLIT>(p, w < 0 ? 0 : w), done = it;
     bool finished = false;                           // `done` is an item whose rows are still in tensor memory
+    bool done_adds = false, done_ends = true;        // LONG: the run that is finished is not the first, is the last of its item
     float m_run = 0.0f, l_run = 0.0f, m_done = 0.0f, l_done = 0.0f;
     while (true) {
       uint32_t packed[64];                           // two keys per 32-bit column
@@ -300,6 +306,9 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (j == 0) {
           m_run = mx;
           l_run = 0.0f;
+        } else if (LONG && j % kAttnRun == 0) {      // (the maximum goes on: a run of scores that are all -inf stays without weight)
+          m_run = fmaxf(m_run, mx);
+          l_run = 0.0f;
         } else {
           rescale = __any_sync(0xffffffffu, mx > m_run);
           if (rescale) {
@@ -334,10 +343,29 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           finished = false;
           float oa[32], ob[32];
           tmem_ld32x2(lane_addr + kColO, lane_addr + kColO + 32, oa, ob);
+          if constexpr (LONG) {
+            float* const kept = p.kept + (size_t)blockIdx.x * kAttnPartialFloats + row;      // (read back by the thread that wrote it)
+            if (done_adds) {
+              const float earlier = ex2(__ldcg(kept + kAttnRows * kAttnHeadDim) - m_done);
+              l_done = fmaf(__ldcg(kept + kAttnRows * kAttnHeadDim + kAttnRows), earlier, l_done);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) oa[i] = fmaf(__ldcg(kept + i * kAttnRows), earlier, oa[i]);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) ob[i] = fmaf(__ldcg(kept + (32 + i) * kAttnRows), earlier, ob[i]);
+            }
+            if (!done_ends) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) __stcg(kept + i * kAttnRows, oa[i]);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) __stcg(kept + (32 + i) * kAttnRows, ob[i]);
+              __stcg(kept + kAttnRows * kAttnHeadDim, m_done);
+              __stcg(kept + kAttnRows * kAttnHeadDim + kAttnRows, l_done);
+            }
+          }
           // ---- a split item: leave this half's rows and state in the workspace; whoever arrives second merges.
           // Nobody waits for the other half.  The arrival is counted per lane quadrant, which is one warp here.
-          bool writes = true;
-          if (SPLIT && done.split) {
+          bool writes = !LONG || done_ends;
+          if (SPLIT && done.split && writes) {
             float* const mine = p.partial + ((size_t)done.slot * 2 + done.half) * kAttnPartialFloats;
             const float* const other = p.partial + ((size_t)done.slot * 2 + (done.half ^ 1)) * kAttnPartialFloats;
             // a column of the 64 after the other: a warp's 32 rows are one line
@@ -412,11 +440,16 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       tmem_st_wait();
       arrive(p_full);
       ++t;
-      if (++j == it.n_kv) {
+      const bool ends = ++j == it.n_kv;
+      if (ends || (LONG && j % kAttnRun == 0)) {
         finished = true;
         done = it;
         m_done = m_run;
         l_done = l_run;
+        done_adds = j > kAttnRun;
+        done_ends = ends;
+      }
+      if (ends) {
         j = 0;
         w = attn_nth_item(++ii, n_items);
         if (w >= 0) it = attn_item<SPLIT>(p, w);
@@ -440,6 +473,12 @@ attention_bf16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kColumns) : "memory");
   }
+}
+
+using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, AttnParams);
+Kernel kernel_of(bool split, bool runs) {
+  return split ? (runs ? attention_bf16_kernel<true, true> : attention_bf16_kernel<true, false>)
+               : (runs ? attention_bf16_kernel<false, true> : attention_bf16_kernel<false, false>);
 }
 
 }  // namespace
@@ -500,14 +539,15 @@ AttnSchedule attention_bf16_schedule(int64_t heads, int q_tiles, int sms, bool m
 }
 
 bool attention_bf16_prepare() {
-  return cudaFuncSetAttribute(attention_bf16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone) == cudaSuccess &&
-         cudaFuncSetAttribute(attention_bf16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone) == cudaSuccess;
+  for (const bool split : {false, true})
+    for (const bool runs : {false, true})
+      if (cudaFuncSetAttribute(kernel_of(split, runs), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone) != cudaSuccess) return false;
+  return true;
 }
 
 cudaError_t attention_bf16_launch(bool pdl, dim3 grid, bool alone, cudaStream_t s, const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
                                   const CUtensorMap& out, const CUtensorMap& out16, const AttnParams& p) {
-  return launch_kernel(pdl, p.split_from < p.q_tiles ? attention_bf16_kernel<true> : attention_bf16_kernel<false>, grid, dim3(kThreads),
-                       alone ? kSmemAlone : kSmem, s, q, k, v, out, out16, p);
+  return launch_kernel(pdl, kernel_of(p.split_from < p.q_tiles, p.kept != nullptr), grid, dim3(kThreads), alone ? kSmemAlone : kSmem, s, q, k, v, out, out16, p);
 }
 
 }  // namespace kb200

@@ -8,14 +8,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("scale", [0.5, 4.0])
-@pytest.mark.parametrize("batch,tokens,heads", [(2, 2, 2), (2, 127, 2), (3, 129, 2), (6, 333, 12),          # one item per CTA
-                                                (2, 1024, 5), (2, 2048, 5),                                # query tiles in halves, alone and in pairs
-                                                (8, 1024, 12), (5, 900, 12), (16, 128, 20)])               # several items per CTA
-def test_attention_on_bf16_operands(batch, tokens, heads, scale):
-    """Q, K and V are columns of x times a power of two, so they are the same bf16 numbers here and there.  What is left is
-    the rounding of the probabilities to bf16 (2^-9 at most, 2^-9 / sqrt(3) = 1.1e-3 in the mean square, averaged by the sum over
-    the values; a row of one key has none) and float32 sums: 2e-3."""
+def attention(batch, tokens, heads, weight=None, bias=None):
+    """One matmul that makes Q, K and V of x, and the attention over them -> the executable, its mask."""
     from kiln_b200.codegen import program_from_plan
     from kiln_b200.runtime import GPUExecutable
     from perf import cases
@@ -35,22 +29,61 @@ def test_attention_on_bf16_operands(batch, tokens, heads, scale):
     p.bmm(w.as_((batch * heads, tokens, tokens)), v.as_((batch * heads, tokens, hd)), o)
     p.copy(o.as_((batch, tokens, heads, hd), (heads * tokens * hd, hd, tokens * hd, 1)), p.y)
     plan = p.spec()
-    rng = np.random.default_rng(0)
-    consts = cases._constants(plan.const_shapes, rng)
-    weight = np.zeros((d, 3 * d), np.float32)
-    weight[rng.integers(0, d, 3 * d), np.arange(3 * d)] = np.repeat([scale, scale, 1.0], d)
-    consts["weight.transpose"], consts["bias"] = weight, np.zeros(3 * d, np.float32)
+    consts = {"mask": cases._constants({"mask": (tokens, tokens)}, None)["mask"], "weight.transpose": weight,
+              "bias": np.zeros(3 * d, np.float32) if bias is None else bias}
     exe = GPUExecutable(program_from_plan(plan, "bf16"), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
     assert "attention_fused" in exe.impls
-    gen = torch.Generator(device="cuda").manual_seed(0)
-    x = torch.randn(batch * tokens, d, generator=gen, device="cuda").bfloat16().float()
+    return exe, torch.from_numpy(consts["mask"]).cuda().double()
+
+
+def columns_of_x(d, scale, values=1.0):
+    """Q, K (times a power of two) and V as columns of x: the same bf16 numbers here and in the reference."""
+    rng = np.random.default_rng(0)
+    weight = np.zeros((d, 3 * d), np.float32)
+    weight[rng.integers(0, d, 3 * d), np.arange(3 * d)] = np.repeat([scale, scale, values], d)
+    return weight
+
+
+def inputs(batch, tokens, heads):
+    return torch.randn(batch * tokens, 64 * heads, generator=torch.Generator(device="cuda").manual_seed(0), device="cuda").bfloat16().float()
+
+
+def exact(x, weight, mask, batch, tokens, heads):
+    q, k, v = (x.double() @ torch.from_numpy(weight).cuda().double()).view(batch, tokens, 3, heads, 64).permute(2, 0, 3, 1, 4)
+    for b in range(batch):
+        yield torch.stack([torch.softmax(q[b, h] @ k[b, h].T * 0.125 + mask, -1) @ v[b, h] for h in range(heads)])
+
+
+@pytest.mark.parametrize("scale", [0.5, 4.0])
+@pytest.mark.parametrize("batch,tokens,heads", [(2, 2, 2), (2, 127, 2), (3, 129, 2), (6, 333, 12),          # one item per CTA
+                                                (2, 1024, 5), (2, 2048, 5),                                # query tiles in halves, alone and in pairs
+                                                (8, 1024, 12), (5, 900, 12), (16, 128, 20),                # several items per CTA
+                                                (2, 2049, 2), (2, 4097, 2), (2, 2300, 40)])                # longer than a run of 16 key tiles
+def test_attention_on_bf16_operands(batch, tokens, heads, scale):
+    """What is left beside equal operands is the rounding of the probabilities to bf16 (2^-9 at most, 2^-9 / sqrt(3) = 1.1e-3 in the mean
+    square, averaged by the sum over the values; a row of one key has none) and float32 sums: 2e-3."""
+    weight = columns_of_x(64 * heads, scale)
+    exe, mask = attention(batch, tokens, heads, weight)
+    x = inputs(batch, tokens, heads)
     outs = [exe(x)[0] for _ in range(3)]
     exe.status()
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
-    mask = torch.from_numpy(consts["mask"]).cuda().double()
-    qkv = (x.double() @ torch.from_numpy(weight).cuda().double()).view(batch, tokens, 3, heads, hd).permute(2, 0, 3, 1, 4)
-    for b in range(batch):
-        want = torch.softmax(qkv[0, b] @ qkv[1, b].transpose(-1, -2) * 0.125 + mask, -1) @ qkv[2, b]
+    for b, want in enumerate(exact(x, weight, mask, batch, tokens, heads)):
         got = outs[0][b].permute(1, 0, 2).double()
         assert float((got - want).norm() / want.norm()) <= 2e-3
         assert float((got - want).abs().max() / want.abs().max()) <= 4e-3        # (every row: 2^-8)
+
+
+@pytest.mark.parametrize("split", ["0", "1"])
+def test_long_sums_are_not_cut_short(split, monkeypatch):
+    """One value for all keys: the result is that value, but for the probabilities' rounding (over 512 rows of 8064 keys and more: 1.1e-3 / sqrt(512 *
+    8064) = 6e-7) and for what the tensor core cuts off its sums, at most a unit in the last place (2^-23 to 2^-24 of the sum) per 16 keys, on average
+    half of one.  In runs of 2048 keys that is 128 x 2^-24 = 7.6e-6 at most on average; 8192 in one go are 3.1e-5."""
+    monkeypatch.setenv("KILN_GPU_ATTENTION_SPLIT", split)
+    batch, tokens, heads = 2, 8192, 2
+    d = 64 * heads
+    value = float(torch.tensor(1 / 3).bfloat16())
+    exe, _ = attention(batch, tokens, heads, columns_of_x(d, 0.5, 0.0), np.repeat(np.float32([0, 0, value]), d))
+    got = exe(inputs(batch, tokens, heads))[0].double()[:, -128:] / value - 1
+    exe.status()
+    assert abs(float(got.mean())) <= 7.6e-6
