@@ -499,10 +499,12 @@ int attention_item_tiles(int entry, int split_from) {
 }
 
 // Cycles from the first tile to the last of the longest SM, by walking the items the way the CTAs do.  Measured inside the
-// kernel: a key tile takes a CTA 2300 cycles when it has the SM to itself and 2900 beside another, an item 1000 more (its
-// rows' way out, its part of the copies' latency).  A half costs 6500 (rows and state to the workspace, fence, counter, the
-// other half's rows; one sequence of 256 tokens 5.7 -> 8.1 us), so only long items are worth it: 1024 tokens 12.3 -> 12.1 us,
-// 2048 tokens 21.7 -> 20.4.
+// kernel: a key tile takes a CTA 2300 cycles when it has the SM to itself, an item 1000 more (its
+// rows' way out, its part of the copies' latency).  Beside another CTA a tile counts as 3300 (2900 inside the loop): fitted with the
+// half's cost to 78 launches of 4 to 128 heads and 2 to 16 query tiles, every schedule of each timed.  The one it chooses is 0.5 % from
+// the best on average and 5 % at most.  (With 2900: 1.7 %; 24 heads of 1024 tokens 15.0 us with halves on two CTAs an SM,
+// 13.6 whole with one.)  A half costs 6500 (rows and state to the workspace, fence, counter, the other half's rows; one sequence
+// of 256 tokens 5.7 -> 8.1 us), so only long items are worth it: 1024 tokens 12.3 -> 12.1 us, 2048 tokens 21.7 -> 20.4.
 static int64_t schedule_cycles(int64_t heads, int q_tiles, int split_from, int sms, bool alone) {
   const std::vector<int> order = attention_item_order(q_tiles, split_from);
   const int64_t items = heads * (int64_t)order.size();
@@ -518,7 +520,7 @@ static int64_t schedule_cycles(int64_t heads, int q_tiles, int split_from, int s
     int64_t own = work[(size_t)i];
     if (!alone && i + sms < grid) {                  // the CTA beside it
       const int64_t other = work[(size_t)(i + sms)];
-      own = std::min(own, other) * 29 / 23 + (std::max(own, other) - std::min(own, other));
+      own = std::min(own, other) * 33 / 23 + (std::max(own, other) - std::min(own, other));
     }
     longest = std::max(longest, own);
   }

@@ -87,3 +87,13 @@ def test_long_sums_are_not_cut_short(split, monkeypatch):
     got = exe(inputs(batch, tokens, heads))[0].double()[:, -128:] / value - 1
     exe.status()
     assert abs(float(got.mean())) <= 7.6e-6
+
+
+@pytest.mark.parametrize("heads,split", [(12, False), (5, True)])
+def test_query_tiles_are_shared_where_sms_are_idle(heads, split, monkeypatch):
+    """24 heads of eight query tiles fill the SMs with whole tiles (13.6 us; halves of the long ones on two CTAs an SM 15.0); ten do not."""
+    x, weight = inputs(2, 1024, heads), columns_of_x(64 * heads, 0.5)
+    got = attention(2, 1024, heads, weight)[0](x)[0]
+    monkeypatch.setenv("KILN_GPU_ATTENTION_SPLIT", "0")
+    whole = attention(2, 1024, heads, weight)[0](x)[0]
+    assert torch.equal(got, whole) != split
