@@ -139,11 +139,12 @@ __global__ void __launch_bounds__(kGemvWarps * 32) mm_gemv_kernel(const __grid_c
   const int64_t b = blockIdx.z;
   const GemvOperand oa = gemv_a(p), ob = gemv_b(p);
   const int64_t n = (int64_t)blockIdx.x * kGemvCols + lane % kLanes * VEC;
-  const int K = (int)p.K, k_per = (K + kGemvWarps - 1) / kGemvWarps;
-  const int k_end = min((warp + 1) * k_per, K);
-  const int k_first = warp * k_per + lane / kLanes;
-  const float* const A = oa.ptr + b * oa.batch_stride;
-  const float* const B = ob.ptr + b * ob.batch_stride + n;
+  // this warp's part of K, counted from its first row: 32 bits are enough for that
+  const int64_t k_per = (p.K + kGemvWarps - 1) / kGemvWarps, k_lo = warp * k_per;
+  const int k_end = (int)(k_lo + k_per < p.K ? k_per : k_lo < p.K ? p.K - k_lo : 0);
+  const int k_first = lane / kLanes;
+  const float* const A = oa.ptr + b * oa.batch_stride + k_lo * oa.stride;
+  const float* const B = ob.ptr + b * ob.batch_stride + k_lo * ob.stride + n;
   const bool live = n < p.N;                      // (VEC = 4: N is a multiple of four)
   float w[kLoads][VEC], acc[VEC];
 #pragma unroll

@@ -34,3 +34,22 @@ def test_one_row(n, k, gelu):
     got, want = exe(x)[0], (x.double() @ w + b)
     assert torch.equal(torch.isinf(want), torch.isinf(got)) or gelu
     assert not bool(torch.isnan(got[torch.isposinf(want)]).any())
+
+
+@pytest.mark.parametrize("n", [4, 3])
+def test_more_rows_than_32_bits_count(n):
+    """2^31 + 4096 rows, all of them the same one (stride 0).  Every sum is a whole number of 2^-20, so those of a lane are exact to the 2^24th (n = 4: 2^24 + 32
+    rows) or stop growing there (n = 3: 2^26 + 128 rows in a lane): the results are that many rows, short of the lanes' remainders."""
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable
+    from perf import cases
+
+    k = 2**31 + 4096
+    p = cases._Plan("rows", (1, 1), (1, n))
+    p.kernel("matmul", [("matmul", [("operand", 0), ("operand", 1)], (1, n))], [p.x.as_((1, k), (0, 0)), p.const("w", 1, n).as_((k, n), (0, 1))], [(0, p.y)])
+    plan = p.spec()
+    exe = GPUExecutable(program_from_plan(plan, "fp32"), plan.arena_bytes, {"w": np.full((1, n), 2.0**-20, np.float32)}, plan.input_shapes, plan.output_shapes)
+    assert exe.impls == ["mm_gemv"]
+    got = exe(torch.ones(1, 1, device="cuda"))[0].double()
+    want = 32 * (4 * 2.0**24 if n == 4 else 2.0**24) * 2.0**-20
+    assert float((got / want - 1).abs().max()) <= 1e-5
