@@ -4,6 +4,8 @@
 // accumulator while it is still in registers, out-of-range tile elements read as 0 and are not
 // stored (codegen.py:513-517, 524).  tcgen05 has no IEEE-FP32 operand kind, so this is the path
 // for allow_tf32=False; it is also the fallback for operands the tensor-core path cannot take.
+#include <type_traits>
+
 #include "device_math.cuh"
 #include "kb200_internal.h"
 #include "matmul.h"
@@ -89,8 +91,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) mm_simt_kernel(const __
 // Decode shape, M == 1: the weight matrix is read exactly once, so the kernel is bound by how many
 // bytes it keeps in flight and by the latencies around that.  Each CTA owns 32 output columns; its 32 warps split K and
 // combine through shared memory in warp order, which keeps the result deterministic.  A warp reads four rows of 128 bytes per
-// instruction (VEC = 4; one where rows are off a 16-byte pitch), up to 24 rows at once: all of K = 768, 9.4 MB over the 96 CTAs of a
-// 3072-wide layer.  Those of a frozen weight are requested before the wait for the previous kernel, whose
+// instruction, up to 24 rows at once: all of K = 768, 9.4 MB over the 96 CTAs of a 3072-wide layer.  (Rows off a 16-byte pitch:
+// VEC = 1, one row per instruction, 16 at once.)  Those of a frozen weight are requested before the wait for the previous kernel, whose
 // tail they then arrive under.  The parameters are this kernel's own 0.4 KB: those of the general epilogue are 2.9 KB, which every
 // launch pays for on the host and again in a cold constant cache.
 constexpr int kGemvWarps = 32;
@@ -146,49 +148,65 @@ __global__ void __launch_bounds__(kGemvWarps * 32) mm_gemv_kernel(const __grid_c
   const float* const A = oa.ptr + b * oa.batch_stride + k_lo * oa.stride;
   const float* const B = ob.ptr + b * ob.batch_stride + k_lo * ob.stride + n;
   const bool live = n < p.N;                      // (VEC = 4: N is a multiple of four)
-  float w[kLoads][VEC], acc[VEC];
+  float acc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) acc[e] = 0.0f;
-  auto fetch = [&](int k0) {
-    const float* row = B + k0 * ob.stride;
+  if constexpr (VEC == 1) {
+    // A row is one load of the warp, so whole blocks of rows go without a test of each: with one, 1 x 3001 x 2048 took 10.2 us,
+    // 5.4 without; 1 x 4097 x 1537 10.2 and 4.7, 1 x 50257 x 768 60.5 and 47.8.
+    pdl_wait();
+    pdl_launch_dependents();
+    auto block = [&](int k, auto rows) {
+      constexpr int R = decltype(rows)::value;
+      float w[R], a[R];
 #pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      if (live && k0 + u * kStep < k_end) {
-        if constexpr (VEC == 4) {
-          const float4 t = __ldg(reinterpret_cast<const float4*>(row));
-          w[u][0] = t.x; w[u][1] = t.y; w[u][2] = t.z; w[u][3] = t.w;
-        } else {
-          w[u][0] = __ldg(row);
+      for (int u = 0; u < R; ++u) {
+        w[u] = __ldg(B + (k + u) * ob.stride);
+        a[u] = __ldg(A + (k + u) * oa.stride);
+      }
+#pragma unroll
+      for (int u = 0; u < R; ++u) acc[0] = fmaf(a[u], w[u], acc[0]);
+    };
+    if (live) {
+      int k = k_first;
+      for (; k + 16 <= k_end; k += 16) block(k, std::integral_constant<int, 16>{});
+      for (; k + 8 <= k_end; k += 8) block(k, std::integral_constant<int, 8>{});
+      for (; k < k_end; ++k) block(k, std::integral_constant<int, 1>{});
+    }
+  } else {
+    float w[kLoads][VEC];
+    auto fetch = [&](int k0) {
+      const float* row = B + k0 * ob.stride;
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const float4 t = live && k0 + u * kStep < k_end ? __ldg(reinterpret_cast<const float4*>(row)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w[u][0] = t.x; w[u][1] = t.y; w[u][2] = t.z; w[u][3] = t.w;
+        row += kStep * ob.stride;
+      }
+    };
+    const bool early = gemv_frozen(p);
+    if (early) fetch(k_first);
+    pdl_wait();                 // the producer of this kernel's inputs has completed
+    pdl_launch_dependents();    // the next kernel may begin its start-up
+    if (!early) fetch(k_first);
+    for (int k0 = k_first;;) {
+      float a[kLoads];
+      const float* x = A + k0 * oa.stride;
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        a[u] = k0 + u * kStep < k_end ? __ldg(x) : 0.0f;
+        x += kStep * oa.stride;
+      }
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u)
+        if (k0 + u * kStep < k_end) {               // (an infinite or NaN element of neither operand may meet a row that is not there)
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) acc[e] = fmaf(a[u], w[u][e], acc[e]);
         }
-      } else {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) w[u][e] = 0.0f;
-      }
-      row += kStep * ob.stride;
+      k0 += kGemvRows;
+      if (k0 - lane / kLanes >= k_end) break;       // (the same for all lanes)
+      fetch(k0);
     }
-  };
-  const bool early = gemv_frozen(p);
-  if (early) fetch(k_first);
-  pdl_wait();                 // the producer of this kernel's inputs has completed
-  pdl_launch_dependents();    // the next kernel may begin its start-up
-  if (!early) fetch(k_first);
-  for (int k0 = k_first;;) {
-    float a[kLoads];
-    const float* x = A + k0 * oa.stride;
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u) {
-      a[u] = k0 + u * kStep < k_end ? __ldg(x) : 0.0f;
-      x += kStep * oa.stride;
-    }
-#pragma unroll
-    for (int u = 0; u < kLoads; ++u)
-      if (k0 + u * kStep < k_end) {               // (an infinite or NaN element of neither operand may meet a row that is not there)
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(a[u], w[u][e], acc[e]);
-      }
-    k0 += kGemvRows;
-    if (k0 - lane / kLanes >= k_end) break;       // (the same for all lanes)
-    fetch(k0);
   }
   // the rows that a warp has read side by side
 #pragma unroll
