@@ -726,15 +726,24 @@ int resident_quads(const Plan& plan) {
   return known;
 }
 
-// Tile width and estimated cycles of the slowest SM pair: rounds of tiles, the cycles of a slab, ~20 bytes a clock to drain the
-// last tile, ~6300 for the rest.  A slab of 256 columns takes its 512 tensor cycles and a little; below that the 24 to 28 KB of
-// its operands' way from L2 take longer than the multiplying, more so with most SMs at it (an SM gets 60 to 75 bytes a
-// clock; two slabs per step at 128 columns, 490 with one).  Fitted to 2048 x 3072 x 768 and 2048 x 768 x 3072 in TF32.
-// The widths between 128 and 256 are for the last round: 2048 x 3072 x 768 TF32 20.2 us at 128 columns (three rounds, 64 of 74 pairs),
-// 22.2 at 256 (96 tiles), 18.3 at 192 (128 tiles, two rounds); 8192 x 768 x 3072 BF16 66.2 at 256, 59.5 at 192 (with its pass
+// Tile width and estimated cycles of a launch: 8000 once, and per round of tiles its drain and the cycles of its slabs, more of them the
+// more of the pairs are at work (one SM gets 60 to 75 bytes a clock from L2; a slab of 256 columns has 512 cycles of multiplying).
+// K in halves: the exchange and its own start instead.  Lines through 512 launches in TF32 and BF16, every width and both
+// forms of each timed: 160 to 4096 rows of sixteen weights from 256 x 1024 to 4096 x 4096.  The choice is 0.2 % (TF32) and 0.1 % (BF16)
+// from the best on average; the estimate before, through 2048 x 3072 x 768 and 2048 x 768 x 3072 in TF32, was 1.6 % and 1.2 %, with halves
+// 17 % slower than a tile of 128 columns where K is 512 to 2048 (1792 x 640 x 512 9.2 against 7.8 us).
+// The widths between 128 and 256 are for the last round: 2048 x 3072 x 768 TF32 21.2 us at 128 columns (three rounds, 64 of 74 pairs),
+// 23.5 at 256 (96 tiles), 19.5 at 192 (128 tiles, two rounds); 8192 x 768 x 3072 BF16 66.2 at 256, 59.5 at 192 (with its pass
 // over A); 8192 x 2304 x 768 36.1 at 256, 39.7 at 192.
-struct PairWidth { int bn, busy_cycles, light_cycles; };      // cycles of a slab with most of the pairs at work | with at most three quarters
-constexpr PairWidth kPairWidths[] = {{256, 553, 553}, {224, 490, 482}, {192, 433, 408}, {160, 395, 362}, {128, 365, 325}};
+struct PairWidth {
+  int bn;
+  int alone, full;                     // cycles of a slab with one pair at work | with all of them
+  int drain;                           // of a round
+  int half_alone, half_full, halves;   // K in halves: cycles of a slab, and of all that runs once (0: this width does not come in halves)
+};
+constexpr PairWidth kPairWidths[] = {
+    {256, 485, 637, 4310, 508, 627, 13270}, {224, 419, 566, 3730, 0, 0, 0}, {192, 354, 496, 3400, 380, 475, 11110}, {160, 292, 429, 3130, 0, 0, 0}, {128, 243, 406, 2400, 0, 0, 0}};
+constexpr int64_t kPairOnce = 8000, kPairHalvesBusy = 3320;      // (halves: with all pairs at work)
 
 int64_t slabs_of(const PlanKernel& k) {
   const int slab_k = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;
@@ -745,9 +754,8 @@ bool width_fits(const PlanKernel& k, const PairWidth& w, bool b_kmajor) {
   const int chunk_n = k.desc.precision == KB200_PREC_BF16 ? 64 : 32;      // an N-major B comes in whole chunks of columns
   return !(w.bn > 128 && w.bn / 2 >= k.N) && (b_kmajor || w.bn / 2 % chunk_n == 0);
 }
-int64_t slab_cycles(const PairWidth& w, int64_t tiles, int64_t share, bool two_slabs) {
-  return w.bn == 128 && !two_slabs ? 490 : 4 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles;
-}
+// (one slab per step: what a step costs on its own shows where it multiplies for less)
+int64_t one_slab(const PairWidth& w, bool two_slabs) { return w.bn == 128 && !two_slabs ? 125 : 0; }
 
 // A launch that has the GPU to itself.  What decides the order of a matmul's sums -- whether K goes in halves, and by these cycles
 // whether another kernel runs it -- is said here, by its shape and the GPU alone: results must not depend on plans in flight.
@@ -756,12 +764,14 @@ PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, bool b
   PairPlan best{0, false, 0};
   for (const PairWidth& w : kPairWidths) {
     if (!width_fits(k, w, b_kmajor)) continue;
-    const int64_t tiles = tiles_of(k, w);
-    const int64_t cycles = (tiles + share - 1) / share * slabs * slab_cycles(w, tiles, share, two_slabs) + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    const int64_t tiles = tiles_of(k, w), rounds = (tiles + share - 1) / share;
+    int64_t cycles = kPairOnce + rounds * (slabs * (w.alone + one_slab(w, two_slabs)) + w.drain) + slabs * (w.full - w.alone) * tiles / share;
+    // (Beyond ~80 us the GPU is at its power limit, where the bytes a tile moves for its work count: 4096^3 TF32 191 us at 256 columns, 201 at 192.)
+    if (cycles > 150000) cycles += cycles * (256 - w.bn) / 2560;
     if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
-    // K in halves on twice the pairs: the exchange of half a tile costs ~2500, and half as much is left to drain
-    if (w.bn % 64 || w.bn == 128 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
-    const int64_t halved = (slabs + 1) / 2 * (8 * tiles <= 3 * share ? w.light_cycles : w.busy_cycles) + 6300 + 2500 + (int64_t)w.bn * 64 * 4 / 20;
+    // K in halves on twice the pairs
+    if (w.halves == 0 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
+    const int64_t halved = w.halves + (slabs + 1) / 2 * w.half_alone + ((slabs + 1) / 2 * (w.half_full - w.half_alone) + kPairHalvesBusy) * 2 * tiles / share;
     if (halved < best.cycles) best = {w.bn, true, halved};
   }
   return best;
@@ -778,9 +788,9 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
   int64_t least = 0;
   for (const PairWidth& w : kPairWidths) {
     if (!width_fits(k, w, b_kmajor)) continue;
-    const int64_t tiles = tiles_of(k, w), slab = slab_cycles(w, tiles, share, two_slabs);
+    const int64_t tiles = tiles_of(k, w), slab = w.full + one_slab(w, two_slabs);
     const bool by_work = plan.others_in_flight && plan.concurrency == 1 && tiles >= share;
-    const int64_t cycles = by_work ? tiles * slabs * slab / share + 6300 : (tiles + share - 1) / share * slabs * slab + 6300 + (int64_t)w.bn * 128 * 4 / 20;
+    const int64_t cycles = by_work ? tiles * slabs * slab / share : (tiles + share - 1) / share * slabs * slab + w.drain;
     if (best == 0 || cycles < least) best = w.bn, least = cycles;
   }
   return best;
@@ -788,7 +798,9 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
 
 }  // namespace
 
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, b_kmajor).cycles; }
+// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9: of 288 launches that both take, the
+// choice is 0.1 % from the better one in BF16 and 0.1 % in TF32, 0.2 and 0.3 with the estimate before)
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, b_kmajor).cycles * 7 / 8; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
