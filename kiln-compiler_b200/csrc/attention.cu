@@ -809,13 +809,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) {
-    for (int s = 0; s < (EXACT ? 1 : 2); ++s)
-      for (uint32_t i = 0; i < 4096u; ++i)
-        if ((mbar_try_wait(k_full + 8 * s, 0) || mbar_try_wait(k_full + 8 * s, 1)) &&
-            (mbar_try_wait(v_full + 8 * s, 0) || mbar_try_wait(v_full + 8 * s, 1)))
-          break;
-  }
+  if (abort_flag && threadIdx.x == 0) let_copies_land();
   __syncthreads();
   if (warp == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -609,11 +609,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) {
-    // copies may still be in flight towards this CTA's shared memory: give them a bounded time to land
-    const long long t0 = clock64();
-    while (clock64() - t0 < 400000) { }
-  }
+  if (abort_flag && threadIdx.x == 0) let_copies_land();
   // neither CTA leaves (or frees TMEM the other's MMAs write) before both are done
   cluster_arrive();
   cluster_wait();

@@ -564,11 +564,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     cluster_arrive_relaxed();
   }
   // ---------------- exit ----------------
-  if (abort_flag && threadIdx.x == 0) {
-    // copies may still be in flight towards this CTA's shared memory: give them a bounded time to land
-    const long long t0 = clock64();
-    while (clock64() - t0 < 400000) { }
-  }
+  if (abort_flag && threadIdx.x == 0) let_copies_land();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   // Every CTA of the cluster has received everything: so every copy out of THIS shared memory has landed

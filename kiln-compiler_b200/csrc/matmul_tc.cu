@@ -803,12 +803,7 @@ mm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   // ---------------- common exit ----------------
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) {
-    // give copies that may still be in flight a bounded time to land before shared memory is released
-    for (int s = 0; s < p.stages; ++s)
-      for (uint32_t i = 0; i < 4096u; ++i)
-        if (mbar_try_wait(full0 + 8 * s, 0) || mbar_try_wait(full0 + 8 * s, 1)) break;
-  }
+  if (abort_flag && threadIdx.x == 0) let_copies_land();
   __syncthreads();
   if (warp == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -70,6 +70,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// What a CTA that gives up does before it releases its shared memory: copies may be in flight towards it, and a barrier does not say
+// whether any are (asked for either parity, one of the two answers is always yes).  They get 400000 cycles, 0.2 ms, to land.
+__device__ __forceinline__ void let_copies_land() {
+  const long long t0 = clock64();
+  while (clock64() - t0 < 400000) { }
+}
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
