@@ -378,7 +378,7 @@ static void launch_chain(const Plan& plan, const PlanKernel& k, cudaStream_t s) 
     for (int i = 0; i < rank; ++i) p.stride[o][i] = (int32_t)(k.ops[o].stride[i] * (i == rank - 1 ? VEC : 1));
   }
   p.chain = k.chain;
-  p.stream_out = streams_out(k, k.chain.out_slot, numel_of(d)) ? 1 : 0;
+  p.stream_out = streams_out(plan, k, k.chain.out_slot, numel_of(d)) ? 1 : 0;
   int64_t blocks = ((int64_t)p.nvec + 256 * U - 1) / (256 * U);
   // beyond the cap every block takes the same number of grid-stride steps (no ragged last wave)
   const int64_t cap = (int64_t)plan.sm_count * 64;

@@ -886,7 +886,7 @@ int pair_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& o
   p.N = k.N;
   p.out16 = out16;
   p.store32 = store32 ? 1 : 0;
-  p.stream_out = streams_out(k, k.chain.out_slot, k.batch * k.M * k.N) ? 1 : 0;
+  p.stream_out = streams_out(plan, k, k.chain.out_slot, k.batch * k.M * k.N) ? 1 : 0;
   p.slot_bytes = slot_bytes_wanted;
   p.slots = 1;
   const int stage_bytes = kps * (kPairATileBytes + p.half_bn * 128);

@@ -1058,10 +1058,11 @@ KB200_EXPORT int kb200_plan_create(const kb200_kernel_desc* descs, int n, int de
   KB200_CUDA(cudaGetDeviceCount(&count));
   if (device < 0 || device >= count) return fail(KB200_ERR_ARGUMENT, "kb200_plan_create: no CUDA device %d", device);
   // (three attributes: cudaGetDeviceProperties takes 3 ms)
-  int major = 0, minor = 0, sm_count = 0;
+  int major = 0, minor = 0, sm_count = 0, l2_bytes = 0;
   KB200_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
   KB200_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
   KB200_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+  KB200_CUDA(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
   if (major != 10)
     return fail(KB200_ERR_UNSUPPORTED, "kb200_plan_create: device %d is sm_%d%d; this library is built for sm_100a only",
                 device, major, minor);
@@ -1073,6 +1074,7 @@ KB200_EXPORT int kb200_plan_create(const kb200_kernel_desc* descs, int n, int de
   if (!plan) return fail(KB200_ERR_ARGUMENT, "kb200_plan_create: out of host memory");
   plan->device = device;
   plan->sm_count = sm_count;
+  plan->l2_bytes = l2_bytes;
   plan->kernels.resize(n);
   for (int i = 0; i < n; ++i) {
     PlanKernel& k = plan->kernels[i];
