@@ -97,3 +97,35 @@ def test_query_tiles_are_shared_where_sms_are_idle(heads, split, monkeypatch):
     monkeypatch.setenv("KILN_GPU_ATTENTION_SPLIT", "0")
     whole = attention(2, 1024, heads, weight)[0](x)[0]
     assert torch.equal(got, whole) != split
+
+
+@pytest.mark.parametrize("batch,tokens,heads", [(2, 700, 2), (3, 1024, 6), (8, 1024, 12), (2, 2300, 2)])
+def test_a_token_without_numbers(batch, tokens, heads):
+    """A token that is NaN makes its own rows and all later ones of its sequence NaN, whatever the maxima drop of it; the tiles of 128 queries
+    before it do not see it, nor does the next sequence."""
+    weight = columns_of_x(64 * heads, 0.5)
+    exe, _ = attention(batch, tokens, heads, weight)
+    x = inputs(batch, tokens, heads)
+    clean = exe(x)[0].clone()
+    for at in (0, 130, tokens - 1):
+        y = x.clone()
+        y[at, 0] = float("nan")                       # (through the zeros of the matmul: all of the token's Q, K and V)
+        got = exe(y)[0]
+        assert bool(torch.isnan(got[0, at:]).all())
+        assert torch.equal(got[0, :at // 128 * 128], clean[0, :at // 128 * 128]) and torch.equal(got[1:], clean[1:])
+    exe.status()
+
+
+@pytest.mark.parametrize("batch,tokens,heads", [(2, 700, 2), (3, 1024, 6), (2, 2300, 2)])
+def test_one_token_far_above_the_rest(batch, tokens, heads):
+    """A token of 1000s, 2e6 its own score: to each later query it is all or nothing."""
+    weight = columns_of_x(64 * heads, 0.5)
+    exe, mask = attention(batch, tokens, heads, weight)
+    x = inputs(batch, tokens, heads)
+    x[150] = 1000.0
+    got = exe(x)[0]
+    exe.status()
+    for b, want in enumerate(exact(x, weight, mask, batch, tokens, heads)):
+        want, have = want.permute(1, 0, 2), got[b].double()
+        assert float((have - want).norm() / want.norm()) <= 2e-3
+        assert float(((have - want).abs() / want.abs().amax(-1, keepdim=True)).max()) <= 8e-3      # (of its row's largest: 2^-8, and 2^-9 of each of the terms that make less of it)

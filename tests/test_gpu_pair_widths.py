@@ -92,3 +92,33 @@ def test_the_quicker_form_is_taken(m, n, k, precision, how):
     assert f"mm_pair {how}" in exe.details[0] and ("splits" in how) == ("splits" in exe.details[0]), exe.details
     want = x @ c["weight.transpose"] + c["bias"]
     assert float((got - want).norm() / want.norm()) <= BOUND[precision]
+
+
+@pytest.mark.parametrize("batch,m,n,k", [(2, 512, 768, 3072), (3, 300, 736, 2052)])
+def test_k_in_halves_of_a_batch_and_an_operand_along_n(batch, m, n, k):
+    """Batched, B an activation [K, N] in TF32: the second pair of a cluster starts in the middle of its rows."""
+    from perf import cases
+
+    p = cases._Plan("product", (batch * k, 128), (batch, m, n))
+    b = p.buffer(batch * k, n)
+    p.linear(p.x, "0.", n, b)
+    p.bmm(p.const("a", batch, m, k), b.as_((batch, k, n)), p.y)
+    exe, x, c, got = run(p, "tf32")
+    assert "mm_pair" in exe.details[1] and "2 splits" in exe.details[1], exe.details
+    want = c["a"] @ (x @ c["0.weight.transpose"] + c["0.bias"]).view(batch, k, n)
+    assert float((got - want).norm() / want.norm()) <= 2 * BOUND["tf32"]
+    assert float((got - want).abs().max() / want.std()) <= 20 * BOUND["tf32"]
+
+
+@pytest.mark.parametrize("m", [2048, 1990])
+def test_k_in_halves_where_only_the_bf16_copy_is_stored(m):
+    from perf import cases
+
+    p = cases._Plan("mlp", (m, 3072), (m, 768))
+    f = p.buffer(m, 768)
+    p.linear(p.x, "0.", 768, f)
+    p.linear(f, "2.", 768, p.y)
+    exe, x, c, got = run(p, "bf16")
+    assert "mm_pair" in exe.details[0] and "2 splits" in exe.details[0], exe.details
+    want = (x @ c["0.weight.transpose"] + c["0.bias"]) @ c["2.weight.transpose"] + c["2.bias"]
+    assert float((got - want).norm() / want.norm()) <= 2 * BOUND["bf16"]
