@@ -392,6 +392,7 @@ def roofline_of(built, precision, iters=10):
     launches per CUDA graph); roofline of the one with the largest share."""
     pk, pk_kind = peaks()
     exe, plan = built.exe, built.plan
+    exe.set_concurrency(1)      # (as it is bound for itself: the step's modules have each other beside them)
     times = exe.profile_launches(exe.static_inputs[0], iters=iters)
     total = sum(ms for _, ms in times)
     i = max(range(len(times)), key=lambda j: times[j][1])
@@ -741,7 +742,7 @@ def gpu_arm(args, dist, rank, world, local):
     # INFLIGHT compiled modules (own arena, static buffers and stream each) run round-robin, as a server
     # keeps several requests in flight: copies of one group overlap kernels of another.  A whole step of
     # 64 sequences is one CUDA graph, so a busy host does not starve the GPU of launches.  Every kernel
-    # of an eight-sequence graph is large enough for the whole GPU, so the plans are not told to share it.
+    # of an eight-sequence graph is large enough for the whole GPU, so the plans are told of each other but not to share it.
     built = Built(HEAD_CASE, precision)
     for _ in range(INFLIGHT - 1):
         built.another()

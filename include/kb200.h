@@ -188,8 +188,8 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * KB200_OPT_FUSE_ATTENTION (default 1): when the plan contains the reference's five-kernel
  * attention chain (K^T copy, QK^T * scale + causal mask, softmax, PV, head merge; see
  * tests/models/transformer.py:16-25 of the reference), or the seven-kernel chain of a batch of
- * sequences, run it as one fused kernel (in FP32 precision: with float32 products, behind a small
- * launch that prepares the operands' tails when the tensor cores are used).  The kernel list and
+ * sequences, run it as one fused kernel (in FP32 precision: with float32 products; on the tensor cores with the
+ * operands' tails, which the projection in front writes where it can, else a small launch).  The kernel list and
  * arena offsets stay the reference's; the score buffers are then never written.  0 keeps one launch
  * per planned kernel.
  * KB200_OPT_DEPENDENT_LAUNCH (default 1): kernels are enqueued with programmatic stream
@@ -209,14 +209,15 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * This is what the reference's plans contain behind every Linear on a [batch, tokens, d] input: its
  * fusion pass cannot take the activation or the residual add into the matmul's kernel across the
  * reshape between them (kiln/passes/fusion.py:26-35).  0 launches every planned kernel.
- * KB200_OPT_MIRROR_ONLY (default 1, BF16 mode): a LayerNorm or matmul whose output is read only by
+ * KB200_OPT_MIRROR_ONLY (default 1, BF16 mode): a LayerNorm, matmul or fused attention whose output is read only by
  * kernels that take its bf16 mirror (tensor-core matmul operands, the fused attention) does not store
  * the float32 values: that arena region then holds stale data, which no planned kernel reads.  0 stores
  * both, for a caller that inspects intermediate buffers.
  * KB200_OPT_FP32_ATTENTION (default 0, FP32 precision): which kernel runs the fused attention.
  * 0 = by size (the tensor-core kernel, three TF32 products per float32 product, for sequences of whole
  * tiles of 128 tokens whose work items fill a quarter of the SMs, where it is estimated faster and no
- * matmul of the chain asked for IEEE behaviour on non-finite operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores.
+ * matmul of the chain asked for IEEE behaviour on non-finite operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores, with
+ * the tails from a launch of its own (the same bits).
  * KB200_OPT_ATTENTION_SPLIT (default 1): in a launch that leaves SMs idle (one long sequence,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.

@@ -115,7 +115,7 @@ struct AttnState {
   const float* span_lo = nullptr;
   int64_t span_n4 = 0;
   bool tails_ready = false;        // ... written by the projection in front
-  bool own_pass = false;           // ... always by a pass of this launch's own: the kernel was asked for, not chosen
+  bool own_pass = false;           // ... always by a pass of this launch's own: asked for by option, the kernel runs by itself, whatever is in front
 };
 
 // tails[i] = src[i] minus its 19 leading bits (what a TF32 operand keeps): the second terms of the
@@ -744,7 +744,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (SPLIT && ok && it.split) {
         float* const mine = p.partial + ((size_t)it.slot * 2 + it.half) * kAttnPartialFloats;
         const float* const other = p.partial + ((size_t)it.slot * 2 + (it.half ^ 1)) * kAttnPartialFloats;
-        // a column of the 64 after the other: a warp's 32 rows are one line (row by row, 32 lines per store, it cost 0.9 us more)
+        // a column of the 64 after the other: a warp's 32 rows are one line (row by row, 32 lines per store, 1024 tokens took 26.3 us, 24.2 so)
 #pragma unroll
         for (int i = 0; i < 32; ++i) __stcg(mine + (group * 32 + i) * kRows + row, o[i]);
         if (group == 0) {

@@ -40,8 +40,8 @@ constexpr int kAttnRun = 16;                 // bf16 kernel: key tiles whose out
 struct AttnItem { int h, seq, q0, n_kv, qt, j0, half, slot; bool split; };
 
 // This CTA's r-th item (-1: none).  Items are ordered heaviest first; rounds alternate direction over the CTAs, so that
-// the CTA with the heaviest item of one round takes the lightest of the next (24 key tiles at most per CTA instead of
-// 27 for 8 x 12 x 8 items on 148 CTAs).
+// the CTA with the heaviest item of one round takes the lightest of the next (8 x 12 x 8 items: 24 key tiles at most per CTA instead of
+// 27 on 148 CTAs, 13 instead of 15 on 296).
 __device__ __forceinline__ int attn_nth_item(int r, int n_items) {
   const int w = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
   return w < n_items ? w : -1;

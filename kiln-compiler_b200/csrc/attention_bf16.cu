@@ -22,7 +22,7 @@
 //   * 112 KB of shared memory: two tiles each of Q, K and V, a 4 KB staging slot per softmax warp.
 // 32-key blocks above the diagonal are not computed (3/8 of a diagonal tile's exponentials); an item's rows are finished behind
 // the first exponentials of the next.  Eight sequences of 1024 tokens and 12 heads: 39.4 us with one query tile per SM, 27.5 now
-// (the exponentials alone: 11.3); 2048 tokens of one sequence 22.6 -> 20.9, six sequences of 333 tokens 9.3 -> 8.5.
+// (the exponentials alone: 11.3); 2048 tokens of one sequence 22.6 -> 20.9, six sequences of 333 tokens 9.4 -> 8.5.
 //
 // 192 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 softmax, one per tensor-memory lane quadrant.  CTAs are
 // persistent, items as in attention.cu.  Every wait is bounded (see matmul_tc.cu).

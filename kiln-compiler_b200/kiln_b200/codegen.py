@@ -91,8 +91,8 @@ def default_matmul_config(graph, kernel):
     """The configuration used without measuring (role of codegen.py:563-598).
 
     All zeros: the library then applies its own rule when buffers are bound -- with more than 128
-    rows, 256-row tiles on SM pairs (256 or 128 columns by a cost model of rounds, issue and
-    tensor time); otherwise the widest 128-row tile that still gives every SM a tile, and, when
+    rows, 256-row tiles on SM pairs (128 to 256 columns, K whole or in halves, by a cost model of
+    rounds, slabs and drains); otherwise the widest 128-row tile that still gives every SM a tile, and, when
     even that leaves SMs idle (128-token projections, 768-wide layers), a split of K so that every
     SM streams a share of the operands.  The autotuner searches around this default.
     """
