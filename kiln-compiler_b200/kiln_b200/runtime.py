@@ -460,6 +460,7 @@ class StreamedBatch:
         shares = (self.concurrency, min(requests, len(self.executables)) > 1)
         for e in self.executables:
             if e.shares != shares:
+                self.graph = None
                 e.set_concurrency(*shares)
 
     def _enqueue(self, sources, sinks, kernels=True):
