@@ -1,0 +1,219 @@
+// Exact FP32 on SM pairs: which matmuls, tile widths, launches.  The kernel and why it is built as it is: matmul_exact.cuh.
+#include <cuda.h>
+
+#include "kb200_internal.h"
+#include "matmul_exact.cuh"
+#include "matmul_exact.h"
+
+namespace kb200 {
+
+namespace {
+
+using ExactKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ExactParams);
+
+template <int BLOCKS, bool SPLIT>
+ExactKernel exact_kernel(int fin) {
+  switch (fin) {
+    case FIN_BIAS: return mm_exact_kernel<BLOCKS, FIN_BIAS, SPLIT>;
+    case FIN_BIAS_GELU: return mm_exact_kernel<BLOCKS, FIN_BIAS_GELU, SPLIT>;
+    case FIN_BIAS_RES: return mm_exact_kernel<BLOCKS, FIN_BIAS_RES, SPLIT>;
+    default: return mm_exact_kernel<BLOCKS, FIN_NONE, SPLIT>;
+  }
+}
+
+struct ExactState {
+  CUtensorMap map_a, map_b, map_out, map_res, map_tail;
+  ExactParams params;
+  ExactKernel kernel = nullptr;
+  size_t smem = 0;
+  unsigned grid = 0;
+  bool split = false;
+  int bias_slot = -1, res_slot = -1;
+};
+
+// The chains that are finished here: nothing, + column, + column then GELU, + column + matrix, all of it in float4 and 16-byte rows.
+int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot) {
+  const Chain& c = k.chain;
+  *bias_slot = *res_slot = -1;
+  if (c.n == 0) return FIN_NONE;
+  const ChainStep* s = c.steps;
+  if (s[0].op != CH_ADD || s[0].slot < 0) return -1;
+  const DevOperand& b = k.ops[s[0].slot];
+  if (b.stride[1] != 0 || b.stride[2] != 1 || !aligned16(b.ptr)) return -1;
+  *bias_slot = s[0].slot;
+  if (c.n == 1) return FIN_BIAS;
+  if (c.n != 2) return -1;
+  if (s[1].op == CH_GELU_TANH) return FIN_BIAS_GELU;
+  if (s[1].op != CH_ADD || s[1].slot < 0) return -1;
+  const DevOperand& r = k.ops[s[1].slot];
+  if (r.stride[2] != 1 || r.stride[1] < k.N || r.stride[1] % 4 || !aligned16(r.ptr)) return -1;
+  *res_slot = s[1].slot;
+  return FIN_BIAS_RES;
+}
+
+// Clusters of two pairs that fit the GPU at once.
+int resident_quads(const Plan& plan) {
+  int& known = plan.resident_exact_quads;
+  if (known == 0) {
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(plan.sm_count / 4 * 4), 1, 1);
+    cfg.blockDim = dim3(kExactThreads, 1, 1);
+    cfg.dynamicSmemBytes = kExactSmem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 4;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const ExactKernel kernel = mm_exact_kernel<2, FIN_BIAS, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExactSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    known = n > 0 ? n : -1;
+  }
+  return known;
+}
+
+struct ExactPlan { int bn; bool split; int64_t cycles; };
+
+// Tile width, whether K goes in halves and estimated cycles, the pass over A included: all that runs once, the steps of the rounds, what
+// they cost more the more of the pairs are at work, and per round its drain.  Lines through 419 launches: 160 to 4096 rows of eleven weights
+// from 256 x 1024 to 4096 x 1024, every width timed (2 to 4 % off in the mean square); the choice is 0.07 % from the best on average.  (A
+// step of 256 columns has 1536 cycles of multiplying, of 128 columns 768, and the operands come in at 48 KB: 1024 x 2304 x 768 16.3 us at 128
+// columns, 19.9 at 256; 4096 x 3072 x 768 54.1 at 256.)  Plans in flight are no argument: results must not depend on them.
+struct ExactWidth { int bn, once, step, busy, drain; };
+constexpr ExactWidth kExactWidths[] = {{256, 12560, 1497, 574, 4516}, {192, 12550, 1092, 496, 3039}, {160, 11270, 910, 342, 3575}, {128, 12065, 705, 374, 2543}};
+constexpr ExactWidth kExactHalves = {128, 14616, 733, 208, 1695};        // K in halves on twice the pairs
+
+ExactPlan plan_exact(const Plan& plan, int64_t m, int64_t n, int64_t k) {
+  const int64_t pairs = plan.sm_count / 2, steps = (k + kExactStepK - 1) / kExactStepK, pass = m * k / 714;
+  ExactPlan best{0, false, 0};
+  for (const ExactWidth& w : kExactWidths) {
+    if (w.bn > 128 && w.bn / 2 >= n) continue;
+    const int64_t tiles = ((m + 255) / 256) * ((n + w.bn - 1) / w.bn), rounds = (tiles + pairs - 1) / pairs;
+    const int64_t cycles = w.once + pass + rounds * (steps * w.step + w.drain) + steps * w.busy * tiles / pairs;
+    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
+  }
+  const ExactWidth& h = kExactHalves;
+  const int64_t tiles = ((m + 255) / 256) * ((n + h.bn - 1) / h.bn), half = (steps + 1) / 2;
+  if (steps >= 4 && tiles <= resident_quads(plan)) {
+    const int64_t cycles = h.once + pass + half * h.step + (half * h.busy + h.drain) * 2 * tiles / pairs;
+    if (cycles < best.cycles) best = {h.bn, true, cycles};
+  }
+  return best;
+}
+
+}  // namespace
+
+int64_t exact_cycles(const Plan& plan, const PlanKernel& k) {
+  const kb200_kernel_desc& d = k.desc;
+  int bias_slot, res_slot;
+  if (!k.has_chain || k.batch != 1 || k.M <= 128 || k.N < 128 || k.N % 4 || finish_of(k, &bias_slot, &res_slot) < 0) return -1;
+  for (int i : {0, 1, 2, 3, 4, 6})
+    if (d.cfg[i] != 0) return -1;                      // a tile, stage or split was asked for
+  if (((k.M + 255) / 256) * ((k.N + 127) / 128) >= (int64_t(1) << 20) || k.K >= (int64_t(1) << 24)) return -1;
+  const DevOperand& O = k.ops[k.chain.out_slot];
+  if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
+  return plan_exact(plan, k.M, k.N, k.K).cycles;
+}
+
+int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands& ops, void** state) {
+  *state = nullptr;
+  const kb200_kernel_desc& d = k.desc;
+  ExactState* st = new ExactState();
+  ExactParams& p = st->params;
+  const ExactPlan how = plan_exact(plan, k.M, k.N, k.K);
+  const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
+  p.bn = how.bn;
+  p.half_bn = how.bn / 2;
+  st->split = how.split;
+  p.steps = (int)((k.K + kExactStepK - 1) / kExactStepK);
+  p.first_steps = (p.steps + 1) / 2;
+  p.sums = 512 / how.bn < kExactMaxSums ? 512 / how.bn : kExactMaxSums;
+  const int stage_bytes = 2 * (kExactABytes + p.half_bn * 128), rest = kExactWarps * kExactSlot;
+  p.stages = (kExactSmem - rest) / stage_bytes < kExactMaxStages ? (kExactSmem - rest) / stage_bytes : kExactMaxStages;
+  st->smem = (size_t)p.stages * stage_bytes + rest;
+  // D = F32, A and B = F16, both K-major, N = bn, M = 256 over the pair
+  p.idesc = (1u << 4) | ((uint32_t)(p.bn >> 3) << 17) | ((256u >> 4) << 24);
+  p.tiles_n = (int)((k.N + p.bn - 1) / p.bn);
+  p.num_tiles = (int)((k.M + 255) / 256) * p.tiles_n;
+  p.magic_tn = ((uint64_t(1) << 40) + p.tiles_n - 1) / p.tiles_n;
+  p.kernel_index = kernel_index;
+  p.status = plan.d_status;
+  p.M = (int)k.M;
+  p.N = (int)k.N;
+  p.a_scale = ops.a_scale;
+  p.b_scale = ops.b_scale;
+  p.bias = st->bias_slot >= 0 ? k.ops[st->bias_slot].ptr : nullptr;
+  p.res = st->res_slot >= 0 ? k.ops[st->res_slot].ptr : nullptr;
+  p.res_row = st->res_slot >= 0 ? k.ops[st->res_slot].stride[1] : 0;
+  p.a = k.ops[d.a_slot].ptr;
+  p.a_row = k.ops[d.a_slot].stride[1];
+  p.b = k.ops[d.b_slot].ptr;
+  p.b_k = k.ops[d.b_slot].stride[1];
+  p.b_n = k.ops[d.b_slot].stride[2];
+  p.K = k.K;
+  p.stream_out = streams_out(plan, k, k.chain.out_slot, k.M * k.N) ? 1 : 0;
+  const DevOperand& O = k.ops[k.chain.out_slot];
+  p.with_tail = k.tail_out != nullptr ? 1 : 0;
+  // Persistent pairs, up to this plan's share of the GPU with several in flight.
+  const int pairs = plan.sm_count / 2, share = plan.concurrency > 1 && pairs / plan.concurrency > 0 ? pairs / plan.concurrency : pairs;
+  const int rounds = (p.num_tiles + share - 1) / share;
+  st->grid = (unsigned)(st->split ? 4 * p.num_tiles : 2 * ((p.num_tiles + rounds - 1) / rounds));
+  bool ok = encode_map(&st->map_a, true, ops.a, k.K, k.M, 2, ops.pitch, k.M * ops.pitch, kExactStepK, 128, false, 2) &&
+            encode_map(&st->map_b, true, ops.b, k.K, k.N, 2, ops.pitch, k.N * ops.pitch, kExactStepK, p.half_bn, false, 2) &&
+            encode_map_store(&st->map_out, false, O.ptr, k.N, k.M, 1, O.stride[1], 0);
+  st->map_res = st->map_tail = st->map_out;
+  if (ok && p.res) ok = encode_map_store(&st->map_res, false, p.res, k.N, k.M, 1, p.res_row, 0);
+  if (ok && p.with_tail) ok = set_map_address(&st->map_tail, k.tail_out);
+  if (!ok) { delete st; return KB200_OK; }
+  st->kernel = st->split ? exact_kernel<2, true>(fin) : p.bn > 192 ? exact_kernel<4, false>(fin) : p.bn > 128 ? exact_kernel<3, false>(fin) : exact_kernel<2, false>(fin);
+  const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExactSmem);
+  if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_exact_kernel)"); }
+  cudaFuncAttributes attributes;
+  KB200_CUDA(cudaFuncGetAttributes(&attributes, st->kernel));
+  if (attributes.numRegs != 168) { delete st; return KB200_OK; }      // (the warps that ask for more would wait for ever)
+  *state = st;
+  return KB200_OK;
+}
+
+int exact_launch(const Plan& plan, const void* state, cudaStream_t s) {
+  const ExactState* st = static_cast<const ExactState*>(state);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(st->grid, 1, 1);
+  cfg.blockDim = dim3(kExactThreads, 1, 1);
+  cfg.dynamicSmemBytes = st->smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = st->split ? 4 : 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = plan.pdl ? 2 : 1;
+  KB200_CUDA(cudaLaunchKernelEx(&cfg, st->kernel, st->map_a, st->map_b, st->map_out, st->map_res, st->map_tail, st->params));
+  return KB200_OK;
+}
+
+bool exact_repoint(const PlanKernel& k, void* state) {
+  ExactState* st = static_cast<ExactState*>(state);
+  st->params.a = k.ops[k.desc.a_slot].ptr;
+  if (st->bias_slot >= 0) st->params.bias = k.ops[st->bias_slot].ptr;
+  if (st->res_slot >= 0) st->params.res = k.ops[st->res_slot].ptr;
+  return set_map_address(&st->map_out, k.ops[k.chain.out_slot].ptr) && (st->res_slot < 0 || set_map_address(&st->map_res, k.ops[st->res_slot].ptr));
+}
+
+std::string exact_detail(const void* state) {
+  const ExactState* st = static_cast<const ExactState*>(state);
+  return "mm_exact " + std::to_string(st->params.bn) + " columns" + (st->split ? ", 2 splits" : "");
+}
+
+bool exact_writes_tails(const void* state) { return static_cast<const ExactState*>(state)->params.with_tail != 0; }
+
+void exact_destroy(void* state) { delete static_cast<ExactState*>(state); }
+
+}  // namespace kb200

@@ -1,0 +1,32 @@
+// Exact FP32 as products of float16 pairs on SM pairs (matmul_exact.cu), as matmul_tc.cu sees it, and the splitting of operands into such
+// pairs (split_rows.cu).
+#pragma once
+
+#include "kb200_internal.h"
+
+namespace kb200 {
+
+struct ExactOperands {
+  const void* a;             // [2, M, pitch] float16, the plane of heads and that of tails
+  const void* b;             // [2, N, pitch], rows along K
+  int64_t pitch;
+  const float* a_scale;      // [M] and [N]: what products of the terms are to be multiplied by
+  const float* b_scale;
+};
+
+// Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
+int64_t exact_cycles(const Plan& plan, const PlanKernel& k);
+// *state stays null when the operands cannot be described; a non-zero return is an error.
+int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands& ops, void** state);
+int exact_launch(const Plan& plan, const void* state, cudaStream_t s);
+bool exact_repoint(const PlanKernel& k, void* state);      // the operand pointers of `k` have moved
+std::string exact_detail(const void* state);
+bool exact_writes_tails(const void* state);
+void exact_destroy(void* state);
+
+// float32 rows of `cols` elements -> the two planes and the scales.  A pass in front of a launch, or once for a weight.
+int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, int64_t rows, int64_t cols, bool pdl, cudaStream_t s);
+// Do float16 pairs hold this weight [K, N] as well as TF32 pairs would, whatever A is?  Synchronises.
+int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, bool* suits);
+
+}  // namespace kb200

@@ -44,6 +44,7 @@
 #include "matmul_pair.h"
 #include "tc_common.cuh"
 #include "tc_epilogue.cuh"
+#include "tc_pair.cuh"
 
 namespace kb200 {
 
@@ -105,65 +106,6 @@ struct PairParams {
   int n_steps;
   PairStep steps[kMaxChain];
 };
-
-__device__ __forceinline__ int pair_div(int x, uint64_t magic) { return (int)(((uint64_t)(uint32_t)x * magic) >> 40); }
-
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-template <bool BF16>
-__device__ __forceinline__ void umma_pair(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if (BF16) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on)
-        : "memory");
-  }
-}
-// Arrives, when every MMA issued so far by this thread has completed, on the mbarrier at this offset
-// in BOTH CTAs of the pair (a commit, not a copy: the arrival is what is sent to the two CTAs).  One
-// instruction: a commit costs the issuing thread about as much as two MMAs.
-__device__ __forceinline__ void umma_pair_commit(uint32_t bar, uint16_t pair_ctas) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(pair_ctas)
-               : "memory");
-}
-__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
-// Bulk copy from this CTA's shared memory into another's of the cluster, where it completes on a barrier.
-__device__ __forceinline__ void push_block(uint32_t remote_dst, uint32_t src, uint32_t bytes, uint32_t remote_bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(remote_dst), "r"(src), "r"(bytes), "r"(remote_bar)
-               : "memory");
-}
-// At most `allowed` of this thread's most recent bulk-store groups may still be reading shared memory.
-__device__ __forceinline__ void store_wait_read(int allowed) {
-  switch (allowed) {
-    case 0: asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.bulk.wait_group.read 2;" ::: "memory"); break;
-    default: asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory"); break;
-  }
-}
 
 // One stage of this CTA's half of the B tile.
 template <int KPS>

@@ -34,6 +34,7 @@
 #include "device_math.cuh"
 #include "kb200_internal.h"
 #include "matmul.h"
+#include "matmul_exact.h"
 #include "matmul_pair.h"
 #include "matmul_small.h"
 #include "tc_common.cuh"
@@ -971,7 +972,15 @@ struct TcState {
   float* b_tail = nullptr;
   int64_t tail_pitch = 0;
   CUtensorMap map_at, map_bt;
+  // exact FP32 on float16 pairs: the operands' planes of heads and tails, [2, M or N, pitch], and their scales (see split_rows.cu)
+  struct Pairs16 {
+    void* a = nullptr;
+    void* b = nullptr;
+    float* scales = nullptr;                  // of B's columns (read in float4), then of A's rows
+    int64_t pitch = 0;
+  } pairs16;
   void* small = nullptr;      // state of the kernel for few tiles (matmul_small.cu) when it runs this matmul
+  void* exact = nullptr;      // state of the kernel on float16 pairs (matmul_exact.cu) when it runs this matmul
   void* pair = nullptr;       // state of the CTA-pair kernel (matmul_pair.cu) when it runs this matmul
 };
 
@@ -1012,6 +1021,12 @@ void drop_copies(TcState* st) {
   st->a_tail = st->b_tail = nullptr;
 }
 
+void drop_pairs16(TcState* st) {
+  for (void* p : {st->pairs16.a, st->pairs16.b, static_cast<void*>(st->pairs16.scales)})
+    if (p) cudaFree(p);
+  st->pairs16 = TcState::Pairs16();
+}
+
 // Can a tensor map of float32 elements describe rows of this stride at this address?
 bool rows_describable(const DevOperand& o, int64_t row_stride, int64_t batch) {
   return aligned16(o.ptr) && row_stride % 4 == 0 && (batch == 1 || o.stride[0] % 4 == 0);
@@ -1040,6 +1055,45 @@ cudaError_t launch_copy(const TcState::Copy& c, bool bf16, const DevOperand& o, 
                        (uint32_t)(batch * c.rows), (uint32_t)c.rows, (uint32_t)c.cols, (uint32_t)c.pitch, o.stride[0], row_stride);
 }
 
+// Exact FP32 on float16 pairs (matmul_exact.cu): the weight is split once, here, from rows along K (`turn`: it is turned first).
+// st->exact stays null where the weight or the memory does not suit.
+int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool turn, int64_t b_row) {
+  const kb200_kernel_desc& d = k.desc;
+  const DevOperand& B = k.ops[d.b_slot];
+  const int64_t pitch = (k.K + 63) / 64 * 64;              // rows on 128-byte lines
+  const uint64_t a_bytes = (uint64_t)k.M * pitch * 4;
+  bool suits = false;
+  const int rc = split_suits(B.ptr, B.stride[1], B.stride[2], k.K, k.N, &suits);
+  if (rc || !suits || a_bytes > plan.copy_budget) return rc;
+  TcState::Pairs16& h = st->pairs16;
+  float* turned = nullptr;
+  cudaError_t e = cudaMalloc(&h.a, a_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&h.b, (size_t)k.N * pitch * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&h.scales, (size_t)(k.M + k.N) * sizeof(float));
+  if (e == cudaSuccess && turn) e = cudaMalloc(&turned, (size_t)k.N * k.K * sizeof(float));
+  if (e == cudaSuccess && turn)
+    e = launch_kernel(false, transpose_rows_kernel<float>, dim3((unsigned)((k.K + 31) / 32), (unsigned)((k.N + 31) / 32)), dim3(256), 0, nullptr,
+                      (const float*)B.ptr, turned, (int)k.K, (int)k.N, B.stride[1], k.K);
+  h.pitch = pitch;
+  int status = KB200_OK;
+  if (e == cudaSuccess) {
+    status = split_rows(turn ? turned : B.ptr, turn ? k.K : b_row, h.b, pitch, h.scales, k.N, k.K, false, nullptr);
+    e = cudaDeviceSynchronize();
+  }
+  if (turned) cudaFree(turned);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    drop_pairs16(st);
+    return KB200_OK;
+  }
+  if (status) return status;
+  KB200_CUDA(e);
+  status = exact_bind(plan, k, kernel_index, ExactOperands{h.a, h.b, pitch, h.scales + k.N, h.scales}, &st->exact);
+  if (status || !st->exact) drop_pairs16(st);
+  else plan.copy_budget -= a_bytes;
+  return status;
+}
+
 }  // namespace
 
 void tc_destroy(PlanKernel& k);
@@ -1063,6 +1117,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // plan's budget for all of its copies, and where that is used up the operand is read as it is.
   const bool frozen = d.operands[d.b_slot].base_kind == KB200_BASE_CONST;
   drop_copies(st);
+  drop_pairs16(st);
   const bool may_turn = frozen && B.stride[2] == 1 && k.batch == 1 && k.N <= (int64_t(1) << 20);
   const bool may_presplit = d.precision == KB200_PREC_FP32 && frozen && k.batch == 1;
   const uint64_t additions = st->bf16 ? 0 : (uint64_t)k.N * ((k.K + 31) / 32 * 32) * sizeof(float) * ((may_turn ? 1 : 0) + (may_presplit ? 1 : 0));
@@ -1083,6 +1138,10 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // bytes a clock.
   if (st->small) small_destroy(st->small);
   st->small = nullptr;
+  if (st->pair) pair_destroy(st->pair);
+  st->pair = nullptr;
+  if (st->exact) exact_destroy(st->exact);
+  st->exact = nullptr;
   const bool presplit = may_presplit && room;
   st->b_copy.once = frozen;
   st->b_copy.turned = turn;
@@ -1138,6 +1197,20 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // (its exact-FP32 form multiplies with the tails of B: without room for them this file's kernel makes them as it goes)
   const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
   const bool small = few > 0 && tails_ready && (many == 0 || few < many || close_only);
+  // Float16 pairs on SM pairs: where there are many tiles (fewer are summed more closely than that kernel does, see accumulate_limit) and the
+  // estimates say so, its pass over A included.
+  if (presplit && plain && plan.few_tiles == 0 && ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128) > 16) {
+    const int64_t cycles = exact_cycles(plan, k) * 9 / 10;         // (of 1.9 to the ns; the small kernel's are 1.65)
+    if (cycles > 0 && (few < 0 || cycles < few) && (many == 0 || cycles < many)) {
+      const int rc = bind_pairs16(plan, k, kernel_index, st, turn, b_src_row);
+      if (rc) return rc;
+      if (st->exact) {
+        plan.copy_budget += turn ? additions / 2 : 0;
+        k.launches = 2;
+        return KB200_OK;
+      }
+    }
+  }
   if (close_only && !small) {
     if (room) plan.copy_budget += additions;
     tc_destroy(k);
@@ -1361,10 +1434,6 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     if (form != SMALL_A_MAPPED) return fail(KB200_ERR_UNSUPPORTED, "matmul %s: the operands cannot be described to TMA", d.name);
   }
   // More than 128 rows: 256-row tiles on SM pairs (matmul_pair.cu) when that kernel covers the epilogue.
-  if (st->pair) {
-    pair_destroy(st->pair);
-    st->pair = nullptr;
-  }
   if (pair_eligible(plan, k, b_kmajor, b_map_cols)) {
     const int rc = pair_bind(plan, k, kernel_index, po, &st->pair);
     if (rc) return rc;
@@ -1428,6 +1497,10 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
     KB200_CUDA(launch_kernel(plan.pdl, tail_rows_kernel<false>, dim3(cvt_grid(k.M * ((k.K + 3) / 4), cap)), dim3(256), 0, s, src, st->a_tail, (uint32_t)k.M,
                              (uint32_t)k.K, row, st->tail_pitch, (float*)nullptr));
   }
+  if (st->exact) {
+    const int rc = split_rows(k.ops[d.a_slot].ptr, k.ops[d.a_slot].stride[1], st->pairs16.a, st->pairs16.pitch, st->pairs16.scales + k.N, k.M, k.K, plan.pdl, s);
+    return rc ? rc : exact_launch(plan, st->exact, s);
+  }
   if (st->small) return small_launch(plan, st->small, s);
   if (st->pair) return pair_launch(plan, st->pair, s);
   cudaLaunchConfig_t cfg = {};
@@ -1468,6 +1541,7 @@ bool tc_repoint(PlanKernel& k) {
   for (int o = 0; o < k.n_ops; ++o) st->params.mm.ops[o].ptr = k.ops[o].ptr;
   const void* a = st->bf16 || st->a_copy.data ? nullptr : k.ops[d.a_slot].ptr;
   const void* b = st->bf16 || st->b_copy.data ? nullptr : k.ops[d.b_slot].ptr;
+  if (st->exact) return exact_repoint(k, st->exact);
   if (st->small) return small_repoint(k, st->small);
   if (st->pair) return pair_repoint(k, st->pair, a, b);
   bool ok = (!a || set_map_address(&st->map_a, a)) && (!b || set_map_address(&st->map_b, b));
@@ -1478,7 +1552,8 @@ bool tc_repoint(PlanKernel& k) {
 std::string tc_detail(const PlanKernel& k) {
   const TcState* st = static_cast<const TcState*>(k.tc);
   if (!st) return "";
-  const std::string copies = std::string(st->a_copy.data ? ", A copied" : "") + (st->b_copy.data ? ", B copied" : "");
+  const std::string copies = std::string(st->a_copy.data || st->pairs16.a ? ", A copied" : "") + (st->b_copy.data ? ", B copied" : "");
+  if (st->exact) return exact_detail(st->exact) + copies;
   if (st->small) return small_detail(st->small) + copies;
   if (st->pair) return pair_detail(st->pair) + copies;
   return "mm_tc " + std::to_string(st->params.bn) + " columns, " + std::to_string(st->params.splits) + " splits" + copies;
@@ -1486,15 +1561,17 @@ std::string tc_detail(const PlanKernel& k) {
 
 bool tc_writes_tails(const PlanKernel& k) {
   const TcState* st = static_cast<const TcState*>(k.tc);
-  return st && st->small && small_writes_tails(st->small);
+  return st && ((st->small && small_writes_tails(st->small)) || (st->exact && exact_writes_tails(st->exact)));
 }
 
 void tc_destroy(PlanKernel& k) {
   TcState* st = static_cast<TcState*>(k.tc);
   if (!st) return;
   drop_copies(st);
+  drop_pairs16(st);
   if (st->pair) pair_destroy(st->pair);
   if (st->small) small_destroy(st->small);
+  if (st->exact) exact_destroy(st->exact);
   delete st;
   k.tc = nullptr;
 }

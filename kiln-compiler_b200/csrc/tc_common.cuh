@@ -266,6 +266,11 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
+// ... that orders nothing of this thread's memory accesses beyond its own CTA, for a barrier that only says "this far" (tensor memory has
+// been read: tcgen05.fence orders that).  The release over the cluster above costs ~900 cycles, this 26.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -321,16 +326,16 @@ inline EncodeFn encode_fn() {
   return fn;
 }
 
-// A 3-D tiled map over [batch, rows, cols] with cols contiguous; box = (box_cols, box_rows, 1).
+// A 3-D tiled map over [batch, rows, cols] with cols contiguous; box = (box_cols, box_rows, box_batch).  (`bf16`: 16-bit elements.)
 inline bool encode_map(CUtensorMap* map, bool bf16, const void* base, int64_t cols, int64_t rows, int64_t batch,
-                int64_t row_stride_elems, int64_t batch_stride_elems, int box_cols, int box_rows, bool atom32) {
+                int64_t row_stride_elems, int64_t batch_stride_elems, int box_cols, int box_rows, bool atom32, int box_batch = 1) {
   EncodeFn fn = encode_fn();
   if (!fn) return false;
   const int esz = bf16 ? 2 : 4;
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
   cuuint64_t strides[2] = {(cuuint64_t)row_stride_elems * esz, (cuuint64_t)(batch > 1 ? batch_stride_elems : row_stride_elems * rows) * esz};
   if (strides[1] == 0) strides[1] = strides[0] * rows;
-  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, (cuuint32_t)box_batch};
   cuuint32_t elem[3] = {1, 1, 1};
   CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base),
                   dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -251,7 +251,6 @@ class GPUExecutable:
         self.launch_names = [l.name for l in program.launches]
         self.kernel_names = list(dict.fromkeys(l.kernel for l in program.launches))
         self._read_plan()
-        self.graph = None
         self.use_cuda_graphs = bool(cuda_graphs)
         self.relocatable = bool(self._lib.kb200_plan_relocatable(self._plan))
         self._call_lib = _cabi.load_call()
@@ -263,6 +262,7 @@ class GPUExecutable:
     # -- binding and launching ------------------------------------------------------------
 
     def _bind(self):
+        self.graph = None          # (it would launch on copies that are gone)
         consts = [self.constants[n] for n in self.const_names]
         cp, cs, cn = _ptr_array(consts)
         ip, is_, in_ = _ptr_array(self.static_inputs)
@@ -282,7 +282,6 @@ class GPUExecutable:
         self._bind()
         self.shares = (int(plans_in_flight), bool(others))
         self._read_plan()
-        self.graph = None
 
     def _read_plan(self):
         """What the plan, as it is bound now, runs."""
