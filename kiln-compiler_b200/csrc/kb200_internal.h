@@ -99,6 +99,13 @@ struct PlanKernel {
   void* shadow_out = nullptr;     // producer side: mirror address of this kernel's (single) output, or null
   const void* a_shadow = nullptr; // consumer side: mirror address of operand A / B, or null (convert per launch)
   const void* b_shadow = nullptr;
+  // FP32, a LayerNorm whose reader multiplies float16 pairs (matmul_exact.cuh): where its rows go as such, `pitch` apart, the tails `plane` behind
+  // the heads, or null.  mirror_only: the float32 rows are then stored where they hold infinities, which that reader sums from them.
+  struct Planes {
+    void* heads = nullptr;
+    int64_t plane = 0, pitch = 0;
+    float* scales = nullptr;
+  } planes_out;
   float* tail_out = nullptr;      // FP32: where the tails of the output (what a TF32 operand drops) go as well, same offsets, or null
   bool mirror_only = false;       // producer side: every reader of the output takes the mirror, the float32 store is dropped
   // An elementwise kernel that only continues the matmul in front of it (the activation or the residual
@@ -186,6 +193,8 @@ bool attention_reads_mirror(const PlanKernel& k);
 float* attention_tails(const PlanKernel& k);            // FP32 on the tensor cores: the tails of Q, K and V, or null
 void attention_tails_come_ready(PlanKernel& k);         // ... which the projection writes
 bool matmul_writes_tails(const PlanKernel& k);
+bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);      // multiplies float16 pairs of A, split by a pass of its own ...
+void matmul_planes_come_ready(PlanKernel& k);                                   // ... or by A's producer
 bool attention_may_drop_float32(const PlanKernel& k);    // writes a bf16 copy, and its float32 rows only where they were planned
 void attention_drop_float32(PlanKernel& k);
 bool tc_eligible(const PlanKernel& k);

@@ -11,6 +11,8 @@ void tc_destroy(PlanKernel& k);
 bool tc_repoint(PlanKernel& k);
 std::string tc_detail(const PlanKernel& k);
 bool tc_writes_tails(const PlanKernel& k);
+bool tc_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);
+void tc_planes_come_ready(PlanKernel& k);
 
 int choose_matmul(Plan& plan, PlanKernel& k) {
   (void)plan;
@@ -45,6 +47,8 @@ bool repoint_matmul(PlanKernel& k) { return tc_repoint(k); }
 
 std::string matmul_detail(const PlanKernel& k) { return tc_detail(k); }
 
+bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes) { return k.impl == IMPL_MM_TC && tc_takes_planes(k, planes); }
+void matmul_planes_come_ready(PlanKernel& k) { tc_planes_come_ready(k); }
 bool matmul_writes_tails(const PlanKernel& k) { return k.impl == IMPL_MM_TC && tc_writes_tails(k); }
 
 void destroy_matmul(PlanKernel& k) { tc_destroy(k); }

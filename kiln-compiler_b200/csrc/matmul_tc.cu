@@ -978,6 +978,7 @@ struct TcState {
     void* b = nullptr;
     float* scales = nullptr;                  // of B's columns (read in float4), then of A's rows
     int64_t pitch = 0;
+    bool ready = false;                       // A's producer writes its planes
   } pairs16;
   void* small = nullptr;      // state of the kernel for few tiles (matmul_small.cu) when it runs this matmul
   void* exact = nullptr;      // state of the kernel on float16 pairs (matmul_exact.cu) when it runs this matmul
@@ -1498,7 +1499,7 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
                              (uint32_t)k.K, row, st->tail_pitch, (float*)nullptr));
   }
   if (st->exact) {
-    const int rc = split_rows(k.ops[d.a_slot].ptr, k.ops[d.a_slot].stride[1], st->pairs16.a, st->pairs16.pitch, st->pairs16.scales + k.N, k.M, k.K, plan.pdl, s);
+    const int rc = st->pairs16.ready ? KB200_OK : split_rows(k.ops[d.a_slot].ptr, k.ops[d.a_slot].stride[1], st->pairs16.a, st->pairs16.pitch, st->pairs16.scales + k.N, k.M, k.K, plan.pdl, s);
     return rc ? rc : exact_launch(plan, st->exact, s);
   }
   if (st->small) return small_launch(plan, st->small, s);
@@ -1552,7 +1553,7 @@ bool tc_repoint(PlanKernel& k) {
 std::string tc_detail(const PlanKernel& k) {
   const TcState* st = static_cast<const TcState*>(k.tc);
   if (!st) return "";
-  const std::string copies = std::string(st->a_copy.data || st->pairs16.a ? ", A copied" : "") + (st->b_copy.data ? ", B copied" : "");
+  const std::string copies = std::string(st->a_copy.data || (st->pairs16.a && !st->pairs16.ready) ? ", A copied" : "") + (st->b_copy.data ? ", B copied" : "");
   if (st->exact) return exact_detail(st->exact) + copies;
   if (st->small) return small_detail(st->small) + copies;
   if (st->pair) return pair_detail(st->pair) + copies;
@@ -1562,6 +1563,18 @@ std::string tc_detail(const PlanKernel& k) {
 bool tc_writes_tails(const PlanKernel& k) {
   const TcState* st = static_cast<const TcState*>(k.tc);
   return st && ((st->small && small_writes_tails(st->small)) || (st->exact && exact_writes_tails(st->exact)));
+}
+
+bool tc_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes) {
+  const TcState* st = static_cast<const TcState*>(k.tc);
+  if (!st || !st->exact) return false;
+  *planes = PlanKernel::Planes{st->pairs16.a, k.M * st->pairs16.pitch, st->pairs16.pitch, st->pairs16.scales + k.N};
+  return true;
+}
+
+void tc_planes_come_ready(PlanKernel& k) {
+  static_cast<TcState*>(k.tc)->pairs16.ready = true;
+  k.launches = 1;
 }
 
 void tc_destroy(PlanKernel& k) {

@@ -11,8 +11,11 @@
 //                  reductions): one read and one write of the tensor, HBM-bound.
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "device_math.cuh"
 #include "kb200_internal.h"
+#include "split16.cuh"
 
 namespace kb200 {
 
@@ -141,6 +144,11 @@ struct RowFastParams {
   int64_t pre_out_stride0, pre_out_stride1;
 };
 
+// PLANES: and the rows as float16 pairs, see split_rows.cu.  (Of its own: 40 bytes more of parameters cost the other launches 0.35 us of host time.)
+struct RowPlanesParams : RowFastParams {
+  PlanKernel::Planes planes;
+};
+
 enum { ROW_LAYERNORM = 0, ROW_SOFTMAX = 1 };
 
 // VEC consecutive floats as one access.
@@ -180,14 +188,18 @@ __device__ __forceinline__ float row_fold(const float (&v)[VEC]) { return VEC ==
 // the last float4 of the tensor is read element by element where it would reach past its end.
 // Softmax only (16384 x 333: 18.0 us with single floats, 10.2; 16384 x 4093: 124, 114): the affine parameters of
 // a LayerNorm would still come as single floats, four lanes apart, and 16384 x 771 took 30.9 us against 28.2.
-template <int MODE, int VEC, int N, bool WIDE, bool PRE, bool SHIFT, bool AHEAD>
-__global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_constant__ RowFastParams p) {
+//
+// PLANES: a LayerNorm whose reader multiplies float16 pairs leaves its rows as such, their scale by a third reduction.
+template <int MODE, int VEC, int N, bool WIDE, bool PRE, bool SHIFT, bool AHEAD, bool PLANES>
+__global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_constant__ std::conditional_t<PLANES, RowPlanesParams, RowFastParams> p) {
   const int lane = WIDE ? threadIdx.x : (threadIdx.x & 31);
   const int lanes = WIDE ? blockDim.x : 32;
   const int64_t row = WIDE ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   static_assert(!SHIFT || (VEC == 4 && !PRE && MODE == ROW_SOFTMAX), "shifted rows come as float4, without operands beside them");
   const int units = SHIFT ? (p.inner + 6) >> 2 : VEC == 1 ? p.inner : p.inner >> 2;
+  static_assert(!PLANES || (VEC == 4 && MODE == ROW_LAYERNORM), "pairs are made of float4");
   __shared__ float partial[WIDE ? 64 : 1];
+  [[maybe_unused]] __shared__ uint32_t partial_most[WIDE && PLANES ? 32 : 1];
   // Each reduction of a WIDE row has its own half of `partial`: no barrier between the reads of one and the writes of the next.
   auto across = [&](float v, bool is_max, int which) {
     v = is_max ? warp_max(v) : warp_sum(v);
@@ -309,6 +321,11 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
         }
 #pragma unroll
         for (int e = 0; e < VEC; ++e) y[e] = v[i][e] * rstd * g[at][e] + b[at][e];
+        if constexpr (PLANES) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) v[i][e] = y[e];
+          continue;
+        }
         if (p.store32) row_store<VEC>(out + VEC * j, y);
         if (p.out16 != nullptr) {
           if (VEC == 1) {
@@ -321,6 +338,31 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
             *reinterpret_cast<uint2*>(p.out16 + out_off + 4 * j) = packed;
           }
         }
+      }
+    }
+    if constexpr (PLANES) {
+      uint32_t most = 0;
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (live[i])
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) most = max(most, magnitude_bits(v[i][e]));
+      most = warp_umax(most);
+      if constexpr (WIDE) {
+        const int l = threadIdx.x & 31;
+        if (l == 0) partial_most[threadIdx.x >> 5] = most;
+        __syncthreads();
+        most = warp_umax(l < (lanes >> 5) ? partial_most[l] : 0u);
+      }
+      const RowScale scale(most);
+      if (lane == 0) p.planes.scales[row] = scale.back;
+      __half* const heads = static_cast<__half*>(p.planes.heads) + row * p.planes.pitch;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (!live[i]) continue;
+        const int j = lane + lanes * i;
+        store_terms(heads + 4 * j, heads + p.planes.plane + 4 * j, make_float4(v[i][0], v[i][1], v[i][2], v[i][3]), scale.by);
+        if (p.store32 || scale.marked) row_store<VEC>(out + VEC * j, v[i]);
       }
     }
   } else {
@@ -368,14 +410,14 @@ constexpr int64_t kRowLimit = 512 * 32, kShiftedLimit = kRowLimit - 8;
 
 enum { ROW_FLOATS = 0, ROW_VECTORS = 1, ROW_SHIFTED = 2 };      // how rows are accessed
 
-template <int MODE, bool PRE>
-static void launch_rows(const RowFastParams& p, int access, int sm_count, bool pdl, cudaStream_t s) {
+template <int MODE, bool PRE, bool PLANES>
+static void launch_rows(const std::conditional_t<PLANES, RowPlanesParams, RowFastParams>& p, int access, int sm_count, bool pdl, cudaStream_t s) {
   const bool vec = access != ROW_FLOATS;
   const int units = access == ROW_SHIFTED ? (p.inner + 6) / 4 : vec ? p.inner / 4 : p.inner;
   const int n = (units + 31) / 32;                  // accesses per lane if one warp takes the row
   unsigned grid, block;
-#define KB200_ROW_CASE(VEC, N, WIDE, AHEAD) launch_kernel(pdl, row_kernel<MODE, VEC, N, WIDE, PRE, false, AHEAD>, dim3(grid), dim3(block), 0, s, p)
-#define KB200_SHIFT_CASE(N, WIDE) launch_kernel(pdl, row_kernel<MODE, 4, N, WIDE, false, true, false>, dim3(grid), dim3(block), 0, s, p)
+#define KB200_ROW_CASE(VEC, N, WIDE, AHEAD) launch_kernel(pdl, row_kernel<MODE, VEC, N, WIDE, PRE, false, AHEAD, PLANES>, dim3(grid), dim3(block), 0, s, p)
+#define KB200_SHIFT_CASE(N, WIDE) launch_kernel(pdl, row_kernel<MODE, 4, N, WIDE, false, true, false, false>, dim3(grid), dim3(block), 0, s, p)
   if (n <= (vec && MODE == ROW_LAYERNORM ? 6 : 8)) {
     // a warp per row; few rows spread over more blocks.  (A LayerNorm of 8 float4 a lane, or either of 12,
     // spills; four warps of a quarter each do not.  With a chain in front, a LayerNorm of four float4 and softmaxes of four or
@@ -400,7 +442,7 @@ static void launch_rows(const RowFastParams& p, int access, int sm_count, bool p
       else if (n <= 6 && few) KB200_ROW_CASE(4, 6, false, true);
       else if (n <= 6) KB200_ROW_CASE(4, 6, false, false);
       else if constexpr (MODE == ROW_SOFTMAX) KB200_ROW_CASE(4, 8, false, true);
-    } else {
+    } else if constexpr (!PLANES) {
       if (n <= 2) KB200_ROW_CASE(1, 2, false, true);
       else if (n <= 4) KB200_ROW_CASE(1, 4, false, true);
       else KB200_ROW_CASE(1, 8, false, true);
@@ -421,17 +463,20 @@ static void launch_rows(const RowFastParams& p, int access, int sm_count, bool p
   }
   if (vec && per == 4) KB200_ROW_CASE(4, 4, true, false);
   else if (vec) KB200_ROW_CASE(4, 8, true, false);
-  else if (per == 8) KB200_ROW_CASE(1, 8, true, false);
-  else if (per == 16) KB200_ROW_CASE(1, 16, true, false);
-  else KB200_ROW_CASE(1, 32, true, false);
+  else if constexpr (!PLANES) {
+    if (per == 8) KB200_ROW_CASE(1, 8, true, false);
+    else if (per == 16) KB200_ROW_CASE(1, 16, true, false);
+    else KB200_ROW_CASE(1, 32, true, false);
+  }
 #undef KB200_ROW_CASE
 #undef KB200_SHIFT_CASE
 }
 
 template <int MODE>
 static void launch_row_fast(const RowFastParams& p, int access, int sm_count, bool pdl, cudaStream_t s) {
-  if (p.n_pre > 0 || p.pre_out != nullptr) launch_rows<MODE, true>(p, access, sm_count, pdl, s);
-  else launch_rows<MODE, false>(p, access, sm_count, pdl, s);
+  const bool pre = p.n_pre > 0 || p.pre_out != nullptr;
+  if (pre) launch_rows<MODE, true, false>(p, access, sm_count, pdl, s);
+  else launch_rows<MODE, false, false>(p, access, sm_count, pdl, s);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -542,8 +587,16 @@ int launch_row(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
       p.inv_n = k.ln_inv_n;
       p.eps = k.ln_eps;
       p.out16 = static_cast<__nv_bfloat16*>(k.shadow_out);
-      p.store32 = (k.mirror_only && p.out16 != nullptr) ? 0 : 1;
-      launch_row_fast<ROW_LAYERNORM>(p, access, plan.sm_count, plan.pdl, s);
+      p.store32 = k.mirror_only && (p.out16 != nullptr || k.planes_out.heads != nullptr) ? 0 : 1;
+      if (k.planes_out.heads != nullptr) {          // (rows of float4)
+        RowPlanesParams with;
+        static_cast<RowFastParams&>(with) = p;
+        with.planes = k.planes_out;
+        if (p.n_pre > 0 || p.pre_out != nullptr) launch_rows<ROW_LAYERNORM, true, true>(with, ROW_VECTORS, plan.sm_count, plan.pdl, s);
+        else launch_rows<ROW_LAYERNORM, false, true>(with, ROW_VECTORS, plan.sm_count, plan.pdl, s);
+      } else {
+        launch_row_fast<ROW_LAYERNORM>(p, access, plan.sm_count, plan.pdl, s);
+      }
     } else {
       launch_row_fast<ROW_SOFTMAX>(p, access, plan.sm_count, plan.pdl, s);
     }

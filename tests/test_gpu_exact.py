@@ -123,3 +123,63 @@ def test_weights_that_make_up_for_a_row_s_spread_keep_the_other_kernels():
     x = x * torch.from_numpy(spread).cuda()
     want = x.double() @ c["weight.transpose"] + c["bias"]
     assert float((call(exe, x).double() - want).norm() / want.norm()) <= 5e-6          # (the other kernels': 2^-23 per 8 of K in one accumulator)
+
+
+def norm_linear(d, n, m=1024, second_reader=False):
+    """LayerNorm and a Linear behind it; a residual of the LayerNorm's output for a second reader."""
+    from perf import cases
+
+    p = cases._Plan("norm_linear", (m, d), (m, n))
+    h = p.buffer(m, d)
+    p.layernorm(p.x, "ln.", h)
+    p.linear(h, "fc.", n, p.y, residual=h if second_reader else None)
+    return p.spec()
+
+
+def run_plan(plan, consts, x, **env):
+    import os
+
+    from kiln_b200.codegen import program_from_plan
+    from kiln_b200.runtime import GPUExecutable
+
+    with pytest.MonkeyPatch.context() as patch:
+        for name, value in env.items():
+            patch.setenv(name, value)
+        exe = GPUExecutable(program_from_plan(plan, "fp32"), plan.arena_bytes, consts, plan.input_shapes, plan.output_shapes)
+    return exe, call(exe, x)
+
+
+@pytest.mark.parametrize("d,n,second_reader", [(768, 2304, False), (2048, 2048, True), (772, 2304, False), (128, 4096, False), (4096, 1024, False), (8196, 768, False)])
+def test_a_layernorm_leaves_its_rows_split(d, n, second_reader):
+    """A warp or a block per row; the same bits whether the float32 rows are stored as well or not."""
+    from perf import cases
+
+    plan = norm_linear(d, n, second_reader=second_reader)
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    x = torch.randn(1024, d, device="cuda") * 3 + 1
+    exe, got = run_plan(plan, consts, x)
+    assert "mm_exact" in exe.details[1] and "A copied" not in exe.details[1] and exe.device_launches == 2, exe.details
+    _, stored = run_plan(plan, consts, x, KILN_GPU_MIRROR_ONLY="0")
+    assert torch.equal(got, stored)
+    c = {name: torch.from_numpy(v).cuda().double() for name, v in consts.items()}
+    h = torch.nn.functional.layer_norm(x.double(), (d,), c["ln.weight"], c["ln.bias"], 1e-5)
+    want = h @ c["fc.weight.transpose"] + c["fc.bias"] + (h if second_reader else 0)
+    assert float((got.double() - want).norm() / want.norm()) <= 2 * BOUND          # (the LayerNorm's own float32 sums)
+
+
+def test_infinities_a_layernorm_makes():
+    """A scale of infinity: its column is infinite in every row, which the matmul then sums from the float32 rows."""
+    from perf import cases
+
+    d, n = 768, 2304
+    plan = norm_linear(d, n)
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    consts["ln.weight"][5] = np.inf
+    x = torch.randn(1024, d, device="cuda")
+    x[9, 3] = float("nan")
+    exe, got = run_plan(plan, consts, x)
+    assert "mm_exact" in exe.details[1] and exe.device_launches == 2, exe.details
+    h5 = (x[:, 5] - x.mean(1)) * float("inf")
+    want = h5[:, None] * torch.from_numpy(consts["fc.weight.transpose"][5]).cuda()
+    rows = torch.arange(1024, device="cuda") != 9
+    assert torch.equal(got[rows], want[rows]) and bool(got[9].isnan().all())
