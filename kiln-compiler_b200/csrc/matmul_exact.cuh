@@ -146,7 +146,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
-  cluster_arrive();                   // every CTA's barriers exist once all have arrived
+  cluster_arrive_relaxed();           // every CTA's barriers exist once all have arrived (fence.mbarrier_init is what orders)
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -196,7 +196,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         const int m = tm * 256 + (int)rank * 128, n = tn * p.bn + (int)rank * p.half_bn;
         int k = step0 * kExactStepK;
         for (int i = 0; i < n_steps; ++i, k += kExactStepK) {
-          ok = all_waited(mbar_wait_cluster(empty0 + 8 * s, parity, abort_ptr), 1);
+          ok = all_waited(mbar_wait_long(empty0 + 8 * s, parity, abort_ptr), 1);
           if (!ok) break;
           const bool b_here = ahead > 0;           // expected and requested above
           const uint32_t bar = full_leader0 + 8 * s, dst = ring + (uint32_t)(s * stage_bytes);
@@ -299,7 +299,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         for (int q = 0; q < 32; ++q) sums[j][q] = 0.0f;
       // The first pass over what finishes a tile is a rehearsal, as in matmul_pair.cu: its code is cold at every launch.
       for (int i = 0; i < n_steps && !dry; ++i) {
-        if (!mbar_wait_cluster(ready0 + 8 * sum, ready_parity, abort_ptr)) give_up(3);
+        if (!mbar_wait_long(ready0 + 8 * sum, ready_parity, abort_ptr)) give_up(3);
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -340,7 +340,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       if constexpr (SPLIT) {
         if (!dry) {
           const uint32_t other = cta ^ 2u;
-          if (e == 0 && lane == 0) mbar_arrive_cluster(map_to_cta(bar0 + 8 * BAR_PEER, other));      // this CTA's ring may be written
+          if (e == 0 && lane == 0) mbar_arrive_remote(map_to_cta(bar0 + 8 * BAR_PEER, other));      // this CTA's ring may be written
           uint32_t coming = 0;
           for (int c = half; c < blocks; c += 2)
             if (c >= first_block && c < end_block && rows_ok && n0 + 32 * c < p.N) coming += 4096;
@@ -472,7 +472,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   if (abort_flag && threadIdx.x == 0) let_copies_land();
   __syncwarp();
   // neither CTA leaves (or frees TMEM the other's MMAs write) before both are done
-  cluster_arrive();
+  cluster_arrive_relaxed();
   cluster_wait();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

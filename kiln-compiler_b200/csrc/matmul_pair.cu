@@ -166,7 +166,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   // producer and the MMA thread need now, under the set-up, instead of in front of the first copy.
   // Both CTAs' barriers must exist before either signals the other: arrive on the cluster barrier as
   // soon as this CTA's are initialised, wait for it after the TMEM allocation below.
-  cluster_arrive();
+  cluster_arrive_relaxed();
   if (lane == 0 && warp < 2)
     asm volatile("" ::"r"(p.bn), "r"(p.idesc), "r"(p.num_tiles), "l"(p.magic_tn), "l"(p.magic_tpb), "l"(p.status) : "memory");
   if (warp == 2 && lane < kMaxChain) chain_steps[lane] = p.steps[lane];
@@ -228,7 +228,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       const int n_col = tn_i * bn + (int)rank * half_bn;
       int k_elem = first_kb * step_k;
       for (int kb = 0; kb < num_kb; ++kb, k_elem += step_k) {
-        const bool got = mbar_wait_cluster(empty0 + 8 * s, wait_parity, abort_ptr);
+        const bool got = mbar_wait_long(empty0 + 8 * s, wait_parity, abort_ptr);
         if (!__all_sync(0xffffffffu, got ? 1 : 0)) {
           if (lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 1); *abort_ptr = 1; }
           ok = false;
@@ -273,7 +273,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         const int acc = i & 1;
         const uint32_t aph = (i >> 1) & 1;
         // both CTAs' epilogue warps have drained this accumulator (two tiles ago)
-        const bool drained = mbar_wait_cluster(tempty0 + 8 * acc, aph ^ 1, abort_ptr);
+        const bool drained = mbar_wait_long(tempty0 + 8 * acc, aph ^ 1, abort_ptr);
         if (!__all_sync(0xffffffffu, drained ? 1 : 0)) {
           if (lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 4); *abort_ptr = 1; }
           break;
@@ -429,7 +429,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       if constexpr (SPLIT) {
         if (!dry) {
           const uint32_t other = cta ^ 2u;
-          if (e == 0 && lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bars[kBarPeer]), other));      // this CTA's ring may be written
+          if (e == 0 && lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bars[kBarPeer]), other));      // this CTA's ring may be written
           uint32_t coming = 0;
           for (int c = 32 * group; c < p.half_bn; c += 32 * kPairWarpsPerQuad)
             if (rows_ok && n0 + c_first + c < p.N) coming += 4096;
@@ -541,7 +541,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
       // this warp has read the accumulator: hand it back to the leader's MMA thread
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty_leader0 + 8 * acc);
+      if (lane == 0) mbar_arrive_remote(tempty_leader0 + 8 * acc);
       tile += num_pairs;
       ++i;
     }
@@ -553,7 +553,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
   __syncthreads();
   if (abort_flag && threadIdx.x == 0) let_copies_land();
   // neither CTA leaves (or frees TMEM the other's MMAs write) before both are done
-  cluster_arrive();
+  cluster_arrive_relaxed();
   cluster_wait();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

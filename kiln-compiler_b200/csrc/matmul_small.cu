@@ -215,7 +215,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   // without a split is no cluster launch and keeps off the cluster instructions (a store to a mapped
   // address in one is an illegal instruction).
   const bool clustered = p.splits > 1;
-  if (clustered) cluster_arrive();
+  if (clustered) cluster_arrive_relaxed();        // (fence.mbarrier_init above is what orders)
   const uint32_t tmem = tmem_slot;
   [[maybe_unused]] const uint32_t tmem_a = tmem + (uint32_t)((EXACT ? p.acc_slots + 1 : 1) * BN);      // the slabs of A
   volatile int* abort_ptr = &abort_flag;

@@ -70,6 +70,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The same for a wait that is expected to last: the thread is suspended between polls, for a time the hardware chooses.
+__device__ __forceinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok != 0) return true;
+    if ((i & 63) == 63 && *abort_flag) return false;
+  }
+  return false;
+}
+
 // What a CTA that gives up does before it releases its shared memory: copies may be in flight towards it, and a barrier does not say
 // whether any are (asked for either parity, one of the two answers is always yes).  They get 400000 cycles, 0.2 ms, to land.
 __device__ __forceinline__ void let_copies_land() {
