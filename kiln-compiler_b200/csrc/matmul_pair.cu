@@ -416,7 +416,7 @@ mm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
         res_ready = true;
       }
       if (!dry) {
-        bool got = mbar_wait_cluster_relaxed(tfull0 + 8 * acc, aph, abort_ptr);
+        bool got = mbar_wait_long(tfull0 + 8 * acc, aph, abort_ptr);
         if (!got && lane == 0 && !*abort_ptr) { atomicCAS(p.status, 0, (p.kernel_index << 8) | 3); *abort_ptr = 1; }
         ok = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0 && !*abort_ptr;
         if (!ok) break;

@@ -70,7 +70,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
-// The same for a wait that is expected to last: the thread is suspended between polls, for a time the hardware chooses.
+// The same for a wait that is expected to last: the thread is suspended between polls, for a time the hardware chooses, and leaves the issue
+// slots and the barrier's shared-memory bank to the threads that feed the tensor cores.
 __device__ __forceinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < kWaitLimit; ++i) {
     uint32_t ok;
@@ -302,17 +303,6 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < kWaitLimit; ++i) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((i & 63) == 63 && *abort_flag) return false;
-  }
-  return false;
-}
-// The same for a wait that is expected to last (an epilogue warp waiting for its tile): the thread
-// sleeps between polls, so that sixteen waiting warps leave the issue slots and the barrier's
-// shared-memory bank to the threads that feed the tensor cores.
-__device__ __forceinline__ bool mbar_wait_cluster_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    __nanosleep(100);
     if ((i & 63) == 63 && *abort_flag) return false;
   }
   return false;
