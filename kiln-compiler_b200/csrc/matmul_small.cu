@@ -17,11 +17,12 @@
 // The sum over the splits runs in rank order, so results do not depend on timing.
 //
 // Per CTA, 352 threads: warp 0 loads A, warp 10 loads B, warp 1 issues the MMAs, warps 2-9 (two per tensor-memory
-// lane quadrant) move A to tensor memory, then drain, exchange and finish.  An A that a tensor map cannot describe, or
-// that is float32 where the MMAs want bf16, is read by warps 2-9 themselves (GATHER).  Waits are bounded as
-// in matmul_tc.cu.
+// lane quadrant) move A to tensor memory, then drain, exchange and finish.  An A that is float32 where the MMAs want bf16 is rounded on that
+// way; one whose rows are on no pitch of 16 bytes comes through four tensor maps (GATHER).  Waits are bounded as in matmul_tc.cu.
 #include <cuda.h>
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
@@ -67,12 +68,14 @@ struct SmallParams {
   const float* bias;
   const float* res;
   int64_t res_row;
-  const float* a;                  // GATHER and exact FP32: A as it is in memory, rows of K elements a_row apart
+  const float* a;                  // exact FP32: A as it is in memory, rows of K elements a_row apart
   int64_t a_row;
   const float* b;                  // exact FP32: B as it is in memory, and its strides along K and N
   int64_t b_k, b_n;
   int K;
-  int a_rows;                      // rows of a box of A: the tile's, or M where that is less
+  int a_rows;                      // rows of a box of A: the tile's, or M where that is less (GATHER: a quarter, in each map)
+  int a_maps;                      // GATHER
+  int a_shift[4];
   float* out;                      // null: only the bf16 copy is stored
   __nv_bfloat16* out16;            // or null
   float* out_tail;                 // exact FP32: the output minus its 19 leading bits, for a consumer that splits it, or null
@@ -85,49 +88,35 @@ struct SmallParams {
 __host__ __device__ constexpr int slabs_per_step(int mode) { return mode == SMALL_EXACT || mode == SMALL_BF16_A32 ? 1 : 2; }
 // A stage: the slabs of A (one of float32 for bf16 products is two boxes of 32 columns), then those of B (exact FP32: and its tails)
 __host__ __device__ constexpr int a_slab_bytes(int mode) { return mode == SMALL_BF16_A32 ? 2 * kSmallABytes : kSmallABytes; }
+__host__ __device__ constexpr int gather_pitch_floats(int mode) { return mode == SMALL_EXACT ? 36 : 68; }      // of a row in shared memory, see GatherMaps
+__host__ __device__ constexpr int a_stage_bytes(int mode, bool gather) {
+  return gather ? kSmallM * gather_pitch_floats(mode) * 4 : slabs_per_step(mode) * a_slab_bytes(mode);
+}
 __host__ __device__ constexpr int b_boxes(int mode) { return mode == SMALL_BF16_A32 ? 1 : 2; }
-__host__ __device__ constexpr int stage_bytes_of(int mode, int bn) { return slabs_per_step(mode) * a_slab_bytes(mode) + b_boxes(mode) * bn * 128; }
+__host__ __device__ constexpr int stage_bytes_of(int mode, int bn, bool gather) { return a_stage_bytes(mode, gather) + b_boxes(mode) * bn * 128; }
 
 __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
   __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// This warp's 32 rows of a slab of A, for GATHER: float32 in global memory, rows from any element on.  Lane l has column l
-// of every row (BF16: columns 2l and 2l + 1), so that a warp reads whole lines.  Rows past the last are the last one
-// again (they make accumulator rows that nobody reads), columns past K are zeros.
-template <bool BF16>
-__device__ __forceinline__ void gather_rows(float (&raw)[BF16 ? 64 : 32], const SmallParams& p, int row0, int col0, int lane) {
-  const int last = p.M - 1;
-  constexpr int kCols = BF16 ? 2 : 1;
-  const int col = col0 + kCols * lane;
-#pragma unroll
-  for (int r = 0; r < 32; ++r) {
-    const float* const at = p.a + min(row0 + r, last) * p.a_row + col;
-#pragma unroll
-    for (int c = 0; c < kCols; ++c) raw[kCols * r + c] = col + c < p.K ? at[c] : 0.f;
-  }
-}
-
-// The same rows into a slab of A as the copy engine would have left them: 128-byte rows, 16-byte units XORed with the row.
-template <bool BF16>
-__device__ __forceinline__ void park_rows(uint8_t* slab, const float (&raw)[BF16 ? 64 : 32], int row0, int lane) {
-#pragma unroll
-  for (int r = 0; r < 32; ++r) {
-    const int row = row0 + r;
-    uint32_t* const at = reinterpret_cast<uint32_t*>(slab + row * 128 + (((lane >> 2) ^ (row & 7)) << 4)) + (lane & 3);
-    *at = BF16 ? pack_bf16(raw[(2 * r) % (BF16 ? 64 : 32)], raw[(2 * r + 1) % (BF16 ? 64 : 32)]) : __float_as_uint(raw[r]);
-  }
-}
+// The rows of A on no pitch (GATHER): four tensor maps, of every fourth row each, whose pitch is four rows and so a multiple of 16 bytes.  A
+// map's base is rounded down to 16 bytes, `shift` floats in front of its first row; boxes are four columns wider than a step and the warps
+// that move A read from `shift` on.  Row 4 i + c of a tile is accumulator row 32 c + i: a warp's 32 rows are of one map and have one shift.
+// (Rows of 36 or 68 floats in shared memory: an odd number of 16-byte units, so that a warp's loads have no bank conflicts.)
+struct GatherMaps { CUtensorMap of[4]; };
+template <bool GATHER> __device__ __forceinline__ int matrix_row(int row) { return GATHER ? 4 * (row & 31) + (row >> 5) : row; }
 
 // What a TF32 operand does not hold of x.
 __device__ __forceinline__ float dropped_bits(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
 
 // Exact FP32: an infinite operand makes a NaN of its tail's products (inf x 0, inf - inf) where float32 has an infinity.  Results
-// that are NaN, of rows m, m + rows_apart, ... below m_end and columns n to n + 3, done over as the CUDA cores do them.
-template <int FIN>
-__device__ __noinline__ void redo_in_float32(const SmallParams& p, int m, int m_end, int rows_apart, int n) {
-  for (; m < m_end; m += rows_apart) {
+// that are NaN, of the tile's accumulator rows `row`, row + rows_apart, ... below row_end and columns n to n + 3, done over as the CUDA cores do them.
+template <int FIN, bool GATHER>
+__device__ __noinline__ void redo_in_float32(const SmallParams& p, int m0, int row, int row_end, int rows_apart, int n) {
+  for (; row < row_end; row += rows_apart) {
+    const int m = m0 + matrix_row<GATHER>(row);
+    if (m >= p.M) continue;
     for (int c = n; c < n + 4 && c < p.N; ++c) {
       float* const out = p.out + (int64_t)m * p.out_row + c;
       if (*out == *out) continue;
@@ -145,13 +134,13 @@ __device__ __noinline__ void redo_in_float32(const SmallParams& p, int m, int m_
   }
 }
 
-// BN: columns of a tile, 64, 96 or 128.  GATHER: warps 2-9 read A from global memory.  Of a Linear of 333 x 1000 x 771 the
-// pass that copied A to aligned rows, and the one that made bf16 of a float32 A, was a launch of ~2.3 us in front of this one.
+// BN: columns of a tile, 64, 96 or 128.  GATHER: rows of A on no pitch.  Of a Linear of 333 x 1000 x 771 the pass that copied A to aligned
+// rows, and the one that made bf16 of a float32 A, was a launch of ~2.3 us in front of this one.
 // DRAINS: exact FP32, more steps than the accumulators take.  (The adding up in the loop, and its registers, cost 3 % where it does
 // nothing: 1024 x 768 x 3072 29.0 us, 27.9 without.)
 template <int MODE, int FIN, int BN, bool GATHER, bool DRAINS>
 __global__ void __launch_bounds__(kSmallThreads, 1)
-mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+mm_small_kernel(const __grid_constant__ std::conditional_t<GATHER, GatherMaps, CUtensorMap> tma_a, const __grid_constant__ CUtensorMap tma_b,
                 const __grid_constant__ CUtensorMap tma_bt, const __grid_constant__ SmallParams p) {
   constexpr bool EXACT = MODE == SMALL_EXACT;
   constexpr int kSmallBBytes = BN * 128;
@@ -161,7 +150,8 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   constexpr int kSlabs = slabs_per_step(MODE);
   constexpr bool A32 = MODE == SMALL_BF16_A32, BF16 = MODE == SMALL_BF16 || A32;
   constexpr bool ALTERNATE = kSlabs == 1;                       // the two groups of warps that move A take alternate steps
-  constexpr int kSlabA = a_slab_bytes(MODE), kBBoxes = b_boxes(MODE), kStage = stage_bytes_of(MODE, BN);
+  constexpr int kSlabA = a_slab_bytes(MODE), kBBoxes = b_boxes(MODE), kStage = stage_bytes_of(MODE, BN, GATHER), kStageA = a_stage_bytes(MODE, GATHER);
+  constexpr int kGatherRow = gather_pitch_floats(MODE) * 4;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[3 * kSmallMaxStages + 4 + kSmallMaxSlots];
   __shared__ uint32_t tmem_slot;
@@ -184,7 +174,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < p.stages; ++s) {
-      mbar_init(full0 + 8 * s, GATHER ? 1 : 2);
+      mbar_init(full0 + 8 * s, 2);
       mbar_init(empty0 + 8 * s, 1);
       mbar_init(split0 + 8 * s, ALTERNATE ? kSmallEpiWarps / 2 : kSmallEpiWarps);
     }
@@ -196,7 +186,11 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     mbar_expect_tx(received, (uint32_t)(kTileBytes / p.splits * (p.splits - 1)));     // (an arrival, too; a launch without a split does not use it)
   }
   if (threadIdx.x == 32) {
-    prefetch_tensormap(&tma_a);
+    if constexpr (GATHER) {
+      for (int c = 0; c < 4; ++c) prefetch_tensormap(&tma_a.of[c]);
+    } else {
+      prefetch_tensormap(&tma_a);
+    }
     prefetch_tensormap(&tma_b);
     if (EXACT) prefetch_tensormap(&tma_bt);
   }
@@ -230,22 +224,27 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (!got && lane == 0) give_up(site);
     return __all_sync(0xffffffffu, got ? 1 : 0) != 0;
   };
-  if ((warp == 0 && !GATHER) || warp == 10) {
+  if (warp == 0 || warp == 10) {
     // ---------------- TMA producers, one per operand ----------------
-    const bool is_a = !GATHER && warp == 0;
+    const bool is_a = warp == 0;
     int s = 0, k_elem = step0 * kSlabs * p.slab_k;
     uint32_t parity = 1;
     for (int i = 0; i < n_steps; ++i) {
       if (i >= p.stages && !all_waited(mbar_wait(empty0 + 8 * s, parity, abort_ptr), 1)) break;
-      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kSlabs * kSlabA;
+      const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kStageA;
       if (elect_one()) {
-        mbar_expect_tx(bar, is_a ? kSlabs * (kSlabA / kSmallM) * p.a_rows : kBBoxes * kSmallBBytes);
+        mbar_expect_tx(bar, !is_a ? kBBoxes * kSmallBBytes : GATHER ? p.a_maps * p.a_rows * kGatherRow : kSlabs * (kSlabA / kSmallM) * p.a_rows);
+        if constexpr (GATHER) {
+          if (is_a)
+            for (int c = 0; c < p.a_maps; ++c) tma_load_3d(dst + c * 32 * kGatherRow, &tma_a.of[c], bar, k_elem, tm * 32, 0);
+        }
         // (a slab past the end of K, in the last step of an odd number, is a box outside the tensor: zeros)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int k = EXACT ? k_elem : A32 ? k_elem + j * 32 : k_elem + j * p.slab_k;
           if (is_a) {
-            if (j < kSlabs || A32) tma_load_3d(dst + j * kSmallABytes, &tma_a, bar, k, tm * kSmallM, 0);
+            if constexpr (!GATHER)
+              if (j < kSlabs || A32) tma_load_3d(dst + j * kSmallABytes, &tma_a, bar, k, tm * kSmallM, 0);
           } else if (j < kBBoxes) {
             const CUtensorMap* map = EXACT && j ? &tma_bt : &tma_b;
             if (p.b_kmajor) tma_load_3d(b_dst + j * kSmallBBytes, map, bar, k, tn * BN, 0);
@@ -257,8 +256,6 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       k_elem += kSlabs * p.slab_k;
       if (++s == p.stages) { s = 0; parity ^= 1; }
     }
-  } else if (warp == 0) {
-    // (GATHER: A is read by warps 2-9)
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     const uint64_t b_fixed = p.b_kmajor ? make_desc(0, 16, 1024) : make_desc(0, p.b_lbo, p.b_sbo, p.b_layout);
@@ -276,7 +273,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       ok = all_waited(mbar_wait(split0 + 8 * s, parity, abort_ptr), 2);        // this step's A is in tensor memory (and so its B has landed)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kSlabs * kSlabA)) >> 4;
+      const uint32_t b16 = (ring + (uint32_t)(s * kStage + kStageA)) >> 4;
       const uint32_t on = elect_one() ? 1u : 0u;
       // (the 14-bit address field: the CTA rank in the upper bits of a cluster's shared window must not spill over)
       auto desc = [&](uint32_t at) { return b_fixed | (uint64_t)(at & 0x3FFFu); };
@@ -337,7 +334,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     if (FIN != FIN_NONE && n < p.N) bias = load4(p.bias + n);
     auto load_res = [&](int r) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int m = m0 + band0 + r;
+      const int m = m0 + matrix_row<GATHER>(band0 + r);
       if (FIN == FIN_BIAS_RES && r < band_rows && m < p.M && n < p.N) x = load4(p.res + (int64_t)m * p.res_row + n);
       return x;
     };
@@ -386,23 +383,9 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       int s = ALTERNATE ? half : 0;
       uint32_t parity = 0;
       const int row = quad * 32 + lane;
-      // GATHER: a step ahead in registers, then through this warp's rows of the slab in shared memory
-      constexpr int kRaw = BF16 ? 64 : 32;
-      [[maybe_unused]] float raw[GATHER ? kRaw : 1];
-      [[maybe_unused]] auto fetch = [&](int i) {
-        if constexpr (GATHER)
-          gather_rows<BF16>(raw, p, m0 + quad * 32, ((step0 + i) * kSlabs + (ALTERNATE ? 0 : half)) * p.slab_k, lane);
-      };
-      if (GATHER && s < n_steps) fetch(s);
+      [[maybe_unused]] const int shift = GATHER ? p.a_shift[quad] : 0;
       for (int i = s; i < n_steps && ok; i += kEvery) {
         const int buf = i % kABuffers;
-        if constexpr (GATHER) {
-          // (what the MMAs read of this stage went to tensor memory: only this warp has used its rows)
-          __syncwarp();
-          park_rows<BF16>(smem_raw + (ring - raw_at) + s * kStage + (ALTERNATE ? 0 : half * kSlabA), raw, quad * 32, lane);
-          __syncwarp();
-          if (i + kEvery < n_steps) fetch(i + kEvery);
-        }
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
         // (loading and splitting A in front of this wait takes no less time: the issuing warp, in whose scheduler two of these
         // warps are, is held up by them then)
@@ -410,10 +393,28 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint8_t* const src = smem_raw + (ring - raw_at) + s * kStage + (ALTERNATE ? 0 : half * kSlabA) + row * 128;
+        const uint8_t* const src = smem_raw + (ring - raw_at) + s * kStage + (ALTERNATE ? 0 : half * (GATHER ? 128 : kSlabA)) + row * (GATHER ? kGatherRow : 128);
         float v[32];
+        if constexpr (GATHER) {
+          // the 32 (A32: 64) columns of this slab from `shift` on, a uniform number
+          auto from = [&](auto first) {
+            constexpr int S = decltype(first)::value;
+            float raw[A32 ? 68 : 36];
 #pragma unroll
-        for (int q = 0; q < (A32 ? 16 : 8); ++q) {
+            for (int q = 0; q < (A32 ? 17 : 9); ++q) {
+              const float4 x = *reinterpret_cast<const float4*>(src + 16 * q);
+              raw[4 * q] = x.x; raw[4 * q + 1] = x.y; raw[4 * q + 2] = x.z; raw[4 * q + 3] = x.w;
+            }
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] = A32 ? __uint_as_float(pack_bf16(raw[(2 * q + S) % 68], raw[(2 * q + 1 + S) % 68])) : raw[(q + S) % 36];
+          };
+          if (shift == 0) from(std::integral_constant<int, 0>());
+          else if (shift == 1) from(std::integral_constant<int, 1>());
+          else if (shift == 2) from(std::integral_constant<int, 2>());
+          else from(std::integral_constant<int, 3>());
+        }
+#pragma unroll
+        for (int q = GATHER ? 16 : 0; q < (A32 ? 16 : 8); ++q) {
           const float4 x = *reinterpret_cast<const float4*>(src + (q >> 3) * kSmallABytes + (((q & 7) ^ (row & 7)) << 4));
           if (A32) {
             v[2 * q] = __uint_as_float(pack_bf16(x.x, x.y)); v[2 * q + 1] = __uint_as_float(pack_bf16(x.z, x.w));
@@ -509,7 +510,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #pragma unroll 1
       for (int r = r0; r < band_rows; r += kRowsAtOnce) {
         const float4 res_next = load_res(r + kRowsAtOnce);
-        const int row = band0 + r, m = m0 + row;
+        const int row = band0 + r, m = m0 + matrix_row<GATHER>(row);
         const int swizzled = ((u ^ r) & 7) << 4;
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
         const uint8_t* part = area + (cb * band_rows + r) * 128 + swizzled;
@@ -554,7 +555,7 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           *reinterpret_cast<uint2*>(p.out16 + (int64_t)m * p.out_row + n) = packed;
         }
       }
-      if (EXACT && any_nan) redo_in_float32<FIN>(p, m0 + band0 + r0, min(p.M, m0 + band0 + band_rows), kRowsAtOnce, n);
+      if (EXACT && any_nan) redo_in_float32<FIN, GATHER>(p, m0, band0 + r0, band0 + band_rows, kRowsAtOnce, n);
     }
   }
   // (the warp has to be whole for an .aligned barrier)
@@ -576,11 +577,14 @@ mm_small_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 }
 
 using SmallKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, SmallParams);
+using GatherKernel = void (*)(GatherMaps, CUtensorMap, CUtensorMap, SmallParams);
 
 struct SmallState {
   CUtensorMap map_a, map_b, map_bt;
+  GatherMaps maps_a;
   SmallParams params;
-  SmallKernel kernel = nullptr;
+  SmallKernel kernel = nullptr;               // one of these two
+  GatherKernel gather = nullptr;
   unsigned grid = 0;
   size_t smem = 0;
   int bias_slot = -1, res_slot = -1;
@@ -591,37 +595,43 @@ struct SmallState {
 };
 
 template <int MODE, int BN, bool GATHER, bool DRAINS>
-SmallKernel small_kernel_of(int fin) {
+auto small_kernel_of(int fin) {
   switch (fin) {
-    case FIN_BIAS: return mm_small_kernel<MODE, FIN_BIAS, BN, GATHER, DRAINS>;
-    case FIN_BIAS_GELU: return mm_small_kernel<MODE, FIN_BIAS_GELU, BN, GATHER, DRAINS>;
-    case FIN_BIAS_RES: return mm_small_kernel<MODE, FIN_BIAS_RES, BN, GATHER, DRAINS>;
-    default: return mm_small_kernel<MODE, FIN_NONE, BN, GATHER, DRAINS>;
+    case FIN_BIAS: return &mm_small_kernel<MODE, FIN_BIAS, BN, GATHER, DRAINS>;
+    case FIN_BIAS_GELU: return &mm_small_kernel<MODE, FIN_BIAS_GELU, BN, GATHER, DRAINS>;
+    case FIN_BIAS_RES: return &mm_small_kernel<MODE, FIN_BIAS_RES, BN, GATHER, DRAINS>;
+    default: return &mm_small_kernel<MODE, FIN_NONE, BN, GATHER, DRAINS>;
   }
 }
 
-template <int MODE, bool DRAINS>
-SmallKernel small_kernel_of(int fin, int bn, bool gather) {
-  if constexpr (MODE == SMALL_EXACT) {
-    if (gather) return small_kernel_of<MODE, 64, true, DRAINS>(fin);
-  } else if constexpr (MODE != SMALL_BF16_A32) {
-    if (gather) return bn == 128 ? small_kernel_of<MODE, 128, true, DRAINS>(fin) : bn == 96 ? small_kernel_of<MODE, 96, true, DRAINS>(fin) : small_kernel_of<MODE, 64, true, DRAINS>(fin);
-  }
-  return bn == 128 ? small_kernel_of<MODE, 128, false, DRAINS>(fin) : bn == 96 ? small_kernel_of<MODE, 96, false, DRAINS>(fin) : small_kernel_of<MODE, 64, false, DRAINS>(fin);
+template <int MODE, bool GATHER, bool DRAINS>
+auto small_kernel_of(int fin, int bn) {
+  return bn == 128 ? small_kernel_of<MODE, 128, GATHER, DRAINS>(fin) : bn == 96 ? small_kernel_of<MODE, 96, GATHER, DRAINS>(fin) : small_kernel_of<MODE, 64, GATHER, DRAINS>(fin);
 }
 
-SmallKernel small_kernel(int mode, int fin, int bn, bool gather, bool drains) {
+SmallKernel small_kernel(int mode, int fin, int bn, bool drains) {
   switch (mode) {
-    case SMALL_BF16: return small_kernel_of<SMALL_BF16, false>(fin, bn, gather);
-    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32, false>(fin, bn, gather);
-    case SMALL_EXACT: return drains ? small_kernel_of<SMALL_EXACT, true>(fin, bn, gather) : small_kernel_of<SMALL_EXACT, false>(fin, bn, gather);
-    default: return small_kernel_of<SMALL_TF32, false>(fin, bn, gather);
+    case SMALL_BF16: return small_kernel_of<SMALL_BF16, false, false>(fin, bn);
+    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32, false, false>(fin, bn);
+    case SMALL_EXACT: return drains ? small_kernel_of<SMALL_EXACT, false, true>(fin, bn) : small_kernel_of<SMALL_EXACT, false, false>(fin, bn);
+    default: return small_kernel_of<SMALL_TF32, false, false>(fin, bn);
   }
 }
+
+GatherKernel gather_kernel(int mode, int fin, int bn, bool drains) {
+  switch (mode) {
+    case SMALL_BF16_A32: return small_kernel_of<SMALL_BF16_A32, true, false>(fin, bn);
+    case SMALL_EXACT: return drains ? small_kernel_of<SMALL_EXACT, true, true>(fin, bn) : small_kernel_of<SMALL_EXACT, true, false>(fin, bn);
+    default: return small_kernel_of<SMALL_TF32, true, false>(fin, bn);
+  }
+}
+
+// Floats between the 16-byte boundary in front of row c of A and the row.
+int gather_shift(const DevOperand& a, int c) { return (int)(reinterpret_cast<uintptr_t>(a.ptr + c * a.stride[1]) / sizeof(float) % 4); }
 
 int small_mode(int precision, SmallA form) {
   if (precision == KB200_PREC_FP32) return SMALL_EXACT;
-  return precision != KB200_PREC_BF16 ? SMALL_TF32 : form == SMALL_A_FLOAT32 ? SMALL_BF16_A32 : SMALL_BF16;
+  return precision != KB200_PREC_BF16 ? SMALL_TF32 : form == SMALL_A_MAPPED ? SMALL_BF16 : SMALL_BF16_A32;
 }
 
 // The chains this kernel finishes: nothing, + column, + column then GELU, + column + matrix.  `vectors`: whether all that it
@@ -719,6 +729,20 @@ int accumulate_limit(int64_t m, int64_t n, int64_t k, bool close) {
 
 struct SmallPlan { int bn, splits; int64_t cycles; };
 
+// Bytes behind the ring: the others' parts of a band, and the own partial tile where the ring cannot hold it.
+int exchange_bytes(int mode, int bn, bool gather, int splits, int stages) {
+  const int tile_bytes = kSmallM * bn * 4;
+  return tile_bytes / splits * (splits - 1) + (stages * stage_bytes_of(mode, bn, gather) >= tile_bytes ? 0 : tile_bytes);
+}
+
+// Stages of a CTA with `most` steps: all of them, as far as shared memory goes.
+int ring_stages(int mode, int bn, bool gather, int splits, int most) {
+  int stages = most < kSmallMaxStages ? most : kSmallMaxStages;
+  while ((size_t)stages * stage_bytes_of(mode, bn, gather) + exchange_bytes(mode, bn, gather, splits, stages) + 1024 > (size_t)kSmallSmem) --stages;
+  if (slabs_per_step(mode) == 1 && stages < most) stages &= ~1;              // a ring that is used again: see the warps that move A
+  return stages;
+}
+
 // Tile width, K split and estimated cycles, from fits to measured launches (128 to 1024 rows, 768 and 3072 of K, each
 // width and split).  A step, one 128-byte slab of K, is bound by shared memory: the operands land there
 // at 128 bytes a clock and every MMA reads its operands again (exact FP32: twelve of them, A from tensor
@@ -726,17 +750,17 @@ struct SmallPlan { int bn, splits; int64_t cycles; };
 // more have two blocks to a warp to drain, eight CTAs more to exchange.  (Plans in flight are no argument: results must not depend on them.)
 // 96 columns fit some row counts better than either neighbour (exact FP32: 1024 x 3072 x 768 36.4 -> 32.6 us,
 // 1024 x 768 x 3072 31.2 -> 27.8, 364 x 768 x 3072 22.3 -> 16.4).
-// GATHER: a warp loads, parks and reads back a slab of A one step ahead of its use, bound by the load/store unit (rows off the
-// lines: two of them to a load): what it adds to a step against the copied A (65 to 3000 of K).
+// GATHER: four copies to a step for one, and rows that start off the lines; with a ring of two stages (the other forms may have three in the
+// same memory) a step waits for its copies.  Copies of A in front of the kernel -> four maps, 384 launches of 2 to 1000 rows: 333 x 1000 x 771 TF32
+// 8.7 -> 7.0 us, 128 x 768 x 1537 BF16 7.7 -> 6.2, 600 x 1000 x 771 FP32 16.3 -> 13.3.
 SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, bool chunked, bool close, const Plan& plan) {
   const int64_t slab_k = mode == SMALL_BF16 || mode == SMALL_BF16_A32 ? 64 : 32, slabs = (k + slab_k - 1) / slab_k;
   SmallPlan best{64, 1, 0};
-  const int64_t fetch = !gather ? 0 : mode == SMALL_EXACT ? 600 : mode == SMALL_BF16 ? 1450 : 1100;
+  const int64_t fetch = !gather ? 0 : 150;
   const int asked_bn = plan.few_tiles % 1000, asked_splits = plan.few_tiles / 1000 % 10;
   for (int bn : {64, 96, 128}) {
     if (asked_bn != 0 && bn != asked_bn) continue;
     if (bn == 96 && chunked) continue;                  // an N-major B comes in chunks of 64 bf16 columns
-    if (bn > 64 && gather && mode == SMALL_EXACT) continue;      // rows of A and 64 sums do not fit the registers together
     const int64_t step = mode == SMALL_EXACT ? 435 + 4 * bn : mode == SMALL_BF16_A32 ? 450 + bn * 25 / 32 : 198 + bn * 13 / 8;
     const int64_t once = (bn == 64 ? 7500 : 10050) + (mode == SMALL_EXACT ? 600 : 0);
     const int64_t tiles = ((m + kSmallM - 1) / kSmallM) * ((n + bn - 1) / bn);
@@ -750,7 +774,9 @@ SmallPlan plan_small(int64_t m, int64_t n, int64_t k, int mode, bool gather, boo
       }
       const int64_t resident = resident_clusters(plan, s);
       const int64_t rounds = (tiles + resident - 1) / resident;
-      const int64_t cycles = rounds * ((steps + s - 1) / s * (slabs_per_step(mode) * step + fetch) + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
+      const int64_t most = (steps + s - 1) / s;
+      const int64_t short_ring = gather && most > 2 && ring_stages(mode, bn, gather, s, (int)most) < 3 ? slabs_per_step(mode) * step / 3 : 0;
+      const int64_t cycles = rounds * (most * (slabs_per_step(mode) * step + fetch + short_ring) + once + (s == 8 ? 1000 : s > 1 ? 350 : 0));
       if (best.cycles == 0 || cycles < best.cycles) best = {bn, s, cycles};
     }
   }
@@ -800,16 +826,10 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.splits = how.splits;
   p.tiles_n = (int)((k.N + bn - 1) / bn);
   const int64_t tiles = ((k.M + kSmallM - 1) / kSmallM) * p.tiles_n;
-  const int stage_bytes = stage_bytes_of(mode, bn);
+  const int stage_bytes = stage_bytes_of(mode, bn, gather);
   const int most = (p.num_steps + p.splits - 1) / p.splits;
-  p.stages = most < kSmallMaxStages ? most : kSmallMaxStages;
-  const int tile_bytes = kSmallM * bn * 4;
-  // the others' parts of a band, and the own partial tile where the ring cannot hold it
-  auto exchange_of = [&](int stages) { return tile_bytes / p.splits * (p.splits - 1) + (stages * stage_bytes >= tile_bytes ? 0 : tile_bytes); };
-  while ((size_t)p.stages * stage_bytes + exchange_of(p.stages) + 1024 > (size_t)kSmallSmem) --p.stages;
-  if (per_step == 1 && p.stages < most) p.stages &= ~1;                    // a ring that is used again: see the warps that move A
-  const int exchange = exchange_of(p.stages);
-  st->smem = (size_t)p.stages * stage_bytes + exchange + 1024;
+  p.stages = ring_stages(mode, bn, gather, p.splits, most);
+  st->smem = (size_t)p.stages * stage_bytes + exchange_bytes(mode, bn, gather, p.splits, p.stages) + 1024;
   st->grid = (unsigned)(tiles * p.splits);
   p.b_kmajor = ops.b_kmajor ? 1 : 0;
   p.b_static = ops.b_static ? 1 : 0;
@@ -846,7 +866,7 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.out_row = O.stride[1];
   p.out_tail = mode == SMALL_EXACT && vectors ? k.tail_out : nullptr;
   const DevOperand& A = k.ops[d.a_slot];
-  p.a = gather || mode == SMALL_EXACT ? A.ptr : nullptr;
+  p.a = mode == SMALL_EXACT ? A.ptr : nullptr;
   const DevOperand& B = k.ops[d.b_slot];
   p.b = B.ptr;
   p.b_k = B.stride[1];
@@ -855,18 +875,32 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   p.K = (int)k.K;
   // (Rows of shared memory that no box fills make accumulator rows that nobody reads.)
   p.a_rows = (int)(k.M < kSmallM ? k.M : kSmallM);
-  st->a_moves = form == SMALL_A_FLOAT32 || (!gather && ops.a_base == A.ptr);
+  st->a_moves = gather || form == SMALL_A_FLOAT32 || ops.a_base == A.ptr;
   st->b_moves = ops.b_base == k.ops[d.b_slot].ptr;
-  bool ok = gather || (form == SMALL_A_FLOAT32 ? encode_map(&st->map_a, false, A.ptr, k.K, k.M, 1, A.stride[1], 0, 32, p.a_rows, false)
+  bool ok = true;
+  if (gather) {
+    p.a_rows = (int)(k.M < kSmallM ? (k.M + 3) / 4 : kSmallM / 4);          // (rows that are not there cost a box as much as others)
+    p.a_maps = (int)(k.M < 4 ? k.M : 4);
+    for (int c = 0; c < p.a_maps && ok; ++c) {
+      p.a_shift[c] = gather_shift(A, c);
+      ok = encode_map_rows(&st->maps_a.of[c], A.ptr + c * A.stride[1] - p.a_shift[c], k.K + p.a_shift[c], (k.M - c + 3) / 4, 4 * A.stride[1], gather_pitch_floats(mode), p.a_rows);
+    }
+    for (int c = p.a_maps; c < 4; ++c) {           // (not used)
+      st->maps_a.of[c] = st->maps_a.of[0];
+      p.a_shift[c] = 0;
+    }
+  }
+  if (!gather) ok = (form == SMALL_A_FLOAT32 ? encode_map(&st->map_a, false, A.ptr, k.K, k.M, 1, A.stride[1], 0, 32, p.a_rows, false)
                                                : encode_map(&st->map_a, ops.bf16, ops.a_base, k.K, k.M, 1, ops.a_row, 0, slab_k, p.a_rows, false));
   if (ok && ops.b_kmajor) ok = encode_map(&st->map_b, ops.bf16, ops.b_base, k.K, k.N, 1, ops.b_row, 0, slab_k, bn, false);
   else if (ok) ok = encode_map4(&st->map_b, ops.bf16, ops.b_base, chunk, k.K, ops.b_cols / chunk, 1, ops.b_row, 0, slab_k, bn / chunk, !ops.bf16);
-  if (gather) st->map_a = st->map_b;          // not used
   st->map_bt = st->map_b;
   if (ok && b_tail) ok = set_map_address(&st->map_bt, b_tail);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = small_kernel(mode, fin, bn, gather, st->drains);
-  const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
+  if (gather) st->gather = gather_kernel(mode, fin, bn, st->drains);
+  else st->kernel = small_kernel(mode, fin, bn, st->drains);
+  const cudaError_t e = gather ? cudaFuncSetAttribute(st->gather, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem)
+                               : cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_small_kernel)"); }
   *state = st;
   return KB200_OK;
@@ -894,7 +928,8 @@ int small_launch(const Plan& plan, const void* state, cudaStream_t s) {
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  KB200_CUDA(cudaLaunchKernelEx(&cfg, st->kernel, st->map_a, st->map_b, st->map_bt, st->params));
+  if (st->gather) KB200_CUDA(cudaLaunchKernelEx(&cfg, st->gather, st->maps_a, st->map_b, st->map_bt, st->params));
+  else KB200_CUDA(cudaLaunchKernelEx(&cfg, st->kernel, st->map_a, st->map_b, st->map_bt, st->params));
   return KB200_OK;
 }
 
@@ -904,7 +939,11 @@ bool small_repoint(const PlanKernel& k, void* state) {
   if (st->res_slot >= 0) st->params.res = k.ops[st->res_slot].ptr;
   if (st->params.a) st->params.a = k.ops[k.desc.a_slot].ptr;
   if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
-  return (!st->a_moves || set_map_address(&st->map_a, k.ops[k.desc.a_slot].ptr)) &&
+  const DevOperand& A = k.ops[k.desc.a_slot];
+  bool ok = true;
+  for (int c = 0; st->gather && c < st->params.a_maps; ++c)      // (by a multiple of 16 bytes: the shifts stay)
+    ok = ok && set_map_address(&st->maps_a.of[c], A.ptr + c * A.stride[1] - st->params.a_shift[c]);
+  return ok && (st->gather || !st->a_moves || set_map_address(&st->map_a, A.ptr)) &&
          (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));
 }
 

@@ -7,7 +7,7 @@
 namespace kb200 {
 
 // How the kernel takes A: through a tensor map of ops.a_base (a mirror or a copy, or A itself), through one of the float32 A
-// for bf16 products, or read by its own warps, float32 at any pitch.
+// for bf16 products, or through four, float32 at any pitch.
 enum SmallA : int { SMALL_A_MAPPED, SMALL_A_FLOAT32, SMALL_A_GATHERED };
 
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.

@@ -351,6 +351,18 @@ inline bool encode_map(CUtensorMap* map, bool bf16, const void* base, int64_t co
   return r == CUDA_SUCCESS;
 }
 
+// Rows of float32 on any 16-byte pitch into rows of box_cols floats as they are, without a swizzle.
+inline bool encode_map_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int64_t row_stride_elems, int box_cols, int box_rows) {
+  EncodeFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
+  cuuint64_t strides[2] = {(cuuint64_t)row_stride_elems * 4, (cuuint64_t)(row_stride_elems * rows) * 4};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  cuuint32_t elem[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // A 4-D tiled map over an N-major matrix [batch, rows, n_chunks * chunk] seen as
 // (chunk, rows, n_chunks, batch): one box (chunk, box_rows, box_chunks, 1) lands in shared memory as
 // box_chunks consecutive blocks of [box_rows x chunk], the layout the N-major MMA descriptor walks.
