@@ -140,6 +140,7 @@ struct Plan {
   bool mirror_only = true;       // BF16 mode: an output that only mirror readers consume is not stored as float32
   bool others_in_flight = false; // KB200_OPT_OTHERS_IN_FLIGHT
   int concurrency = 1;           // plans the caller keeps in flight on this GPU at once (tile heuristics assume their share of the SMs)
+  std::vector<void*> scales;     // FP32: scales of float16 pairs whose bound is known, made when the plan is bound
   void* arena16 = nullptr;       // bf16 mirror of the arena (library-owned, only when some matmul reads it)
   uint64_t arena16_bytes = 0;
   // bound buffers (for re-validation and the tensor-core path)
@@ -195,6 +196,7 @@ void attention_tails_come_ready(PlanKernel& k);         // ... which the project
 bool matmul_writes_tails(const PlanKernel& k);
 bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);      // multiplies float16 pairs of A, split by a pass of its own ...
 void matmul_planes_come_ready(PlanKernel& k);                                   // ... or by A's producer
+bool matmul_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, const float* scale, bool store32);      // (see exact_write_pairs)
 bool attention_may_drop_float32(const PlanKernel& k);    // writes a bf16 copy, and its float32 rows only where they were planned
 void attention_drop_float32(PlanKernel& k);
 bool tc_eligible(const PlanKernel& k);

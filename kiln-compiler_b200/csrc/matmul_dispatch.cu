@@ -13,6 +13,7 @@ std::string tc_detail(const PlanKernel& k);
 bool tc_writes_tails(const PlanKernel& k);
 bool tc_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);
 void tc_planes_come_ready(PlanKernel& k);
+bool tc_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, const float* scale, bool store32);
 
 int choose_matmul(Plan& plan, PlanKernel& k) {
   (void)plan;
@@ -49,6 +50,9 @@ std::string matmul_detail(const PlanKernel& k) { return tc_detail(k); }
 
 bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes) { return k.impl == IMPL_MM_TC && tc_takes_planes(k, planes); }
 void matmul_planes_come_ready(PlanKernel& k) { tc_planes_come_ready(k); }
+bool matmul_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, const float* scale, bool store32) {
+  return k.impl == IMPL_MM_TC && tc_write_pairs(k, to, scale, store32);
+}
 bool matmul_writes_tails(const PlanKernel& k) { return k.impl == IMPL_MM_TC && tc_writes_tails(k); }
 
 void destroy_matmul(PlanKernel& k) { tc_destroy(k); }

@@ -159,6 +159,8 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   p.stream_out = streams_out(plan, k, k.chain.out_slot, k.M * k.N) ? 1 : 0;
   const DevOperand& O = k.ops[k.chain.out_slot];
   p.with_tail = k.tail_out != nullptr ? 1 : 0;
+  p.pair_scale = nullptr;
+  p.store32 = 1;
   // Persistent pairs, up to this plan's share of the GPU with several in flight.
   const int pairs = plan.sm_count / 2, share = plan.concurrency > 1 && pairs / plan.concurrency > 0 ? pairs / plan.concurrency : pairs;
   const int rounds = (p.num_tiles + share - 1) / share;
@@ -210,6 +212,16 @@ bool exact_repoint(const PlanKernel& k, void* state) {
 std::string exact_detail(const void* state) {
   const ExactState* st = static_cast<const ExactState*>(state);
   return "mm_exact " + std::to_string(st->params.bn) + " columns" + (st->split ? ", 2 splits" : "");
+}
+
+bool exact_write_pairs(const PlanKernel& k, void* state, const PlanKernel::Planes& to, const float* scale, bool store32) {
+  ExactState* st = static_cast<ExactState*>(state);
+  if (st->params.with_tail || st->res_slot >= 0 ||
+      !encode_map_store(&st->map_tail, true, to.heads, k.N, k.M, 2, to.pitch, to.plane))
+    return false;
+  st->params.pair_scale = scale;
+  st->params.store32 = store32 ? 1 : 0;
+  return true;
 }
 
 bool exact_writes_tails(const void* state) { return static_cast<const ExactState*>(state)->params.with_tail != 0; }

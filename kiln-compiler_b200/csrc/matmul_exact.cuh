@@ -24,6 +24,7 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
@@ -76,6 +77,10 @@ struct ExactParams {
   int64_t a_row, b_k, b_n, K;
   int stream_out;        // the output leaves L2 first: see streams_out
   int with_tail;         // the output minus its 19 leading bits is stored as well, for a consumer that splits it
+  // ... or float16 pairs of it, times a power of two for every 32 columns: its bound is known (see layernorm_bounds), its rows hold no
+  // infinities where those of A hold none, and the float32 output may be left out
+  const float* pair_scale;
+  int store32;
 };
 
 // Results of a row of A with infinities, whose float16 terms are NaN, done over as the CUDA cores do them, in the block of 32 x 32 that a
@@ -103,6 +108,26 @@ __device__ __forceinline__ void add_staged(float (&v)[32], const uint8_t* block,
     const float2 a = fadd2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(t.x, t.y));
     const float2 b = fadd2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(t.z, t.w));
     v[4 * q] = a.x; v[4 * q + 1] = a.y; v[4 * q + 2] = b.x; v[4 * q + 3] = b.y;
+  }
+}
+
+// A 32 x 32 block, this lane's row, as float16 pairs: 64-byte rows of heads, then those of tails, swizzled as the 16-bit store maps want them.
+__device__ __forceinline__ void stage_pairs(uint8_t* block, const float (&v)[32], int lane, float scale) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t h[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = fmul2(make_float2(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]), make_float2(scale, scale));
+      const __half2 head = __floats2half2_rn(x.x, x.y);
+      const float2 back = __half22float2(head);
+      const __half2 tail = __floats2half2_rn(x.x - back.x, x.y - back.y);
+      h[i] = *reinterpret_cast<const uint32_t*>(&head);
+      t[i] = *reinterpret_cast<const uint32_t*>(&tail);
+    }
+    uint8_t* const at = block + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4);
+    *reinterpret_cast<uint4*>(at) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(at + 2048) = make_uint4(t[0], t[1], t[2], t[3]);
   }
 }
 
@@ -428,14 +453,28 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           add_staged(v, at_ptr, lane);
         }
         __syncwarp();
-        stage_rows(at_ptr, at_ptr, v, lane, false);
         const bool redo = row_scale < 0.0f && !dry;
-        if (redo) redo_row<FIN>(p, at_ptr, lane, m_first + lane, n);
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0 && !dry) {
-          tma_store_3d(&tma_out, at, n, m_first, 0, policy);
-          tma_store_commit();
+        if (p.store32) {
+          stage_rows(at_ptr, at_ptr, v, lane, false);
+          if (redo) redo_row<FIN>(p, at_ptr, lane, m_first + lane, n);
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0 && !dry) {
+            tma_store_3d(&tma_out, at, n, m_first, 0, policy);
+            tma_store_commit();
+          }
+        }
+        if (p.pair_scale != nullptr) {
+          if (p.store32 && lane == 0) store_wait_read(0);
+          __syncwarp();
+          stage_pairs(at_ptr, v, lane, __ldg(p.pair_scale + (n >> 5)));
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0 && !dry) {
+            tma_store_3d(&tma_tail, at, n, m_first, 0);
+            tma_store_3d(&tma_tail, at + 2048, n, m_first, 1);
+            tma_store_commit();
+          }
         }
         if (p.with_tail && !dry) {
           if (redo) {

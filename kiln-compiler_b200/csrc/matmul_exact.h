@@ -22,10 +22,15 @@ int exact_launch(const Plan& plan, const void* state, cudaStream_t s);
 bool exact_repoint(const PlanKernel& k, void* state);      // the operand pointers of `k` have moved
 std::string exact_detail(const void* state);
 bool exact_writes_tails(const void* state);
+// Float16 pairs of the output into `to` as well, times `scale` by 32 columns, or only those.  False: not this launch.
+bool exact_write_pairs(const PlanKernel& k, void* state, const PlanKernel::Planes& to, const float* scale, bool store32);
 void exact_destroy(void* state);
 
 // float32 rows of `cols` elements -> the two planes and the scales.  A pass in front of a launch, or once for a weight.
 int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, int64_t rows, int64_t cols, bool pdl, cudaStream_t s);
+// |LayerNorm(x) B + bias| per column of B [K, N] for any x, at most: of the normalised row, 1 / sqrt(inv_n) long, by Cauchy and Schwarz.  `bounds`: [n]
+// on the host.  Synchronises.
+int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds);
 // Do float16 pairs hold this weight [K, N] as well as TF32 pairs would, whatever A is?  Synchronises.
 int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, bool* suits);
 

@@ -1577,6 +1577,11 @@ void tc_planes_come_ready(PlanKernel& k) {
   k.launches = 1;
 }
 
+bool tc_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, const float* scale, bool store32) {
+  TcState* st = static_cast<TcState*>(k.tc);
+  return st && st->exact && exact_write_pairs(k, st->exact, to, scale, store32);
+}
+
 void tc_destroy(PlanKernel& k) {
   TcState* st = static_cast<TcState*>(k.tc);
   if (!st) return;

@@ -1,12 +1,14 @@
 // The C ABI of libkb200.so: descriptor validation, buffer binding with bounds checks, launch
 // dispatch.  Declared and documented in include/kb200.h.
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <new>
 
 #include "kb200_internal.h"
+#include "matmul_exact.h"
 
 #define KB200_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -967,25 +969,98 @@ static int assign_shadows(Plan& plan) {
   return KB200_OK;
 }
 
-// Exact FP32 on float16 pairs of a LayerNorm's rows: the LayerNorm, which has a row in registers, splits it; no pass in front of the
-// matmul does, and the float32 rows are not stored where nobody else reads them.  (1024 x 768: QKV 16.3 -> 13.5 us, fc + GELU 19.2 -> 16.5.)
-static void hand_on_planes(Plan& plan) {
+// The LayerNorm that writes exactly operand A of this matmul, in rows of float4, or null.
+static PlanKernel* layernorm_in_front(Plan& plan, size_t ki) {
+  PlanKernel& k = plan.kernels[ki];
+  const int a = k.desc.a_slot;
+  const Span x = span_of(k, a);
+  if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) return nullptr;
+  PlanKernel* const from = mirroring_producer(plan, ki, x);
+  if (from == nullptr || from->impl != IMPL_ROW_LAYERNORM || !from->row_vec) return nullptr;
+  const DevOperand &out = from->ops[from->out_slot], &in = k.ops[a];
+  return out.ptr == in.ptr && out.stride[0] == in.stride[1] && from->desc.iter_shape[0] == k.M && from->desc.iter_shape[1] == k.K ? from : nullptr;
+}
+
+// Bounds of a matmul's results by column, whatever the input: of a LayerNorm's rows and frozen parameters, with a bias and a GELU (which is
+// no larger than its argument).  *bounds stays empty where nothing is known.
+static int result_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
+  const PlanKernel& k = plan.kernels[ki];
+  bounds->clear();
+  const PlanKernel* const norm = layernorm_in_front(plan, ki);
+  auto frozen = [](const PlanKernel& of, int slot) { return of.desc.operands[slot].base_kind == KB200_BASE_CONST; };
+  if (norm == nullptr || !frozen(*norm, norm->g_slot) || !frozen(*norm, norm->b_slot) || !(norm->ln_inv_n > 0.0f) || !(norm->ln_eps >= 0.0f)) return KB200_OK;
+  if (k.batch != 1 || !k.has_chain || k.n_ops != k.desc.n_operands || !frozen(k, k.desc.b_slot) || k.chain.n > 2) return KB200_OK;
+  const float* bias = nullptr;
+  if (k.chain.n >= 1) {
+    const ChainStep& s = k.chain.steps[0];
+    if (s.op != CH_ADD || s.slot < 0 || !frozen(k, s.slot) || k.ops[s.slot].stride[1] != 0 || k.ops[s.slot].stride[2] != 1) return KB200_OK;
+    bias = k.ops[s.slot].ptr;
+  }
+  if (k.chain.n == 2 && k.chain.steps[1].op != CH_GELU_TANH) return KB200_OK;
+  const DevOperand& B = k.ops[k.desc.b_slot];
+  const int rc = layernorm_bounds(B.ptr, B.stride[1], B.stride[2], k.K, k.N, norm->ops[norm->g_slot].ptr, norm->ops[norm->b_slot].ptr, bias, norm->ln_inv_n, bounds);
+  if (rc) return rc;
+  for (float b : *bounds)
+    if (!(b < 1e30f)) { bounds->clear(); break; }
+  return KB200_OK;
+}
+
+// `host` on the device, for as long as the plan is bound as it is.  Null where memory is short.
+static float* keep_scales(Plan& plan, const std::vector<float>& host) {
+  float* device = nullptr;
+  if (cudaMalloc(&device, host.size() * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  plan.scales.push_back(device);
+  return cudaMemcpy(device, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess ? device : nullptr;
+}
+
+// The power of two that brings what is at most `bound` to 2^14 to 2^15.
+static float pair_scale(float bound) {
+  int e = 0;
+  frexpf(bound > 1e-30f ? bound : 1e-30f, &e);
+  return ldexpf(1.0f, 15 - e);
+}
+
+// Exact FP32 on float16 pairs whose producer can write them: no pass in front of the matmul splits its rows, and the float32 rows are not stored
+// where nobody else reads them.  A LayerNorm has a row in registers and finds its scale; a matmul behind one has a scale for all rows, by
+// the bound of its results.  (1024 x 768: QKV 16.3 -> 13.0 us, fc + GELU 19.2 -> 15.9; projection behind it 20.2 -> 17.0.)
+static int hand_on_planes(Plan& plan) {
   for (size_t ki = 0; ki < plan.kernels.size(); ++ki) {
     PlanKernel& k = plan.kernels[ki];
     PlanKernel::Planes planes;
     if (k.desc.kclass != KB200_K_MATMUL || !matmul_takes_planes(k, &planes)) continue;
     const int a = k.desc.a_slot;
+    auto reads_here = [&](const PlanKernel& r, int slot) { return &r == &k && slot == a; };
+    if (PlanKernel* const norm = layernorm_in_front(plan, ki)) {
+      if (norm->planes_out.heads != nullptr) continue;
+      norm->planes_out = planes;
+      matmul_planes_come_ready(k);
+      norm->mirror_only = plan.mirror_only && only_read_as(plan, (size_t)(norm - plan.kernels.data()), span_of(*norm, norm->out_slot), reads_here);
+      continue;
+    }
     const Span x = span_of(k, a);
     if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) continue;
     PlanKernel* const from = mirroring_producer(plan, ki, x);
-    if (from == nullptr || from->impl != IMPL_ROW_LAYERNORM || from->planes_out.heads != nullptr || !from->row_vec) continue;
-    const DevOperand &out = from->ops[from->out_slot], &in = k.ops[a];
-    if (out.ptr != in.ptr || out.stride[0] != in.stride[1] || from->desc.iter_shape[0] != k.M || from->desc.iter_shape[1] != k.K) continue;
+    if (from == nullptr || from->impl != IMPL_MM_TC || from->planes_out.heads != nullptr || from->M != k.M || from->N != k.K) continue;
+    const DevOperand &out = from->ops[from->chain.out_slot], &in = k.ops[a];
+    if (out.ptr != in.ptr || out.stride[1] != in.stride[1]) continue;
+    const size_t fi = (size_t)(from - plan.kernels.data());
+    std::vector<float> bounds;
+    const int rc = result_bounds(plan, fi, &bounds);
+    if (rc) return rc;
+    if (bounds.empty()) continue;
+    const float scale = pair_scale(*std::max_element(bounds.begin(), bounds.end()));
+    const float* const by = keep_scales(plan, std::vector<float>((size_t)(from->N + 31) / 32, scale));
+    const bool alone = plan.mirror_only && only_read_as(plan, fi, span_of(*from, from->chain.out_slot), reads_here);
+    if (by == nullptr || !matmul_write_pairs(*from, planes, by, !alone)) continue;
     from->planes_out = planes;
+    const std::vector<float> back((size_t)k.M, 1.0f / scale);
+    KB200_CUDA(cudaMemcpy(planes.scales, back.data(), back.size() * sizeof(float), cudaMemcpyHostToDevice));
     matmul_planes_come_ready(k);
-    from->mirror_only = plan.mirror_only && only_read_as(plan, (size_t)(from - plan.kernels.data()), span_of(*from, from->out_slot),
-                                                         [&](const PlanKernel& r, int slot) { return &r == &k && slot == a; });
   }
+  return KB200_OK;
 }
 
 constexpr size_t kMaxIo = 16;      // inputs and outputs (each) a call may bring buffers for
@@ -1157,6 +1232,8 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   int prev = 0;
   cudaGetDevice(&prev);
   KB200_CUDA(cudaSetDevice(plan.device));
+  for (void* p : plan.scales) cudaFree(p);
+  plan.scales.clear();
   int rc = KB200_OK;
   // phase 1: resolve pointers, pick an implementation per kernel
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
@@ -1228,7 +1305,7 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     for (const PlanKernel& k : plan.kernels)
       if (plan.kernels[i].impl == IMPL_ATTN_FUSED && k.tail_out != nullptr && k.tail_out == attention_tails(plan.kernels[i]) && matmul_writes_tails(k))
         attention_tails_come_ready(plan.kernels[i]);
-  if (rc == KB200_OK) hand_on_planes(plan);
+  if (rc == KB200_OK) rc = hand_on_planes(plan);
   cudaSetDevice(prev);
   if (rc) return rc;
   collect_io_refs(plan);
@@ -1403,6 +1480,7 @@ KB200_EXPORT void kb200_plan_destroy(kb200_plan* p) {
   }
   if (plan->d_status) cudaFree(plan->d_status);
   if (plan->arena16) cudaFree(plan->arena16);
+  for (void* scale : plan->scales) cudaFree(scale);
   cudaSetDevice(prev);
   delete plan;
 }

@@ -10,6 +10,8 @@
 // sign and the worst size; 1e-8 in the mean), and other weights keep the other kernels (`split_suits`).
 //
 // What bounds the pass: it is a launch of ~2.3 us in front of a matmul; 4 bytes read and 4 written per element.
+#include <math.h>
+
 #include "kb200_internal.h"
 #include "matmul_exact.h"
 #include "split16.cuh"
@@ -80,7 +82,46 @@ __global__ void __launch_bounds__(256) largest_kernel(const float* __restrict__ 
   if (threadIdx.x == 0) out[blockIdx.x] = most;
 }
 
+// One block per column of a weight: see layernorm_bounds.
+__global__ void __launch_bounds__(256) bound_kernel(const float* __restrict__ b, int64_t b_k, int64_t b_n, int k, const float* __restrict__ gamma,
+                                                    const float* __restrict__ beta, const float* __restrict__ bias, float length, float* __restrict__ out) {
+  __shared__ float partial[2][8];
+  const float* const column = b + blockIdx.x * b_n;
+  float squares = 0.0f, shifts = 0.0f;
+  for (int i = threadIdx.x; i < k; i += 256) {
+    const float w = column[i * b_k], g = gamma[i] * w;
+    squares += g * g;
+    shifts += fabsf(beta[i] * w);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    squares += __shfl_xor_sync(0xffffffffu, squares, o);
+    shifts += __shfl_xor_sync(0xffffffffu, shifts, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    partial[0][threadIdx.x >> 5] = squares;
+    partial[1][threadIdx.x >> 5] = shifts;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      squares += partial[0][w];
+      shifts += partial[1][w];
+    }
+    out[blockIdx.x] = 1.01f * (length * sqrtf(squares) + shifts + (bias != nullptr ? fabsf(bias[blockIdx.x]) : 0.0f));      // (1 %: float32 sums)
+  }
+}
+
 }  // namespace
+
+int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds) {
+  bounds->assign((size_t)n, INFINITY);
+  float* device = nullptr;
+  KB200_CUDA(cudaMalloc(&device, (size_t)n * sizeof(float)));
+  cudaError_t e = launch_kernel(false, bound_kernel, dim3((unsigned)n), dim3(256), 0, nullptr, b, b_k, b_n, (int)k, gamma, beta, bias, sqrtf(1.0f / inv_n), device);
+  if (e == cudaSuccess) e = cudaMemcpy(bounds->data(), device, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost);
+  cudaFree(device);
+  return e == cudaSuccess ? KB200_OK : cuda_fail(e, "the bounds of a matmul's results");
+}
 
 int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, int64_t rows, int64_t cols, bool pdl, cudaStream_t s) {
   __half* const heads = static_cast<__half*>(planes);

@@ -183,3 +183,32 @@ def test_infinities_a_layernorm_makes():
     want = h5[:, None] * torch.from_numpy(consts["fc.weight.transpose"][5]).cuda()
     rows = torch.arange(1024, device="cuda") != 9
     assert torch.equal(got[rows], want[rows]) and bool(got[9].isnan().all())
+
+
+@pytest.mark.parametrize("m,d,wide", [(1024, 768, 3072), (1000, 772, 3004), (2048, 512, 2048)])
+@pytest.mark.parametrize("gelu", [True, False])
+def test_a_matmul_behind_a_layernorm_leaves_its_rows_split(m, d, wide, gelu):
+    """Its results have a known bound: two Linears and the LayerNorm in front are three launches, and a row of NaN stays one."""
+    from perf import cases
+
+    p = cases._Plan("mlp", (m, d), (m, d))
+    h, f = p.buffer(m, d), p.buffer(m, wide)
+    p.layernorm(p.x, "ln.", h)
+    p.linear(h, "fc.", wide, f, gelu=gelu)
+    p.linear(f, "proj.", d, p.y)
+    plan = p.spec()
+    consts = cases._constants(plan.const_shapes, np.random.default_rng(0))
+    consts["fc.bias"] += np.float32(3)
+    x = torch.randn(m, d, device="cuda") * torch.exp2(torch.linspace(-20, 20, m, device="cuda"))[:, None]
+    x[7, 3] = float("nan")
+    exe, got = run_plan(plan, consts, x)
+    assert all("mm_exact" in detail and "A copied" not in detail for detail in exe.details[1:]) and exe.device_launches == 3, exe.details
+    _, stored = run_plan(plan, consts, x, KILN_GPU_MIRROR_ONLY="0")
+    assert torch.equal(got.nan_to_num(), stored.nan_to_num())
+    c = {name: torch.from_numpy(v).cuda().double() for name, v in consts.items()}
+    h = torch.nn.functional.layer_norm(x.double(), (d,), c["ln.weight"], c["ln.bias"], 1e-5)
+    f = h @ c["fc.weight.transpose"] + c["fc.bias"]
+    want = (torch.nn.functional.gelu(f, approximate="tanh") if gelu else f) @ c["proj.weight.transpose"] + c["proj.bias"]
+    rows = torch.arange(m, device="cuda") != 7
+    assert bool(got[7].isnan().all())
+    assert float((got.double() - want)[rows].norm() / want[rows].norm()) <= 3 * BOUND
