@@ -33,10 +33,13 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <utility>
 #include <vector>
 
 #include "attention.h"
+#include "attention_pairs.cuh"
+#include "attention_softmax.cuh"
 #include "device_math.cuh"
 #include "kb200_internal.h"
 #include "tc_common.cuh"
@@ -80,6 +83,11 @@ struct AttnF32Params {
   int split_from;
   float* partial;            // [split item][2 halves][64 x 64 output | 64 maxima | 64 sums]
   int* arrivals;             // [split item], zero between launches
+  // The rows as float16 pairs as well (see split_rows.cu), times `pair_scale`: their bound is known; or null.  store32: and as float32
+  __half* heads;
+  int64_t plane, pitch;
+  float pair_scale;
+  int store32;
 };
 constexpr int kFPartialFloats = kFTile * kHeadDim + 2 * kFTile;
 
@@ -115,6 +123,21 @@ struct AttnState {
   const float* span_lo = nullptr;
   int64_t span_n4 = 0;
   bool tails_ready = false;        // ... written by the projection in front
+  // FP32 mode on float16 pairs (attention_pairs.cuh): planes of the projection's whole output, written by it or by a pass over it
+  struct Pairs {
+    bool used = false, ready = false;
+    const float* src = nullptr;    // that output: rows x cols, src_row apart
+    int64_t src_row = 0, rows = 0, cols = 0, pitch = 0;
+    void* planes = nullptr;
+    float* factors = nullptr;      // [H] qk | [H] v_back | scale of the merged heads' pairs | [cols / 32] scales of the planes
+    CUtensorMap q, k, v, qt, kt, vt, outh, outt;
+    PairsParams params;
+    const float* by() const { return factors + 2 * params.a.H + 1; }
+  } pairs;
+  float out_bound = 0.0f;          // FP32 mode: of the merged heads, convex combinations of V's rows, where it is known
+  bool ieee = false;               // the plan asked for IEEE behaviour on non-finite operands
+  bool asked = false;              // a kernel was asked for by option
+  bool may_split = false;
   bool own_pass = false;           // ... always by a pass of this launch's own: asked for by option, the kernel runs by itself, whatever is in front
 };
 
@@ -138,37 +161,6 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const float4* __restrict
   pdl_wait();                 // the producer of this kernel's inputs has completed
   pdl_launch_dependents();    // the next kernel may begin its start-up
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) dst[i] = src[i];
-}
-
-// Scores of one 32-column block -> probabilities, in place; returns their sum.  `first_col` is the
-// block's first key relative to the query tile's first row (only used on the diagonal tile).
-template <bool DIAGONAL>
-__device__ __forceinline__ float probabilities32(float (&v)[32], float scale_log2, float m_use, int first_col, int row) {
-  const float2 scale2 = make_float2(scale_log2, scale_log2), shift2 = make_float2(-m_use, -m_use);
-  float2 sum2 = make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    const float2 t = ffma2(make_float2(v[i], v[i + 1]), scale2, shift2);     // two exponents per instruction
-    float2 pr = make_float2(ex2(t.x), ex2(t.y));
-    if (DIAGONAL && first_col + i > row) pr.x = 0.0f;
-    if (DIAGONAL && first_col + i + 1 > row) pr.y = 0.0f;
-    v[i] = pr.x;
-    v[i + 1] = pr.y;
-    sum2 = fadd2(sum2, pr);
-  }
-  return sum2.x + sum2.y;
-}
-template <bool DIAGONAL>
-__device__ __forceinline__ float row_max32(const float (&v)[32], float m, int first_col, int row) {
-  if (DIAGONAL) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (first_col + i <= row) m = fmaxf(m, v[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) m = fmax3(m, v[i], v[i + 1]);
-  }
-  return m;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -387,8 +379,12 @@ __global__ void __launch_bounds__(kFThreads, 2) attention_fp32_kernel(const __gr
   for (int i = 0; i < kFRows; ++i) {
     if (qt * kFTile + ty + 8 * i >= p.T) break;
     const float inv = 1.0f / l_run[i];
-    *reinterpret_cast<float4*>(og + (int64_t)(ty + 8 * i) * p.out_row_stride) =
-        make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
+    const float4 y = make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
+    if (p.store32) *reinterpret_cast<float4*>(og + (int64_t)(ty + 8 * i) * p.out_row_stride) = y;
+    if (p.heads != nullptr) {
+      __half* const at = p.heads + (row0 + (int64_t)qt * kFTile + ty + 8 * i) * p.pitch + h * kHeadDim + 4 * tx;
+      store_terms(at, at + p.plane, y, p.pair_scale);
+    }
   }
 }
 
@@ -888,6 +884,31 @@ struct AttnChain {
   bool ieee = false;                  // ... and were asked to behave like FMA matmuls on non-finite operands (config bit 1024)
 };
 
+// Split tiles' partial results, counters and order, and what `runs` CTAs keep between runs of key tiles.
+bool split_workspace(AttnState* st, const std::vector<int>& entries, int64_t runs) {
+  AttnParams& p = st->params;
+  const int64_t split_tiles = (int64_t)p.B * p.H * (p.q_tiles - p.split_from);
+  const size_t partial_bytes = (size_t)split_tiles * 2 * kAttnPartialFloats * sizeof(float);
+  const size_t counter_bytes = (size_t)split_tiles * 4 * sizeof(int);
+  const std::vector<unsigned short> order(entries.begin(), entries.end());
+  const size_t order_bytes = (order.size() * sizeof(unsigned short) + 15) & ~size_t(15);
+  const size_t kept_bytes = runs * kAttnPartialFloats * sizeof(float);
+  if (cudaMalloc(&st->split_scratch, partial_bytes + counter_bytes + order_bytes + kept_bytes) != cudaSuccess ||
+      cudaMemset(static_cast<uint8_t*>(st->split_scratch) + partial_bytes, 0, counter_bytes) != cudaSuccess ||
+      cudaMemcpy(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes, order.data(),
+                 order.size() * sizeof(unsigned short), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaGetLastError();
+    if (st->split_scratch) cudaFree(st->split_scratch);
+    st->split_scratch = nullptr;
+    return false;
+  }
+  p.partial = static_cast<float*>(st->split_scratch);
+  p.arrivals = reinterpret_cast<int*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes);
+  p.order = reinterpret_cast<const unsigned short*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes);
+  if (runs > 0) p.kept = reinterpret_cast<float*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes + order_bytes);
+  return true;
+}
+
 // Shared tail of the two matchers: the intermediates must be dead afterwards, the mask causal; then
 // the state is built and the plan kernels are marked.
 bool finish_fusion(Plan& plan, const AttnChain& c) {
@@ -939,6 +960,8 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   // its last tokens reads zeros behind them (as the stores' maps drop those rows): any length works.
   AttnState* st = new AttnState();
   st->exact = c.exact;
+  st->ieee = c.ieee;
+  st->asked = plan.fp32_attention == 1;
   // FP32 mode: the CUDA-core kernel (64 queries per CTA, long prefixes split), or the tensor-core kernel (128 queries and a pass
   // over Q, K and V for their tails) for sequences of whole tiles that fill a quarter of the SMs, where that is estimated
   // faster.  Both estimates are a line through launches of 16 to 333 tokens and 4 to 96 heads, in ns: a fixed part, key
@@ -1049,6 +1072,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   p.order = nullptr;
   const bool may_split = plan.concurrency == 1 &&          // (other plans in flight fill the SMs this one leaves idle)
                          plan.attention_split;
+  st->may_split = may_split;
   if (c.bf16 && !aliased) {      // (the kernel for bf16 operands, unless nobody writes them)
     const AttnSchedule schedule = attention_bf16_schedule(B * H, p.q_tiles, plan.sm_count, may_split);
     p.split_from = schedule.split_from;
@@ -1059,28 +1083,11 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   p.kept = nullptr;
   const std::vector<int> entries = attention_item_order(p.q_tiles, p.split_from);
   const bool runs = c.bf16 && !aliased && attention_item_tiles(entries[0], p.split_from) > kAttnRun;
-  if (p.split_from < p.q_tiles || runs) {
-    const int64_t split_tiles = B * H * (p.q_tiles - p.split_from);
-    const size_t partial_bytes = (size_t)split_tiles * 2 * kAttnPartialFloats * sizeof(float);
-    const size_t counter_bytes = (size_t)split_tiles * 4 * sizeof(int);
-    const std::vector<unsigned short> order(entries.begin(), entries.end());
-    const size_t order_bytes = (order.size() * sizeof(unsigned short) + 15) & ~size_t(15);
-    const size_t kept_bytes = runs ? attention_bf16_ctas(st->alone, plan.sm_count) * kAttnPartialFloats * sizeof(float) : 0;
-    if (cudaMalloc(&st->split_scratch, partial_bytes + counter_bytes + order_bytes + kept_bytes) != cudaSuccess ||
-        cudaMemset(static_cast<uint8_t*>(st->split_scratch) + partial_bytes, 0, counter_bytes) != cudaSuccess ||
-        cudaMemcpy(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes, order.data(),
-                   order.size() * sizeof(unsigned short), cudaMemcpyHostToDevice) != cudaSuccess) {
-      cudaGetLastError();
-      if (st->split_scratch) cudaFree(st->split_scratch);
-      if (st->staged_out) cudaFree(st->staged_out);
-      if (st->tails) cudaFree(st->tails);
-      delete st;
-      return false;
-    }
-    p.partial = static_cast<float*>(st->split_scratch);
-    p.arrivals = reinterpret_cast<int*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes);
-    p.order = reinterpret_cast<const unsigned short*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes);
-    if (runs) p.kept = reinterpret_cast<float*>(static_cast<uint8_t*>(st->split_scratch) + partial_bytes + counter_bytes + order_bytes);
+  if ((p.split_from < p.q_tiles || runs) && !split_workspace(st, entries, runs ? attention_bf16_ctas(st->alone, plan.sm_count) : 0)) {
+    if (st->staged_out) cudaFree(st->staged_out);
+    if (st->tails) cudaFree(st->tails);
+    delete st;
+    return false;
   }
   const int64_t items = B * H * (p.q_tiles + (p.q_tiles - p.split_from));
   st->grid = dim3((unsigned)(items < plan.sm_count ? items : plan.sm_count), 1, 1);     // persistent: at most one CTA per SM
@@ -1098,6 +1105,8 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     const int64_t n_split = f.q_tiles - f.split_from, split_items = B * H * n_split;
     f.partial = nullptr;
     f.arrivals = nullptr;
+    f.heads = nullptr;
+    f.store32 = 1;
     if (split_items > 0) {
       const size_t partial_bytes = (size_t)split_items * 2 * kFPartialFloats * sizeof(float);
       if (cudaMalloc(&st->f32_scratch, partial_bytes + (size_t)split_items * sizeof(int)) != cudaSuccess ||
@@ -1334,7 +1343,16 @@ bool attention_wants_bf16(const PlanKernel& k) { return k.attn && static_cast<co
 int attention_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
   const AttnState* st = static_cast<const AttnState*>(k.attn);
   const bool split = st->params.split_from < st->params.q_tiles;     // some query tiles are shared by two CTAs
-  if (st->exact_tc) {
+  if (st->pairs.used) {
+    const AttnState::Pairs& h = st->pairs;
+    if (!h.ready) {
+      const int64_t blocks = (h.rows * (h.cols / 4) + 1023) / 1024;
+      KB200_CUDA(launch_kernel(plan.pdl, attention_pairs_pass, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), dim3(256), 0, s, h.src, h.src_row,
+                               static_cast<__half*>(h.planes), h.rows * h.pitch, h.pitch, h.by(), (uint32_t)h.rows, (uint32_t)(h.cols / 4)));
+    }
+    KB200_CUDA(launch_kernel(plan.pdl, split ? attention_pairs_kernel<true> : attention_pairs_kernel<false>, st->grid, dim3(kPairsThreads), kPairsSmem, s, h.q,
+                             h.k, h.v, h.qt, h.kt, h.vt, st->map_out, h.outh, h.outt, h.params));
+  } else if (st->exact_tc) {
     const int64_t blocks = (st->span_n4 + 255) / 256;
     if (!st->tails_ready)
       KB200_CUDA(launch_kernel(plan.pdl, tails_kernel, dim3((unsigned)(blocks < 1184 ? blocks : 1184)), dim3(256), 0, s,
@@ -1465,7 +1483,7 @@ void attention_elide_copy(Plan& plan, size_t first) {
   }
   for (auto& [k, slot] : redirect) k->ops[slot].ptr = st->staged_out;
   st->final_out = nullptr;
-  holder.launches = 1 + (st->exact_tc && !st->tails_ready ? 1 : 0);
+  holder.launches = 1 + ((st->exact_tc && !st->tails_ready) || (st->pairs.used && !st->pairs.ready) ? 1 : 0);
 }
 
 bool attention_may_drop_float32(const PlanKernel& k) {
@@ -1473,6 +1491,137 @@ bool attention_may_drop_float32(const PlanKernel& k) {
   return st && st->bf16 && st->params.out16 != nullptr;
 }
 void attention_drop_float32(PlanKernel& k) { static_cast<AttnState*>(k.attn)->params.out32 = false; }
+
+// FP32 mode: float16 pairs of Q, K and V, whose bounds by column of the projection's output (rows x bounds.size(), `src_row` apart) are known.
+// Taken where every head's columns are alike enough (see split_suits: q . k and the merged heads keep what TF32 pairs would) and the
+// estimates say so.
+int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_t src_row, int64_t rows, const std::vector<float>& bounds) {
+  AttnState* st = static_cast<AttnState*>(holder.attn);
+  const int64_t cols = (int64_t)bounds.size();
+  AttnParams& p = st->params;
+  if (!st->exact || rows != (int64_t)p.B * p.T || st->row_stride != src_row || cols % 32 != 0 || src_row % 4 || !aligned16(src) ||
+      rows * (cols / 4) >= (int64_t(1) << 31))
+    return KB200_OK;
+  const int64_t width = (int64_t)p.H * kHeadDim;
+  const int64_t first[3] = {st->q_ptr - src, st->k_ptr - src, st->v_ptr - src};
+  std::vector<float> factors(2 * p.H + 1, 1.0f), by((size_t)cols / 32, 0.0f);
+  float out_bound = 0.0f;
+  for (int role = 0; role < 3; ++role) {
+    if (first[role] < 0 || first[role] % 32 || first[role] + width > cols) return KB200_OK;
+    for (int h = 0; h < p.H; ++h) {
+      const auto at = bounds.begin() + first[role] + h * kHeadDim;
+      const float most = *std::max_element(at, at + kHeadDim), least = *std::min_element(at, at + kHeadDim);
+      if (!(most <= 1024.0f * least) || most > 1e18f || least < 1e-18f) return KB200_OK;
+      int e = 0;
+      frexpf(most, &e);
+      const float scale = ldexpf(1.0f, 15 - e);
+      float* const blocks = &by[(size_t)(first[role] / 32 + 2 * h)];
+      if (blocks[0] != 0.0f || blocks[1] != 0.0f) return KB200_OK;          // views that overlap
+      blocks[0] = blocks[1] = scale;
+      factors[(size_t)(role == 2 ? p.H + h : h)] /= scale;
+      if (role == 2) out_bound = std::max(out_bound, most);
+    }
+  }
+  for (int h = 0; h < p.H; ++h) factors[h] *= p.scale_log2;
+  for (float& b : by)
+    if (b == 0.0f) b = 1.0f;
+  st->out_bound = out_bound;
+  if (st->ieee || st->asked) return KB200_OK;
+  // The CUDA-core kernel (see finish_fusion) stays where it is quicker: little work.
+  const int64_t sms = plan.sm_count, items = (int64_t)p.B * p.H * p.q_tiles, tiles64 = p.T <= 64 ? 1 : 2 * p.q_tiles;
+  const int64_t fma_ns = 4200 + 2250 * tiles64 * (((int64_t)p.B * p.H * tiles64 + sms - 1) / sms);
+  const int64_t pairs_ns = 6000 + 1500 * p.q_tiles * ((items + sms - 1) / sms);
+  if (!st->exact_tc && pairs_ns > fma_ns) return KB200_OK;
+  AttnState::Pairs h;
+  h.src = src; h.src_row = src_row; h.rows = rows; h.cols = cols;
+  h.pitch = (cols + 63) / 64 * 64;
+  factors.insert(factors.end(), by.begin(), by.end());
+  const bool made = cudaMalloc(&h.planes, (size_t)rows * h.pitch * 4) == cudaSuccess && cudaMalloc(&h.factors, factors.size() * sizeof(float)) == cudaSuccess &&
+                    cudaMemcpy(h.factors, factors.data(), factors.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess;
+  const uint16_t* const heads = static_cast<const uint16_t*>(h.planes);
+  const uint16_t* const tails = heads + rows * h.pitch;
+  CUtensorMap* const maps[3][2] = {{&h.q, &h.qt}, {&h.k, &h.kt}, {&h.v, &h.vt}};
+  bool ok = made;
+  for (int role = 0; role < 3 && ok; ++role)
+    ok = encode_map_heads(maps[role][0], true, heads + first[role], kHeadDim, p.T, p.H, p.B, h.pitch, kHeadDim, kRows, false) &&
+         encode_map_heads(maps[role][1], true, tails + first[role], kHeadDim, p.T, p.H, p.B, h.pitch, kHeadDim, kRows, false);
+  ok = ok && cudaFuncSetAttribute(attention_pairs_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairsSmem) == cudaSuccess &&
+       cudaFuncSetAttribute(attention_pairs_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairsSmem) == cudaSuccess;
+  // Long query tiles of a launch that leaves SMs idle are shared by two CTAs, as in finish_fusion.
+  if (ok && !st->exact_tc && st->may_split && p.q_tiles >= 8 && items <= 2 * sms) {
+    p.split_from = p.q_tiles / 2;
+    if (!split_workspace(st, attention_item_order(p.q_tiles, p.split_from), 0)) {
+      p.split_from = p.q_tiles;
+      ok = false;
+    }
+  }
+  if (!ok) {
+    cudaGetLastError();
+    if (h.planes) cudaFree(h.planes);
+    if (h.factors) cudaFree(h.factors);
+    return KB200_OK;
+  }
+  h.used = true;
+  h.outh = h.outt = st->map_out;
+  h.params.a = p;
+  h.params.a.idesc_qk = (1u << 4) | ((uint32_t)(kRows >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);          // D = F32, A/B = F16
+  h.params.a.idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(kHeadDim >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+  h.params.qk = h.factors;
+  h.params.v_back = h.factors + p.H;
+  h.params.out_scale = nullptr;
+  h.params.store32 = 1;
+  const int64_t all = (int64_t)p.B * p.H * (p.q_tiles + (p.q_tiles - p.split_from));
+  st->grid = dim3((unsigned)(all < sms ? all : sms), 1, 1);
+  if (st->tails) cudaFree(st->tails);
+  if (st->f32_scratch) cudaFree(st->f32_scratch);
+  st->tails = nullptr;
+  st->f32_scratch = nullptr;
+  st->exact_tc = false;
+  st->pairs = h;
+  holder.launches = (st->staged_out && st->final_out ? 2 : 1) + 1;
+  return KB200_OK;
+}
+
+// The planes the projection in front may write, and their scales by 32 columns; false where a pass does it.
+bool attention_takes_pairs(const PlanKernel& k, PlanKernel::Planes* planes, const float** scale) {
+  const AttnState* st = static_cast<const AttnState*>(k.attn);
+  if (!st || !st->pairs.used || st->own_pass) return false;
+  *planes = PlanKernel::Planes{st->pairs.planes, st->pairs.rows * st->pairs.pitch, st->pairs.pitch, nullptr};
+  *scale = st->pairs.by();
+  return true;
+}
+// Can the merged heads leave as float16 pairs (rows of `pitch`), times a power of two that `back` undoes?  `drop`: and the float32 rows not at all.
+bool attention_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, bool drop, float* back) {
+  AttnState* st = static_cast<AttnState*>(k.attn);
+  if (!st || st->exact_tc || st->out_bound == 0.0f || (st->staged_out && st->final_out)) return false;
+  AttnState::Pairs& h = st->pairs;
+  const AttnParams& p = st->params;
+  const int64_t width = (int64_t)p.H * kHeadDim;
+  uint16_t* const heads = static_cast<uint16_t*>(to.heads);
+  int e = 0;
+  frexpf(st->out_bound, &e);
+  const float scale = ldexpf(1.0f, 15 - e);
+  *back = 1.0f / scale;
+  if (!h.used) {
+    st->f32.heads = reinterpret_cast<__half*>(heads);
+    st->f32.plane = to.plane;
+    st->f32.pitch = to.pitch;
+    st->f32.pair_scale = scale;
+    st->f32.store32 = drop ? 0 : 1;
+    return true;
+  }
+  if (!encode_map_store(&h.outh, true, heads, width, p.T, p.B, to.pitch, p.T * to.pitch) ||
+      !encode_map_store(&h.outt, true, heads + to.plane, width, p.T, p.B, to.pitch, p.T * to.pitch) ||
+      cudaMemcpy(h.factors + 2 * p.H, &scale, sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+    return false;
+  h.params.out_scale = h.factors + 2 * p.H;
+  h.params.store32 = drop ? 0 : 1;
+  return true;
+}
+void attention_pairs_come_ready(PlanKernel& k) {
+  static_cast<AttnState*>(k.attn)->pairs.ready = true;
+  --k.launches;
+}
 
 float* attention_tails(const PlanKernel& k) {
   const AttnState* st = static_cast<const AttnState*>(k.attn);
@@ -1513,6 +1662,8 @@ void attention_destroy(PlanKernel& k) {
     if (st->f32_scratch) cudaFree(st->f32_scratch);
     if (st->tails) cudaFree(st->tails);
     if (st->split_scratch) cudaFree(st->split_scratch);
+    if (st->pairs.planes) cudaFree(st->pairs.planes);
+    if (st->pairs.factors) cudaFree(st->pairs.factors);
     delete st;
   }
   k.attn = nullptr;

@@ -193,6 +193,10 @@ bool attention_wants_bf16(const PlanKernel& k);
 bool attention_reads_mirror(const PlanKernel& k);
 float* attention_tails(const PlanKernel& k);            // FP32 on the tensor cores: the tails of Q, K and V, or null
 void attention_tails_come_ready(PlanKernel& k);         // ... which the projection writes
+int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_t src_row, int64_t rows, const std::vector<float>& bounds);      // FP32 on float16 pairs
+bool attention_takes_pairs(const PlanKernel& k, PlanKernel::Planes* planes, const float** scale);
+void attention_pairs_come_ready(PlanKernel& k);
+bool attention_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, bool drop, float* back);
 bool matmul_writes_tails(const PlanKernel& k);
 bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);      // multiplies float16 pairs of A, split by a pass of its own ...
 void matmul_planes_come_ready(PlanKernel& k);                                   // ... or by A's producer

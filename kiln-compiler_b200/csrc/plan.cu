@@ -1030,6 +1030,20 @@ static int hand_on_planes(Plan& plan) {
   for (size_t ki = 0; ki < plan.kernels.size(); ++ki) {
     PlanKernel& k = plan.kernels[ki];
     PlanKernel::Planes planes;
+    const float* scale = nullptr;
+    Span x{nullptr, nullptr};
+    if (k.impl != IMPL_ATTN_FUSED || !attention_takes_pairs(k, &planes, &scale) || !attention_operand_span(k, &x.lo, &x.hi)) continue;
+    PlanKernel* const from = mirroring_producer(plan, ki, x);
+    if (from == nullptr || from->impl != IMPL_MM_TC || from->planes_out.heads != nullptr) continue;
+    const bool alone = plan.mirror_only && only_read_as(plan, (size_t)(from - plan.kernels.data()), span_of(*from, from->chain.out_slot),
+                                                        [&](const PlanKernel& r, int) { return &r == &k; });
+    if (!matmul_write_pairs(*from, planes, scale, !alone)) continue;
+    from->planes_out = planes;
+    attention_pairs_come_ready(k);
+  }
+  for (size_t ki = 0; ki < plan.kernels.size(); ++ki) {
+    PlanKernel& k = plan.kernels[ki];
+    PlanKernel::Planes planes;
     if (k.desc.kclass != KB200_K_MATMUL || !matmul_takes_planes(k, &planes)) continue;
     const int a = k.desc.a_slot;
     auto reads_here = [&](const PlanKernel& r, int slot) { return &r == &k && slot == a; };
@@ -1043,6 +1057,20 @@ static int hand_on_planes(Plan& plan) {
     const Span x = span_of(k, a);
     if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) continue;
     PlanKernel* const from = mirroring_producer(plan, ki, x);
+    if (from != nullptr && from->impl == IMPL_ATTN_FUSED) {
+      // the merged heads, convex combinations of V's rows
+      const size_t fi = (size_t)(from - plan.kernels.data());
+      int64_t elems = 0;
+      const DevOperand* const y = attention_output(plan, fi, &elems);
+      float back = 0.0f;
+      if (y->ptr != k.ops[a].ptr || k.ops[a].stride[1] != k.K || k.ops[a].stride[2] != 1 || elems != k.M * k.K) continue;
+      const bool alone = plan.mirror_only && only_read_as(plan, fi, Span{y->ptr, y->ptr + elems}, reads_here);
+      if (!attention_write_pairs(*from, planes, alone, &back)) continue;
+      const std::vector<float> all((size_t)k.M, back);
+      KB200_CUDA(cudaMemcpy(planes.scales, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice));
+      matmul_planes_come_ready(k);
+      continue;
+    }
     if (from == nullptr || from->impl != IMPL_MM_TC || from->planes_out.heads != nullptr || from->M != k.M || from->N != k.K) continue;
     const DevOperand &out = from->ops[from->chain.out_slot], &in = k.ops[a];
     if (out.ptr != in.ptr || out.stride[1] != in.stride[1]) continue;
@@ -1269,6 +1297,18 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   if (rc == KB200_OK) rc = assign_shadows(plan);
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i)
     if (plan.kernels[i].impl == IMPL_ATTN_FUSED) attention_elide_copy(plan, i);
+  // FP32 attention on float16 pairs, where the bounds of Q, K and V are known
+  for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
+    Span x{nullptr, nullptr};
+    PlanKernel& k = plan.kernels[i];
+    if (k.impl != IMPL_ATTN_FUSED || k.desc.precision != KB200_PREC_FP32 || !attention_operand_span(k, &x.lo, &x.hi)) continue;
+    const PlanKernel* const from = mirroring_producer(plan, i, x);
+    if (from == nullptr || from->impl != IMPL_MM_TC) continue;
+    std::vector<float> bounds;
+    rc = result_bounds(plan, (size_t)(from - plan.kernels.data()), &bounds);
+    const DevOperand& out = from->ops[from->chain.out_slot];
+    if (rc == KB200_OK && !bounds.empty() && out.stride[2] == 1) rc = attention_use_pairs(plan, k, out.ptr, out.stride[1], from->M, bounds);
+  }
   // FP32 attention on the tensor cores: the projection that wrote exactly Q, K and V can write their tails as well
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
     Span x{nullptr, nullptr};

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
@@ -209,6 +210,26 @@ __device__ __forceinline__ void stage_rows(uint8_t* sf, uint8_t* sh, const float
       packed.w = *reinterpret_cast<uint32_t*>(&w3);
       *reinterpret_cast<uint4*>(sh + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = packed;
     }
+  }
+}
+
+// A 32 x 32 block, this lane's row, as float16 pairs: 64-byte rows of heads, then those of tails, swizzled as the 16-bit store maps want them.
+__device__ __forceinline__ void stage_pairs(uint8_t* block, const float (&v)[32], int lane, float scale) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t h[4], t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = fmul2(make_float2(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]), make_float2(scale, scale));
+      const __half2 head = __floats2half2_rn(x.x, x.y);
+      const float2 back = __half22float2(head);
+      const __half2 tail = __floats2half2_rn(x.x - back.x, x.y - back.y);
+      h[i] = *reinterpret_cast<const uint32_t*>(&head);
+      t[i] = *reinterpret_cast<const uint32_t*>(&tail);
+    }
+    uint8_t* const at = block + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4);
+    *reinterpret_cast<uint4*>(at) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(at + 2048) = make_uint4(t[0], t[1], t[2], t[3]);
   }
 }
 
