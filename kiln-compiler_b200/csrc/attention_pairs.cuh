@@ -6,7 +6,10 @@
 //   * a group's probabilities lie over its own 64 scores, 32 columns of heads and 32 of tails, so both S buffers carry them;
 //   * the tensor core cuts off a bit of an accumulator with every MMA: sums in it are over 64 keys (the head dimension in Q K^T), small
 //     products first, and everything beyond is added up in float32 registers.
-// So it takes sequences of any length, which the TF32 form, 1.9e-6 from float64, left to the CUDA cores.
+// From float64, merged heads of 12 heads: 1024 tokens 2.1e-7 (TF32 1.8e-6, the CUDA cores 2.6e-7), 2048 tokens 2.1e-7 (1.8e-6, 3.3e-7), 200 tokens
+// 2.8e-7 (1.0e-6, 2.6e-7).  So it takes sequences of any length, which the TF32 form left to the CUDA cores: 12 heads of 1500 tokens
+// 126 -> 25 us, of 333 tokens 18.1 -> 11.3 with the pass, 96 heads of 1024 tokens 128 (TF32) -> 53.  What bounds a tile is the softmax warps (a score costs
+// them a maximum, an exponential, four conversions and their stores) beside 36 MMAs of ~50 cycles of issue.
 #pragma once
 
 #include <cuda.h>
@@ -32,12 +35,12 @@ constexpr int kPairsSlot = 4096;                        // a warp's output block
 constexpr int kPairsExchange = 2 * (2 * 2 * kAttnRows * 4);
 constexpr int kPairsSmem = 5 * kPairsTile + kPairsExchange + 8 * kPairsSlot + 1024;
 constexpr int kPairsThreads = 320;
-constexpr float kPairsShift = 14.0f;                    // probabilities are at most 1: times 2^14
+constexpr float kPairsUp = 16384.0f;                    // probabilities are at most 1: times 2^14.  (Not in the exponent, whose fraction would lose four bits.)
 
 struct PairsParams {
   AttnParams a;
   const float* qk;          // by head: what a product of Q and K is to be multiplied by, times scale x log2(e)
-  const float* v_back;      // ... and one with V
+  const float* v_back;      // ... and one with V, the probabilities' 2^14 included
   const float* out_scale;   // pairs of the merged heads leave as well, times *out_scale, through map_outh and map_outt; or null
   int store32;
 };
@@ -46,9 +49,10 @@ struct PairsParams {
 __device__ __forceinline__ void split_probabilities(const float (&v)[32], uint32_t* heads, uint32_t* tails) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+    const float2 x = fmul2(make_float2(v[2 * i], v[2 * i + 1]), make_float2(kPairsUp, kPairsUp));
+    const __half2 h = __floats2half2_rn(x.x, x.y);
     const float2 back = __half22float2(h);
-    const __half2 t = __floats2half2_rn(v[2 * i] - back.x, v[2 * i + 1] - back.y);
+    const __half2 t = __floats2half2_rn(x.x - back.x, x.y - back.y);
     heads[i] = *reinterpret_cast<const uint32_t*>(&h);
     tails[i] = *reinterpret_cast<const uint32_t*>(&t);
   }
@@ -305,11 +309,11 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const float alpha = ex2(m_run - m_new);       // 0 while m_run = -inf
         float sum;
         if (diagonal) {
-          sum = probabilities32<true>(va, qk, m_new - kPairsShift, c0, row);
-          sum += probabilities32<true>(vb, qk, m_new - kPairsShift, c0 + 32, row);
+          sum = probabilities32<true>(va, qk, m_new, c0, row);
+          sum += probabilities32<true>(vb, qk, m_new, c0 + 32, row);
         } else {
-          sum = probabilities32<false>(va, qk, m_new - kPairsShift, 0, 0);
-          sum += probabilities32<false>(vb, qk, m_new - kPairsShift, 0, 0);
+          sum = probabilities32<false>(va, qk, m_new, 0, 0);
+          sum += probabilities32<false>(vb, qk, m_new, 0, 0);
         }
         uint32_t heads[32], tails[32];
         split_probabilities(va, heads, tails);
