@@ -664,12 +664,12 @@ int resident_quads(const Plan& plan) {
   return known;
 }
 
-// Tile width and estimated cycles of a launch: 8000 once, and per round of tiles its drain and the cycles of its slabs, more of them the
+// Tile width and estimated cycles of a launch: 6700 once, and per round of tiles its drain and the cycles of its slabs, more of them the
 // more of the pairs are at work (one SM gets 60 to 75 bytes a clock from L2; a slab of 256 columns has 512 cycles of multiplying).
 // K in halves: the exchange and its own start instead.  Lines through 512 launches in TF32 and BF16, every width and both
-// forms of each timed: 160 to 4096 rows of sixteen weights from 256 x 1024 to 4096 x 4096.  The choice is 0.2 % (TF32) and 0.1 % (BF16)
-// from the best on average; the estimate before, through 2048 x 3072 x 768 and 2048 x 768 x 3072 in TF32, was 1.6 % and 1.2 %, with halves
-// 17 % slower than a tile of 128 columns where K is 512 to 2048 (1792 x 640 x 512 9.2 against 7.8 us).
+// forms of each timed: 160 to 4096 rows of sixteen weights from 256 x 1024 to 4096 x 4096.  The choice is 0.1 % from the best on average,
+// and against the few-tiles kernel 0.1 % (TF32) and 0.2 % (BF16); with the lines of the epilogue that released over the cluster it was 0.2 %, and 0.8
+// and 0.5 % (1024 x 2304 x 768 BF16 10.2 against 9.5 us, 256 x 4096 x 1000 TF32 10.6 against 9.7).
 // The widths between 128 and 256 are for the last round: 2048 x 3072 x 768 TF32 21.2 us at 128 columns (three rounds, 64 of 74 pairs),
 // 23.5 at 256 (96 tiles), 19.5 at 192 (128 tiles, two rounds); 8192 x 768 x 3072 BF16 66.2 at 256, 59.5 at 192 (with its pass
 // over A); 8192 x 2304 x 768 36.1 at 256, 39.7 at 192.
@@ -680,8 +680,8 @@ struct PairWidth {
   int half_alone, half_full, halves;   // K in halves: cycles of a slab, and of all that runs once (0: this width does not come in halves)
 };
 constexpr PairWidth kPairWidths[] = {
-    {256, 485, 637, 4310, 508, 627, 13270}, {224, 419, 566, 3730, 0, 0, 0}, {192, 354, 496, 3400, 380, 475, 11110}, {160, 292, 429, 3130, 0, 0, 0}, {128, 243, 406, 2400, 0, 0, 0}};
-constexpr int64_t kPairOnce = 8000, kPairHalvesBusy = 3320;      // (halves: with all pairs at work)
+    {256, 490, 607, 3960, 505, 683, 12080}, {224, 430, 552, 3460, 0, 0, 0}, {192, 362, 485, 2730, 383, 496, 9970}, {160, 304, 412, 2570, 0, 0, 0}, {128, 256, 387, 2080, 0, 0, 0}};
+constexpr int64_t kPairOnce = 6700, kPairHalvesBusy = 1860;      // (halves: with all pairs at work)
 // A matrix operand of the epilogue arrives under the exchange of halves; without one it adds to the drain.  Of 156 launches with a
 // residual behind another kernel, widths and halves of each timed, the choice is then 0.06 us from the best on average, 0.19 without
 // (1400 x 768 x 768 TF32 15.5 us at 128 columns, 15.2 in halves; 1400 x 1024 x 4096 BF16 34.3 and 32.1).
@@ -743,8 +743,7 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
 
 }  // namespace
 
-// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9: of 288 launches that both take, the
-// choice is 0.1 % from the better one in BF16 and 0.1 % in TF32, 0.2 and 0.3 with the estimate before)
+// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9)
 int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, b_kmajor).cycles * 7 / 8; }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {

@@ -1193,7 +1193,7 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
     const int64_t tiles = ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128), sms = plan.sm_count;
     if (d.precision == KB200_PREC_FP32) many = (tiles + sms - 1) / sms * ((k.K + slab_k - 1) / slab_k) * 1150 + 16500;
     else if (pair_eligible(plan, k, b_kmajor, b_map_cols)) many = pair_cycles(plan, k, b_kmajor);
-    if (many > 0 && copy_a) many += 4000;
+    if (many > 0 && copy_a) many += 4500;
   }
   // (its exact-FP32 form multiplies with the tails of B: without room for them this file's kernel makes them as it goes)
   const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
