@@ -884,6 +884,18 @@ struct AttnChain {
   bool ieee = false;                  // ... and were asked to behave like FMA matmuls on non-finite operands (config bit 1024)
 };
 
+// *odd: is anything of a [T, T] mask not the causal one's, 0 on and below the diagonal and -inf above?  (Looked at on the host, the mask of 1024 tokens
+// was 4 of the 4.3 ms that binding a BF16 block takes.)
+__global__ void __launch_bounds__(256) mask_kernel(const float* __restrict__ mask, int64_t T, int* odd) {
+  const int64_t row = blockIdx.x;
+  bool wrong = false;
+  for (int64_t col = threadIdx.x; col < T; col += 256) {
+    const float v = mask[row * T + col];
+    wrong = wrong || (col <= row ? v != 0.0f : v != -CUDART_INF_F);
+  }
+  if (wrong) *odd = 1;
+}
+
 // Split tiles' partial results, counters and order, and what `runs` CTAs keep between runs of key tiles.
 bool split_workspace(AttnState* st, const std::vector<int>& entries, int64_t runs) {
   AttnParams& p = st->params;
@@ -944,16 +956,14 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
 
   // --- the mask must be the causal one: 0 on and below the diagonal, -inf above ---
   {
-    std::vector<float> host((size_t)T * T);
-    if (cudaMemcpy(host.data(), c.mask->ptr, host.size() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    for (int64_t r = 0; r < T; ++r)
-      for (int64_t col = 0; col < T; ++col) {
-        const float v = host[(size_t)r * T + col];
-        if (col <= r ? v != 0.0f : !(v < 0.0f && isinf(v))) return false;
-      }
+    int* odd = nullptr;
+    int found = 1;
+    const bool looked = cudaMalloc(&odd, sizeof(int)) == cudaSuccess && cudaMemset(odd, 0, sizeof(int)) == cudaSuccess &&
+                        launch_kernel(false, mask_kernel, dim3((unsigned)T), dim3(256), 0, nullptr, (const float*)c.mask->ptr, T, odd) == cudaSuccess &&
+                        cudaMemcpy(&found, odd, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (odd) cudaFree(odd);
+    if (!looked) cudaGetLastError();
+    if (!looked || found != 0) return false;
   }
 
   // Q, K, V as [sequence, head, token, 64] views.  The token dim ends with the sequence, so the tile of
@@ -1591,10 +1601,15 @@ bool attention_takes_pairs(const PlanKernel& k, PlanKernel::Planes* planes, cons
   *scale = st->pairs.by();
   return true;
 }
+bool attention_may_write_pairs(const PlanKernel& k) {
+  const AttnState* st = static_cast<const AttnState*>(k.attn);
+  return st && !st->exact_tc && st->out_bound != 0.0f && !(st->staged_out && st->final_out);
+}
+
 // Can the merged heads leave as float16 pairs (rows of `pitch`), times a power of two that `back` undoes?  `drop`: and the float32 rows not at all.
 bool attention_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, bool drop, float* back) {
   AttnState* st = static_cast<AttnState*>(k.attn);
-  if (!st || st->exact_tc || st->out_bound == 0.0f || (st->staged_out && st->final_out)) return false;
+  if (!attention_may_write_pairs(k)) return false;
   AttnState::Pairs& h = st->pairs;
   const AttnParams& p = st->params;
   const int64_t width = (int64_t)p.H * kHeadDim;

@@ -106,6 +106,10 @@ struct PlanKernel {
     int64_t plane = 0, pitch = 0;
     float* scales = nullptr;
   } planes_out;
+  // FP32: bounds of a matmul's results by column (see result_bounds), once they have been looked for, and whether its producer will split its rows
+  std::vector<float> bounds;
+  bool bounds_known = false;
+  bool planes_expected = false;
   float* tail_out = nullptr;      // FP32: where the tails of the output (what a TF32 operand drops) go as well, same offsets, or null
   bool mirror_only = false;       // producer side: every reader of the output takes the mirror, the float32 store is dropped
   // An elementwise kernel that only continues the matmul in front of it (the activation or the residual
@@ -196,6 +200,7 @@ void attention_tails_come_ready(PlanKernel& k);         // ... which the project
 int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_t src_row, int64_t rows, const std::vector<float>& bounds);      // FP32 on float16 pairs
 bool attention_takes_pairs(const PlanKernel& k, PlanKernel::Planes* planes, const float** scale);
 void attention_pairs_come_ready(PlanKernel& k);
+bool attention_may_write_pairs(const PlanKernel& k);
 bool attention_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, bool drop, float* back);
 bool matmul_writes_tails(const PlanKernel& k);
 bool matmul_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes);      // multiplies float16 pairs of A, split by a pass of its own ...

@@ -982,10 +982,9 @@ static PlanKernel* layernorm_in_front(Plan& plan, size_t ki) {
 }
 
 // Bounds of a matmul's results by column, whatever the input: of a LayerNorm's rows and frozen parameters, with a bias and a GELU (which is
-// no larger than its argument).  *bounds stays empty where nothing is known.
-static int result_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
+// no larger than its argument).  Empty where nothing is known.
+static int look_for_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
   const PlanKernel& k = plan.kernels[ki];
-  bounds->clear();
   const PlanKernel* const norm = layernorm_in_front(plan, ki);
   auto frozen = [](const PlanKernel& of, int slot) { return of.desc.operands[slot].base_kind == KB200_BASE_CONST; };
   if (norm == nullptr || !frozen(*norm, norm->g_slot) || !frozen(*norm, norm->b_slot) || !(norm->ln_inv_n > 0.0f) || !(norm->ln_eps >= 0.0f)) return KB200_OK;
@@ -1004,6 +1003,13 @@ static int result_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
     if (!(b < 1e30f)) { bounds->clear(); break; }
   return KB200_OK;
 }
+static int result_bounds(Plan& plan, size_t ki, const std::vector<float>** bounds) {
+  PlanKernel& k = plan.kernels[ki];
+  *bounds = &k.bounds;
+  if (k.bounds_known) return KB200_OK;
+  k.bounds_known = true;
+  return look_for_bounds(plan, ki, &k.bounds);
+}
 
 // `host` on the device, for as long as the plan is bound as it is.  Null where memory is short.
 static float* keep_scales(Plan& plan, const std::vector<float>& host) {
@@ -1021,6 +1027,32 @@ static float pair_scale(float bound) {
   int e = 0;
   frexpf(bound > 1e-30f ? bound : 1e-30f, &e);
   return ldexpf(1.0f, 15 - e);
+}
+
+// Will operand A come as float16 pairs, should the matmul multiply those?  Asked before it is bound, and after its producer was.
+static int expect_planes(Plan& plan, size_t ki) {
+  PlanKernel& k = plan.kernels[ki];
+  if (const PlanKernel* const norm = layernorm_in_front(plan, ki)) {
+    k.planes_expected = true;
+    for (size_t i = 0; i < ki; ++i)            // (a LayerNorm has one reader that it splits its rows for)
+      if (plan.kernels[i].planes_expected && layernorm_in_front(plan, i) == norm) k.planes_expected = false;
+    return KB200_OK;
+  }
+  const int a = k.desc.a_slot;
+  const Span x = span_of(k, a);
+  if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) return KB200_OK;
+  const PlanKernel* const from = mirroring_producer(plan, ki, x);
+  if (from == nullptr) return KB200_OK;
+  if (from->impl == IMPL_ATTN_FUSED) {
+    k.planes_expected = attention_may_write_pairs(*from);
+    return KB200_OK;
+  }
+  PlanKernel::Planes planes;
+  if (from->impl != IMPL_MM_TC || !matmul_takes_planes(*from, &planes) || from->N != k.K) return KB200_OK;
+  const std::vector<float>* bounds = nullptr;
+  const int rc = result_bounds(plan, (size_t)(from - plan.kernels.data()), &bounds);
+  k.planes_expected = rc == KB200_OK && !bounds->empty();
+  return rc;
 }
 
 // Exact FP32 on float16 pairs whose producer can write them: no pass in front of the matmul splits its rows, and the float32 rows are not stored
@@ -1075,11 +1107,11 @@ static int hand_on_planes(Plan& plan) {
     const DevOperand &out = from->ops[from->chain.out_slot], &in = k.ops[a];
     if (out.ptr != in.ptr || out.stride[1] != in.stride[1]) continue;
     const size_t fi = (size_t)(from - plan.kernels.data());
-    std::vector<float> bounds;
+    const std::vector<float>* bounds = nullptr;
     const int rc = result_bounds(plan, fi, &bounds);
     if (rc) return rc;
-    if (bounds.empty()) continue;
-    const float scale = pair_scale(*std::max_element(bounds.begin(), bounds.end()));
+    if (bounds->empty()) continue;
+    const float scale = pair_scale(*std::max_element(bounds->begin(), bounds->end()));
     const float* const by = keep_scales(plan, std::vector<float>((size_t)(from->N + 31) / 32, scale));
     const bool alone = plan.mirror_only && only_read_as(plan, fi, span_of(*from, from->chain.out_slot), reads_here);
     if (by == nullptr || !matmul_write_pairs(*from, planes, by, !alone)) continue;
@@ -1272,6 +1304,8 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     k.mirror_only = false;
     k.tail_out = nullptr;
     k.planes_out = PlanKernel::Planes();
+    k.bounds.clear();
+    k.bounds_known = k.planes_expected = false;
     k.absorbed_by = -1;
     k.n_ops = k.desc.n_operands;
     rc = resolve(plan, k, (int)i);
@@ -1304,10 +1338,10 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     if (k.impl != IMPL_ATTN_FUSED || k.desc.precision != KB200_PREC_FP32 || !attention_operand_span(k, &x.lo, &x.hi)) continue;
     const PlanKernel* const from = mirroring_producer(plan, i, x);
     if (from == nullptr || from->impl != IMPL_MM_TC) continue;
-    std::vector<float> bounds;
+    const std::vector<float>* bounds = nullptr;
     rc = result_bounds(plan, (size_t)(from - plan.kernels.data()), &bounds);
     const DevOperand& out = from->ops[from->chain.out_slot];
-    if (rc == KB200_OK && !bounds.empty() && out.stride[2] == 1) rc = attention_use_pairs(plan, k, out.ptr, out.stride[1], from->M, bounds);
+    if (rc == KB200_OK && !bounds->empty() && out.stride[2] == 1) rc = attention_use_pairs(plan, k, out.ptr, out.stride[1], from->M, *bounds);
   }
   // FP32 attention on the tensor cores: the projection that wrote exactly Q, K and V can write their tails as well
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
@@ -1339,7 +1373,9 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
   }
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i) {
     PlanKernel& k = plan.kernels[i];
-    if (k.desc.kclass == KB200_K_MATMUL && k.impl != IMPL_FUSED_AWAY) rc = bind_matmul(plan, k);
+    if (k.desc.kclass != KB200_K_MATMUL || k.impl == IMPL_FUSED_AWAY) continue;
+    if (k.impl == IMPL_MM_TC && k.desc.precision == KB200_PREC_FP32) rc = expect_planes(plan, i);
+    if (rc == KB200_OK) rc = bind_matmul(plan, k);
   }
   for (size_t i = 0; i < plan.kernels.size() && rc == KB200_OK; ++i)
     for (const PlanKernel& k : plan.kernels)
