@@ -31,7 +31,7 @@ int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, flo
 // |LayerNorm(x) B + bias| per column of B [K, N] for any x, at most: of the normalised row, 1 / sqrt(inv_n) long, by Cauchy and Schwarz.  `bounds`: [n]
 // on the host.  Synchronises.
 int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds);
-// Do float16 pairs hold this weight [K, N] as well as TF32 pairs would, whatever A is?  Synchronises.
-int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, bool* suits);
+// Do float16 pairs hold this weight [K, N] as well as TF32 pairs would, whatever A is?  `scratch`: k words on the device.  Synchronises.
+int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, uint32_t* scratch, bool* suits);
 
 }  // namespace kb200

@@ -1023,8 +1023,7 @@ void drop_copies(TcState* st) {
 }
 
 void drop_pairs16(TcState* st) {
-  for (void* p : {st->pairs16.a, st->pairs16.b, static_cast<void*>(st->pairs16.scales)})
-    if (p) cudaFree(p);
+  if (st->pairs16.a) cudaFree(st->pairs16.a);         // (all three are one allocation)
   st->pairs16 = TcState::Pairs16();
 }
 
@@ -1063,15 +1062,24 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
   const DevOperand& B = k.ops[d.b_slot];
   const int64_t pitch = (k.K + 63) / 64 * 64;              // rows on 128-byte lines
   const uint64_t a_bytes = (uint64_t)k.M * pitch * 4;
-  bool suits = false;
-  const int rc = split_suits(B.ptr, B.stride[1], B.stride[2], k.K, k.N, &suits);
-  if (rc || !suits || a_bytes > plan.copy_budget) return rc;
+  if (a_bytes > plan.copy_budget) return KB200_OK;
   TcState::Pairs16& h = st->pairs16;
-  float* turned = nullptr;
-  cudaError_t e = cudaMalloc(&h.a, a_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&h.b, (size_t)k.N * pitch * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&h.scales, (size_t)(k.M + k.N) * sizeof(float));
-  if (e == cudaSuccess && turn) e = cudaMalloc(&turned, (size_t)k.N * k.K * sizeof(float));
+  const size_t turned_floats = turn ? (size_t)k.N * k.K : 0;
+  float* turned = nullptr;                                 // for the time of binding: the weight as rows along K, and K numbers of split_suits
+  cudaError_t e = cudaMalloc(&turned, (turned_floats + k.K) * sizeof(float));
+  bool suits = false;
+  if (e == cudaSuccess) {
+    const int rc = split_suits(B.ptr, B.stride[1], B.stride[2], k.K, k.N, reinterpret_cast<uint32_t*>(turned + turned_floats), &suits);
+    if (rc || !suits) {
+      cudaFree(turned);
+      return rc;
+    }
+    e = cudaMalloc(&h.a, a_bytes + (size_t)k.N * pitch * 4 + (size_t)(k.M + k.N) * sizeof(float));
+  }
+  if (e == cudaSuccess) {
+    h.b = static_cast<uint8_t*>(h.a) + a_bytes;            // (rows of 128 bytes: both stay aligned)
+    h.scales = reinterpret_cast<float*>(static_cast<uint8_t*>(h.b) + (size_t)k.N * pitch * 4);
+  }
   if (e == cudaSuccess && turn)
     e = launch_kernel(false, transpose_rows_kernel<float>, dim3((unsigned)((k.K + 31) / 32), (unsigned)((k.N + 31) / 32)), dim3(256), 0, nullptr,
                       (const float*)B.ptr, turned, (int)k.K, (int)k.N, B.stride[1], k.K);

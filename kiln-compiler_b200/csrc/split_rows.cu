@@ -142,14 +142,11 @@ int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, flo
   return KB200_OK;
 }
 
-int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, bool* suits) {
+int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, uint32_t* device, bool* suits) {
   *suits = false;
-  uint32_t* device = nullptr;
-  KB200_CUDA(cudaMalloc(&device, (size_t)k * sizeof(uint32_t)));
   std::vector<uint32_t> most((size_t)k);
   cudaError_t e = launch_kernel(false, largest_kernel, dim3((unsigned)k), dim3(256), 0, nullptr, b, b_k, b_n, (int)n, device);
   if (e == cudaSuccess) e = cudaMemcpy(most.data(), device, (size_t)k * sizeof(uint32_t), cudaMemcpyDeviceToHost);
-  cudaFree(device);
   if (e != cudaSuccess) return cuda_fail(e, "the largest elements of a weight");
   uint32_t lo = 255, hi = 0;
   for (uint32_t m : most) {
