@@ -279,13 +279,9 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 // (orders nothing: for a barrier that only says "this far")
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta); orders this thread's
-// earlier writes -- and, through a preceding CTA barrier, its CTA's -- before the arrival, cluster-wide.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
-}
-// ... that orders nothing of this thread's memory accesses beyond its own CTA, for a barrier that only says "this far" (tensor memory has
-// been read: tcgen05.fence orders that).  The release over the cluster above costs ~900 cycles, this 26.
+// Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta).  Orders nothing of this thread's memory accesses beyond
+// its own CTA: for a barrier that only says "this far" (tensor memory has been read: tcgen05.fence orders that).  With a release over the
+// cluster (.release.cluster) an arrival costs ~900 cycles, this 26.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
