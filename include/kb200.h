@@ -18,11 +18,11 @@
  * plan's status word, and kb200_plan_bind allocates the library-owned scratch
  * (in BF16 mode a bf16 mirror of the arena and packed bf16 copies of constant
  * matmul operands; in the other modes copies of them laid out along K, for exact
- * FP32 the operands' tails, and aligned copies of operands that a tensor map cannot
+ * FP32 the operands' tails or both operands as pairs of float16, and aligned copies of operands that a tensor map cannot
  * describe, a quarter of the free memory for all of them; a staging buffer for a fused attention whose output aliases
- * its inputs; in FP32 mode the fused attention's scratch: the operands' tails or
- * the split tiles' partial results), converts the constants (cudaDeviceSynchronize) and reads the
- * attention mask back once (a blocking copy).  kb200_plan_launch and
+ * its inputs; in FP32 mode the fused attention's scratch: the operands' tails or pairs and
+ * the split tiles' partial results), converts the constants (cudaDeviceSynchronize) and has a kernel look at the
+ * attention mask (a blocking copy of its answer).  kb200_plan_launch and
  * kb200_kernel_launch neither allocate nor synchronise and are therefore
  * capturable into a CUDA graph; kb200_plan_status is a blocking 4-byte copy.
  */
@@ -71,9 +71,10 @@ typedef enum kb200_kclass {
 /* Arithmetic mode of a matmul's operands (accumulation is always FP32).
  * FP32 corresponds to input_precision="ieee", TF32 to "tf32"
  * (codegen.py:515-516); BF16 is a backend-internal mode with no IR dtype.
- * FP32 on the tensor cores is three TF32 products of split operands: within 1e-5 of exact for
- * finite operands, but in the kernels for many tiles NOT IEEE for non-finite ones (an infinite operand
- * element yields NaN, see cfg[6] bit 1024 below for the CUDA-core kernel that is). */
+ * FP32 on the tensor cores is three products of split operands -- pairs of float16 under a power of two per row where
+ * the weight is frozen and suits, else pairs of TF32: within 1e-5 of exact for finite operands, but in the single-CTA
+ * kernel on TF32 pairs NOT IEEE for non-finite ones (an infinite operand element yields NaN, see cfg[6] bit 1024 below
+ * for the CUDA-core kernel that is; the others sum such rows over in float32). */
 typedef enum kb200_precision {
   KB200_PREC_FP32 = 0,
   KB200_PREC_TF32 = 1,
@@ -148,7 +149,7 @@ typedef struct kb200_kernel_desc {
    * cfg[0] also selects the tensor-core kernel: 0 = library picks, 128 = single-CTA 128-row tiles,
    * 256 = 256-row tiles on SM pairs (cfg[1] then 128 or 256 columns, cfg[2] slabs per step).
    * cfg[6] option bits of the tensor-core matmul (0 = defaults): 512 = two MMA issuers for 64-column
-   * single-CTA tiles; 1024 = an FP32-precision matmul runs on the CUDA cores instead of as three TF32
+   * single-CTA tiles; 1024 = an FP32-precision matmul runs on the CUDA cores instead of as three
    * products of split operands -- needed when an OPERAND may hold +-inf: the split gives inf - inf = NaN
    * tails, so the product is NaN where IEEE arithmetic gives +-inf (the Python side sets this bit on every
    * matmul when KILN_GPU_FP32_MATMUL=ieee), cfg[7] epilogue stores of the tensor-core matmul (0 = library picks,
@@ -189,7 +190,7 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * attention chain (K^T copy, QK^T * scale + causal mask, softmax, PV, head merge; see
  * tests/models/transformer.py:16-25 of the reference), or the seven-kernel chain of a batch of
  * sequences, run it as one fused kernel (in FP32 precision: with float32 products; on the tensor cores with the
- * operands' tails, which the projection in front writes where it can, else a small launch).  The kernel list and
+ * operands' tails or pairs, which the projection in front writes where it can, else a small launch).  The kernel list and
  * arena offsets stay the reference's; the score buffers are then never written.  0 keeps one launch
  * per planned kernel.
  * KB200_OPT_DEPENDENT_LAUNCH (default 1): kernels are enqueued with programmatic stream
@@ -209,25 +210,26 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * This is what the reference's plans contain behind every Linear on a [batch, tokens, d] input: its
  * fusion pass cannot take the activation or the residual add into the matmul's kernel across the
  * reshape between them (kiln/passes/fusion.py:26-35).  0 launches every planned kernel.
- * KB200_OPT_MIRROR_ONLY (default 1, BF16 mode): a LayerNorm, matmul or fused attention whose output is read only by
- * kernels that take its bf16 mirror (tensor-core matmul operands, the fused attention) does not store
- * the float32 values: that arena region then holds stale data, which no planned kernel reads.  0 stores
+ * KB200_OPT_MIRROR_ONLY (default 1, BF16 and FP32 mode): a LayerNorm, matmul or fused attention whose output is read only by
+ * kernels that take its bf16 mirror, or in FP32 mode its pairs of float16 (tensor-core matmul operands, the fused attention),
+ * does not store the float32 values (a LayerNorm does for a row with infinities or NaN): that arena region then holds stale data, which no planned kernel reads.  0 stores
  * both, for a caller that inspects intermediate buffers.
  * KB200_OPT_FP32_ATTENTION (default 0, FP32 precision): which kernel runs the fused attention.
- * 0 = by size (the tensor-core kernel, three TF32 products per float32 product, for sequences of whole
- * tiles of 128 tokens whose work items fill a quarter of the SMs, where it is estimated faster and no
- * matmul of the chain asked for IEEE behaviour on non-finite operands; else the CUDA-core kernel), 1 = always the CUDA-core kernel, 2 = always the tensor cores, with
- * the tails from a launch of its own (the same bits).
+ * 0 = by size and by what is known of the operands: behind a projection whose results the plan can bound (frozen, behind a LayerNorm)
+ * the kernel on pairs of float16, three products per float32 product, for any length above 128 tokens where it is estimated faster than the
+ * CUDA-core kernel; else the kernel with three TF32 products, for sequences of whole tiles of 128 tokens whose work items fill a
+ * quarter of the SMs; else, and where a matmul of the chain asked for IEEE behaviour on non-finite operands, the CUDA-core kernel.
+ * 1 = always the CUDA-core kernel, 2 = always the tensor cores on TF32, with the tails from a launch of its own (the same bits).
  * KB200_OPT_ATTENTION_SPLIT (default 1): in a launch that leaves SMs idle (one long sequence,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.
  * KB200_OPT_WEIGHT_COPIES (default 1, FP32 and TF32 precision): frozen weights are also kept laid out along K
- * and, for FP32, with their tails (twice the weight's own bytes in FP32, once in TF32), as far as a quarter of the
- * free memory goes.  0 = every weight is read where it is, as it is beyond that.
+ * and, for FP32, with their tails, or as pairs of float16 beside a buffer for A's (twice the weight's own bytes in FP32, or once and A's bytes;
+ * once in TF32), as far as a quarter of the free memory goes.  0 = every weight is read where it is, as it is beyond that.
  * KB200_OPT_FEW_TILES (default 0): asks the matmul kernel for few tiles for one of its forms instead of the one it
  * estimates to be quickest, where it covers a matmul: tile columns (64, 96 or 128) + 1000 * K splits (1, 2, 4 or 8)
- * + 10000 * (1 + how A comes, if not through a tensor map of its own: 0 a copy, 1 as float32 for BF16, 2 read by the
- * kernel's warps); a part that is 0 is left to the estimate, a form that the matmul cannot take to the other
+ * + 10000 * (1 + how A comes, if not through a tensor map of its own: 0 a copy, 1 as float32 for BF16, 2 through four
+ * maps, one per residue of its rows); a part that is 0 is left to the estimate, a form that the matmul cannot take to the other
  * kernels.
  * KB200_OPT_OTHERS_IN_FLIGHT (default 0): 1 = other plans run on this GPU at the same time, each with the whole of it
  * (KB200_OPT_CONCURRENCY 1): the last round of a matmul's tiles is then filled by them, and the tile width goes by the work

@@ -8,10 +8,11 @@
 // chain and the mask is the causal one, a fused kernel replaces the five launches: it reads Q, K and
 // V as strided views of the QKV projection's output and writes the merged-heads buffer, the only
 // value of the chain that is live afterwards.  The plan itself (kernel list, arena offsets) is
-// untouched; the score buffers are simply never written.  Three kernels: `attention_kernel` on the tensor
-// cores -- for TF32 operands (described next) and, with its EXACT parameter, for FP32
-// mode (the same structure with three TF32 MMAs per product) --, `attention_fp32_kernel` for short
-// sequences in FP32 mode (CUDA cores), and the one for bf16 operands in attention_bf16.cu.
+// untouched; the score buffers are simply never written.  Kernels: `attention_kernel` on the tensor
+// cores -- for TF32 operands (described next) and, with its EXACT parameter, for FP32 mode behind operands
+// that nothing bounds (the same structure with three TF32 MMAs per product) --, the one on float16 pairs for
+// the other chains in FP32 mode (attention_pairs.cuh), `attention_fp32_kernel` for short sequences there (CUDA
+// cores), and the one for bf16 operands in attention_bf16.cu.
 //
 // Persistent CTAs (one per SM) walk the (sequence, head, 128-query tile) work items, heaviest first, in
 // steps of the grid size: barrier set-up, the TMEM allocation and the latency of an item's first

@@ -135,7 +135,7 @@ struct Plan {
   int few_tiles = 0;             // KB200_OPT_FEW_TILES: the form of the matmul kernel for few tiles that is to be used, 0 = by estimate
   mutable int resident_clusters[9] = {};   // by cluster size, as the few-tiles matmul asked for them (0: not yet)
   mutable int resident_quads = 0;      // clusters of two SM pairs that fit at once, as the pair matmul asked (0: not yet)
-  mutable int resident_exact_quads = 0;      // ... and the exact one
+  mutable int resident_exact_parts[5] = {};  // ... and the exact one, by pairs to a cluster
   uint64_t copy_budget = 0;      // bytes that FP32 and TF32 matmuls may still take for copies, while the plan is bound
   bool weight_copies = true;     // FP32 and TF32: frozen weights are also kept along K, and with their tails, where memory is plenty
   bool fold_copies = true;       // a matmul reads a K-contiguous B at its source; the plan's transposing copy is not launched

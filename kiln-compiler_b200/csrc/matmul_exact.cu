@@ -27,7 +27,7 @@ struct ExactState {
   ExactKernel kernel = nullptr;
   size_t smem = 0;
   unsigned grid = 0;
-  bool split = false;
+  int parts = 1;                         // of K
   int bias_slot = -1, res_slot = -1;
 };
 
@@ -51,18 +51,18 @@ int finish_of(const PlanKernel& k, int* bias_slot, int* res_slot) {
   return FIN_BIAS_RES;
 }
 
-// Clusters of two pairs that fit the GPU at once.
-int resident_quads(const Plan& plan) {
-  int& known = plan.resident_exact_quads;
+// Clusters of `parts` pairs that fit the GPU at once.
+int resident_parts(const Plan& plan, int parts) {
+  int& known = plan.resident_exact_parts[parts];
   if (known == 0) {
     int n = 0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(plan.sm_count / 4 * 4), 1, 1);
+    cfg.gridDim = dim3((unsigned)(plan.sm_count / (2 * parts) * 2 * parts), 1, 1);
     cfg.blockDim = dim3(kExactThreads, 1, 1);
     cfg.dynamicSmemBytes = kExactSmem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 4;
+    attr.val.clusterDim.x = 2 * parts;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -77,32 +77,36 @@ int resident_quads(const Plan& plan) {
   return known;
 }
 
-struct ExactPlan { int bn; bool split; int64_t cycles; };
+struct ExactPlan { int bn, parts; int64_t cycles; };
 
-// Tile width, whether K goes in halves and estimated cycles, the pass over A included: all that runs once, the steps of the rounds, what
-// they cost more the more of the pairs are at work, and per round its drain.  Lines through 419 launches: 160 to 4096 rows of eleven weights
-// from 256 x 1024 to 4096 x 1024, every width timed (2 to 4 % off in the mean square); the choice is 0.07 % from the best on average.  (A
+// Tile width, parts of K and estimated cycles, the pass over A included: all that runs once, the steps of the rounds, what
+// they cost more the more of the pairs are at work, and per round its drain.  Lines through 419 launches, and 336 for the parts of K: 160 to 4096 rows of
+// eleven weights from 256 x 1024 to 4096 x 1024, every width timed (2 to 4 % off in the mean square); the choice is 0.2 % from the best on average.
+// us with two, three and four parts: 333 x 768 x 3072 17.6, 15.2, 14.3 (26.7 in one); 512 x 768 x 3072 18.1, 16.0, 15.2; 1024 x 512 x 2048 15.7, 14.3.  (Of
+// 24 tiles the clusters of three pairs do not all fit at once: 1024 x 768 x 3072 keeps halves.)  (A
 // step of 256 columns has 1536 cycles of multiplying, of 128 columns 768, and the operands come in at 48 KB: 1024 x 2304 x 768 16.3 us at 128
 // columns, 19.9 at 256; 4096 x 3072 x 768 54.1 at 256.)  Plans in flight are no argument: results must not depend on them.
 struct ExactWidth { int bn, once, step, busy, drain; };
-constexpr ExactWidth kExactWidths[] = {{256, 12560, 1497, 574, 4516}, {192, 12550, 1092, 496, 3039}, {160, 11270, 910, 342, 3575}, {128, 12065, 705, 374, 2543}};
-constexpr ExactWidth kExactHalves = {128, 14616, 733, 208, 1695};        // K in halves on twice the pairs
+constexpr ExactWidth kExactWidths[] = {{256, 11060, 1497, 574, 4516}, {192, 11050, 1092, 496, 3039}, {160, 9770, 910, 342, 3575}, {128, 10565, 705, 374, 2543}};
+// K in two, three and four parts on as many times the pairs
+constexpr ExactWidth kExactParts[] = {{128, 12915, 706, 259, 1945}, {128, 12823, 736, 214, 3606}, {128, 10919, 625, 406, 7082}};
 
 // (Of all that runs once, ~4300 are the pass, which a producer that splits A's rows takes over: 1024 x 2304 x 768 16.3 -> 13.0 us.)
 ExactPlan plan_exact(const Plan& plan, int64_t m, int64_t n, int64_t k, bool split) {
   const int64_t pairs = plan.sm_count / 2, steps = (k + kExactStepK - 1) / kExactStepK, pass = split ? -4300 : m * k / 714;
-  ExactPlan best{0, false, 0};
+  ExactPlan best{0, 1, 0};
   for (const ExactWidth& w : kExactWidths) {
     if (w.bn > 128 && w.bn / 2 >= n) continue;
     const int64_t tiles = ((m + 255) / 256) * ((n + w.bn - 1) / w.bn), rounds = (tiles + pairs - 1) / pairs;
     const int64_t cycles = w.once + pass + rounds * (steps * w.step + w.drain) + steps * w.busy * tiles / pairs;
-    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
+    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, 1, cycles};
   }
-  const ExactWidth& h = kExactHalves;
-  const int64_t tiles = ((m + 255) / 256) * ((n + h.bn - 1) / h.bn), half = (steps + 1) / 2;
-  if (steps >= 4 && tiles <= resident_quads(plan)) {
-    const int64_t cycles = h.once + pass + half * h.step + (half * h.busy + h.drain) * 2 * tiles / pairs;
-    if (cycles < best.cycles) best = {h.bn, true, cycles};
+  for (int parts = 2; parts <= 4; ++parts) {
+    const ExactWidth& h = kExactParts[parts - 2];
+    const int64_t tiles = ((m + 255) / 256) * ((n + h.bn - 1) / h.bn), part = (steps + parts - 1) / parts;
+    if (steps < 2 * parts || tiles * parts > pairs || tiles > resident_parts(plan, parts)) continue;
+    const int64_t cycles = h.once + pass + part * h.step + (part * h.busy + h.drain) * parts * tiles / pairs;
+    if (cycles < best.cycles) best = {h.bn, parts, cycles};
   }
   return best;
 }
@@ -130,9 +134,8 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   const int fin = finish_of(k, &st->bias_slot, &st->res_slot);
   p.bn = how.bn;
   p.half_bn = how.bn / 2;
-  st->split = how.split;
+  st->parts = p.parts = how.parts;
   p.steps = (int)((k.K + kExactStepK - 1) / kExactStepK);
-  p.first_steps = (p.steps + 1) / 2;
   p.sums = 512 / how.bn < kExactMaxSums ? 512 / how.bn : kExactMaxSums;
   const int stage_bytes = 2 * (kExactABytes + p.half_bn * 128), rest = kExactWarps * kExactSlot;
   p.stages = (kExactSmem - rest) / stage_bytes < kExactMaxStages ? (kExactSmem - rest) / stage_bytes : kExactMaxStages;
@@ -165,7 +168,7 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   // Persistent pairs, up to this plan's share of the GPU with several in flight.
   const int pairs = plan.sm_count / 2, share = plan.concurrency > 1 && pairs / plan.concurrency > 0 ? pairs / plan.concurrency : pairs;
   const int rounds = (p.num_tiles + share - 1) / share;
-  st->grid = (unsigned)(st->split ? 4 * p.num_tiles : 2 * ((p.num_tiles + rounds - 1) / rounds));
+  st->grid = (unsigned)(st->parts > 1 ? 2 * st->parts * p.num_tiles : 2 * ((p.num_tiles + rounds - 1) / rounds));
   bool ok = encode_map(&st->map_a, true, ops.a, k.K, k.M, 2, ops.pitch, k.M * ops.pitch, kExactStepK, 128, false, 2) &&
             encode_map(&st->map_b, true, ops.b, k.K, k.N, 2, ops.pitch, k.N * ops.pitch, kExactStepK, p.half_bn, false, 2) &&
             encode_map_store(&st->map_out, false, O.ptr, k.N, k.M, 1, O.stride[1], 0);
@@ -173,7 +176,7 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   if (ok && p.res) ok = encode_map_store(&st->map_res, false, p.res, k.N, k.M, 1, p.res_row, 0);
   if (ok && p.with_tail) ok = set_map_address(&st->map_tail, k.tail_out);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = st->split ? exact_kernel<2, true>(fin) : p.bn > 192 ? exact_kernel<4, false>(fin) : p.bn > 128 ? exact_kernel<3, false>(fin) : exact_kernel<2, false>(fin);
+  st->kernel = st->parts > 1 ? exact_kernel<2, true>(fin) : p.bn > 192 ? exact_kernel<4, false>(fin) : p.bn > 128 ? exact_kernel<3, false>(fin) : exact_kernel<2, false>(fin);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExactSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_exact_kernel)"); }
   cudaFuncAttributes attributes;
@@ -192,7 +195,7 @@ int exact_launch(const Plan& plan, const void* state, cudaStream_t s) {
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = st->split ? 4 : 2;
+  attr[0].val.clusterDim.x = 2 * st->parts;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
@@ -212,7 +215,7 @@ bool exact_repoint(const PlanKernel& k, void* state) {
 
 std::string exact_detail(const void* state) {
   const ExactState* st = static_cast<const ExactState*>(state);
-  return "mm_exact " + std::to_string(st->params.bn) + " columns" + (st->split ? ", 2 splits" : "");
+  return "mm_exact " + std::to_string(st->params.bn) + " columns" + (st->parts > 1 ? ", " + std::to_string(st->parts) + " splits" : "");
 }
 
 bool exact_write_pairs(const PlanKernel& k, void* state, const PlanKernel::Planes& to, const float* scale, bool store32) {

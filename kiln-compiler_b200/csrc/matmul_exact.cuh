@@ -18,8 +18,9 @@
 //   warps 4-11  two per tensor-memory lane quadrant; a lane has a row, warp h of a quadrant the 32-column blocks h, h + 2, ...: adds up
 //               the steps, then scales, finishes and stores its blocks while the tensor cores work on the next tile
 //
-// Few tiles and a long K (SPLIT): a cluster of two pairs, each with half of K for the same tile; the sums of the other pair's half of the
-// columns are sent into that CTA's ring, idle by then, as bulk copies.
+// Few tiles and a long K (SPLIT): a cluster of two to four pairs, each with its part of K for the same tile of 128 columns.  A pair finishes
+// some of the tile's 32-column blocks: the sums of the others' are sent into their rings, idle by then, as bulk copies, and added up in the
+// order of the pairs.
 // Every wait is bounded: see matmul_pair.cu.
 #pragma once
 
@@ -58,7 +59,7 @@ enum : int { FIN_NONE = 0, FIN_BIAS, FIN_BIAS_GELU, FIN_BIAS_RES };
 
 struct ExactParams {
   int bn, half_bn, stages, steps;
-  int first_steps;       // SPLIT: of the first pair
+  int parts;             // SPLIT: pairs to a tile, two to four, each with its part of K
   int sums;              // accumulators in turn
   uint32_t idesc;
   int tiles_n, num_tiles;
@@ -110,6 +111,12 @@ __device__ __forceinline__ void add_staged(float (&v)[32], const uint8_t* block,
   }
 }
 
+// K in parts: the first of a tile's four blocks that pair `part` finishes (two, two | two, one, one | one each), a block's pair, and where in
+// the area for it a part comes, in blocks of a lane quadrant.
+__device__ __forceinline__ int first_block_of(int part, int parts) { return parts == 2 ? 2 * part : parts == 3 && part > 0 ? part + 1 : part; }
+__device__ __forceinline__ int owner_of(int block, int parts) { return parts == 2 ? block >> 1 : parts == 3 && block > 0 ? block - 1 : block; }
+__device__ __forceinline__ int received_at(int block, int from, int parts) { return (block * (parts - 1) + from) * 4; }
+
 // BLOCKS: 32-column blocks of a tile per warp, at most.
 template <int BLOCKS, int FIN, bool SPLIT>
 __global__ void __launch_bounds__(kExactThreads, 1)
@@ -127,12 +134,13 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   const int warp = warp_index(), lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  // with SPLIT the CTAs 0, 1 and 2, 3 of a cluster are a pair each, `pair` counts clusters, and a cluster has one tile
-  const uint32_t leader = SPLIT ? rank & 2u : 0u, cta = rank;
+  // with SPLIT the CTAs 0, 1 and 2, 3 (and so on) of a cluster are a pair each, `pair` counts clusters, and a cluster has one tile
+  const uint32_t leader = SPLIT ? rank & 6u : 0u;
   rank &= 1u;
-  const int pair = blockIdx.x >> (SPLIT ? 2 : 1), num_pairs = gridDim.x >> (SPLIT ? 2 : 1);
-  const int step0 = SPLIT && leader != 0 ? p.first_steps : 0;                                     // this pair's steps of K
-  const int n_steps = !SPLIT ? p.steps : leader != 0 ? p.steps - p.first_steps : p.first_steps;
+  const int parts = SPLIT ? p.parts : 1, part = (int)leader / 2;
+  const int pair = SPLIT ? (int)blockIdx.x / (2 * parts) : blockIdx.x >> 1, num_pairs = SPLIT ? p.num_tiles : gridDim.x >> 1;
+  const int step0 = SPLIT ? (part * p.steps + parts - 1) / parts : 0;                             // this pair's steps of K
+  const int n_steps = SPLIT ? ((part + 1) * p.steps + parts - 1) / parts - step0 : p.steps;
   const uint16_t pair_ctas = (uint16_t)(3u << leader);
   const uint32_t bar0 = smem_u32(&bars[0]);
   const uint32_t full0 = bar0 + 8 * BAR_FULL, empty0 = bar0 + 8 * BAR_EMPTY, ready0 = bar0 + 8 * BAR_READY, added0 = bar0 + 8 * BAR_ADDED;
@@ -146,7 +154,8 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
   if (warp == 0) {
     if (lane == 0) abort_flag = 0;
     for (int b = lane; b < BAR_COUNT; b += 32)
-      mbar_init(bar0 + 8 * b, b >= BAR_ADDED && b < BAR_RES ? 2 * kExactWarps : 1);      // both CTAs' warps release an accumulator
+      // (both CTAs' warps release an accumulator; a CTA of every other pair says that its ring is idle)
+      mbar_init(bar0 + 8 * b, b >= BAR_ADDED && b < BAR_RES ? 2 * kExactWarps : SPLIT && b == BAR_PEER ? parts - 1 : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
@@ -263,7 +272,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     const uint32_t added_leader0 = map_to_cta(added0, leader);
     const int blocks = p.bn / 32;
     // the blocks of a tile that this pair finishes
-    const int first_block = SPLIT && leader != 0 ? blocks / 2 : 0, end_block = SPLIT ? first_block + blocks / 2 : blocks;
+    const int first_block = SPLIT ? first_block_of(part, parts) : 0, end_block = SPLIT ? first_block_of(part + 1, parts) : blocks;
     const uint64_t policy = l2_policy(p.stream_out != 0);
     uint32_t res_phase = 0;
     int sum = 0;
@@ -338,24 +347,20 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #pragma unroll
             for (int q = 0; q < 32; ++q) v[q] = sums[i][q];
       };
-      // SPLIT: the sums of the other pair's columns leave for its CTA with the same rows, those of this one's columns come from there.  The
-      // rings are idle: one half of this CTA's is what it sends, the other half what it gets.
-      [[maybe_unused]] const uint32_t recv_area = (uint32_t)(blocks / 2 * 4 * 4096);
+      // SPLIT: the sums of the other pairs' columns leave for their CTAs with the same rows, those of this one's columns (a block a warp, at most)
+      // come from there.  The rings are idle: behind the four blocks that this CTA may send is what it gets, by block and pair.
+      [[maybe_unused]] const uint32_t recv_area = (uint32_t)(blocks * 4 * 4096);
       if constexpr (SPLIT) {
         if (!dry) {
-          const uint32_t other = cta ^ 2u;
-          if (e == 0 && lane == 0) mbar_arrive_remote(map_to_cta(bar0 + 8 * BAR_PEER, other));      // this CTA's ring may be written
-          uint32_t coming = 0;
-          for (int c = half; c < blocks; c += 2)
-            if (c >= first_block && c < end_block && rows_ok && n0 + 32 * c < p.N) coming += 4096;
-          if (lane == 0 && coming != 0) mbar_expect_tx(recv_bar, coming);
+          if (e == 0 && lane < parts && lane != part) mbar_arrive_remote(map_to_cta(bar0 + 8 * BAR_PEER, 2 * lane + rank));      // this CTA's ring may be written
+          if (lane == 0 && first_own >= 0) mbar_expect_tx(recv_bar, (uint32_t)(parts - 1) * 4096u);
           bool free = false;
 #pragma unroll 1
           for (int j = 0; j < BLOCKS; ++j) {
             const int c = half + 2 * j;
             if (c >= blocks || !rows_ok || n0 + 32 * c >= p.N) break;
             if (c >= first_block && c < end_block) continue;
-            const uint32_t at = (uint32_t)(((c - (blocks / 2 - first_block)) * 4 + quad) * 4096);
+            const uint32_t at = (uint32_t)((c * 4 + quad) * 4096);
             float v[32];
             pick(v, j);
             uint8_t* const mine = smem_raw + at;
@@ -366,7 +371,11 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
               free = all_waited(mbar_wait_cluster(bar0 + 8 * BAR_PEER, 0, abort_ptr), 7);
               if (!free) break;
             }
-            if (lane == 0) push_block(map_to_cta(ring + recv_area + at, other), ring + at, 4096, map_to_cta(recv_bar, other));
+            if (lane == 0) {
+              const int owner = owner_of(c, parts);
+              const uint32_t to = recv_area + (uint32_t)(received_at(c - first_block_of(owner, parts), part < owner ? part : part - 1, parts) + quad) * 4096u;
+              push_block(map_to_cta(ring + to, 2 * owner + rank), ring + at, 4096, map_to_cta(recv_bar, 2 * owner + rank));
+            }
           }
         }
       }
@@ -402,7 +411,8 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           if (!dry) {
             if (!mbar_wait_cluster(recv_bar, 0, abort_ptr)) give_up(6);
             __syncwarp();
-            add_staged(v, smem_raw + recv_area + ((c - first_block) * 4 + quad) * 4096, lane);
+            for (int from = 0; from < parts - 1; ++from)
+              add_staged(v, smem_raw + recv_area + (received_at(c - first_block, from, parts) + quad) * 4096, lane);
           }
         }
         // (the columns' scales first: their exponents are within 2^60, a row's need not be)

@@ -803,6 +803,13 @@ int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64
   return plan_small(k.M, k.N, k.K, small_mode(d.precision, form), form == SMALL_A_GATHERED, bf16 && !b_kmajor, close, plan).cycles;
 }
 
+int small_sum_length(const Plan& plan, const PlanKernel& k) {
+  const SmallPlan how = plan_small(k.M, k.N, k.K, SMALL_EXACT, false, false, false, plan);
+  const int64_t steps = (k.K + 31) / 32;
+  const Accumulate a = accumulate_as((int)((steps + how.splits - 1) / how.splits), how.bn, accumulate_limit(k.M, k.N, k.K, false));
+  return a.shift == 2 ? 4 * a.steps : 1 << a.shift;
+}
+
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, bool close, void** state) {
   *state = nullptr;
   if (k.desc.precision == KB200_PREC_FP32 && b_tail == nullptr)

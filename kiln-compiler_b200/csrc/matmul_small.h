@@ -13,6 +13,8 @@ enum SmallA : int { SMALL_A_MAPPED, SMALL_A_FLOAT32, SMALL_A_GATHERED };
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
 // `close`: exact FP32 as near to float64 as float32 sums on the CUDA cores.
 int64_t small_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols, SmallA form, bool close);
+// Exact FP32: MMAs along K that go into one accumulator, where the kernel covers this matmul.
+int small_sum_length(const Plan& plan, const PlanKernel& k);
 // Tensor maps and launch parameters.  `b_tail`: exact FP32, the tails of B in the layout of ops.b_base.
 // *state stays null when the operands cannot be described; a non-zero return is an error.
 int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& ops, const float* b_tail, SmallA form, bool close,

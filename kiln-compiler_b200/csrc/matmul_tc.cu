@@ -1206,10 +1206,13 @@ int tc_bind(Plan& plan, PlanKernel& k, int kernel_index) {
   // (its exact-FP32 form multiplies with the tails of B: without room for them this file's kernel makes them as it goes)
   const bool tails_ready = d.precision != KB200_PREC_FP32 || presplit;
   const bool small = few > 0 && tails_ready && (many == 0 || few < many || close_only);
-  // Float16 pairs on SM pairs: where there are many tiles (fewer are summed more closely than that kernel does, see accumulate_limit) and the
-  // estimates say so, its pass over A included.
-  if (presplit && plain && plan.few_tiles == 0 && ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128) > 16) {
-    const int64_t cycles = exact_cycles(plan, k) * 9 / 10;         // (of 1.9 to the ns; the small kernel's are 1.65)
+  // Float16 pairs on SM pairs: where there are many tiles (fewer are summed more closely than that kernel does, see accumulate_limit; so are more of
+  // a short K: with four MMAs to an accumulator 1.1e-7, here 2.1e-7, with eight 2.5e-7) and the estimates say so, its pass over A included.
+  if (presplit && plain && plan.few_tiles == 0 && ((k.M + kTileM - 1) / kTileM) * ((k.N + 127) / 128) > 16 && (few < 0 || small_sum_length(plan, k) > 4)) {
+    int64_t cycles = exact_cycles(plan, k) * 22 / 25;              // (of 1.93 to the ns; the small kernel's are 1.67: 391 shapes, none slower by it)
+    // With a pass in front it is two launches, 6 to 11 us of the host's (1000 x 768 x 512 8.9 us for the GPU; a call of it 9.3 to 11.6, of the small
+    // kernel 9.8 to 10.3).
+    if (cycles > 0 && cycles < 19000 && !k.planes_expected) cycles = 19000;
     if (cycles > 0 && (few < 0 || cycles < few) && (many == 0 || cycles < many)) {
       const int rc = bind_pairs16(plan, k, kernel_index, st, turn, b_src_row);
       if (rc) return rc;

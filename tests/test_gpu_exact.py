@@ -50,7 +50,9 @@ def call(exe, x):
 @pytest.mark.parametrize("m,n,k,form", [(1024, 2304, 768, "128 columns"), (1000, 2300, 772, "128 columns"), (2048, 4092, 1028, "160 columns"),
                                         (700, 4096, 1024, "192 columns"), (2000, 3068, 772, "192 columns"), (513, 4096, 4096, "192 columns"),
                                         (3000, 3072, 768, "256 columns"), (3001, 3004, 516, "256 columns"),
-                                        (1024, 768, 3072, "128 columns, 2 splits"), (999, 772, 2052, "128 columns, 2 splits")])
+                                        (1024, 768, 3072, "128 columns, 2 splits"), (999, 772, 2052, "128 columns, 2 splits"),
+                                        (1024, 512, 2048, "128 columns, 3 splits"), (999, 508, 2052, "128 columns, 3 splits"),
+                                        (512, 768, 3072, "128 columns, 4 splits"), (300, 644, 3084, "128 columns, 4 splits")])
 def test_widths(m, n, k, form):
     exe, x, c = build(m, n, k, positive=True)
     assert f"mm_exact {form}" in exe.details[0], exe.details
@@ -61,7 +63,7 @@ def test_widths(m, n, k, form):
 
 
 @pytest.mark.parametrize("chain", ["none", "bias", "gelu", "residual"])
-@pytest.mark.parametrize("m,n,k", [(1024, 768, 3072), (1500, 2308, 772)])
+@pytest.mark.parametrize("m,n,k", [(1024, 768, 3072), (1500, 2308, 772), (999, 508, 2052), (300, 644, 3084)])
 def test_chains(m, n, k, chain):
     exe, x, c = build(m, n, k, chain)
     assert "mm_exact" in exe.details[0], exe.details
