@@ -707,17 +707,21 @@ PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, bool b
   classify_steps(k, nullptr, &matrix);
   const int64_t once = kPairOnce + (matrix != nullptr ? kPairMatrixOperand : 0);
   PairPlan best{0, false, 0};
+  int64_t least = 0;                    // what `best` is compared by
   for (const PairWidth& w : kPairWidths) {
     if (!width_fits(k, w, b_kmajor)) continue;
     const int64_t tiles = tiles_of(k, w), rounds = (tiles + share - 1) / share;
     int64_t cycles = once + rounds * (slabs * (w.alone + one_slab(w, two_slabs)) + w.drain) + slabs * (w.full - w.alone) * tiles / share;
     // (Beyond ~80 us the GPU is at its power limit, where the bytes a tile moves for its work count: 4096^3 TF32 191 us at 256 columns, 201 at 192.)
     if (cycles > 150000) cycles += cycles * (256 - w.bn) / 2560;
-    if (best.bn == 0 || cycles < best.cycles) best = {w.bn, false, cycles};
+    if (best.bn == 0 || cycles < least) best = {w.bn, false, cycles}, least = cycles;
     // K in halves on twice the pairs
     if (w.halves == 0 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
     const int64_t halved = w.halves + (slabs + 1) / 2 * w.half_alone + ((slabs + 1) / 2 * (w.half_full - w.half_alone) + kPairHalvesBusy) * 2 * tiles / share;
-    if (halved < best.cycles) best = {w.bn, true, halved};
+    // (Of two that cost alike by the lines halves move fewer bytes: 1900 x 960 x 3840 TF32 25.8 us at 128 columns with its operands in L2 and up to 31
+    // behind another matmul, 25.8 and 26.4 in halves of 256.)
+    const int64_t as = slabs < 64 ? halved : halved * 49 / 50;
+    if (as < least) best = {w.bn, true, halved}, least = as;
   }
   return best;
 }
@@ -743,8 +747,12 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
 
 }  // namespace
 
-// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9)
-int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) { return plan_pair(plan, k, true, b_kmajor).cycles * 7 / 8; }
+// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9.  A GELU in float32 costs this kernel's last
+// tile 0.9 us, that one's, spread over more warps, 0.55: 1002 x 1024 x 256 6.55 and 6.15, without it 5.5 both.)
+int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) {
+  const bool gelu = k.desc.precision == KB200_PREC_TF32 && k.chain.n > 0 && k.chain.steps[k.chain.n - 1].op == CH_GELU_TANH;
+  return (plan_pair(plan, k, true, b_kmajor).cycles + (gelu ? 700 : 0)) * 7 / 8;
+}
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
   const kb200_kernel_desc& d = k.desc;
