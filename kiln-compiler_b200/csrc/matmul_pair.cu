@@ -668,8 +668,8 @@ int resident_quads(const Plan& plan) {
 // more of the pairs are at work (one SM gets 60 to 75 bytes a clock from L2; a slab of 256 columns has 512 cycles of multiplying).
 // K in halves: the exchange and its own start instead.  Lines through 512 launches in TF32 and BF16, every width and both
 // forms of each timed: 160 to 4096 rows of sixteen weights from 256 x 1024 to 4096 x 4096.  The choice is 0.1 % from the best on average,
-// and against the few-tiles kernel 0.1 % (TF32) and 0.2 % (BF16); with the lines of the epilogue that released over the cluster it was 0.2 %, and 0.8
-// and 0.5 % (1024 x 2304 x 768 BF16 10.2 against 9.5 us, 256 x 4096 x 1000 TF32 10.6 against 9.7).
+// with the lines of the epilogue that released over the cluster it was 0.2 %, and against the few-tiles kernel 0.8
+// and 0.5 % (TF32, BF16; 1024 x 2304 x 768 BF16 10.2 against 9.5 us, 256 x 4096 x 1000 TF32 10.6 against 9.7).
 // The widths between 128 and 256 are for the last round: 2048 x 3072 x 768 TF32 21.2 us at 128 columns (three rounds, 64 of 74 pairs),
 // 23.5 at 256 (96 tiles), 19.5 at 192 (128 tiles, two rounds); 8192 x 768 x 3072 BF16 66.2 at 256, 59.5 at 192 (with its pass
 // over A); 8192 x 2304 x 768 36.1 at 256, 39.7 at 192.
@@ -747,11 +747,12 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
 
 }  // namespace
 
-// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.9.  A GELU in float32 costs this kernel's last
+// (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.86: of 281 launches the choice is then 0.1 % (TF32)
+// and 0.3 % (BF16) from the better kernel.  A GELU in float32 costs this kernel's last
 // tile 0.9 us, that one's, spread over more warps, 0.55: 1002 x 1024 x 256 6.55 and 6.15, without it 5.5 both.)
 int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) {
   const bool gelu = k.desc.precision == KB200_PREC_TF32 && k.chain.n > 0 && k.chain.steps[k.chain.n - 1].op == CH_GELU_TANH;
-  return (plan_pair(plan, k, true, b_kmajor).cycles + (gelu ? 700 : 0)) * 7 / 8;
+  return (plan_pair(plan, k, true, b_kmajor).cycles + (gelu ? 700 : 0)) * 8 / 9;
 }
 
 bool pair_eligible(const Plan& plan, const PlanKernel& k, bool b_kmajor, int64_t b_cols) {
