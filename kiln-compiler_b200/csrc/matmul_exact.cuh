@@ -394,8 +394,10 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         if (c >= end_block || n >= p.N) break;          // uniform across the warp
         const uint32_t at = staging(j);
         uint8_t* const at_ptr = smem_raw + (at - ring);
-        if (j != first_own && !last && lane == 0) {
-          store_wait_read(0);                           // the slot's last bulk store has finished reading it
+        // What is staged in the slot may still be on its way out: with a short K a tile's sums are ready before the last tile's store has read
+        // it.  (A residual's first block is there already, behind a wait of its own.)
+        if (at == slot && lane == 0 && !(FIN == FIN_BIAS_RES && j == first_own)) {
+          store_wait_read(0);
           if (FIN == FIN_BIAS_RES) request(j);
         }
         float scale = scale_of[0], bias = bias_of[0];
