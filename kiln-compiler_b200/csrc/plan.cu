@@ -1029,20 +1029,25 @@ static float pair_scale(float bound) {
   return ldexpf(1.0f, 15 - e);
 }
 
+// Operand A of this matmul, if it lies in the arena, and the kernel that wrote all of it last, or null.
+static PlanKernel* producer_of_a(Plan& plan, size_t ki) {
+  const PlanKernel& k = plan.kernels[ki];
+  const Span x = span_of(k, k.desc.a_slot);
+  if (k.desc.operands[k.desc.a_slot].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) return nullptr;
+  return mirroring_producer(plan, ki, x);
+}
+
 // Will operand A come as float16 pairs, should the matmul multiply those?  Asked before it is bound, and after its producer was.
 static int expect_planes(Plan& plan, size_t ki) {
   PlanKernel& k = plan.kernels[ki];
-  if (const PlanKernel* const norm = layernorm_in_front(plan, ki)) {
+  const PlanKernel* const from = producer_of_a(plan, ki);
+  if (from == nullptr) return KB200_OK;
+  for (size_t i = 0; i < ki; ++i)            // (a kernel has one reader that it splits its rows for)
+    if (plan.kernels[i].planes_expected && producer_of_a(plan, i) == from) return KB200_OK;
+  if (layernorm_in_front(plan, ki) != nullptr) {
     k.planes_expected = true;
-    for (size_t i = 0; i < ki; ++i)            // (a LayerNorm has one reader that it splits its rows for)
-      if (plan.kernels[i].planes_expected && layernorm_in_front(plan, i) == norm) k.planes_expected = false;
     return KB200_OK;
   }
-  const int a = k.desc.a_slot;
-  const Span x = span_of(k, a);
-  if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) return KB200_OK;
-  const PlanKernel* const from = mirroring_producer(plan, ki, x);
-  if (from == nullptr) return KB200_OK;
   if (from->impl == IMPL_ATTN_FUSED) {
     k.planes_expected = attention_may_write_pairs(*from);
     return KB200_OK;
@@ -1086,10 +1091,10 @@ static int hand_on_planes(Plan& plan) {
       norm->mirror_only = plan.mirror_only && only_read_as(plan, (size_t)(norm - plan.kernels.data()), span_of(*norm, norm->out_slot), reads_here);
       continue;
     }
-    const Span x = span_of(k, a);
-    if (k.desc.operands[a].base_kind != KB200_BASE_ARENA || x.lo < plan.arena || x.hi > plan.arena + plan.arena_bytes / 4) continue;
-    PlanKernel* const from = mirroring_producer(plan, ki, x);
-    if (from != nullptr && from->impl == IMPL_ATTN_FUSED) {
+    // (planes for one reader: what another one multiplies would be left unwritten)
+    PlanKernel* const from = producer_of_a(plan, ki);
+    if (from == nullptr || from->planes_out.heads != nullptr) continue;
+    if (from->impl == IMPL_ATTN_FUSED) {
       // the merged heads, convex combinations of V's rows
       const size_t fi = (size_t)(from - plan.kernels.data());
       int64_t elems = 0;
@@ -1098,12 +1103,13 @@ static int hand_on_planes(Plan& plan) {
       if (y->ptr != k.ops[a].ptr || k.ops[a].stride[1] != k.K || k.ops[a].stride[2] != 1 || elems != k.M * k.K) continue;
       const bool alone = plan.mirror_only && only_read_as(plan, fi, Span{y->ptr, y->ptr + elems}, reads_here);
       if (!attention_write_pairs(*from, planes, alone, &back)) continue;
+      from->planes_out = planes;
       const std::vector<float> all((size_t)k.M, back);
       KB200_CUDA(cudaMemcpy(planes.scales, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice));
       matmul_planes_come_ready(k);
       continue;
     }
-    if (from == nullptr || from->impl != IMPL_MM_TC || from->planes_out.heads != nullptr || from->M != k.M || from->N != k.K) continue;
+    if (from->impl != IMPL_MM_TC || from->M != k.M || from->N != k.K) continue;
     const DevOperand &out = from->ops[from->chain.out_slot], &in = k.ops[a];
     if (out.ptr != in.ptr || out.stride[1] != in.stride[1]) continue;
     const size_t fi = (size_t)(from - plan.kernels.data());
