@@ -135,7 +135,7 @@ struct AttnState {
     PairsParams params;
     const float* by() const { return factors + 2 * params.a.H + 1; }
   } pairs;
-  float out_bound = 0.0f;          // FP32 mode: of the merged heads, convex combinations of V's rows, where it is known
+  float out_bound = 0.0f;          // FP32 mode: of the merged heads, convex combinations of V's rows, where it is known and much the same for all
   bool ieee = false;               // the plan asked for IEEE behaviour on non-finite operands
   bool asked = false;              // a kernel was asked for by option
   bool may_split = false;
@@ -1516,7 +1516,7 @@ int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_
   const int64_t width = (int64_t)p.H * kHeadDim;
   const int64_t first[3] = {st->q_ptr - src, st->k_ptr - src, st->v_ptr - src};
   std::vector<float> factors(2 * p.H + 1, 1.0f), by((size_t)cols / 32, 0.0f);
-  float out_bound = 0.0f;
+  float out_bound = 0.0f, out_least = INFINITY;
   for (int role = 0; role < 3; ++role) {
     if (first[role] < 0 || first[role] % 32 || first[role] + width > cols) return KB200_OK;
     for (int h = 0; h < p.H; ++h) {
@@ -1530,13 +1530,13 @@ int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_
       if (blocks[0] != 0.0f || blocks[1] != 0.0f) return KB200_OK;          // views that overlap
       blocks[0] = blocks[1] = scale;
       factors[(size_t)(role == 2 ? p.H + h : h)] /= role == 2 ? scale * kPairsUp : scale;
-      if (role == 2) out_bound = std::max(out_bound, most);
+      if (role == 2) out_bound = std::max(out_bound, most), out_least = std::min(out_least, least);
     }
   }
   for (int h = 0; h < p.H; ++h) factors[h] *= p.scale_log2;
   for (float& b : by)
     if (b == 0.0f) b = 1.0f;
-  st->out_bound = out_bound;
+  if (out_bound <= 1024.0f * out_least) st->out_bound = out_bound;      // (one power of two for the merged heads, as for a matmul's results)
   if (st->ieee || st->asked) return KB200_OK;
   // The CUDA-core kernel (see finish_fusion) stays where it is quicker, and for one tile of keys in few items, where it is 8 % nearer to float64
   // (12 heads of 128 tokens 2.2e-7 and 2.3e-7, 9.0 and 8.0 us).

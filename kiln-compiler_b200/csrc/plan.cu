@@ -1029,6 +1029,15 @@ static float pair_scale(float bound) {
   return ldexpf(1.0f, 15 - e);
 }
 
+// Can results with these bounds by column leave as float16 pairs under one power of two?  A column whose bound is far above the others' -- a unit that a
+// bias of -1e9 switches off, say -- would leave the others none of the bits.  (Columns that are zero for any input take no part.)
+static bool one_scale_suits(const std::vector<float>& bounds) {
+  float least = INFINITY, most = 0.0f;
+  for (float b : bounds)
+    if (b != 0.0f) least = std::min(least, b), most = std::max(most, b);
+  return most > 0.0f && most <= 1024.0f * least;
+}
+
 // Operand A of this matmul, if it lies in the arena, and the kernel that wrote all of it last, or null.
 static PlanKernel* producer_of_a(Plan& plan, size_t ki) {
   const PlanKernel& k = plan.kernels[ki];
@@ -1056,7 +1065,7 @@ static int expect_planes(Plan& plan, size_t ki) {
   if (from->impl != IMPL_MM_TC || !matmul_takes_planes(*from, &planes) || from->N != k.K) return KB200_OK;
   const std::vector<float>* bounds = nullptr;
   const int rc = result_bounds(plan, (size_t)(from - plan.kernels.data()), &bounds);
-  k.planes_expected = rc == KB200_OK && !bounds->empty();
+  k.planes_expected = rc == KB200_OK && one_scale_suits(*bounds);
   return rc;
 }
 
@@ -1116,7 +1125,7 @@ static int hand_on_planes(Plan& plan) {
     const std::vector<float>* bounds = nullptr;
     const int rc = result_bounds(plan, fi, &bounds);
     if (rc) return rc;
-    if (bounds->empty()) continue;
+    if (!one_scale_suits(*bounds)) continue;
     const float scale = pair_scale(*std::max_element(bounds->begin(), bounds->end()));
     const float* const by = keep_scales(plan, std::vector<float>((size_t)(from->N + 31) / 32, scale));
     const bool alone = plan.mirror_only && only_read_as(plan, fi, span_of(*from, from->chain.out_slot), reads_here);
