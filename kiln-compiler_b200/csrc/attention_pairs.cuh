@@ -1,5 +1,5 @@
 // Fused causal attention in exact FP32 on float16 pairs: QK^T -> online softmax -> PV with float32 products, each of three float16 ones
-// (x 2^e = h + t, see split_rows.cu; the probabilities are split here, times 2^14).  Role, items, pipeline and the softmax of two threads
+// (x 2^e = h + 2^-11 t, see split_rows.cu; the probabilities are split here, times 2^14).  Role, items, pipeline and the softmax of two threads
 // a row are attention_kernel's (attention.cu); what differs:
 //   * Q, K and V come as two planes of float16 under a power of two per head, whose bound the plan knows (see result_bounds); both fit
 //     shared memory twice, where the TF32 form's heads and tails fit once, and multiply at twice the rate;
@@ -52,7 +52,8 @@ __device__ __forceinline__ void split_probabilities(const float (&v)[32], uint32
     const float2 x = fmul2(make_float2(v[2 * i], v[2 * i + 1]), make_float2(kPairsUp, kPairsUp));
     const __half2 h = __floats2half2_rn(x.x, x.y);
     const float2 back = __half22float2(h);
-    const __half2 t = __floats2half2_rn(x.x - back.x, x.y - back.y);
+    const float2 rest = ffma2(back, make_float2(-kTailUp, -kTailUp), fmul2(x, make_float2(kTailUp, kTailUp)));
+    const __half2 t = __floats2half2_rn(rest.x, rest.y);
     heads[i] = *reinterpret_cast<const uint32_t*>(&h);
     tails[i] = *reinterpret_cast<const uint32_t*>(&t);
   }
@@ -174,9 +175,11 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int pass = 0; pass < 3; ++pass) {
         const uint32_t qa = q_smem + (pass == 0 ? kPairsPlane : 0), ka = kb + (pass == 1 ? kPairsPlane : 0);
 #pragma unroll
-        for (int kd = 0; kd < 4; ++kd)
-          umma_if(on, tmem_base + (uint32_t)s * 128, make_desc(qa + kd * 32, 16, 1024), make_desc(ka + kd * 32, 16, 1024), p.idesc_qk,
-                  (pass | kd) != 0 ? 1u : 0u, true);
+        for (int kd = 0; kd < 4; ++kd) {
+          const uint64_t q_desc = make_desc(qa + kd * 32, 16, 1024), k_desc = make_desc(ka + kd * 32, 16, 1024);
+          if (pass == 2 && kd == 0) umma_onto<kTailBits>(on, tmem_base + (uint32_t)s * 128, q_desc, k_desc, p.idesc_qk);
+          else umma_if(on, tmem_base + (uint32_t)s * 128, q_desc, k_desc, p.idesc_qk, (pass | kd) != 0 ? 1u : 0u, true);
+        }
       }
       if (on) {
         umma_commit(sfull0 + 8 * s);
@@ -205,9 +208,11 @@ attention_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         for (int pass = 0; pass < 3; ++pass) {
           const uint32_t pa = tmem_base + (uint32_t)(s * 128 + g * 64 + (pass == 0 ? 32 : 0)), va = vb + (pass == 1 ? kPairsPlane : 0);
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ts_if(on, o_addr, pa + (uint32_t)(kk * 8), make_desc(va + (uint32_t)(g * 4 + kk) * 2048, kPairsPlane, 1024, 2), p.idesc_pv,
-                       (pass | kk) != 0 ? 1u : 0u, true);
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint64_t v_desc = make_desc(va + (uint32_t)(g * 4 + kk) * 2048, kPairsPlane, 1024, 2);
+            if (pass == 2 && kk == 0) umma_ts_onto<kTailBits>(on, o_addr, pa, v_desc, p.idesc_pv);
+            else umma_ts_if(on, o_addr, pa + (uint32_t)(kk * 8), v_desc, p.idesc_pv, (pass | kk) != 0 ? 1u : 0u, true);
+          }
         }
       }
       if (on) {

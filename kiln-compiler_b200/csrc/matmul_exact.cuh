@@ -8,7 +8,8 @@
 // Why the sums leave tensor memory after every 64 of K: the tensor core cuts off a bit of the accumulator with every MMA, ~4.5e-8 of it for 8 of K on
 // the average, an error that adds up along the sign of what is in it (positive operands, 768 of K in one accumulator
 // 4.2e-6, in two 2.3e-6).  The epilogue's warps, idle during a main loop, add every step's products up in registers, rounded as
-// float32 sums are; the next steps go to other columns meanwhile.  The step's small products come first, while its accumulator is small.
+// float32 sums are; the next steps go to other columns meanwhile.  The step's small products come first, while its accumulator is small; the first
+// large one brings it down by 2^11, the power of two of the tails.
 //
 // Tiles are 256 x BN on the two SMs of a cluster (`.cta_group::2`), as in matmul_pair.cu, whose notes on pairs, producers and the leader's
 // barriers hold here too; persistent, one CTA per SM, 384 threads:
@@ -28,6 +29,7 @@
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
+#include "split16.cuh"
 #include "tc_common.cuh"
 #include "tc_epilogue.cuh"
 #include "tc_pair.cuh"
@@ -252,7 +254,10 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             umma_pair<true>(on, d, desc(a + k), desc(bt + k), idesc, 1u);
           }
 #pragma unroll
-          for (int k = 0; k < 8; k += 2) umma_pair<true>(on, d, desc(a + k), desc(b + k), idesc, 1u);
+          for (int k = 0; k < 8; k += 2) {
+            if (k == 0) umma_pair_onto<kTailBits>(on, d, desc(a), desc(b), idesc);
+            else umma_pair<true>(on, d, desc(a + k), desc(b + k), idesc, 1u);
+          }
           if (on) {
             umma_pair_commit(empty0 + 8 * s, pair_ctas);
             umma_pair_commit(ready0 + 8 * sum, pair_ctas);

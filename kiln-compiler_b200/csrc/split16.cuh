@@ -25,13 +25,18 @@ struct RowScale {
 
 __device__ __forceinline__ uint32_t warp_umax(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 
+// Tails are kept times 2^11, as large as their heads, so that they are normal numbers as long as those are.  Products of a head and a tail
+// then are too, and are summed first; the accumulator is brought down by 2^11 with the first product of two heads (see umma_pair_onto).
+constexpr int kTailBits = 11;
+constexpr float kTailUp = 1 << kTailBits;
+
 __device__ __forceinline__ void store_terms(__half* heads, __half* tails, const float4& x, float scale) {
   const float v[4] = {x.x * scale, x.y * scale, x.z * scale, x.w * scale};
   __half h[4], t[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     h[e] = __float2half_rn(v[e]);
-    t[e] = __float2half_rn(v[e] - __half2float(h[e]));
+    t[e] = __float2half_rn((v[e] - __half2float(h[e])) * kTailUp);
   }
   *reinterpret_cast<uint2*>(heads) = *reinterpret_cast<const uint2*>(h);
   *reinterpret_cast<uint2*>(tails) = *reinterpret_cast<const uint2*>(t);

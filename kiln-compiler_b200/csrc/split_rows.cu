@@ -1,13 +1,12 @@
-// Float32 operands of an exact matmul as two float16 terms: x 2^e = h + t, h the nearest float16 and t the nearest to what is left, with
-// one power of two per row that puts the row's largest element at 2^14 to 2^15.  Role of the operand precision of the reference's
+// Float32 operands of an exact matmul as two float16 terms: x 2^e = h + 2^-11 t, h the nearest float16 and t the nearest to what is left times
+// 2^11, with one power of two per row that puts the row's largest element at 2^14 to 2^15.  Role of the operand precision of the reference's
 // `tl.dot(..., input_precision="ieee")` (kiln/gpu/codegen.py:515).
 //
-// How much of x they hold: all but 2^-24 |x| where x 2^e is 1/2 and more, and 2^-25 2^-e = 2^-40 to 2^-39 of the row's largest element where
-// it is less (t is subnormal there).  Two TF32 terms, which have float32's exponents, hold all but 2^-22 to 2^-24 of every x.  So a product of
-// a small element and a large one of the other operand is as good as before only while the other operand does not make up for the
-// row's spread: a weight whose columns' largest elements along K, max over n of |b[k, n]|, are within 2^10 of each other leaves an
-// error of at most K 2^-29 of what the row's largest element adds to some result of the row (768: 1.4e-6 if all had one
-// sign and the worst size; 1e-8 in the mean), and other weights keep the other kernels (`split_suits`).
+// How much of x they hold: all but 2^-22 |x| (2^-24 in the mean) as long as h is a normal number, down to 2^-28 of the row's largest element, and
+// 2^-36 2^-e = 2^-51 to 2^-50 of that where x is less.  (With tails as they are, t is subnormal from 2^-15 of the largest element on and held 2^-40 of
+// it: of results that use none of the features 2^24 times the others, 1.8e-5.)  Two TF32 terms, which have float32's exponents, hold all but
+// 2^-22 to 2^-24 of every x; weights whose columns' largest elements along K, max over n of |b[k, n]|, are more than 2^10 apart keep
+// the kernels that multiply those (`split_suits`).
 //
 // What bounds the pass: it is a launch of ~2.3 us in front of a matmul; 4 bytes read and 4 written per element.
 #include <math.h>

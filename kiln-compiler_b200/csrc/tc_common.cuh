@@ -238,6 +238,23 @@ __device__ __forceinline__ void umma_ts_if(uint32_t on, uint32_t tmem_d, uint32_
         : "memory");
   }
 }
+// 16-bit operands: D = A B + D 2^-DOWN, A from shared and from tensor memory.
+template <int DOWN>
+__device__ __forceinline__ void umma_onto(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.eq.b32 p, 0, 0;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %5;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(on), "n"(DOWN)
+      : "memory");
+}
+template <int DOWN>
+__device__ __forceinline__ void umma_ts_onto(uint32_t on, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.eq.b32 p, 0, 0;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %5;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(on), "n"(DOWN)
+      : "memory");
+}
 
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
   asm volatile(

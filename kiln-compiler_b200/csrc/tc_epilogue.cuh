@@ -7,6 +7,7 @@
 
 #include "device_math.cuh"
 #include "kb200_internal.h"
+#include "split16.cuh"
 #include "tc_common.cuh"
 
 namespace kb200 {
@@ -223,7 +224,8 @@ __device__ __forceinline__ void stage_pairs(uint8_t* block, const float (&v)[32]
       const float2 x = fmul2(make_float2(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]), make_float2(scale, scale));
       const __half2 head = __floats2half2_rn(x.x, x.y);
       const float2 back = __half22float2(head);
-      const __half2 tail = __floats2half2_rn(x.x - back.x, x.y - back.y);
+      const float2 rest = ffma2(back, make_float2(-kTailUp, -kTailUp), fmul2(x, make_float2(kTailUp, kTailUp)));
+      const __half2 tail = __floats2half2_rn(rest.x, rest.y);
       h[i] = *reinterpret_cast<const uint32_t*>(&head);
       t[i] = *reinterpret_cast<const uint32_t*>(&tail);
     }

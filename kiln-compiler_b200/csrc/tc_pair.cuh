@@ -37,6 +37,15 @@ __device__ __forceinline__ void umma_pair(uint32_t on, uint32_t tmem_d, uint64_t
         : "memory");
   }
 }
+// 16-bit operands: D = A B + D 2^-DOWN.
+template <int DOWN>
+__device__ __forceinline__ void umma_pair_onto(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.eq.b32 p, 0, 0;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %5;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(on), "n"(DOWN)
+      : "memory");
+}
 // Arrives, when every MMA issued so far by this thread has completed, on the mbarrier at this offset
 // in BOTH CTAs of the pair (a commit, not a copy: the arrival is what is sent to the two CTAs).  One
 // instruction: a commit costs the issuing thread about as much as two MMAs.
