@@ -1598,7 +1598,7 @@ int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_
 bool attention_takes_pairs(const PlanKernel& k, PlanKernel::Planes* planes, const float** scale) {
   const AttnState* st = static_cast<const AttnState*>(k.attn);
   if (!st || !st->pairs.used || st->own_pass) return false;
-  *planes = PlanKernel::Planes{st->pairs.planes, st->pairs.rows * st->pairs.pitch, st->pairs.pitch, nullptr};
+  *planes = PlanKernel::Planes{st->pairs.planes, st->pairs.rows * st->pairs.pitch, st->pairs.pitch, nullptr, nullptr};
   *scale = st->pairs.by();
   return true;
 }

@@ -105,6 +105,7 @@ struct PlanKernel {
     void* heads = nullptr;
     int64_t plane = 0, pitch = 0;
     float* scales = nullptr;
+    uint8_t* marks = nullptr;     // which rows go into more planes (see split16.cuh)
   } planes_out;
   // FP32: bounds of a matmul's results by column (see result_bounds), once they have been looked for, and whether its producer will split its rows
   std::vector<float> bounds;

@@ -151,6 +151,7 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   p.N = (int)k.N;
   p.a_scale = ops.a_scale;
   p.b_scale = ops.b_scale;
+  p.a_marks = ops.a_marks;
   p.bias = st->bias_slot >= 0 ? k.ops[st->bias_slot].ptr : nullptr;
   p.res = st->res_slot >= 0 ? k.ops[st->res_slot].ptr : nullptr;
   p.res_row = st->res_slot >= 0 ? k.ops[st->res_slot].stride[1] : 0;
@@ -169,7 +170,7 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   const int pairs = plan.sm_count / 2, share = plan.concurrency > 1 && pairs / plan.concurrency > 0 ? pairs / plan.concurrency : pairs;
   const int rounds = (p.num_tiles + share - 1) / share;
   st->grid = (unsigned)(st->parts > 1 ? 2 * st->parts * p.num_tiles : 2 * ((p.num_tiles + rounds - 1) / rounds));
-  bool ok = encode_map(&st->map_a, true, ops.a, k.K, k.M, 2, ops.pitch, k.M * ops.pitch, kExactStepK, 128, false, 2) &&
+  bool ok = encode_map(&st->map_a, true, ops.a, k.K, k.M, 2 * kLevels, ops.pitch, k.M * ops.pitch, kExactStepK, 128, false, 2) &&
             encode_map(&st->map_b, true, ops.b, k.K, k.N, 2, ops.pitch, k.N * ops.pitch, kExactStepK, p.half_bn, false, 2) &&
             encode_map_store(&st->map_out, false, O.ptr, k.N, k.M, 1, O.stride[1], 0);
   st->map_res = st->map_tail = st->map_out;

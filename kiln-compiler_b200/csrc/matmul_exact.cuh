@@ -22,6 +22,12 @@
 // Few tiles and a long K (SPLIT): a cluster of two to four pairs, each with its part of K for the same tile of 128 columns.  A pair finishes
 // some of the tile's 32-column blocks: the sums of the others' are sent into their rings, idle by then, as bulk copies, and added up in the
 // order of the pairs.
+//
+// Rows of A whose elements are more than 2^28 apart come in further levels (split16.cuh): their tiles go over K once more per level, with the planes of
+// that level and the same ones of B, and the sums of its steps are multiplied by the level's power of two as they are added up, by 0 for rows
+// that have none.  Why not per row: a tile multiplies 256 of them anyway.  1024 x 2304 x 768 15.5 us (with the pass), one such row 20.0, all 23.7, all with
+// two levels 30.5; 4096^3 331, 365, 643, 984.  Of normally distributed rows about one in 10^5 has such an element by chance.  (Where no row has
+// one, asking costs a launch behind another ~0.2 us: 1024 x 768 block 75.6 -> 77.8.)
 // Every wait is bounded: see matmul_pair.cu.
 #pragma once
 
@@ -71,6 +77,7 @@ struct ExactParams {
   int M, N;
   const float* a_scale;  // what a row's products are to be multiplied by; below zero: the row holds infinities (see redo_row)
   const float* b_scale;
+  const uint8_t* a_marks;      // by row, zero up to the last tile's end: the levels behind the first that it has
   const float* bias;
   const float* res;      // as the map of it, for redo_row
   int64_t res_row;
@@ -118,6 +125,21 @@ __device__ __forceinline__ void add_staged(float (&v)[32], const uint8_t* block,
 __device__ __forceinline__ int first_block_of(int part, int parts) { return parts == 2 ? 2 * part : parts == 3 && part > 0 ? part + 1 : part; }
 __device__ __forceinline__ int owner_of(int block, int parts) { return parts == 2 ? block >> 1 : parts == 3 && block > 0 ? block - 1 : block; }
 __device__ __forceinline__ int received_at(int block, int from, int parts) { return (block * (parts - 1) + from) * 4; }
+
+// The marks of a tile's 256 rows, a lane's eight of them, and the levels behind the first that a tile with these has.  (Both volatile: asked for in
+// front of the tile's steps and looked at behind them, not ~700 cycles of L2 in front of the first.)
+__device__ __forceinline__ uint2 tile_marks(const ExactParams& p, int tm, int lane) {
+  uint2 marks;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(marks.x), "=r"(marks.y) : "l"(p.a_marks + (int64_t)tm * 256 + lane * 8) : "memory");
+  return marks;
+}
+__device__ __forceinline__ int levels_behind(uint2 marks) {
+  uint32_t any;
+  asm volatile("or.b32 %0, %1, %2;" : "=r"(any) : "r"(marks.x), "r"(marks.y));
+  any |= any >> 16;
+  any |= any >> 8;
+  return __popc(__reduce_or_sync(0xffffffffu, any & 3u));
+}
 
 // BLOCKS: 32-column blocks of a tile per warp, at most.
 template <int BLOCKS, int FIN, bool SPLIT>
@@ -209,26 +231,29 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       for (int tile = pair; tile < p.num_tiles && ok; tile += num_pairs) {
         const int tm = pair_div(tile, p.magic_tn), tn = tile - tm * p.tiles_n;
         const int m = tm * 256 + (int)rank * 128, n = tn * p.bn + (int)rank * p.half_bn;
-        int k = step0 * kExactStepK;
-        for (int i = 0; i < n_steps; ++i, k += kExactStepK) {
-          ok = all_waited(mbar_wait_long(empty0 + 8 * s, parity, abort_ptr), 1);
-          if (!ok) break;
-          const bool b_here = ahead > 0;           // expected and requested above
-          const uint32_t bar = full_leader0 + 8 * s, dst = ring + (uint32_t)(s * stage_bytes);
-          if (elect_one()) {
-            // the leader's barrier counts the bytes of both CTAs
-            if (!b_here && rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
-            tma_load_3d_pair(dst, &tma_a, bar, k, m, 0);
-            if (!b_here) tma_load_3d_pair(dst + 2 * kExactABytes, &tma_b, bar, k, n, 0);
+        const uint2 marks = tile_marks(p, tm, lane);
+        for (int level = 0, more = 0; level <= more && ok; ++level) {
+          int k = step0 * kExactStepK;
+          for (int i = 0; i < n_steps; ++i, k += kExactStepK) {
+            ok = all_waited(mbar_wait_long(empty0 + 8 * s, parity, abort_ptr), 1);
+            if (!ok) break;
+            const bool b_here = ahead > 0;           // expected and requested above
+            const uint32_t bar = full_leader0 + 8 * s, dst = ring + (uint32_t)(s * stage_bytes);
+            if (elect_one()) {
+              // the leader's barrier counts the bytes of both CTAs
+              if (!b_here && rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * (uint32_t)stage_bytes);
+              tma_load_3d_pair(dst, &tma_a, bar, k, m, 2 * level);
+              if (!b_here) tma_load_3d_pair(dst + 2 * kExactABytes, &tma_b, bar, k, n, 0);
+            }
+            __syncwarp();
+            if (b_here) --ahead;
+            if (++s == p.stages) { s = 0; parity ^= 1; }
           }
-          __syncwarp();
-          if (b_here) --ahead;
-          if (++s == p.stages) { s = 0; parity ^= 1; }
+          if (level == 0) more = levels_behind(marks);
         }
       }
     } else if (warp == 1) {
       // ---------------- MMA issuer (leader CTA) ----------------
-      // (A step asks nothing of the tile it belongs to.)
       if (rank == 0) {
         const int stages = p.stages, sums = p.sums, bn = p.bn;
         const uint32_t idesc = p.idesc;
@@ -238,10 +263,12 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         const uint32_t first16 = (ring >> 4) & 0x3FFFu, stage16 = (uint32_t)stage_bytes >> 4, plane16 = (uint32_t)b_plane >> 4;
         const uint32_t fixed_lo = (uint32_t)fixed, fixed_hi = (uint32_t)(fixed >> 32);
         auto desc = [&](uint32_t at) { return ((uint64_t)fixed_hi << 32) | (fixed_lo + at); };
-        const int total = (p.num_tiles - pair + num_pairs - 1) / num_pairs * n_steps;
         int s = 0, sum = 0;
         uint32_t parity = 0, added_parity = 1;
-        for (int g = 0; g < total; ++g) {
+        // (One loop over all steps: a level's or a tile's end is looked at behind its last one, off the path of the others.)
+        int tile = pair, left = n_steps, level = 0, more = 0;
+        uint2 marks = tile < p.num_tiles ? tile_marks(p, pair_div(tile, p.magic_tn), lane) : make_uint2(0, 0);
+        while (tile < p.num_tiles) {
           // both CTAs' warps have added up what was here
           if (!all_waited(mbar_wait(added0 + 8 * sum, added_parity, abort_ptr), 4) || !all_waited(mbar_wait(full0 + 8 * s, parity, abort_ptr), 2)) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -265,6 +292,15 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
           __syncwarp();
           if (++s == stages) { s = 0; parity ^= 1; }
           if (++sum == sums) { sum = 0; added_parity ^= 1; }
+          if (--left == 0) {
+            left = n_steps;
+            if (level == 0) more = levels_behind(marks);
+            if (level++ == more) {
+              level = 0;
+              tile += num_pairs;
+              if (tile < p.num_tiles) marks = tile_marks(p, pair_div(tile, p.magic_tn), lane);
+            }
+          }
         }
       }
     }
@@ -290,6 +326,7 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
       const int m_first = tm * 256 + (int)rank * 128 + quad * 32, n0 = tn * p.bn;
       const bool rows_ok = m_first < p.M;
       const float row_scale = m_first + lane < p.M ? p.a_scale[m_first + lane] : 1.0f;
+      const uint2 marks = tile_marks(p, tm, lane);
       // scales and biases of this warp's columns, a lane's of each block, before the sums are ready
       float scale_of[BLOCKS], bias_of[BLOCKS];
 #pragma unroll
@@ -316,31 +353,42 @@ mm_exact_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #pragma unroll
         for (int q = 0; q < 32; ++q) sums[j][q] = 0.0f;
       // The first pass over what finishes a tile is a rehearsal, as in matmul_pair.cu: its code is cold at every launch.
-      for (int i = 0; i < n_steps && !dry; ++i) {
-        if (!mbar_wait_long(ready0 + 8 * sum, ready_parity, abort_ptr)) give_up(3);
-        ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t at = tmem + lanes + (uint32_t)(sum * p.bn + 32 * half);
-#pragma unroll
-        for (int j = 0; j < BLOCKS; j += kAtOnce) {
-          if (half + 2 * j >= blocks) break;
-          float w[kAtOnce][32];
-          if (kAtOnce == 2 && j + 1 < BLOCKS && half + 2 * j + 2 < blocks) tmem_ld32x2(at + (uint32_t)(64 * j), at + (uint32_t)(64 * j + 64), w[0], w[kAtOnce - 1]);
-          else tmem_ld32(at + (uint32_t)(64 * j), w[0]);
-#pragma unroll
-          for (int i = 0; i < kAtOnce && j + i < BLOCKS; ++i)
-#pragma unroll
-            for (int q = 0; q < 32; q += 2) {
-              const float2 t = fadd2(make_float2(sums[j + i][q], sums[j + i][q + 1]), make_float2(w[i][q], w[i][q + 1]));
-              sums[j + i][q] = t.x;
-              sums[j + i][q + 1] = t.y;
-            }
+      float2 down = make_float2(1.0f, 1.0f);
+      for (int level = 0, more = 0; level <= more && ok; ++level) {
+        if (level > 0) {       // (rows that have no such level: whatever finite numbers its planes hold)
+          const bool taken = (p.a_marks[m_first + lane] >> (level - 1) & 1u) != 0;
+          down.x = down.y = !taken ? 0.0f : level == 1 ? 1.0f / kLevelUp : 1.0f / kLevelUp / kLevelUp;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(added_leader0 + 8 * sum);
-        if (++sum == p.sums) { sum = 0; ready_parity ^= 1; }
+        for (int i = 0; i < n_steps && !dry; ++i) {
+          if (!mbar_wait_long(ready0 + 8 * sum, ready_parity, abort_ptr)) give_up(3);
+          ok = __shfl_sync(0xffffffffu, *abort_ptr ? 0 : 1, 0) != 0;
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t at = tmem + lanes + (uint32_t)(sum * p.bn + 32 * half);
+#pragma unroll
+          for (int j = 0; j < BLOCKS; j += kAtOnce) {
+            if (half + 2 * j >= blocks) break;
+            float w[kAtOnce][32];
+            if (kAtOnce == 2 && j + 1 < BLOCKS && half + 2 * j + 2 < blocks) tmem_ld32x2(at + (uint32_t)(64 * j), at + (uint32_t)(64 * j + 64), w[0], w[kAtOnce - 1]);
+            else tmem_ld32(at + (uint32_t)(64 * j), w[0]);
+#pragma unroll
+            for (int i = 0; i < kAtOnce && j + i < BLOCKS; ++i)
+#pragma unroll
+              for (int q = 0; q < 32; q += 2) {
+                const float2 t = ffma2(make_float2(w[i][q], w[i][q + 1]), down, make_float2(sums[j + i][q], sums[j + i][q + 1]));
+                sums[j + i][q] = t.x;
+                sums[j + i][q + 1] = t.y;
+              }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(added_leader0 + 8 * sum);
+          if (++sum == p.sums) { sum = 0; ready_parity ^= 1; }
+        }
+        if (ok && level == 0) {
+          more = levels_behind(marks);
+          if (dry) break;
+        }
       }
       if (!ok) break;
       auto pick = [&](float (&v)[32], int j) {

@@ -7,11 +7,12 @@
 namespace kb200 {
 
 struct ExactOperands {
-  const void* a;             // [2, M, pitch] float16, the plane of heads and that of tails
+  const void* a;             // [kLevels][2, M, pitch] float16, the plane of heads and that of tails of every level (see split16.cuh)
   const void* b;             // [2, N, pitch], rows along K
   int64_t pitch;
   const float* a_scale;      // [M] and [N]: what products of the terms are to be multiplied by
   const float* b_scale;
+  const uint8_t* a_marks;    // [M rounded up to whole tiles]: the levels of A's rows
 };
 
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
@@ -26,12 +27,13 @@ bool exact_writes_tails(const void* state);
 bool exact_write_pairs(const PlanKernel& k, void* state, const PlanKernel::Planes& to, const float* scale, bool store32);
 void exact_destroy(void* state);
 
-// float32 rows of `cols` elements -> the two planes and the scales.  A pass in front of a launch, or once for a weight.
-int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, int64_t rows, int64_t cols, bool pdl, cudaStream_t s);
+// float32 rows of `cols` elements -> the two planes and the scales; with `marks` of every level.  A pass in front of a launch, or once for a weight.
+int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, uint8_t* marks, int64_t rows, int64_t cols, bool pdl, cudaStream_t s);
 // |LayerNorm(x) B + bias| per column of B [K, N] for any x, at most: of the normalised row, 1 / sqrt(inv_n) long, by Cauchy and Schwarz.  `bounds`: [n]
-// on the host.  Synchronises.
+// on the host; empty where a column's result for a row of nearly equal elements (whose LayerNorm is next to beta) is below 2^-30 of its bound, so
+// that float16 pairs under the bound's power of two might not hold it: no biases at all, as a rule.  Synchronises.
 int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds);
-// Do float16 pairs hold this weight [K, N] as well as TF32 pairs would, whatever A is?  `scratch`: k words on the device.  Synchronises.
+// Do float16 pairs hold this weight [K, N] as well as TF32 pairs would?  `scratch`: k + 1 words on the device.  Synchronises.
 int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, uint32_t* scratch, bool* suits);
 
 }  // namespace kb200

@@ -37,6 +37,7 @@
 #include "matmul_exact.h"
 #include "matmul_pair.h"
 #include "matmul_small.h"
+#include "split16.cuh"
 #include "tc_common.cuh"
 #include "tc_epilogue.cuh"
 
@@ -977,6 +978,7 @@ struct TcState {
     void* a = nullptr;
     void* b = nullptr;
     float* scales = nullptr;                  // of B's columns (read in float4), then of A's rows
+    uint8_t* marks = nullptr;                 // the levels of A's rows, zero behind them
     int64_t pitch = 0;
     bool ready = false;                       // A's producer writes its planes
   } pairs16;
@@ -1061,12 +1063,13 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
   const kb200_kernel_desc& d = k.desc;
   const DevOperand& B = k.ops[d.b_slot];
   const int64_t pitch = (k.K + 63) / 64 * 64;              // rows on 128-byte lines
-  const uint64_t a_bytes = (uint64_t)k.M * pitch * 4;
+  const uint64_t a_bytes = (uint64_t)k.M * pitch * 4 * kLevels;
   if (a_bytes > plan.copy_budget) return KB200_OK;
+  const size_t scale_bytes = (size_t)(k.M + k.N + 3) / 4 * 4 * sizeof(float), mark_bytes = (size_t)(k.M + 255) / 256 * 256;
   TcState::Pairs16& h = st->pairs16;
   const size_t turned_floats = turn ? (size_t)k.N * k.K : 0;
-  float* turned = nullptr;                                 // for the time of binding: the weight as rows along K, and K numbers of split_suits
-  cudaError_t e = cudaMalloc(&turned, (turned_floats + k.K) * sizeof(float));
+  float* turned = nullptr;                                 // for the time of binding: the weight as rows along K, and K + 1 numbers of split_suits
+  cudaError_t e = cudaMalloc(&turned, (turned_floats + k.K + 1) * sizeof(float));
   bool suits = false;
   if (e == cudaSuccess) {
     const int rc = split_suits(B.ptr, B.stride[1], B.stride[2], k.K, k.N, reinterpret_cast<uint32_t*>(turned + turned_floats), &suits);
@@ -1074,11 +1077,14 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
       cudaFree(turned);
       return rc;
     }
-    e = cudaMalloc(&h.a, a_bytes + (size_t)k.N * pitch * 4 + (size_t)(k.M + k.N) * sizeof(float));
+    e = cudaMalloc(&h.a, a_bytes + (size_t)k.N * pitch * 4 + scale_bytes + mark_bytes);
   }
   if (e == cudaSuccess) {
     h.b = static_cast<uint8_t*>(h.a) + a_bytes;            // (rows of 128 bytes: both stay aligned)
     h.scales = reinterpret_cast<float*>(static_cast<uint8_t*>(h.b) + (size_t)k.N * pitch * 4);
+    h.marks = reinterpret_cast<uint8_t*>(h.scales) + scale_bytes;
+    e = cudaMemsetAsync(h.marks, 0, mark_bytes, nullptr);
+    if (e == cudaSuccess) e = cudaMemsetAsync(static_cast<uint8_t*>(h.a) + a_bytes / kLevels, 0, a_bytes / kLevels * (kLevels - 1), nullptr);       // (multiplied, times 0)
   }
   if (e == cudaSuccess && turn)
     e = launch_kernel(false, transpose_rows_kernel<float>, dim3((unsigned)((k.K + 31) / 32), (unsigned)((k.N + 31) / 32)), dim3(256), 0, nullptr,
@@ -1086,7 +1092,7 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
   h.pitch = pitch;
   int status = KB200_OK;
   if (e == cudaSuccess) {
-    status = split_rows(turn ? turned : B.ptr, turn ? k.K : b_row, h.b, pitch, h.scales, k.N, k.K, false, nullptr);
+    status = split_rows(turn ? turned : B.ptr, turn ? k.K : b_row, h.b, pitch, h.scales, nullptr, k.N, k.K, false, nullptr);
     e = cudaDeviceSynchronize();
   }
   if (turned) cudaFree(turned);
@@ -1097,7 +1103,7 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
   }
   if (status) return status;
   KB200_CUDA(e);
-  status = exact_bind(plan, k, kernel_index, ExactOperands{h.a, h.b, pitch, h.scales + k.N, h.scales}, &st->exact);
+  status = exact_bind(plan, k, kernel_index, ExactOperands{h.a, h.b, pitch, h.scales + k.N, h.scales, h.marks}, &st->exact);
   if (status || !st->exact) drop_pairs16(st);
   else plan.copy_budget -= a_bytes;
   return status;
@@ -1510,7 +1516,7 @@ int tc_launch(const Plan& plan, const PlanKernel& k, cudaStream_t s) {
                              (uint32_t)k.K, row, st->tail_pitch, (float*)nullptr));
   }
   if (st->exact) {
-    const int rc = st->pairs16.ready ? KB200_OK : split_rows(k.ops[d.a_slot].ptr, k.ops[d.a_slot].stride[1], st->pairs16.a, st->pairs16.pitch, st->pairs16.scales + k.N, k.M, k.K, plan.pdl, s);
+    const int rc = st->pairs16.ready ? KB200_OK : split_rows(k.ops[d.a_slot].ptr, k.ops[d.a_slot].stride[1], st->pairs16.a, st->pairs16.pitch, st->pairs16.scales + k.N, st->pairs16.marks, k.M, k.K, plan.pdl, s);
     return rc ? rc : exact_launch(plan, st->exact, s);
   }
   if (st->small) return small_launch(plan, st->small, s);
@@ -1579,7 +1585,7 @@ bool tc_writes_tails(const PlanKernel& k) {
 bool tc_takes_planes(const PlanKernel& k, PlanKernel::Planes* planes) {
   const TcState* st = static_cast<const TcState*>(k.tc);
   if (!st || !st->exact) return false;
-  *planes = PlanKernel::Planes{st->pairs16.a, k.M * st->pairs16.pitch, st->pairs16.pitch, st->pairs16.scales + k.N};
+  *planes = PlanKernel::Planes{st->pairs16.a, k.M * st->pairs16.pitch, st->pairs16.pitch, st->pairs16.scales + k.N, st->pairs16.marks};
   return true;
 }
 

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
   const int units = SHIFT ? (p.inner + 6) >> 2 : VEC == 1 ? p.inner : p.inner >> 2;
   static_assert(!PLANES || (VEC == 4 && MODE == ROW_LAYERNORM), "pairs are made of float4");
   __shared__ float partial[WIDE ? 64 : 1];
-  [[maybe_unused]] __shared__ uint32_t partial_most[WIDE && PLANES ? 32 : 1];
+  [[maybe_unused]] __shared__ uint32_t partial_most[WIDE && PLANES ? 32 : 1], partial_least[WIDE && PLANES ? 32 : 1];
   // Each reduction of a WIDE row has its own half of `partial`: no barrier between the reads of one and the writes of the next.
   auto across = [&](float v, bool is_max, int which) {
     v = is_max ? warp_max(v) : warp_sum(v);
@@ -341,27 +341,39 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256) row_kernel(const __grid_cons
       }
     }
     if constexpr (PLANES) {
-      uint32_t most = 0;
+      uint32_t most = 0, least = ~0u;
 #pragma unroll
       for (int i = 0; i < N; ++i)
         if (live[i])
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) most = max(most, magnitude_bits(v[i][e]));
+          for (int e = 0; e < VEC; ++e) {
+            most = max(most, magnitude_bits(v[i][e]));
+            least = min(least, magnitude_bits(v[i][e]) - 1u);
+          }
       most = warp_umax(most);
+      least = warp_umin(least);
       if constexpr (WIDE) {
         const int l = threadIdx.x & 31;
-        if (l == 0) partial_most[threadIdx.x >> 5] = most;
+        if (l == 0) {
+          partial_most[threadIdx.x >> 5] = most;
+          partial_least[threadIdx.x >> 5] = least;
+        }
         __syncthreads();
         most = warp_umax(l < (lanes >> 5) ? partial_most[l] : 0u);
+        least = warp_umin(l < (lanes >> 5) ? partial_least[l] : ~0u);
       }
       const RowScale scale(most);
-      if (lane == 0) p.planes.scales[row] = scale.back;
+      const uint32_t marks = row_marks(most, least);
+      if (lane == 0) {
+        p.planes.scales[row] = scale.back;
+        p.planes.marks[row] = (uint8_t)marks;
+      }
       __half* const heads = static_cast<__half*>(p.planes.heads) + row * p.planes.pitch;
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         if (!live[i]) continue;
         const int j = lane + lanes * i;
-        store_terms(heads + 4 * j, heads + p.planes.plane + 4 * j, make_float4(v[i][0], v[i][1], v[i][2], v[i][3]), scale.by);
+        store_levels(heads + 4 * j, p.planes.plane, make_float4(v[i][0], v[i][1], v[i][2], v[i][3]), scale.by, marks);
         if (p.store32 || scale.marked) row_store<VEC>(out + VEC * j, v[i]);
       }
     }
