@@ -72,7 +72,8 @@ typedef enum kb200_kclass {
  * FP32 corresponds to input_precision="ieee", TF32 to "tf32"
  * (codegen.py:515-516); BF16 is a backend-internal mode with no IR dtype.
  * FP32 on the tensor cores is three products of split operands -- pairs of float16 under a power of two per row where
- * the weight is frozen and suits, else pairs of TF32: within 1e-5 of exact for finite operands, but in the single-CTA
+ * the weight is frozen and suits, else pairs of TF32: within 1e-5 of exact for finite operands (the 2-norm of a row or column of results;
+ * float16 pairs hold elements below 2^-84 of their row's largest to 2^-107 of that), but in the single-CTA
  * kernel on TF32 pairs NOT IEEE for non-finite ones (an infinite operand element yields NaN, see cfg[6] bit 1024 below
  * for the CUDA-core kernel that is; the others sum such rows over in float32). */
 typedef enum kb200_precision {
@@ -219,12 +220,13 @@ int kb200_plan_bind(kb200_plan* plan, void* arena, uint64_t arena_bytes,
  * the kernel on pairs of float16, three products per float32 product, for any length above 128 tokens where it is estimated faster than the
  * CUDA-core kernel; else the kernel with three TF32 products, for sequences of whole tiles of 128 tokens whose work items fill a
  * quarter of the SMs; else, and where a matmul of the chain asked for IEEE behaviour on non-finite operands, the CUDA-core kernel.
- * 1 = always the CUDA-core kernel, 2 = always the tensor cores on TF32, with the tails from a launch of its own (the same bits).
+ * 1 = always the CUDA-core kernel; 2 = always the tensor cores, on pairs of float16 where the bounds are known and else on TF32, with the pairs or
+ * tails from a launch of its own (the same bits); 3 = always the tensor cores on TF32, likewise.
  * KB200_OPT_ATTENTION_SPLIT (default 1): in a launch that leaves SMs idle (one long sequence,
  * KB200_OPT_CONCURRENCY 1) the fused attention shares its long query tiles between two CTAs, which
  * merge their halves through a workspace.  0 keeps every query tile on one CTA.
  * KB200_OPT_WEIGHT_COPIES (default 1, FP32 and TF32 precision): frozen weights are also kept laid out along K
- * and, for FP32, with their tails, or as pairs of float16 beside a buffer for A's (twice the weight's own bytes in FP32, or once and A's bytes;
+ * and, for FP32, with their tails, or as pairs of float16 beside a buffer for A's (twice the weight's own bytes in FP32, or once and three times A's bytes;
  * once in TF32), as far as a quarter of the free memory goes.  0 = every weight is read where it is, as it is beyond that.
  * KB200_OPT_FEW_TILES (default 0): asks the matmul kernel for few tiles for one of its forms instead of the one it
  * estimates to be quickest, where it covers a matmul: tile columns (64, 96 or 128) + 1000 * K splits (1, 2, 4 or 8)
@@ -267,7 +269,8 @@ int kb200_plan_relocatable(const kb200_plan* plan);
 int kb200_plan_run(kb200_plan* plan, void* const* inputs, int n_inputs, void* const* outputs, int n_outputs,
                    void* cuda_stream);
 
-/* Enqueues kernel `i` alone (profiling, autotuning). */
+/* Enqueues kernel `i` alone (profiling, autotuning).  What producers leave for it beside the arena -- bf16 mirrors, tails or float16
+ * pairs of its operands -- is then as it was after their last run, whatever the arena holds. */
 int kb200_kernel_launch(kb200_plan* plan, int i, void* cuda_stream);
 
 /* Number of device kernel launches kb200_plan_launch enqueues (a Kiln kernel
@@ -278,8 +281,8 @@ int kb200_plan_launch_count(const kb200_plan* plan);
  * "row_layernorm", "mm_tcgen05", ...).  Never NULL for a valid i. */
 const char* kb200_kernel_impl(const kb200_plan* plan, int i);
 
-/* What runs a bound kernel `i`, in more words: for a tensor-core matmul the kernel ("mm_small", "mm_pair", "mm_tc"),
- * its tile, its split and the operands it copies.  Valid until the thread's next call of this function. */
+/* What runs a bound kernel `i`, in more words: for a tensor-core matmul the kernel ("mm_small", "mm_exact", "mm_pair", "mm_tc"),
+ * its tile, its split and the operands it copies; for a fused attention in FP32 which of its kernels.  Valid until the thread's next call of this function. */
 const char* kb200_kernel_detail(const kb200_plan* plan, int i);
 
 /* Number of fused scalar steps kernel `i` applies per element as bound: the epilogue chain of a

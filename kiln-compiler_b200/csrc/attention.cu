@@ -972,7 +972,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
   AttnState* st = new AttnState();
   st->exact = c.exact;
   st->ieee = c.ieee;
-  st->asked = plan.fp32_attention == 1;
+  st->asked = plan.fp32_attention == 1 || plan.fp32_attention == 3;
   // FP32 mode: the CUDA-core kernel (64 queries per CTA, long prefixes split), or the tensor-core kernel (128 queries and a pass
   // over Q, K and V for their tails) for sequences of whole tiles that fill a quarter of the SMs, where that is estimated
   // faster.  Both estimates are a line through launches of 16 to 333 tokens and 4 to 96 heads, in ns: a fixed part, key
@@ -987,7 +987,7 @@ bool finish_fusion(Plan& plan, const AttnChain& c) {
     const int64_t tc_ns = 6800 + 2400 * q_tiles * ((B * H * q_tiles + sms - 1) / sms) + B * T * 3 * H * hd * 8 / 6500;
     st->exact_tc = !c.ieee && T % kRows == 0 && B * H * q_tiles * 4 >= sms && tc_ns <= fma_ns;
     if (plan.fp32_attention == 1) st->exact_tc = false;
-    if (plan.fp32_attention == 2) st->exact_tc = st->own_pass = true;
+    if (plan.fp32_attention >= 2) st->exact_tc = st->own_pass = true;
   }
   if ((!c.exact || st->exact_tc) && (!encode_map_heads(&st->map_q, false, c.q, hd, T, H, B, rs, 32, kRows, false) ||
                                      !encode_map_heads(&st->map_k, false, c.k, hd, T, H, B, rs, 32, kRows, false) ||
@@ -1638,6 +1638,12 @@ bool attention_write_pairs(PlanKernel& k, const PlanKernel::Planes& to, bool dro
 void attention_pairs_come_ready(PlanKernel& k) {
   static_cast<AttnState*>(k.attn)->pairs.ready = true;
   --k.launches;
+}
+
+std::string attention_detail(const PlanKernel& k) {
+  const AttnState* st = static_cast<const AttnState*>(k.attn);
+  if (!st || !st->exact) return "attention_fused";
+  return st->pairs.used ? "attention_fused on float16 pairs" : st->exact_tc ? "attention_fused on TF32 pairs" : "attention_fused on the CUDA cores";
 }
 
 float* attention_tails(const PlanKernel& k) {

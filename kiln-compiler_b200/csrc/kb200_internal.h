@@ -131,7 +131,7 @@ struct Plan {
   std::vector<PlanKernel> kernels;
   int* d_status = nullptr;       // device status word for bounded waits
   bool fuse_attention = true;    // replace the five-kernel attention chain by the fused kernel when it matches
-  int fp32_attention = 0;        // FP32 precision: 0 = pick the fused attention kernel by size, 1 = CUDA cores, 2 = tensor cores
+  int fp32_attention = 0;        // FP32 precision: 0 = pick the fused attention kernel by size, 1 = CUDA cores, 2 = tensor cores, 3 = TF32 pairs on them
   bool attention_split = true;   // share long query tiles between two CTAs when a launch would leave SMs idle
   int few_tiles = 0;             // KB200_OPT_FEW_TILES: the form of the matmul kernel for few tiles that is to be used, 0 = by estimate
   mutable int resident_clusters[9] = {};   // by cluster size, as the few-tiles matmul asked for them (0: not yet)
@@ -196,6 +196,7 @@ int attention_try_fuse(Plan& plan, size_t first);    // plan kernels replaced fr
 int attention_chain_length(const PlanKernel& k);
 bool attention_wants_bf16(const PlanKernel& k);
 bool attention_reads_mirror(const PlanKernel& k);
+std::string attention_detail(const PlanKernel& k);      // with the kernel that runs it
 float* attention_tails(const PlanKernel& k);            // FP32 on the tensor cores: the tails of Q, K and V, or null
 void attention_tails_come_ready(PlanKernel& k);         // ... which the projection writes
 int attention_use_pairs(Plan& plan, PlanKernel& holder, const float* src, int64_t src_row, int64_t rows, const std::vector<float>& bounds);      // FP32 on float16 pairs

@@ -1415,7 +1415,7 @@ KB200_EXPORT int kb200_plan_set_option(kb200_plan* p, int option, int value) {
     case KB200_OPT_CONCURRENCY: plan.concurrency = value < 1 ? 1 : value; return KB200_OK;
     case KB200_OPT_ABSORB_ELEMENTWISE: plan.absorb_elementwise = value != 0; return KB200_OK;
     case KB200_OPT_MIRROR_ONLY: plan.mirror_only = value != 0; return KB200_OK;
-    case KB200_OPT_FP32_ATTENTION: plan.fp32_attention = value < 0 || value > 2 ? 0 : value; return KB200_OK;
+    case KB200_OPT_FP32_ATTENTION: plan.fp32_attention = value < 0 || value > 3 ? 0 : value; return KB200_OK;
     case KB200_OPT_ATTENTION_SPLIT: plan.attention_split = value != 0; return KB200_OK;
     case KB200_OPT_WEIGHT_COPIES: plan.weight_copies = value != 0; return KB200_OK;
     case KB200_OPT_FEW_TILES: plan.few_tiles = value < 0 ? 0 : value; return KB200_OK;
@@ -1490,7 +1490,7 @@ KB200_EXPORT const char* kb200_kernel_detail(const kb200_plan* p, int i) {
   const Plan& plan = *reinterpret_cast<const Plan*>(p);
   if (i < 0 || i >= (int)plan.kernels.size() || !plan.bound) return "";
   const PlanKernel& k = plan.kernels[i];
-  text = k.impl == IMPL_MM_TC ? matmul_detail(k) : impl_name(k.impl);
+  text = k.impl == IMPL_MM_TC ? matmul_detail(k) : k.impl == IMPL_ATTN_FUSED ? attention_detail(k) : impl_name(k.impl);
   return text.c_str();
 }
 

@@ -234,9 +234,9 @@ class GPUExecutable:
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_ABSORB_ELEMENTWISE, int(absorb)), self._lib)
         mirror_only = os.environ.get("KILN_GPU_MIRROR_ONLY", "1") not in ("0", "false", "False", "")
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_MIRROR_ONLY, int(mirror_only)), self._lib)
-        # FP32 mode's fused attention: KILN_GPU_FP32_ATTENTION=fma / tensor forces the CUDA-core or the
-        # tensor-core kernel (default: by size); KILN_GPU_ATTENTION_SPLIT=0 keeps every query tile on one CTA.
-        fp32_attention = {"fma": 1, "tensor": 2}.get(os.environ.get("KILN_GPU_FP32_ATTENTION", "").lower(), 0)
+        # FP32 mode's fused attention: KILN_GPU_FP32_ATTENTION=fma / tensor / tf32 forces the CUDA-core kernel, the
+        # tensor cores, or TF32 pairs on them (default: by size); KILN_GPU_ATTENTION_SPLIT=0 keeps every query tile on one CTA.
+        fp32_attention = {"fma": 1, "tensor": 2, "tf32": 3}.get(os.environ.get("KILN_GPU_FP32_ATTENTION", "").lower(), 0)
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_FP32_ATTENTION, fp32_attention), self._lib)
         split = os.environ.get("KILN_GPU_ATTENTION_SPLIT", "1") not in ("0", "false", "False", "")
         _cabi.check(self._lib.kb200_plan_set_option(self._plan, _cabi.OPT_ATTENTION_SPLIT, int(split)), self._lib)
