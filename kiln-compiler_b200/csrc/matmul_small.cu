@@ -74,8 +74,6 @@ struct SmallParams {
   int64_t b_k, b_n;
   int K;
   int a_rows;                      // rows of a box of A: the tile's, or M where that is less (GATHER: a quarter, in each map)
-  int a_maps;                      // GATHER
-  int a_shift[4];
   float* out;                      // null: only the bf16 copy is stored
   __nv_bfloat16* out16;            // or null
   float* out_tail;                 // exact FP32: the output minus its 19 leading bits, for a consumer that splits it, or null
@@ -104,7 +102,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
 // map's base is rounded down to 16 bytes, `shift` floats in front of its first row; boxes are four columns wider than a step and the warps
 // that move A read from `shift` on.  Row 4 i + c of a tile is accumulator row 32 c + i: a warp's 32 rows are of one map and have one shift.
 // (Rows of 36 or 68 floats in shared memory: an odd number of 16-byte units, so that a warp's loads have no bank conflicts.)
-struct GatherMaps { CUtensorMap of[4]; };
+// (`count` and `shift` are here, not in SmallParams, whose other launches would pass them along.)
+struct GatherMaps {
+  CUtensorMap of[4];
+  int count;
+  int shift[4];
+};
 template <bool GATHER> __device__ __forceinline__ int matrix_row(int row) { return GATHER ? 4 * (row & 31) + (row >> 5) : row; }
 
 // What a TF32 operand does not hold of x.
@@ -233,10 +236,12 @@ mm_small_kernel(const __grid_constant__ std::conditional_t<GATHER, GatherMaps, C
       if (i >= p.stages && !all_waited(mbar_wait(empty0 + 8 * s, parity, abort_ptr), 1)) break;
       const uint32_t bar = full0 + 8 * s, dst = ring + (uint32_t)(s * kStage), b_dst = dst + kStageA;
       if (elect_one()) {
-        mbar_expect_tx(bar, !is_a ? kBBoxes * kSmallBBytes : GATHER ? p.a_maps * p.a_rows * kGatherRow : kSlabs * (kSlabA / kSmallM) * p.a_rows);
+        uint32_t a_bytes = kSlabs * (kSlabA / kSmallM) * p.a_rows;
+        if constexpr (GATHER) a_bytes = tma_a.count * p.a_rows * kGatherRow;
+        mbar_expect_tx(bar, is_a ? a_bytes : kBBoxes * kSmallBBytes);
         if constexpr (GATHER) {
           if (is_a)
-            for (int c = 0; c < p.a_maps; ++c) tma_load_3d(dst + c * 32 * kGatherRow, &tma_a.of[c], bar, k_elem, tm * 32, 0);
+            for (int c = 0; c < tma_a.count; ++c) tma_load_3d(dst + c * 32 * kGatherRow, &tma_a.of[c], bar, k_elem, tm * 32, 0);
         }
         // (a slab past the end of K, in the last step of an odd number, is a box outside the tensor: zeros)
 #pragma unroll
@@ -383,7 +388,8 @@ mm_small_kernel(const __grid_constant__ std::conditional_t<GATHER, GatherMaps, C
       int s = ALTERNATE ? half : 0;
       uint32_t parity = 0;
       const int row = quad * 32 + lane;
-      [[maybe_unused]] const int shift = GATHER ? p.a_shift[quad] : 0;
+      [[maybe_unused]] int shift = 0;
+      if constexpr (GATHER) shift = tma_a.shift[quad];
       for (int i = s; i < n_steps && ok; i += kEvery) {
         const int buf = i % kABuffers;
         if (!mbar_wait(full0 + 8 * s, parity, abort_ptr)) give_up(7);
@@ -887,14 +893,14 @@ int small_bind(Plan& plan, PlanKernel& k, int kernel_index, const PairOperands& 
   bool ok = true;
   if (gather) {
     p.a_rows = (int)(k.M < kSmallM ? (k.M + 3) / 4 : kSmallM / 4);          // (rows that are not there cost a box as much as others)
-    p.a_maps = (int)(k.M < 4 ? k.M : 4);
-    for (int c = 0; c < p.a_maps && ok; ++c) {
-      p.a_shift[c] = gather_shift(A, c);
-      ok = encode_map_rows(&st->maps_a.of[c], A.ptr + c * A.stride[1] - p.a_shift[c], k.K + p.a_shift[c], (k.M - c + 3) / 4, 4 * A.stride[1], gather_pitch_floats(mode), p.a_rows);
+    st->maps_a.count = (int)(k.M < 4 ? k.M : 4);
+    for (int c = 0; c < st->maps_a.count && ok; ++c) {
+      st->maps_a.shift[c] = gather_shift(A, c);
+      ok = encode_map_rows(&st->maps_a.of[c], A.ptr + c * A.stride[1] - st->maps_a.shift[c], k.K + st->maps_a.shift[c], (k.M - c + 3) / 4, 4 * A.stride[1], gather_pitch_floats(mode), p.a_rows);
     }
-    for (int c = p.a_maps; c < 4; ++c) {           // (not used)
+    for (int c = st->maps_a.count; c < 4; ++c) {           // (not used)
       st->maps_a.of[c] = st->maps_a.of[0];
-      p.a_shift[c] = 0;
+      st->maps_a.shift[c] = 0;
     }
   }
   if (!gather) ok = (form == SMALL_A_FLOAT32 ? encode_map(&st->map_a, false, A.ptr, k.K, k.M, 1, A.stride[1], 0, 32, p.a_rows, false)
@@ -948,8 +954,8 @@ bool small_repoint(const PlanKernel& k, void* state) {
   if (st->params.out) st->params.out = k.ops[k.chain.out_slot].ptr;
   const DevOperand& A = k.ops[k.desc.a_slot];
   bool ok = true;
-  for (int c = 0; st->gather && c < st->params.a_maps; ++c)      // (by a multiple of 16 bytes: the shifts stay)
-    ok = ok && set_map_address(&st->maps_a.of[c], A.ptr + c * A.stride[1] - st->params.a_shift[c]);
+  for (int c = 0; st->gather && c < st->maps_a.count; ++c)      // (by a multiple of 16 bytes: the shifts stay)
+    ok = ok && set_map_address(&st->maps_a.of[c], A.ptr + c * A.stride[1] - st->maps_a.shift[c]);
   return ok && (st->gather || !st->a_moves || set_map_address(&st->map_a, A.ptr)) &&
          (!st->b_moves || set_map_address(&st->map_b, k.ops[k.desc.b_slot].ptr));
 }
