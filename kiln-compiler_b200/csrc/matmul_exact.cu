@@ -111,6 +111,10 @@ ExactPlan plan_exact(const Plan& plan, int64_t m, int64_t n, int64_t k, bool spl
   return best;
 }
 
+ExactKernel kernel_for(const ExactPlan& how, int fin) {
+  return how.parts > 1 ? exact_kernel<2, true>(fin) : how.bn > 192 ? exact_kernel<4, false>(fin) : how.bn > 128 ? exact_kernel<3, false>(fin) : exact_kernel<2, false>(fin);
+}
+
 }  // namespace
 
 int64_t exact_cycles(const Plan& plan, const PlanKernel& k) {
@@ -123,6 +127,14 @@ int64_t exact_cycles(const Plan& plan, const PlanKernel& k) {
   const DevOperand& O = k.ops[k.chain.out_slot];
   if (O.stride[2] != 1 || O.stride[1] % 4 || O.stride[1] < k.N || !aligned16(O.ptr)) return -1;
   return plan_exact(plan, k.M, k.N, k.K, k.planes_expected).cycles;
+}
+
+int exact_runs(const Plan& plan, const PlanKernel& k, bool* runs) {
+  int bias_slot, res_slot;
+  cudaFuncAttributes attributes;
+  KB200_CUDA(cudaFuncGetAttributes(&attributes, kernel_for(plan_exact(plan, k.M, k.N, k.K, k.planes_expected), finish_of(k, &bias_slot, &res_slot))));
+  *runs = attributes.numRegs == 168;
+  return KB200_OK;
 }
 
 int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands& ops, void** state) {
@@ -177,12 +189,9 @@ int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands&
   if (ok && p.res) ok = encode_map_store(&st->map_res, false, p.res, k.N, k.M, 1, p.res_row, 0);
   if (ok && p.with_tail) ok = set_map_address(&st->map_tail, k.tail_out);
   if (!ok) { delete st; return KB200_OK; }
-  st->kernel = st->parts > 1 ? exact_kernel<2, true>(fin) : p.bn > 192 ? exact_kernel<4, false>(fin) : p.bn > 128 ? exact_kernel<3, false>(fin) : exact_kernel<2, false>(fin);
+  st->kernel = kernel_for(how, fin);
   const cudaError_t e = cudaFuncSetAttribute(st->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kExactSmem);
   if (e != cudaSuccess) { delete st; return cuda_fail(e, "cudaFuncSetAttribute(mm_exact_kernel)"); }
-  cudaFuncAttributes attributes;
-  KB200_CUDA(cudaFuncGetAttributes(&attributes, st->kernel));
-  if (attributes.numRegs != 168) { delete st; return KB200_OK; }      // (the warps that ask for more would wait for ever)
   *state = st;
   return KB200_OK;
 }

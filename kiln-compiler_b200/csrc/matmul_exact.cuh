@@ -26,7 +26,7 @@
 // Rows of A whose elements are more than 2^28 apart come in further levels (split16.cuh): their tiles go over K once more per level, with the planes of
 // that level and the same ones of B, and the sums of its steps are multiplied by the level's power of two as they are added up, by 0 for rows
 // that have none.  Why not per row: a tile multiplies 256 of them anyway.  1024 x 2304 x 768 15.5 us (with the pass), one such row 20.0, all 23.7, all with
-// two levels 30.5; 4096^3 331, 365, 643, 984.  Of normally distributed rows about one in 10^5 has such an element by chance.  (Where no row has
+// two levels 30.5; 4096^3 331, 365, 643, 984.  Of normally distributed rows of 768 one in 2 10^5 has such an element by chance.  (Where no row has
 // one, asking costs a launch behind another ~0.2 us: 1024 x 768 block 75.6 -> 77.8.)
 // Every wait is bounded: see matmul_pair.cu.
 #pragma once

@@ -17,6 +17,8 @@ struct ExactOperands {
 
 // Estimated cycles of a launch, or -1 when the kernel does not cover this matmul.
 int64_t exact_cycles(const Plan& plan, const PlanKernel& k);
+// Does this build of its kernel have the registers that its warps share out?  (With fewer those that ask for more would wait for ever.)
+int exact_runs(const Plan& plan, const PlanKernel& k, bool* runs);
 // *state stays null when the operands cannot be described; a non-zero return is an error.
 int exact_bind(Plan& plan, PlanKernel& k, int kernel_index, const ExactOperands& ops, void** state);
 int exact_launch(const Plan& plan, const void* state, cudaStream_t s);

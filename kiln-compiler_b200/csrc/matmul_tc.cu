@@ -1065,6 +1065,8 @@ int bind_pairs16(Plan& plan, PlanKernel& k, int kernel_index, TcState* st, bool 
   const int64_t pitch = (k.K + 63) / 64 * 64;              // rows on 128-byte lines
   const uint64_t a_bytes = (uint64_t)k.M * pitch * 4 * kLevels;
   if (a_bytes > plan.copy_budget) return KB200_OK;
+  bool runs = false;
+  if (const int rc = exact_runs(plan, k, &runs); rc || !runs) return rc;
   const size_t scale_bytes = (size_t)(k.M + k.N + 3) / 4 * 4 * sizeof(float), mark_bytes = (size_t)(k.M + 255) / 256 * 256;
   TcState::Pairs16& h = st->pairs16;
   const size_t turned_floats = turn ? (size_t)k.N * k.K : 0;
