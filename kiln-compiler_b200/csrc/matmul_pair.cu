@@ -719,7 +719,8 @@ PairPlan plan_pair(const Plan& plan, const PlanKernel& k, bool two_slabs, bool b
     if (w.halves == 0 || slabs < 8 || 2 * tiles > share || tiles > resident_quads(plan)) continue;
     const int64_t halved = w.halves + (slabs + 1) / 2 * w.half_alone + ((slabs + 1) / 2 * (w.half_full - w.half_alone) + kPairHalvesBusy) * 2 * tiles / share;
     // (Of two that cost alike by the lines halves move fewer bytes: 1900 x 960 x 3840 TF32 25.8 us at 128 columns with its operands in L2 and up to 31
-    // behind another matmul, 25.8 and 26.4 in halves of 256.)
+    // behind another matmul, 25.8 and 26.4 in halves of 256.  Of 264 launches of 300 to 3600 rows with 64 slabs and more, ten go by it, TF32 of 3840 and BF16 of
+    // 7680 of K: 2 to 24 % less time each, 11 % on average.)
     const int64_t as = slabs < 64 ? halved : halved * 49 / 50;
     if (as < least) best = {w.bn, true, halved}, least = as;
   }
@@ -749,7 +750,8 @@ int width_in_flight(const Plan& plan, const PlanKernel& k, bool two_slabs, bool 
 
 // (in the few-tiles kernel's cycles, which its estimate counts at 1.65 to the ns, this one's at 1.86: of 281 launches the choice is then 0.1 % (TF32)
 // and 0.3 % (BF16) from the better kernel.  A GELU in float32 costs this kernel's last
-// tile 0.9 us, that one's, spread over more warps, 0.55: 1002 x 1024 x 256 6.55 and 6.15, without it 5.5 both.)
+// tile 0.9 us, that one's, spread over more warps, 0.55: 1002 x 1024 x 256 6.55 and 6.15, without it 5.5 both.  Of 140 TF32 launches with a GELU, 200 to 1700 rows, 17 go by it, K of 512
+// and 768: 4 to 10 % less time each.)
 int64_t pair_cycles(const Plan& plan, const PlanKernel& k, bool b_kmajor) {
   const bool gelu = k.desc.precision == KB200_PREC_TF32 && k.chain.n > 0 && k.chain.steps[k.chain.n - 1].op == CH_GELU_TANH;
   return (plan_pair(plan, k, true, b_kmajor).cycles + (gelu ? 700 : 0)) * 8 / 9;
