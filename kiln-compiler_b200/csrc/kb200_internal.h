@@ -110,6 +110,7 @@ struct PlanKernel {
   // FP32: bounds of a matmul's results by column (see result_bounds), once they have been looked for, and whether its producer will split its rows
   std::vector<float> bounds;
   bool bounds_known = false;
+  bool bounds_near = false;       // ... whether no row's results are far below them
   bool planes_expected = false;
   float* tail_out = nullptr;      // FP32: where the tails of the output (what a TF32 operand drops) go as well, same offsets, or null
   bool mirror_only = false;       // producer side: every reader of the output takes the mirror, the float32 store is dropped

@@ -32,9 +32,9 @@ void exact_destroy(void* state);
 // float32 rows of `cols` elements -> the two planes and the scales; with `marks` of every level.  A pass in front of a launch, or once for a weight.
 int split_rows(const float* src, int64_t s_row, void* planes, int64_t pitch, float* scale, uint8_t* marks, int64_t rows, int64_t cols, bool pdl, cudaStream_t s);
 // |LayerNorm(x) B + bias| per column of B [K, N] for any x, at most: of the normalised row, 1 / sqrt(inv_n) long, by Cauchy and Schwarz.  `bounds`: [n]
-// on the host; empty where a column's result for a row of nearly equal elements (whose LayerNorm is next to beta) is below 2^-30 of its bound, so
-// that float16 pairs under the bound's power of two might not hold it: no biases at all, as a rule.  Synchronises.
-int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds);
+// on the host.  `near`: no column's result for a row of nearly equal elements (whose LayerNorm is next to beta) is below 2^-30 of its bound; else,
+// without any biases as a rule, float16 pairs under the bound's power of two do not hold the results of rows of next to nothing.  Synchronises.
+int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds, bool* near);
 // Do float16 pairs hold this weight [K, N] as well as TF32 pairs would?  `scratch`: k + 1 words on the device.  Synchronises.
 int split_suits(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, uint32_t* scratch, bool* suits);
 

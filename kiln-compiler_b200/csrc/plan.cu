@@ -983,7 +983,7 @@ static PlanKernel* layernorm_in_front(Plan& plan, size_t ki) {
 
 // Bounds of a matmul's results by column, whatever the input: of a LayerNorm's rows and frozen parameters, with a bias and a GELU (which is
 // no larger than its argument).  Empty where nothing is known.
-static int look_for_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
+static int look_for_bounds(Plan& plan, size_t ki, std::vector<float>* bounds, bool* near) {
   const PlanKernel& k = plan.kernels[ki];
   const PlanKernel* const norm = layernorm_in_front(plan, ki);
   auto frozen = [](const PlanKernel& of, int slot) { return of.desc.operands[slot].base_kind == KB200_BASE_CONST; };
@@ -997,7 +997,7 @@ static int look_for_bounds(Plan& plan, size_t ki, std::vector<float>* bounds) {
   }
   if (k.chain.n == 2 && k.chain.steps[1].op != CH_GELU_TANH) return KB200_OK;
   const DevOperand& B = k.ops[k.desc.b_slot];
-  const int rc = layernorm_bounds(B.ptr, B.stride[1], B.stride[2], k.K, k.N, norm->ops[norm->g_slot].ptr, norm->ops[norm->b_slot].ptr, bias, norm->ln_inv_n, bounds);
+  const int rc = layernorm_bounds(B.ptr, B.stride[1], B.stride[2], k.K, k.N, norm->ops[norm->g_slot].ptr, norm->ops[norm->b_slot].ptr, bias, norm->ln_inv_n, bounds, near);
   if (rc) return rc;
   for (float b : *bounds)
     if (!(b < 1e30f)) { bounds->clear(); break; }
@@ -1008,7 +1008,7 @@ static int result_bounds(Plan& plan, size_t ki, const std::vector<float>** bound
   *bounds = &k.bounds;
   if (k.bounds_known) return KB200_OK;
   k.bounds_known = true;
-  return look_for_bounds(plan, ki, &k.bounds);
+  return look_for_bounds(plan, ki, &k.bounds, &k.bounds_near);
 }
 
 // `host` on the device, for as long as the plan is bound as it is.  Null where memory is short.
@@ -1029,11 +1029,13 @@ static float pair_scale(float bound) {
   return ldexpf(1.0f, 15 - e);
 }
 
-// Can results with these bounds by column leave as float16 pairs under one power of two?  A column whose bound is far above the others' -- a unit that a
-// bias of -1e9 switches off, say -- would leave the others none of the bits.  (Columns that are zero for any input take no part.)
-static bool one_scale_suits(const std::vector<float>& bounds) {
+// Can a matmul's results, whose bounds have been looked for, leave as float16 pairs under one power of two?  A column whose bound is far above the
+// others' -- a unit that a bias of -1e9 switches off, say -- would leave the others none of the bits, and so would a bound that a row's results may be
+// far below.  (Columns that are zero for any input take no part.)
+static bool one_scale_suits(const PlanKernel& k) {
+  if (!k.bounds_near) return false;
   float least = INFINITY, most = 0.0f;
-  for (float b : bounds)
+  for (float b : k.bounds)
     if (b != 0.0f) least = std::min(least, b), most = std::max(most, b);
   return most > 0.0f && most <= 1024.0f * least;
 }
@@ -1065,7 +1067,7 @@ static int expect_planes(Plan& plan, size_t ki) {
   if (from->impl != IMPL_MM_TC || !matmul_takes_planes(*from, &planes) || from->N != k.K) return KB200_OK;
   const std::vector<float>* bounds = nullptr;
   const int rc = result_bounds(plan, (size_t)(from - plan.kernels.data()), &bounds);
-  k.planes_expected = rc == KB200_OK && one_scale_suits(*bounds);
+  k.planes_expected = rc == KB200_OK && one_scale_suits(*from);
   return rc;
 }
 
@@ -1125,7 +1127,7 @@ static int hand_on_planes(Plan& plan) {
     const std::vector<float>* bounds = nullptr;
     const int rc = result_bounds(plan, fi, &bounds);
     if (rc) return rc;
-    if (!one_scale_suits(*bounds)) continue;
+    if (!one_scale_suits(*from)) continue;
     const float scale = pair_scale(*std::max_element(bounds->begin(), bounds->end()));
     const float* const by = keep_scales(plan, std::vector<float>((size_t)(from->N + 31) / 32, scale));
     const bool alone = plan.mirror_only && only_read_as(plan, fi, span_of(*from, from->chain.out_slot), reads_here);
@@ -1320,7 +1322,7 @@ KB200_EXPORT int kb200_plan_bind(kb200_plan* p, void* arena, uint64_t arena_byte
     k.tail_out = nullptr;
     k.planes_out = PlanKernel::Planes();
     k.bounds.clear();
-    k.bounds_known = k.planes_expected = false;
+    k.bounds_known = k.bounds_near = k.planes_expected = false;
     k.absorbed_by = -1;
     k.n_ops = k.desc.n_operands;
     rc = resolve(plan, k, (int)i);

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) bound_kernel(const float* __restrict__ b,
 
 }  // namespace
 
-int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds) {
+int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_t n, const float* gamma, const float* beta, const float* bias, float inv_n, std::vector<float>* bounds, bool* near) {
   std::vector<float> both((size_t)n * 2);
   float* device = nullptr;
   KB200_CUDA(cudaMalloc(&device, both.size() * sizeof(float)));
@@ -152,11 +152,8 @@ int layernorm_bounds(const float* b, int64_t b_k, int64_t b_n, int64_t k, int64_
   cudaFree(device);
   if (e != cudaSuccess) return cuda_fail(e, "the bounds of a matmul's results");
   bounds->assign(both.begin(), both.begin() + n);
-  for (int64_t i = 0; i < n; ++i)
-    if (both[i] != 0.0f && !(both[n + i] >= both[i] * 0x1p-30f)) {
-      bounds->clear();
-      break;
-    }
+  *near = true;
+  for (int64_t i = 0; i < n && *near; ++i) *near = both[i] == 0.0f || both[n + i] >= both[i] * 0x1p-30f;
   return KB200_OK;
 }
 

@@ -43,3 +43,21 @@ def test_tails_of_the_projection_are_those_of_the_pass(tokens, batch, odd):
     if not odd:
         added, want = reference(consts, x, 12)
         assert float((got.double() - want).norm() / added.norm()) <= BOUND["tf32"]
+
+
+@pytest.mark.parametrize("std", [1.0, 1e-8])
+@pytest.mark.parametrize("tokens,batch", [(1024, None), (333, 6)])
+def test_blocks_without_biases(tokens, batch, std):
+    """Rows of next to nothing come out of a LayerNorm far below the bounds of what follows."""
+    from test_gpu_attention_pairs import BOUND as PAIRS
+
+    def change(consts, x):
+        for name in consts:
+            if name.endswith("bias"):
+                consts[name][:] = 0
+        x *= std
+
+    exe, consts, x, got = block(tokens, 12, batch, change)
+    assert any("on float16 pairs" in detail for detail in exe.details), exe.details
+    added, want = reference(consts, x, 12)
+    assert float((got.double() - want).norm() / added.norm()) <= PAIRS

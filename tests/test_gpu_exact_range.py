@@ -33,7 +33,7 @@ def errors(got, want, dim):
     return (got.double() - want).norm(dim=dim) / want.norm(dim=dim)
 
 
-@pytest.mark.parametrize("odd", ["a unit switched off", "a unit switched off for good", "a column of zeros"])
+@pytest.mark.parametrize("odd", ["a unit switched off", "a unit switched off for good", "a column of zeros", "a column far above"])
 def test_units_of_very_different_bounds(odd):
     """One power of two for all of a Linear's results would be that of the largest bound: the others keep their bits."""
     m, d, wide = 1024, 768, 3072
@@ -41,11 +41,15 @@ def test_units_of_very_different_bounds(odd):
     if odd == "a column of zeros":
         consts["fc.weight.transpose"][:, 5] = 0
         consts["fc.bias"][5] = 0
+    elif odd == "a column far above":
+        consts["fc.weight.transpose"][:, 5] *= np.float32(2.0**20)
+        consts["proj.weight.transpose"][5, ::2] = 0          # half of the results do not use it
     else:
         consts["fc.bias"][5] = -1e20 if odd.endswith("good") else -1e9
     x = torch.randn(m, d, generator=torch.Generator(device="cuda").manual_seed(0), device="cuda")
     exe, got = run_plan(plan, consts, x)
-    assert float(errors(got, mlp_reference(consts, x), 1).max()) <= 4 * BOUND
+    looked_at = slice(None, None, 2 if odd == "a column far above" else 1)
+    assert float(errors(got[:, looked_at], mlp_reference(consts, x)[:, looked_at], 1).max()) <= 4 * BOUND
     assert all("mm_exact" in detail for detail in exe.details[1:]), exe.details
     assert ("A copied" in exe.details[2]) == (odd != "a column of zeros"), exe.details
 
