@@ -7,7 +7,8 @@
 //   * the tensor core cuts off a bit of an accumulator with every MMA: sums in it are over 64 keys (the head dimension in Q K^T), small
 //     products first, and everything beyond is added up in float32 registers.
 // From float64, merged heads of 12 heads: 1024 tokens 2.1e-7 (TF32 1.8e-6, the CUDA cores 2.6e-7), 2048 tokens 2.1e-7 (1.8e-6, 3.3e-7), 200 tokens
-// 2.8e-7 (1.0e-6, 2.6e-7).  So it takes sequences of any length, which the TF32 form left to the CUDA cores: 12 heads of 1500 tokens
+// 2.8e-7 (1.0e-6, 2.6e-7); with the projection's error, four seeds: 129 tokens 2.4e-7 (CUDA cores 2.1e-7), 333 2.7e-7 (2.5e-7), 512 2.7e-7 (2.6e-7), 1024
+// 2.8e-7 (2.9e-7): what four MMAs of 16 dims cut off a score.  So it takes sequences of any length, which the TF32 form left to the CUDA cores: 12 heads of 1500 tokens
 // 126 -> 25 us, of 333 tokens 18.1 -> 11.3 with the pass, 96 heads of 1024 tokens 128 (TF32) -> 53.  What bounds a tile is the softmax warps (a score costs
 // them a maximum, an exponential, four conversions and their stores) beside 36 MMAs of ~50 cycles of issue.
 #pragma once
